@@ -1,0 +1,113 @@
+"""Elementwise programs as the chain kernel runs them: random programs, lengths around the groups of four and the blocks of
+1024, unaligned tensors, several loads of one input, unused inputs, accumulation."""
+import numpy as np
+import pytest
+
+from conftest import rel_err_ok
+
+pytestmark = pytest.mark.gpu
+
+BINARY, UNARY = ("add", "sub", "mul", "div"), ("neg", "abs", "tanh", "relu", "gelu", "elu", "exp", "log")
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    yield c
+    c.sync()
+    c.destroy()
+
+
+def random_program(r, length, ninputs):
+    """Values stay away from zero denominators and overflow: div and log read an input (positive), exp reads a tanh."""
+    prog, inputs, tanhs = [("input", 0, 0, 0.0)], [0], []
+    while len(prog) < length:
+        k, kind = len(prog), r.integers(0, 8)
+        if kind == 0 and k < length - 1:
+            prog.append(("input", int(r.integers(0, ninputs)), 0, 0.0))
+            inputs.append(k)
+        elif kind == 1 and k < length - 1:
+            prog.append(("const", 0, 0, float(np.float32(r.uniform(-1, 1)))))
+        elif kind <= 4:
+            op = BINARY[r.integers(0, 4)]
+            b = int(r.choice(inputs)) if op == "div" else int(r.integers(0, k))
+            if op == "mul":             # products of products would grow without bound
+                b = int(r.choice(inputs))
+            prog.append((op, k - 1 if r.integers(0, 2) else int(r.integers(0, k)), b, 0.0))
+        else:
+            op = UNARY[r.integers(0, 8)]
+            a = int(r.integers(0, k))
+            if op == "log":
+                a = int(r.choice(inputs))
+            if op == "exp":
+                if not tanhs:
+                    op = "tanh"
+                else:
+                    a = int(r.choice(tanhs))
+            if op == "tanh":
+                tanhs.append(k)
+            prog.append((op, a, 0, 0.0))
+    return prog
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 515, 1023, 1028, 2051, 70001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_random_programs(ctx, oracle, n, shift):
+    r = np.random.Generator(np.random.Philox(n * 2 + shift))
+    for length in (1, 2, 5, 12, 24):
+        ninputs = int(r.integers(1, 5))
+        prog = random_program(r, length, ninputs)
+        x = [(np.abs(r.standard_normal(n)) * 0.5 + 0.75).astype(np.float32) for _ in range(ninputs)]
+        seed = r.standard_normal(n).astype(np.float32)
+
+        def place(a):       # shift = 1: one element past a 16-byte boundary
+            return ctx.init_tensor_f32((n + shift,), np.concatenate([np.zeros(shift, np.float32), a]))
+
+        at = lambda t: t.ptr + 4 * shift                                   # noqa: E731
+        take = lambda t: ctx.to_numpy(t)[shift:]                           # noqa: E731
+        xd, sd, out = [place(a) for a in x], place(seed), place(np.zeros(n, np.float32))
+        k = int(r.integers(0, length))
+        kept = place(np.zeros(n, np.float32))
+        ctx.eltwise_chain_fwd(prog, [at(t) for t in xd], at(out), n, saved={k: at(kept)})
+        ref, saved = oracle.eltwise_fwd(prog, x, save=(k,))
+        # each of up to 24 operations contributes a few units of 2^-24 of values of order one
+        for got, want in ((take(out), ref), (take(kept), saved[k])):
+            ok, worst = rel_err_ok(got, want, 2e-5)
+            assert ok, (prog, worst)
+        base = [r.standard_normal(n).astype(np.float32) for _ in range(ninputs)]
+        gref = oracle.eltwise_bwd(prog, x, seed)
+        for accumulate in (False, True):
+            gd = [place(b) for b in base]
+            want_grad = [bool(r.integers(0, 4)) for _ in range(ninputs)]
+            ctx.eltwise_chain_bwd(prog, [at(t) for t in xd], at(sd), [at(g) if w else None for g, w in zip(gd, want_grad)], n,
+                                  accumulate=accumulate)
+            for g, w, b, gr in zip(gd, want_grad, base, gref):
+                ok, worst = rel_err_ok(take(g), (b + gr if accumulate else gr) if w else b, 5e-5)
+                assert ok, (prog, accumulate, worst)
+
+
+def test_output_may_overwrite_an_input(ctx, oracle):
+    r = np.random.Generator(np.random.Philox(9))
+    n = 5003
+    w, g = r.standard_normal(n).astype(np.float32), r.standard_normal(n).astype(np.float32)
+    prog = [("input", 0, 0, 0.0), ("input", 1, 0, 0.0), ("const", 0, 0, 0.5), ("mul", 1, 2, 0.0), ("sub", 0, 3, 0.0)]
+    wd = ctx.init_tensor_f32((n,), w)
+    ctx.eltwise_chain_fwd(prog, [wd, ctx.init_tensor_f32((n,), g)], wd, n)
+    assert np.array_equal(ctx.to_numpy(wd), oracle.eltwise_fwd(prog, [w, g])[0])
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+def test_gelu_of_extreme_values(ctx, dtype):
+    # the limits: x for large positive, zero for large negative, NaN stays NaN, +inf stays +inf
+    x = np.array([0.0, -0.0, 30.0, -30.0, 3e4, -3e4, np.inf, np.nan, 1e-6, -1e-6], np.float32)
+    n = x.size
+    init = {"f32": ctx.init_tensor_f32, "f16": ctx.init_tensor_f16, "bf16": ctx.init_tensor_bf16}[dtype]
+    t, out = init((n,), x), init((n,), np.zeros(n))
+    ctx.eltwise_chain_fwd([("input", 0, 0, 0.0), ("gelu", 0, 0, 0.0)], [t], out, n, dtype=dtype)
+    back = ctx.new_tensor((n,))
+    ctx.convert(out, dtype, back, "f32", n)
+    ctx.convert(t, dtype, t32 := ctx.new_tensor((n,)), "f32", n)
+    y, x = ctx.to_numpy(back), ctx.to_numpy(t32)
+    assert y[0] == 0 and y[1] == 0 and y[2] == x[2] and y[3] == 0 and y[4] == x[4] and y[5] == 0 and np.isposinf(y[6]) and np.isnan(y[7])
+    assert np.allclose(y[8:], 0.5 * x[8:], rtol=2e-2, atol=0) or dtype == "f16"       # 1e-6 is a subnormal half
