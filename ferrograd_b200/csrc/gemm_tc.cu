@@ -433,8 +433,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmA16, const __grid_constant__ CUtensorMap tmB16, Epilogue ep) {
     static_assert(FMT == 0 || BK == 32, "the bf16 planes use 64-byte rows: 32 values of k per block");
-    // FMT 2 (bf16) and 3 (f16): the operands ARE 16-bit tensors, loaded as they lie (K-major, 64 values of
-    // k = one 128-byte row per k-block) and multiplied by one kind::f16 MMA per 16 values of k.
+    // FMT 2 (bf16) and 3 (f16): the operands ARE 16-bit tensors, loaded as they lie (64 values of k per k-block)
+    // and multiplied by one kind::f16 MMA per 16 values of k.
     constexpr bool kDirect16 = FMT >= 2;
     constexpr uint32_t KBE = kDirect16 ? 2 * BK : BK;            // values of k per k-block
     constexpr uint32_t kChunk = kDirect16 ? 1024 : kChunkK;      // 16-bit results tolerate the longer chain
@@ -530,8 +530,18 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const uint32_t sa = base + s * Cfg::kStageBytes;
                     if (kDirect16) {
                         if (leader) mbar_expect_tx(full_bar(s), 2 * Cfg::kStageBytes);   // both CTAs' bytes
-                        tma_load_3d_pair(sa, &tmA16, lf, (int)(kb * KBE), (int)m0, 0);
-                        tma_load_3d_pair(sa + Cfg::kABytes, &tmB16, lf, (int)(kb * KBE), (int)nb0, 0);
+                        // One operand tile = 128 rows x 64 values of k.  K-major storage: one box; MN-major storage
+                        // ([k][rows]): two boxes of 64 rows x 64 k, each [k][64 rows], 8 KiB.
+                        auto load16 = [&](uint32_t dst, const CUtensorMap* t16, bool mn, uint32_t r0) {
+                            if (!mn) {
+                                tma_load_3d_pair(dst, t16, lf, (int)(kb * KBE), (int)r0, 0);
+                            } else {
+                                tma_load_3d_pair(dst, t16, lf, (int)r0, (int)(kb * KBE), 0);
+                                tma_load_3d_pair(dst + 8192, t16, lf, (int)(r0 + 64), (int)(kb * KBE), 0);
+                            }
+                        };
+                        load16(sa, &tmA16, ep.a_mn != 0, m0);
+                        load16(sa + Cfg::kABytes, &tmB16, ep.b_mn != 0, nb0);
                         continue;
                     }
                     if (leader) mbar_expect_tx(full_bar(s), 2 * Cfg::kStageBytes);   // both CTAs' bytes
@@ -614,12 +624,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         const uint64_t b_hi = make_desc_kmajor<BK * 4>(sa + Cfg::kABytes);
                         const uint32_t first = (kb == c * kChunkKB) ? 0u : 1u;   // a chunk starts from zero
                         if (kDirect16) {
-                            constexpr uint32_t idesc16 = make_idesc(FMT == 2 ? 1u /*bf16*/ : 0u /*f16*/, 2 * BM, BN);
+                            // K-major: 16 values of k are 32 bytes inside the swizzled row.  MN-major: 16 k-rows are two
+                            // 1024-byte atoms, and the tile's two 64-row column blocks are 8 KiB apart.
+                            const uint32_t idesc16 = make_idesc(FMT == 2 ? 1u /*bf16*/ : 0u /*f16*/, 2 * BM, BN) |
+                                                     (ep.a_mn ? kIdescAMnMajor : 0u) | (ep.b_mn ? kIdescBMnMajor : 0u);
+                            const uint64_t a_d = ep.a_mn ? make_desc_mnmajor(sa, 8192, 1024, 2) : a_hi;
+                            const uint64_t b_d = ep.b_mn ? make_desc_mnmajor(sa + Cfg::kABytes, 8192, 1024, 2) : b_hi;
+                            const uint32_t a_adv = ep.a_mn ? 128u : 2u, b_adv = ep.b_mn ? 128u : 2u;
 #pragma unroll
-                            for (int kk = 0; kk < (int)KBE / 16; ++kk) {
-                                const uint64_t adv = (uint64_t)(kk * 16 * 2 >> 4);
-                                mma_f16_pair(d_tmem, a_hi + adv, b_hi + adv, idesc16, first | (uint32_t)kk);
-                            }
+                            for (int kk = 0; kk < (int)KBE / 16; ++kk)
+                                mma_f16_pair(d_tmem, a_d + (uint64_t)(kk * a_adv), b_d + (uint64_t)(kk * b_adv), idesc16,
+                                             first | (uint32_t)kk);
                         } else if (FMT == 0) {
                             const uint64_t a_lo = make_desc_kmajor<BK * 4>(sa + BM * BK * 4);
                             const uint64_t b_lo = make_desc_kmajor<BK * 4>(sa + Cfg::kABytes + HB * BK * 4);
@@ -1277,10 +1292,17 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     int32_t s;
     constexpr bool kDirect16 = FMT >= 2;
     if (kDirect16) {
-        // the operands themselves: one 16-bit "plane", 64 values of k (128 bytes) per row of a k-block
-        const int elem = FMT == 2 ? 1 : 2;
-        if ((s = make_tmap(ctx, &tmA16, a.p16, elem, 1, ep.M, ep.K, a.ld16, BM, 2 * BK)) != FG_OK) return s;
-        if ((s = make_tmap(ctx, &tmB16, b.p16, elem, 1, ep.N, ep.K, b.ld16, Cfg::kBN / 2, 2 * BK)) != FG_OK) return s;
+        // the operands themselves, 64 values of k per k-block: boxes of 128 rows x 64 k, or 64 k x 64 rows when the
+        // rows are contiguous
+        auto map16 = [&](CUtensorMap* t, const PlaneSet& o, uint32_t rows, uint32_t tile_rows) -> int32_t {
+            const int elem = FMT == 2 ? 1 : 2;
+            if (!o.mn) return make_tmap(ctx, t, o.p16, elem, 1, rows, ep.K, o.ld16, tile_rows, 2 * BK);
+            return make_tmap3(ctx, t, o.p16, elem, rows, ep.K, 1, (uint64_t)o.ld16 * 2, (uint64_t)ep.K * o.ld16 * 2, 64, 2 * BK, 1);
+        };
+        if ((s = map16(&tmA16, a, ep.M, BM)) != FG_OK) return s;
+        if ((s = map16(&tmB16, b, ep.N, Cfg::kBN / 2)) != FG_OK) return s;
+        ep.a_mn = a.mn ? 1u : 0u;
+        ep.b_mn = b.mn ? 1u : 0u;
         tmA = tmA16;
         tmB = tmB16;
     } else {
@@ -2042,10 +2064,10 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
 
 // ------------------------------------------------------------------------------------
 // 16-bit storage (f16 / bf16 tensors, f32 accumulation).  The operands are multiplied as they
-// are: one kind::f16 MMA per 16 values of k, no operand planes.  What the tensor core needs is
-// the contraction index contiguous, rows 16-byte aligned; an operand that already lies that way
-// is loaded in place, the others go through prep16_kernel (copy with padded pitch and/or
-// transpose, optionally fused with dY * act'(saved) and the bias gradient's column sums).
+// lie: one kind::f16 MMA per 16 values of k, read through K-major or MN-major descriptors, so
+// nothing is transposed.  What the loads need is a 16-byte aligned base and row pitch; a tensor
+// without them is copied once with its pitch padded, and dZ = dY * act'(saved) is formed once
+// (both by prep16_kernel, which also sums dZ's columns for the bias gradient).
 // ------------------------------------------------------------------------------------
 namespace {
 
@@ -2054,9 +2076,8 @@ struct Prep16Args {
     const void* saved;    // non-NULL: value = x * act'(saved), rounded to the storage type
     int act;
     uint32_t R, C;
-    void* n_out;          // [R][ld_n] or NULL
-    void* t_out;          // [C][ld_t] or NULL
-    uint32_t ld_n, ld_t;
+    void* out;            // [R][ld] or NULL
+    uint32_t ld;
     float* colsum_part;   // [ceil(R/32)][C] f32 or NULL
 };
 
@@ -2067,63 +2088,93 @@ template <typename T> __device__ __forceinline__ T lp_from_float(float v);
 template <> __device__ __forceinline__ __half lp_from_float<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 lp_from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-template <typename T>
+// W columns per thread (8: one 128-bit access; 1: any shape and alignment), 32 rows x 32 * W columns per block.
+template <typename T, int W>
 __global__ void __launch_bounds__(256) prep16_kernel(const Prep16Args a) {
-    __shared__ T tile[32][33];
-    __shared__ float cs[8][33];
-    const uint32_t c = blockIdx.x * 32 + threadIdx.x;
+    __shared__ float cs[8][32 * W + 1];
+    const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * W;
     const uint32_t r0 = blockIdx.y * 32;
-    float colsum = 0.0f;
+    struct __align__(W * 2) Vec { T e[W]; };
+    float sum[W];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const uint32_t lr = threadIdx.y + 8 * k, r = r0 + lr;
-        T v = lp_from_float<T>(0.0f);
-        if (r < a.R && c < a.C) {
-            const size_t i = (size_t)r * a.C + c;
-            v = static_cast<const T*>(a.x)[i];
-            if (a.saved)
-                v = lp_from_float<T>(lp_to_float(v) * fg_act_grad(a.act, lp_to_float(static_cast<const T*>(a.saved)[i])));
-            if (a.n_out) static_cast<T*>(a.n_out)[(size_t)r * a.ld_n + c] = v;
-            colsum += lp_to_float(v);
-        }
-        tile[lr][threadIdx.x] = v;
-    }
-    if (a.colsum_part) cs[threadIdx.y][threadIdx.x] = colsum;
-    __syncthreads();
-    if (a.colsum_part && threadIdx.y == 0 && c < a.C) {
-        float t = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t += cs[k][threadIdx.x];
-        a.colsum_part[(size_t)blockIdx.y * a.C + c] = t;
-    }
-    if (a.t_out) {
-        const uint32_t tr = r0 + threadIdx.x;          // row of x = column of the transposed copy
+    for (int w = 0; w < W; ++w) sum[w] = 0.0f;
+    if (c < a.C) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint32_t lc = threadIdx.y + 8 * k, tc = blockIdx.x * 32 + lc;
-            if (tc < a.C && tr < a.R) static_cast<T*>(a.t_out)[(size_t)tc * a.ld_t + tr] = tile[threadIdx.x][lc];
+            const uint32_t r = r0 + threadIdx.y + 8 * k;
+            if (r >= a.R) break;
+            const size_t i = (size_t)r * a.C + c;
+            Vec v = *reinterpret_cast<const Vec*>(static_cast<const T*>(a.x) + i);
+            if (a.saved) {
+                const Vec sv = *reinterpret_cast<const Vec*>(static_cast<const T*>(a.saved) + i);
+#pragma unroll
+                for (int w = 0; w < W; ++w) v.e[w] = lp_from_float<T>(lp_to_float(v.e[w]) * fg_act_grad(a.act, lp_to_float(sv.e[w])));
+            }
+            if (a.out) *reinterpret_cast<Vec*>(static_cast<T*>(a.out) + (size_t)r * a.ld + c) = v;
+#pragma unroll
+            for (int w = 0; w < W; ++w) sum[w] += lp_to_float(v.e[w]);
         }
+    }
+    if (!a.colsum_part) return;
+#pragma unroll
+    for (int w = 0; w < W; ++w) cs[threadIdx.y][threadIdx.x * W + w] = sum[w];
+    __syncthreads();
+    const uint32_t t = threadIdx.y * 32 + threadIdx.x, col = blockIdx.x * (32 * W) + t;
+    if (t < 32 * W && col < a.C) {
+        float z = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) z += cs[k][t];
+        a.colsum_part[(size_t)blockIdx.y * a.C + col] = z;
     }
 }
 
-int32_t launch_prep16(fg_ctx* ctx, int dtype, const Prep16Args& a, uint32_t* chunks_out = nullptr) {
-    dim3 grid((a.C + 31) / 32, (a.R + 31) / 32), block(32, 8);
+int32_t launch_prep16(fg_ctx* ctx, int dtype, const Prep16Args& a) {
+    const bool vec = a.C % 8 == 0 && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved));      // a.out is ours: aligned, pitch % 8 == 0
+    const uint32_t w = vec ? 256 : 32;
+    dim3 grid((a.C + w - 1) / w, (a.R + 31) / 32), block(32, 8);
     if (grid.y > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "16-bit GEMM operand has too many rows");
-    if (chunks_out) *chunks_out = grid.y;
-    if (dtype == FG_DTYPE_F16) prep16_kernel<__half><<<grid, block, 0, ctx->stream>>>(a);
-    else prep16_kernel<__nv_bfloat16><<<grid, block, 0, ctx->stream>>>(a);
+    if (dtype == FG_DTYPE_F16) {
+        if (vec) prep16_kernel<__half, 8><<<grid, block, 0, ctx->stream>>>(a);
+        else prep16_kernel<__half, 1><<<grid, block, 0, ctx->stream>>>(a);
+    } else {
+        if (vec) prep16_kernel<__nv_bfloat16, 8><<<grid, block, 0, ctx->stream>>>(a);
+        else prep16_kernel<__nv_bfloat16, 1><<<grid, block, 0, ctx->stream>>>(a);
+    }
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
 
 inline uint32_t pad8(uint32_t x) { return (x + 7u) & ~7u; }
-// An operand [rows, kdim] whose contraction index is contiguous can be loaded in place when every row
-// starts on a 16-byte boundary.
-inline bool in_place16(const void* p, uint32_t kdim) { return fg_aligned16(p) && kdim % 8 == 0; }
+// A dense [rows, cols] tensor can be loaded in place when every row starts on a 16-byte boundary.
+inline bool in_place16(const void* p, uint32_t cols) { return fg_aligned16(p) && cols % 8 == 0; }
+inline uint64_t copy16_bytes(const void* p, uint32_t rows, uint32_t cols) { return in_place16(p, cols) ? 0 : (uint64_t)rows * pad8(cols) * 2 + 256; }
 
-int32_t lowp_gemm(fg_ctx* ctx, int dtype, const void* a_rows, uint32_t lda, const void* b_rows, uint32_t ldb, uint32_t M,
-                  uint32_t N, uint32_t K, void* C, const float* bias32, int act, void* preact) {
-    PlaneSet pa{nullptr, (__nv_bfloat16*)a_rows, 0, lda}, pb{nullptr, (__nv_bfloat16*)b_rows, 0, ldb};
+// x itself, or its copy with a padded pitch; *ld receives the pitch.
+int32_t loadable16(fg_ctx* ctx, int dtype, const void* x, uint32_t rows, uint32_t cols, const void** out, uint32_t* ld) {
+    *out = x;
+    *ld = cols;
+    if (in_place16(x, cols)) return FG_OK;
+    void* p;
+    int32_t s = fg_ws_alloc(ctx, (uint64_t)rows * pad8(cols) * 2, &p);
+    if (s != FG_OK) return s;
+    Prep16Args a{};
+    a.x = x; a.R = rows; a.C = cols; a.out = p; a.ld = pad8(cols);
+    *out = p;
+    *ld = a.ld;
+    return launch_prep16(ctx, dtype, a);
+}
+
+// An operand whose rows are the output's rows or columns; mn: the storage is [contraction][rows].
+PlaneSet operand16(const void* p, uint32_t ld, bool mn) {
+    PlaneSet o{};
+    o.p16 = (__nv_bfloat16*)p;
+    o.ld16 = ld;
+    o.mn = mn;
+    return o;
+}
+
+int32_t lowp_gemm(fg_ctx* ctx, int dtype, const PlaneSet& pa, const PlaneSet& pb, uint32_t M, uint32_t N, uint32_t K, void* C,
+                  const float* bias32, int act, void* preact) {
     Epilogue ep{(float*)C, bias32, (float*)preact, M, N, K, act, ctx->dev_status, nullptr, 0, 1, dtype};
     return dtype == FG_DTYPE_BF16 ? launch_tc_pair<32, 2>(ctx, pa, pb, ep) : launch_tc_pair<32, 3>(ctx, pa, pb, ep);
 }
@@ -2141,31 +2192,20 @@ int32_t fg_gemm_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, act >= FG_ACT_NONE && act <= FG_ACT_GELU, "fg_gemm_lowp: unknown activation");
     FG_REQUIRE(ctx, fg_aligned16(C) && (!preact_out || fg_aligned16(preact_out)), "fg_gemm_lowp: outputs must be 16-byte aligned");
     if (!ctx->tmap_encode) return fg_fail(ctx, FG_ERR_UNSUPPORTED_FEATURE, "fg_gemm_lowp: tensor maps unavailable");
-    const uint32_t ldk = pad8(K);
-    const bool a_direct = in_place16(A, K);
-    const uint64_t need = (uint64_t)N * ldk * 2 + (a_direct ? 0 : (uint64_t)M * ldk * 2) + (uint64_t)N * 4 + kPairPartialBytes + 2048;
+    const uint64_t need = copy16_bytes(A, M, K) + copy16_bytes(B, K, N) + (uint64_t)N * 4 + kPairPartialBytes + 2048;
     { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
     int32_t s;
-    void *bt, *ac = nullptr, *bias32 = nullptr;
-    if ((s = fg_ws_alloc(ctx, (uint64_t)N * ldk * 2, &bt)) != FG_OK) return s;
-    Prep16Args pb{};
-    pb.x = B; pb.R = K; pb.C = N; pb.t_out = bt; pb.ld_t = ldk;          // B [K,N] -> [N][K]
-    if ((s = launch_prep16(ctx, dtype, pb)) != FG_OK) return s;
-    const void* a_rows = A;
-    uint32_t lda = K;
-    if (!a_direct) {
-        if ((s = fg_ws_alloc(ctx, (uint64_t)M * ldk * 2, &ac)) != FG_OK) return s;
-        Prep16Args pa{};
-        pa.x = A; pa.R = M; pa.C = K; pa.n_out = ac; pa.ld_n = ldk;
-        if ((s = launch_prep16(ctx, dtype, pa)) != FG_OK) return s;
-        a_rows = ac;
-        lda = ldk;
-    }
+    const void *a, *b;
+    uint32_t lda, ldb;
+    if ((s = loadable16(ctx, dtype, A, M, K, &a, &lda)) != FG_OK) return s;
+    if ((s = loadable16(ctx, dtype, B, K, N, &b, &ldb)) != FG_OK) return s;
+    void* bias32 = nullptr;
     if (bias) {
         if ((s = fg_ws_alloc(ctx, (uint64_t)N * 4, &bias32)) != FG_OK) return s;
         if ((s = fg_convert_launch(ctx, bias, dtype, bias32, FG_DTYPE_F32, N)) != FG_OK) return s;
     }
-    return lowp_gemm(ctx, dtype, a_rows, lda, bt, ldk, M, N, K, C, (const float*)bias32, act, preact_out);
+    // A [M][K] has the contraction index contiguous, B [K][N] its rows (the output's columns)
+    return lowp_gemm(ctx, dtype, operand16(a, lda, false), operand16(b, ldb, true), M, N, K, C, (const float*)bias32, act, preact_out);
 }
 
 int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uint32_t K, const void* A, const void* B,
@@ -2181,65 +2221,46 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
     FG_REQUIRE(ctx, (!dA || fg_aligned16(dA)) && (!dB || fg_aligned16(dB)), "fg_gemm_bwd_lowp: outputs must be 16-byte aligned");
     if (!ctx->tmap_encode) return fg_fail(ctx, FG_ERR_UNSUPPORTED_FEATURE, "fg_gemm_bwd_lowp: tensor maps unavailable");
     const bool fuse = act != FG_ACT_NONE;
-    const uint32_t ldn = pad8(N), ldm = pad8(M);
-    const bool dz_direct = !fuse && in_place16(dY, N);       // dZ == dY, usable as the [M rows, N contiguous] operand
-    const bool b_direct = in_place16(B, N);
+    const bool dz_direct = !fuse && in_place16(dY, N);       // dZ == dY, loadable as it lies
     const uint32_t nchunk_rows = (M + 31) / 32;
     uint64_t need = 4096 + 2 * kPairPartialBytes;
-    if (dA) need += (dz_direct ? 0 : (uint64_t)M * ldn * 2) + (b_direct ? 0 : (uint64_t)K * ldn * 2);
-    if (dB) need += (uint64_t)N * ldm * 2 + (uint64_t)K * ldm * 2;
+    if ((dA || dB) && !dz_direct) need += (uint64_t)M * pad8(N) * 2 + 256;
+    if (dA) need += copy16_bytes(B, K, N);
+    if (dB) need += copy16_bytes(A, M, K);
     if (dbias) need += (uint64_t)nchunk_rows * N * 4 + (uint64_t)N * 4 + 512;
     { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
     int32_t s;
-    void *dz_n = nullptr, *dz_t = nullptr, *cs_part = nullptr;
+    void *dz = const_cast<void*>(dY), *cs_part = nullptr;
     Prep16Args pz{};
     pz.x = dY; pz.saved = fuse ? saved : nullptr; pz.act = act; pz.R = M; pz.C = N;
-    if (dA && !dz_direct) {
-        if ((s = fg_ws_alloc(ctx, (uint64_t)M * ldn * 2, &dz_n)) != FG_OK) return s;
-        pz.n_out = dz_n; pz.ld_n = ldn;
+    if ((dA || dB) && !dz_direct) {
+        if ((s = fg_ws_alloc(ctx, (uint64_t)M * pad8(N) * 2, &dz)) != FG_OK) return s;
+        pz.out = dz; pz.ld = pad8(N);
     }
-    if (dB) {
-        if ((s = fg_ws_alloc(ctx, (uint64_t)N * ldm * 2, &dz_t)) != FG_OK) return s;
-        pz.t_out = dz_t; pz.ld_t = ldm;
-    }
+    const uint32_t ldz = pz.out ? pz.ld : N;
     if (dbias) {
         if ((s = fg_ws_alloc(ctx, (uint64_t)nchunk_rows * N * 4, &cs_part)) != FG_OK) return s;
         pz.colsum_part = (float*)cs_part;
     }
-    uint32_t cs_chunks = 0;
-    if (pz.n_out || pz.t_out || pz.colsum_part) {
-        if ((s = launch_prep16(ctx, dtype, pz, &cs_chunks)) != FG_OK) return s;
-    }
+    if ((pz.out || pz.colsum_part) && (s = launch_prep16(ctx, dtype, pz)) != FG_OK) return s;
+    const void* x;
+    uint32_t ldx;
     if (dB) {
-        // dB[K,N] = A^T · dZ: contraction over M; operands A^T [K][M] and dZ^T [N][M]
-        void* at;
-        if ((s = fg_ws_alloc(ctx, (uint64_t)K * ldm * 2, &at)) != FG_OK) return s;
-        Prep16Args pa{};
-        pa.x = A; pa.R = M; pa.C = K; pa.t_out = at; pa.ld_t = ldm;
-        if ((s = launch_prep16(ctx, dtype, pa)) != FG_OK) return s;
-        if ((s = lowp_gemm(ctx, dtype, at, ldm, dz_t, ldm, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr)) != FG_OK) return s;
+        // dB[K,N] = A^T · dZ: contraction over M, the row index of both tensors
+        if ((s = loadable16(ctx, dtype, A, M, K, &x, &ldx)) != FG_OK) return s;
+        if ((s = lowp_gemm(ctx, dtype, operand16(x, ldx, true), operand16(dz, ldz, true), K, N, M, dB, nullptr, FG_ACT_NONE, nullptr)) != FG_OK)
+            return s;
     }
     if (dbias) {
         void* db32;
         if ((s = fg_ws_alloc(ctx, (uint64_t)N * 4, &db32)) != FG_OK) return s;
-        if ((s = fg_colsum_fold_launch(ctx, N, cs_chunks, (const float*)cs_part, (float*)db32)) != FG_OK) return s;
+        if ((s = fg_colsum_fold_launch(ctx, N, nchunk_rows, (const float*)cs_part, (float*)db32)) != FG_OK) return s;
         if ((s = fg_convert_launch(ctx, db32, FG_DTYPE_F32, dbias, dtype, N)) != FG_OK) return s;
     }
     if (dA) {
-        // dA[M,K] = dZ · B^T: contraction over N; dZ [M][N] and B [K][N] both have it contiguous already
-        const void* b_rows = B;
-        uint32_t ldb = N;
-        if (!b_direct) {
-            void* bc;
-            if ((s = fg_ws_alloc(ctx, (uint64_t)K * ldn * 2, &bc)) != FG_OK) return s;
-            Prep16Args pb{};
-            pb.x = B; pb.R = K; pb.C = N; pb.n_out = bc; pb.ld_n = ldn;
-            if ((s = launch_prep16(ctx, dtype, pb)) != FG_OK) return s;
-            b_rows = bc;
-            ldb = ldn;
-        }
-        const void* z_rows = dz_direct ? dY : dz_n;
-        if ((s = lowp_gemm(ctx, dtype, z_rows, dz_direct ? N : ldn, b_rows, ldb, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr)) != FG_OK)
+        // dA[M,K] = dZ · B^T: contraction over N, contiguous in both
+        if ((s = loadable16(ctx, dtype, B, K, N, &x, &ldx)) != FG_OK) return s;
+        if ((s = lowp_gemm(ctx, dtype, operand16(dz, ldz, false), operand16(x, ldx, false), M, K, N, dA, nullptr, FG_ACT_NONE, nullptr)) != FG_OK)
             return s;
     }
     return FG_OK;
