@@ -663,10 +663,15 @@ int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, cons
 int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* out) {
     const uint32_t chunk = 256;
     const uint32_t nchunks = (rows + chunk - 1) / chunk;
+    dim3 grid((cols + 31) / 32, nchunks), block(32, 8);
+    if (nchunks == 1) {      // the only partial is the sum
+        colsum_partial_kernel<<<grid, block, 0, ctx->stream>>>(rows, cols, chunk, x, out);
+        FG_LAUNCHED(ctx);
+        return FG_OK;
+    }
     void* part;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)nchunks * cols * sizeof(float), &part);
     if (s != FG_OK) return s;
-    dim3 grid((cols + 31) / 32, nchunks), block(32, 8);
     colsum_partial_kernel<<<grid, block, 0, ctx->stream>>>(rows, cols, chunk, x, (float*)part);
     FG_LAUNCHED(ctx);
     colsum_fold_kernel<<<(cols + 31) / 32, 256, 0, ctx->stream>>>(cols, nchunks, (const float*)part, out);

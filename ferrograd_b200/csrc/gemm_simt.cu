@@ -8,77 +8,92 @@
 // accepted.  Used for small shapes (the 2->16->2 MLP), as the on-device exact reference
 // for the tensor-core path, and when FG_GEMM_SIMT is requested.
 //
-// 64x64 output tile per CTA, 16x16 threads, 4x4 outputs per thread, k tiles of 16.
+// TM x TN output tile per CTA, a thread owns RPT rows x 4 columns, k tiles of 32 through two shared-memory buffers.
 #include <atomic>
 
 #include "fg_internal.cuh"
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int TK = 32;
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(uint32_t M, uint32_t N, uint32_t K,
+// The order of a sum is fixed, so K cannot be split and what counts is the time per k tile: the next tile's words are
+// requested before this one is multiplied, and a tile costs one barrier (384 x 256 x 10: 21.4 -> 6.9 us, 64 x 16 x 2:
+// 4.8 -> 2.5 us against unpipelined 64 x 64 x 16 tiles).  Which tile: see fg_gemm_simt_batched_launch.
+template <bool TA, bool TB, int TM, int TN, int RPT>
+__global__ void __launch_bounds__(TM * TN / (4 * RPT)) gemm_simt_kernel(uint32_t M, uint32_t N, uint32_t K,
                                                         const float* __restrict__ A, const float* __restrict__ B,
                                                         float* __restrict__ C, const float* __restrict__ bias, int act,
                                                         float* __restrict__ preact, uint64_t sA, uint64_t sB, uint64_t sC) {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
+    constexpr int T = TM * TN / (4 * RPT), NA = TM * TK / T, NB = TN * TK / T;
+    static_assert(RPT == 1 || RPT == 4, "a thread's rows are read as one word or one float4");
+    __shared__ __align__(16) float As[2][TK][TM + 4];
+    __shared__ __align__(16) float Bs[2][TK][TN + 4];
     // blockIdx.z is the matrix of a batch (the reference puts the batch index in the grid's z too:
     // crates/fused_gpu/src/dispatch/backend/kernel/forward.rs:159-190); the strides are in elements
     A += blockIdx.z * sA;
     B += blockIdx.z * sB;
     C += blockIdx.z * sC;
     if (preact) preact += blockIdx.z * sC;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int tx = threadIdx.x % (TN / 4), ty = threadIdx.x / (TN / 4);
     const uint32_t m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    float acc[4][4];
+    float ra[NA], rb[NB];
+    // opA[m0+m, k0+k] and opB[k0+k, n0+n], lanes along the stored tensor's contiguous index
+    auto fetch = [&](uint32_t k0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < NA; ++i) {
+            const int e = threadIdx.x + i * T, m = TA ? e % TM : e / TK, k = TA ? e / TM : e % TK;
+            const uint32_t gm = m0 + m, gk = k0 + k;
+            ra[i] = (gm < M && gk < K) ? (TA ? A[(size_t)gk * M + gm] : A[(size_t)gm * K + gk]) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int e = threadIdx.x + i * T, n = TB ? e / TK : e % TN, k = TB ? e % TK : e / TN;
+            const uint32_t gn = n0 + n, gk = k0 + k;
+            rb[i] = (gn < N && gk < K) ? (TB ? B[(size_t)gn * K + gk] : B[(size_t)gk * N + gn]) : 0.0f;
+        }
+    };
+    float acc[RPT][4];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 
-    for (uint32_t k0 = 0; k0 < K; k0 += TK) {
-        // A tile: As[k][m] = opA[m0+m, k0+k]
+    fetch(0);
+    int buf = 0;
+    for (uint32_t k0 = 0; k0 < K; k0 += TK, buf ^= 1) {
 #pragma unroll
-        for (int e = threadIdx.x; e < TM * TK; e += 256) {
-            int m, k;
-            if (TA) { m = e % TM; k = e / TM; }     // A stored [K, M]: m contiguous
-            else    { k = e % TK; m = e / TK; }     // A stored [M, K]: k contiguous
-            uint32_t gm = m0 + m, gk = k0 + k;
-            float v = 0.0f;
-            if (gm < M && gk < K) v = TA ? A[(size_t)gk * M + gm] : A[(size_t)gm * K + gk];
-            As[k][m] = v;
+        for (int i = 0; i < NA; ++i) {
+            const int e = threadIdx.x + i * T;
+            As[buf][TA ? e / TM : e % TK][TA ? e % TM : e / TK] = ra[i];
         }
-        // B tile: Bs[k][n] = opB[k0+k, n0+n]
 #pragma unroll
-        for (int e = threadIdx.x; e < TN * TK; e += 256) {
-            int n, k;
-            if (TB) { k = e % TK; n = e / TK; }     // B stored [N, K]: k contiguous
-            else    { n = e % TN; k = e / TN; }     // B stored [K, N]: n contiguous
-            uint32_t gn = n0 + n, gk = k0 + k;
-            float v = 0.0f;
-            if (gn < N && gk < K) v = TB ? B[(size_t)gn * K + gk] : B[(size_t)gk * N + gn];
-            Bs[k][n] = v;
+        for (int i = 0; i < NB; ++i) {
+            const int e = threadIdx.x + i * T;
+            Bs[buf][TB ? e % TK : e / TN][TB ? e / TK : e % TN] = rb[i];
         }
-        __syncthreads();
+        __syncthreads();        // the buffer written next was last read before the previous tile's barrier
+        if (k0 + TK < K) fetch(k0 + TK);
 #pragma unroll
         for (int k = 0; k < TK; ++k) {
-            float a[4], b[4];
+            float a[RPT];
+            if constexpr (RPT == 4) {
+                const float4 t = *reinterpret_cast<const float4*>(&As[buf][k][ty * 4]);
+                a[0] = t.x; a[1] = t.y; a[2] = t.z; a[3] = t.w;
+            } else {
+                a[0] = As[buf][k][ty];
+            }
+            const float4 t = *reinterpret_cast<const float4*>(&Bs[buf][k][tx * 4]);
+            const float b[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RPT; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t gm = m0 + ty * 4 + i;
+    for (int i = 0; i < RPT; ++i) {
+        uint32_t gm = m0 + ty * RPT + i;
         if (gm >= M) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -91,6 +106,17 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(uint32_t M, uint32_t N, 
             C[o] = fg_act_fwd(act, z);
         }
     }
+}
+
+template <int TM, int TN, int RPT>
+void launch_simt_tile(fg_ctx* ctx, bool ta, bool tb, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, const float* A, uint64_t sA,
+                      const float* B, uint64_t sB, float* C, uint64_t sC, const float* bias, int act, float* preact) {
+    constexpr int T = TM * TN / (4 * RPT);
+    const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, batch);
+    if (!ta && !tb) gemm_simt_kernel<false, false, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    else if (ta && !tb) gemm_simt_kernel<true, false, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    else if (!ta && tb) gemm_simt_kernel<false, true, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    else gemm_simt_kernel<true, true, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
 }
 
 // ---- skinny outputs (N <= 16, e.g. a 10-class output layer) ----
@@ -614,14 +640,13 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
 int32_t fg_gemm_simt_batched_launch(fg_ctx* ctx, int transA, int transB, uint32_t batch, uint32_t M, uint32_t N, uint32_t K,
                                     const float* A, uint64_t sA, const float* B, uint64_t sB, float* C, uint64_t sC,
                                     const float* bias, int act, float* preact_out) {
-    dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, batch);
-    if (grid.y > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: M too large");
+    if (M > 65535u * 64u) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: M too large");
     if (batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: more than 65535 matrices in a batch");
     if (batch == 0) return FG_OK;
-    if (!transA && !transB) gemm_simt_kernel<false, false><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact_out, sA, sB, sC);
-    else if (transA && !transB) gemm_simt_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact_out, sA, sB, sC);
-    else if (!transA && transB) gemm_simt_kernel<false, true><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact_out, sA, sB, sC);
-    else gemm_simt_kernel<true, true><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact_out, sA, sB, sC);
+    // 64 x 64 tiles (the most arithmetic per word read) once they give every SM a block; 16-row tiles before that.
+    const bool large = (uint64_t)((M + 63) / 64) * ((N + 63) / 64) * batch >= (uint64_t)ctx->sm_count || M > 65535u * 16u;
+    if (large) launch_simt_tile<64, 64, 4>(ctx, transA, transB, batch, M, N, K, A, sA, B, sB, C, sC, bias, act, preact_out);
+    else launch_simt_tile<16, 32, 1>(ctx, transA, transB, batch, M, N, K, A, sA, B, sB, C, sC, bias, act, preact_out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
