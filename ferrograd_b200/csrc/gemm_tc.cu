@@ -58,7 +58,9 @@ struct Epilogue {
     const float* mul_saved;           // optional [M,N]: C = (acc + bias) * act'(mul_saved), act = mul_act
     int mul_act;
     float* colsum_part;               // optional [ceil(M/32)][N]: column sums of the stored C per 32-row block
-    uint32_t group;                   // pair kernel: tile rows per group of the tile order (see pair_tile_origin)
+    uint32_t group;                   // tile rows per group of the tile order (see pair_tile_origin)
+    uint32_t batch;                   // conversion kernel: matrices in this launch (0 or 1: one) ...
+    uint64_t c_batch;                 // ... and the elements between two of them in C and preact
 #ifdef FG_GEMM_PROFILE
     uint32_t dbg;                     // diagnostic build: bit 0 = leave out the global stores of the epilogue
 #endif
@@ -891,18 +893,20 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
 }
 
-// Folds the K-shares of the pair kernel's tail tiles in a fixed order, then does what the pair kernel's own
-// epilogue does for a whole tile: bias, activation (or the act' factor), store, bf16 pairs, column sums.
-// 64 blocks of 256 threads per tile, one 32 x 32 sub-block each (so that a block owns whole 32-row column
-// sums); thread t handles four consecutive columns of row t / 8.
-__global__ void __launch_bounds__(256) gemm_tc_pair_fold_kernel(Epilogue ep) {
-    constexpr uint32_t TM = 2 * BM, TN = 256;
+// Folds the K-shares of tiles of TM x TN in a fixed order, then does what the kernels' own epilogues do for a whole
+// tile: bias, activation (or the act' factor), store, bf16 pairs, column sums.
+// A block of 256 threads per 32 x 32 sub-block (so that a block owns whole 32-row column sums); thread t handles four
+// consecutive columns of row t / 8.
+template <int TM, int TN>
+__global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
     __shared__ float cs_sm[8][32];
+    constexpr uint32_t kSubN = TN / 32, kSubs = (TM / 32) * kSubN;
     const uint32_t pairs_m = (ep.M + TM - 1) / TM, pairs_n = (ep.N + TN - 1) / TN;
-    const uint32_t tail = blockIdx.x >> 6, sub = blockIdx.x & 63u;
-    uint32_t m0, n0;
-    pair_tile_origin(ep.t_full + tail, pairs_m, pairs_n, TM, TN, ep.group, m0, n0);
-    const uint32_t lrow = (sub >> 3) * 32 + (threadIdx.x >> 3), lcol = (sub & 7u) * 32 + (threadIdx.x & 7u) * 4;
+    const uint32_t tail = blockIdx.x / kSubs, sub = blockIdx.x % kSubs;
+    uint32_t m0, n0, tile = ep.t_full + tail, bz = 0;
+    if (ep.batch > 1) { bz = tile / (pairs_m * pairs_n); tile -= bz * (pairs_m * pairs_n); }
+    pair_tile_origin(tile, pairs_m, pairs_n, TM, TN, ep.group, m0, n0);
+    const uint32_t lrow = (sub / kSubN) * 32 + (threadIdx.x >> 3), lcol = (sub % kSubN) * 32 + (threadIdx.x & 7u) * 4;
     const uint32_t row = m0 + lrow, col = n0 + lcol;
     const bool live = row < ep.M && col < ep.N;
     float ov[4] = {0.f, 0.f, 0.f, 0.f};
@@ -918,8 +922,8 @@ __global__ void __launch_bounds__(256) gemm_tc_pair_fold_kernel(Epilogue ep) {
 #pragma unroll
             for (int t = 0; t < 4; ++t) if (col + t < ep.N) zz[t] += ep.bias[col + t];
         }
-        const size_t off = (size_t)row * ep.N + col;
-        const bool vec_ok = (ep.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
+        const size_t off = bz * ep.c_batch + (size_t)row * ep.N + col;
+        const bool vec_ok = (ep.N % 4 == 0) && (ep.c_batch % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
                             (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0);
         if (vec_ok && col + 3 < ep.N) {
             const float4 zin = make_float4(zz[0], zz[1], zz[2], zz[3]);
@@ -955,7 +959,7 @@ __global__ void __launch_bounds__(256) gemm_tc_pair_fold_kernel(Epilogue ep) {
         for (int t = 0; t < 4; ++t) cs_sm[warp][lane * 4 + t] = ov[t];
     }
     __syncthreads();
-    const uint32_t row0 = m0 + (sub >> 3) * 32, c = n0 + (sub & 7u) * 32 + threadIdx.x;
+    const uint32_t row0 = m0 + (sub / kSubN) * 32, c = n0 + (sub % kSubN) * 32 + threadIdx.x;
     if (threadIdx.x < 32 && row0 < ep.M && c < ep.N) {
         float t = 0.0f;
 #pragma unroll
@@ -978,6 +982,7 @@ struct PlaneSet {
     uint32_t ld32, ld16;
     uint64_t plane16;      // elements between the two bf16 planes (0: rows * ld16, planes back to back)
     bool mn;               // storage is [contraction][rows] (rows contiguous): the f32 tensor itself with its pairs
+    uint64_t batch32;      // elements between two matrices of a batch (0: rows * ld32 of the storage)
 };
 
 struct SplitArgs {
@@ -1136,6 +1141,447 @@ __global__ void __launch_bounds__(256) split_vec_kernel(SplitArgs a) {
         if (tc < a.C && tr < a.R)
             store_planes4<FMT>(a.t, a.C, tc, tr,
                                make_float4(tv[cg * 4 + 0][lc], tv[cg * 4 + 1][lc], tv[cg * 4 + 2][lc], tv[cg * 4 + 3][lc]));
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// One pass over a dense [R, C] tensor of any storage type, for what cannot be read in place: a copy with a padded pitch
+// (a bulk-tensor load wants 16-byte row pitches), dZ = dY * act'(saved), and the column sums of the value over each 32 rows
+// (the bias gradient's partials).  grid.z is the matrix of a batch.
+// ------------------------------------------------------------------------------------
+struct PrepArgs {
+    const void* x;
+    const void* saved;    // non-NULL: value = x * act'(saved), rounded to the storage type
+    int act;
+    uint32_t R, C;
+    uint64_t x_batch;     // elements between two matrices of x and saved
+    void* out;            // [R][ld] per matrix, matrices R * ld apart, or NULL
+    uint32_t ld;
+    void* copy;           // optional second copy, dense, matrices R * C apart
+    float* colsum_part;   // [ceil(R/32)][C] f32 or NULL (one matrix)
+};
+
+template <typename T> __device__ __forceinline__ float lp_to_float(T v);
+template <> __device__ __forceinline__ float lp_to_float<float>(float v) { return v; }
+template <> __device__ __forceinline__ float lp_to_float<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float lp_to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <typename T> __device__ __forceinline__ T lp_from_float(float v);
+template <> __device__ __forceinline__ float lp_from_float<float>(float v) { return v; }
+template <> __device__ __forceinline__ __half lp_from_float<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 lp_from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
+// W columns per thread (16 bytes, or 1: any shape and alignment), 32 rows x 32 * W columns per block.
+template <typename T, int W>
+__global__ void __launch_bounds__(256) prep_kernel(const PrepArgs a) {
+    __shared__ float cs[8][32 * W + 1];
+    const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * W;
+    const uint32_t r0 = blockIdx.y * 32;
+    struct __align__(W * sizeof(T)) Vec { T e[W]; };
+    const T* const x = static_cast<const T*>(a.x) + blockIdx.z * a.x_batch;
+    const T* const saved = a.saved ? static_cast<const T*>(a.saved) + blockIdx.z * a.x_batch : nullptr;
+    T* const out = a.out ? static_cast<T*>(a.out) + (size_t)blockIdx.z * a.R * a.ld : nullptr;
+    T* const copy = a.copy ? static_cast<T*>(a.copy) + (size_t)blockIdx.z * a.R * a.C : nullptr;
+    float sum[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) sum[w] = 0.0f;
+    if (c < a.C) {
+        Vec v[4], sv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {       // all loads first
+            const uint32_t r = r0 + threadIdx.y + 8 * k;
+            if (r >= a.R) continue;
+            v[k] = *reinterpret_cast<const Vec*>(x + (size_t)r * a.C + c);
+            if (saved) sv[k] = *reinterpret_cast<const Vec*>(saved + (size_t)r * a.C + c);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t r = r0 + threadIdx.y + 8 * k;
+            if (r >= a.R) continue;
+            if (saved) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) v[k].e[w] = lp_from_float<T>(lp_to_float(v[k].e[w]) * fg_act_grad(a.act, lp_to_float(sv[k].e[w])));
+            }
+            if (out) *reinterpret_cast<Vec*>(out + (size_t)r * a.ld + c) = v[k];
+            if (copy) *reinterpret_cast<Vec*>(copy + (size_t)r * a.C + c) = v[k];
+#pragma unroll
+            for (int w = 0; w < W; ++w) sum[w] += lp_to_float(v[k].e[w]);
+        }
+    }
+    if (!a.colsum_part) return;
+#pragma unroll
+    for (int w = 0; w < W; ++w) cs[threadIdx.y][threadIdx.x * W + w] = sum[w];
+    __syncthreads();
+    const uint32_t t = threadIdx.y * 32 + threadIdx.x, col = blockIdx.x * (32 * W) + t;
+    if (t < 32 * W && col < a.C) {
+        float z = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) z += cs[k][t];
+        a.colsum_part[(size_t)blockIdx.y * a.C + col] = z;
+    }
+}
+
+// a.out, when given, is scratch: 16-byte aligned with a 16-byte pitch.
+int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 1) {
+    const uint32_t per16 = dtype == FG_DTYPE_F32 ? 4 : 8;
+    const bool vec = a.C % per16 == 0 && a.x_batch % per16 == 0 && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved)) &&
+                     (!a.copy || fg_aligned16(a.copy));
+    const uint32_t w = 32 * (vec ? per16 : 1);
+    dim3 grid((a.C + w - 1) / w, (a.R + 31) / 32, batch), block(32, 8);
+    if (grid.y > 65535 || batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM operand has too many rows");
+    const double es = dtype == FG_DTYPE_F32 ? 4.0 : 2.0;
+    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT,
+                                    es * batch * a.R * a.C * (1.0 + (a.saved ? 1.0 : 0.0) + (a.out ? 1.0 : 0.0) + (a.copy ? 1.0 : 0.0)));
+    if (dtype == FG_DTYPE_F32) {
+        if (vec) prep_kernel<float, 4><<<grid, block, 0, ctx->stream>>>(a);
+        else prep_kernel<float, 1><<<grid, block, 0, ctx->stream>>>(a);
+    } else if (dtype == FG_DTYPE_F16) {
+        if (vec) prep_kernel<__half, 8><<<grid, block, 0, ctx->stream>>>(a);
+        else prep_kernel<__half, 1><<<grid, block, 0, ctx->stream>>>(a);
+    } else {
+        if (vec) prep_kernel<__nv_bfloat16, 8><<<grid, block, 0, ctx->stream>>>(a);
+        else prep_kernel<__nv_bfloat16, 1><<<grid, block, 0, ctx->stream>>>(a);
+    }
+    fg_time_end(ctx, tr);
+    FG_LAUNCHED(ctx);
+    return FG_OK;
+}
+
+// ------------------------------------------------------------------------------------
+// Conversion kernel: small and middling products of f32 tensors, straight from the tensors.
+// The pair kernel needs bf16 pairs in HBM and works in 256 x 256 tiles on two SMs; a product of a
+// few such tiles leaves most SMs idle, and making the pairs of a tensor that is read once costs
+// as much as reading it twice more.  Here a CTA owns a 128 x BN tile, loads the raw f32 words of
+// both operands (half the bytes of tensor plus pairs) and eight converter warps write the bf16
+// planes of each k-block beside it in shared memory, in the layout a bulk-tensor load would have
+// given them.  A matrix index and a K-share ride in the grid, so that one launch covers a batch and
+// fills the SMs; K-shares are folded by gemm_tc_fold_kernel.
+//   warp 0 loads, warp 1 issues MMAs, warps 2..9 drain accumulators and store, warps 10..17 convert.
+// Measured (before: operand planes or pairs, then a 256 x 256 or 128-row tile each): 100 x 4096 x 4096 129 -> 43 us,
+// 16 x (384 x 512 x 320) forward and backward 1528 -> 101 us, a 384-sample layer of 256 x 256 21.7 -> 9.8 us per product.
+// Bound by the converters and shared-memory bandwidth: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB
+// into the converters, 64 KB out of them and 64 KB into the MMAs, 192 KB at 128 B per cycle.
+// ------------------------------------------------------------------------------------
+template <int BN>
+struct ConvCfg {
+    static constexpr int kA32 = BM * 32 * 4, kB32 = BN * 32 * 4;    // f32 tiles; the two bf16 planes take as much again
+    static constexpr int kStageBytes = 2 * (kA32 + kB32);
+    static constexpr int kStages = BN == 128 ? 3 : 4;
+    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+    static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
+    static_assert(kStageBytes >= 8 * 32 * 32 * 4, "the epilogue stages its blocks in the first stage");
+    static constexpr int kTmemCols = 2 * BN;
+};
+constexpr int kConvThreads = 576;
+
+// The split of a tile of ROWS rows x 32 k, eight elements per thread and step (256 threads): the words are rounded to tf32
+// in place (hi; an MMA would truncate them, which doubles what the cross terms have to carry: 1.9e-6 against 1.5e-6 of the
+// result's 2-norm), the planes are bf16(x) and bf16(x - hi).
+// K-major f32: rows of 128 bytes, 16-byte chunk c of row r at c ^ (r & 7); bf16: planes of [ROWS][64 bytes], chunk c of row
+// r at c ^ (r / 2 & 3).  MN-major f32: blocks of 32 rows, [k][128 bytes] each, 32-byte chunk j of k-row k at j ^ (k & 3);
+// bf16: blocks of 64 rows, [plane][k][128 bytes] each, 16-byte chunk c of k-row k at c ^ (k & 7).
+// Lanes are dealt so that the 128-bit accesses of eight lanes fall into different banks.
+template <int ROWS>
+__device__ __forceinline__ void convert_tile(unsigned char* t32, bool mn, uint32_t ct) {
+    unsigned char* const t16 = t32 + ROWS * 128;
+#pragma unroll
+    for (uint32_t o = ct; o < ROWS * 4; o += 256) {
+        unsigned char *s0, *s1, *h, *l;
+        bool swap = false;
+        if (!mn) {
+            const uint32_t r = o >> 2, q = o & 3u, x = r & 7u, off = r * 64 + ((q ^ (r >> 1 & 3u)) << 4);
+            s0 = t32 + r * 128 + ((2 * q ^ x) << 4);
+            s1 = t32 + r * 128 + (((2 * q + 1) ^ x) << 4);
+            h = t16 + off;
+            l = h + ROWS * 64;
+        } else {
+            const uint32_t j = o & 3u, lo = o >> 2 & 1u, k = o >> 3 & 31u, blk = o >> 8;    // 64-row block blk, its half lo
+            unsigned char* const s = t32 + (blk * 2 + lo) * 4096 + k * 128 + ((j ^ (k & 3u)) << 5);
+            swap = lo != 0;
+            s0 = s + (swap ? 16 : 0);
+            s1 = s + (swap ? 0 : 16);
+            h = t16 + blk * 8192 + k * 128 + (((lo * 4 + j) ^ (k & 7u)) << 4);
+            l = h + 4096;
+        }
+        const float4 p = *reinterpret_cast<const float4*>(s0), q4 = *reinterpret_cast<const float4*>(s1);
+        const Split4 sp = split4<1>(p), sq = split4<1>(q4);
+        *reinterpret_cast<float4*>(s0) = sp.hi;
+        *reinterpret_cast<float4*>(s1) = sq.hi;
+        const uint2 h0 = pack_bf16x4(swap ? q4 : p), h1 = pack_bf16x4(swap ? p : q4);
+        const uint2 l0 = pack_bf16x4(swap ? sq.lo : sp.lo), l1 = pack_bf16x4(swap ? sp.lo : sq.lo);
+        *reinterpret_cast<uint4*>(h) = make_uint4(h0.x, h0.y, h1.x, h1.y);
+        *reinterpret_cast<uint4*>(l) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+    }
+}
+
+// Descriptors of one converted operand tile: the f32 words, the two planes, and how far one MMA's k advances them.
+struct ConvOperand {
+    uint64_t f, h, l;
+    uint32_t adv32, adv16;
+};
+template <int ROWS>
+__device__ __forceinline__ ConvOperand conv_operand(uint32_t t32, bool mn) {
+    const uint32_t t16 = t32 + ROWS * 128;
+    ConvOperand o;
+    if (!mn) {
+        o.f = make_desc_kmajor<128>(t32);
+        o.h = make_desc_kmajor<64>(t16);
+        o.l = make_desc_kmajor<64>(t16 + ROWS * 64);
+        o.adv32 = 2; o.adv16 = 2;
+    } else {
+        o.f = make_desc_mnmajor(t32, 4096, 512, 1);
+        o.h = make_desc_mnmajor(t16, 8192, 1024, 2);
+        o.l = make_desc_mnmajor(t16 + 4096, 8192, 1024, 2);
+        o.adv32 = 64; o.adv16 = 128;
+    }
+    return o;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kConvThreads, 1)
+gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epilogue ep) {
+    using Cfg = ConvCfg<BN>;
+    constexpr int S = Cfg::kStages, BK = 32, CPT = BN / 2;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    unsigned char* const base_ptr = smem_raw + (base - raw);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base_ptr + S * Cfg::kStageBytes);
+    const uint32_t bar0 = base + S * Cfg::kStageBytes;
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };            // the f32 words have landed
+    auto conv_bar = [&](int s) { return bar0 + 8u * (S + s); };      // the bf16 planes are written
+    auto empty_bar = [&](int s) { return bar0 + 8u * (2 * S + s); };
+    auto acc_full_bar = [&](int b) { return bar0 + 8u * (3 * S + b); };
+    auto acc_empty_bar = [&](int b) { return bar0 + 8u * (3 * S + 2 + b); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 3 * S + 4);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t tiles_m = (ep.M + BM - 1) / BM, tiles_n = (ep.N + BN - 1) / BN, bz = blockIdx.z;
+    uint32_t m0, n0;
+    pair_tile_origin(blockIdx.x, tiles_m, tiles_n, BM, BN, ep.group, m0, n0);
+    const uint32_t nkb_all = (ep.K + BK - 1) / BK;
+    const uint32_t kb0 = (uint32_t)((uint64_t)blockIdx.y * nkb_all / ep.split);
+    const uint32_t nkb = (uint32_t)((uint64_t)(blockIdx.y + 1) * nkb_all / ep.split) - kb0;     // the host keeps split <= nkb_all
+    constexpr uint32_t kChunkKB = kChunkK / BK;
+    const uint32_t nchunks = (nkb + kChunkKB - 1) / kChunkKB;
+
+    __shared__ int s_abort;      // see gemm_tc_kernel
+    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(ep.dev_status);
+    __syncthreads();
+    if (s_abort != 0) return;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(conv_bar(s), 8); mbar_init(empty_bar(s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full_bar(b), 1); mbar_init(acc_empty_bar(b), 8); }
+        fence_mbar_init();
+        prefetch_tmap(&tmA);
+        prefetch_tmap(&tmB);
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), Cfg::kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool a_mn = ep.a_mn != 0, b_mn = ep.b_mn != 0;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // ---- producer ----
+            for (uint32_t i = 0; i < nkb; ++i) {
+                const int s = i % S;
+                if (!mbar_wait_bounded(empty_bar(s), ((i / S) & 1u) ^ 1u, kWaitCycles)) {
+                    atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
+                    break;
+                }
+                mbar_expect_tx(full_bar(s), Cfg::kA32 + Cfg::kB32);
+                const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + 2 * Cfg::kA32;
+                const int k = (int)((kb0 + i) * BK);
+                if (!a_mn) tma_load_3d(sa, &tmA, full_bar(s), k, (int)m0, (int)bz);
+                else
+#pragma unroll
+                    for (int j = 0; j < BM / 32; ++j) tma_load_3d(sa + j * 4096, &tmA, full_bar(s), (int)(m0 + 32 * j), k, (int)bz);
+                if (!b_mn) tma_load_3d(sb, &tmB, full_bar(s), k, (int)n0, (int)bz);
+                else
+#pragma unroll
+                    for (int j = 0; j < BN / 32; ++j) tma_load_3d(sb + j * 4096, &tmB, full_bar(s), (int)(n0 + 32 * j), k, (int)bz);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // ---- MMA issuer ----
+            const uint32_t mnbits = (a_mn ? kIdescAMnMajor : 0u) | (b_mn ? kIdescBMnMajor : 0u);
+            const uint32_t idesc32 = make_idesc(2u /*tf32*/, BM, BN) | mnbits, idesc16 = make_idesc(1u /*bf16*/, BM, BN) | mnbits;
+            bool ok = true;
+            for (uint32_t c = 0; c < nchunks && ok; ++c) {
+                const uint32_t buf = c & 1u;
+                if (!mbar_wait_bounded(acc_empty_bar(buf), ((c >> 1) & 1u) ^ 1u, kWaitCycles)) {
+                    atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + buf * BN;
+                const uint32_t end = min(nkb, (c + 1) * kChunkKB);
+                for (uint32_t i = c * kChunkKB; i < end; ++i) {
+                    const int s = i % S;
+                    if (!mbar_wait_bounded(conv_bar(s), (i / S) & 1u, kWaitCycles)) {
+                        atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sa = base + s * Cfg::kStageBytes;
+                    const ConvOperand a = conv_operand<BM>(sa, a_mn), b = conv_operand<BN>(sa + 2 * Cfg::kA32, b_mn);
+                    const uint32_t first = (i == c * kChunkKB) ? 0u : 1u;      // a chunk starts from zero
+#pragma unroll
+                    for (int kk = 0; kk < BK / 16; ++kk) {
+                        mma_f16(d_tmem, a.l + (uint64_t)(kk * a.adv16), b.h + (uint64_t)(kk * b.adv16), idesc16, first | (uint32_t)kk);
+                        mma_f16(d_tmem, a.h + (uint64_t)(kk * a.adv16), b.l + (uint64_t)(kk * b.adv16), idesc16, 1u);
+                    }
+#pragma unroll
+                    for (int kk = 0; kk < BK / UK; ++kk)
+                        mma_tf32(d_tmem, a.f + (uint64_t)(kk * a.adv32), b.f + (uint64_t)(kk * b.adv32), idesc32, 1u);
+                    mma_commit(empty_bar(s));
+                }
+                if (ok) mma_commit(acc_full_bar(buf));
+            }
+        }
+    } else if (warp >= 10) {
+        // ---- converters ----
+        const uint32_t ct = threadIdx.x - 320;
+        for (uint32_t i = 0; i < nkb; ++i) {
+            const int s = i % S;
+            const bool got = mbar_wait_bounded(full_bar(s), (i / S) & 1u, kWaitCycles);
+            if (!__all_sync(0xffffffffu, got)) {
+                if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
+                break;
+            }
+            unsigned char* const sa = base_ptr + s * Cfg::kStageBytes;
+            convert_tile<BM>(sa, a_mn, ct);
+            convert_tile<BN>(sa + 2 * Cfg::kA32, b_mn, ct);
+            fence_proxy_async();        // the planes are read by the tensor core
+            __syncwarp();
+            if (lane == 0) mbar_arrive(conv_bar(s));
+        }
+    } else {
+        // ---- accumulate + epilogue: warps 2..9; warp w may touch TMEM lanes 32*(w%4) .. +31 ----
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        float sum[CPT];
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) sum[j] = 0.0f;
+        bool ok = true;
+        for (uint32_t c = 0; c < nchunks; ++c) {
+            const uint32_t buf = c & 1u;
+            bool got = mbar_wait_bounded(acc_full_bar(buf), (c >> 1) & 1u, kWaitCycles + kWaitCycles / 2);
+            got = __all_sync(0xffffffffu, got);
+            if (!got) {
+                if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_EPI_WAIT);
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * CPT;
+#pragma unroll
+            for (int g = 0; g < CPT / 32; ++g) {
+                uint32_t r[32];
+                tmem_ld_32x32(t0 + g * 32, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sum[g * 32 + j] += __uint_as_float(r[j]);
+            }
+            tc_fence_before();
+            if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+        }
+        if (ok) {
+            // Every load and MMA of this CTA has finished (the last chunk is complete), so the first stage is free: each
+            // warp passes 32 x 32 blocks through its 4 KB of it and writes 4 rows x 128 bytes per instruction.
+            // A K-share goes out raw into its slot.
+            const bool part = ep.split > 1;
+            const uint32_t slot = (bz * gridDim.x + blockIdx.x) * ep.split + blockIdx.y;
+            float* const pout = part ? ep.partial + (size_t)slot * (BM * BN) : nullptr;
+            const size_t cb = (size_t)bz * ep.c_batch;
+            const bool vec = (ep.N % 4 == 0) && (ep.c_batch % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
+                             (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0) &&
+                             (!ep.mul_saved || (reinterpret_cast<uintptr_t>(ep.mul_saved) & 15u) == 0);
+            float4* const tb4 = reinterpret_cast<float4*>(base_ptr) + (warp - 2) * (32 * 8);
+            const uint32_t rsub = lane >> 3, cc = lane & 7;
+            const uint32_t row0 = m0 + q * 32;
+#pragma unroll
+            for (int g = 0; g < CPT / 32; ++g) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    tb4[lane * 8 + (c ^ (lane & 7))] = make_float4(sum[g * 32 + 4 * c], sum[g * 32 + 4 * c + 1],
+                                                                   sum[g * 32 + 4 * c + 2], sum[g * 32 + 4 * c + 3]);
+                __syncwarp();
+                const uint32_t lcol = half * CPT + g * 32 + cc * 4, col = n0 + lcol;
+                if (part) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t lr = i * 4 + rsub;
+                        *reinterpret_cast<float4*>(pout + (size_t)(q * 32 + lr) * BN + lcol) = tb4[lr * 8 + (cc ^ (lr & 7))];
+                    }
+                    __syncwarp();
+                    continue;
+                }
+                float4 bz4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (ep.bias) {
+                    if (col < ep.N) bz4.x = ep.bias[col];
+                    if (col + 1 < ep.N) bz4.y = ep.bias[col + 1];
+                    if (col + 2 < ep.N) bz4.z = ep.bias[col + 2];
+                    if (col + 3 < ep.N) bz4.w = ep.bias[col + 3];
+                }
+                float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
+                const bool fast = vec && col + 3 < ep.N;
+#pragma unroll 4
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t lr = i * 4 + rsub, row = row0 + lr;
+                    float4 z = tb4[lr * 8 + (cc ^ (lr & 7))];
+                    z.x += bz4.x; z.y += bz4.y; z.z += bz4.z; z.w += bz4.w;
+                    if (row < ep.M && col < ep.N) {
+                        const size_t off = cb + (size_t)row * ep.N + col;
+                        float4 o;
+                        if (fast) {
+                            if (ep.mul_saved) {
+                                const float4 sv = __ldg(reinterpret_cast<const float4*>(ep.mul_saved + off));
+                                o = make_float4(z.x * fg_act_grad_sel(ep.mul_act, sv.x), z.y * fg_act_grad_sel(ep.mul_act, sv.y),
+                                                z.z * fg_act_grad_sel(ep.mul_act, sv.z), z.w * fg_act_grad_sel(ep.mul_act, sv.w));
+                            } else if (ep.act != FG_ACT_NONE) {
+                                o = make_float4(fg_act_fwd_sel(ep.act, z.x), fg_act_fwd_sel(ep.act, z.y), fg_act_fwd_sel(ep.act, z.z),
+                                                fg_act_fwd_sel(ep.act, z.w));
+                            } else o = z;
+                            if (ep.preact) *reinterpret_cast<float4*>(ep.preact + off) = z;
+                            *reinterpret_cast<float4*>(ep.C + off) = o;
+                            if (ep.c_pairs) fg_store_pairs4(ep.c_pairs, ep.c_pairs_stride, off, o);
+                        } else {
+                            o = epi_store_edge(z, off, col, ep.N, (char*)ep.C, (char*)ep.preact, ep.c_pairs, ep.c_pairs_stride, ep.mul_saved,
+                                               ep.mul_act, ep.act, FG_DTYPE_F32);
+                        }
+                        cs.x += o.x; cs.y += o.y; cs.z += o.z; cs.w += o.w;
+                    }
+                }
+                if (ep.colsum_part) {
+                    cs.x += __shfl_xor_sync(0xffffffffu, cs.x, 8); cs.x += __shfl_xor_sync(0xffffffffu, cs.x, 16);
+                    cs.y += __shfl_xor_sync(0xffffffffu, cs.y, 8); cs.y += __shfl_xor_sync(0xffffffffu, cs.y, 16);
+                    cs.z += __shfl_xor_sync(0xffffffffu, cs.z, 8); cs.z += __shfl_xor_sync(0xffffffffu, cs.z, 16);
+                    cs.w += __shfl_xor_sync(0xffffffffu, cs.w, 8); cs.w += __shfl_xor_sync(0xffffffffu, cs.w, 16);
+                    if (lane < 8 && row0 < ep.M) {
+                        float* d = ep.colsum_part + (size_t)(row0 >> 5) * ep.N + col;
+                        if (col < ep.N) d[0] = cs.x;
+                        if (col + 1 < ep.N) d[1] = cs.y;
+                        if (col + 2 < ep.N) d[2] = cs.z;
+                        if (col + 3 < ep.N) d[3] = cs.w;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
 }
 
@@ -1386,12 +1832,128 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     gemm_tc_pair_kernel<BK, FMT><<<grid, kPairThreads, Cfg::kSmemBytes, ctx->stream>>>(tmA, tmB, tmA16, tmB16, ep);
     FG_LAUNCHED(ctx);
     if (ep.split > 1) {
-        gemm_tc_pair_fold_kernel<<<(unsigned)((ntiles - ep.t_full) * 64), 256, 0, ctx->stream>>>(ep);
+        gemm_tc_fold_kernel<2 * BM, 256><<<(unsigned)((ntiles - ep.t_full) * 64), 256, 0, ctx->stream>>>(ep);
         FG_LAUNCHED(ctx);
     }
     fg_time_end(ctx, tr);
     return FG_OK;
 }
+
+// ---- conversion kernel, host side ----
+struct ConvPlan {
+    uint32_t bn, split;
+    double cycles;       // estimate; 0: cannot run
+};
+// Estimated SM cycles of the kernels for [M,K] x [K,N] (times `batch`), from their per-k-block costs and fixed overheads.
+ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32_t batch) {
+    ConvPlan best{128, 1, 0.0};
+    const uint64_t sms = (uint64_t)ctx->sm_count, nkb = (K + 31) / 32;
+    for (uint32_t bn = 128; bn >= 64; bn -= 64) {
+        const uint64_t tiles = (uint64_t)((M + BM - 1) / BM) * ((N + bn - 1) / bn) * batch;
+        for (uint64_t split = 1; split <= 16 && (split == 1 || (split * 4 <= nkb && tiles * split <= 2 * sms)); ++split) {
+            const uint64_t waves = (tiles * split + sms - 1) / sms, kb = (nkb + split - 1) / split;
+            double c = (double)waves * ((double)kb * (bn == 128 ? 1300.0 : 950.0) + 6000.0);
+            if (split > 1) c += 5000.0 + (double)(tiles * split) * BM * bn * 4.0 / 2000.0;      // the fold's launch and its reads
+            if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, (uint32_t)split, c};
+        }
+    }
+    return best;
+}
+uint64_t conv_partial_bytes(const ConvPlan& p, uint32_t M, uint32_t N, uint32_t batch) {
+    if (p.split <= 1) return 0;
+    return (uint64_t)((M + BM - 1) / BM) * ((N + p.bn - 1) / p.bn) * batch * p.split * BM * p.bn * 4 + 256;
+}
+// The pair kernel for one matrix: 256 x 256 tiles on SM pairs, plus the passes that make the pairs of `prep` elements.
+double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double prep_elems, int prep_launches) {
+    const uint64_t pairs = (uint64_t)ctx->sm_count / 2, tiles = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
+    const double tile = (double)((K + 31) / 32) * 1150.0, whole = (double)(tiles / pairs) * tile;
+    const uint64_t rem = tiles % pairs;
+    double tail = rem ? tile : 0.0;
+    const uint64_t nchunks = (K + kChunkK - 1) / kChunkK;
+    uint64_t split = rem ? pairs / rem : 1;
+    if (split > nchunks / 2) split = nchunks / 2;
+    if (split > 4) split = 4;
+    if (split >= 2 && ctx->opt_split_k) tail = tail / (double)split + 8000.0;
+    return whole + tail + 9000.0 + prep_elems * 8.0 / 2500.0 + 4000.0 * prep_launches;
+}
+inline bool conv_allowed(const fg_ctx* ctx) { return ctx->opt_pairs && ctx->opt_tile_pair < 0 && ctx->tmap_encode; }
+
+template <int BN>
+int32_t launch_conv_bn(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, Epilogue ep, uint32_t batch) {
+    using Cfg = ConvCfg<BN>;
+    CUtensorMap tm[2];
+    int32_t s;
+    const PlaneSet* ops[2] = {&a, &b};
+    const uint32_t rows[2] = {ep.M, ep.N}, tile[2] = {(uint32_t)BM, (uint32_t)BN};
+    for (int i = 0; i < 2; ++i) {
+        const PlaneSet& o = *ops[i];
+        const uint64_t apart = (o.batch32 ? o.batch32 : (uint64_t)(o.mn ? ep.K : rows[i]) * o.ld32) * 4;
+        if (!o.mn) s = make_tmap3(ctx, &tm[i], o.p32, 0, ep.K, rows[i], batch, (uint64_t)o.ld32 * 4, apart, 32, tile[i], 1);
+        else s = make_tmap3(ctx, &tm[i], o.p32, 0, rows[i], ep.K, batch, (uint64_t)o.ld32 * 4, apart, 32, 32, 1, true);
+        if (s != FG_OK) return s;
+    }
+    ep.a_mn = a.mn ? 1u : 0u;
+    ep.b_mn = b.mn ? 1u : 0u;
+    static std::atomic<uint64_t> attr_done{0};       // one bit per device
+    if (!(attr_done.load(std::memory_order_acquire) >> (ctx->device & 63) & 1ull)) {
+        FG_CUDA(ctx, FG_ERR_INTERNAL,
+                cudaFuncSetAttribute(gemm_tc_conv_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+        attr_done.fetch_or(1ull << (ctx->device & 63), std::memory_order_release);
+    }
+    const uint64_t tiles_m = (ep.M + BM - 1) / BM, tiles = tiles_m * ((ep.N + BN - 1) / BN);
+    if (tiles > (1ull << 30) || batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM: too many tiles");
+    ep.group = (uint32_t)tiles_m;         // down the columns of tiles: the CTAs at work share a few tile columns of B
+    ep.batch = batch;
+    ep.t_full = 0;
+    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, 2.0 * batch * ep.M * ep.N * ep.K);
+    gemm_tc_conv_kernel<BN><<<dim3((unsigned)tiles, ep.split, batch), kConvThreads, Cfg::kSmemBytes, ctx->stream>>>(tm[0], tm[1], ep);
+    FG_LAUNCHED(ctx);
+    if (ep.split > 1) {
+        gemm_tc_fold_kernel<BM, BN><<<(unsigned)(tiles * batch * (BM / 32) * (BN / 32)), 256, 0, ctx->stream>>>(ep);
+        FG_LAUNCHED(ctx);
+    }
+    fg_time_end(ctx, tr);
+    return FG_OK;
+}
+// The caller has reserved conv_partial_bytes().
+int32_t launch_conv(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilogue& ep_in, const ConvPlan& p, uint32_t batch) {
+    Epilogue ep = ep_in;
+    ep.split = p.split;
+    ep.partial = nullptr;
+    if (p.split > 1) {
+        void* part;
+        int32_t s = fg_ws_alloc(ctx, conv_partial_bytes(p, ep.M, ep.N, batch), &part);
+        if (s != FG_OK) return s;
+        ep.partial = (float*)part;
+    }
+    return p.bn == 128 ? launch_conv_bn<128>(ctx, a, b, ep, batch) : launch_conv_bn<64>(ctx, a, b, ep, batch);
+}
+
+// A dense [R, C] f32 tensor (`batch` of them, x_batch apart) can be loaded as it lies when rows and matrices start on
+// 16-byte boundaries; otherwise from a padded copy.
+inline bool in_place32(const float* x, uint32_t C, uint32_t batch, uint64_t x_batch) {
+    return fg_aligned16(x) && C % 4 == 0 && (batch == 1 || x_batch % 4 == 0);
+}
+inline uint64_t copy32_bytes(const float* x, uint32_t R, uint32_t C, uint32_t batch, uint64_t x_batch) {
+    return in_place32(x, C, batch, x_batch) ? 0 : (uint64_t)batch * R * round4(C) * 4 + 256;
+}
+int32_t loadable32(fg_ctx* ctx, const float* x, uint32_t R, uint32_t C, uint32_t batch, uint64_t x_batch, PlaneSet* o) {
+    *o = PlaneSet{};
+    o->p32 = const_cast<float*>(x);
+    o->ld32 = C;
+    o->batch32 = x_batch;
+    if (in_place32(x, C, batch, x_batch)) return FG_OK;
+    void* p;
+    int32_t s = fg_ws_alloc(ctx, (uint64_t)batch * R * round4(C) * 4, &p);
+    if (s != FG_OK) return s;
+    PrepArgs a{};
+    a.x = x; a.R = R; a.C = C; a.x_batch = x_batch; a.out = p; a.ld = round4(C);
+    o->p32 = (float*)p;
+    o->ld32 = a.ld;
+    o->batch32 = (uint64_t)R * a.ld;
+    return launch_prep(ctx, FG_DTYPE_F32, a, batch);
+}
+inline PlaneSet as_operand(PlaneSet o, bool mn) { o.mn = mn; return o; }
 
 // C[M,N] = act(Aop·Bopᵀ + bias) where the A operand's planes have M rows and the B operand's N rows.
 int32_t tc_gemm(fg_ctx* ctx, int fmt, const PlaneSet& a, const PlaneSet& b, uint32_t M, uint32_t N, uint32_t K, float* C,
@@ -1531,6 +2093,27 @@ int32_t paired_gemm(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, uint32_t 
     return launch_tc_pair<32, 1>(ctx, a, b, ep);
 }
 
+// How one tensor-core product of f32 tensors [M,K] x [K,N] runs: operand planes written by a pre-pass (any shape), the pair
+// kernel on tensors with their pairs, or the conversion kernel on the tensors alone.
+enum { kRoutePlanes = 0, kRoutePair = 1, kRouteConv = 2 };
+struct Route {
+    int kind;
+    ConvPlan conv;
+};
+// pair_ok: the pair kernel can read the operands as they lie.  missing / missing_n: elements and tensors whose pairs would
+// have to be made for it.  copied / copied_n: the same for the padded copies the conversion kernel would need.
+Route pick_route(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool pair_ok, double missing, int missing_n, double copied, int copied_n) {
+    Route r{pair_ok ? (int)kRoutePair : (int)kRoutePlanes, ConvPlan{}};
+    if (!conv_allowed(ctx)) return r;
+    r.conv = plan_conv(ctx, M, N, K, 1);
+    const double conv = r.conv.cycles + copied * 8.0 / 2500.0 + 4000.0 * copied_n;
+    // planes: both operands read and written twice over, transposed on the way, then 256 x 256 or 128-row tiles
+    const double other = pair_ok ? pair_cycles(ctx, M, N, K, missing, missing_n)
+                       : M > (uint32_t)BM && N > 128 ? pair_cycles(ctx, M, N, K, 2.0 * ((double)M * K + (double)N * K), 2) : 1e30;
+    if (conv <= other) r.kind = kRouteConv;
+    return r;
+}
+
 // Which path a request takes: 0 = SIMT, otherwise the plane format + 1.
 int pick_path(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K) {
     if (mode == FG_GEMM_SIMT) return 0;
@@ -1571,9 +2154,27 @@ int32_t gemm_fwd_core(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
         return s != FG_OK ? s : pairs_after();
     }
     const int fmt = path - 1;
-    const uint32_t pitch_a = transA ? M : K, pitch_b = transB ? K : N;
+    const uint32_t pitch_a = transA ? M : K, pitch_b = transB ? K : N, rows_a = transA ? K : M, rows_b = transB ? N : K;
     const bool aligned = fg_aligned16(A.x) && fg_aligned16(B.x) && fg_aligned16(C) && (!preact_out || fg_aligned16(preact_out));
-    if (fmt == 1 && aligned && paired_shape_ok(ctx, M, N, K, pitch_a, pitch_b) && N % 4 == 0) {
+    const bool pair_ok = fmt == 1 && aligned && paired_shape_ok(ctx, M, N, K, pitch_a, pitch_b) && N % 4 == 0;
+    if (fmt == 1) {
+        const uint64_t ca = copy32_bytes(A.x, rows_a, pitch_a, 1, 0), cb = copy32_bytes(B.x, rows_b, pitch_b, 1, 0);
+        const Route r = pick_route(ctx, M, N, K, pair_ok, (A.pairs ? 0.0 : (double)M * K) + (B.pairs ? 0.0 : (double)K * N), !A.pairs + !B.pairs,
+                                   (ca ? (double)M * K : 0.0) + (cb ? (double)K * N : 0.0), (ca != 0) + (cb != 0));
+        if (r.kind == kRouteConv) {
+            int32_t s = fg_ws_ensure(ctx, ca + cb + conv_partial_bytes(r.conv, M, N, 1) + 1024);
+            if (s != FG_OK) return s;
+            PlaneSet pa, pb;
+            if ((s = loadable32(ctx, A.x, rows_a, pitch_a, 1, 0, &pa)) != FG_OK) return s;
+            if ((s = loadable32(ctx, B.x, rows_b, pitch_b, 1, 0, &pb)) != FG_OK) return s;
+            Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
+            ep.c_pairs = c_pairs;
+            ep.c_pairs_stride = c_stride;
+            // A operand: rows = M, B operand: rows = N; the contraction runs along the columns of [M,K] and of [N,K]
+            return launch_conv(ctx, as_operand(pa, transA != 0), as_operand(pb, transB == 0), ep, r.conv, 1);
+        }
+    }
+    if (pair_ok) {
         // The tensors themselves are the operands; pairs the caller does not keep are made here (8 bytes
         // of traffic per element, no transposition).
         const uint64_t mk = (uint64_t)M * K, kn = (uint64_t)K * N;
@@ -1782,22 +2383,98 @@ uint64_t bwd_planes_need(uint32_t M, uint32_t N, uint32_t K) {
     return need;
 }
 
-// Both products of a backward step straight from the f32 tensors and their pairs?
-bool bwd_paired_ok(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool want_dA, bool want_dB) {
-    if (N % 8 != 0 || K % 8 != 0) return false;
-    if (want_dB && !paired_shape_ok(ctx, K, N, M, K, N)) return false;     // dB [K,N], contraction over M
-    if (want_dA && !paired_shape_ok(ctx, M, K, N, N, N)) return false;     // dA [M,K], contraction over N
-    return want_dA || want_dB;
-}
-
 // Backward of Y = A·B given dZ = dL/dY (already multiplied by this layer's act'), on f32 tensors with pairs:
 //   dB [K,N] = Aᵀ·dZ, then the exchange (if asked for), then
 //   dA [M,K] = (dZ·Bᵀ) * act'(o.mul_saved) with its pairs (o.pairs) and its column sums (dbias_prev [K]) --
 //   i.e. the dZ of the layer below and that layer's bias gradient come out of the dA epilogue.
 // Pairs that are not supplied are made in the scratch arena.  The caller has reserved bwd_paired_need().
 uint64_t bwd_paired_need(uint32_t M, uint32_t N, uint32_t K) {
+    // (the conversion kernel's K-shares take less than kPairPartialBytes, its padded copies less than the planes)
     return 4ull * ((uint64_t)M * K + (uint64_t)K * N + (uint64_t)M * N) + (uint64_t)((M + 31) / 32) * K * 4 +
            2 * kPairPartialBytes + 4096 + fg_gemm_skinny_scratch_bytes(M, N, K) + bwd_planes_need(M, N, K);
+}
+
+struct BwdRoutes {
+    Route dB, dA;
+    bool planes;      // a wanted product takes the planes route: both do
+};
+BwdRoutes pick_bwd_routes(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, const float* dB,
+                          const float* dA, const float* mul_saved) {
+    BwdRoutes r{};
+    const double mk = (double)M * K, kn = (double)K * N, mn = (double)M * N;
+    const bool tc = pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 2, n8 = N % 8 == 0 && K % 8 == 0;
+    const bool cz = !in_place32(dZ.x, N, 1, 0);
+    // a pair product of any wanted gradient that cannot run sends both to the planes, as long as the other cannot be converted
+    if (dB) {
+        const bool pair = n8 && fg_aligned16(A.x) && fg_aligned16(dB) && fg_aligned16(dZ.x) && paired_shape_ok(ctx, K, N, M, K, N);
+        const bool ca = !in_place32(A.x, K, 1, 0);
+        r.dB = (tc || pair) ? pick_route(ctx, K, N, M, pair, (A.pairs ? 0.0 : mk) + (dZ.pairs ? 0.0 : mn), !A.pairs + !dZ.pairs,
+                                         (ca ? mk : 0.0) + (cz ? mn : 0.0), ca + cz) : Route{kRoutePlanes, ConvPlan{}};
+        r.planes |= r.dB.kind == kRoutePlanes;
+    }
+    if (dA) {
+        const bool pair = n8 && fg_aligned16(B.x) && fg_aligned16(dA) && fg_aligned16(dZ.x) && (!mul_saved || fg_aligned16(mul_saved)) &&
+                          paired_shape_ok(ctx, M, K, N, N, N);
+        const bool cb = !in_place32(B.x, N, 1, 0);
+        r.dA = (tc || pair) ? pick_route(ctx, M, K, N, pair, (B.pairs ? 0.0 : kn) + (dZ.pairs ? 0.0 : mn), !B.pairs + !dZ.pairs,
+                                         (cb ? kn : 0.0) + (cz ? mn : 0.0), cb + cz) : Route{kRoutePlanes, ConvPlan{}};
+        r.planes |= r.dA.kind == kRoutePlanes;
+    }
+    return r;
+}
+
+// The two products of a backward step by their routes; dZ has row pitch ldz (N, or padded for the conversion kernel).
+int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, uint32_t ldz,
+                          const BwdRoutes& rt, float* dB, float* dA, const PairedOut& o, float* exch_buf, uint64_t exch_count) {
+    int32_t s;
+    const uint64_t mk = (uint64_t)M * K, kn = (uint64_t)K * N, mn = (uint64_t)M * N;
+    const bool pair_b = dB && rt.dB.kind == kRoutePair, pair_a = dA && rt.dA.kind == kRoutePair;
+    auto make_pairs = [&](PairedArg& t, uint64_t n) -> int32_t {
+        if (t.pairs) return FG_OK;
+        void* q;
+        int32_t e = fg_ws_alloc(ctx, n * 4, &q);
+        if (e != FG_OK || (e = launch_pairs(ctx, t.x, n, (__nv_bfloat16*)q, n)) != FG_OK) return e;
+        t.pairs = q; t.stride = n;
+        return FG_OK;
+    };
+    PlaneSet z32;
+    if ((pair_a || pair_b) && (s = make_pairs(dZ, mn)) != FG_OK) return s;
+    if ((dB && !pair_b) || (dA && !pair_a)) {
+        if (ldz == N && (s = loadable32(ctx, dZ.x, M, N, 1, 0, &z32)) != FG_OK) return s;
+        if (ldz != N) { z32 = PlaneSet{}; z32.p32 = const_cast<float*>(dZ.x); z32.ld32 = ldz; }
+    }
+    if (pair_b) {
+        if ((s = make_pairs(A, mk)) != FG_OK) return s;
+        // operands Aᵀ (rows = K) and dZᵀ (rows = N), both read from [M, .] storage: contraction over the rows
+        const PlaneSet pa = paired_operand(A.x, A.pairs, A.stride, K, false);
+        const PlaneSet pz = paired_operand(dZ.x, dZ.pairs, dZ.stride, N, false);
+        if ((s = paired_gemm(ctx, pa, pz, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr, PairedOut{nullptr, 0, nullptr, 0, nullptr})) != FG_OK)
+            return s;
+    } else if (dB) {
+        PlaneSet a32;
+        if ((s = loadable32(ctx, A.x, M, K, 1, 0, &a32)) != FG_OK) return s;
+        const Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
+        if ((s = launch_conv(ctx, as_operand(a32, true), as_operand(z32, true), ep, rt.dB.conv, 1)) != FG_OK) return s;
+    }
+    if (exch_buf && (s = fg_allreduce_sum_f32(ctx, exch_buf, exch_count)) != FG_OK) return s;
+    if (pair_a) {
+        if ((s = make_pairs(B, kn)) != FG_OK) return s;
+        // operands dZ (rows = M) and B (rows = K), both with the contraction index N contiguous
+        const PlaneSet pz = paired_operand(dZ.x, dZ.pairs, dZ.stride, N, true);
+        const PlaneSet pb = paired_operand(B.x, B.pairs, B.stride, N, true);
+        if ((s = paired_gemm(ctx, pz, pb, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr, o)) != FG_OK) return s;
+    } else if (dA) {
+        PlaneSet b32;
+        if ((s = loadable32(ctx, B.x, K, N, 1, 0, &b32)) != FG_OK) return s;
+        Epilogue ep{dA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
+        ep.c_pairs = o.pairs;
+        ep.c_pairs_stride = o.stride;
+        ep.mul_saved = o.mul_saved;
+        ep.mul_act = o.mul_act;
+        ep.colsum_part = o.colsum_part;
+        if ((s = launch_conv(ctx, as_operand(z32, false), as_operand(b32, false), ep, rt.dA.conv, 1)) != FG_OK) return s;
+    }
+    return FG_OK;
 }
 
 int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, float* dB,
@@ -1822,43 +2499,12 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         }
         return FG_OK;
     }
-    const bool aligned = (!dB || (fg_aligned16(A.x) && fg_aligned16(dB))) && (!dA || (fg_aligned16(B.x) && fg_aligned16(dA))) &&
-                         fg_aligned16(dZ.x) && (!o.mul_saved || fg_aligned16(o.mul_saved));
-    if (aligned && bwd_paired_ok(ctx, M, N, K, dA != nullptr, dB != nullptr)) {
-        const uint64_t mk = (uint64_t)M * K, kn = (uint64_t)K * N, mn = (uint64_t)M * N;
-        if (!dZ.pairs) {
-            if ((s = fg_ws_alloc(ctx, mn * 4, &p)) != FG_OK) return s;
-            if ((s = launch_pairs(ctx, dZ.x, mn, (__nv_bfloat16*)p, mn)) != FG_OK) return s;
-            dZ.pairs = p; dZ.stride = mn;
-        }
-        if (dB) {
-            if (!A.pairs) {
-                if ((s = fg_ws_alloc(ctx, mk * 4, &p)) != FG_OK) return s;
-                if ((s = launch_pairs(ctx, A.x, mk, (__nv_bfloat16*)p, mk)) != FG_OK) return s;
-                A.pairs = p; A.stride = mk;
-            }
-            // operands Aᵀ (rows = K) and dZᵀ (rows = N), both read from [M, .] storage: contraction over the rows
-            const PlaneSet pa = paired_operand(A.x, A.pairs, A.stride, K, false);
-            const PlaneSet pz = paired_operand(dZ.x, dZ.pairs, dZ.stride, N, false);
-            if ((s = paired_gemm(ctx, pa, pz, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr, PairedOut{nullptr, 0, nullptr, 0, nullptr})) != FG_OK)
-                return s;
-        }
-        if (exch_buf && (s = fg_allreduce_sum_f32(ctx, exch_buf, exch_count)) != FG_OK) return s;
-        if (dA) {
-            if (!B.pairs) {
-                if ((s = fg_ws_alloc(ctx, kn * 4, &p)) != FG_OK) return s;
-                if ((s = launch_pairs(ctx, B.x, kn, (__nv_bfloat16*)p, kn)) != FG_OK) return s;
-                B.pairs = p; B.stride = kn;
-            }
-            // operands dZ (rows = M) and B (rows = K), both with the contraction index N contiguous
-            const PlaneSet pz = paired_operand(dZ.x, dZ.pairs, dZ.stride, N, true);
-            const PlaneSet pb = paired_operand(B.x, B.pairs, B.stride, N, true);
-            PairedOut po = o;
-            po.colsum_part = cs_part;
-            if ((s = paired_gemm(ctx, pz, pb, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr, po)) != FG_OK) return s;
-            if (cs_part && (s = fg_colsum_fold_launch(ctx, K, cs_chunks, cs_part, dbias_prev)) != FG_OK) return s;
-        }
-        return FG_OK;
+    const BwdRoutes rt = pick_bwd_routes(ctx, M, N, K, A, B, dZ, dB, dA, o.mul_saved);
+    if (!rt.planes && (dA || dB)) {
+        PairedOut po = o;
+        po.colsum_part = cs_part;
+        if ((s = gemm_bwd_products(ctx, M, N, K, A, B, dZ, N, rt, dB, dA, po, exch_buf, exch_count)) != FG_OK) return s;
+        return cs_part ? fg_colsum_fold_launch(ctx, K, cs_chunks, cs_part, dbias_prev) : FG_OK;
     }
     // Any other shape: operand planes, then what the dA epilogue would have done as passes of their own.
     if ((s = gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, A.x, B.x, dZ.x, FG_ACT_NONE, nullptr, dA, dB, nullptr, nullptr, exch_buf,
@@ -1894,27 +2540,65 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, !dB || A, "fg_gemm_bwd_f32: dB needs A");
     const bool fuse = act != FG_ACT_NONE;
     const int path = pick_path(ctx, mode, M, N, K);
-    const bool aligned = fg_aligned16(dY) && (!saved || fg_aligned16(saved)) && (!dZ_out || fg_aligned16(dZ_out)) &&
-                         (!dA || (fg_aligned16(B) && fg_aligned16(dA))) && (!dB || (fg_aligned16(A) && fg_aligned16(dB)));
-    if (path == 2 && N > 16 && aligned && bwd_paired_ok(ctx, M, N, K, dA != nullptr, dB != nullptr)) {
-        // dZ with its pairs and the bias gradient's partials in one pass, then both products from the tensors themselves
+    if (path == 2 && N > 16 && (dA || dB)) {
+        // dZ (with its pairs, if a product needs them) and the bias gradient's partials in one pass, then both products
+        // from the tensors themselves
         const uint64_t mn = (uint64_t)M * N;
         const uint32_t cs_chunks = (M + 31) / 32;
-        const uint64_t need = bwd_paired_need(M, N, K) + mn * 4 + (uint64_t)cs_chunks * N * 4 + 1024;
-        { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
-        int32_t s;
-        void *pz = nullptr, *dzb = dZ_out, *csp = nullptr;
-        if ((s = fg_ws_alloc(ctx, mn * 4, &pz)) != FG_OK) return s;
-        if (fuse && !dzb && (s = fg_ws_alloc(ctx, mn * 4, &dzb)) != FG_OK) return s;
-        if (dbias && (s = fg_ws_alloc(ctx, (uint64_t)cs_chunks * N * 4, &csp)) != FG_OK) return s;
-        if ((s = launch_dz_pairs(ctx, M, N, dY, fuse ? saved : nullptr, act, (float*)dzb, (__nv_bfloat16*)pz, mn, (float*)csp)) != FG_OK)
-            return s;
-        if (dbias && (s = fg_colsum_fold_launch(ctx, N, cs_chunks, (const float*)csp, dbias)) != FG_OK) return s;
-        const float* dz_src = dzb ? (const float*)dzb : dY;
-        return gemm_bwd_paired_core(ctx, M, N, K, PairedArg{A, nullptr, 0}, PairedArg{B, nullptr, 0}, PairedArg{dz_src, pz, mn}, dB, dA,
-                                    PairedOut{nullptr, 0, nullptr, 0, nullptr}, nullptr, exch_buf, exch_count);
+        const bool vec_z = N % 8 == 0 && fg_aligned16(dY) && (!fuse || fg_aligned16(saved)) && (!dZ_out || fg_aligned16(dZ_out));
+        // dZ is new when there is an activation: it will lie in the scratch arena (or dZ_out) with a usable pitch
+        const bool own_z = fuse || !in_place32(dY, N, 1, 0);
+        const float* const z_like = own_z ? nullptr : dY;      // only its alignment counts
+        const bool z_dense = N % 4 == 0;
+        const BwdRoutes rt = pick_bwd_routes(ctx, M, N, K, PairedArg{A, nullptr, 0}, PairedArg{B, nullptr, 0}, PairedArg{z_like, nullptr, 0}, dB, dA, nullptr);
+        const bool want_pairs = (dB && rt.dB.kind == kRoutePair) || (dA && rt.dA.kind == kRoutePair);
+        if (!rt.planes && (!want_pairs || vec_z)) {
+            const uint64_t need = bwd_paired_need(M, N, K) + (uint64_t)M * round4(N) * 4 + mn * 4 + (uint64_t)cs_chunks * N * 4 + 1024;
+            { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
+            int32_t s;
+            void *pz = nullptr, *dzb = nullptr, *csp = nullptr;
+            if (dbias && (s = fg_ws_alloc(ctx, (uint64_t)cs_chunks * N * 4, &csp)) != FG_OK) return s;
+            PairedArg z{dY, nullptr, 0};
+            if (want_pairs) {
+                dzb = dZ_out;
+                if ((s = fg_ws_alloc(ctx, mn * 4, &pz)) != FG_OK) return s;
+                if (fuse && !dzb && (s = fg_ws_alloc(ctx, mn * 4, &dzb)) != FG_OK) return s;
+                if ((s = launch_dz_pairs(ctx, M, N, dY, fuse ? saved : nullptr, act, (float*)dzb, (__nv_bfloat16*)pz, mn, (float*)csp)) != FG_OK)
+                    return s;
+                if (dzb) z.x = (const float*)dzb;
+                z.pairs = pz; z.stride = mn;
+            } else if (own_z || csp || dZ_out) {
+                PrepArgs a{};
+                a.x = dY; a.saved = fuse ? saved : nullptr; a.act = act; a.R = M; a.C = N;
+                a.colsum_part = (float*)csp;
+                if (own_z && !(z_dense && dZ_out && fg_aligned16(dZ_out))) {
+                    if ((s = fg_ws_alloc(ctx, (uint64_t)M * round4(N) * 4, &dzb)) != FG_OK) return s;
+                    a.out = dzb; a.ld = round4(N);
+                    a.copy = dZ_out;
+                } else a.copy = dZ_out;
+                if ((s = launch_prep(ctx, FG_DTYPE_F32, a)) != FG_OK) return s;
+                if (own_z) z.x = dzb ? (const float*)dzb : dZ_out;
+            }
+            if (dbias && (s = fg_colsum_fold_launch(ctx, N, cs_chunks, (const float*)csp, dbias)) != FG_OK) return s;
+            return gemm_bwd_products(ctx, M, N, K, PairedArg{A, nullptr, 0}, PairedArg{B, nullptr, 0}, z, own_z && !z_dense && !want_pairs ? round4(N) : N, rt,
+                                     dB, dA, PairedOut{nullptr, 0, nullptr, 0, nullptr}, exch_buf, exch_count);
+        }
     }
     return gemm_bwd_planes(ctx, mode, M, N, K, A, B, dY, act, saved, dA, dB, dbias, dZ_out, exch_buf, exch_count);
+}
+
+}  // namespace
+
+namespace {
+
+// One launch of the conversion kernel for `batch` products, or a loop over them?  The loop's cost per matrix is the pair
+// kernel's when the matrix suits it (its pairs are made for the whole batch at once), otherwise a pre-pass and a
+// partly filled wave per matrix.
+bool batch_converts(const fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, bool pair_ok, ConvPlan* p) {
+    if (!conv_allowed(ctx) || batch > 65535) return false;
+    *p = plan_conv(ctx, M, N, K, batch);
+    const double elems = (double)M * K + (double)K * N;
+    return p->cycles <= (double)batch * pair_cycles(ctx, M, N, K, pair_ok ? elems : 2.0 * elems, 2);
 }
 
 }  // namespace
@@ -1969,10 +2653,10 @@ int32_t fg_gemm_bwd_paired_f32(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, 
 
 // Batched forms: `batch` independent products, operand t at base + t*stride (strides in elements).
 // The reference steps A, B and C by one matrix per Z index of a rank-3 matmul (kernel/forward.rs:159-190).
-// Rank-3 products.  Small matrices (the SIMT path's range) run as ONE launch with the matrix index in the grid's
-// z, as the reference's generated kernel does (kernel/forward.rs:159-190).  Larger ones use the tensor cores: the
-// bf16 pairs of the whole batch are made by one pass per operand, then one GEMM launch per matrix reads its slice
-// (batch + 2 launches, and a launch that fills the GPU gains nothing from being merged with its neighbours).
+// Rank-3 products.  Small matrices (the SIMT path's range) and middling ones (the conversion kernel) run as ONE launch
+// with the matrix index in the grid's z, as the reference's generated kernel does (kernel/forward.rs:159-190).  Large
+// ones: the bf16 pairs of the whole batch are made by one pass per operand, then one GEMM launch per matrix reads its
+// slice (batch + 2 launches, and a launch that fills the GPU gains nothing from being merged with its neighbours).
 int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, const float* A,
                             uint64_t strideA, const float* B, uint64_t strideB, float* C, uint64_t strideC,
                             const float* bias, int32_t act, float* preact_out) {
@@ -1985,6 +2669,20 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
     if (batch == 0 || (uint64_t)M * N == 0) return FG_OK;
     if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && K > 0)
         return fg_gemm_simt_batched_launch(ctx, 0, 0, batch, M, N, K, A, strideA, B, strideB, C, strideC, bias, act, preact_out);
+    if (pick_path(ctx, mode, M, N, K) == 2 && (N > 16 || mode != FG_GEMM_AUTO)) {
+        ConvPlan cp;
+        if (batch_converts(ctx, batch, M, N, K, paired_shape_ok(ctx, M, N, K, K, N), &cp)) {
+            const uint64_t need = copy32_bytes(A, M, K, batch, strideA) + copy32_bytes(B, K, N, batch, strideB) +
+                                  conv_partial_bytes(cp, M, N, batch) + 1024;
+            int32_t s = fg_ws_ensure(ctx, need);
+            PlaneSet pa, pb;
+            if (s != FG_OK || (s = loadable32(ctx, A, M, K, batch, strideA, &pa)) != FG_OK) return s;
+            if ((s = loadable32(ctx, B, K, N, batch, strideB, &pb)) != FG_OK) return s;
+            Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
+            ep.c_batch = strideC;
+            return launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, cp, batch);
+        }
+    }
     const bool dense = strideA == (uint64_t)M * K && strideB == (uint64_t)K * N;
     // the condition under which every per-matrix call below takes the path that reads pairs
     const bool shared_pairs = dense && mode == FG_GEMM_AUTO && N > 16 && N % 4 == 0 && strideC % 4 == 0 && fg_aligned16(A) &&
@@ -2051,6 +2749,46 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
                                                    FG_ACT_NONE, nullptr)) != FG_OK) return s;
         return FG_OK;
     }
+    if (pick_path(ctx, mode, M, N, K) == 2 && (N > 16 || mode != FG_GEMM_AUTO)) {
+        ConvPlan cb{}, ca{};
+        const bool n8 = N % 8 == 0 && K % 8 == 0;
+        const bool all = (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N), &cb)) &&
+                         (!dA || batch_converts(ctx, batch, M, K, N, n8 && paired_shape_ok(ctx, M, K, N, N, N), &ca));
+        if (all) {
+            // dZ for the whole batch in one pass, then one launch per product
+            const bool own_z = act != FG_ACT_NONE;
+            const uint64_t need = (own_z ? (uint64_t)batch * M * round4(N) * 4 + 256 : copy32_bytes(dY, M, N, batch, strideC)) +
+                                  (dB ? copy32_bytes(A, M, K, batch, strideA) + conv_partial_bytes(cb, K, N, batch) : 0) +
+                                  (dA ? copy32_bytes(B, K, N, batch, strideB) + conv_partial_bytes(ca, M, K, batch) : 0) + 2048;
+            int32_t s = fg_ws_ensure(ctx, need);
+            if (s != FG_OK) return s;
+            PlaneSet z, x;
+            if (own_z) {
+                void* p;
+                if ((s = fg_ws_alloc(ctx, (uint64_t)batch * M * round4(N) * 4, &p)) != FG_OK) return s;
+                PrepArgs a{};
+                a.x = dY; a.saved = saved; a.act = act; a.R = M; a.C = N; a.x_batch = strideC; a.out = p; a.ld = round4(N);
+                if ((s = launch_prep(ctx, FG_DTYPE_F32, a, batch)) != FG_OK) return s;
+                z = PlaneSet{};
+                z.p32 = (float*)p;
+                z.ld32 = round4(N);
+                z.batch32 = (uint64_t)M * round4(N);
+            } else if ((s = loadable32(ctx, dY, M, N, batch, strideC, &z)) != FG_OK) return s;
+            if (dB) {
+                if ((s = loadable32(ctx, A, M, K, batch, strideA, &x)) != FG_OK) return s;
+                Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
+                ep.c_batch = strideB;
+                if ((s = launch_conv(ctx, as_operand(x, true), as_operand(z, true), ep, cb, batch)) != FG_OK) return s;
+            }
+            if (dA) {
+                if ((s = loadable32(ctx, B, K, N, batch, strideB, &x)) != FG_OK) return s;
+                Epilogue ep{dA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
+                ep.c_batch = strideA;
+                if ((s = launch_conv(ctx, as_operand(z, false), as_operand(x, false), ep, ca, batch)) != FG_OK) return s;
+            }
+            return FG_OK;
+        }
+    }
     for (uint32_t t = 0; t < batch; ++t) {
         int32_t s = fg_gemm_bwd_f32(ctx, mode, M, N, K, A ? A + t * strideA : nullptr, B ? B + t * strideB : nullptr,
                                     dY + t * strideC, act, saved ? saved + t * strideC : nullptr,
@@ -2067,82 +2805,9 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
 // lie: one kind::f16 MMA per 16 values of k, read through K-major or MN-major descriptors, so
 // nothing is transposed.  What the loads need is a 16-byte aligned base and row pitch; a tensor
 // without them is copied once with its pitch padded, and dZ = dY * act'(saved) is formed once
-// (both by prep16_kernel, which also sums dZ's columns for the bias gradient).
+// (both by prep_kernel, which also sums dZ's columns for the bias gradient).
 // ------------------------------------------------------------------------------------
 namespace {
-
-struct Prep16Args {
-    const void* x;        // [R, C] 16-bit
-    const void* saved;    // non-NULL: value = x * act'(saved), rounded to the storage type
-    int act;
-    uint32_t R, C;
-    void* out;            // [R][ld] or NULL
-    uint32_t ld;
-    float* colsum_part;   // [ceil(R/32)][C] f32 or NULL
-};
-
-template <typename T> __device__ __forceinline__ float lp_to_float(T v);
-template <> __device__ __forceinline__ float lp_to_float<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float lp_to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename T> __device__ __forceinline__ T lp_from_float(float v);
-template <> __device__ __forceinline__ __half lp_from_float<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 lp_from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-// W columns per thread (8: one 128-bit access; 1: any shape and alignment), 32 rows x 32 * W columns per block.
-template <typename T, int W>
-__global__ void __launch_bounds__(256) prep16_kernel(const Prep16Args a) {
-    __shared__ float cs[8][32 * W + 1];
-    const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * W;
-    const uint32_t r0 = blockIdx.y * 32;
-    struct __align__(W * 2) Vec { T e[W]; };
-    float sum[W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) sum[w] = 0.0f;
-    if (c < a.C) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t r = r0 + threadIdx.y + 8 * k;
-            if (r >= a.R) break;
-            const size_t i = (size_t)r * a.C + c;
-            Vec v = *reinterpret_cast<const Vec*>(static_cast<const T*>(a.x) + i);
-            if (a.saved) {
-                const Vec sv = *reinterpret_cast<const Vec*>(static_cast<const T*>(a.saved) + i);
-#pragma unroll
-                for (int w = 0; w < W; ++w) v.e[w] = lp_from_float<T>(lp_to_float(v.e[w]) * fg_act_grad(a.act, lp_to_float(sv.e[w])));
-            }
-            if (a.out) *reinterpret_cast<Vec*>(static_cast<T*>(a.out) + (size_t)r * a.ld + c) = v;
-#pragma unroll
-            for (int w = 0; w < W; ++w) sum[w] += lp_to_float(v.e[w]);
-        }
-    }
-    if (!a.colsum_part) return;
-#pragma unroll
-    for (int w = 0; w < W; ++w) cs[threadIdx.y][threadIdx.x * W + w] = sum[w];
-    __syncthreads();
-    const uint32_t t = threadIdx.y * 32 + threadIdx.x, col = blockIdx.x * (32 * W) + t;
-    if (t < 32 * W && col < a.C) {
-        float z = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) z += cs[k][t];
-        a.colsum_part[(size_t)blockIdx.y * a.C + col] = z;
-    }
-}
-
-int32_t launch_prep16(fg_ctx* ctx, int dtype, const Prep16Args& a) {
-    const bool vec = a.C % 8 == 0 && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved));      // a.out is ours: aligned, pitch % 8 == 0
-    const uint32_t w = vec ? 256 : 32;
-    dim3 grid((a.C + w - 1) / w, (a.R + 31) / 32), block(32, 8);
-    if (grid.y > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "16-bit GEMM operand has too many rows");
-    if (dtype == FG_DTYPE_F16) {
-        if (vec) prep16_kernel<__half, 8><<<grid, block, 0, ctx->stream>>>(a);
-        else prep16_kernel<__half, 1><<<grid, block, 0, ctx->stream>>>(a);
-    } else {
-        if (vec) prep16_kernel<__nv_bfloat16, 8><<<grid, block, 0, ctx->stream>>>(a);
-        else prep16_kernel<__nv_bfloat16, 1><<<grid, block, 0, ctx->stream>>>(a);
-    }
-    FG_LAUNCHED(ctx);
-    return FG_OK;
-}
 
 inline uint32_t pad8(uint32_t x) { return (x + 7u) & ~7u; }
 // A dense [rows, cols] tensor can be loaded in place when every row starts on a 16-byte boundary.
@@ -2157,11 +2822,11 @@ int32_t loadable16(fg_ctx* ctx, int dtype, const void* x, uint32_t rows, uint32_
     void* p;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)rows * pad8(cols) * 2, &p);
     if (s != FG_OK) return s;
-    Prep16Args a{};
+    PrepArgs a{};
     a.x = x; a.R = rows; a.C = cols; a.out = p; a.ld = pad8(cols);
     *out = p;
     *ld = a.ld;
-    return launch_prep16(ctx, dtype, a);
+    return launch_prep(ctx, dtype, a);
 }
 
 // An operand whose rows are the output's rows or columns; mn: the storage is [contraction][rows].
@@ -2231,7 +2896,7 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
     { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
     int32_t s;
     void *dz = const_cast<void*>(dY), *cs_part = nullptr;
-    Prep16Args pz{};
+    PrepArgs pz{};
     pz.x = dY; pz.saved = fuse ? saved : nullptr; pz.act = act; pz.R = M; pz.C = N;
     if ((dA || dB) && !dz_direct) {
         if ((s = fg_ws_alloc(ctx, (uint64_t)M * pad8(N) * 2, &dz)) != FG_OK) return s;
@@ -2242,7 +2907,7 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
         if ((s = fg_ws_alloc(ctx, (uint64_t)nchunk_rows * N * 4, &cs_part)) != FG_OK) return s;
         pz.colsum_part = (float*)cs_part;
     }
-    if ((pz.out || pz.colsum_part) && (s = launch_prep16(ctx, dtype, pz)) != FG_OK) return s;
+    if ((pz.out || pz.colsum_part) && (s = launch_prep(ctx, dtype, pz)) != FG_OK) return s;
     const void* x;
     uint32_t ldx;
     if (dB) {

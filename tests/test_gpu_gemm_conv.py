@@ -1,0 +1,111 @@
+"""The conversion kernel (f32 tensors straight into tensor-core tiles), its K-shares, padded copies and batches: sizes around
+tiles of 128 x 64 / 128, k-blocks of 32 and accumulation chunks of 256."""
+import numpy as np
+import pytest
+
+from conftest import rel_err_ok
+
+pytestmark = pytest.mark.gpu
+# Two tensor-core terms per product: the cross terms are rounded to bf16 (2^-18 of the product at most), and up to 64 MMAs
+# add into one accumulator with truncation (64 * 2^-24): about 5e-6 of the result's rms, five times that at the worst of
+# a million elements.  After an activation, errors of z are compared with the rms of y, which is smaller.
+TOL, TOL_ACT = 4e-5, 1e-4
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    yield c
+    assert c.device_status() == 0
+    c.destroy()
+
+
+def rng(seed):
+    return np.random.Generator(np.random.Philox(seed))
+
+
+def up(ctx, a):
+    return ctx.init_tensor_f32(a.shape, np.ascontiguousarray(a, np.float32))
+
+
+def check(x, ref, tol, what):
+    ok, worst = rel_err_ok(x, ref, tol)
+    assert ok, f"{what}: {worst:.3g} x {tol}"
+
+
+# (M, N, K): one tile; edges of tiles; ragged pitches; long K cut into shares; many tiles
+SHAPES = [(64, 256, 256), (100, 1000, 1024), (128, 128, 256), (129, 65, 544), (65, 4100, 4096), (200, 333, 77), (257, 130, 8200),
+          (1000, 1001, 777), (384, 256, 200), (70, 17, 3600)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("tA,tB", [(False, False), (True, False), (False, True), (True, True)])
+def test_forward(ctx, oracle, M, N, K, tA, tB):
+    r = rng(M + 3 * N + 7 * K + tA + 2 * tB)
+    A, B = r.standard_normal((K, M) if tA else (M, K), np.float32), r.standard_normal((N, K) if tB else (K, N), np.float32) * 0.1
+    bias = r.standard_normal(N, np.float32)
+    C, P = ctx.new_tensor((M, N)), ctx.new_tensor((M, N))
+    ctx.gemm(up(ctx, A), up(ctx, B), C, M, N, K, transA=tA, transB=tB, bias=up(ctx, bias), act="gelu", preact_out=P)
+    y, z = oracle.bias_act_fwd(oracle.gemm(A, B, transA=tA, transB=tB, f64=True).astype(np.float32), bias, "gelu")
+    check(ctx.to_numpy(P), z, TOL, "pre-activation")
+    check(ctx.to_numpy(C), y, TOL_ACT, "output")
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("act,dz_out", [("none", False), ("none", True), ("tanh", False), ("gelu", True)])
+def test_backward(ctx, oracle, M, N, K, act, dz_out):
+    r = rng(M * 5 + N + K)
+    A, B = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    dY, saved = r.standard_normal((M, N), np.float32), np.tanh(r.standard_normal((M, N))).astype(np.float32)
+    dz = oracle.act_bwd(dY, saved, act)
+    dA, dB, db = ctx.new_tensor((M, K)), ctx.new_tensor((K, N)), ctx.new_tensor((N,))
+    Z = ctx.new_tensor((M, N)) if dz_out else None
+    Ad, Bd, Yd, Sd = up(ctx, A), up(ctx, B), up(ctx, dY), up(ctx, saved) if act != "none" else None
+    ctx.gemm_bwd(Ad, Bd, Yd, M, N, K, act=act, saved=Sd, dA=dA, dB=dB, dbias=db, dZ_out=Z)
+    check(ctx.to_numpy(dA), oracle.gemm(dz, B, transB=True, f64=True), TOL, "dA")
+    check(ctx.to_numpy(dB), oracle.gemm(A, dz, transA=True, f64=True), TOL, "dB")
+    check(ctx.to_numpy(db), dz.astype(np.float64).sum(0), TOL, "dbias")
+    if dz_out:
+        check(ctx.to_numpy(Z), dz, 1e-5, "dZ")
+    only = ctx.new_tensor((K, N))
+    ctx.gemm_bwd(Ad, None, Yd, M, N, K, act=act, saved=Sd, dB=only)
+    check(ctx.to_numpy(only), oracle.gemm(A, dz, transA=True, f64=True), TOL, "dB alone")
+
+
+def test_unaligned_operands(ctx, oracle):
+    # tensors that start one element off a 16-byte boundary are read from padded copies
+    M, N, K = 192, 260, 400
+    r = rng(5)
+    A, B = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    off = lambda a: up(ctx, np.concatenate([[0], a.ravel()]).astype(np.float32))          # noqa: E731
+    Ad, Bd, C = off(A), off(B), ctx.new_tensor((M * N + 1,))
+    ctx.gemm(Ad.ptr + 4, Bd.ptr + 4, C.ptr + 4, M, N, K)
+    check(ctx.to_numpy(C)[1:].reshape(M, N), oracle.gemm(A, B, f64=True), TOL, "unaligned")
+
+
+@pytest.mark.parametrize("T,M,N,K", [(2, 64, 256, 256), (5, 130, 100, 333), (16, 384, 320, 512), (3, 65, 515, 1024), (40, 64, 64, 1100)])
+@pytest.mark.parametrize("gap", [0, 4, 6])
+def test_batched(ctx, oracle, T, M, N, K, gap):
+    # gap: elements between the matrices of a batch beyond their own size
+    r = rng(T + M + N + K + gap)
+    act = "tanh" if gap else "none"
+    sizes = [M * K + gap, K * N + gap, M * N + gap]
+    A, B, dY, S = (r.standard_normal((T, s)).astype(np.float32) for s in (*sizes, sizes[2]))
+    B *= 0.1
+    S = np.tanh(S)
+    a = lambda x, t, shape: x[t, :shape[0] * shape[1]].reshape(shape)                     # noqa: E731
+    C, dA, dB = (ctx.init_tensor_f32((T, s), np.full((T, s), 7.0)) for s in (sizes[2], sizes[0], sizes[1]))
+    Ad, Bd, Yd, Sd = (up(ctx, x) for x in (A, B, dY, S))
+    ctx.gemm_batched(Ad, Bd, C, T, M, N, K, act=act, strides=sizes)
+    ctx.gemm_batched_bwd(Ad, Bd, Yd, T, M, N, K, act=act, saved=Sd if act != "none" else None, dA=dA, dB=dB, strides=sizes)
+    got, gA, gB = (ctx.to_numpy(x) for x in (C, dA, dB))
+    for t in range(T):
+        At, Bt = a(A, t, (M, K)), a(B, t, (K, N))
+        y, _ = oracle.bias_act_fwd(oracle.gemm(At, Bt, f64=True).astype(np.float32), None, act)
+        dz = oracle.act_bwd(a(dY, t, (M, N)), a(S, t, (M, N)), act)
+        check(a(got, t, (M, N)), y, TOL_ACT, f"output {t}")
+        check(a(gA, t, (M, K)), oracle.gemm(dz, Bt, transB=True, f64=True), TOL, f"dA {t}")
+        check(a(gB, t, (K, N)), oracle.gemm(At, dz, transA=True, f64=True), TOL, f"dB {t}")
+    if gap:                         # what lies between the matrices is not touched
+        assert (got[:, M * N:] == 7.0).all() and (gA[:, M * K:] == 7.0).all() and (gB[:, K * N:] == 7.0).all()
