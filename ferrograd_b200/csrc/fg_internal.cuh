@@ -303,8 +303,9 @@ uint64_t fg_gemm_skinny_scratch_bytes(uint32_t M, uint32_t N, uint32_t K);   // 
 int32_t fg_gemm_skinny_n_launch(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, const float* A, const float* B, float* C,
                                 const float* bias, int act, float* preact_out);
 // Optional extras of the dA kernel: dA = (dZ·Bᵀ) * act'(mul_saved), its bf16 pairs, and partial column sums
-// (the partials of the bias gradient of the layer below): room for [ceil(M/32)][K]; the launch reports how many
-// rows it wrote.
+// (the partials of the bias gradient of the layer below): room for [fg_gemm_skinny_colsum_rows(M)][K]; the launch
+// reports how many rows it wrote.
+uint32_t fg_gemm_skinny_colsum_rows(uint32_t M);
 struct fg_skinny_extras {
     const float* mul_saved;
     int mul_act;

@@ -300,12 +300,21 @@ __global__ void __launch_bounds__(256) skinny_fold_slices_kernel(uint32_t M, uin
     C[o] = fg_act_fwd(act, z);
 }
 
-constexpr int TN_ROWS = 64;   // rows of A per partial sum in the dB kernel
+constexpr int TN_ROWS = 64;   // rows of A per partial sum in the dB kernel, at most
+
+// Rows per chunk: 64, or 32 or 16 when chunks of 64 would give fewer than 128 blocks (a block walks its rows one latency
+// after another: 384 rows x 256 columns in six blocks took 8.0 us).
+inline uint32_t tn_chunk_rows(uint32_t M, uint32_t Kd) {
+    const uint64_t gx = (Kd + 511) / 512;
+    uint32_t rows = TN_ROWS;
+    while (rows > 16 && gx * ((M + rows - 1) / rows) < 128) rows /= 2;
+    return rows;
+}
 
 // part[block row][n][j] = sum over the block row's chunks' rows m of A[m][j] * dZ[m][n]   (A is [M, Kd], dZ is [M, N]).
 // A thread owns four consecutive j; the chunk's rows of dZ sit in shared memory and are broadcast.
 template <int NT, bool VEC>
-__global__ void __launch_bounds__(128, 4) gemm_skinny_tn_partial_kernel(uint32_t M, uint32_t Kd, uint32_t N,
+__global__ void __launch_bounds__(128, 4) gemm_skinny_tn_partial_kernel(uint32_t M, uint32_t Kd, uint32_t N, uint32_t chunk_rows,
                                                                      const float* __restrict__ A,
                                                                      const float* __restrict__ dZ,
                                                                      float* __restrict__ part) {
@@ -317,12 +326,12 @@ __global__ void __launch_bounds__(128, 4) gemm_skinny_tn_partial_kernel(uint32_t
     for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[q][n] = 0.0f;
-    // A block walks the 64-row chunks blockIdx.y, + gridDim.y, ... and keeps its sums in registers across them:
+    // A block walks the chunks blockIdx.y, + gridDim.y, ... and keeps its sums in registers across them:
     // the number of partial results is the number of block rows (at most what the SMs hold at once), whatever M is.
-    for (uint32_t m0 = blockIdx.y * TN_ROWS; m0 < M; m0 += gridDim.y * TN_ROWS) {
-        const uint32_t rows = min((uint32_t)TN_ROWS, M - m0);
+    for (uint32_t m0 = blockIdx.y * chunk_rows; m0 < M; m0 += gridDim.y * chunk_rows) {
+        const uint32_t rows = min(chunk_rows, M - m0);
         __syncthreads();                                    // the previous chunk's rows of dZ are no longer read
-        for (uint32_t e = threadIdx.x; e < TN_ROWS * NT; e += 128) {
+        for (uint32_t e = threadIdx.x; e < chunk_rows * NT; e += 128) {
             const uint32_t r = e / NT, n = e % NT;
             zs[r][n] = (r < rows && n < N) ? dZ[(size_t)(m0 + r) * N + n] : 0.0f;
         }
@@ -523,9 +532,10 @@ uint64_t fg_gemm_skinny_scratch_bytes(uint32_t M, uint32_t N, uint32_t K) {
     const uint64_t fwd_t = 16 * kp * 4 + 256;                                            // transposed B
     const uint64_t fwd_s = (uint64_t)((K + SK_SLICE - 1) / SK_SLICE) * M * 16 * 4 + 256;  // per-slice partial sums
     const uint64_t fwd = fwd_t > fwd_s ? fwd_t : fwd_s;
-    // dB partials: one [N][K] block per block row, and there are at most as many block rows as 64-row chunks or
-    // as four blocks per SM allow (fewer than 2048 on any GPU)
-    uint64_t rows = (M + TN_ROWS - 1) / TN_ROWS;
+    // dB partials: one [N][K] block per block row, and there are at most as many block rows as chunks or as four blocks
+    // per SM allow (fewer than 2048 on any GPU)
+    const uint32_t chunk = tn_chunk_rows(M, K);
+    uint64_t rows = (M + chunk - 1) / chunk;
     if (rows > 2048) rows = 2048;
     const uint64_t bwd = rows * K * N * 4 + 256;
     return fwd > bwd ? fwd : bwd;
@@ -573,8 +583,16 @@ int32_t fg_gemm_skinny_n_launch(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K,
     return FG_OK;
 }
 
+// Rows of column-sum partials the dA launch may write, which is what its caller must have room for: one per chunk of rows
+// for a small M (a block that walks four chunks waits four times: 384 x 256 in 12 blocks took 15 us), and never more than
+// the SMs' thread slots need.
+uint32_t fg_gemm_skinny_colsum_rows(uint32_t M) {
+    const uint32_t chunks = (M + NT_ROWS - 1) / NT_ROWS, r32 = (M + 31) / 32;
+    return chunks <= 1024 ? chunks : r32 > 1024 ? r32 : 1024;
+}
+
 // dA[M, K] = dZ · B^T with dZ [M, N], B [K, N], N <= 16.  With extras->colsum_part, *colsum_rows receives the
-// number of partial rows written (at most ceil(M / 32), which is what the caller must have room for).
+// number of partial rows written (at most fg_gemm_skinny_colsum_rows(M)).
 int32_t fg_gemm_skinny_nt_launch(fg_ctx* ctx, uint32_t M, uint32_t K, uint32_t N, const float* dZ, const float* B,
                                  float* dA, const fg_skinny_extras* extras, uint32_t* colsum_rows) {
     if (N > SKN) return fg_fail(ctx, FG_ERR_INTERNAL, "skinny GEMM: N too large");
@@ -598,7 +616,7 @@ int32_t fg_gemm_skinny_nt_launch(fg_ctx* ctx, uint32_t M, uint32_t K, uint32_t N
     uint32_t gy = (uint32_t)((uint64_t)per_sm * ctx->sm_count / gx);
     if (gy < 1) gy = 1;
     if (gy > chunks) gy = chunks;
-    if (gy > (M + 31) / 32) gy = (M + 31) / 32;       // the caller's room for column-sum partials
+    if (gy > fg_gemm_skinny_colsum_rows(M)) gy = fg_gemm_skinny_colsum_rows(M);       // the caller's room for column-sum partials
     if (gy > 65535) gy = 65535;
     if (colsum_rows) *colsum_rows = gy;
     dim3 grid(gx, gy);
@@ -614,11 +632,14 @@ int32_t fg_gemm_skinny_nt_launch(fg_ctx* ctx, uint32_t M, uint32_t K, uint32_t N
 int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t N, const float* A, const float* dZ,
                                  float* dB) {
     if (N > SKN) return fg_fail(ctx, FG_ERR_INTERNAL, "skinny GEMM: N too large");
-    // block rows: as many as the SMs hold at once (four blocks of 128 threads per SM), at most one per 64-row chunk
-    const uint32_t gx = (Kd + 511) / 512;
+    // One chunk of rows: the exact path's kernel adds the same products in the same order and needs no fold (64 x 2 x 16: one
+    // launch of 3 us instead of two of 11 + 2 us).
+    if (M <= TN_ROWS) return fg_gemm_simt_launch(ctx, 1, 0, Kd, N, M, A, dZ, dB, nullptr, FG_ACT_NONE, nullptr);
+    // block rows: as many as the SMs hold at once (four blocks of 128 threads per SM), at most one per chunk
+    const uint32_t gx = (Kd + 511) / 512, chunk = tn_chunk_rows(M, Kd);
     uint32_t nchunks = (uint32_t)(4ull * ctx->sm_count / gx);
     if (nchunks < 1) nchunks = 1;
-    if (nchunks > (M + TN_ROWS - 1) / TN_ROWS) nchunks = (M + TN_ROWS - 1) / TN_ROWS;
+    if (nchunks > (M + chunk - 1) / chunk) nchunks = (M + chunk - 1) / chunk;
     void* part;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)nchunks * Kd * N * 4, &part);
     if (s != FG_OK) return s;
@@ -626,8 +647,8 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
     const bool vec = (Kd % 4 == 0) && fg_aligned16(A);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SKINNY, 4.0 * M * Kd);                // A read once
     FG_SKINNY_DISPATCH(N, {
-        if (vec) gemm_skinny_tn_partial_kernel<NT, true><<<grid, 128, 0, ctx->stream>>>(M, Kd, N, A, dZ, (float*)part);
-        else gemm_skinny_tn_partial_kernel<NT, false><<<grid, 128, 0, ctx->stream>>>(M, Kd, N, A, dZ, (float*)part);
+        if (vec) gemm_skinny_tn_partial_kernel<NT, true><<<grid, 128, 0, ctx->stream>>>(M, Kd, N, chunk, A, dZ, (float*)part);
+        else gemm_skinny_tn_partial_kernel<NT, false><<<grid, 128, 0, ctx->stream>>>(M, Kd, N, chunk, A, dZ, (float*)part);
     });
     FG_LAUNCHED(ctx);
     const uint64_t n = (uint64_t)Kd * N;

@@ -2388,9 +2388,10 @@ uint64_t bwd_planes_need(uint32_t M, uint32_t N, uint32_t K) {
 //   dA [M,K] = (dZ·Bᵀ) * act'(o.mul_saved) with its pairs (o.pairs) and its column sums (dbias_prev [K]) --
 //   i.e. the dZ of the layer below and that layer's bias gradient come out of the dA epilogue.
 // Pairs that are not supplied are made in the scratch arena.  The caller has reserved bwd_paired_need().
+uint32_t colsum_room(uint32_t M, uint32_t N) { return N <= 16 ? fg_gemm_skinny_colsum_rows(M) : (M + 31) / 32; }
 uint64_t bwd_paired_need(uint32_t M, uint32_t N, uint32_t K) {
     // (the conversion kernel's K-shares take less than kPairPartialBytes, its padded copies less than the planes)
-    return 4ull * ((uint64_t)M * K + (uint64_t)K * N + (uint64_t)M * N) + (uint64_t)((M + 31) / 32) * K * 4 +
+    return 4ull * ((uint64_t)M * K + (uint64_t)K * N + (uint64_t)M * N) + (uint64_t)colsum_room(M, N) * K * 4 +
            2 * kPairPartialBytes + 4096 + fg_gemm_skinny_scratch_bytes(M, N, K) + bwd_planes_need(M, N, K);
 }
 
@@ -2484,7 +2485,7 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
     const uint32_t cs_chunks = (M + 31) / 32;
     float* cs_part = nullptr;
     if (dA && dbias_prev) {
-        if ((s = fg_ws_alloc(ctx, (uint64_t)cs_chunks * K * 4, &p)) != FG_OK) return s;
+        if ((s = fg_ws_alloc(ctx, (uint64_t)colsum_room(M, N) * K * 4, &p)) != FG_OK) return s;
         cs_part = (float*)p;
     }
     if (N <= 16) {

@@ -102,10 +102,12 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ w, float
 
 // ---- several tensors in one launch ----
 // A model whose weights are separate tensors (the reference's layout) would otherwise pay one launch per tensor,
-// most of them tiny (biases).  The tensors are cut into chunks of kMultiChunk elements; chunk c belongs to the
-// tensor t with first_chunk[t] <= c < first_chunk[t + 1]; CTAs stride over the chunks.
+// most of them tiny (biases).  The tensors are cut into chunks; chunk c belongs to the tensor t with
+// first_chunk[t] <= c < first_chunk[t + 1]; CTAs stride over the chunks.
+// A chunk is 8192 elements, eight passes of a block, or down to 1024, one pass, while that leaves fewer than four blocks
+// per SM: a small model is bound by the latency of those passes (120,000 parameters with adamw: 8.3 us at 8192).
 constexpr int kMultiMax = 16;
-constexpr uint32_t kMultiChunk = 8192;
+constexpr uint32_t kMultiChunkMax = 8192, kMultiChunkMin = 1024;
 struct MultiArgs {
     float* w[kMultiMax];
     float* g[kMultiMax];
@@ -115,6 +117,7 @@ struct MultiArgs {
     uint64_t pairs_stride[kMultiMax];
     uint64_t n[kMultiMax];
     uint32_t first_chunk[kMultiMax + 1];
+    uint32_t chunk;
     int count;
 };
 
@@ -131,8 +134,8 @@ __global__ void __launch_bounds__(256) update_multi_kernel(const __grid_constant
     for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         int t = 0;
         while (t + 1 < a.count && ch >= a.first_chunk[t + 1]) ++t;
-        const uint64_t base = (uint64_t)(ch - a.first_chunk[t]) * kMultiChunk;
-        const uint64_t n = a.n[t], end = min(n, base + kMultiChunk);
+        const uint64_t base = (uint64_t)(ch - a.first_chunk[t]) * a.chunk;
+        const uint64_t n = a.n[t], end = min(n, base + a.chunk);
         float* const w = a.w[t];
         float* const g = a.g[t];
         float* const m = a.m[t];
@@ -186,14 +189,17 @@ int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t
         MultiArgs a;
         memset(&a, 0, sizeof(a));
         double bytes = 0.0;
-        uint64_t chunks = 0;
+        uint64_t chunks = 0, total = 0;
         int cnt = 0;
-        for (uint32_t k = k0; k < count && cnt < kMultiMax; ++k) {
+        for (uint32_t k = k0; k < count && k < k0 + kMultiMax; ++k) total += t[k].n;
+        a.chunk = kMultiChunkMax;
+        while (a.chunk > kMultiChunkMin && total / a.chunk < 4ull * (uint64_t)ctx->sm_count) a.chunk /= 2;
+        for (uint32_t k = k0; k < count && k < k0 + kMultiMax; ++k) {
             if (t[k].n == 0) continue;
             a.w[cnt] = t[k].w; a.g[cnt] = t[k].g; a.m[cnt] = t[k].m; a.v[cnt] = t[k].v;
             a.pairs[cnt] = (__nv_bfloat16*)t[k].w_pairs; a.pairs_stride[cnt] = t[k].pairs_stride; a.n[cnt] = t[k].n;
             a.first_chunk[cnt] = (uint32_t)chunks;
-            chunks += (t[k].n + kMultiChunk - 1) / kMultiChunk;
+            chunks += (t[k].n + a.chunk - 1) / a.chunk;
             bytes += ((adam ? 28.0 : 12.0) + (zero_grad ? 4.0 : 0.0) + (t[k].w_pairs ? 4.0 : 0.0)) * (double)t[k].n;
             ++cnt;
         }

@@ -1,0 +1,53 @@
+"""The narrow layer's backward kernels at few samples, where chunks shrink and a single chunk takes the exact path, and the
+multi-tensor update at the sizes where its chunks shrink."""
+import numpy as np
+import pytest
+
+from conftest import rel_err_ok
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    yield c
+    c.sync()
+    c.destroy()
+
+
+def check(x, ref, what):
+    # sums of at most 1100 f32 products in chunks of 16 to 64: 2^-24 * sqrt(1100) * 5 with the reference's own error on top
+    ok, worst = rel_err_ok(x, ref, 2e-5)
+    assert ok, f"{what}: {worst:.3g}"
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 2, 16), (8, 16, 5), (64, 16, 2), (65, 10, 33), (100, 4, 520), (384, 12, 256), (1100, 3, 64)])
+def test_backward(ctx, oracle, M, N, K):
+    r = np.random.Generator(np.random.Philox(M + N + K))
+    f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
+    up = lambda a: ctx.init_tensor_f32(a.shape, a)                            # noqa: E731
+    A, B, dZ, saved = f(M, K), f(K, N), f(M, N), np.tanh(f(M, K))
+    dB, dA, db, db_below = (ctx.new_tensor(s) for s in ((K, N), (M, K), (N,), (K,)))
+    sa = (M * K + 7) // 8 * 8
+    ctx.gemm_bwd_paired(up(A), up(B), up(dZ), M, N, K, dB=dB, dbias=db, dA=dA, below_act="tanh", below_saved=up(saved),
+                        dA_pairs=ctx.alloc_zeroed(4 * sa), dA_stride=sa, below_dbias=db_below)
+    ref = oracle.act_bwd(oracle.gemm(dZ, B, transB=True, f64=True), saved, "tanh")
+    check(ctx.to_numpy(dB), oracle.gemm(A, dZ, transA=True, f64=True), "dB")
+    check(ctx.to_numpy(dA), ref, "dA")
+    check(ctx.to_numpy(db), dZ.astype(np.float64).sum(0), "dbias")
+    check(ctx.to_numpy(db_below), ref.astype(np.float64).sum(0), "bias gradient of the layer below")
+
+
+@pytest.mark.parametrize("sizes", [(1,), (1023, 1025), (5000, 0, 3), (700_001, 17), tuple([300] * 15 + [0] + [500] * 4)])
+def test_update_of_several_tensors(ctx, oracle, sizes):
+    r = np.random.Generator(np.random.Philox(len(sizes)))
+    w, g = [r.standard_normal(n).astype(np.float32) for n in sizes], [r.standard_normal(n).astype(np.float32) for n in sizes]
+    place = lambda a: ctx.init_tensor_f32((max(a.size, 1),), a if a.size else np.zeros(1, np.float32))       # noqa: E731
+    wd, gd = [place(a) for a in w], [place(a) for a in g]
+    ctx.sgd_step_multi([dict(w=a, g=b, n=n) for a, b, n in zip(wd, gd, sizes)], 0.1)
+    for a, b, n, dw, dg in zip(w, g, sizes, wd, gd):
+        if n:
+            oracle.sgd(a, b, 0.1)
+            assert np.array_equal(ctx.to_numpy(dw), a) and (ctx.to_numpy(dg) == 0).all()
