@@ -221,12 +221,44 @@ __device__ __forceinline__ void prefetch_row(uint32_t dst, const float* src, uin
     }
 }
 
+// Four elements of the outputs: e * inv, and for the loss (p - onehot) * scale.  Only the float4 that holds the label (i ==
+// lab / 4) is looked at element by element.
+template <int MODE>
+__device__ __forceinline__ void softmax_put4(const CeArgs& a, float4* o0, float4* o1, uint32_t i, uint32_t lab, float4 e, float inv, bool stream) {
+    const float4 p = make_float4(e.x * inv, e.y * inv, e.z * inv, e.w * inv);
+    auto put = [&](float4* o, float4 v) { if (stream) __stcs(o + i, v); else o[i] = v; };
+    if (MODE == 0) {
+        put(o0, p);
+    } else {
+        if (o1) put(o1, p);
+        if (o0) {
+            float4 g = p;
+            if (i == lab >> 2) {
+                const uint32_t t = lab & 3u;
+                g.x -= t == 0 ? 1.f : 0.f; g.y -= t == 1 ? 1.f : 0.f; g.z -= t == 2 ? 1.f : 0.f; g.w -= t == 3 ? 1.f : 0.f;
+            }
+            put(o0, make_float4(g.x * a.scale, g.y * a.scale, g.z * a.scale, g.w * a.scale));
+        }
+    }
+}
+// The lowest index among a thread's four elements that equal the row's maximum (fmaxf and == both pass over NaN).
+__device__ __forceinline__ void first_equal4(uint32_t& mi, float4 v, float mx, uint32_t c) {
+    if (v.w == mx) mi = min(mi, c + 3);
+    if (v.z == mx) mi = min(mi, c + 2);
+    if (v.y == mx) mi = min(mi, c + 1);
+    if (v.x == mx) mi = min(mi, c);
+}
+
+// All 32 warps meet at every barrier, so what counts is the instructions and barriers of a row: 8192 x 32000 with loss,
+// gradient and predicted class 419 -> 387 us with four barriers instead of eight, the label looked for in one float4 and the
+// class found by comparing with the maximum afterwards (5.4 TB/s).
 template <int MODE>
 __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int* dev_status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);             // cols floats
-    __shared__ float red[32];
-    __shared__ uint32_t redi[32];
+    // one array per reduction, so that each costs one barrier: an array is written again only after two more barriers
+    __shared__ float red_max[32], red_sum[32];
+    __shared__ uint32_t s_arg;
     __shared__ __align__(8) unsigned long long bar_storage;
     const uint32_t bar = smem_u32(&bar_storage);
     const uint32_t cols = a.cols, ncol4 = cols >> 2, row_bytes = cols * 4u;
@@ -241,7 +273,15 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
     if (tid == 0 && row < a.rows) prefetch_row(smem_u32(stage), a.x + (size_t)row * cols, row_bytes, bar);
     uint32_t parity = 0;
 
+    const int lane = tid & 31, warp = tid >> 5;
     for (; row < a.rows; row += gridDim.x) {
+        // the label's values are fetched long before they are used
+        uint32_t lab = 0xffffffffu;
+        float xlab = 0.0f;
+        if (MODE == 1) {
+            lab = a.labels[row];
+            if (tid == 0 && lab < cols) xlab = a.x[(size_t)row * cols + lab];
+        }
         // 1. wait for this row in shared memory, move it to registers
         bool ok = mbar_wait_bounded(bar, parity);
         parity ^= 1u;
@@ -258,6 +298,7 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
             uint32_t i = tid + j * kRowT;
             v[j] = i < ncol4 ? s4[i] : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
         }
+        if (MODE == 1 && tid == 0) s_arg = 0xffffffffu;
         __syncthreads();   // everyone has read the staging buffer
         // 2. start streaming the next row while this one is processed
         const uint32_t next = row + gridDim.x;
@@ -265,26 +306,22 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             prefetch_row(smem_u32(stage), a.x + (size_t)next * cols, row_bytes, bar);
         }
-        // 3. max (and argmax)
+        // 3. max, then the first column that has it
         float mx = -CUDART_INF_F;
+#pragma unroll
+        for (int j = 0; j < kRowNV; ++j)
+            mx = fmaxf(fmaxf(mx, fmaxf(v[j].x, v[j].y)), fmaxf(v[j].z, v[j].w));
+        mx = warp_max(mx);
+        if (lane == 0) red_max[warp] = mx;
+        __syncthreads();
+        mx = warp_max(red_max[lane]);
         if (MODE == 1 && a.argmax) {
             uint32_t mi = 0xffffffffu;
 #pragma unroll
-            for (int j = 0; j < kRowNV; ++j) {
-                uint32_t c = 4u * (tid + j * kRowT);
-                argmax_merge(mx, mi, v[j].x, c);
-                argmax_merge(mx, mi, v[j].y, c + 1);
-                argmax_merge(mx, mi, v[j].z, c + 2);
-                argmax_merge(mx, mi, v[j].w, c + 3);
-            }
-            uint32_t am = block_argmax(mx, mi, red, redi);
-            if (tid == 0) a.argmax[row] = am;
-        } else {
-#pragma unroll
             for (int j = 0; j < kRowNV; ++j)
-                mx = fmaxf(fmaxf(mx, fmaxf(v[j].x, v[j].y)), fmaxf(v[j].z, v[j].w));
+                if (tid + j * kRowT < ncol4) first_equal4(mi, v[j], mx, 4u * (tid + j * kRowT));
+            if (mi != 0xffffffffu) atomicMin(&s_arg, mi);
         }
-        mx = block_max(mx, red);
         // 4. e = exp(x - max), sum
         float s = 0.0f;
 #pragma unroll
@@ -295,38 +332,22 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
             v[j].w = expf(v[j].w - mx);
             s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
         }
-        s = block_sum(s, red);
+        s = warp_sum(s);
+        if (lane == 0) red_sum[warp] = s;
+        __syncthreads();
+        s = warp_sum(red_sum[lane]);
         const float inv = 1.0f / s;
-        uint32_t lab = 0xffffffffu;
-        if (MODE == 1) {
-            lab = a.labels[row];
-            if (tid == 0 && a.loss_row)
-                a.loss_row[row] = lab < cols ? (logf(s) + mx) - a.x[(size_t)row * cols + lab] : 0.0f;
+        if (MODE == 1 && tid == 0) {
+            if (a.argmax) a.argmax[row] = s_arg;
+            if (a.loss_row) a.loss_row[row] = lab < cols ? (logf(s) + mx) - xlab : 0.0f;
         }
         // 5. write
         float4* o0 = MODE == 0 ? reinterpret_cast<float4*>(a.y + (size_t)row * cols)
                                : (a.dlogits ? reinterpret_cast<float4*>(a.dlogits + (size_t)row * cols) : nullptr);
         float4* o1 = (MODE == 1 && a.probs) ? reinterpret_cast<float4*>(a.probs + (size_t)row * cols) : nullptr;
 #pragma unroll
-        for (int j = 0; j < kRowNV; ++j) {
-            uint32_t i = tid + j * kRowT;
-            if (i < ncol4) {
-                float4 p = make_float4(v[j].x * inv, v[j].y * inv, v[j].z * inv, v[j].w * inv);
-                if (MODE == 0) {
-                    __stcs(o0 + i, p);
-                } else {
-                    if (o1) __stcs(o1 + i, p);
-                    if (o0) {
-                        uint32_t c = 4u * i;
-                        float4 g = make_float4((p.x - (c == lab ? 1.f : 0.f)) * a.scale,
-                                               (p.y - (c + 1 == lab ? 1.f : 0.f)) * a.scale,
-                                               (p.z - (c + 2 == lab ? 1.f : 0.f)) * a.scale,
-                                               (p.w - (c + 3 == lab ? 1.f : 0.f)) * a.scale);
-                        __stcs(o0 + i, g);
-                    }
-                }
-            }
-        }
+        for (int j = 0; j < kRowNV; ++j)
+            if (tid + j * kRowT < ncol4) softmax_put4<MODE>(a, o0, o1, tid + j * kRowT, lab, v[j], inv, true);
     }
 }
 
@@ -499,8 +520,13 @@ __global__ void ce_elem_kernel(const float* __restrict__ p, const uint32_t* __re
 // Fixed-order mean of the per-row losses (one CTA).
 __global__ void mean_kernel(const float* __restrict__ x, uint32_t n, float* __restrict__ out) {
     __shared__ float red[32];
-    float s = 0.0f;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
+    float s = 0.0f, v[8];
+    for (uint64_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {      // eight loads in flight, added in order
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = i0 + j * blockDim.x < n ? x[i0 + j * blockDim.x] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += v[j];
+    }
     s = block_sum(s, red);
     if (threadIdx.x == 0) *out = s / (float)n;
 }
