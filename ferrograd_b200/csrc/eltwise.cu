@@ -261,18 +261,20 @@ template <int DT, int W> __device__ __forceinline__ void stw(void* p, uint64_t i
 // The host turns a chain (forward, or backward = the values it needs followed by the adjoints) into a list of
 // single-result operations: instructions whose result nobody reads are dropped, an adjoint's first contribution is a
 // plain result and only later ones add, and results live in a few slots that are reused once their last reader has run.
-// `last` as an operand is the result of the operation just before, which stays in registers.
-enum : uint32_t { VM_LD = 64, VM_ST, VM_LDADD, VM_G_COPY, VM_G_NEG, VM_G_MUL, VM_G_DIV, VM_G_DIVB, VM_G_ABS, VM_G_TANH, VM_G_RELU,
-                  VM_G_GELU, VM_G_ELU };     // below 64: the fg_ew codes, result = op(x, y)
+// The kernel keeps one set of values in registers: the result of the operation just before (`last`).  An operation takes
+// its first operand there (fetched from its slot if it is another value) and leaves its result there.
+enum : uint32_t { VM_G_TANH = 14, VM_G_RELU, VM_G_GELU, VM_G_ELU, VM_G_ABS,      // after the fg_ew codes: result = op(x, y)
+                  VM_LD, VM_LD2, VM_ST, VM_LDADD, VM_COPY };
+static_assert(FG_EW_ELU + 1 == (int)VM_G_TANH, "the operation codes are dense: one jump table");
 constexpr uint32_t kLast = 254, kNone = 255;
-struct VmOp {            // x, y, z, acc: slot, kLast or kNone.  dst: slot or kNone
+struct VmOp {            // x, y: slot, kLast or kNone.  acc: slot (result = acc + op) or kNone.  dst: slot or kNone
     uint8_t op, dst, x, y;
-    uint8_t z, acc, ptr, pad;
+    uint8_t acc, ptr, ptr2, dst2;      // VM_LD2: ptr2 goes to slot dst2, ptr to `last` and dst
     float imm;
-    uint32_t pad2;
+    uint32_t pad;
 };
 static_assert(sizeof(VmOp) == 16, "one 128-bit constant load per operation");
-constexpr int kVmMaxOps = 136;      // backward: 24 values, the seed, two adjoints per instruction, 24 + 2 * 8 for the input gradients
+constexpr int kVmMaxOps = 200;      // backward: 24 values, the seed, at most five operations per instruction, 24 + 2 * 8 for the input gradients
 constexpr int kVmMaxPtrs = FG_EW_MAX_INPUTS + 1 + FG_EW_MAX_INSTR;
 struct VmArgs {
     uint4 ops[kVmMaxOps];
@@ -280,6 +282,7 @@ struct VmArgs {
     int nops, vec;
     uint64_t n;
 };
+static_assert(sizeof(VmArgs) <= 4096, "kernel parameters");
 
 constexpr int kVmThreads = 128;
 
@@ -302,21 +305,21 @@ template <int W> __device__ __forceinline__ void slot_st(float4* sm, uint32_t sl
     }
 }
 
-// One operation on W elements: the op-code is decoded once, the lanes loop inside each case.
+// One operation on W elements, in place: the op-code is decoded once, the lanes loop inside each case.
 #define FG_VM_LANES(expr)                                                                                   \
     do {                                                                                                    \
-        _Pragma("unroll") for (int w = 0; w < W; ++w) { const float xx = x[w], yy = y[w]; (void)xx; (void)yy; r[w] = (expr); } \
+        _Pragma("unroll") for (int w = 0; w < W; ++w) { const float xx = x[w], yy = y[w]; (void)xx; (void)yy; x[w] = (expr); } \
     } while (0)
 template <int DT, int W>
-__device__ __forceinline__ void vm_op(uint32_t op, float imm, const float* x, const float* y, const float* z, float* r) {
+__device__ __forceinline__ void vm_op(uint32_t op, float imm, float* x, const float* y) {
     typedef Stored<DT> S;
     switch (op) {
         case FG_EW_CONST: FG_VM_LANES(S::r(imm)); break;
         case FG_EW_ADD: FG_VM_LANES(S::r(xx + yy)); break;
         case FG_EW_SUB: FG_VM_LANES(S::r(xx - yy)); break;
-        case FG_EW_MUL: case VM_G_MUL: FG_VM_LANES(S::r(xx * yy)); break;
-        case FG_EW_DIV: case VM_G_DIV: FG_VM_LANES(S::r(__fdiv_rn(xx, yy))); break;
-        case FG_EW_NEG: case VM_G_NEG: FG_VM_LANES(-xx); break;
+        case FG_EW_MUL: FG_VM_LANES(S::r(xx * yy)); break;
+        case FG_EW_DIV: FG_VM_LANES(S::r(__fdiv_rn(xx, yy))); break;
+        case FG_EW_NEG: FG_VM_LANES(-xx); break;
         case FG_EW_ABS: FG_VM_LANES(fabsf(xx)); break;
         case FG_EW_EXP: FG_VM_LANES(S::r(expf(xx))); break;
         case FG_EW_LOG: FG_VM_LANES(S::r(logf(xx))); break;
@@ -324,15 +327,13 @@ __device__ __forceinline__ void vm_op(uint32_t op, float imm, const float* x, co
         case FG_EW_RELU: FG_VM_LANES(xx > 0.0f ? xx : 0.0f); break;
         case FG_EW_GELU: FG_VM_LANES(S::r(fg_gelu_fwd(xx))); break;
         case FG_EW_ELU: FG_VM_LANES(xx >= 0.0f ? xx : S::r(expf(xx) - 1.0f)); break;
-        // adjoints: x is the adjoint of the result, y (and z) the values the derivative needs
-        case VM_G_COPY: FG_VM_LANES(xx); break;
-        case VM_G_DIVB: FG_VM_LANES(-S::r(__fdiv_rn(S::r(xx * yy), S::r(z[w] * z[w])))); break;      // y numerator, z denominator
-        case VM_G_ABS: FG_VM_LANES(yy >= 0.0f ? xx : -xx); break;
+        // adjoints: x is the adjoint of the result, y the value the derivative is taken at
         case VM_G_TANH: FG_VM_LANES(S::r(xx * S::r(1.0f - S::r(yy * yy)))); break;
         case VM_G_RELU: FG_VM_LANES(xx * (yy > 0.0f ? 1.0f : 0.0f)); break;
         case VM_G_GELU: FG_VM_LANES(S::r(xx * S::r(fg_gelu_grad(yy)))); break;
         case VM_G_ELU: FG_VM_LANES(yy >= 0.0f ? xx : S::r(xx * S::r(yy + 1.0f))); break;
-        default: FG_VM_LANES(0.0f); break;
+        case VM_G_ABS: FG_VM_LANES(yy >= 0.0f ? xx : -xx); break;
+        default: break;      // VM_COPY
     }
 }
 #undef FG_VM_LANES
@@ -350,61 +351,47 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2,
             o[0] = S::ld(p, i);
         }
     };
-    float last[W];
+    float last[W], y[W];
 #pragma unroll
-    for (int w = 0; w < W; ++w) last[w] = 0.0f;
-    auto operand = [&](uint32_t slot, float* o) {
-        if (slot < kLast) slot_ld<W>(sm, slot, o);
-        else {
-#pragma unroll
-            for (int w = 0; w < W; ++w) o[w] = last[w];
-        }
-    };
+    for (int w = 0; w < W; ++w) last[w] = y[w] = 0.0f;
+    uint4 c = a.ops[0];
 #pragma unroll 1
     for (int k = 0; k < a.nops; ++k) {
-        const uint4 c = a.ops[k];
         const uint32_t op = c.x & 255u, dst = c.x >> 8 & 255u, xs = c.x >> 16 & 255u, ys = c.x >> 24;
-        const uint32_t zs = c.y & 255u, accs = c.y >> 8 & 255u, ptr = c.y >> 16 & 255u;
-        float x[W];
-        if (op == VM_LD) {
+        const uint32_t acc = c.y & 255u, ptr = c.y >> 8 & 255u, ptr2 = c.y >> 16 & 255u, dst2 = c.y >> 24;
+        const float imm = __uint_as_float(c.z);
+        c = a.ops[k + 1 < kVmMaxOps ? k + 1 : k];       // the next operation's code is on its way during this one
+        if (ys == kLast) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) y[w] = last[w];
+        } else if (ys != kNone) {
+            slot_ld<W>(sm, ys, y);
+        }
+        if (xs < kLast) slot_ld<W>(sm, xs, last);
+        if (op < VM_LD) {
+            vm_op<DT, W>(op, imm, last, y);
+        } else if (op == VM_LD) {
             load(a.ptr[ptr], last);
-        } else {
-            operand(xs, x);
-            if (op == VM_ST) {
-                if constexpr (W == 8) {
-                    S::st4w(a.ptr[ptr], i, x);
-                    if (two) S::st4w(a.ptr[ptr], i2, x + 4);
-                } else {
-                    S::st(a.ptr[ptr], i, x[0]);
-                }
-                continue;
-            }
-            float y[W], r[W];
-            if (op == VM_LDADD) {
-                load(a.ptr[ptr], y);
-#pragma unroll
-                for (int w = 0; w < W; ++w) r[w] = S::r(y[w] + x[w]);
+        } else if (op == VM_LD2) {                      // both on their way at once
+            load(a.ptr[ptr2], y);
+            load(a.ptr[ptr], last);
+            slot_st<W>(sm, dst2, y);
+        } else if (op == VM_ST) {
+            if constexpr (W == 8) {
+                S::st4w(a.ptr[ptr], i, last);
+                if (two) S::st4w(a.ptr[ptr], i2, last + 4);
             } else {
-                float z[W];
-                if (ys != kNone) operand(ys, y);
-                else {
-#pragma unroll
-                    for (int w = 0; w < W; ++w) y[w] = 0.0f;
-                }
-                if (zs != kNone) operand(zs, z);
-                else {
-#pragma unroll
-                    for (int w = 0; w < W; ++w) z[w] = 0.0f;
-                }
-                vm_op<DT, W>(op, __uint_as_float(c.z), x, y, z, r);
-                if (accs != kNone) {
-                    operand(accs, z);
-#pragma unroll
-                    for (int w = 0; w < W; ++w) r[w] = S::r(z[w] + r[w]);
-                }
+                S::st(a.ptr[ptr], i, last[0]);
             }
+        } else if (op == VM_LDADD) {
+            load(a.ptr[ptr], y);
 #pragma unroll
-            for (int w = 0; w < W; ++w) last[w] = r[w];
+            for (int w = 0; w < W; ++w) last[w] = S::r(y[w] + last[w]);
+        }
+        if (acc != kNone) {
+            slot_ld<W>(sm, acc, y);
+#pragma unroll
+            for (int w = 0; w < W; ++w) last[w] = S::r(y[w] + last[w]);
         }
         if (dst != kNone) slot_st<W>(sm, dst, last);
     }
@@ -413,8 +400,9 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2,
 // A block takes 1024 consecutive elements at a time, thread t the groups of four t and t + 128 of them (every access of a
 // warp is contiguous).  The last n % 4 elements go singly, on the last block, which has the least other work.
 //
-// What bounds it: instruction issue.  gelu(x * y) + x on 32 Mi f32 elements: forward 147 -> 141 us, backward 340 -> 141 us
-// against one interpreter step per instruction and lane-wise slots; x / (1 + exp(-x)) * y on 3 M halves 68 -> 49 us for both.
+// What bounds it: instruction issue (about 25 instructions to fetch, decode and store an operation, shared by eight elements).
+// gelu(x * y) + x on 32 Mi f32 elements: forward 147 -> 100 us, backward 340 -> 168 us against one interpreter step per
+// instruction and word-wise slots; x / (1 + exp(-x)) * y on 3 M halves 18.4 -> 14.8 us and 49.6 -> 30 us.
 template <int DT>
 __global__ void __launch_bounds__(kVmThreads) chain_kernel(const __grid_constant__ VmArgs a) {
     extern __shared__ float4 chain_smem[];
@@ -431,49 +419,80 @@ __global__ void __launch_bounds__(kVmThreads) chain_kernel(const __grid_constant
 
 // ---- host side: a chain as a list of operations ----
 struct VmBuilder {
-    struct Node { int op, x, y, z, acc, ptr; float imm; int id; };    // operands are result ids, -1 = none
+    struct Node { int op, x, y, acc, ptr; float imm; int id, ptr2, id2; };    // operands are result ids, -1 = none
     Node node[kVmMaxOps];
     int n = 0, ids = 0;
-    int emit(int op, int x, int y, int z, int acc, int ptr, float imm) {
+    int emit(int op, int x, int y, int acc, int ptr, float imm) {
         const int id = op == (int)VM_ST ? -1 : ids++;
-        node[n++] = Node{op, x, y, z, acc, ptr, imm, id};
+        node[n++] = Node{op, x, y, acc, ptr, imm, id, -1, -1};
         return id;
     }
+    // Loads before the first store move to the front (at most four: each holds a slot until it is used) and go two at a time.
+    void gather_loads() {
+        Node ld[4], rest[kVmMaxOps];
+        int nl = 0, nr = 0;
+        bool stored = false;
+        for (int i = 0; i < n; ++i) {
+            stored |= node[i].op == (int)VM_ST;
+            if (node[i].op == (int)VM_LD && !stored && nl < 4) ld[nl++] = node[i];
+            else rest[nr++] = node[i];
+        }
+        n = 0;
+        int i = 0;
+        for (; i + 1 < nl; i += 2) {
+            node[n] = ld[i + 1];
+            node[n].op = VM_LD2;
+            node[n].ptr2 = ld[i].ptr;
+            node[n++].id2 = ld[i].id;
+        }
+        if (i < nl) node[n++] = ld[i];
+        for (int j = 0; j < nr; ++j) node[n++] = rest[j];
+    }
     // Assigns slots by the results' life times and writes the kernel's operations; returns the number of slots.
-    int finish(VmArgs* a) const {
+    int finish(VmArgs* a) {
+        gather_loads();
         int last_use[kVmMaxOps], slot[kVmMaxOps];
         bool stored[kVmMaxOps], taken[kVmMaxOps];
         for (int i = 0; i < ids; ++i) { last_use[i] = -1; slot[i] = -1; stored[i] = false; }
-        for (int i = 0; i < n; ++i) taken[i] = false;
-        int prev = -1;      // the result that is in `last` before operation i
+        for (int i = 0; i < kVmMaxOps; ++i) taken[i] = false;
+        auto next_last = [](const Node& o, int prev) { return o.id >= 0 ? o.id : o.x >= 0 ? o.x : prev; };
+        int prev = -1;      // the value that is in `last` before operation i
         for (int i = 0; i < n; ++i) {
-            for (int u : {node[i].x, node[i].y, node[i].z, node[i].acc})
+            Node& o = node[i];
+            // what is in the registers serves as the first operand where the order does not matter
+            if ((o.op == FG_EW_ADD || o.op == FG_EW_MUL) && o.y == prev && o.x != prev) { const int t = o.x; o.x = o.y; o.y = t; }
+            for (int u : {o.x, o.y})
                 if (u >= 0 && u != prev) { stored[u] = true; last_use[u] = i; }
-            if (node[i].id >= 0) prev = node[i].id;
+            if (o.acc >= 0) { stored[o.acc] = true; last_use[o.acc] = i; }
+            if (o.id2 >= 0) { stored[o.id2] = true; if (last_use[o.id2] < i) last_use[o.id2] = i; }
+            prev = next_last(o, prev);
         }
         int nslots = 0;
+        auto take = [&](int id) -> uint8_t {
+            int f = 0;
+            while (taken[f]) ++f;
+            taken[f] = true;
+            slot[id] = f;
+            if (f + 1 > nslots) nslots = f + 1;
+            return (uint8_t)f;
+        };
         prev = -1;
         for (int i = 0; i < n; ++i) {
             const Node& o = node[i];
             auto where = [&](int u) -> uint8_t { return u < 0 ? (uint8_t)kNone : u == prev ? (uint8_t)kLast : (uint8_t)slot[u]; };
             VmOp v{};
             v.op = (uint8_t)o.op;
-            v.x = where(o.x); v.y = where(o.y); v.z = where(o.z); v.acc = where(o.acc);
+            v.x = where(o.x); v.y = where(o.y);
+            v.acc = o.acc < 0 ? (uint8_t)kNone : (uint8_t)slot[o.acc];
             v.ptr = (uint8_t)(o.ptr < 0 ? 0 : o.ptr);
+            v.ptr2 = (uint8_t)(o.ptr2 < 0 ? 0 : o.ptr2);
             v.imm = o.imm;
+            if (o.id2 >= 0) v.dst2 = take(o.id2);
             // a slot whose last reader this is may receive the result: operands are read before it is written
-            for (int u : {o.x, o.y, o.z, o.acc})
-                if (u >= 0 && slot[u] >= 0 && last_use[u] == i) taken[slot[u]] = false;
-            v.dst = (uint8_t)kNone;
-            if (o.id >= 0 && stored[o.id]) {
-                int f = 0;
-                while (taken[f]) ++f;
-                taken[f] = true;
-                slot[o.id] = f;
-                v.dst = (uint8_t)f;
-                if (f + 1 > nslots) nslots = f + 1;
-            }
-            if (o.id >= 0) prev = o.id;
+            for (int u : {o.x, o.y, o.acc, o.id2})
+                if (u >= 0 && slot[u] >= 0 && last_use[u] == i && !(u == o.id2 && o.op != (int)VM_LD2)) taken[slot[u]] = false;
+            v.dst = o.id >= 0 && stored[o.id] ? take(o.id) : (uint8_t)kNone;
+            prev = next_last(o, prev);
             memcpy(&a->ops[i], &v, sizeof(v));
         }
         a->nops = n;
@@ -488,10 +507,10 @@ void build_values(VmBuilder& b, const fg_ew_instr* prog, int ninstr, const bool*
     for (int k = 0; k < ninstr; ++k) {
         if (!need[k]) continue;
         const fg_ew_instr& in = prog[k];
-        if (in.op == FG_EW_INPUT) id[k] = b.emit(VM_LD, -1, -1, -1, -1, in.a, 0.0f);
-        else if (in.op == FG_EW_CONST) id[k] = b.emit(in.op, -1, -1, -1, -1, -1, in.imm);
-        else id[k] = b.emit(in.op, id[in.a], ew_two_operands(in.op) ? id[in.b] : -1, -1, -1, -1, in.imm);
-        if (saved && saved[k]) b.emit(VM_ST, id[k], -1, -1, -1, saved_ptr0 + k, 0.0f);
+        if (in.op == FG_EW_INPUT) id[k] = b.emit(VM_LD, -1, -1, -1, in.a, 0.0f);
+        else if (in.op == FG_EW_CONST) id[k] = b.emit(in.op, -1, -1, -1, -1, in.imm);
+        else id[k] = b.emit(in.op, id[in.a], ew_two_operands(in.op) ? id[in.b] : -1, -1, -1, in.imm);
+        if (saved && saved[k]) b.emit(VM_ST, id[k], -1, -1, saved_ptr0 + k, 0.0f);
     }
 }
 // Marks everything the marked instructions read.
@@ -512,7 +531,7 @@ void build_forward(VmBuilder& b, const fg_ew_instr* prog, int ninstr, void* cons
     for (int k = 0; k < ninstr; ++k) need[k] = k == ninstr - 1 || (saved && saved[k]);
     close_over(prog, ninstr, need);
     build_values(b, prog, ninstr, need, id, saved, kPtrSaved);
-    b.emit(VM_ST, id[ninstr - 1], -1, -1, -1, kPtrOut, 0.0f);
+    b.emit(VM_ST, id[ninstr - 1], -1, -1, kPtrOut, 0.0f);
 }
 
 // Adjoints are added up in the order of the program walked backwards, operand a before operand b, and an input that is
@@ -545,29 +564,35 @@ void build_backward(VmBuilder& b, const fg_ew_instr* prog, int ninstr, int ninpu
     build_values(b, prog, ninstr, need, id, nullptr, 0);
     bool flows = false;
     for (int k = 0; k < ninstr; ++k) flows |= prog[k].op == FG_EW_INPUT && active[k] && touched[k];
-    if (flows) adj[ninstr - 1] = b.emit(VM_LD, -1, -1, -1, -1, kPtrOut, 0.0f);
+    if (flows) adj[ninstr - 1] = b.emit(VM_LD, -1, -1, -1, kPtrOut, 0.0f);
     for (int k = ninstr - 1; k >= 0 && flows; --k) {
         const fg_ew_instr& in = prog[k];
         if (!touched[k] || !active[k] || in.op == FG_EW_INPUT || in.op == FG_EW_CONST) continue;
         const int g = adj[k];
-        auto add = [&](int to, int op, int y, int z) {
-            if (adj[to] < 0 && op == (int)VM_G_COPY) adj[to] = g;            // a first contribution that is the adjoint itself
-            else adj[to] = b.emit(op, g, y, z, adj[to], -1, 0.0f);
+        auto add = [&](int to, int op, int x, int y) {
+            if (adj[to] < 0 && op == (int)VM_COPY) adj[to] = x;              // a first contribution that is the adjoint itself
+            else adj[to] = b.emit(op, x, y, adj[to], -1, 0.0f);
         };
         const bool da = active[in.a], db = ew_two_operands(in.op) && active[in.b];
         switch (in.op) {
-            case FG_EW_ADD: if (da) add(in.a, VM_G_COPY, -1, -1); if (db) add(in.b, VM_G_COPY, -1, -1); break;
-            case FG_EW_SUB: if (da) add(in.a, VM_G_COPY, -1, -1); if (db) add(in.b, VM_G_NEG, -1, -1); break;
-            case FG_EW_MUL: if (da) add(in.a, VM_G_MUL, id[in.b], -1); if (db) add(in.b, VM_G_MUL, id[in.a], -1); break;
-            case FG_EW_DIV: if (da) add(in.a, VM_G_DIV, id[in.b], -1); if (db) add(in.b, VM_G_DIVB, id[in.a], id[in.b]); break;
-            case FG_EW_NEG: add(in.a, VM_G_NEG, -1, -1); break;
-            case FG_EW_ABS: add(in.a, VM_G_ABS, id[in.a], -1); break;
-            case FG_EW_EXP: add(in.a, VM_G_MUL, id[k], -1); break;
-            case FG_EW_LOG: add(in.a, VM_G_DIV, id[in.a], -1); break;
-            case FG_EW_TANH: add(in.a, VM_G_TANH, id[k], -1); break;
-            case FG_EW_RELU: add(in.a, VM_G_RELU, id[k], -1); break;
-            case FG_EW_GELU: add(in.a, VM_G_GELU, id[in.a], -1); break;
-            case FG_EW_ELU: add(in.a, VM_G_ELU, id[k], -1); break;
+            case FG_EW_ADD: if (da) add(in.a, VM_COPY, g, -1); if (db) add(in.b, VM_COPY, g, -1); break;
+            case FG_EW_SUB: if (da) add(in.a, VM_COPY, g, -1); if (db) add(in.b, FG_EW_NEG, g, -1); break;
+            case FG_EW_MUL: if (da) add(in.a, FG_EW_MUL, g, id[in.b]); if (db) add(in.b, FG_EW_MUL, g, id[in.a]); break;
+            case FG_EW_DIV:
+                if (da) add(in.a, FG_EW_DIV, g, id[in.b]);
+                if (db) {       // - (g * a) / (b * b), every step rounded
+                    const int den = b.emit(FG_EW_MUL, id[in.b], id[in.b], -1, -1, 0.0f), num = b.emit(FG_EW_MUL, g, id[in.a], -1, -1, 0.0f);
+                    add(in.b, FG_EW_NEG, b.emit(FG_EW_DIV, num, den, -1, -1, 0.0f), -1);
+                }
+                break;
+            case FG_EW_NEG: add(in.a, FG_EW_NEG, g, -1); break;
+            case FG_EW_ABS: add(in.a, VM_G_ABS, g, id[in.a]); break;
+            case FG_EW_EXP: add(in.a, FG_EW_MUL, g, id[k]); break;
+            case FG_EW_LOG: add(in.a, FG_EW_DIV, g, id[in.a]); break;
+            case FG_EW_TANH: add(in.a, VM_G_TANH, g, id[k]); break;
+            case FG_EW_RELU: add(in.a, VM_G_RELU, g, id[k]); break;
+            case FG_EW_GELU: add(in.a, VM_G_GELU, g, id[in.a]); break;
+            case FG_EW_ELU: add(in.a, VM_G_ELU, g, id[k]); break;
             default: break;
         }
     }
@@ -576,11 +601,11 @@ void build_backward(VmBuilder& b, const fg_ew_instr* prog, int ninstr, int ninpu
         int sum = -1;
         for (int k = ninstr - 1; k >= 0; --k) {
             if (prog[k].op != FG_EW_INPUT || prog[k].a != j || adj[k] < 0) continue;
-            sum = sum < 0 ? adj[k] : b.emit(FG_EW_ADD, sum, adj[k], -1, -1, -1, 0.0f);
+            sum = sum < 0 ? adj[k] : b.emit(FG_EW_ADD, sum, adj[k], -1, -1, 0.0f);
         }
-        if (sum < 0) sum = b.emit(FG_EW_CONST, -1, -1, -1, -1, -1, 0.0f);       // nothing flows into this input
-        if (accumulate) sum = b.emit(VM_LDADD, sum, -1, -1, -1, kPtrSaved + j, 0.0f);
-        b.emit(VM_ST, sum, -1, -1, -1, kPtrSaved + j, 0.0f);
+        if (sum < 0) sum = b.emit(FG_EW_CONST, -1, -1, -1, -1, 0.0f);       // nothing flows into this input
+        if (accumulate) sum = b.emit(VM_LDADD, sum, -1, -1, kPtrSaved + j, 0.0f);
+        b.emit(VM_ST, sum, -1, -1, kPtrSaved + j, 0.0f);
     }
 }
 
@@ -601,7 +626,7 @@ __global__ void __launch_bounds__(256) convert_kernel(const void* __restrict__ s
 // are at most 24 values and 24 adjoints): the limit is raised once per device and kernel.
 constexpr int kSlotBytes = 8 * kVmThreads * (int)sizeof(float);
 constexpr int kChainSmemMax = 2 * FG_EW_MAX_INSTR * kSlotBytes;
-int32_t launch_chain(fg_ctx* ctx, int dtype, const VmBuilder& b, VmArgs& a, double bytes) {
+int32_t launch_chain(fg_ctx* ctx, int dtype, VmBuilder& b, VmArgs& a, double bytes) {
     static std::atomic<uint64_t> done[3];
     const uint64_t bit = 1ull << (ctx->device & 63);
     const size_t smem = (size_t)b.finish(&a) * kSlotBytes;
