@@ -45,7 +45,10 @@ void* open_nccl() {
     return nullptr;
 }
 
-__global__ void fg_counter_increment_kernel(uint32_t* c) { *c += 1u; }
+__global__ void fg_counter_increment_kernel(uint32_t* c) {
+    fg_grid_enter();
+    *c += 1u;
+}
 
 }  // namespace
 
@@ -497,7 +500,7 @@ int32_t fg_memset_zero(fg_ctx* ctx, void* dev, uint64_t bytes) {
 int32_t fg_counter_increment(fg_ctx* ctx, uint32_t* counter_dev) {
     FG_ENTER(ctx);
     FG_REQUIRE(ctx, counter_dev != nullptr, "fg_counter_increment: NULL pointer");
-    fg_counter_increment_kernel<<<1, 1, 0, ctx->stream>>>(counter_dev);
+    fg_launch(ctx, fg_counter_increment_kernel, 1, 1, 0, counter_dev);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }

@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(256) bias_act_kernel(uint32_t rows, uint32_t c
 template <bool VEC>
 __global__ void __launch_bounds__(256) act_bwd_kernel(uint64_t n, int act, const float* __restrict__ dy,
                                                       const float* __restrict__ saved, float* __restrict__ dz) {
+    fg_grid_enter();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nv = VEC ? n >> 2 : 0;
     if constexpr (VEC) for (uint64_t i = g; i < nv; i += stride) {
@@ -89,6 +90,7 @@ template <class TERM, bool VEC>
 __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ pred, const float* __restrict__ target,
                                                    uint64_t n, float scale, float* __restrict__ loss_elem,
                                                    float* __restrict__ grad, float* __restrict__ partials) {
+    fg_grid_enter();
     __shared__ float red[8];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nv = VEC ? n >> 2 : 0;
@@ -123,6 +125,7 @@ __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ pre
 // One CTA folds the partials in a fixed order.
 __global__ void __launch_bounds__(256) fold_partials_kernel(const float* __restrict__ partials, int n,
                                                             float* __restrict__ out) {
+    fg_grid_enter();
     __shared__ float red[8];
     float s = 0.0f;
     for (int i = threadIdx.x; i < n; i += 256) s += partials[i];
@@ -138,6 +141,7 @@ __global__ void __launch_bounds__(256) fold_partials_kernel(const float* __restr
 
 // Sum of n values, stage 1: one partial per CTA (grid-stride over float4, fixed order inside a CTA).
 __global__ void __launch_bounds__(256) sum_partial_kernel(const float* __restrict__ x, uint64_t n, float* __restrict__ partials) {
+    fg_grid_enter();
     __shared__ float red[8];
     float s = 0.0f;
     const uint64_t nv = ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) ? n >> 2 : 0, stride = (uint64_t)gridDim.x * blockDim.x;
@@ -159,6 +163,7 @@ __global__ void __launch_bounds__(256) sum_partial_kernel(const float* __restric
 // Column sums, stage 1: block (32 x 8) covers 32 columns and `chunk` rows.
 __global__ void __launch_bounds__(256) colsum_partial_kernel(uint32_t rows, uint32_t cols, uint32_t chunk,
                                                              const float* __restrict__ x, float* __restrict__ part) {
+    fg_grid_enter();
     __shared__ float red[8][33];
     const uint32_t c = blockIdx.x * 32 + threadIdx.x;
     const uint32_t r0 = blockIdx.y * chunk;
@@ -179,6 +184,7 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(uint32_t rows, uint
 // (so the chain of dependent loads is an eighth as long), then the eight sums are added in order.
 __global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_t nchunks,
                                                           const float* __restrict__ part, float* __restrict__ out) {
+    fg_grid_enter();
     __shared__ float red[8][33];
     const uint32_t cx = threadIdx.x & 31u, gy = threadIdx.x >> 5;
     const uint32_t c = blockIdx.x * 32 + cx;
@@ -405,6 +411,7 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2,
 // instruction and word-wise slots; x / (1 + exp(-x)) * y on 3 M halves 18.4 -> 14.8 us and 49.6 -> 30 us.
 template <int DT>
 __global__ void __launch_bounds__(kVmThreads) chain_kernel(const __grid_constant__ VmArgs a) {
+    fg_grid_enter();
     extern __shared__ float4 chain_smem[];
     float4* const sm = chain_smem + threadIdx.x;
     const uint64_t nv = a.vec ? a.n >> 2 : 0;
@@ -642,7 +649,7 @@ int32_t launch_chain(fg_ctx* ctx, int dtype, VmBuilder& b, VmArgs& a, double byt
     const int per_sm = (int)(fit < 1 ? 1 : fit > 16 ? 16 : fit);
     const int grid = fg_stream_grid(ctx, a.vec ? (a.n / 4 + 1) / 2 : a.n, kVmThreads, per_sm);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, bytes);
-    kernel<<<grid, kVmThreads, smem, ctx->stream>>>(a);
+    fg_launch(ctx, kernel, grid, kVmThreads, smem, a);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;
@@ -672,15 +679,15 @@ int32_t fg_act_bwd_launch(fg_ctx* ctx, uint64_t n, int act, const float* dy, con
     const bool vec = aligned16(dy) && aligned16(saved) && aligned16(dz);
     const int grid = fg_stream_grid(ctx, vec ? (n + 3) / 4 : n, 256, 8);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (act == FG_ACT_NONE ? 8.0 : 12.0) * n);
-    if (vec) act_bwd_kernel<true><<<grid, 256, 0, ctx->stream>>>(n, act, dy, saved, dz);
-    else act_bwd_kernel<false><<<grid, 256, 0, ctx->stream>>>(n, act, dy, saved, dz);
+    if (vec) fg_launch(ctx, act_bwd_kernel<true>, grid, 256, 0, n, act, dy, saved, dz);
+    else fg_launch(ctx, act_bwd_kernel<false>, grid, 256, 0, n, act, dy, saved, dz);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
 
 int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, float* out) {
-    colsum_fold_kernel<<<(cols + 31) / 32, 256, 0, ctx->stream>>>(cols, nchunks, part, out);
+    fg_launch(ctx, colsum_fold_kernel, (cols + 31) / 32, 256, 0, cols, nchunks, part, out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
@@ -690,16 +697,16 @@ int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float*
     const uint32_t nchunks = (rows + chunk - 1) / chunk;
     dim3 grid((cols + 31) / 32, nchunks), block(32, 8);
     if (nchunks == 1) {      // the only partial is the sum
-        colsum_partial_kernel<<<grid, block, 0, ctx->stream>>>(rows, cols, chunk, x, out);
+        fg_launch(ctx, colsum_partial_kernel, grid, block, 0, rows, cols, chunk, x, out);
         FG_LAUNCHED(ctx);
         return FG_OK;
     }
     void* part;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)nchunks * cols * sizeof(float), &part);
     if (s != FG_OK) return s;
-    colsum_partial_kernel<<<grid, block, 0, ctx->stream>>>(rows, cols, chunk, x, (float*)part);
+    fg_launch(ctx, colsum_partial_kernel, grid, block, 0, rows, cols, chunk, x, (float*)part);
     FG_LAUNCHED(ctx);
-    colsum_fold_kernel<<<(cols + 31) / 32, 256, 0, ctx->stream>>>(cols, nchunks, (const float*)part, out);
+    fg_launch(ctx, colsum_fold_kernel, (cols + 31) / 32, 256, 0, cols, nchunks, (const float*)part, out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
@@ -743,9 +750,9 @@ int32_t fg_sum_f32(fg_ctx* ctx, const float* x, uint64_t n, float* out) {
     void* p;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &p);
     if (s != FG_OK) return s;
-    sum_partial_kernel<<<grid, 256, 0, ctx->stream>>>(x, n, (float*)p);
+    fg_launch(ctx, sum_partial_kernel, grid, 256, 0, x, n, (float*)p);
     FG_LAUNCHED(ctx);
-    fold_partials_kernel<<<1, 256, 0, ctx->stream>>>((const float*)p, grid, out);
+    fg_launch(ctx, fold_partials_kernel, 1, 256, 0, (const float*)p, grid, out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
@@ -769,12 +776,12 @@ int32_t fg_mse_loss_grad(fg_ctx* ctx, const float* pred, const float* target, ui
         partials = (float*)p;
     }
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (8.0 + (loss_elem_out ? 4.0 : 0.0) + (grad_out ? 4.0 : 0.0)) * n);
-    if (vec) loss_kernel<MseTerm, true><<<grid, 256, 0, ctx->stream>>>(pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
-    else loss_kernel<MseTerm, false><<<grid, 256, 0, ctx->stream>>>(pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
+    if (vec) fg_launch(ctx, loss_kernel<MseTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
+    else fg_launch(ctx, loss_kernel<MseTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     if (loss_sum_out) {
-        fold_partials_kernel<<<1, 256, 0, ctx->stream>>>(partials, grid, loss_sum_out);
+        fg_launch(ctx, fold_partials_kernel, 1, 256, 0, partials, grid, loss_sum_out);
         FG_LAUNCHED(ctx);
     }
     return FG_OK;
@@ -799,12 +806,12 @@ int32_t fg_bce_loss_grad(fg_ctx* ctx, const float* pred, const float* target, ui
         partials = (float*)p;
     }
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (8.0 + (loss_elem_out ? 4.0 : 0.0) + (grad_out ? 4.0 : 0.0)) * n);
-    if (vec) loss_kernel<BceTerm, true><<<grid, 256, 0, ctx->stream>>>(pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
-    else loss_kernel<BceTerm, false><<<grid, 256, 0, ctx->stream>>>(pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
+    if (vec) fg_launch(ctx, loss_kernel<BceTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
+    else fg_launch(ctx, loss_kernel<BceTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     if (loss_sum_out) {
-        fold_partials_kernel<<<1, 256, 0, ctx->stream>>>(partials, grid, loss_sum_out);
+        fg_launch(ctx, fold_partials_kernel, 1, 256, 0, partials, grid, loss_sum_out);
         FG_LAUNCHED(ctx);
     }
     return FG_OK;

@@ -7,6 +7,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <utility>
+
 #include "../../include/ferrograd_b200.h"
 
 // Device error word bits, set by kernels whose bounded waits ran out.
@@ -124,6 +126,29 @@ struct FgRange {
     do { cudaError_t _e = cudaGetLastError(); \
          if (_e != cudaSuccess) return fg_fail_cuda((ctx), FG_ERR_LAUNCH_FAILURE, "kernel launch", _e); \
          if ((ctx)->capturing) (ctx)->capture_launches++; else (ctx)->launches++; } while (0)
+
+// Back-to-back launches of short kernels.  A kernel launched with fg_launch may be set up while the kernel before it on the
+// stream still runs (programmatic stream serialization); fg_grid_enter(), its first statement in every thread, waits until
+// everything before it has finished and is visible, then lets the next such kernel be set up.  Seven launches of a ragged
+// layer's backward pass 75.8 -> 60.5 us, the 16 of a 2-16-2 training step 33.4 -> 28.7 us.
+template <typename... P, typename... A>
+inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ctx->comm ? 0 : 1;      // with a communicator the stream also forks and joins: plain order there
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // FG_LAUNCHED reports its error
+}
+__device__ __forceinline__ void fg_grid_enter() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
 
 // Brackets one kernel launch with events when timing is enabled (never while capturing).
 inline fg_time_rec* fg_time_begin(fg_ctx* ctx, int kind, double work) {

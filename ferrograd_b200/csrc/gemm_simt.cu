@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(TM * TN / (4 * RPT)) gemm_simt_kernel(uint32_t
                                                         const float* __restrict__ A, const float* __restrict__ B,
                                                         float* __restrict__ C, const float* __restrict__ bias, int act,
                                                         float* __restrict__ preact, uint64_t sA, uint64_t sB, uint64_t sC) {
+    fg_grid_enter();
     constexpr int T = TM * TN / (4 * RPT), NA = TM * TK / T, NB = TN * TK / T;
     static_assert(RPT == 1 || RPT == 4, "a thread's rows are read as one word or one float4");
     __shared__ __align__(16) float As[2][TK][TM + 4];
@@ -113,10 +114,10 @@ void launch_simt_tile(fg_ctx* ctx, bool ta, bool tb, uint32_t batch, uint32_t M,
                       const float* B, uint64_t sB, float* C, uint64_t sC, const float* bias, int act, float* preact) {
     constexpr int T = TM * TN / (4 * RPT);
     const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, batch);
-    if (!ta && !tb) gemm_simt_kernel<false, false, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
-    else if (ta && !tb) gemm_simt_kernel<true, false, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
-    else if (!ta && tb) gemm_simt_kernel<false, true, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
-    else gemm_simt_kernel<true, true, TM, TN, RPT><<<grid, T, 0, ctx->stream>>>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    if (!ta && !tb) fg_launch(ctx, gemm_simt_kernel<false, false, TM, TN, RPT>, grid, T, 0, M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    else if (ta && !tb) fg_launch(ctx, gemm_simt_kernel<true, false, TM, TN, RPT>, grid, T, 0, M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    else if (!ta && tb) fg_launch(ctx, gemm_simt_kernel<false, true, TM, TN, RPT>, grid, T, 0, M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
+    else fg_launch(ctx, gemm_simt_kernel<true, true, TM, TN, RPT>, grid, T, 0, M, N, K, A, B, C, bias, act, preact, sA, sB, sC);
 }
 
 // ---- skinny outputs (N <= 16, e.g. a 10-class output layer) ----
@@ -232,6 +233,7 @@ template <int NT>
 __global__ void __launch_bounds__(256, 2) gemm_skinny_n_slice_kernel(uint32_t M, uint32_t N, uint32_t K, uint32_t rows_per_block,
                                                                      const float* __restrict__ A, const float* __restrict__ B,
                                                                      float* __restrict__ part) {
+    fg_grid_enter();
     __shared__ __align__(16) float bt[NT][SK_SLICE];
     const uint32_t k0 = blockIdx.x * SK_SLICE, kw = min((uint32_t)SK_SLICE, K - k0);
     for (uint32_t e = threadIdx.x; e < NT * SK_SLICE; e += 256) (&bt[0][0])[e] = 0.0f;
@@ -288,6 +290,7 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_n_slice_kernel(uint32_t M,
 __global__ void __launch_bounds__(256) skinny_fold_slices_kernel(uint32_t M, uint32_t N, uint32_t nslices,
                                                                  const float* __restrict__ part, const float* __restrict__ bias,
                                                                  int act, float* __restrict__ C, float* __restrict__ preact) {
+    fg_grid_enter();
     const uint32_t i = blockIdx.x * 256 + threadIdx.x;      // over M x 16
     if (i >= M * 16) return;
     const uint32_t m = i >> 4, n = i & 15;
@@ -318,6 +321,7 @@ __global__ void __launch_bounds__(128, 4) gemm_skinny_tn_partial_kernel(uint32_t
                                                                      const float* __restrict__ A,
                                                                      const float* __restrict__ dZ,
                                                                      float* __restrict__ part) {
+    fg_grid_enter();
     __shared__ float zs[TN_ROWS][NT];
     const uint32_t j0 = (blockIdx.x * 128 + threadIdx.x) * 4;
     const bool active = j0 < Kd;
@@ -405,6 +409,7 @@ template <int NT>
 __global__ void __launch_bounds__(128) gemm_skinny_nt_kernel(uint32_t M, uint32_t K, uint32_t N,
                                                              const float* __restrict__ dZ, const float* __restrict__ B,
                                                              float* __restrict__ dA, fg_skinny_extras ex) {
+    fg_grid_enter();
     __shared__ float zs[NT_ROWS][NT];
     const uint32_t k0 = (blockIdx.x * 128 + threadIdx.x) * 4;
     const bool active = k0 < K;
@@ -494,6 +499,7 @@ __global__ void __launch_bounds__(128) gemm_skinny_nt_kernel(uint32_t M, uint32_
 // eight sums are added in order.
 __global__ void __launch_bounds__(256) fold_chunks_kernel(uint32_t Kd, uint32_t N, uint32_t nchunks, const float* __restrict__ part,
                                                           float* __restrict__ out) {
+    fg_grid_enter();
     __shared__ float red[8][33];
     const uint64_t total = (uint64_t)Kd * N;
     const uint32_t cx = threadIdx.x & 31u, gy = threadIdx.x >> 5;
@@ -562,9 +568,9 @@ int32_t fg_gemm_skinny_n_launch(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K,
         dim3 grid(nslices, (M + rpb - 1) / rpb);
         if (grid.y > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "skinny GEMM: too many rows");
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SKINNY, 4.0 * M * K);                 // A read once
-        FG_SKINNY_DISPATCH(N, (gemm_skinny_n_slice_kernel<NT><<<grid, 256, 0, ctx->stream>>>(M, N, K, rpb, A, B, (float*)part)));
+        FG_SKINNY_DISPATCH(N, (fg_launch(ctx, gemm_skinny_n_slice_kernel<NT>, grid, 256, 0, M, N, K, rpb, A, B, (float*)part)));
         FG_LAUNCHED(ctx);
-        skinny_fold_slices_kernel<<<(M * 16 + 255) / 256, 256, 0, ctx->stream>>>(M, N, nslices, (const float*)part, bias, act, C, preact_out);
+        fg_launch(ctx, skinny_fold_slices_kernel, (M * 16 + 255) / 256, 256, 0, M, N, nslices, (const float*)part, bias, act, C, preact_out);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -622,7 +628,7 @@ int32_t fg_gemm_skinny_nt_launch(fg_ctx* ctx, uint32_t M, uint32_t K, uint32_t N
     dim3 grid(gx, gy);
     // dA written once; with extras also the saved tensor read and the pairs (as many bytes again) written
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SKINNY, 4.0 * M * K * (1.0 + (ex.mul_saved ? 1.0 : 0.0) + (ex.pairs ? 1.0 : 0.0)));
-    FG_SKINNY_DISPATCH(N, (gemm_skinny_nt_kernel<NT><<<grid, 128, 0, ctx->stream>>>(M, K, N, dZ, B, dA, ex)));
+    FG_SKINNY_DISPATCH(N, (fg_launch(ctx, gemm_skinny_nt_kernel<NT>, grid, 128, 0, M, K, N, dZ, B, dA, ex)));
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;
@@ -647,12 +653,12 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
     const bool vec = (Kd % 4 == 0) && fg_aligned16(A);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SKINNY, 4.0 * M * Kd);                // A read once
     FG_SKINNY_DISPATCH(N, {
-        if (vec) gemm_skinny_tn_partial_kernel<NT, true><<<grid, 128, 0, ctx->stream>>>(M, Kd, N, chunk, A, dZ, (float*)part);
-        else gemm_skinny_tn_partial_kernel<NT, false><<<grid, 128, 0, ctx->stream>>>(M, Kd, N, chunk, A, dZ, (float*)part);
+        if (vec) fg_launch(ctx, gemm_skinny_tn_partial_kernel<NT, true>, grid, 128, 0, M, Kd, N, chunk, A, dZ, (float*)part);
+        else fg_launch(ctx, gemm_skinny_tn_partial_kernel<NT, false>, grid, 128, 0, M, Kd, N, chunk, A, dZ, (float*)part);
     });
     FG_LAUNCHED(ctx);
     const uint64_t n = (uint64_t)Kd * N;
-    fold_chunks_kernel<<<fg_stream_grid(ctx, n * 8, 256, 8), 256, 0, ctx->stream>>>(Kd, N, nchunks, (const float*)part, dB);
+    fg_launch(ctx, fold_chunks_kernel, fg_stream_grid(ctx, n * 8, 256, 8), 256, 0, Kd, N, nchunks, (const float*)part, dB);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;

@@ -899,6 +899,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // consecutive columns of row t / 8.
 template <int TM, int TN>
 __global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
+    fg_grid_enter();
     __shared__ float cs_sm[8][32];
     constexpr uint32_t kSubN = TN / 32, kSubs = (TM / 32) * kSubN;
     const uint32_t pairs_m = (ep.M + TM - 1) / TM, pairs_n = (ep.N + TN - 1) / TN;
@@ -1173,6 +1174,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 lp_from_float<__nv_bfloat16
 // W columns per thread (16 bytes, or 1: any shape and alignment), 32 rows x 32 * W columns per block.
 template <typename T, int W>
 __global__ void __launch_bounds__(256) prep_kernel(const PrepArgs a) {
+    fg_grid_enter();
     __shared__ float cs[8][32 * W + 1];
     const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * W;
     const uint32_t r0 = blockIdx.y * 32;
@@ -1232,14 +1234,14 @@ int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT,
                                     es * batch * a.R * a.C * (1.0 + (a.saved ? 1.0 : 0.0) + (a.out ? 1.0 : 0.0) + (a.copy ? 1.0 : 0.0)));
     if (dtype == FG_DTYPE_F32) {
-        if (vec) prep_kernel<float, 4><<<grid, block, 0, ctx->stream>>>(a);
-        else prep_kernel<float, 1><<<grid, block, 0, ctx->stream>>>(a);
+        if (vec) fg_launch(ctx, prep_kernel<float, 4>, grid, block, 0, a);
+        else fg_launch(ctx, prep_kernel<float, 1>, grid, block, 0, a);
     } else if (dtype == FG_DTYPE_F16) {
-        if (vec) prep_kernel<__half, 8><<<grid, block, 0, ctx->stream>>>(a);
-        else prep_kernel<__half, 1><<<grid, block, 0, ctx->stream>>>(a);
+        if (vec) fg_launch(ctx, prep_kernel<__half, 8>, grid, block, 0, a);
+        else fg_launch(ctx, prep_kernel<__half, 1>, grid, block, 0, a);
     } else {
-        if (vec) prep_kernel<__nv_bfloat16, 8><<<grid, block, 0, ctx->stream>>>(a);
-        else prep_kernel<__nv_bfloat16, 1><<<grid, block, 0, ctx->stream>>>(a);
+        if (vec) fg_launch(ctx, prep_kernel<__nv_bfloat16, 8>, grid, block, 0, a);
+        else fg_launch(ctx, prep_kernel<__nv_bfloat16, 1>, grid, block, 0, a);
     }
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
@@ -1339,6 +1341,7 @@ __device__ __forceinline__ ConvOperand conv_operand(uint32_t t32, bool mn) {
 template <int BN>
 __global__ void __launch_bounds__(kConvThreads, 1)
 gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epilogue ep) {
+    fg_grid_enter();
     using Cfg = ConvCfg<BN>;
     constexpr int S = Cfg::kStages, BK = 32, CPT = BN / 2;
     extern __shared__ unsigned char smem_raw[];
@@ -1832,7 +1835,7 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     gemm_tc_pair_kernel<BK, FMT><<<grid, kPairThreads, Cfg::kSmemBytes, ctx->stream>>>(tmA, tmB, tmA16, tmB16, ep);
     FG_LAUNCHED(ctx);
     if (ep.split > 1) {
-        gemm_tc_fold_kernel<2 * BM, 256><<<(unsigned)((ntiles - ep.t_full) * 64), 256, 0, ctx->stream>>>(ep);
+        fg_launch(ctx, gemm_tc_fold_kernel<2 * BM, 256>, (unsigned)((ntiles - ep.t_full) * 64), 256, 0, ep);
         FG_LAUNCHED(ctx);
     }
     fg_time_end(ctx, tr);
@@ -1906,10 +1909,10 @@ int32_t launch_conv_bn(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, Epilog
     ep.batch = batch;
     ep.t_full = 0;
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, 2.0 * batch * ep.M * ep.N * ep.K);
-    gemm_tc_conv_kernel<BN><<<dim3((unsigned)tiles, ep.split, batch), kConvThreads, Cfg::kSmemBytes, ctx->stream>>>(tm[0], tm[1], ep);
+    fg_launch(ctx, gemm_tc_conv_kernel<BN>, dim3((unsigned)tiles, ep.split, batch), kConvThreads, Cfg::kSmemBytes, tm[0], tm[1], ep);
     FG_LAUNCHED(ctx);
     if (ep.split > 1) {
-        gemm_tc_fold_kernel<BM, BN><<<(unsigned)(tiles * batch * (BM / 32) * (BN / 32)), 256, 0, ctx->stream>>>(ep);
+        fg_launch(ctx, gemm_tc_fold_kernel<BM, BN>, (unsigned)(tiles * batch * (BM / 32) * (BN / 32)), 256, 0, ep);
         FG_LAUNCHED(ctx);
     }
     fg_time_end(ctx, tr);
@@ -2003,6 +2006,7 @@ int32_t tc_gemm(fg_ctx* ctx, int fmt, const PlaneSet& a, const PlaneSet& b, uint
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) pairs_kernel(const float* __restrict__ x, uint64_t n, __nv_bfloat16* __restrict__ pairs,
                                                     uint64_t plane_stride) {
+    fg_grid_enter();
     const uint64_t nv = n >> 2, stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride)
         fg_store_pairs4(pairs, plane_stride, i * 4, __ldcs(reinterpret_cast<const float4*>(x) + i));
@@ -2016,6 +2020,7 @@ __global__ void __launch_bounds__(256) pairs_kernel(const float* __restrict__ x,
 __global__ void __launch_bounds__(128) dz_pairs_kernel(uint32_t R, uint32_t C, const float* dy, const float* __restrict__ saved,
                                                        int act, float* dz, __nv_bfloat16* __restrict__ pairs,
                                                        uint64_t plane_stride, float* __restrict__ colsum_part) {
+    fg_grid_enter();
     const uint32_t c = (blockIdx.x * 128 + threadIdx.x) * 4;
     if (c >= C) return;
     const uint32_t r0 = blockIdx.y * 32, r1 = min(R, r0 + 32);
@@ -2034,7 +2039,7 @@ __global__ void __launch_bounds__(128) dz_pairs_kernel(uint32_t R, uint32_t C, c
 
 int32_t launch_pairs(fg_ctx* ctx, const float* x, uint64_t n, __nv_bfloat16* pairs, uint64_t plane_stride) {
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT, 8.0 * (double)n);
-    pairs_kernel<<<fg_stream_grid(ctx, (n + 3) / 4, 256, 8), 256, 0, ctx->stream>>>(x, n, pairs, plane_stride);
+    fg_launch(ctx, pairs_kernel, fg_stream_grid(ctx, (n + 3) / 4, 256, 8), 256, 0, x, n, pairs, plane_stride);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;
@@ -2045,7 +2050,7 @@ int32_t launch_dz_pairs(fg_ctx* ctx, uint32_t R, uint32_t C, const float* dy, co
     dim3 grid((C + 511) / 512, (R + 31) / 32);
     if (grid.y > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM operand has too many rows");
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT, 4.0 * R * C * (1.0 + (saved ? 1.0 : 0.0) + (dz ? 1.0 : 0.0) + (pairs ? 1.0 : 0.0)));
-    dz_pairs_kernel<<<grid, 128, 0, ctx->stream>>>(R, C, dy, saved, act, dz, pairs, plane_stride, colsum_part);
+    fg_launch(ctx, dz_pairs_kernel, grid, 128, 0, R, C, dy, saved, act, dz, pairs, plane_stride, colsum_part);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;

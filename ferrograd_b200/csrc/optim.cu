@@ -124,6 +124,7 @@ struct MultiArgs {
 template <bool ADAM, bool ZERO>
 __global__ void __launch_bounds__(256) update_multi_kernel(const __grid_constant__ MultiArgs a, AdamConsts c, uint32_t step,
                                                            const uint32_t* __restrict__ step_dev) {
+    fg_grid_enter();
     float inv_bc1 = 1.0f, inv_bc2 = 1.0f;
     if (ADAM) {
         const uint32_t t = step_dev ? *step_dev : step;
@@ -210,11 +211,11 @@ int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t
         const int grid = (int)std::min<uint64_t>(chunks, (uint64_t)ctx->sm_count * 8);
         fg_time_rec* tr = fg_time_begin(ctx, adam ? FG_KERNEL_ADAMW : FG_KERNEL_SGD, bytes);
         if (adam) {
-            if (zero_grad) update_multi_kernel<true, true><<<grid, 256, 0, ctx->stream>>>(a, c, step, step_dev);
-            else update_multi_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(a, c, step, step_dev);
+            if (zero_grad) fg_launch(ctx, update_multi_kernel<true, true>, grid, 256, 0, a, c, step, step_dev);
+            else fg_launch(ctx, update_multi_kernel<true, false>, grid, 256, 0, a, c, step, step_dev);
         } else {
-            if (zero_grad) update_multi_kernel<false, true><<<grid, 256, 0, ctx->stream>>>(a, c, step, step_dev);
-            else update_multi_kernel<false, false><<<grid, 256, 0, ctx->stream>>>(a, c, step, step_dev);
+            if (zero_grad) fg_launch(ctx, update_multi_kernel<false, true>, grid, 256, 0, a, c, step, step_dev);
+            else fg_launch(ctx, update_multi_kernel<false, false>, grid, 256, 0, a, c, step, step_dev);
         }
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);

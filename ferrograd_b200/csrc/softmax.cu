@@ -491,6 +491,7 @@ __device__ __forceinline__ void softmax_put(const CeArgs& a, size_t off, uint32_
 
 template <int MODE, int NV>
 __global__ void __launch_bounds__(256) softmax_warp_kernel(CeArgs a) {
+    fg_grid_enter();
     const uint32_t cols = a.cols, lane = threadIdx.x & 31u, step = gridDim.x * 8;
     for (uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5); row < a.rows; row += step) {
         const size_t base = (size_t)row * cols;
@@ -615,6 +616,7 @@ __global__ void __launch_bounds__(1024) softmax_edge_kernel(CeArgs a) {
 template <int NV>
 __global__ void __launch_bounds__(256) softmax_bwd_warp_kernel(uint32_t rows, uint32_t cols, const float* __restrict__ y,
                                                                const float* __restrict__ dy, float* __restrict__ dx, int accumulate) {
+    fg_grid_enter();
     const uint32_t lane = threadIdx.x & 31u, step = gridDim.x * 8;
     for (uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += step) {
         const size_t base = (size_t)row * cols + lane;
@@ -722,6 +724,7 @@ __global__ void softmax_bwd_kernel(uint32_t rows, uint32_t cols, const float* __
 // The reference's unfused per-element CE on probabilities.
 __global__ void ce_elem_kernel(const float* __restrict__ p, const uint32_t* __restrict__ labels, uint32_t rows,
                                uint32_t cols, float* __restrict__ loss, float* __restrict__ grad) {
+    fg_grid_enter();
     const uint64_t n = (uint64_t)rows * cols;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t r = (uint32_t)(i / cols), c = (uint32_t)(i - (uint64_t)r * cols);
@@ -734,6 +737,7 @@ __global__ void ce_elem_kernel(const float* __restrict__ p, const uint32_t* __re
 
 // Fixed-order mean of the per-row losses (one CTA).
 __global__ void mean_kernel(const float* __restrict__ x, uint32_t n, float* __restrict__ out) {
+    fg_grid_enter();
     __shared__ float red[32];
     float s = 0.0f, v[8];
     for (uint64_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {      // eight loads in flight, added in order
@@ -801,9 +805,9 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
     if (a.cols <= kWarpRowCols) {
         const int grid = rows_grid(ctx, ((uint64_t)a.rows + 7) / 8, 256);
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
-        if (a.cols <= 32) softmax_warp_kernel<MODE, 1><<<grid, 256, 0, ctx->stream>>>(a);
-        else if (a.cols <= 128) softmax_warp_kernel<MODE, 4><<<grid, 256, 0, ctx->stream>>>(a);
-        else softmax_warp_kernel<MODE, 16><<<grid, 256, 0, ctx->stream>>>(a);
+        if (a.cols <= 32) fg_launch(ctx, softmax_warp_kernel<MODE, 1>, grid, 256, 0, a);
+        else if (a.cols <= 128) fg_launch(ctx, softmax_warp_kernel<MODE, 4>, grid, 256, 0, a);
+        else fg_launch(ctx, softmax_warp_kernel<MODE, 16>, grid, 256, 0, a);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -866,9 +870,9 @@ int32_t fg_softmax_bwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* y
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, (accumulate ? 16.0 : 12.0) * rows * cols);
     if (cols <= kWarpRowCols) {
         const int grid = rows_grid(ctx, ((uint64_t)rows + 7) / 8, 256);
-        if (cols <= 32) softmax_bwd_warp_kernel<1><<<grid, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
-        else if (cols <= 128) softmax_bwd_warp_kernel<4><<<grid, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
-        else softmax_bwd_warp_kernel<16><<<grid, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
+        if (cols <= 32) fg_launch(ctx, softmax_bwd_warp_kernel<1>, grid, 256, 0, rows, cols, y, dy, dx, accumulate);
+        else if (cols <= 128) fg_launch(ctx, softmax_bwd_warp_kernel<4>, grid, 256, 0, rows, cols, y, dy, dx, accumulate);
+        else fg_launch(ctx, softmax_bwd_warp_kernel<16>, grid, 256, 0, rows, cols, y, dy, dx, accumulate);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -904,7 +908,7 @@ int32_t fg_softmax_ce_fwd_bwd(fg_ctx* ctx, const float* logits, const uint32_t* 
     int32_t s = launch_rows<1>(ctx, a);
     if (s != FG_OK) return s;
     if (loss_mean_out) {
-        mean_kernel<<<1, 1024, 0, ctx->stream>>>(loss_row_out, rows, loss_mean_out);
+        fg_launch(ctx, mean_kernel, 1, 1024, 0, loss_row_out, rows, loss_mean_out);
         FG_LAUNCHED(ctx);
     }
     return FG_OK;
@@ -917,7 +921,7 @@ int32_t fg_ce_loss_grad(fg_ctx* ctx, const float* probs, const uint32_t* labels,
     FG_REQUIRE(ctx, cols >= 1, "fg_ce_loss_grad: cols must be >= 1");
     if (rows == 0) return FG_OK;
     int grid = fg_stream_grid(ctx, (uint64_t)rows * cols, 256, 8);
-    ce_elem_kernel<<<grid, 256, 0, ctx->stream>>>(probs, labels, rows, cols, loss_out, grad_out);
+    fg_launch(ctx, ce_elem_kernel, grid, 256, 0, probs, labels, rows, cols, loss_out, grad_out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
