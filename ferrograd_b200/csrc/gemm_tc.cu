@@ -1253,13 +1253,13 @@ int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 
 // The pair kernel needs bf16 pairs in HBM and works in 256 x 256 tiles on two SMs; a product of a
 // few such tiles leaves most SMs idle, and making the pairs of a tensor that is read once costs
 // as much as reading it twice more.  Here a CTA owns a 128 x BN tile, loads the raw f32 words of
-// both operands (half the bytes of tensor plus pairs) and eight converter warps write the bf16
+// both operands (half the bytes of tensor plus pairs) and converter warps write the bf16
 // planes of each k-block beside it in shared memory, in the layout a bulk-tensor load would have
 // given them.  A matrix index and a K-share ride in the grid, so that one launch covers a batch and
 // fills the SMs; K-shares are folded by gemm_tc_fold_kernel.
-//   warp 0 loads, warp 1 issues MMAs, warps 2..9 drain accumulators and store, warps 10..17 convert.
-// Measured (before: operand planes or pairs, then a 256 x 256 or 128-row tile each): 100 x 4096 x 4096 129 -> 43 us,
-// 16 x (384 x 512 x 320) forward and backward 1528 -> 101 us, a 384-sample layer of 256 x 256 21.7 -> 9.8 us per product.
+//   warp 0 loads, warp 1 issues MMAs, warps 2..9 drain accumulators and store, the others convert.
+// Measured (before: operand planes or pairs, then a 256 x 256 or 128-row tile each): 100 x 4096 x 4096 129 -> 36 us,
+// 16 x (384 x 512 x 320) forward and backward 1530 -> 87 us, a 384-sample layer of 256 x 256 21.7 -> 9.8 us per product.
 // Bound by the converters and shared-memory bandwidth: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB
 // into the converters, 64 KB out of them and 64 KB into the MMAs, 192 KB at 128 B per cycle.
 // ------------------------------------------------------------------------------------
@@ -1268,25 +1268,33 @@ struct ConvCfg {
     static constexpr int kA32 = BM * 32 * 4, kB32 = BN * 32 * 4;    // f32 tiles; the two bf16 planes take as much again
     static constexpr int kStageBytes = 2 * (kA32 + kB32);
     static constexpr int kStages = BN == 128 ? 3 : 4;
+    // Converters: all eight warps on each k-block in turn (BN = 128), or two per stage (BN = 64), see the kernel.
+    static constexpr int kGroups = BN == 128 ? 1 : kStages, kGroup = 256 / kGroups;
+    static constexpr int kThreads = 320 + 256;
     static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
     static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
     static_assert(kStageBytes >= 8 * 32 * 32 * 4, "the epilogue stages its blocks in the first stage");
     static constexpr int kTmemCols = 2 * BN;
 };
-constexpr int kConvThreads = 576;
 
-// The split of a tile of ROWS rows x 32 k, eight elements per thread and step (256 threads): the words are rounded to tf32
+// The split of a tile of ROWS rows x 32 k, eight elements per thread and step: the words are rounded to tf32
 // in place (hi; an MMA would truncate them, which doubles what the cross terms have to carry: 1.9e-6 against 1.5e-6 of the
 // result's 2-norm), the planes are bf16(x) and bf16(x - hi).
 // K-major f32: rows of 128 bytes, 16-byte chunk c of row r at c ^ (r & 7); bf16: planes of [ROWS][64 bytes], chunk c of row
 // r at c ^ (r / 2 & 3).  MN-major f32: blocks of 32 rows, [k][128 bytes] each, 32-byte chunk j of k-row k at j ^ (k & 3);
 // bf16: blocks of 64 rows, [plane][k][128 bytes] each, 16-byte chunk c of k-row k at c ^ (k & 7).
 // Lanes are dealt so that the 128-bit accesses of eight lanes fall into different banks.
-template <int ROWS>
+// Nearest tf32 value, ties away from zero (cvt.rna), in two integer operations: the conversion unit is a fraction as wide.
+// A NaN may lose its payload here; the planes keep the product NaN.
+__device__ __forceinline__ float4 round_tf32(float4 v) {
+    auto r = [](float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); };
+    return make_float4(r(v.x), r(v.y), r(v.z), r(v.w));
+}
+template <int ROWS, int GROUP>
 __device__ __forceinline__ void convert_tile(unsigned char* t32, bool mn, uint32_t ct) {
     unsigned char* const t16 = t32 + ROWS * 128;
-#pragma unroll
-    for (uint32_t o = ct; o < ROWS * 4; o += 256) {
+#pragma unroll 2
+    for (uint32_t o = ct; o < ROWS * 4; o += GROUP) {
         unsigned char *s0, *s1, *h, *l;
         bool swap = false;
         if (!mn) {
@@ -1305,11 +1313,13 @@ __device__ __forceinline__ void convert_tile(unsigned char* t32, bool mn, uint32
             l = h + 4096;
         }
         const float4 p = *reinterpret_cast<const float4*>(s0), q4 = *reinterpret_cast<const float4*>(s1);
-        const Split4 sp = split4<1>(p), sq = split4<1>(q4);
-        *reinterpret_cast<float4*>(s0) = sp.hi;
-        *reinterpret_cast<float4*>(s1) = sq.hi;
-        const uint2 h0 = pack_bf16x4(swap ? q4 : p), h1 = pack_bf16x4(swap ? p : q4);
-        const uint2 l0 = pack_bf16x4(swap ? sq.lo : sp.lo), l1 = pack_bf16x4(swap ? sp.lo : sq.lo);
+        const float4 ph = round_tf32(p), qh = round_tf32(q4);
+        *reinterpret_cast<float4*>(s0) = ph;
+        *reinterpret_cast<float4*>(s1) = qh;
+        const uint2 hp = pack_bf16x4(p), hq = pack_bf16x4(q4);
+        const uint2 lp = pack_bf16x4(make_float4(p.x - ph.x, p.y - ph.y, p.z - ph.z, p.w - ph.w));
+        const uint2 lq = pack_bf16x4(make_float4(q4.x - qh.x, q4.y - qh.y, q4.z - qh.z, q4.w - qh.w));
+        const uint2 h0 = swap ? hq : hp, h1 = swap ? hp : hq, l0 = swap ? lq : lp, l1 = swap ? lp : lq;
         *reinterpret_cast<uint4*>(h) = make_uint4(h0.x, h0.y, h1.x, h1.y);
         *reinterpret_cast<uint4*>(l) = make_uint4(l0.x, l0.y, l1.x, l1.y);
     }
@@ -1339,7 +1349,7 @@ __device__ __forceinline__ ConvOperand conv_operand(uint32_t t32, bool mn) {
 }
 
 template <int BN>
-__global__ void __launch_bounds__(kConvThreads, 1)
+__global__ void __launch_bounds__(ConvCfg<BN>::kThreads, 1)
 gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epilogue ep) {
     fg_grid_enter();
     using Cfg = ConvCfg<BN>;
@@ -1373,7 +1383,7 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (s_abort != 0) return;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(conv_bar(s), 8); mbar_init(empty_bar(s), 1); }
+        for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(conv_bar(s), Cfg::kGroup / 32); mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full_bar(b), 1); mbar_init(acc_empty_bar(b), 8); }
         fence_mbar_init();
         prefetch_tmap(&tmA);
@@ -1451,18 +1461,23 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
         }
     } else if (warp >= 10) {
-        // ---- converters ----
-        const uint32_t ct = threadIdx.x - 320;
-        for (uint32_t i = 0; i < nkb; ++i) {
+        // ---- converters.  With a group per stage one's waits (for the loads, shared memory and the proxy fence) pass under
+        // the others' work: 128 x 64 tiles 0.71 -> 0.6 us per k-block, the 200-256-256-10 step 97 -> 89 us; with 128 x 128 tiles
+        // three groups of three warps lost 9 % against all eight warps together.  Either every group takes every k-block or
+        // every stage belongs to one group: a stage is then refilled only after its group has converted it, so that no wait,
+        // which names a phase by its parity alone, can meet the phase before or after the one it means. ----
+        static_assert(Cfg::kGroups == 1 || Cfg::kGroups == S, "see above");
+        const uint32_t ct = (threadIdx.x - 320) % Cfg::kGroup;
+        for (uint32_t i = (threadIdx.x - 320) / Cfg::kGroup; i < nkb; i += Cfg::kGroups) {
             const int s = i % S;
+            unsigned char* const sa = base_ptr + s * Cfg::kStageBytes;
             const bool got = mbar_wait_bounded(full_bar(s), (i / S) & 1u, kWaitCycles);
             if (!__all_sync(0xffffffffu, got)) {
                 if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
                 break;
             }
-            unsigned char* const sa = base_ptr + s * Cfg::kStageBytes;
-            convert_tile<BM>(sa, a_mn, ct);
-            convert_tile<BN>(sa + 2 * Cfg::kA32, b_mn, ct);
+            convert_tile<BM, Cfg::kGroup>(sa, a_mn, ct);
+            convert_tile<BN, Cfg::kGroup>(sa + 2 * Cfg::kA32, b_mn, ct);
             fence_proxy_async();        // the planes are read by the tensor core
             __syncwarp();
             if (lane == 0) mbar_arrive(conv_bar(s));
@@ -1855,8 +1870,11 @@ ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32
         const uint64_t tiles = (uint64_t)((M + BM - 1) / BM) * ((N + bn - 1) / bn) * batch;
         for (uint64_t split = 1; split <= 16 && (split == 1 || (split * 4 <= nkb && tiles * split <= 2 * sms)); ++split) {
             const uint64_t waves = (tiles * split + sms - 1) / sms, kb = (nkb + split - 1) / split;
-            double c = (double)waves * ((double)kb * (bn == 128 ? 1300.0 : 950.0) + 6000.0);
-            if (split > 1) c += 5000.0 + (double)(tiles * split) * BM * bn * 4.0 / 2000.0;      // the fold's launch and its reads
+            // measured slopes and offsets: 0.9 and 0.6 us per k-block, 7.2 and 5.3 us around them; a ragged N stored straight
+            // from the tiles, element by element, 6 us more; the fold 2 us and 4.3 TB/s
+            double c = (double)waves * ((double)kb * (bn == 128 ? 1700.0 : 1150.0) + (bn == 128 ? 13000.0 : 9800.0) +
+                                        (split == 1 && N % 4 != 0 ? 11000.0 : 0.0));
+            if (split > 1) c += 3700.0 + (double)(tiles * split) * BM * bn * 4.0 / 2300.0;
             if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, (uint32_t)split, c};
         }
     }
@@ -1869,7 +1887,7 @@ uint64_t conv_partial_bytes(const ConvPlan& p, uint32_t M, uint32_t N, uint32_t 
 // The pair kernel for one matrix: 256 x 256 tiles on SM pairs, plus the passes that make the pairs of `prep` elements.
 double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double prep_elems, int prep_launches) {
     const uint64_t pairs = (uint64_t)ctx->sm_count / 2, tiles = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
-    const double tile = (double)((K + 31) / 32) * 1150.0, whole = (double)(tiles / pairs) * tile;
+    const double tile = (double)((K + 31) / 32) * 1250.0, whole = (double)(tiles / pairs) * tile;
     const uint64_t rem = tiles % pairs;
     double tail = rem ? tile : 0.0;
     const uint64_t nchunks = (K + kChunkK - 1) / kChunkK;
@@ -1877,7 +1895,8 @@ double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double
     if (split > nchunks / 2) split = nchunks / 2;
     if (split > 4) split = 4;
     if (split >= 2 && ctx->opt_split_k) tail = tail / (double)split + 8000.0;
-    return whole + tail + 9000.0 + prep_elems * 8.0 / 2500.0 + 4000.0 * prep_launches;
+    // (512 x 512 x 512: 22 us of which the products are 9; set-up and the last tile's epilogue are the rest)
+    return whole + tail + 23000.0 + prep_elems * 8.0 / 2500.0 + 3700.0 * prep_launches;
 }
 inline bool conv_allowed(const fg_ctx* ctx) { return ctx->opt_pairs && ctx->opt_tile_pair < 0 && ctx->tmap_encode; }
 
@@ -1909,7 +1928,7 @@ int32_t launch_conv_bn(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, Epilog
     ep.batch = batch;
     ep.t_full = 0;
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, 2.0 * batch * ep.M * ep.N * ep.K);
-    fg_launch(ctx, gemm_tc_conv_kernel<BN>, dim3((unsigned)tiles, ep.split, batch), kConvThreads, Cfg::kSmemBytes, tm[0], tm[1], ep);
+    fg_launch(ctx, gemm_tc_conv_kernel<BN>, dim3((unsigned)tiles, ep.split, batch), Cfg::kThreads, Cfg::kSmemBytes, tm[0], tm[1], ep);
     FG_LAUNCHED(ctx);
     if (ep.split > 1) {
         fg_launch(ctx, gemm_tc_fold_kernel<BM, BN>, (unsigned)(tiles * batch * (BM / 32) * (BN / 32)), 256, 0, ep);
@@ -2559,7 +2578,13 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
         const BwdRoutes rt = pick_bwd_routes(ctx, M, N, K, PairedArg{A, nullptr, 0}, PairedArg{B, nullptr, 0}, PairedArg{z_like, nullptr, 0}, dB, dA, nullptr);
         const bool want_pairs = (dB && rt.dB.kind == kRoutePair) || (dA && rt.dA.kind == kRoutePair);
         if (!rt.planes && (!want_pairs || vec_z)) {
-            const uint64_t need = bwd_paired_need(M, N, K) + (uint64_t)M * round4(N) * 4 + mn * 4 + (uint64_t)cs_chunks * N * 4 + 1024;
+            uint64_t need = (uint64_t)cs_chunks * N * 4 + 2048;
+            if (want_pairs) need += bwd_paired_need(M, N, K) + mn * 4;
+            else {       // never more than the operand planes of these shapes would take
+                if (own_z) need += (uint64_t)M * round4(N) * 4 + 256;
+                if (dB) need += copy32_bytes(A, M, K, 1, 0) + conv_partial_bytes(rt.dB.conv, K, N, 1);
+                if (dA) need += copy32_bytes(B, K, N, 1, 0) + conv_partial_bytes(rt.dA.conv, M, K, 1);
+            }
             { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
             int32_t s;
             void *pz = nullptr, *dzb = nullptr, *csp = nullptr;
@@ -2605,6 +2630,14 @@ bool batch_converts(const fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, u
     *p = plan_conv(ctx, M, N, K, batch);
     const double elems = (double)M * K + (double)K * N;
     return p->cycles <= (double)batch * pair_cycles(ctx, M, N, K, pair_ok ? elems : 2.0 * elems, 2);
+}
+
+// Scratch for a whole batch.  Where it cannot be had (out of memory, or a recording whose arena was sized for less), the
+// loop over the matrices, which needs one matrix's worth, takes its place.
+bool batch_scratch(fg_ctx* ctx, uint64_t bytes) {
+    if (fg_ws_ensure(ctx, bytes) == FG_OK) return true;
+    cudaGetLastError();
+    return false;
 }
 
 }  // namespace
@@ -2680,13 +2713,15 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
         if (batch_converts(ctx, batch, M, N, K, paired_shape_ok(ctx, M, N, K, K, N), &cp)) {
             const uint64_t need = copy32_bytes(A, M, K, batch, strideA) + copy32_bytes(B, K, N, batch, strideB) +
                                   conv_partial_bytes(cp, M, N, batch) + 1024;
-            int32_t s = fg_ws_ensure(ctx, need);
-            PlaneSet pa, pb;
-            if (s != FG_OK || (s = loadable32(ctx, A, M, K, batch, strideA, &pa)) != FG_OK) return s;
-            if ((s = loadable32(ctx, B, K, N, batch, strideB, &pb)) != FG_OK) return s;
-            Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
-            ep.c_batch = strideC;
-            return launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, cp, batch);
+            if (batch_scratch(ctx, need)) {
+                int32_t s;
+                PlaneSet pa, pb;
+                if ((s = loadable32(ctx, A, M, K, batch, strideA, &pa)) != FG_OK) return s;
+                if ((s = loadable32(ctx, B, K, N, batch, strideB, &pb)) != FG_OK) return s;
+                Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
+                ep.c_batch = strideC;
+                return launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, cp, batch);
+            }
         }
     }
     const bool dense = strideA == (uint64_t)M * K && strideB == (uint64_t)K * N;
@@ -2760,14 +2795,13 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
         const bool n8 = N % 8 == 0 && K % 8 == 0;
         const bool all = (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N), &cb)) &&
                          (!dA || batch_converts(ctx, batch, M, K, N, n8 && paired_shape_ok(ctx, M, K, N, N, N), &ca));
-        if (all) {
-            // dZ for the whole batch in one pass, then one launch per product
-            const bool own_z = act != FG_ACT_NONE;
-            const uint64_t need = (own_z ? (uint64_t)batch * M * round4(N) * 4 + 256 : copy32_bytes(dY, M, N, batch, strideC)) +
-                                  (dB ? copy32_bytes(A, M, K, batch, strideA) + conv_partial_bytes(cb, K, N, batch) : 0) +
-                                  (dA ? copy32_bytes(B, K, N, batch, strideB) + conv_partial_bytes(ca, M, K, batch) : 0) + 2048;
-            int32_t s = fg_ws_ensure(ctx, need);
-            if (s != FG_OK) return s;
+        // dZ for the whole batch in one pass, then one launch per product
+        const bool own_z = act != FG_ACT_NONE;
+        const uint64_t need = (own_z ? (uint64_t)batch * M * round4(N) * 4 + 256 : copy32_bytes(dY, M, N, batch, strideC)) +
+                              (dB ? copy32_bytes(A, M, K, batch, strideA) + conv_partial_bytes(cb, K, N, batch) : 0) +
+                              (dA ? copy32_bytes(B, K, N, batch, strideB) + conv_partial_bytes(ca, M, K, batch) : 0) + 2048;
+        if (all && batch_scratch(ctx, need)) {
+            int32_t s;
             PlaneSet z, x;
             if (own_z) {
                 void* p;
