@@ -638,7 +638,7 @@ def run_ours(args, rank, world, local_rank):
             "e2e": {"value": gb * args.steps / (e2e_ms / 1e3), "unit": "samples/s", "ms_per_step": e2e_ms / args.steps,
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "tensor", "kernel": "gemm_tc_pair_kernel (+ gemm_tc_pair_fold_kernel)", "achieved": ach,
+            "roofline": {"bound": "tensor", "kernel": "gemm_tc_pair_kernel (+ gemm_tc_fold_kernel)", "achieved": ach,
                          "peak": own_peak, "unit": "TFLOP/s", "frac": ach / own_peak if own_peak else None,
                          "traffic": gemm_traffic_per_launch(args.workload),
                          "launches": int(gemm_n), "avg_launch_ms": gemm_ms / max(gemm_n, 1),
