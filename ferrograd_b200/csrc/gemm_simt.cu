@@ -640,7 +640,7 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
     if (N > SKN) return fg_fail(ctx, FG_ERR_INTERNAL, "skinny GEMM: N too large");
     // One chunk of rows: the exact path's kernel adds the same products in the same order and needs no fold (64 x 2 x 16: one
     // launch of 3 us instead of two of 11 + 2 us).
-    if (M <= TN_ROWS) return fg_gemm_simt_launch(ctx, 1, 0, Kd, N, M, A, dZ, dB, nullptr, FG_ACT_NONE, nullptr);
+    if (M <= TN_ROWS && Kd <= 65535u * 64u) return fg_gemm_simt_launch(ctx, 1, 0, Kd, N, M, A, dZ, dB, nullptr, FG_ACT_NONE, nullptr);
     // block rows: as many as the SMs hold at once (four blocks of 128 threads per SM), at most one per chunk
     const uint32_t gx = (Kd + 511) / 512, chunk = tn_chunk_rows(M, Kd);
     uint32_t nchunks = (uint32_t)(4ull * ctx->sm_count / gx);

@@ -2565,7 +2565,8 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, !dB || A, "fg_gemm_bwd_f32: dB needs A");
     const bool fuse = act != FG_ACT_NONE;
     const int path = pick_path(ctx, mode, M, N, K);
-    if (path == 2 && N > 16 && (dA || dB)) {
+    // (prep_kernel takes up to 65535 * 32 rows, the planes twice as many)
+    if (path == 2 && N > 16 && (dA || dB) && M <= 65535u * 32u) {
         // dZ (with its pairs, if a product needs them) and the bias gradient's partials in one pass, then both products
         // from the tensors themselves
         const uint64_t mn = (uint64_t)M * N;
@@ -2793,7 +2794,7 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
     if (pick_path(ctx, mode, M, N, K) == 2 && (N > 16 || mode != FG_GEMM_AUTO)) {
         ConvPlan cb{}, ca{};
         const bool n8 = N % 8 == 0 && K % 8 == 0;
-        const bool all = (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N), &cb)) &&
+        const bool all = M <= 65535u * 32u && (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N), &cb)) &&
                          (!dA || batch_converts(ctx, batch, M, K, N, n8 && paired_shape_ok(ctx, M, K, N, N, N), &ca));
         // dZ for the whole batch in one pass, then one launch per product
         const bool own_z = act != FG_ACT_NONE;
