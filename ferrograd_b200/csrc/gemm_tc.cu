@@ -925,7 +925,8 @@ __global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
         }
         const size_t off = bz * ep.c_batch + (size_t)row * ep.N + col;
         const bool vec_ok = (ep.N % 4 == 0) && (ep.c_batch % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
-                            (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0);
+                            (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0) &&
+                            (!ep.mul_saved || (reinterpret_cast<uintptr_t>(ep.mul_saved) & 15u) == 0);
         if (vec_ok && col + 3 < ep.N) {
             const float4 zin = make_float4(zz[0], zz[1], zz[2], zz[3]);
             float4 o;

@@ -109,3 +109,22 @@ def test_batched(ctx, oracle, T, M, N, K, gap):
         check(a(gB, t, (K, N)), oracle.gemm(At, dz, transA=True, f64=True), TOL, f"dB {t}")
     if gap:                         # what lies between the matrices is not touched
         assert (got[:, M * N:] == 7.0).all() and (gA[:, M * K:] == 7.0).all() and (gB[:, K * N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("shift_saved,shift_out", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(128, 512, 512), (100, 256, 1024), (384, 256, 256), (512, 128, 384)])
+def test_backward_onto_the_layer_below(ctx, oracle, M, N, K, shift_saved, shift_out):
+    # dA * act'(saved) and its column sums in the epilogue, or in the fold when K is cut into shares; the layer below's tensor
+    # and dA may start one element off a 16-byte boundary
+    r = rng(M + N + K)
+    A, B = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    dZ, saved = r.standard_normal((M, N), np.float32), np.tanh(r.standard_normal((M, K))).astype(np.float32)
+    place = lambda a, shift: up(ctx, np.concatenate([np.zeros(shift, np.float32), a.ravel()]))          # noqa: E731
+    S, dA = place(saved, shift_saved), place(np.zeros((M, K), np.float32), shift_out)
+    dB, below = ctx.new_tensor((K, N)), ctx.new_tensor((K,))
+    ctx.gemm_bwd_paired(up(ctx, A), up(ctx, B), up(ctx, dZ), M, N, K, dB=dB, dA=dA.ptr + 4 * shift_out, below_act="tanh",
+                        below_saved=S.ptr + 4 * shift_saved, below_dbias=below)
+    want = oracle.gemm(dZ, B, transB=True, f64=True) * (1.0 - saved.astype(np.float64) ** 2)
+    check(ctx.to_numpy(dA)[shift_out:].reshape(M, K), want, TOL, "dA")
+    check(ctx.to_numpy(dB), oracle.gemm(A, dZ, transA=True, f64=True), TOL, "dB")
+    check(ctx.to_numpy(below), want.sum(0), TOL, "bias gradient of the layer below")
