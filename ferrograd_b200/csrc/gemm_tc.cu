@@ -1226,7 +1226,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepArgs a) {
 // a.out, when given, is scratch: 16-byte aligned with a 16-byte pitch.
 int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 1) {
     const uint32_t per16 = dtype == FG_DTYPE_F32 ? 4 : 8;
-    const bool vec = a.C % per16 == 0 && a.x_batch % per16 == 0 && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved)) &&
+    const bool vec = a.C % per16 == 0 && (batch == 1 || a.x_batch % per16 == 0) && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved)) &&
                      (!a.copy || fg_aligned16(a.copy));
     const uint32_t w = 32 * (vec ? per16 : 1);
     dim3 grid((a.C + w - 1) / w, (a.R + 31) / 32, batch), block(32, 8);
@@ -1964,7 +1964,7 @@ int32_t loadable32(fg_ctx* ctx, const float* x, uint32_t R, uint32_t C, uint32_t
     *o = PlaneSet{};
     o->p32 = const_cast<float*>(x);
     o->ld32 = C;
-    o->batch32 = x_batch;
+    o->batch32 = batch > 1 ? x_batch : 0;      // one matrix: its stride need not suit a tensor map
     if (in_place32(x, C, batch, x_batch)) return FG_OK;
     void* p;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)batch * R * round4(C) * 4, &p);
@@ -2721,7 +2721,7 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
                 if ((s = loadable32(ctx, A, M, K, batch, strideA, &pa)) != FG_OK) return s;
                 if ((s = loadable32(ctx, B, K, N, batch, strideB, &pb)) != FG_OK) return s;
                 Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
-                ep.c_batch = strideC;
+                ep.c_batch = batch > 1 ? strideC : 0;
                 return launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, cp, batch);
             }
         }
@@ -2819,13 +2819,13 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
             if (dB) {
                 if ((s = loadable32(ctx, A, M, K, batch, strideA, &x)) != FG_OK) return s;
                 Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
-                ep.c_batch = strideB;
+                ep.c_batch = batch > 1 ? strideB : 0;
                 if ((s = launch_conv(ctx, as_operand(x, true), as_operand(z, true), ep, cb, batch)) != FG_OK) return s;
             }
             if (dA) {
                 if ((s = loadable32(ctx, B, K, N, batch, strideB, &x)) != FG_OK) return s;
                 Epilogue ep{dA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
-                ep.c_batch = strideA;
+                ep.c_batch = batch > 1 ? strideA : 0;
                 if ((s = launch_conv(ctx, as_operand(z, false), as_operand(x, false), ep, ca, batch)) != FG_OK) return s;
             }
             return FG_OK;

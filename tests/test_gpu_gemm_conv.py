@@ -84,8 +84,9 @@ def test_unaligned_operands(ctx, oracle):
     check(ctx.to_numpy(C)[1:].reshape(M, N), oracle.gemm(A, B, f64=True), TOL, "unaligned")
 
 
-@pytest.mark.parametrize("T,M,N,K", [(2, 64, 256, 256), (5, 130, 100, 333), (16, 384, 320, 512), (3, 65, 515, 1024), (40, 64, 64, 1100)])
-@pytest.mark.parametrize("gap", [0, 4, 6])
+@pytest.mark.parametrize("T,M,N,K", [(1, 64, 256, 256), (1, 130, 100, 333), (2, 64, 256, 256), (5, 130, 100, 333), (16, 384, 320, 512),
+                                     (3, 65, 515, 1024), (40, 64, 64, 1100)])
+@pytest.mark.parametrize("gap", [0, 1, 4, 6])
 def test_batched(ctx, oracle, T, M, N, K, gap):
     # gap: elements between the matrices of a batch beyond their own size
     r = rng(T + M + N + K + gap)
