@@ -2634,6 +2634,12 @@ bool batch_converts(const fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, u
     return p->cycles <= (double)batch * pair_cycles(ctx, M, N, K, pair_ok ? elems : 2.0 * elems, 2);
 }
 
+// Arguments that the per-matrix entry points refuse (an unknown mode, K = 0) are left to the loop, which asks them.
+bool batch_route_open(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_t K) {
+    return mode >= FG_GEMM_AUTO && mode <= FG_GEMM_TF32_BF16X2 && K >= 1 && pick_path(ctx, mode, M, N, K) == 2 &&
+           (N > 16 || mode != FG_GEMM_AUTO);
+}
+
 // Scratch for a whole batch.  Where it cannot be had (out of memory, or a recording whose arena was sized for less), the
 // loop over the matrices, which needs one matrix's worth, takes its place.
 bool batch_scratch(fg_ctx* ctx, uint64_t bytes) {
@@ -2710,7 +2716,7 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
     if (batch == 0 || (uint64_t)M * N == 0) return FG_OK;
     if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && K > 0)
         return fg_gemm_simt_batched_launch(ctx, 0, 0, batch, M, N, K, A, strideA, B, strideB, C, strideC, bias, act, preact_out);
-    if (pick_path(ctx, mode, M, N, K) == 2 && (N > 16 || mode != FG_GEMM_AUTO)) {
+    if (batch_route_open(ctx, mode, M, N, K)) {
         ConvPlan cp;
         if (batch_converts(ctx, batch, M, N, K, paired_shape_ok(ctx, M, N, K, K, N), &cp)) {
             const uint64_t need = copy32_bytes(A, M, K, batch, strideA) + copy32_bytes(B, K, N, batch, strideB) +
@@ -2792,7 +2798,7 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
                                                    FG_ACT_NONE, nullptr)) != FG_OK) return s;
         return FG_OK;
     }
-    if (pick_path(ctx, mode, M, N, K) == 2 && (N > 16 || mode != FG_GEMM_AUTO)) {
+    if (batch_route_open(ctx, mode, M, N, K)) {
         ConvPlan cb{}, ca{};
         const bool n8 = N % 8 == 0 && K % 8 == 0;
         const bool all = M <= 65535u * 32u && (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N), &cb)) &&

@@ -129,3 +129,18 @@ def test_backward_onto_the_layer_below(ctx, oracle, M, N, K, shift_saved, shift_
     check(ctx.to_numpy(dA)[shift_out:].reshape(M, K), want, TOL, "dA")
     check(ctx.to_numpy(dB), oracle.gemm(A, dZ, transA=True, f64=True), TOL, "dB")
     check(ctx.to_numpy(below), want.sum(0), TOL, "bias gradient of the layer below")
+
+
+def test_batched_refuses_what_one_product_refuses(ctx):
+    # an unknown mode and a contraction over nothing: an argument error as from the per-matrix calls, before any launch
+    from ferrograd_b200.backend import GEMM_MODE
+    M, N, K, T = 256, 256, 256, 4
+    t = ctx.new_tensor((T * 256 * 256,))
+    p = t.ptr
+    before = ctx.launch_count()
+    for mode, k in ((7, K), (-1, K), (GEMM_MODE["tf32_bf16x2"], 0)):
+        one = ctx.lib.fg_gemm_f32(ctx.handle, mode, 0, 0, M, N, k, p, p, p, None, 0, None)
+        assert one != 0
+        assert ctx.lib.fg_gemm_batched_f32(ctx.handle, mode, T, M, N, k, p, M * k, p, k * N, p, M * N, None, 0, None) == one
+        assert ctx.lib.fg_gemm_batched_bwd_f32(ctx.handle, mode, T, M, N, k, p, M * k, p, k * N, p, M * N, 0, None, p, p) == one
+    assert ctx.launch_count() == before
