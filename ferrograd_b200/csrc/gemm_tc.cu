@@ -2422,39 +2422,45 @@ uint64_t bwd_paired_need(uint32_t M, uint32_t N, uint32_t K) {
 
 struct BwdRoutes {
     Route dB, dA;
-    bool planes;      // a wanted product takes the planes route: both do
+    bool planes;      // every wanted product runs from operand planes
 };
+// Both wanted products may take the pair kernel or neither: its main term is truncated where the planes and the conversion
+// kernel round it (1.9e-6 against 1.5e-6 of the result's 2-norm), and a layer with one product that the pair kernel cannot
+// run keeps the smaller error in both.  Between planes and conversion each product follows its estimate: 128 x 8192 x 8192
+// 290 us, against 414 with both converted and 458 with both from planes.
 BwdRoutes pick_bwd_routes(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, const float* dB,
                           const float* dA, const float* mul_saved) {
     BwdRoutes r{};
     const double mk = (double)M * K, kn = (double)K * N, mn = (double)M * N;
-    const bool tc = pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 2, n8 = N % 8 == 0 && K % 8 == 0;
+    const bool n8 = N % 8 == 0 && K % 8 == 0 && fg_aligned16(dZ.x);
+    const bool pair = (!dB || (n8 && fg_aligned16(A.x) && fg_aligned16(dB) && paired_shape_ok(ctx, K, N, M, K, N))) &&
+                      (!dA || (n8 && fg_aligned16(B.x) && fg_aligned16(dA) && (!mul_saved || fg_aligned16(mul_saved)) &&
+                               paired_shape_ok(ctx, M, K, N, N, N)));
+    const bool tc = pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 2;
     const bool cz = !in_place32(dZ.x, N, 1, 0);
-    // a pair product of any wanted gradient that cannot run sends both to the planes, as long as the other cannot be converted
-    if (dB) {
-        const bool pair = n8 && fg_aligned16(A.x) && fg_aligned16(dB) && fg_aligned16(dZ.x) && paired_shape_ok(ctx, K, N, M, K, N);
-        const bool ca = !in_place32(A.x, K, 1, 0);
-        r.dB = (tc || pair) ? pick_route(ctx, K, N, M, pair, (A.pairs ? 0.0 : mk) + (dZ.pairs ? 0.0 : mn), !A.pairs + !dZ.pairs,
-                                         (ca ? mk : 0.0) + (cz ? mn : 0.0), ca + cz) : Route{kRoutePlanes, ConvPlan{}};
-        r.planes |= r.dB.kind == kRoutePlanes;
-    }
-    if (dA) {
-        const bool pair = n8 && fg_aligned16(B.x) && fg_aligned16(dA) && fg_aligned16(dZ.x) && (!mul_saved || fg_aligned16(mul_saved)) &&
-                          paired_shape_ok(ctx, M, K, N, N, N);
-        const bool cb = !in_place32(B.x, N, 1, 0);
-        r.dA = (tc || pair) ? pick_route(ctx, M, K, N, pair, (B.pairs ? 0.0 : kn) + (dZ.pairs ? 0.0 : mn), !B.pairs + !dZ.pairs,
-                                         (cb ? kn : 0.0) + (cz ? mn : 0.0), cb + cz) : Route{kRoutePlanes, ConvPlan{}};
-        r.planes |= r.dA.kind == kRoutePlanes;
-    }
+    bool all = true, any = false;       // of the wanted products, from planes
+    auto pick = [&](uint32_t m, uint32_t n, uint32_t k, double elems, bool pairs, bool copied) {
+        const Route x = (tc || pair) ? pick_route(ctx, m, n, k, pair, (pairs ? 0.0 : elems) + (dZ.pairs ? 0.0 : mn), !pairs + !dZ.pairs,
+                                                  (copied ? elems : 0.0) + (cz ? mn : 0.0), copied + cz) : Route{kRoutePlanes, ConvPlan{}};
+        all &= x.kind == kRoutePlanes;
+        any |= x.kind == kRoutePlanes;
+        return x;
+    };
+    if (dB) r.dB = pick(K, N, M, mk, A.pairs != nullptr, !in_place32(A.x, K, 1, 0));
+    if (dA) r.dA = pick(M, K, N, kn, B.pairs != nullptr, !in_place32(B.x, N, 1, 0));
+    // a dZ of padded pitch, as the conversion kernel would have it, cannot be split into planes
+    r.planes = all || (any && N % 4 != 0);
     return r;
 }
 
-// The two products of a backward step by their routes; dZ has row pitch ldz (N, or padded for the conversion kernel).
+// The two products of a backward step by their routes; dZ has row pitch ldz (N, or padded for the conversion kernel).  The
+// caller has reserved what they carve.
 int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, uint32_t ldz,
                           const BwdRoutes& rt, float* dB, float* dA, const PairedOut& o, float* exch_buf, uint64_t exch_count) {
     int32_t s;
     const uint64_t mk = (uint64_t)M * K, kn = (uint64_t)K * N, mn = (uint64_t)M * N;
     const bool pair_b = dB && rt.dB.kind == kRoutePair, pair_a = dA && rt.dA.kind == kRoutePair;
+    const bool conv_b = dB && rt.dB.kind == kRouteConv, conv_a = dA && rt.dA.kind == kRouteConv;
     auto make_pairs = [&](PairedArg& t, uint64_t n) -> int32_t {
         if (t.pairs) return FG_OK;
         void* q;
@@ -2465,7 +2471,7 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
     };
     PlaneSet z32;
     if ((pair_a || pair_b) && (s = make_pairs(dZ, mn)) != FG_OK) return s;
-    if ((dB && !pair_b) || (dA && !pair_a)) {
+    if (conv_b || conv_a) {
         if (ldz == N && (s = loadable32(ctx, dZ.x, M, N, 1, 0, &z32)) != FG_OK) return s;
         if (ldz != N) { z32 = PlaneSet{}; z32.p32 = const_cast<float*>(dZ.x); z32.ld32 = ldz; }
     }
@@ -2476,12 +2482,13 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         const PlaneSet pz = paired_operand(dZ.x, dZ.pairs, dZ.stride, N, false);
         if ((s = paired_gemm(ctx, pa, pz, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr, PairedOut{nullptr, 0, nullptr, 0, nullptr})) != FG_OK)
             return s;
-    } else if (dB) {
+    } else if (conv_b) {
         PlaneSet a32;
         if ((s = loadable32(ctx, A.x, M, K, 1, 0, &a32)) != FG_OK) return s;
         const Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
         if ((s = launch_conv(ctx, as_operand(a32, true), as_operand(z32, true), ep, rt.dB.conv, 1)) != FG_OK) return s;
-    }
+    } else if (dB && (s = gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, A.x, nullptr, dZ.x, FG_ACT_NONE, nullptr, nullptr, dB, nullptr,
+                                          nullptr, nullptr, 0)) != FG_OK) return s;
     if (exch_buf && (s = fg_allreduce_sum_f32(ctx, exch_buf, exch_count)) != FG_OK) return s;
     if (pair_a) {
         if ((s = make_pairs(B, kn)) != FG_OK) return s;
@@ -2489,7 +2496,7 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         const PlaneSet pz = paired_operand(dZ.x, dZ.pairs, dZ.stride, N, true);
         const PlaneSet pb = paired_operand(B.x, B.pairs, B.stride, N, true);
         if ((s = paired_gemm(ctx, pz, pb, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr, o)) != FG_OK) return s;
-    } else if (dA) {
+    } else if (conv_a) {
         PlaneSet b32;
         if ((s = loadable32(ctx, B.x, K, N, 1, 0, &b32)) != FG_OK) return s;
         Epilogue ep{dA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
@@ -2499,6 +2506,8 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         ep.mul_act = o.mul_act;
         ep.colsum_part = o.colsum_part;
         if ((s = launch_conv(ctx, as_operand(z32, false), as_operand(b32, false), ep, rt.dA.conv, 1)) != FG_OK) return s;
+    } else if (dA) {        // (o is left to the caller)
+        return gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, nullptr, B.x, dZ.x, FG_ACT_NONE, nullptr, dA, nullptr, nullptr, nullptr, nullptr, 0);
     }
     return FG_OK;
 }
@@ -2530,13 +2539,14 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         PairedOut po = o;
         po.colsum_part = cs_part;
         if ((s = gemm_bwd_products(ctx, M, N, K, A, B, dZ, N, rt, dB, dA, po, exch_buf, exch_count)) != FG_OK) return s;
-        return cs_part ? fg_colsum_fold_launch(ctx, K, cs_chunks, cs_part, dbias_prev) : FG_OK;
-    }
-    // Any other shape: operand planes, then what the dA epilogue would have done as passes of their own.
-    if ((s = gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, A.x, B.x, dZ.x, FG_ACT_NONE, nullptr, dA, dB, nullptr, nullptr, exch_buf,
-                             exch_count)) != FG_OK)
+        if (!dA || rt.dA.kind != kRoutePlanes)
+            return cs_part ? fg_colsum_fold_launch(ctx, K, cs_chunks, cs_part, dbias_prev) : FG_OK;
+    } else if ((s = gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, A.x, B.x, dZ.x, FG_ACT_NONE, nullptr, dA, dB, nullptr, nullptr, exch_buf,
+                                    exch_count)) != FG_OK) {
         return s;
+    }
     if (!dA) return FG_OK;
+    // dA came from operand planes: what the other kernels' epilogues would have done, as passes of their own
     const uint64_t mk = (uint64_t)M * K;
     if (K % 4 == 0 && fg_aligned16(dA) && (!o.mul_saved || fg_aligned16(o.mul_saved))) {
         if (o.mul_saved || o.pairs || cs_part) {
@@ -2582,10 +2592,12 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
         if (!rt.planes && (!want_pairs || vec_z)) {
             uint64_t need = (uint64_t)cs_chunks * N * 4 + 2048;
             if (want_pairs) need += bwd_paired_need(M, N, K) + mn * 4;
-            else {       // never more than the operand planes of these shapes would take
+            else {       // dZ and what each product carves: never more than the operand planes of both would take
                 if (own_z) need += (uint64_t)M * round4(N) * 4 + 256;
-                if (dB) need += copy32_bytes(A, M, K, 1, 0) + conv_partial_bytes(rt.dB.conv, K, N, 1);
-                if (dA) need += copy32_bytes(B, K, N, 1, 0) + conv_partial_bytes(rt.dA.conv, M, K, 1);
+                if (dB) need += rt.dB.kind == kRoutePlanes ? planes_bytes(1, N, M) + planes_bytes(1, K, M) + kPairPartialBytes + 4096
+                                                           : copy32_bytes(A, M, K, 1, 0) + conv_partial_bytes(rt.dB.conv, K, N, 1);
+                if (dA) need += rt.dA.kind == kRoutePlanes ? planes_bytes(1, M, N) + planes_bytes(1, K, N) + kPairPartialBytes + 4096
+                                                           : copy32_bytes(B, K, N, 1, 0) + conv_partial_bytes(rt.dA.conv, M, K, 1);
             }
             { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
             int32_t s;

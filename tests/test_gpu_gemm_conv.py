@@ -144,3 +144,35 @@ def test_batched_refuses_what_one_product_refuses(ctx):
         assert ctx.lib.fg_gemm_batched_f32(ctx.handle, mode, T, M, N, k, p, M * k, p, k * N, p, M * N, None, 0, None) == one
         assert ctx.lib.fg_gemm_batched_bwd_f32(ctx.handle, mode, T, M, N, k, p, M * k, p, k * N, p, M * N, 0, None, p, p) == one
     assert ctx.launch_count() == before
+
+
+@pytest.mark.parametrize("M,N,K", [(96, 2048, 2048), (128, 1024, 4096), (128, 4096, 1024), (4096, 64, 4096), (16384, 32, 1024), (300, 100, 304)])
+@pytest.mark.parametrize("paired", [False, True])
+def test_backward_keeps_the_error_of_the_planes(ctx, oracle, M, N, K, paired):
+    # Layers of which one gradient does not suit the pair kernel (few samples, few outputs): both gradients keep a rounded
+    # main term.  The 2-norm error of a million sums is stable to a percent or so; a truncated main term adds a quarter.
+    from ferrograd_b200 import GpuContext
+    r = rng(M + N + K)
+    A, B = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    dZ = r.standard_normal((M, N), np.float32)
+    S = np.tanh(r.standard_normal((M, K))).astype(np.float32)
+    z64 = dZ.astype(np.float64)
+    refA, refB = z64 @ B.astype(np.float64).T, A.astype(np.float64).T @ z64
+    if paired:
+        refA *= 1.0 - S.astype(np.float64) ** 2
+
+    def errors(c):
+        dA, dB, below = c.new_tensor((M, K)), c.new_tensor((K, N)), c.new_tensor((K,))
+        if paired:
+            c.gemm_bwd_paired(up(c, A), up(c, B), up(c, dZ), M, N, K, dB=dB, dA=dA, below_act="tanh", below_saved=up(c, S), below_dbias=below)
+            check(c.to_numpy(below), refA.sum(0), TOL, "bias gradient of the layer below")
+        else:
+            c.gemm_bwd(up(c, A), up(c, B), up(c, dZ), M, N, K, dA=dA, dB=dB)
+        return [np.linalg.norm(c.to_numpy(g) - ref) / np.linalg.norm(ref) for g, ref in ((dA, refA), (dB, refB))]
+
+    planes = GpuContext(0)
+    planes.set_option("gemm_pairs", "0")
+    want = errors(planes)
+    planes.destroy()
+    got = errors(ctx)
+    assert got[0] <= 1.08 * want[0] and got[1] <= 1.08 * want[1], (got, want)
