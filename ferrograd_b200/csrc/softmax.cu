@@ -758,6 +758,14 @@ double ce_bytes(const CeArgs& a) {
 
 // Threads of a block that holds a row of `cols` words at `nv` words per thread.
 int held_threads(uint32_t cols, int nv) { return (int)(((cols + nv - 1) / nv + 31) / 32 * 32); }
+// ... and of the kernels that stream a row several times, for what none of those take: rows whose tensors lie differently
+// modulo 16 bytes, and longer ones.  Rows that the SMs hold at once at 1024 threads each get them (64 x 4096: 10 us, 16 with
+// 256); of many rows a short one is done by fewer threads (50000 x 600 forward: 111 us with 128, 289 with 1024; 10000 x 3000:
+// 109 with 256, 137; 3750 x 8000 backward: 145 with 256, 107).
+int stream_threads(const fg_ctx* ctx, uint32_t rows, uint32_t cols) {
+    if (rows <= 2u * (uint32_t)ctx->sm_count || cols > 4096) return 1024;
+    return cols <= 2048 ? 128 : 256;
+}
 constexpr uint32_t kWarpRowCols = 511, kEdgeRowCols = 32768, kEdgeRowColsBwd = 16384;
 inline bool lie_alike(const void* a, const void* b) {
     return !b || ((reinterpret_cast<uintptr_t>(a) ^ reinterpret_cast<uintptr_t>(b)) & 15u) == 0;
@@ -822,7 +830,7 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
         FG_LAUNCHED(ctx);
         return FG_OK;
     }
-    constexpr int threads = 1024;
+    const int threads = stream_threads(ctx, a.rows, a.cols);
     const int grid = rows_grid(ctx, a.rows, threads);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
     if (vec) softmax_stream_kernel<MODE, true><<<grid, threads, 0, ctx->stream>>>(a);
@@ -884,7 +892,7 @@ int32_t fg_softmax_bwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* y
         FG_LAUNCHED(ctx);
         return FG_OK;
     }
-    constexpr int threads = 1024;
+    const int threads = stream_threads(ctx, rows, cols);
     const int grid = rows_grid(ctx, rows, threads);
     if (vec) softmax_bwd_kernel<true><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
     else softmax_bwd_kernel<false><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);

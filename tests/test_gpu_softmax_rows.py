@@ -62,6 +62,37 @@ def test_rows(ctx, oracle, cols, shift):
     assert np.array_equal(ctx.to_numpy(am), x.argmax(1))
 
 
+@pytest.mark.parametrize("cols", [100, 512, 600, 2049, 4096, 8193, 16385])
+@pytest.mark.parametrize("rows", [21, 300])
+def test_tensors_that_lie_differently(ctx, oracle, rows, cols):
+    # each tensor off a 16-byte boundary by another number of elements: the kernels that stream a row, by words
+    r = np.random.Generator(np.random.Philox(cols))
+    x, dy, base = ((2 * r.standard_normal((rows, cols))).astype(np.float32) for _ in range(3))
+    labels = r.integers(0, cols, rows).astype(np.uint32)
+
+    def place(a, shift):
+        t = ctx.init_tensor_f32((a.size + shift,), np.concatenate([np.full(shift, 7.0, np.float32), a.ravel()]))
+        return t, t.ptr + 4 * shift, lambda: ctx.to_numpy(t)[shift:].reshape(rows, cols)
+
+    (_x, xp, _), (_d, dp, _), (_y, yp, y), (_g, gp, g) = place(x, 0), place(dy, 1), place(base, 2), place(base, 3)
+    ctx.softmax_fwd(xp, yp, rows, cols)
+    yref = oracle.softmax_fwd(x)
+    check(y(), yref, "softmax")
+    ctx.softmax_bwd(yp, dp, gp, rows, cols)
+    check(g(), oracle.softmax_bwd(yref, dy), "softmax backward")
+    ctx.softmax_bwd(yp, dp, gp, rows, cols, accumulate=True)
+    check(g(), 2 * oracle.softmax_bwd(yref, dy), "softmax backward, accumulated")
+    (_p, pp, probs), (_l, lp, dl) = place(base, 1), place(base, 2)
+    loss, mean, am = ctx.new_tensor((rows,)), ctx.new_tensor((1,)), ctx.new_tensor((rows,), np.uint32)
+    ctx.softmax_ce(xp, ctx.init_tensor_u32((rows,), labels), rows, cols, grad_scale=0.5, loss_row=loss, loss_mean=mean, dlogits=lp,
+                   probs=pp, argmax=am)
+    onehot = np.zeros((rows, cols), np.float32)
+    onehot[np.arange(rows), labels] = 1.0
+    check(probs(), yref, "probabilities")
+    check(dl(), (yref - onehot) * np.float32(0.5), "gradient")
+    assert np.array_equal(ctx.to_numpy(am), x.argmax(1))
+
+
 @pytest.mark.parametrize("cols", [20, 300, 1003])
 def test_masked_columns_and_in_place(ctx, cols):
     # -inf logits (a mask) get probability zero; the type's lowest value does too; y may be x
