@@ -670,8 +670,11 @@ int32_t fg_gemm_simt_batched_launch(fg_ctx* ctx, int transA, int transB, uint32_
     if (M > 65535u * 64u) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: M too large");
     if (batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: more than 65535 matrices in a batch");
     if (batch == 0) return FG_OK;
-    // 64 x 64 tiles (the most arithmetic per word read) once they give every SM a block; 16-row tiles before that.
-    const bool large = (uint64_t)((M + 63) / 64) * ((N + 63) / 64) * batch >= (uint64_t)ctx->sm_count || M > 65535u * 16u;
+    // Up to four 16 x 32 tiles an SM, as many threads as two 64 x 64 tiles, take no longer than one of those (per 4096 of k:
+    // 98 us for one, 123, 168 and 223 for two to four, 220 for one of 64 x 64); beyond that the larger tiles' arithmetic per
+    // word read counts (768 x 768 x 2048: 117 us against 221).  Both add in the same order.
+    const uint64_t tiles16 = (uint64_t)((M + 15) / 16) * ((N + 31) / 32) * batch;
+    const bool large = tiles16 > 4ull * (uint64_t)ctx->sm_count || M > 65535u * 16u;
     if (large) launch_simt_tile<64, 64, 4>(ctx, transA, transB, batch, M, N, K, A, sA, B, sB, C, sC, bias, act, preact_out);
     else launch_simt_tile<16, 32, 1>(ctx, transA, transB, batch, M, N, K, A, sA, B, sB, C, sC, bias, act, preact_out);
     FG_LAUNCHED(ctx);
