@@ -639,8 +639,10 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
                                  float* dB) {
     if (N > SKN) return fg_fail(ctx, FG_ERR_INTERNAL, "skinny GEMM: N too large");
     // One chunk of rows: the exact path's kernel adds the same products in the same order and needs no fold (64 x 2 x 16: one
-    // launch of 3 us instead of two of 11 + 2 us).
-    if (M <= TN_ROWS && Kd <= 65535u * 64u) return fg_gemm_simt_launch(ctx, 1, 0, Kd, N, M, A, dZ, dB, nullptr, FG_ACT_NONE, nullptr);
+    // launch of 3 us instead of two of 11 + 2 us), until the columns its tiles waste count (64 samples: 16384 x 2 12 us
+    // against 20, 65536 x 2 27 against 20, 65536 x 10 29 against 34, 262144 x 10 88 against 73, x 16 88 against 103).
+    if (M <= TN_ROWS && (Kd <= 8192u * N || (N > 12 && Kd <= 65535u * 64u)))
+        return fg_gemm_simt_launch(ctx, 1, 0, Kd, N, M, A, dZ, dB, nullptr, FG_ACT_NONE, nullptr);
     // block rows: as many as the SMs hold at once (four blocks of 128 threads per SM), at most one per chunk
     const uint32_t gx = (Kd + 511) / 512, chunk = tn_chunk_rows(M, Kd);
     uint32_t nchunks = (uint32_t)(4ull * ctx->sm_count / gx);

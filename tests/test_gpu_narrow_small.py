@@ -23,7 +23,7 @@ def check(x, ref, what):
     assert ok, f"{what}: {worst:.3g}"
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 2, 16), (8, 16, 5), (64, 16, 2), (65, 10, 33), (100, 4, 520), (384, 12, 256), (1100, 3, 64)])
+@pytest.mark.parametrize("M,N,K", [(1, 2, 16), (8, 16, 5), (64, 16, 2), (65, 10, 33), (100, 4, 520), (384, 12, 256), (1100, 3, 64), (64, 1, 8193), (50, 2, 20001)])
 def test_backward(ctx, oracle, M, N, K):
     r = np.random.Generator(np.random.Philox(M + N + K))
     f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
