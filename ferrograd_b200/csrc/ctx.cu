@@ -89,6 +89,23 @@ int32_t fg_ws_ensure(fg_ctx* ctx, uint64_t bytes) {
     return s;
 }
 
+// Is there room for `bytes` more, growing the arena if that can be done?  Unlike fg_ws_ensure, a failure leaves the arena (and
+// the plans recorded against it) as it was, for a caller that has a way to do with less.
+bool fg_ws_try(fg_ctx* ctx, uint64_t bytes) {
+    const uint64_t off = (ctx->ws_used + 255u) & ~uint64_t(255);
+    if (off + bytes <= ctx->ws_bytes) return true;
+    if (ctx->capturing || ctx->ws_used != 0) return false;
+    void* p = nullptr;
+    const uint64_t want = bytes + bytes / 4;
+    if (cudaMalloc(&p, want) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { cudaFree(p); return false; }      // the old arena's users
+    if (ctx->ws) cudaFree(ctx->ws);
+    ctx->ws = (char*)p;
+    ctx->ws_bytes = want;
+    ctx->ws_generation++;
+    return true;
+}
+
 static bool create_events(cudaEvent_t* ev, int n) {
     for (int i = 0; i < n; ++i)
         if (cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming) != cudaSuccess) return false;

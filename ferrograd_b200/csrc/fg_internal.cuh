@@ -174,6 +174,7 @@ inline bool fg_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p)
 int32_t fg_ws_alloc(fg_ctx* ctx, uint64_t bytes, void** out);
 // Room for `bytes` more in the arena (grows it when nothing has been carved yet for this operation).
 int32_t fg_ws_ensure(fg_ctx* ctx, uint64_t bytes);
+bool fg_ws_try(fg_ctx* ctx, uint64_t bytes);      // the same, but a failure changes nothing and is no error
 
 // Grid for a bandwidth-bound grid-stride kernel: a multiple of the SM count.
 inline int fg_stream_grid(const fg_ctx* ctx, uint64_t work_items, int threads, int per_sm) {

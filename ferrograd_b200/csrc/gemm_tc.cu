@@ -2639,11 +2639,10 @@ namespace {
 // One launch of the conversion kernel for `batch` products, or a loop over them?  The loop's cost per matrix is the pair
 // kernel's when the matrix suits it (its pairs are made for the whole batch at once), otherwise a pre-pass and a
 // partly filled wave per matrix.
-bool batch_converts(const fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, bool pair_ok, ConvPlan* p) {
+bool batch_converts(const fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, bool pair_ok) {
     if (!conv_allowed(ctx) || batch > 65535) return false;
-    *p = plan_conv(ctx, M, N, K, batch);
     const double elems = (double)M * K + (double)K * N;
-    return p->cycles <= (double)batch * pair_cycles(ctx, M, N, K, pair_ok ? elems : 2.0 * elems, 2);
+    return plan_conv(ctx, M, N, K, batch).cycles <= (double)batch * pair_cycles(ctx, M, N, K, pair_ok ? elems : 2.0 * elems, 2);
 }
 
 // Arguments that the per-matrix entry points refuse (an unknown mode, K = 0) are left to the loop, which asks them.
@@ -2652,12 +2651,16 @@ bool batch_route_open(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, u
            (N > 16 || mode != FG_GEMM_AUTO);
 }
 
-// Scratch for a whole batch.  Where it cannot be had (out of memory, or a recording whose arena was sized for less), the
-// loop over the matrices, which needs one matrix's worth, takes its place.
-bool batch_scratch(fg_ctx* ctx, uint64_t bytes) {
-    if (fg_ws_ensure(ctx, bytes) == FG_OK) return true;
-    cudaGetLastError();
-    return false;
+// Matrices per launch: the whole batch if the scratch arena has room for it or can be grown (64 x (512 x 512 x 512) backward with
+// an activation: 323 us, 360 in parts).  Otherwise (out of memory, a recording whose arena was sized for less) as many as find
+// room in the arena or in what the loop over the matrices would make of it (`loop`).  need(t): bytes for t matrices.
+template <typename Need>
+uint32_t batch_part(fg_ctx* ctx, uint32_t batch, uint64_t loop, Need need) {
+    if (fg_ws_try(ctx, need(batch))) return batch;
+    const uint64_t room = ctx->capturing || loop < ctx->ws_bytes ? ctx->ws_bytes : loop;
+    uint32_t t = batch;
+    while (t > 1 && (need(t) > room || (batch % t && need(batch % t) > room))) t = (t + 1) / 2;      // (the last part may cut K)
+    return t;
 }
 
 }  // namespace
@@ -2729,19 +2732,25 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
     if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && K > 0)
         return fg_gemm_simt_batched_launch(ctx, 0, 0, batch, M, N, K, A, strideA, B, strideB, C, strideC, bias, act, preact_out);
     if (batch_route_open(ctx, mode, M, N, K)) {
-        ConvPlan cp;
-        if (batch_converts(ctx, batch, M, N, K, paired_shape_ok(ctx, M, N, K, K, N), &cp)) {
-            const uint64_t need = copy32_bytes(A, M, K, batch, strideA) + copy32_bytes(B, K, N, batch, strideB) +
-                                  conv_partial_bytes(cp, M, N, batch) + 1024;
-            if (batch_scratch(ctx, need)) {
-                int32_t s;
+        if (batch_converts(ctx, batch, M, N, K, paired_shape_ok(ctx, M, N, K, K, N))) {
+            auto need = [&](uint32_t t) {
+                return copy32_bytes(A, M, K, t, strideA) + copy32_bytes(B, K, N, t, strideB) +
+                       conv_partial_bytes(plan_conv(ctx, M, N, K, t), M, N, t) + 1024;
+            };
+            const uint32_t part = batch_part(ctx, batch, planes_bytes(1, M, K) + planes_bytes(1, N, K) + kPairPartialBytes + 1024, need);
+            for (uint32_t t0 = 0; t0 < batch; t0 += part) {
+                const uint32_t t = batch - t0 < part ? batch - t0 : part;
                 PlaneSet pa, pb;
-                if ((s = loadable32(ctx, A, M, K, batch, strideA, &pa)) != FG_OK) return s;
-                if ((s = loadable32(ctx, B, K, N, batch, strideB, &pb)) != FG_OK) return s;
-                Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
-                ep.c_batch = batch > 1 ? strideC : 0;
-                return launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, cp, batch);
+                ctx->ws_used = 0;
+                int32_t s = fg_ws_ensure(ctx, need(t));
+                if (s != FG_OK) return s;
+                if ((s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &pa)) != FG_OK) return s;
+                if ((s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &pb)) != FG_OK) return s;
+                Epilogue ep{C + t0 * strideC, bias, preact_out ? preact_out + t0 * strideC : nullptr, M, N, K, act, ctx->dev_status};
+                ep.c_batch = t > 1 ? strideC : 0;
+                if ((s = launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, plan_conv(ctx, M, N, K, t), t)) != FG_OK) return s;
             }
+            return FG_OK;
         }
     }
     const bool dense = strideA == (uint64_t)M * K && strideB == (uint64_t)K * N;
@@ -2811,43 +2820,51 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
         return FG_OK;
     }
     if (batch_route_open(ctx, mode, M, N, K)) {
-        ConvPlan cb{}, ca{};
         const bool n8 = N % 8 == 0 && K % 8 == 0;
-        const bool all = M <= 65535u * 32u && (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N), &cb)) &&
-                         (!dA || batch_converts(ctx, batch, M, K, N, n8 && paired_shape_ok(ctx, M, K, N, N, N), &ca));
-        // dZ for the whole batch in one pass, then one launch per product
+        const bool all = M <= 65535u * 32u && (!dB || batch_converts(ctx, batch, K, N, M, n8 && paired_shape_ok(ctx, K, N, M, K, N))) &&
+                         (!dA || batch_converts(ctx, batch, M, K, N, n8 && paired_shape_ok(ctx, M, K, N, N, N)));
         const bool own_z = act != FG_ACT_NONE;
-        const uint64_t need = (own_z ? (uint64_t)batch * M * round4(N) * 4 + 256 : copy32_bytes(dY, M, N, batch, strideC)) +
-                              (dB ? copy32_bytes(A, M, K, batch, strideA) + conv_partial_bytes(cb, K, N, batch) : 0) +
-                              (dA ? copy32_bytes(B, K, N, batch, strideB) + conv_partial_bytes(ca, M, K, batch) : 0) + 2048;
-        if (all && batch_scratch(ctx, need)) {
-            int32_t s;
+        auto need = [&](uint32_t t) {
+            return (own_z ? (uint64_t)t * M * round4(N) * 4 + 256 : copy32_bytes(dY, M, N, t, strideC)) +
+                   (dB ? copy32_bytes(A, M, K, t, strideA) + conv_partial_bytes(plan_conv(ctx, K, N, M, t), K, N, t) : 0) +
+                   (dA ? copy32_bytes(B, K, N, t, strideB) + conv_partial_bytes(plan_conv(ctx, M, K, N, t), M, K, t) : 0) + 2048;
+        };
+        const uint64_t loop = 2048 + (dA ? planes_bytes(1, M, N) + planes_bytes(1, K, N) + kPairPartialBytes : 0) +
+                              (dB ? planes_bytes(1, N, M) + planes_bytes(1, K, M) + kPairPartialBytes : 0);
+        const uint32_t part = all ? batch_part(ctx, batch, loop, need) : 0;
+        // dZ for a part of the batch in one pass, then one launch per product
+        for (uint32_t t0 = 0; t0 < batch && all; t0 += part) {
+            const uint32_t t = batch - t0 < part ? batch - t0 : part;
+            const float* const dy = dY + t0 * strideC;
             PlaneSet z, x;
+            ctx->ws_used = 0;
+            int32_t s = fg_ws_ensure(ctx, need(t));
+            if (s != FG_OK) return s;
             if (own_z) {
                 void* p;
-                if ((s = fg_ws_alloc(ctx, (uint64_t)batch * M * round4(N) * 4, &p)) != FG_OK) return s;
+                if ((s = fg_ws_alloc(ctx, (uint64_t)t * M * round4(N) * 4, &p)) != FG_OK) return s;
                 PrepArgs a{};
-                a.x = dY; a.saved = saved; a.act = act; a.R = M; a.C = N; a.x_batch = strideC; a.out = p; a.ld = round4(N);
-                if ((s = launch_prep(ctx, FG_DTYPE_F32, a, batch)) != FG_OK) return s;
+                a.x = dy; a.saved = saved + t0 * strideC; a.act = act; a.R = M; a.C = N; a.x_batch = strideC; a.out = p; a.ld = round4(N);
+                if ((s = launch_prep(ctx, FG_DTYPE_F32, a, t)) != FG_OK) return s;
                 z = PlaneSet{};
                 z.p32 = (float*)p;
                 z.ld32 = round4(N);
                 z.batch32 = (uint64_t)M * round4(N);
-            } else if ((s = loadable32(ctx, dY, M, N, batch, strideC, &z)) != FG_OK) return s;
+            } else if ((s = loadable32(ctx, dy, M, N, t, strideC, &z)) != FG_OK) return s;
             if (dB) {
-                if ((s = loadable32(ctx, A, M, K, batch, strideA, &x)) != FG_OK) return s;
-                Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
-                ep.c_batch = batch > 1 ? strideB : 0;
-                if ((s = launch_conv(ctx, as_operand(x, true), as_operand(z, true), ep, cb, batch)) != FG_OK) return s;
+                if ((s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &x)) != FG_OK) return s;
+                Epilogue ep{dB + t0 * strideB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
+                ep.c_batch = t > 1 ? strideB : 0;
+                if ((s = launch_conv(ctx, as_operand(x, true), as_operand(z, true), ep, plan_conv(ctx, K, N, M, t), t)) != FG_OK) return s;
             }
             if (dA) {
-                if ((s = loadable32(ctx, B, K, N, batch, strideB, &x)) != FG_OK) return s;
-                Epilogue ep{dA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
-                ep.c_batch = batch > 1 ? strideA : 0;
-                if ((s = launch_conv(ctx, as_operand(z, false), as_operand(x, false), ep, ca, batch)) != FG_OK) return s;
+                if ((s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &x)) != FG_OK) return s;
+                Epilogue ep{dA + t0 * strideA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
+                ep.c_batch = t > 1 ? strideA : 0;
+                if ((s = launch_conv(ctx, as_operand(z, false), as_operand(x, false), ep, plan_conv(ctx, M, K, N, t), t)) != FG_OK) return s;
             }
-            return FG_OK;
         }
+        if (all) return FG_OK;
     }
     for (uint32_t t = 0; t < batch; ++t) {
         int32_t s = fg_gemm_bwd_f32(ctx, mode, M, N, K, A ? A + t * strideA : nullptr, B ? B + t * strideB : nullptr,

@@ -176,3 +176,66 @@ def test_backward_keeps_the_error_of_the_planes(ctx, oracle, M, N, K, paired):
     planes.destroy()
     got = errors(ctx)
     assert got[0] <= 1.08 * want[0] and got[1] <= 1.08 * want[1], (got, want)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("how", ["recording", "out of memory"])
+def test_batches_without_scratch_for_all_matrices(oracle, shift, how):
+    # dZ of 1001 matrices (66 MB), or padded copies of the operands (330 MB), where the arena cannot grow: they pass through it in
+    # parts, it stays where it is, and a plan recorded before can still be launched
+    import torch
+    from ferrograd_b200 import GpuContext
+    T, M, N, K = 1001, 64, 256, 256
+    r = rng(T + shift)
+    A, B, dY = (r.standard_normal(s, np.float32) for s in ((T, M, K), (T, K, N), (T, M, N)))
+    B *= 0.1
+    c = GpuContext(0)
+    place = lambda a: up(c, np.concatenate([np.zeros(shift, np.float32), a.ravel()]))                   # noqa: E731
+    at = lambda t: t.ptr + 4 * shift                                                                    # noqa: E731
+    Ad, Bd, Yd = place(A), place(B), place(dY)
+    C, dA, dB = place(np.zeros_like(dY)), place(np.zeros_like(A)), place(np.zeros_like(B))
+
+    def both(t):
+        c.gemm_batched(at(Ad), at(Bd), at(C), t, M, N, K, act="tanh")
+        c.gemm_batched_bwd(at(Ad), at(Bd), at(Yd), t, M, N, K, act="tanh", saved=at(C), dA=at(dA), dB=at(dB))
+
+    def record(t):
+        c.plan_begin()
+        both(t)
+        return c.plan_end()
+
+    c.reserve_workspace(48 << 20)       # what one matrix on the general path takes
+    both(40)
+    plan = record(40)
+    arena = c.workspace_bytes()
+    if how == "recording":
+        whole = record(T)
+        whole.launch()
+        whole.destroy()
+    else:
+        filling, left, size = [], torch.empty(32 << 20, dtype=torch.uint8, device="cuda"), 32 << 30
+        try:
+            while size >= 16 << 20:
+                try:
+                    filling.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+                except torch.cuda.OutOfMemoryError:
+                    size //= 2
+            del left                    # for the driver: too little for the 82 MB that all of dZ would take
+            torch.cuda.empty_cache()
+            both(T)
+            c.sync()
+        finally:
+            filling.clear()
+            torch.cuda.empty_cache()
+    assert c.workspace_bytes() == arena < 66 << 20
+    got = c.to_numpy(C)[shift:].reshape(T, M, N)
+    check(got, np.tanh(np.matmul(A, B, dtype=np.float64)), TOL_ACT, "output")
+    dz = dY * (1.0 - got.astype(np.float64) ** 2)
+    check(c.to_numpy(dA)[shift:].reshape(T, M, K), np.matmul(dz, B.transpose(0, 2, 1), dtype=np.float64), TOL, "dA")
+    check(c.to_numpy(dB)[shift:].reshape(T, K, N), np.matmul(A.transpose(0, 2, 1), dz, dtype=np.float64), TOL, "dB")
+    c.memset_zero(C)
+    plan.launch()
+    check(c.to_numpy(C)[shift:shift + 40 * M * N].reshape(40, M, N), got[:40], TOL, "output of the plan recorded first")
+    plan.destroy()
+    assert c.device_status() == 0
+    c.destroy()
