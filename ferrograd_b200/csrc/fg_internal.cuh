@@ -127,10 +127,12 @@ struct FgRange {
          if (_e != cudaSuccess) return fg_fail_cuda((ctx), FG_ERR_LAUNCH_FAILURE, "kernel launch", _e); \
          if ((ctx)->capturing) (ctx)->capture_launches++; else (ctx)->launches++; } while (0)
 
-// Back-to-back launches of short kernels.  A kernel launched with fg_launch may be set up while the kernel before it on the
-// stream still runs (programmatic stream serialization); fg_grid_enter(), its first statement in every thread, waits until
-// everything before it has finished and is visible, then lets the next such kernel be set up.  Seven launches of a ragged
-// layer's backward pass 75.8 -> 60.5 us, the 16 of a 2-16-2 training step 33.4 -> 28.7 us.
+// Back-to-back launches of short kernels.  A kernel launched with fg_launch is set up while the kernel before it on the
+// stream drains (programmatic stream serialization); fg_grid_enter(), its first statement in every thread, waits until
+// everything before it has finished and is visible.  Nothing is triggered early: blocks of the next kernel that wait on the
+// SMs from the start of this one's work on slow it several times over, once the host is ahead (18 x (88 x 24 x 256) backward,
+// two launches: 14.4 us in plain order, 10.8 like this, 30 to 37 with a trigger on entry).  Seven launches of a ragged layer's
+// backward pass 71.6 -> 53.6 us, the 16 of a 2-16-2 training step 36.2 -> 30.1 us.
 template <typename... P, typename... A>
 inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -145,10 +147,7 @@ inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, 
     cfg.numAttrs = ctx->comm ? 0 : 1;      // with a communicator the stream also forks and joins: plain order there
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // FG_LAUNCHED reports its error
 }
-__device__ __forceinline__ void fg_grid_enter() {
-    cudaGridDependencySynchronize();
-    cudaTriggerProgrammaticLaunchCompletion();
-}
+__device__ __forceinline__ void fg_grid_enter() { cudaGridDependencySynchronize(); }
 
 // Brackets one kernel launch with events when timing is enabled (never while capturing).
 inline fg_time_rec* fg_time_begin(fg_ctx* ctx, int kind, double work) {
