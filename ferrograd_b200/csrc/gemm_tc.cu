@@ -1286,7 +1286,8 @@ struct ConvCfg {
 // bf16: blocks of 64 rows, [plane][k][128 bytes] each, 16-byte chunk c of k-row k at c ^ (k & 7).
 // Lanes are dealt so that the 128-bit accesses of eight lanes fall into different banks.
 // Nearest tf32 value, ties away from zero (cvt.rna), in two integer operations: the conversion unit is a fraction as wide.
-// A NaN may lose its payload here; the planes keep the product NaN.
+// A NaN may lose its payload here; the planes keep the product NaN.  Values from 0x7f7ff000 on round to infinity; products of
+// values from 0x7f7f8000 on are not finite in any format with bf16 planes, because bf16(x) is not.
 __device__ __forceinline__ float4 round_tf32(float4 v) {
     auto r = [](float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); };
     return make_float4(r(v.x), r(v.y), r(v.z), r(v.w));
@@ -2425,9 +2426,9 @@ struct BwdRoutes {
     bool planes;      // every wanted product runs from operand planes
 };
 // Both wanted products may take the pair kernel or neither: its main term is truncated where the planes and the conversion
-// kernel round it (1.9e-6 against 1.5e-6 of the result's 2-norm), and a layer with one product that the pair kernel cannot
-// run keeps the smaller error in both.  Between planes and conversion each product follows its estimate: 128 x 8192 x 8192
-// 290 us, against 414 with both converted and 458 with both from planes.
+// kernel round it (dW of 128 x 4096 x 1024: 1.40e-6 against 0.87e-6 of the result's 2-norm), and a layer with one product that
+// the pair kernel cannot run keeps the smaller error in both.  Between planes and conversion each product follows its
+// estimate: 128 x 8192 x 8192 290 us, against 414 with both converted and 458 with both from planes.
 BwdRoutes pick_bwd_routes(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, const float* dB,
                           const float* dA, const float* mul_saved) {
     BwdRoutes r{};

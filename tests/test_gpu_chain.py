@@ -99,15 +99,29 @@ def test_output_may_overwrite_an_input(ctx, oracle):
 
 @pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
 def test_gelu_of_extreme_values(ctx, dtype):
-    # the limits: x for large positive, zero for large negative, NaN stays NaN, +inf stays +inf
-    x = np.array([0.0, -0.0, 30.0, -30.0, 3e4, -3e4, np.inf, np.nan, 1e-6, -1e-6], np.float32)
+    # the limits: x for large positive, zero for large negative, NaN stays NaN, +inf stays +inf; its derivative 1, 0 and 1/2 at zero
+    small = 1e-3 if dtype == "f16" else 1e-6            # a normal number of the type
+    x = np.array([0.0, -0.0, 30.0, -30.0, 3e4, -3e4, np.inf, np.nan, small, -small], np.float32)
     n = x.size
     init = {"f32": ctx.init_tensor_f32, "f16": ctx.init_tensor_f16, "bf16": ctx.init_tensor_bf16}[dtype]
-    t, out = init((n,), x), init((n,), np.zeros(n))
-    ctx.eltwise_chain_fwd([("input", 0, 0, 0.0), ("gelu", 0, 0, 0.0)], [t], out, n, dtype=dtype)
-    back = ctx.new_tensor((n,))
-    ctx.convert(out, dtype, back, "f32", n)
-    ctx.convert(t, dtype, t32 := ctx.new_tensor((n,)), "f32", n)
-    y, x = ctx.to_numpy(back), ctx.to_numpy(t32)
+    prog = [("input", 0, 0, 0.0), ("gelu", 0, 0, 0.0)]
+    t, out, grad, ones = init((n,), x), init((n,), np.zeros(n)), init((n,), np.zeros(n)), init((n,), np.ones(n))
+    ctx.eltwise_chain_fwd(prog, [t], out, n, dtype=dtype)
+    ctx.eltwise_chain_bwd(prog, [t], ones, [grad], n, dtype=dtype)
+
+    def down(v):
+        back = ctx.new_tensor((n,))
+        ctx.convert(v, dtype, back, "f32", n)
+        return ctx.to_numpy(back)
+
+    y, x, g = down(out), down(t), down(grad)
+    # gelu(x) / x = 1/2 + 0.4 x near zero; one rounding of the type (2^-9 in bf16) for x and one for the result
+    near = {"f32": 1e-5, "f16": 2e-3, "bf16": 8e-3}[dtype]
     assert y[0] == 0 and y[1] == 0 and y[2] == x[2] and y[3] == 0 and y[4] == x[4] and y[5] == 0 and np.isposinf(y[6]) and np.isnan(y[7])
-    assert np.allclose(y[8:], 0.5 * x[8:], rtol=2e-2, atol=0) or dtype == "f16"       # 1e-6 is a subnormal half
+    assert np.allclose(y[8:], 0.5 * x[8:], rtol=near, atol=0)
+    assert g[0] == 0.5 and g[1] == 0.5 and g[2] == 1 and g[3] == 0 and g[4] == 1 and g[5] == 0 and np.isnan(g[7])
+    assert np.allclose(g[8:], 0.5, rtol=near, atol=0)
+    if dtype == "f32":                                  # the activation's backward pass on its own
+        dz = ctx.new_tensor((n,))
+        ctx.act_bwd(ones, t, dz, n, "gelu")
+        assert np.array_equal(ctx.to_numpy(dz), g, equal_nan=True)

@@ -84,6 +84,26 @@ def test_unaligned_operands(ctx, oracle):
     check(ctx.to_numpy(C)[1:].reshape(M, N), oracle.gemm(A, B, f64=True), TOL, "unaligned")
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 256, 256), (100, 1000, 1024)])
+def test_values_that_are_not_finite_stay_in_their_row(ctx, oracle, M, N, K):
+    # infinities and NaN make their row of the result not finite and leave the others alone; values whose bf16 plane is finite
+    # (below 2^128 - 2^119) are exact to the usual tolerance of their row
+    r = rng(M + N)
+    A, B = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    A[3, 5], A[40, 0], A[77, K - 1] = np.inf, -np.inf, np.nan
+    A[9] = 0.0
+    A[9, 2] = np.uint32(0x7f7f7fff).view(np.float32)
+    B[2] *= 1e-3
+    C = ctx.new_tensor((M, N))
+    ctx.gemm(up(ctx, A), up(ctx, B), C, M, N, K)
+    got = ctx.to_numpy(C)
+    bad = [3, 40, 77]
+    assert not np.isfinite(got[bad]).any()
+    good = [m for m in range(M) if m not in bad + [9]]
+    check(got[good], A[good].astype(np.float64) @ B.astype(np.float64), TOL, "finite rows")
+    check(got[9] / 1e30, (A[9, 2].astype(np.float64) / 1e30) * B[2].astype(np.float64), TOL, "row of the largest value")
+
+
 @pytest.mark.parametrize("T,M,N,K", [(1, 64, 256, 256), (1, 130, 100, 333), (2, 64, 256, 256), (5, 130, 100, 333), (16, 384, 320, 512),
                                      (3, 65, 515, 1024), (40, 64, 64, 1100)])
 @pytest.mark.parametrize("gap", [0, 1, 4, 6])
