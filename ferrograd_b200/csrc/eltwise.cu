@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_
 // Storage type of a chain's tensors.  Values are held as float in registers; with 16-bit storage every
 // operation's result is rounded to the storage type (round to nearest even), which for + - * / equals
 // native half arithmetic (float carries more than twice the bits, so the double rounding is harmless).
-// ldw / stw move W consecutive elements starting at element i (W = 4: one 128-bit access for f32, one 64-bit
-// access for the 16-bit types; the caller has checked the alignment).
+// ld4w / st4w move four consecutive elements starting at element i (one 128-bit access for f32, one 64-bit access for the
+// 16-bit types; the caller has checked the alignment).
 template <int DT> struct Stored;
 template <> struct Stored<FG_DTYPE_F32> {
     typedef float T;
@@ -256,12 +256,6 @@ template <> struct Stored<FG_DTYPE_BF16> {
         *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p) + i) = u;
     }
 };
-template <int DT, int W> __device__ __forceinline__ void ldw(const void* p, uint64_t i, float* o) {
-    if (W == 4) Stored<DT>::ld4w(p, i, o); else o[0] = Stored<DT>::ld(p, i);
-}
-template <int DT, int W> __device__ __forceinline__ void stw(void* p, uint64_t i, const float* v) {
-    if (W == 4) Stored<DT>::st4w(p, i, v); else Stored<DT>::st(p, i, v[0]);
-}
 
 // ---- chain programs as run by the kernel ----
 // The host turns a chain (forward, or backward = the values it needs followed by the adjoints) into a list of

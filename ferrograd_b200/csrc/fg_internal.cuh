@@ -245,7 +245,6 @@ __device__ __forceinline__ float fg_act_grad(int act, float saved) {
 // 1 / (1 + exp(-a)) with a given pre-multiplied by -log2(e): sigmoid(a) = 1 / (1 + 2^(a * -log2 e)).
 __device__ __forceinline__ float fg_sigmoid_l2(float a_neg_l2) { return fg_rcp_fast(1.0f + fg_ex2_fast(a_neg_l2)); }
 #define FG_NEG_LOG2E (-1.4426950408889634f)
-__device__ __forceinline__ float fg_sigmoid_fast(float a) { return fg_sigmoid_l2(a * FG_NEG_LOG2E); }
 // -log2(e) * 2 * FG_GELU_B * (x + FG_GELU_A x^3) = x * (c1 + c3 x^2)
 #define FG_GELU_C1 (FG_NEG_LOG2E * 2.0f * FG_GELU_B)
 #define FG_GELU_C3 (FG_NEG_LOG2E * 2.0f * FG_GELU_B * FG_GELU_A)

@@ -1,5 +1,5 @@
-// Dense f32 GEMM on the tcgen05 tensor cores with a 3xTF32 split, and the GEMM entry
-// points (forward with fused bias + activation epilogue, backward dA / dB / dbias).
+// Dense f32 and 16-bit GEMM on the tcgen05 tensor cores, and the GEMM entry points (forward with fused bias +
+// activation epilogue, backward dA / dB / dbias).
 //
 // What it replaces: the reference's tiled scalar-FMA matmul and its backward edges
 // (crates/ferrograd-nn/src/op/matmul/mod.rs:17-188, generic.rs:13-325; dA = dC·Bᵀ via
@@ -8,21 +8,20 @@
 // and the activation-derivative factor of the backward chains (op/unary.rs:281-309,
 // :453-472, :588-714).
 //
-// Method.  x = hi + lo with hi = tf32(x), lo = tf32(x - hi); A·B ~= hi·hi + hi·lo + lo·hi,
-// accumulated in f32 in tensor memory (the dropped lo·lo term and the rounding of lo are
-// both ~2^-23 relative).  A pre-pass writes the hi and lo planes of each operand into the
-// scratch arena in K-major form (contraction index contiguous), transposing on the way
-// when the operand is stored the other way round; it can also apply dY * act'(saved) so
-// the backward GEMMs never see an unfused elementwise pass.  The GEMM kernel is a
-// warp-specialised pipeline: one thread issues bulk-tensor loads (no multicast) of the
-// four planes of a k-block into 128-byte-swizzled shared memory, one thread issues
-// three tcgen05.mma per 8-wide k-step, four warps read the accumulators back with
-// tcgen05.ld and apply bias + activation while storing.
-//
-// Data layout in HBM: planes live in the scratch arena as [2][rows][ld] f32 (plane 0 = hi,
-// plane 1 = lo; ld = contraction length rounded up to 4 so row pitches are 16-byte
-// multiples).  One 3-D tensor map per operand: dims {contraction, rows, 2},
-// box {32, tile rows, 2}, so one load brings the hi and the lo tile of a k-block.
+// Method.  An f32 product is a split product: x = hi + lo with hi = tf32(x); A·B ~= hi·hi on kind::tf32 plus the two
+// cross terms, on kind::f16 from bf16 planes (bf16(x), bf16(lo)) or, in the strict 3xTF32 mode, on kind::tf32 from
+// tf32(lo).  Accumulators are f32 in tensor memory, drained in chunks of k; the dropped lo·lo term is ~2^-23 relative.
+// Four ways to get hi and lo to the tensor core, chosen by estimates of their times (pick_route and its callers):
+//   * pairs: the f32 tensor as it lies (the MMA truncates it) beside bf16 planes kept with it or made in one pass;
+//     256 x 256 tiles on SM pairs.  Large products.
+//   * conversion kernel: the f32 tensors alone; warps round and split each k-block in shared memory.  Small and
+//     middling products, batches.
+//   * operand planes: a pre-pass writes hi and lo planes of each operand into the scratch arena, contraction index
+//     contiguous, transposing on the way; dY * act'(saved) is applied there.  Any shape; the strict mode.
+//   * 16-bit tensors go to kind::f16 as they lie, with a padded copy where rows are not 16-byte aligned.
+// Every kernel is a warp-specialised pipeline: one thread issues bulk-tensor loads (no multicast) into swizzled shared
+// memory, one thread issues tcgen05.mma, other warps read the accumulators back with tcgen05.ld and apply bias and
+// activation while storing.
 #include <atomic>
 #include <cuda_bf16.h>
 #include <stdlib.h>

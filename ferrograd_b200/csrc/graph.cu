@@ -620,7 +620,7 @@ static int32_t forward_eager(fg_exec* e) {
                 continue;
             }
             if (e->dtype == FG_DTYPE_F32 && gs.batch > 1) {
-                // rank-3 product: one launch for small matrices, one pairs pass + one launch per matrix for large ones
+                // rank-3 product: one launch for small and middling matrices, one pairs pass + one launch per matrix for large ones
                 s = fg_gemm_batched_f32(e->ctx, e->gemm_mode, gs.batch, gs.M, gs.N, gs.K, vptr(e, gs.a), sa, vptr(e, gs.b), sb,
                                         vptr(e, gs.out), sc, gs.bias >= 0 ? vptr(e, gs.bias) : nullptr, gs.act,
                                         gs.preact ? (float*)gs.preact->ptr : nullptr);

@@ -118,22 +118,9 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Shared-memory matrix descriptor for a K-major operand tile whose rows are 128 bytes
-// (32 f32 / 64 bf16) laid out with the 128-byte swizzle that the TMA load wrote:
-// 8-row groups are 1024 bytes apart (stride byte offset), the leading byte offset is
-// unused for swizzled K-major tiles, descriptor version 1, layout type SWIZZLE_128B.
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024u >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-// The same for rows of ROW_BYTES = 128 or 64 bytes (swizzle span = row length): 8-row groups are
-// 8 * ROW_BYTES apart; layout type 2 = SWIZZLE_128B, 4 = SWIZZLE_64B.
+// Shared-memory matrix descriptor for a K-major operand tile whose rows are ROW_BYTES = 128 or 64 bytes, laid out with the
+// swizzle of that span that the TMA load wrote: 8-row groups are 8 * ROW_BYTES apart (stride byte offset), the leading byte
+// offset is unused for swizzled K-major tiles, descriptor version 1, layout type 2 = SWIZZLE_128B, 4 = SWIZZLE_64B.
 template <int ROW_BYTES>
 __device__ __forceinline__ uint64_t make_desc_kmajor(uint32_t smem_addr) {
     static_assert(ROW_BYTES == 128 || ROW_BYTES == 64, "row length must equal a supported swizzle span");
