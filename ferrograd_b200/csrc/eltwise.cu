@@ -338,17 +338,19 @@ __device__ __forceinline__ void vm_op(uint32_t op, float imm, float* x, const fl
 }
 #undef FG_VM_LANES
 
-// The program on W elements: W = 1, element i, or W = 8, elements i .. i+3 and i2 .. i2+3 (the second four only when `two`).
-template <int DT, int W>
+// The program on W elements: VEC (W = 8), i .. i+3 and i2 .. i2+3 (the second four only when `two`), or singly i, i + 128, ...
+// as far as the tensors go.
+template <int DT, int W, bool VEC>
 __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2, bool two, float4* sm) {
     typedef Stored<DT> S;
     auto load = [&](const void* p, float* o) {
-        if constexpr (W == 8) {
+        if constexpr (VEC) {
             S::ld4w(p, i, o);
             if (two) S::ld4w(p, i2, o + 4);
             else o[4] = o[5] = o[6] = o[7] = 0.0f;
         } else {
-            o[0] = S::ld(p, i);
+#pragma unroll
+            for (int w = 0; w < W; ++w) o[w] = i + w * kVmThreads < a.n ? S::ld(p, i + w * kVmThreads) : 0.0f;
         }
     };
     float last[W], y[W];
@@ -377,11 +379,13 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2,
             load(a.ptr[ptr], last);
             slot_st<W>(sm, dst2, y);
         } else if (op == VM_ST) {
-            if constexpr (W == 8) {
+            if constexpr (VEC) {
                 S::st4w(a.ptr[ptr], i, last);
                 if (two) S::st4w(a.ptr[ptr], i2, last + 4);
             } else {
-                S::st(a.ptr[ptr], i, last[0]);
+#pragma unroll
+                for (int w = 0; w < W; ++w)
+                    if (i + w * kVmThreads < a.n) S::st(a.ptr[ptr], i + w * kVmThreads, last[w]);
             }
         } else if (op == VM_LDADD) {
             load(a.ptr[ptr], y);
@@ -397,25 +401,28 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2,
     }
 }
 
-// A block takes 1024 consecutive elements at a time, thread t the groups of four t and t + 128 of them (every access of a
-// warp is contiguous).  The last n % 4 elements go singly, on the last block, which has the least other work.
+// A block takes 1024 consecutive elements at a time: thread t the groups of four t and t + 128 of them (every access of a
+// warp is contiguous), the last n % 4 elements singly, on the last block, which has the least other work; or, when a tensor
+// starts off the boundary that groups of four need, elements t, t + 128, ... singly.
 //
 // What bounds it: instruction issue (about 25 instructions to fetch, decode and store an operation, shared by eight elements).
 // gelu(x * y) + x on 32 Mi f32 elements: forward 147 -> 100 us, backward 340 -> 168 us against one interpreter step per
-// instruction and word-wise slots; x / (1 + exp(-x)) * y on 3 M halves 18.4 -> 14.8 us and 49.6 -> 30 us.
-template <int DT>
+// instruction and word-wise slots; x / (1 + exp(-x)) * y on 3 M halves 18.4 -> 14.8 us and 49.6 -> 30 us.  Off the boundary:
+// the adjoints of tanh(x / (1 + |y|)) on 3 M words 125 us with one element per thread and operation, 34 with eight.
+template <int DT, bool VEC>
 __global__ void __launch_bounds__(kVmThreads) chain_kernel(const __grid_constant__ VmArgs a) {
     fg_grid_enter();
     extern __shared__ float4 chain_smem[];
     float4* const sm = chain_smem + threadIdx.x;
-    const uint64_t nv = a.vec ? a.n >> 2 : 0;
-    if (blockIdx.x == gridDim.x - 1 || !a.vec) {
-        const uint64_t step = a.vec ? kVmThreads : (uint64_t)gridDim.x * kVmThreads;
-        for (uint64_t i = (nv << 2) + (a.vec ? 0 : (uint64_t)blockIdx.x * kVmThreads) + threadIdx.x; i < a.n; i += step)
-            vm_run<DT, 1>(a, i, 0, false, sm);
+    if constexpr (VEC) {
+        const uint64_t nv = a.n >> 2;
+        if (blockIdx.x == gridDim.x - 1 && (nv << 2) + threadIdx.x < a.n) vm_run<DT, 1, false>(a, (nv << 2) + threadIdx.x, 0, false, sm);
+        for (uint64_t g = (uint64_t)blockIdx.x * (2 * kVmThreads) + threadIdx.x; g < nv; g += (uint64_t)gridDim.x * (2 * kVmThreads))
+            vm_run<DT, 8, true>(a, g << 2, (g + kVmThreads) << 2, g + kVmThreads < nv, sm);
+    } else {
+        for (uint64_t i = (uint64_t)blockIdx.x * (8 * kVmThreads) + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * (8 * kVmThreads))
+            vm_run<DT, 8, false>(a, i, 0, false, sm);
     }
-    for (uint64_t g = (uint64_t)blockIdx.x * (2 * kVmThreads) + threadIdx.x; g < nv; g += (uint64_t)gridDim.x * (2 * kVmThreads))
-        vm_run<DT, 8>(a, g << 2, (g + kVmThreads) << 2, g + kVmThreads < nv, sm);
 }
 
 // ---- host side: a chain as a list of operations ----
@@ -628,20 +635,25 @@ __global__ void __launch_bounds__(256) convert_kernel(const void* __restrict__ s
 constexpr int kSlotBytes = 8 * kVmThreads * (int)sizeof(float);
 constexpr int kChainSmemMax = 2 * FG_EW_MAX_INSTR * kSlotBytes;
 int32_t launch_chain(fg_ctx* ctx, int dtype, VmBuilder& b, VmArgs& a, double bytes) {
-    static std::atomic<uint64_t> done[3];
+    static std::atomic<uint64_t> done[3][2];
     const uint64_t bit = 1ull << (ctx->device & 63);
     const size_t smem = (size_t)b.finish(&a) * kSlotBytes;
     if (smem > (size_t)kChainSmemMax) return fg_fail(ctx, FG_ERR_INTERNAL, "eltwise chain: too many live values");
-    auto kernel = dtype == FG_DTYPE_F32 ? chain_kernel<FG_DTYPE_F32> : dtype == FG_DTYPE_F16 ? chain_kernel<FG_DTYPE_F16> : chain_kernel<FG_DTYPE_BF16>;
-    if (!(done[dtype].load(std::memory_order_acquire) & bit)) {
+    auto of_type = [&](auto vec) {
+        constexpr bool V = decltype(vec)::value;
+        return dtype == FG_DTYPE_F32 ? chain_kernel<FG_DTYPE_F32, V> : dtype == FG_DTYPE_F16 ? chain_kernel<FG_DTYPE_F16, V> : chain_kernel<FG_DTYPE_BF16, V>;
+    };
+    auto kernel = a.vec ? of_type(std::true_type{}) : of_type(std::false_type{});
+    std::atomic<uint64_t>& set = done[dtype][a.vec ? 1 : 0];
+    if (!(set.load(std::memory_order_acquire) & bit)) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmemMax);
         if (e != cudaSuccess) return fg_fail_cuda(ctx, FG_ERR_INTERNAL, "cudaFuncSetAttribute(chain kernel)", e);
-        done[dtype].fetch_or(bit, std::memory_order_release);
+        set.fetch_or(bit, std::memory_order_release);
     }
     // as many blocks as the shared memory lets an SM hold (of at most sixteen)
     const size_t fit = (220u * 1024u) / (smem + 1024);
     const int per_sm = (int)(fit < 1 ? 1 : fit > 16 ? 16 : fit);
-    const int grid = fg_stream_grid(ctx, a.vec ? (a.n / 4 + 1) / 2 : a.n, kVmThreads, per_sm);
+    const int grid = fg_stream_grid(ctx, a.vec ? (a.n / 4 + 1) / 2 : (a.n + 7) / 8, kVmThreads, per_sm);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, bytes);
     fg_launch(ctx, kernel, grid, kVmThreads, smem, a);
     fg_time_end(ctx, tr);
