@@ -650,10 +650,16 @@ __global__ void __launch_bounds__(256) softmax_bwd_warp_kernel(uint32_t rows, ui
     }
 }
 
-template <int NV>
-__global__ void __launch_bounds__(512) softmax_bwd_edge_kernel(uint32_t rows, uint32_t cols, const float* __restrict__ y,
-                                                                const float* __restrict__ dy, float* __restrict__ dx, int accumulate) {
+// ACC adds to dx: what it adds to is fetched with the rest (fetched after the reduction, 2000 x 12000 took 103 us; 79 with the
+// two-pass kernel; 62 so), which needs more threads of fewer groups each.  Without it eight groups per thread are faster:
+// 4096 x 10001 80 us against 88.  ONCE is the evict-first hint, which rows of more than 8192 columns go without: y has often just been
+// written, and a tensor that the L2 holds stays there (500 x 12000 again and again: 16.4 -> 12.3 us, 4096 x 16384 149 -> 121);
+// shorter rows keep it (2000 x 6001 accumulating: 25 us, 33 without).
+template <int NV, bool ACC, bool ONCE>
+__global__ void __launch_bounds__(4096 / NV) softmax_bwd_edge_kernel(uint32_t rows, uint32_t cols, const float* __restrict__ y,
+                                                                 const float* __restrict__ dy, float* __restrict__ dx) {
     __shared__ float red[2][32];        // rows take turns, so that the reduction costs one barrier
+    auto fetch = [](const float4* p) { return ONCE ? __ldcs(p) : *p; };
     const uint32_t t = threadIdx.x, nt = blockDim.x, lane = t & 31u, nw = nt >> 5;
     int turn = 0;
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x, turn ^= 1) {
@@ -662,12 +668,13 @@ __global__ void __launch_bounds__(512) softmax_bwd_edge_kernel(uint32_t rows, ui
         const float4* y4 = reinterpret_cast<const float4*>(y + base + ed.head);
         const float4* d4 = reinterpret_cast<const float4*>(dy + base + ed.head);
         float4* x4 = reinterpret_cast<float4*>(dx + base + ed.head);
-        float4 a[NV], b[NV];
+        float4 a[NV], b[NV], old[NV];
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             const bool in = t + nt * j < ed.n4;
-            a[j] = in ? __ldcs(y4 + t + nt * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            b[j] = in ? __ldcs(d4 + t + nt * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            a[j] = in ? fetch(y4 + t + nt * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            b[j] = in ? fetch(d4 + t + nt * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ACC) old[j] = in ? x4[t + nt * j] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         const float ae = ed.extra < cols ? y[base + ed.extra] : 0.0f, be = ed.extra < cols ? dy[base + ed.extra] : 0.0f;
         float part[NV];
@@ -681,15 +688,12 @@ __global__ void __launch_bounds__(512) softmax_bwd_edge_kernel(uint32_t rows, ui
         for (int j = 0; j < NV; ++j)
             if (t + nt * j < ed.n4) {
                 float4 g = make_float4(a[j].x * (b[j].x - dot), a[j].y * (b[j].y - dot), a[j].z * (b[j].z - dot), a[j].w * (b[j].w - dot));
-                if (accumulate) {
-                    const float4 o = x4[t + nt * j];
-                    g.x += o.x; g.y += o.y; g.z += o.z; g.w += o.w;
-                }
+                if (ACC) { g.x += old[j].x; g.y += old[j].y; g.z += old[j].z; g.w += old[j].w; }
                 x4[t + nt * j] = g;
             }
         if (ed.extra < cols) {
             const float g = ae * (be - dot);
-            dx[base + ed.extra] = accumulate ? dx[base + ed.extra] + g : g;
+            dx[base + ed.extra] = ACC ? dx[base + ed.extra] + g : g;
         }
     }
 }
@@ -897,8 +901,14 @@ int32_t fg_softmax_bwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* y
         return FG_OK;
     }
     if (cols <= kEdgeRowColsBwd && lie_alike(y, dy) && lie_alike(y, dx)) {
-        const int threads = held_threads(cols, 32);
-        softmax_bwd_edge_kernel<8><<<rows_grid(ctx, rows, threads), threads, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
+        const int threads = held_threads(cols, accumulate ? 16 : 32), grid = rows_grid(ctx, rows, threads);
+        if (accumulate) {
+            if (cols > 8192) softmax_bwd_edge_kernel<4, true, false><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
+            else softmax_bwd_edge_kernel<4, true, true><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
+        } else {
+            if (cols > 8192) softmax_bwd_edge_kernel<8, false, false><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
+            else softmax_bwd_edge_kernel<8, false, true><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
+        }
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
