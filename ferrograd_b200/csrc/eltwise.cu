@@ -180,18 +180,23 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(uint32_t rows, uint
         part[(size_t)blockIdx.y * cols + c] = t;
     }
 }
-// out[c] = sum over chunks of part[k][c].  A block covers 32 columns; its eight warps each add every eighth chunk
-// (so the chain of dependent loads is an eighth as long), then the eight sums are added in order.
+// out[c] = sum over chunks of part[k][c].  A block covers 32 columns; its eight warps each add every eighth chunk into eight
+// sums in turn, which are added in pairs, then the warps' sums in order: 64 short chains of additions (50000 rows in 1563
+// chunks: 3.0e-7 of the sums' 2-norm from 64 bits with eight long ones, 1.3e-7 so).
 __global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_t nchunks,
                                                           const float* __restrict__ part, float* __restrict__ out) {
     fg_grid_enter();
     __shared__ float red[8][33];
     const uint32_t cx = threadIdx.x & 31u, gy = threadIdx.x >> 5;
     const uint32_t c = blockIdx.x * 32 + cx;
-    float s = 0.0f;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (c < cols)
-        for (uint32_t k = gy; k < nchunks; k += 8) s += part[(size_t)k * cols + c];
-    red[gy][cx] = s;
+        for (uint64_t k = gy; k < nchunks; k += 64) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (k + 8 * j < nchunks) s[j] += part[(size_t)(k + 8 * j) * cols + c];
+        }
+    red[gy][cx] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
     __syncthreads();
     if (gy == 0 && c < cols) {
         float t = 0.0f;

@@ -166,6 +166,22 @@ def test_batched_refuses_what_one_product_refuses(ctx):
     assert ctx.launch_count() == before
 
 
+@pytest.mark.parametrize("M,N,K", [(50000, 20, 33), (100000, 32, 64)])
+def test_bias_gradient_of_many_samples(ctx, M, N, K):
+    # Sums of M values of order one in chains of at most 32 + M / 2048 additions that are added in pairs.  A chain's roundings,
+    # 2^-25 of a partial sum that grows with the root of its length, add up to about 2^-25 * sqrt(length / 2) of the chain, and
+    # the chains' errors are independent: 2^-25 * sqrt(25) = 1.5e-7 of the 2-norm at the larger size, with half as much again as margin.
+    errors = []
+    for seed in range(4):
+        r = rng(M + seed)
+        A, B, dY = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32), r.standard_normal((M, N), np.float32)
+        db, dB = ctx.new_tensor((N,)), ctx.new_tensor((K, N))
+        ctx.gemm_bwd(up(ctx, A), up(ctx, B), up(ctx, dY), M, N, K, dB=dB, dbias=db)
+        ref = dY.astype(np.float64).sum(0)
+        errors.append(np.linalg.norm(ctx.to_numpy(db) - ref) / np.linalg.norm(ref))
+    assert np.mean(errors) <= 2.3e-7, errors
+
+
 @pytest.mark.parametrize("M,N,K", [(96, 2048, 2048), (128, 1024, 4096), (128, 4096, 1024), (4096, 64, 4096), (16384, 32, 1024), (300, 100, 304)])
 @pytest.mark.parametrize("paired", [False, True])
 def test_backward_keeps_the_error_of_the_planes(ctx, oracle, M, N, K, paired):
