@@ -244,11 +244,13 @@ def test_batches_without_scratch_for_all_matrices(oracle, shift, how):
     both(40)
     plan = record(40)
     arena = c.workspace_bytes()
-    if how == "recording":
-        whole = record(T)
-        whole.launch()
-        whole.destroy()
-    else:
+    whole = record(T)                   # (and every kernel is loaded before the memory is full)
+    whole.launch()
+    c.sync()
+    whole.destroy()
+    if how == "out of memory":
+        for t in (C, dA, dB):
+            c.memset_zero(t)
         filling, left, size = [], torch.empty(32 << 20, dtype=torch.uint8, device="cuda"), 32 << 30
         try:
             while size >= 16 << 20:
@@ -256,7 +258,7 @@ def test_batches_without_scratch_for_all_matrices(oracle, shift, how):
                     filling.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
                 except torch.cuda.OutOfMemoryError:
                     size //= 2
-            del left                    # for the driver: too little for the 82 MB that all of dZ would take
+            del left                    # some room is left, too little for the 82 MB that all of dZ would take
             torch.cuda.empty_cache()
             both(T)
             c.sync()
