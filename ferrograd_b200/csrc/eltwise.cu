@@ -266,23 +266,24 @@ template <> struct Stored<FG_DTYPE_BF16> {
 // The host turns a chain (forward, or backward = the values it needs followed by the adjoints) into a list of
 // single-result operations: instructions whose result nobody reads are dropped, an adjoint's first contribution is a
 // plain result and only later ones add, and results live in a few slots that are reused once their last reader has run.
-// The kernel keeps one set of values in registers: the result of the operation just before (`last`).  An operation takes
-// its first operand there (fetched from its slot if it is another value) and leaves its result there.
+// The kernel keeps one set of values in registers, the result of the operation just before: an operation takes its first
+// operand there (fetched from its slot if it is another value), its second one from a slot, and leaves its result there.
 enum : uint32_t { VM_G_TANH = 14, VM_G_RELU, VM_G_GELU, VM_G_ELU, VM_G_ABS,      // after the fg_ew codes: result = op(x, y)
+                  VM_RSUB, VM_RDIV,                                              // y - x, y / x
                   VM_LD, VM_LD2, VM_ST, VM_LDADD, VM_COPY };
 static_assert(FG_EW_ELU + 1 == (int)VM_G_TANH, "the operation codes are dense: one jump table");
-constexpr uint32_t kLast = 254, kNone = 255;
-struct VmOp {            // x, y: slot, kLast or kNone.  acc: slot (result = acc + op) or kNone.  dst: slot or kNone
-    uint8_t op, dst, x, y;
-    uint8_t acc, ptr, ptr2, dst2;      // VM_LD2: ptr2 goes to slot dst2, ptr to `last` and dst
+constexpr uint32_t kVmFetch = 1, kVmAdd = 2, kVmKeep = 4;       // first operand from slot x; + slot acc; result to slot dst
+struct VmOp {                          // slots as offsets in units of 16 bytes
+    uint8_t op, flags, ptr, ptr2;      // VM_LD2: ptr2 goes to slot x, ptr to the registers
+    uint16_t x, y;
     float imm;
-    uint32_t pad;
+    uint16_t acc, dst;
 };
 static_assert(sizeof(VmOp) == 16, "one 128-bit constant load per operation");
 constexpr int kVmMaxOps = 200;      // backward: 24 values, the seed, at most five operations per instruction, 24 + 2 * 8 for the input gradients
 constexpr int kVmMaxPtrs = FG_EW_MAX_INPUTS + 1 + FG_EW_MAX_INSTR;
 struct VmArgs {
-    uint4 ops[kVmMaxOps];
+    uint4 ops[kVmMaxOps + 1];
     void* ptr[kVmMaxPtrs];
     int nops, vec;
     uint64_t n;
@@ -290,143 +291,220 @@ struct VmArgs {
 static_assert(sizeof(VmArgs) <= 4096, "kernel parameters");
 
 constexpr int kVmThreads = 128;
+constexpr int kVmWords = 8;         // 32-bit words of a value that a thread holds: eight f32 elements, or sixteen 16-bit ones in pairs
+constexpr int kVmSlotUnits = 2 * kVmThreads;
+
+// A value's words: Lanes<DT> does arithmetic on them.  16-bit types stay packed: + - * on two elements at once in the type's
+// own arithmetic, which rounds as an operation in f32 followed by a rounding to the type does (f32 has more than twice the
+// bits); functions and the quotient on f32 lanes.
+template <int DT> struct Lanes {
+    typedef Stored<DT> S;
+    typedef typename std::conditional<DT == FG_DTYPE_F16, __half2, __nv_bfloat162>::type P;
+    static constexpr int kE = 2;
+    static __device__ __forceinline__ P p(uint32_t u) { return *reinterpret_cast<P*>(&u); }
+    static __device__ __forceinline__ uint32_t u(P v) { return *reinterpret_cast<uint32_t*>(&v); }
+    static __device__ __forceinline__ float2 f(uint32_t v) {
+        if constexpr (DT == FG_DTYPE_F16) return __half22float2(p(v));
+        else return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    }
+    static __device__ __forceinline__ uint32_t pack(float a, float b) {
+        if constexpr (DT == FG_DTYPE_F16) return u(__floats2half2_rn(a, b));
+        else return u(__floats2bfloat162_rn(a, b));
+    }
+    static __device__ __forceinline__ uint32_t all(float v) { return pack(v, v); }
+    static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) { return u(__hadd2_rn(p(a), p(b))); }
+    static __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b) { return u(__hsub2_rn(p(a), p(b))); }
+    static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) { return u(__hmul2_rn(p(a), p(b))); }
+    static __device__ __forceinline__ uint32_t neg(uint32_t a) { return a ^ 0x80008000u; }
+    static __device__ __forceinline__ uint32_t abs(uint32_t a) { return a & 0x7fff7fffu; }
+    static __device__ __forceinline__ uint32_t relu(uint32_t a) { return u(__hmax2(p(a), p(0u))); }          // max(NaN, 0) = 0
+    static __device__ __forceinline__ uint32_t positive(uint32_t a) { return u(__hgt2(p(a), p(0u))); }       // 1 or 0
+    static __device__ __forceinline__ uint32_t where_ge0(uint32_t c, uint32_t a, uint32_t b) {               // c >= 0 ? a : b
+        const uint32_t m = __hge2_mask(p(c), p(0u));
+        return (a & m) | (b & ~m);
+    }
+    template <class F> static __device__ __forceinline__ uint32_t map(uint32_t a, F fn) {
+        const float2 x = f(a);
+        return pack(fn(x.x), fn(x.y));
+    }
+    template <class F> static __device__ __forceinline__ uint32_t map(uint32_t a, uint32_t b, F fn) {
+        const float2 x = f(a), y = f(b);
+        return pack(fn(x.x, y.x), fn(x.y, y.y));
+    }
+    // Element h of a word, from or to a tensor
+    static __device__ __forceinline__ uint32_t bits(const void* t, uint64_t i) { return static_cast<const uint16_t*>(t)[i]; }
+    static __device__ __forceinline__ void put(void* t, uint64_t i, uint32_t v) { static_cast<uint16_t*>(t)[i] = (uint16_t)v; }
+};
+template <> struct Lanes<FG_DTYPE_F32> {
+    static constexpr int kE = 1;
+    static __device__ __forceinline__ float f(uint32_t v) { return __uint_as_float(v); }
+    static __device__ __forceinline__ uint32_t u(float v) { return __float_as_uint(v); }
+    static __device__ __forceinline__ uint32_t all(float v) { return u(v); }
+    static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) { return u(f(a) + f(b)); }
+    static __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b) { return u(f(a) - f(b)); }
+    static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) { return u(f(a) * f(b)); }
+    static __device__ __forceinline__ uint32_t neg(uint32_t a) { return a ^ 0x80000000u; }
+    static __device__ __forceinline__ uint32_t abs(uint32_t a) { return a & 0x7fffffffu; }
+    static __device__ __forceinline__ uint32_t relu(uint32_t a) { return u(f(a) > 0.0f ? f(a) : 0.0f); }
+    static __device__ __forceinline__ uint32_t positive(uint32_t a) { return u(f(a) > 0.0f ? 1.0f : 0.0f); }
+    static __device__ __forceinline__ uint32_t where_ge0(uint32_t c, uint32_t a, uint32_t b) { return f(c) >= 0.0f ? a : b; }
+    template <class F> static __device__ __forceinline__ uint32_t map(uint32_t a, F fn) { return u(fn(f(a))); }
+    template <class F> static __device__ __forceinline__ uint32_t map(uint32_t a, uint32_t b, F fn) { return u(fn(f(a), f(b))); }
+};
 
 // Slots are in shared memory (a program is only known at run time, so its values cannot be named registers): a slot holds
-// eight values of each thread as two planes of one float4 per thread, so that every access is a conflict-free 128-bit one.
-template <int W> __device__ __forceinline__ void slot_ld(const float4* sm, uint32_t slot, float* o) {
-    if constexpr (W == 8) {
-        const float4 a = sm[(slot * 2) * kVmThreads], b = sm[(slot * 2 + 1) * kVmThreads];
+// the words of each thread as two planes of one uint4 per thread, so that every access is a conflict-free 128-bit one.
+__device__ __forceinline__ void slot_ld(const uint4* sm, uint32_t off, uint32_t* o) {
+    const uint4 a = sm[off], b = sm[off + kVmThreads];
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+}
+__device__ __forceinline__ void slot_st(uint4* sm, uint32_t off, const uint32_t* v) {
+    sm[off] = make_uint4(v[0], v[1], v[2], v[3]);
+    sm[off + kVmThreads] = make_uint4(v[4], v[5], v[6], v[7]);
+}
+
+// A thread's words of a tensor.  VEC: groups of four elements, kVmThreads groups apart, in a tile that is whole; otherwise
+// single elements, kVmThreads apart, as far as the tensor goes.
+template <int DT, bool VEC>
+__device__ __forceinline__ void words_ld(const void* t, uint64_t i, uint64_t n, uint32_t* o) {
+    if constexpr (VEC && DT == FG_DTYPE_F32) {
+        const uint4* p = reinterpret_cast<const uint4*>(static_cast<const float*>(t) + i);
+        const uint4 a = p[0], b = p[kVmThreads];
         o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-    } else {
-        o[0] = reinterpret_cast<const float*>(sm + slot * 2 * kVmThreads)[0];
-    }
-}
-template <int W> __device__ __forceinline__ void slot_st(float4* sm, uint32_t slot, const float* v) {
-    if constexpr (W == 8) {
-        sm[(slot * 2) * kVmThreads] = make_float4(v[0], v[1], v[2], v[3]);
-        sm[(slot * 2 + 1) * kVmThreads] = make_float4(v[4], v[5], v[6], v[7]);
-    } else {
-        reinterpret_cast<float*>(sm + slot * 2 * kVmThreads)[0] = v[0];
-    }
-}
-
-// One operation on W elements, in place: the op-code is decoded once, the lanes loop inside each case.
-#define FG_VM_LANES(expr)                                                                                   \
-    do {                                                                                                    \
-        _Pragma("unroll") for (int w = 0; w < W; ++w) { const float xx = x[w], yy = y[w]; (void)xx; (void)yy; x[w] = (expr); } \
-    } while (0)
-template <int DT, int W>
-__device__ __forceinline__ void vm_op(uint32_t op, float imm, float* x, const float* y) {
-    typedef Stored<DT> S;
-    switch (op) {
-        case FG_EW_CONST: FG_VM_LANES(S::r(imm)); break;
-        case FG_EW_ADD: FG_VM_LANES(S::r(xx + yy)); break;
-        case FG_EW_SUB: FG_VM_LANES(S::r(xx - yy)); break;
-        case FG_EW_MUL: FG_VM_LANES(S::r(xx * yy)); break;
-        case FG_EW_DIV: FG_VM_LANES(S::r(__fdiv_rn(xx, yy))); break;
-        case FG_EW_NEG: FG_VM_LANES(-xx); break;
-        case FG_EW_ABS: FG_VM_LANES(fabsf(xx)); break;
-        case FG_EW_EXP: FG_VM_LANES(S::r(expf(xx))); break;
-        case FG_EW_LOG: FG_VM_LANES(S::r(logf(xx))); break;
-        case FG_EW_TANH: FG_VM_LANES(S::r(tanhf(xx))); break;
-        case FG_EW_RELU: FG_VM_LANES(xx > 0.0f ? xx : 0.0f); break;
-        case FG_EW_GELU: FG_VM_LANES(S::r(fg_gelu_fwd(xx))); break;
-        case FG_EW_ELU: FG_VM_LANES(xx >= 0.0f ? xx : S::r(expf(xx) - 1.0f)); break;
-        // adjoints: x is the adjoint of the result, y the value the derivative is taken at
-        case VM_G_TANH: FG_VM_LANES(S::r(xx * S::r(1.0f - S::r(yy * yy)))); break;
-        case VM_G_RELU: FG_VM_LANES(xx * (yy > 0.0f ? 1.0f : 0.0f)); break;
-        case VM_G_GELU: FG_VM_LANES(S::r(xx * S::r(fg_gelu_grad(yy)))); break;
-        case VM_G_ELU: FG_VM_LANES(yy >= 0.0f ? xx : S::r(xx * S::r(yy + 1.0f))); break;
-        case VM_G_ABS: FG_VM_LANES(yy >= 0.0f ? xx : -xx); break;
-        default: break;      // VM_COPY
-    }
-}
-#undef FG_VM_LANES
-
-// The program on W elements: VEC (W = 8), i .. i+3 and i2 .. i2+3 (the second four only when `two`), or singly i, i + 128, ...
-// as far as the tensors go.
-template <int DT, int W, bool VEC>
-__device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint64_t i2, bool two, float4* sm) {
-    typedef Stored<DT> S;
-    auto load = [&](const void* p, float* o) {
-        if constexpr (VEC) {
-            S::ld4w(p, i, o);
-            if (two) S::ld4w(p, i2, o + 4);
-            else o[4] = o[5] = o[6] = o[7] = 0.0f;
-        } else {
+    } else if constexpr (VEC) {
+        const uint2* p = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(t) + i);
 #pragma unroll
-            for (int w = 0; w < W; ++w) o[w] = i + w * kVmThreads < a.n ? S::ld(p, i + w * kVmThreads) : 0.0f;
+        for (int j = 0; j < 4; ++j) { const uint2 a = p[j * kVmThreads]; o[2 * j] = a.x; o[2 * j + 1] = a.y; }
+    } else if constexpr (DT == FG_DTYPE_F32) {
+#pragma unroll
+        for (int w = 0; w < kVmWords; ++w) o[w] = i + w * kVmThreads < n ? static_cast<const uint32_t*>(t)[i + w * kVmThreads] : 0u;
+    } else {
+#pragma unroll
+        for (int w = 0; w < kVmWords; ++w) {
+            const uint64_t e = i + 2 * w * kVmThreads;
+            o[w] = (e < n ? Lanes<DT>::bits(t, e) : 0u) | (e + kVmThreads < n ? Lanes<DT>::bits(t, e + kVmThreads) : 0u) << 16;
         }
-    };
-    float last[W], y[W];
+    }
+}
+template <int DT, bool VEC>
+__device__ __forceinline__ void words_st(void* t, uint64_t i, uint64_t n, const uint32_t* v) {
+    if constexpr (VEC && DT == FG_DTYPE_F32) {
+        uint4* p = reinterpret_cast<uint4*>(static_cast<float*>(t) + i);
+        p[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        p[kVmThreads] = make_uint4(v[4], v[5], v[6], v[7]);
+    } else if constexpr (VEC) {
+        uint2* p = reinterpret_cast<uint2*>(static_cast<uint16_t*>(t) + i);
 #pragma unroll
-    for (int w = 0; w < W; ++w) last[w] = y[w] = 0.0f;
-    uint4 c = a.ops[0];
+        for (int j = 0; j < 4; ++j) p[j * kVmThreads] = make_uint2(v[2 * j], v[2 * j + 1]);
+    } else if constexpr (DT == FG_DTYPE_F32) {
+#pragma unroll
+        for (int w = 0; w < kVmWords; ++w)
+            if (i + w * kVmThreads < n) static_cast<uint32_t*>(t)[i + w * kVmThreads] = v[w];
+    } else {
+#pragma unroll
+        for (int w = 0; w < kVmWords; ++w) {
+            const uint64_t e = i + 2 * w * kVmThreads;
+            if (e < n) Lanes<DT>::put(t, e, v[w]);
+            if (e + kVmThreads < n) Lanes<DT>::put(t, e + kVmThreads, v[w] >> 16);
+        }
+    }
+}
+
+// The program on a thread's elements of one tile, the first of them i.  The only values that live from one operation to the
+// next are v[] and the words of the next operation; every second operand is fetched inside the case that reads it.
+template <int DT, bool VEC>
+__device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
+    typedef Lanes<DT> L;
+    uint32_t v[kVmWords];
+#pragma unroll
+    for (int w = 0; w < kVmWords; ++w) v[w] = 0u;
+    uint4 next = a.ops[0];
+#define FG_VM_1(expr) _Pragma("unroll") for (int w = 0; w < kVmWords; ++w) { const uint32_t x = v[w]; v[w] = (expr); } break
+#define FG_VM_2(expr)                                                                                       \
+    {                                                                                                       \
+        uint32_t yy[kVmWords];                                                                              \
+        slot_ld(sm, c.y >> 16, yy);                                                                         \
+        _Pragma("unroll") for (int w = 0; w < kVmWords; ++w) { const uint32_t x = v[w], y = yy[w]; v[w] = (expr); } \
+    } break
 #pragma unroll 1
     for (int k = 0; k < a.nops; ++k) {
-        const uint32_t op = c.x & 255u, dst = c.x >> 8 & 255u, xs = c.x >> 16 & 255u, ys = c.x >> 24;
-        const uint32_t acc = c.y & 255u, ptr = c.y >> 8 & 255u, ptr2 = c.y >> 16 & 255u, dst2 = c.y >> 24;
-        const float imm = __uint_as_float(c.z);
-        c = a.ops[k + 1 < kVmMaxOps ? k + 1 : k];       // the next operation's code is on its way during this one
-        if (ys == kLast) {
-#pragma unroll
-            for (int w = 0; w < W; ++w) y[w] = last[w];
-        } else if (ys != kNone) {
-            slot_ld<W>(sm, ys, y);
-        }
-        if (xs < kLast) slot_ld<W>(sm, xs, last);
-        if (op < VM_LD) {
-            vm_op<DT, W>(op, imm, last, y);
-        } else if (op == VM_LD) {
-            load(a.ptr[ptr], last);
-        } else if (op == VM_LD2) {                      // both on their way at once
-            load(a.ptr[ptr2], y);
-            load(a.ptr[ptr], last);
-            slot_st<W>(sm, dst2, y);
-        } else if (op == VM_ST) {
-            if constexpr (VEC) {
-                S::st4w(a.ptr[ptr], i, last);
-                if (two) S::st4w(a.ptr[ptr], i2, last + 4);
-            } else {
-#pragma unroll
-                for (int w = 0; w < W; ++w)
-                    if (i + w * kVmThreads < a.n) S::st(a.ptr[ptr], i + w * kVmThreads, last[w]);
+        const uint4 c = next;
+        next = a.ops[k + 1];       // the next operation's code is on its way during this one
+        const uint32_t flags = c.x >> 8;
+        if (flags & kVmFetch) slot_ld(sm, c.y & 0xffffu, v);
+        switch (c.x & 255u) {
+            case FG_EW_CONST: {
+                const uint32_t k0 = L::all(__uint_as_float(c.z));
+                FG_VM_1((void(x), k0));
             }
-        } else if (op == VM_LDADD) {
-            load(a.ptr[ptr], y);
+            case FG_EW_ADD: FG_VM_2(L::add(x, y));
+            case FG_EW_SUB: FG_VM_2(L::sub(x, y));
+            case VM_RSUB: FG_VM_2(L::sub(y, x));
+            case FG_EW_MUL: FG_VM_2(L::mul(x, y));
+            case FG_EW_DIV: FG_VM_2(L::map(x, y, [](float p, float q) { return __fdiv_rn(p, q); }));
+            case VM_RDIV: FG_VM_2(L::map(y, x, [](float p, float q) { return __fdiv_rn(p, q); }));
+            case FG_EW_NEG: FG_VM_1(L::neg(x));
+            case FG_EW_ABS: FG_VM_1(L::abs(x));
+            case FG_EW_EXP: FG_VM_1(L::map(x, [](float p) { return expf(p); }));
+            case FG_EW_LOG: FG_VM_1(L::map(x, [](float p) { return logf(p); }));
+            case FG_EW_TANH: FG_VM_1(L::map(x, [](float p) { return tanhf(p); }));
+            case FG_EW_RELU: FG_VM_1(L::relu(x));
+            case FG_EW_GELU: FG_VM_1(L::map(x, [](float p) { return fg_gelu_fwd(p); }));
+            case FG_EW_ELU: FG_VM_1(L::map(x, [](float p) { return p >= 0.0f ? p : expf(p) - 1.0f; }));
+            // adjoints: x is the adjoint of the result, y the value the derivative is taken at
+            case VM_G_TANH: FG_VM_2(L::mul(x, L::sub(L::all(1.0f), L::mul(y, y))));
+            case VM_G_RELU: FG_VM_2(L::mul(x, L::positive(y)));
+            case VM_G_GELU: FG_VM_2(L::mul(x, L::map(y, [](float p) { return fg_gelu_grad(p); })));
+            case VM_G_ELU: FG_VM_2(L::where_ge0(y, x, L::mul(x, L::add(y, L::all(1.0f)))));
+            case VM_G_ABS: FG_VM_2(L::where_ge0(y, x, L::neg(x)));
+            case VM_LD: words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
+            case VM_LD2: {                                  // both on their way at once
+                uint32_t yy[kVmWords];
+                words_ld<DT, VEC>(a.ptr[c.x >> 24], i, a.n, yy);
+                words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v);
+                slot_st(sm, c.y & 0xffffu, yy);
+                break;
+            }
+            case VM_ST: words_st<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
+            case VM_LDADD: {
+                uint32_t yy[kVmWords];
+                words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, yy);
 #pragma unroll
-            for (int w = 0; w < W; ++w) last[w] = S::r(y[w] + last[w]);
+                for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
+                break;
+            }
+            default: break;      // VM_COPY
         }
-        if (acc != kNone) {
-            slot_ld<W>(sm, acc, y);
+        if (flags & kVmAdd) {
+            uint32_t yy[kVmWords];
+            slot_ld(sm, c.w & 0xffffu, yy);
 #pragma unroll
-            for (int w = 0; w < W; ++w) last[w] = S::r(y[w] + last[w]);
+            for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
         }
-        if (dst != kNone) slot_st<W>(sm, dst, last);
+        if (flags & kVmKeep) slot_st(sm, c.w >> 16, v);
     }
+#undef FG_VM_1
+#undef FG_VM_2
 }
 
-// A block takes 1024 consecutive elements at a time: thread t the groups of four t and t + 128 of them (every access of a
-// warp is contiguous), the last n % 4 elements singly, on the last block, which has the least other work; or, when a tensor
-// starts off the boundary that groups of four need, elements t, t + 128, ... singly.
-//
-// What bounds it: instruction issue (about 25 instructions to fetch, decode and store an operation, shared by eight elements).
-// gelu(x * y) + x on 32 Mi f32 elements: forward 147 -> 100 us, backward 340 -> 168 us against one interpreter step per
-// instruction and word-wise slots; x / (1 + exp(-x)) * y on 3 M halves 18.4 -> 14.8 us and 49.6 -> 30 us.  Off the boundary:
-// the adjoints of tanh(x / (1 + |y|)) on 3 M words 125 us with one element per thread and operation, 34 with eight.
+// A block takes one tile of kVmWords words per thread at a time; block 0 of a vectorised launch has the incomplete last tile
+// instead, element by element.
 template <int DT, bool VEC>
-__global__ void __launch_bounds__(kVmThreads) chain_kernel(const __grid_constant__ VmArgs a) {
+__global__ void __launch_bounds__(kVmThreads, 10) chain_kernel(const __grid_constant__ VmArgs a) {
     fg_grid_enter();
-    extern __shared__ float4 chain_smem[];
-    float4* const sm = chain_smem + threadIdx.x;
+    extern __shared__ uint4 chain_smem[];
+    uint4* const sm = chain_smem + threadIdx.x;
+    constexpr uint32_t kTile = kVmWords * Lanes<DT>::kE * kVmThreads;
     if constexpr (VEC) {
-        const uint64_t nv = a.n >> 2;
-        if (blockIdx.x == gridDim.x - 1 && (nv << 2) + threadIdx.x < a.n) vm_run<DT, 1, false>(a, (nv << 2) + threadIdx.x, 0, false, sm);
-        for (uint64_t g = (uint64_t)blockIdx.x * (2 * kVmThreads) + threadIdx.x; g < nv; g += (uint64_t)gridDim.x * (2 * kVmThreads))
-            vm_run<DT, 8, true>(a, g << 2, (g + kVmThreads) << 2, g + kVmThreads < nv, sm);
+        const uint64_t whole = a.n / kTile;
+        const uint32_t rest = a.n % kTile != 0;
+        if (rest && blockIdx.x == 0) {
+            vm_run<DT, false>(a, whole * kTile + threadIdx.x, sm);
+            return;
+        }
+        for (uint64_t t = blockIdx.x - rest; t < whole; t += gridDim.x - rest) vm_run<DT, true>(a, t * kTile + threadIdx.x * 4, sm);
     } else {
-        for (uint64_t i = (uint64_t)blockIdx.x * (8 * kVmThreads) + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * (8 * kVmThreads))
-            vm_run<DT, 8, false>(a, i, 0, false, sm);
+        for (uint64_t t = blockIdx.x; t * kTile < a.n; t += gridDim.x) vm_run<DT, false>(a, t * kTile + threadIdx.x, sm);
     }
 }
 
@@ -472,39 +550,42 @@ struct VmBuilder {
         int prev = -1;      // the value that is in `last` before operation i
         for (int i = 0; i < n; ++i) {
             Node& o = node[i];
-            // what is in the registers serves as the first operand where the order does not matter
-            if ((o.op == FG_EW_ADD || o.op == FG_EW_MUL) && o.y == prev && o.x != prev) { const int t = o.x; o.x = o.y; o.y = t; }
-            for (int u : {o.x, o.y})
-                if (u >= 0 && u != prev) { stored[u] = true; last_use[u] = i; }
+            // what is in the registers serves as the first operand
+            if (o.y == prev && o.x != prev && o.op >= FG_EW_ADD && o.op <= FG_EW_DIV) {
+                const int t = o.x; o.x = o.y; o.y = t;
+                o.op = o.op == FG_EW_SUB ? (int)VM_RSUB : o.op == FG_EW_DIV ? (int)VM_RDIV : o.op;
+            }
+            if (o.x >= 0 && o.x != prev) { stored[o.x] = true; last_use[o.x] = i; }
+            if (o.y >= 0) { stored[o.y] = true; last_use[o.y] = i; }
             if (o.acc >= 0) { stored[o.acc] = true; last_use[o.acc] = i; }
             if (o.id2 >= 0) { stored[o.id2] = true; if (last_use[o.id2] < i) last_use[o.id2] = i; }
             prev = next_last(o, prev);
         }
         int nslots = 0;
-        auto take = [&](int id) -> uint8_t {
+        auto take = [&](int id) {
             int f = 0;
             while (taken[f]) ++f;
             taken[f] = true;
             slot[id] = f;
             if (f + 1 > nslots) nslots = f + 1;
-            return (uint8_t)f;
         };
         prev = -1;
         for (int i = 0; i < n; ++i) {
             const Node& o = node[i];
-            auto where = [&](int u) -> uint8_t { return u < 0 ? (uint8_t)kNone : u == prev ? (uint8_t)kLast : (uint8_t)slot[u]; };
+            auto at = [&](int u) -> uint16_t { return u < 0 ? (uint16_t)0 : (uint16_t)(slot[u] * kVmSlotUnits); };
             VmOp v{};
             v.op = (uint8_t)o.op;
-            v.x = where(o.x); v.y = where(o.y);
-            v.acc = o.acc < 0 ? (uint8_t)kNone : (uint8_t)slot[o.acc];
+            if (o.x >= 0 && o.x != prev) { v.flags |= kVmFetch; v.x = at(o.x); }
+            v.y = at(o.y);
+            if (o.acc >= 0) { v.flags |= kVmAdd; v.acc = at(o.acc); }
             v.ptr = (uint8_t)(o.ptr < 0 ? 0 : o.ptr);
             v.ptr2 = (uint8_t)(o.ptr2 < 0 ? 0 : o.ptr2);
             v.imm = o.imm;
-            if (o.id2 >= 0) v.dst2 = take(o.id2);
+            if (o.id2 >= 0) { take(o.id2); v.x = at(o.id2); }
             // a slot whose last reader this is may receive the result: operands are read before it is written
             for (int u : {o.x, o.y, o.acc, o.id2})
                 if (u >= 0 && slot[u] >= 0 && last_use[u] == i && !(u == o.id2 && o.op != (int)VM_LD2)) taken[slot[u]] = false;
-            v.dst = o.id >= 0 && stored[o.id] ? take(o.id) : (uint8_t)kNone;
+            if (o.id >= 0 && stored[o.id]) { take(o.id); v.flags |= kVmKeep; v.dst = at(o.id); }
             prev = next_last(o, prev);
             memcpy(&a->ops[i], &v, sizeof(v));
         }
@@ -637,7 +718,7 @@ __global__ void __launch_bounds__(256) convert_kernel(const void* __restrict__ s
 
 // A program with many live values needs more than the default 48 KB of dynamic shared memory (4 KB per slot, and there
 // are at most 24 values and 24 adjoints): the limit is raised once per device and kernel.
-constexpr int kSlotBytes = 8 * kVmThreads * (int)sizeof(float);
+constexpr int kSlotBytes = kVmSlotUnits * (int)sizeof(uint4);
 constexpr int kChainSmemMax = 2 * FG_EW_MAX_INSTR * kSlotBytes;
 int32_t launch_chain(fg_ctx* ctx, int dtype, VmBuilder& b, VmArgs& a, double bytes) {
     static std::atomic<uint64_t> done[3][2];
@@ -655,10 +736,14 @@ int32_t launch_chain(fg_ctx* ctx, int dtype, VmBuilder& b, VmArgs& a, double byt
         if (e != cudaSuccess) return fg_fail_cuda(ctx, FG_ERR_INTERNAL, "cudaFuncSetAttribute(chain kernel)", e);
         set.fetch_or(bit, std::memory_order_release);
     }
-    // as many blocks as the shared memory lets an SM hold (of at most sixteen)
+    // As many blocks as an SM holds at once (ten by registers, fewer when the slots fill the shared memory), each with the same
+    // number of tiles: a grid of sixteen per SM ran as one full wave and a second of three quarters.
     const size_t fit = (220u * 1024u) / (smem + 1024);
-    const int per_sm = (int)(fit < 1 ? 1 : fit > 16 ? 16 : fit);
-    const int grid = fg_stream_grid(ctx, a.vec ? (a.n / 4 + 1) / 2 : (a.n + 7) / 8, kVmThreads, per_sm);
+    const uint64_t tile = (uint64_t)kVmWords * (dtype == FG_DTYPE_F32 ? 1 : 2) * kVmThreads;
+    const uint64_t rest = a.vec && a.n % tile ? 1 : 0, tiles = a.vec ? a.n / tile : (a.n + tile - 1) / tile;
+    const uint64_t cap = (uint64_t)ctx->sm_count * (fit < 1 ? 1 : fit > 10 ? 10 : fit) - rest;
+    const uint64_t rounds = tiles ? (tiles + cap - 1) / cap : 1;
+    const int grid = (int)((tiles + rounds - 1) / rounds + rest);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, bytes);
     fg_launch(ctx, kernel, grid, kVmThreads, smem, a);
     fg_time_end(ctx, tr);
