@@ -272,18 +272,18 @@ enum : uint32_t { VM_G_TANH = 14, VM_G_RELU, VM_G_GELU, VM_G_ELU, VM_G_ABS,     
                   VM_RSUB, VM_RDIV,                                              // y - x, y / x
                   VM_LD, VM_LD2, VM_ST, VM_LDADD, VM_COPY };
 static_assert(FG_EW_ELU + 1 == (int)VM_G_TANH, "the operation codes are dense: one jump table");
-constexpr uint32_t kVmFetch = 1, kVmAdd = 2, kVmKeep = 4;       // first operand from slot x; + slot acc; result to slot dst
+constexpr uint32_t kVmFetch = 0x100, kVmAdd = 0x200, kVmKeep = 0x400;       // first operand from slot x; + slot acc; result to slot dst
 struct VmOp {                          // slots as offsets in units of 16 bytes
-    uint8_t op, flags, ptr, ptr2;      // VM_LD2: ptr2 goes to slot x, ptr to the registers
-    uint16_t x, y;
-    float imm;
-    uint16_t acc, dst;
+    uint8_t op, flags, ptr, ptr2;      // VM_LD2: ptr2 goes to slot y, ptr to the registers
+    uint32_t y;                        // FG_EW_CONST: the constant's bits
+    uint16_t x, acc;
+    uint32_t dst;
 };
 static_assert(sizeof(VmOp) == 16, "one 128-bit constant load per operation");
 constexpr int kVmMaxOps = 200;      // backward: 24 values, the seed, at most five operations per instruction, 24 + 2 * 8 for the input gradients
 constexpr int kVmMaxPtrs = FG_EW_MAX_INPUTS + 1 + FG_EW_MAX_INSTR;
 struct VmArgs {
-    uint4 ops[kVmMaxOps + 1];
+    uint4 ops[kVmMaxOps];
     void* ptr[kVmMaxPtrs];
     int nops, vec;
     uint64_t n;
@@ -411,30 +411,34 @@ __device__ __forceinline__ void words_st(void* t, uint64_t i, uint64_t n, const 
 }
 
 // The program on a thread's elements of one tile, the first of them i.  The only values that live from one operation to the
-// next are v[] and the words of the next operation; every second operand is fetched inside the case that reads it.
+// next are v[]; every second operand is fetched inside the case that reads it.
+//
+// What bounds it: instruction issue, on large f32 tensors together with HBM.  Fetching, decoding and keeping one operation
+// takes about 35 instructions for the eight words (70 with both operands live across the loop, ncu's executed instructions).
+// Forward and backward: gelu(x * y) + x on 32 Mi f32 257 -> 211 us (3.8 TB/s), x / (1 + exp(-x)) * y on 3 000 001 halves
+// 42.3 -> 21.5 us, with both launches.  Requesting the next tile's words ahead through cp.async lost 6 % (the copies out of the
+// staging cost more issue slots than the waits); sixteen words per thread gain 3 % in f32 and lose 30 % on halves.
 template <int DT, bool VEC>
 __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
     typedef Lanes<DT> L;
     uint32_t v[kVmWords];
 #pragma unroll
     for (int w = 0; w < kVmWords; ++w) v[w] = 0u;
-    uint4 next = a.ops[0];
 #define FG_VM_1(expr) _Pragma("unroll") for (int w = 0; w < kVmWords; ++w) { const uint32_t x = v[w]; v[w] = (expr); } break
 #define FG_VM_2(expr)                                                                                       \
     {                                                                                                       \
         uint32_t yy[kVmWords];                                                                              \
-        slot_ld(sm, c.y >> 16, yy);                                                                         \
+        slot_ld(sm, c.y, yy);                                                                         \
         _Pragma("unroll") for (int w = 0; w < kVmWords; ++w) { const uint32_t x = v[w], y = yy[w]; v[w] = (expr); } \
     } break
 #pragma unroll 1
     for (int k = 0; k < a.nops; ++k) {
-        const uint4 c = next;
-        next = a.ops[k + 1];       // the next operation's code is on its way during this one
-        const uint32_t flags = c.x >> 8;
-        if (flags & kVmFetch) slot_ld(sm, c.y & 0xffffu, v);
+        const uint4 c = a.ops[k];
+        const uint32_t flags = c.x;
+        if (flags & kVmFetch) slot_ld(sm, c.z & 0xffffu, v);
         switch (c.x & 255u) {
             case FG_EW_CONST: {
-                const uint32_t k0 = L::all(__uint_as_float(c.z));
+                const uint32_t k0 = L::all(__uint_as_float(c.y));
                 FG_VM_1((void(x), k0));
             }
             case FG_EW_ADD: FG_VM_2(L::add(x, y));
@@ -462,7 +466,7 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
                 uint32_t yy[kVmWords];
                 words_ld<DT, VEC>(a.ptr[c.x >> 24], i, a.n, yy);
                 words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v);
-                slot_st(sm, c.y & 0xffffu, yy);
+                slot_st(sm, c.y, yy);
                 break;
             }
             case VM_ST: words_st<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
@@ -473,22 +477,25 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
                 for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
                 break;
             }
-            default: break;      // VM_COPY
+            case VM_COPY: break;
+            default: __builtin_unreachable();      // the host writes no other code: the jump needs no range check
         }
-        if (flags & kVmAdd) {
-            uint32_t yy[kVmWords];
-            slot_ld(sm, c.w & 0xffffu, yy);
+        if (flags & (kVmAdd | kVmKeep)) {
+            if (flags & kVmAdd) {
+                uint32_t yy[kVmWords];
+                slot_ld(sm, c.z >> 16, yy);
 #pragma unroll
-            for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
+                for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
+            }
+            if (flags & kVmKeep) slot_st(sm, c.w, v);
         }
-        if (flags & kVmKeep) slot_st(sm, c.w >> 16, v);
     }
 #undef FG_VM_1
 #undef FG_VM_2
 }
 
 // A block takes one tile of kVmWords words per thread at a time; block 0 of a vectorised launch has the incomplete last tile
-// instead, element by element.
+// instead, element by element, so that no other tile needs bounds.
 template <int DT, bool VEC>
 __global__ void __launch_bounds__(kVmThreads, 10) chain_kernel(const __grid_constant__ VmArgs a) {
     fg_grid_enter();
@@ -575,17 +582,17 @@ struct VmBuilder {
             auto at = [&](int u) -> uint16_t { return u < 0 ? (uint16_t)0 : (uint16_t)(slot[u] * kVmSlotUnits); };
             VmOp v{};
             v.op = (uint8_t)o.op;
-            if (o.x >= 0 && o.x != prev) { v.flags |= kVmFetch; v.x = at(o.x); }
+            if (o.x >= 0 && o.x != prev) { v.flags |= kVmFetch >> 8; v.x = at(o.x); }
             v.y = at(o.y);
-            if (o.acc >= 0) { v.flags |= kVmAdd; v.acc = at(o.acc); }
+            if (o.acc >= 0) { v.flags |= kVmAdd >> 8; v.acc = at(o.acc); }
             v.ptr = (uint8_t)(o.ptr < 0 ? 0 : o.ptr);
             v.ptr2 = (uint8_t)(o.ptr2 < 0 ? 0 : o.ptr2);
-            v.imm = o.imm;
-            if (o.id2 >= 0) { take(o.id2); v.x = at(o.id2); }
+            if (o.op == FG_EW_CONST) memcpy(&v.y, &o.imm, 4);
+            if (o.id2 >= 0) { take(o.id2); v.y = at(o.id2); }
             // a slot whose last reader this is may receive the result: operands are read before it is written
             for (int u : {o.x, o.y, o.acc, o.id2})
                 if (u >= 0 && slot[u] >= 0 && last_use[u] == i && !(u == o.id2 && o.op != (int)VM_LD2)) taken[slot[u]] = false;
-            if (o.id >= 0 && stored[o.id]) { take(o.id); v.flags |= kVmKeep; v.dst = at(o.id); }
+            if (o.id >= 0 && stored[o.id]) { take(o.id); v.flags |= kVmKeep >> 8; v.dst = at(o.id); }
             prev = next_last(o, prev);
             memcpy(&a->ops[i], &v, sizeof(v));
         }
