@@ -1253,28 +1253,31 @@ int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 
 // The pair kernel needs bf16 pairs in HBM and works in 256 x 256 tiles on two SMs; a product of a
 // few such tiles leaves most SMs idle, and making the pairs of a tensor that is read once costs
 // as much as reading it twice more.  Here a CTA owns a 128 x BN tile, loads the raw f32 words of
-// both operands (half the bytes of tensor plus pairs) and converter warps write the bf16
-// planes of each k-block beside it in shared memory, in the layout a bulk-tensor load would have
-// given them.  A matrix index and a K-share ride in the grid, so that one launch covers a batch and
-// fills the SMs; K-shares are folded by gemm_tc_fold_kernel.
+// both operands (half the bytes of tensor plus pairs) and converter warps split each k-block: A into
+// tensor memory, from where the MMAs read it, B's bf16 planes beside its words in shared memory, in the
+// layout a bulk-tensor load would have given them.  A matrix index and a K-share ride in the grid, so that
+// one launch covers a batch and fills the SMs; K-shares are folded by gemm_tc_fold_kernel.
 //   warp 0 loads, warp 1 issues MMAs, warps 2..9 drain accumulators and store, the others convert.
 // Measured (before: operand planes or pairs, then a 256 x 256 or 128-row tile each): 100 x 4096 x 4096 129 -> 36 us,
 // 16 x (384 x 512 x 320) forward and backward 1530 -> 87 us, a 384-sample layer of 256 x 256 21.7 -> 9.8 us per product.
-// Bound by the converters and shared-memory bandwidth: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB
-// into the converters, 64 KB out of them and 64 KB into the MMAs, 192 KB at 128 B per cycle.
+// Bound by shared-memory bandwidth and the converters: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB
+// into the converters, 32 KB out of them (B) and 32 KB into the MMAs (B), 128 KB at 128 B per cycle; with A in shared
+// memory too it was 192 KB (100 x 4096 x 4096 34.9 -> 29.8 us, 16 x (384 x 512 x 320) forward and backward 86.3 -> 75.5 us).
 // ------------------------------------------------------------------------------------
 template <int BN>
 struct ConvCfg {
-    static constexpr int kA32 = BM * 32 * 4, kB32 = BN * 32 * 4;    // f32 tiles; the two bf16 planes take as much again
-    static constexpr int kStageBytes = 2 * (kA32 + kB32);
-    static constexpr int kStages = BN == 128 ? 3 : 4;
-    // Converters: all eight warps on each k-block in turn (BN = 128), or two per stage (BN = 64), see the kernel.
-    static constexpr int kGroups = BN == 128 ? 1 : kStages, kGroup = 256 / kGroups;
+    static constexpr int kA32 = BM * 32 * 4, kB32 = BN * 32 * 4;    // f32 tiles; B's two bf16 planes take as much again
+    static constexpr int kStageBytes = kA32 + 2 * kB32;
+    static constexpr int kStages = BN == 128 ? 4 : 6;
+    static constexpr int kACols = 64;                               // tensor memory per stage: A as f32 and as two bf16 planes
+    // Converters: groups of warps that take the k-blocks in turn, see the kernel.
+    static constexpr int kGroups = BN == 128 ? 1 : 2, kGroup = 256 / kGroups;
     static constexpr int kThreads = 320 + 256;
     static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
     static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
     static_assert(kStageBytes >= 8 * 32 * 32 * 4, "the epilogue stages its blocks in the first stage");
-    static constexpr int kTmemCols = 2 * BN;
+    static constexpr int kTmemCols = 512;
+    static_assert(2 * BN + kStages * kACols <= kTmemCols, "two accumulators and the stages of A");
 };
 
 // The split of a tile of ROWS rows x 32 k, eight elements per thread and step: the words are rounded to tf32
@@ -1324,6 +1327,36 @@ __device__ __forceinline__ void convert_tile(unsigned char* t32, bool mn, uint32
         *reinterpret_cast<uint4*>(h) = make_uint4(h0.x, h0.y, h1.x, h1.y);
         *reinterpret_cast<uint4*>(l) = make_uint4(l0.x, l0.y, l1.x, l1.y);
     }
+}
+
+// The same split of sixteen k of one row of A (128 rows x 32 k, the k from 16 * half on), into tensor memory: the words as the
+// kind::tf32 MMA reads them (one column per k), and the planes (two k per column).  A warp fills the 32 lanes it may touch.
+__device__ __forceinline__ void convert_a_row(const unsigned char* t32, bool mn, uint32_t q, uint32_t lane, uint32_t half, uint32_t taddr) {
+    float x[16];
+    if (!mn) {
+        const unsigned char* const r = t32 + (q * 32 + lane) * 128;
+#pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(r + (((half * 4 + c) ^ (lane & 7u)) << 4));
+            x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
+        }
+    } else {
+        const unsigned char* const b = t32 + q * 4096 + half * 2048 + (lane & 7u) * 4;
+#pragma unroll
+        for (uint32_t k = 0; k < 16; ++k) x[k] = *reinterpret_cast<const float*>(b + k * 128 + (((lane >> 3) ^ (k & 3u)) << 5));
+    }
+    uint32_t f[16], h[8], l[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float4 v = make_float4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]), r = round_tf32(v);
+        f[4 * c] = __float_as_uint(r.x); f[4 * c + 1] = __float_as_uint(r.y); f[4 * c + 2] = __float_as_uint(r.z); f[4 * c + 3] = __float_as_uint(r.w);
+        const uint2 hv = pack_bf16x4(v), lv = pack_bf16x4(make_float4(v.x - r.x, v.y - r.y, v.z - r.z, v.w - r.w));
+        h[2 * c] = hv.x; h[2 * c + 1] = hv.y;
+        l[2 * c] = lv.x; l[2 * c + 1] = lv.y;
+    }
+    tmem_st_32x16(taddr + half * 16, f);
+    tmem_st_32x8(taddr + 32 + half * 8, h);
+    tmem_st_32x8(taddr + 48 + half * 8, l);
 }
 
 // Descriptors of one converted operand tile: the f32 words, the two planes, and how far one MMA's k advances them.
@@ -1410,7 +1443,7 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     break;
                 }
                 mbar_expect_tx(full_bar(s), Cfg::kA32 + Cfg::kB32);
-                const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + 2 * Cfg::kA32;
+                const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + Cfg::kA32;
                 const int k = (int)((kb0 + i) * BK);
                 if (!a_mn) tma_load_3d(sa, &tmA, full_bar(s), k, (int)m0, (int)bz);
                 else
@@ -1425,7 +1458,7 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     } else if (warp == 1) {
         if (lane == 0) {
             // ---- MMA issuer ----
-            const uint32_t mnbits = (a_mn ? kIdescAMnMajor : 0u) | (b_mn ? kIdescBMnMajor : 0u);
+            const uint32_t mnbits = b_mn ? kIdescBMnMajor : 0u;
             const uint32_t idesc32 = make_idesc(2u /*tf32*/, BM, BN) | mnbits, idesc16 = make_idesc(1u /*bf16*/, BM, BN) | mnbits;
             bool ok = true;
             for (uint32_t c = 0; c < nchunks && ok; ++c) {
@@ -1446,28 +1479,29 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     }
                     tc_fence_after();
                     const uint32_t sa = base + s * Cfg::kStageBytes;
-                    const ConvOperand a = conv_operand<BM>(sa, a_mn), b = conv_operand<BN>(sa + 2 * Cfg::kA32, b_mn);
+                    const ConvOperand b = conv_operand<BN>(sa + Cfg::kA32, b_mn);
+                    const uint32_t a = tmem_base + 2 * BN + s * Cfg::kACols;
                     const uint32_t first = (i == c * kChunkKB) ? 0u : 1u;      // a chunk starts from zero
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; ++kk) {
-                        mma_f16(d_tmem, a.l + (uint64_t)(kk * a.adv16), b.h + (uint64_t)(kk * b.adv16), idesc16, first | (uint32_t)kk);
-                        mma_f16(d_tmem, a.h + (uint64_t)(kk * a.adv16), b.l + (uint64_t)(kk * b.adv16), idesc16, 1u);
+                        mma_f16_ta(d_tmem, a + 48 + kk * 8, b.h + (uint64_t)(kk * b.adv16), idesc16, first | (uint32_t)kk);
+                        mma_f16_ta(d_tmem, a + 32 + kk * 8, b.l + (uint64_t)(kk * b.adv16), idesc16, 1u);
                     }
 #pragma unroll
                     for (int kk = 0; kk < BK / UK; ++kk)
-                        mma_tf32(d_tmem, a.f + (uint64_t)(kk * a.adv32), b.f + (uint64_t)(kk * b.adv32), idesc32, 1u);
+                        mma_tf32_ta(d_tmem, a + kk * 8, b.f + (uint64_t)(kk * b.adv32), idesc32, 1u);
                     mma_commit(empty_bar(s));
                 }
                 if (ok) mma_commit(acc_full_bar(buf));
             }
         }
     } else if (warp >= 10) {
-        // ---- converters.  With a group per stage one's waits (for the loads, shared memory and the proxy fence) pass under
-        // the others' work: 128 x 64 tiles 0.71 -> 0.6 us per k-block, the 200-256-256-10 step 97 -> 89 us; with 128 x 128 tiles
-        // three groups of three warps lost 9 % against all eight warps together.  Either every group takes every k-block or
-        // every stage belongs to one group: a stage is then refilled only after its group has converted it, so that no wait,
-        // which names a phase by its parity alone, can meet the phase before or after the one it means. ----
-        static_assert(Cfg::kGroups == 1 || Cfg::kGroups == S, "see above");
+        // ---- converters.  With two groups that take the k-blocks in turn one's waits (for the loads, shared memory and the
+        // proxy fence) pass under the other's work: best for 128 x 64 tiles; with 128 x 128 tiles all eight warps together are
+        // 4 % faster.  A group has the four warps that reach all 128 lanes of tensor memory, or eight.  Every stage belongs to
+        // one group: it is refilled only after its group has converted it, so that no wait, which names a phase by its parity
+        // alone, can meet the phase before or after the one it means. ----
+        static_assert(S % Cfg::kGroups == 0 && Cfg::kGroup % 128 == 0, "see above");
         const uint32_t ct = (threadIdx.x - 320) % Cfg::kGroup;
         for (uint32_t i = (threadIdx.x - 320) / Cfg::kGroup; i < nkb; i += Cfg::kGroups) {
             const int s = i % S;
@@ -1477,8 +1511,13 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
                 break;
             }
-            convert_tile<BM, Cfg::kGroup>(sa, a_mn, ct);
-            convert_tile<BN, Cfg::kGroup>(sa + 2 * Cfg::kA32, b_mn, ct);
+            tc_fence_after();           // the stage's tensor memory has been read: its load was waited for after those MMAs
+            const uint32_t ta = tmem_base + ((uint32_t)(warp & 3) << 21) + 2 * BN + s * Cfg::kACols;
+            if constexpr (Cfg::kGroup == 256) convert_a_row(sa, a_mn, warp & 3, lane, ct >> 7, ta);
+            else { convert_a_row(sa, a_mn, warp & 3, lane, 0, ta); convert_a_row(sa, a_mn, warp & 3, lane, 1, ta); }
+            convert_tile<BN, Cfg::kGroup>(sa + Cfg::kA32, b_mn, ct);
+            tmem_st_wait();
+            tc_fence_before();
             fence_proxy_async();        // the planes are read by the tensor core
             __syncwarp();
             if (lane == 0) mbar_arrive(conv_bar(s));
