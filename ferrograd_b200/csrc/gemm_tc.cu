@@ -455,8 +455,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     auto acc_empty_bar = [&](int b) { return bar0 + 8u * (2 * S + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * S + 4);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank();
+    // (known to be the same in all lanes, as the roles' branches and loops then are: the addresses and descriptors of the loading and
+    // the MMA warp live in uniform registers.  From one lane of a divergent branch, issuing the eight MMAs of a k-block took 770 cycles.)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank(), 0);
     const bool leader = rank == 0;
     const uint32_t pairs_m = (ep.M + 2 * BM - 1) / (2 * BM), pairs_n = (ep.N + BN - 1) / BN;
     const uint32_t ntiles = pairs_m * pairs_n;
@@ -497,12 +499,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     __syncthreads();
     cluster_sync_all();      // the peer's barriers exist before anything is signalled across CTAs
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp < kPairEpiWarp0) {
     reg_release<kPairRegsLow>();
     if (warp == 0) {
-        if (lane == 0) {
+        {
             // ---- producer (both CTAs): own rows of A, own half of B; completion counted on the leader ----
             uint32_t g = 0;      // k-blocks issued so far, across tiles: ring position and phase
             bool ok = true;
@@ -519,14 +521,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const uint32_t ph = (g / S) & 1u;
                     {
                         PROF_T0();
-                        const bool got = mbar_wait_bounded(empty_bar(s), ph ^ 1u, kPairWaitCycles);
+                        const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(empty_bar(s), ph ^ 1u, kPairWaitCycles));
                         PROF_ADD(prof_a);
                         if (!got) {
-                            atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
+                            if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
                             ok = false;
                             break;
                         }
                     }
+                    if (!elect_one()) continue;
                     const uint32_t lf = map_to_cta(full_bar(s), 0);
                     const uint32_t sa = base + s * Cfg::kStageBytes;
                     if (kDirect16) {
@@ -573,11 +576,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 }
             }
 #ifdef FG_GEMM_PROFILE
-            atomicAdd(&g_prof[6], (unsigned long long)prof_a);
+            if (lane == 0) atomicAdd(&g_prof[6], (unsigned long long)prof_a);
 #endif
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader) {
             // ---- MMA issuer (leader CTA only): M = 256 across the pair, N = 256 ----
             constexpr uint32_t idesc = make_idesc(2u /*tf32*/, 2 * BM, BN);
             bool ok = true;
@@ -595,10 +598,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     // the accumulator must have been drained by both CTAs' epilogue warps (two chunks ago)
                     {
                         PROF_T0();
-                        const bool got = mbar_wait_bounded(acc_empty_bar(buf), ((gc >> 1) & 1u) ^ 1u, kPairWaitCycles);
+                        const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(acc_empty_bar(buf), ((gc >> 1) & 1u) ^ 1u, kPairWaitCycles));
                         PROF_ADD(prof_e);
                         if (!got) {
-                            atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+                            if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
                             ok = false;
                             break;
                         }
@@ -611,10 +614,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         const uint32_t ph = (g / S) & 1u;
                         {
                             PROF_T0();
-                            const bool got = mbar_wait_bounded(full_bar(s), ph, kPairWaitCycles);
+                            const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(full_bar(s), ph, kPairWaitCycles));
                             PROF_ADD(prof_f);
                             if (!got) {
-                                atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+                                if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
                                 ok = false;
                                 break;
                             }
@@ -632,19 +635,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                             const uint64_t a_d = ep.a_mn ? make_desc_mnmajor(sa, 8192, 1024, 2) : a_hi;
                             const uint64_t b_d = ep.b_mn ? make_desc_mnmajor(sa + Cfg::kABytes, 8192, 1024, 2) : b_hi;
                             const uint32_t a_adv = ep.a_mn ? 128u : 2u, b_adv = ep.b_mn ? 128u : 2u;
+                            if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < (int)KBE / 16; ++kk)
-                                mma_f16_pair(d_tmem, a_d + (uint64_t)(kk * a_adv), b_d + (uint64_t)(kk * b_adv), idesc16,
-                                             first | (uint32_t)kk);
+                                for (int kk = 0; kk < (int)KBE / 16; ++kk)
+                                    mma_f16_pair(d_tmem, a_d + (uint64_t)(kk * a_adv), b_d + (uint64_t)(kk * b_adv), idesc16,
+                                                 first | (uint32_t)kk);
+                            }
                         } else if (FMT == 0) {
                             const uint64_t a_lo = make_desc_kmajor<BK * 4>(sa + BM * BK * 4);
                             const uint64_t b_lo = make_desc_kmajor<BK * 4>(sa + Cfg::kABytes + HB * BK * 4);
+                            if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < BK / UK; ++kk) {
-                                const uint64_t adv = (uint64_t)(kk * UK * 4 >> 4);
-                                mma_tf32_pair(d_tmem, a_lo + adv, b_hi + adv, idesc, first | (uint32_t)kk);
-                                mma_tf32_pair(d_tmem, a_hi + adv, b_lo + adv, idesc, 1u);
-                                mma_tf32_pair(d_tmem, a_hi + adv, b_hi + adv, idesc, 1u);
+                                for (int kk = 0; kk < BK / UK; ++kk) {
+                                    const uint64_t adv = (uint64_t)(kk * UK * 4 >> 4);
+                                    mma_tf32_pair(d_tmem, a_lo + adv, b_hi + adv, idesc, first | (uint32_t)kk);
+                                    mma_tf32_pair(d_tmem, a_hi + adv, b_lo + adv, idesc, 1u);
+                                    mma_tf32_pair(d_tmem, a_hi + adv, b_hi + adv, idesc, 1u);
+                                }
                             }
                         } else {
                             // Per operand: descriptors of the f32 tile and of its two bf16 planes, and how far
@@ -677,26 +684,33 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                 b_h16 = make_desc_mnmajor(b16, 8192, 1024, 2); b_l16 = make_desc_mnmajor(b16 + 4096, 8192, 1024, 2);
                                 b_adv32 = 64; b_adv16 = 128;
                             }
+                            if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < BK / 16; ++kk) {
-                                mma_f16_pair(d_tmem, a_l16 + (uint64_t)(kk * a_adv16), b_h16 + (uint64_t)(kk * b_adv16), idesc16,
-                                             first | (uint32_t)kk);
-                                mma_f16_pair(d_tmem, a_h16 + (uint64_t)(kk * a_adv16), b_l16 + (uint64_t)(kk * b_adv16), idesc16, 1u);
+                                for (int kk = 0; kk < BK / 16; ++kk) {
+                                    mma_f16_pair(d_tmem, a_l16 + (uint64_t)(kk * a_adv16), b_h16 + (uint64_t)(kk * b_adv16), idesc16,
+                                                 first | (uint32_t)kk);
+                                    mma_f16_pair(d_tmem, a_h16 + (uint64_t)(kk * a_adv16), b_l16 + (uint64_t)(kk * b_adv16), idesc16, 1u);
+                                }
+#pragma unroll
+                                for (int kk = 0; kk < BK / UK; ++kk)
+                                    mma_tf32_pair(d_tmem, a_f + (uint64_t)(kk * a_adv32), b_f + (uint64_t)(kk * b_adv32), idesc_t, 1u);
                             }
-#pragma unroll
-                            for (int kk = 0; kk < BK / UK; ++kk)
-                                mma_tf32_pair(d_tmem, a_f + (uint64_t)(kk * a_adv32), b_f + (uint64_t)(kk * b_adv32), idesc_t, 1u);
                         }
-                        mma_commit_pair(empty_bar(s), 3);        // frees this stage in both CTAs
+                        __syncwarp();
+                        if (elect_one()) mma_commit_pair(empty_bar(s), 3);        // frees this stage in both CTAs
+                        __syncwarp();
                     }
-                    if (ok) mma_commit_pair(acc_full_bar(buf), 3);   // both CTAs may drain their half
+                    if (ok && elect_one()) mma_commit_pair(acc_full_bar(buf), 3);   // both CTAs may drain their half
+                    __syncwarp();
                 }
             }
 #ifdef FG_GEMM_PROFILE
+            if (lane == 0) {
             atomicAdd(&g_prof[0], (unsigned long long)prof_e);
             atomicAdd(&g_prof[1], (unsigned long long)prof_f);
             atomicAdd(&g_prof[2], (unsigned long long)(clock64() - prof_start));
             atomicAdd(&g_prof[7], 1ull);
+            }
 #endif
         }
     }
