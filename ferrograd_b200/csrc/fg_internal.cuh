@@ -127,25 +127,37 @@ struct FgRange {
          if (_e != cudaSuccess) return fg_fail_cuda((ctx), FG_ERR_LAUNCH_FAILURE, "kernel launch", _e); \
          if ((ctx)->capturing) (ctx)->capture_launches++; else (ctx)->launches++; } while (0)
 
-// Back-to-back launches of short kernels.  A kernel launched with fg_launch is set up while the kernel before it on the
-// stream drains (programmatic stream serialization); fg_grid_enter(), its first statement in every thread, waits until
+// Back-to-back launches of short kernels.  A kernel launched with fg_launch (or, in clusters, fg_launch_cluster) is set up while the
+// kernel before it on the stream drains (programmatic stream serialization); fg_grid_enter(), which comes in every thread before
+// anything that reads or writes memory of the device, waits until
 // everything before it has finished and is visible.  Nothing is triggered early: blocks of the next kernel that wait on the
 // SMs from the start of this one's work on slow it several times over, once the host is ahead (18 x (88 x 24 x 256) backward,
 // two launches: 14.4 us in plain order, 10.8 like this, 30 to 37 with a trigger on entry).  Seven launches of a ragged layer's
 // backward pass 71.6 -> 53.6 us, the 16 of a 2-16-2 training step 36.2 -> 30.1 us.
 template <typename... P, typename... A>
-inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+inline void fg_launch_cluster(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = ctx->comm ? 0 : 1;      // with a communicator the stream also forks and joins: plain order there
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (!ctx->comm) {      // with a communicator the stream also forks and joins: plain order there
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // FG_LAUNCHED reports its error
+}
+template <typename... P, typename... A>
+inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    fg_launch_cluster(ctx, kernel, grid, block, smem, 1, std::forward<A>(args)...);
 }
 __device__ __forceinline__ void fg_grid_enter() { cudaGridDependencySynchronize(); }
 

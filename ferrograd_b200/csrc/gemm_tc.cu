@@ -58,8 +58,7 @@ struct Epilogue {
     int mul_act;
     float* colsum_part;               // optional [ceil(M/32)][N]: column sums of the stored C per 32-row block
     uint32_t group;                   // tile rows per group of the tile order (see pair_tile_origin)
-    uint32_t batch;                   // conversion kernel: matrices in this launch (0 or 1: one) ...
-    uint64_t c_batch;                 // ... and the elements between two of them in C and preact
+    uint64_t c_batch;                 // conversion kernel: elements between two matrices of a batch in C and preact
 #ifdef FG_GEMM_PROFILE
     uint32_t dbg;                     // diagnostic build: bit 0 = leave out the global stores of the epilogue
 #endif
@@ -917,9 +916,8 @@ __global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
     constexpr uint32_t kSubN = TN / 32, kSubs = (TM / 32) * kSubN;
     const uint32_t pairs_m = (ep.M + TM - 1) / TM, pairs_n = (ep.N + TN - 1) / TN;
     const uint32_t tail = blockIdx.x / kSubs, sub = blockIdx.x % kSubs;
-    uint32_t m0, n0, tile = ep.t_full + tail, bz = 0;
-    if (ep.batch > 1) { bz = tile / (pairs_m * pairs_n); tile -= bz * (pairs_m * pairs_n); }
-    pair_tile_origin(tile, pairs_m, pairs_n, TM, TN, ep.group, m0, n0);
+    uint32_t m0, n0;
+    pair_tile_origin(ep.t_full + tail, pairs_m, pairs_n, TM, TN, ep.group, m0, n0);
     const uint32_t lrow = (sub / kSubN) * 32 + (threadIdx.x >> 3), lcol = (sub % kSubN) * 32 + (threadIdx.x & 7u) * 4;
     const uint32_t row = m0 + lrow, col = n0 + lcol;
     const bool live = row < ep.M && col < ep.N;
@@ -936,8 +934,8 @@ __global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
 #pragma unroll
             for (int t = 0; t < 4; ++t) if (col + t < ep.N) zz[t] += ep.bias[col + t];
         }
-        const size_t off = bz * ep.c_batch + (size_t)row * ep.N + col;
-        const bool vec_ok = (ep.N % 4 == 0) && (ep.c_batch % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
+        const size_t off = (size_t)row * ep.N + col;
+        const bool vec_ok = (ep.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
                             (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0) &&
                             (!ep.mul_saved || (reinterpret_cast<uintptr_t>(ep.mul_saved) & 15u) == 0);
         if (vec_ok && col + 3 < ep.N) {
@@ -1269,14 +1267,14 @@ int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 
 // as much as reading it twice more.  Here a CTA owns a 128 x BN tile, loads the raw f32 words of
 // both operands (half the bytes of tensor plus pairs) and converter warps split each k-block: A into
 // tensor memory, from where the MMAs read it, B's bf16 planes beside its words in shared memory, in the
-// layout a bulk-tensor load would have given them.  A matrix index and a K-share ride in the grid, so that
-// one launch covers a batch and fills the SMs; K-shares are folded by gemm_tc_fold_kernel.
-//   warp 0 loads, warp 1 issues MMAs, warps 2..9 drain accumulators and store, the others convert.
-// Measured (before: operand planes or pairs, then a 256 x 256 or 128-row tile each): 100 x 4096 x 4096 129 -> 36 us,
-// 16 x (384 x 512 x 320) forward and backward 1530 -> 87 us, a 384-sample layer of 256 x 256 21.7 -> 9.8 us per product.
-// Bound by shared-memory bandwidth and the converters: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB
-// into the converters, 32 KB out of them (B) and 32 KB into the MMAs (B), 128 KB at 128 B per cycle; with A in shared
-// memory too it was 192 KB (100 x 4096 x 4096 34.9 -> 29.8 us, 16 x (384 x 512 x 320) forward and backward 86.3 -> 75.5 us).
+// layout a bulk-tensor load would have given them.  A matrix index rides in the unit number and a K-share in
+// the cluster, so that one launch covers a batch, or both gradients of a layer, and fills the SMs.
+//   warp 0 loads, warp 1 issues MMAs, warps 4..11 drain accumulators and store, warps 12..27 convert.
+// Measured (start: operand planes or pairs, then a 256 x 256 or 128-row tile each; then with A in shared memory, eight converter
+// warps, K-shares folded by a second launch and one launch per product; now): 100 x 4096 x 4096 129 -> 35 -> 30 us,
+// 16 x (384 x 512 x 320) forward and backward 1530 -> 86 -> 51 us, the 200-256-256-10 step 195 -> 91 -> 74 us.
+// Bound by shared-memory bandwidth: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB into the converters, 32 KB
+// out of them (B) and 32 KB into the MMAs (B): 1024 cycles at 128 B per cycle, 1040 measured (128 x 64: 640, 590 - 630 measured).
 // ------------------------------------------------------------------------------------
 template <int BN>
 struct ConvCfg {
@@ -1285,11 +1283,16 @@ struct ConvCfg {
     static constexpr int kStages = BN == 128 ? 4 : 6;
     static constexpr int kACols = 64;                               // tensor memory per stage: A as f32 and as two bf16 planes
     // Converters: groups of warps that take the k-blocks in turn, see the kernel.
-    static constexpr int kGroups = BN == 128 ? 1 : 2, kGroup = 256 / kGroups;
-    static constexpr int kThreads = 320 + 256;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+    static constexpr int kGroups = 2, kGroup = 256;
+    static constexpr int kEpi0 = 4, kConv0 = 12;                    // first epilogue and first converter warp
+    static constexpr int kThreads = kConv0 * 32 + kGroups * kGroup;
+    // registers after the split between the warpgroups (72 each at launch): loads and MMAs, epilogue, converters
+    static constexpr int kRegsLow = 40, kRegsEpi = 104, kRegsConv = 64;
+    static_assert(kThreads == 896 && 128 * kRegsLow + 256 * kRegsEpi + 512 * kRegsConv <= 896 * 72, "the launch's registers");
+    static constexpr int kStoreBytes = 8 * 32 * 32 * 4;             // the epilogue warps' staging blocks
+    static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256;
     static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
-    static_assert(kStageBytes >= 8 * 32 * 32 * 4, "the epilogue stages its blocks in the first stage");
+    static_assert(kStages * kStageBytes >= BM * BN * 4, "a K-share's sums lie in the stages");
     static constexpr int kTmemCols = 512;
     static_assert(2 * BN + kStages * kACols <= kTmemCols, "two accumulators and the stages of A");
 };
@@ -1396,258 +1399,417 @@ __device__ __forceinline__ ConvOperand conv_operand(uint32_t t32, bool mn) {
     return o;
 }
 
-template <int BN>
+// One or two products in a launch (the two gradients of a layer): problem 0's units come first, then problem 1's.
+struct ConvArgs {
+    Epilogue ep[2];
+    uint32_t units0, units;       // units (tile x matrix) of problem 0, and of both
+    uint32_t split;               // K-shares of a unit = CTAs of a cluster
+    int* dev_status;
+};
+
+// Stores groups of four columns from `col` on: bias, activation or act' factor, the optional outputs.  A CTA stores one tile, or
+// a few, with one or two warps per scheduler: their instructions come one after the other, so whatever does not change from row
+// to row is settled before (asked again for every row, storing a 128 x 128 tile took 8000 - 11000 cycles).
+struct ConvStore {
+    uint32_t col;
+    bool live, vec, plain;
+    int kind, act;       // 0: as it is, 1: act, 2: * act'(mul_saved)
+    __device__ __forceinline__ ConvStore(const Epilogue& ep, uint32_t c) : col(c), live(c < ep.N) {
+        // (with vec, N is a multiple of four: a live group is whole)
+        vec = (ep.N % 4 == 0) && (ep.c_batch % 4 == 0) &&
+              (((reinterpret_cast<uintptr_t>(ep.C) | reinterpret_cast<uintptr_t>(ep.preact) | reinterpret_cast<uintptr_t>(ep.mul_saved)) & 15u) == 0);
+        kind = ep.mul_saved ? 2 : ep.act != FG_ACT_NONE ? 1 : 0;
+        act = kind == 2 ? ep.mul_act : ep.act;
+        plain = vec && kind == 0 && !ep.preact && !ep.c_pairs;
+    }
+    // The group at element offset `off`, its bias added.  Returns what was stored in C.
+    __device__ __forceinline__ float4 put_plain(const Epilogue& ep, size_t off, float4 z) const {
+        *reinterpret_cast<float4*>(ep.C + off) = z;
+        return z;
+    }
+    __device__ __forceinline__ float4 put(const Epilogue& ep, size_t off, float4 z) const {
+        if (!vec)
+            return epi_store_edge(z, off, col, ep.N, (char*)ep.C, (char*)ep.preact, ep.c_pairs, ep.c_pairs_stride, ep.mul_saved, ep.mul_act,
+                                  ep.act, FG_DTYPE_F32);
+        float4 o = z;
+        if (kind == 1) {
+            o = make_float4(fg_act_fwd_sel(act, z.x), fg_act_fwd_sel(act, z.y), fg_act_fwd_sel(act, z.z), fg_act_fwd_sel(act, z.w));
+        } else if (kind == 2) {
+            const float4 sv = __ldg(reinterpret_cast<const float4*>(ep.mul_saved + off));
+            o = make_float4(z.x * fg_act_grad_sel(act, sv.x), z.y * fg_act_grad_sel(act, sv.y), z.z * fg_act_grad_sel(act, sv.z),
+                            z.w * fg_act_grad_sel(act, sv.w));
+        }
+        if (ep.preact) *reinterpret_cast<float4*>(ep.preact + off) = z;
+        *reinterpret_cast<float4*>(ep.C + off) = o;
+        if (ep.c_pairs) fg_store_pairs4(ep.c_pairs, ep.c_pairs_stride, off, o);
+        return o;
+    }
+};
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+// Sums over the lanes that hold the same four columns (lanes c, c + 8, c + 16, c + 24).
+__device__ __forceinline__ float4 sum_column_lanes(float4 v) {
+#pragma unroll
+    for (int d = 8; d < 32; d *= 2) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, d); v.y += __shfl_xor_sync(0xffffffffu, v.y, d);
+        v.z += __shfl_xor_sync(0xffffffffu, v.z, d); v.w += __shfl_xor_sync(0xffffffffu, v.w, d);
+    }
+    return v;
+}
+__device__ __forceinline__ void store_colsum(const Epilogue& ep, uint32_t row0, uint32_t col, float4 cs) {
+    float* d = ep.colsum_part + (size_t)(row0 >> 5) * ep.N + col;
+    if (col < ep.N) d[0] = cs.x;
+    if (col + 1 < ep.N) d[1] = cs.y;
+    if (col + 2 < ep.N) d[2] = cs.z;
+    if (col + 3 < ep.N) d[3] = cs.w;
+}
+
+// Units are walked persistently (unit, unit + CTAs, ...): the ring of loads, the conversion and the MMAs run across units, so
+// that a tile is stored while the next one is computed.  With K-shares a cluster of `split` CTAs takes one unit, a share each,
+// and the shares' sums meet through distributed shared memory: every CTA stores every split-th 32 x 32 block of the tile.
+template <int BN, bool TWO, bool SHARES>
 __global__ void __launch_bounds__(ConvCfg<BN>::kThreads, 1)
-gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epilogue ep) {
-    fg_grid_enter();
+gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
+                    const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmB1,
+                    const __grid_constant__ ConvArgs ca) {
     using Cfg = ConvCfg<BN>;
     constexpr int S = Cfg::kStages, BK = 32, CPT = BN / 2;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* const base_ptr = smem_raw + (base - raw);
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base_ptr + S * Cfg::kStageBytes);
-    const uint32_t bar0 = base + S * Cfg::kStageBytes;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base_ptr + S * Cfg::kStageBytes + Cfg::kStoreBytes);
+    const uint32_t bar0 = base + S * Cfg::kStageBytes + Cfg::kStoreBytes;
     auto full_bar = [&](int s) { return bar0 + 8u * s; };            // the f32 words have landed
-    auto conv_bar = [&](int s) { return bar0 + 8u * (S + s); };      // the bf16 planes are written
+    auto conv_bar = [&](int s) { return bar0 + 8u * (S + s); };      // both operands are converted
     auto empty_bar = [&](int s) { return bar0 + 8u * (2 * S + s); };
     auto acc_full_bar = [&](int b) { return bar0 + 8u * (3 * S + b); };
     auto acc_empty_bar = [&](int b) { return bar0 + 8u * (3 * S + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 3 * S + 4);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t tiles_m = (ep.M + BM - 1) / BM, tiles_n = (ep.N + BN - 1) / BN, bz = blockIdx.z;
-    uint32_t m0, n0;
-    pair_tile_origin(blockIdx.x, tiles_m, tiles_n, BM, BN, ep.group, m0, n0);
-    const uint32_t nkb_all = (ep.K + BK - 1) / BK;
-    const uint32_t kb0 = (uint32_t)((uint64_t)blockIdx.y * nkb_all / ep.split);
-    const uint32_t nkb = (uint32_t)((uint64_t)(blockIdx.y + 1) * nkb_all / ep.split) - kb0;     // the host keeps split <= nkb_all
+    // (the warp index is known to be the same in all lanes, as in the pair kernel)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t split = SHARES ? ca.split : 1u, share = SHARES ? cluster_ctarank() : 0u;
+    const uint32_t first = SHARES ? blockIdx.x / split : blockIdx.x, step = SHARES ? ca.units : gridDim.x;
+    struct Unit { uint32_t p, m0, n0, bz, kb0, nkb; };
+    // (each problem's fields are read at addresses known to the compiler: through a pointer they are loads from memory)
+    auto ep_of = [&](uint32_t p, auto field) { return !TWO || p == 0 ? field(ca.ep[0]) : field(ca.ep[1]); };
+    auto unit_at = [&](uint32_t u) -> Unit {
+        Unit t;
+        t.p = TWO && u >= ca.units0 ? 1u : 0u;
+        const uint32_t v = u - (t.p ? ca.units0 : 0u), K = ep_of(t.p, [](const Epilogue& e) { return e.K; });
+        const uint32_t tiles_m = ep_of(t.p, [](const Epilogue& e) { return (e.M + BM - 1) / BM; });
+        const uint32_t tiles = ep_of(t.p, [](const Epilogue& e) { return ((e.M + BM - 1) / BM) * ((e.N + BN - 1) / BN); }), tile = v % tiles;
+        t.bz = v / tiles;
+        t.m0 = tile % tiles_m * BM;      // down the columns of tiles: the CTAs at work share a few tile columns of B
+        t.n0 = tile / tiles_m * BN;
+        const uint32_t all = (K + BK - 1) / BK;      // the host keeps split <= all
+        t.kb0 = (uint32_t)((uint64_t)share * all / split);
+        t.nkb = (uint32_t)((uint64_t)(share + 1) * all / split) - t.kb0;
+        return t;
+    };
+    auto is_mn = [&](uint32_t p, bool& a, bool& b) {
+        a = ep_of(p, [](const Epilogue& e) { return e.a_mn != 0; });
+        b = ep_of(p, [](const Epilogue& e) { return e.b_mn != 0; });
+    };
     constexpr uint32_t kChunkKB = kChunkK / BK;
-    const uint32_t nchunks = (nkb + kChunkKB - 1) / kChunkKB;
-
-    __shared__ int s_abort;      // see gemm_tc_kernel
-    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(ep.dev_status);
-    __syncthreads();
-    if (s_abort != 0) return;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(conv_bar(s), Cfg::kGroup / 32); mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full_bar(b), 1); mbar_init(acc_empty_bar(b), 8); }
         fence_mbar_init();
-        prefetch_tmap(&tmA);
-        prefetch_tmap(&tmB);
+        prefetch_tmap(&tmA0);
+        prefetch_tmap(&tmB0);
+        if (TWO) { prefetch_tmap(&tmA1); prefetch_tmap(&tmB1); }
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), Cfg::kTmemCols);
         tmem_relinquish();
     }
+    // Everything up to here needs nothing of the kernels before this one: it passes while the last of them drains.
+    fg_grid_enter();
+    __shared__ int s_abort;      // see gemm_tc_kernel; the CTAs of a cluster stay together to the end, whatever they have read
+    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(ca.dev_status);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    const bool a_mn = ep.a_mn != 0, b_mn = ep.b_mn != 0;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const bool go = __all_sync(0xffffffffu, s_abort == 0);
 
-    if (warp == 0) {
-        if (lane == 0) {
+    if (warp < Cfg::kEpi0) {
+        reg_release<Cfg::kRegsLow>();
+        if (go && warp == 0) {
             // ---- producer ----
-            for (uint32_t i = 0; i < nkb; ++i) {
-                const int s = i % S;
-                if (!mbar_wait_bounded(empty_bar(s), ((i / S) & 1u) ^ 1u, kWaitCycles)) {
-                    atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
-                    break;
-                }
-                mbar_expect_tx(full_bar(s), Cfg::kA32 + Cfg::kB32);
-                const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + Cfg::kA32;
-                const int k = (int)((kb0 + i) * BK);
-                if (!a_mn) tma_load_3d(sa, &tmA, full_bar(s), k, (int)m0, (int)bz);
-                else
-#pragma unroll
-                    for (int j = 0; j < BM / 32; ++j) tma_load_3d(sa + j * 4096, &tmA, full_bar(s), (int)(m0 + 32 * j), k, (int)bz);
-                if (!b_mn) tma_load_3d(sb, &tmB, full_bar(s), k, (int)n0, (int)bz);
-                else
-#pragma unroll
-                    for (int j = 0; j < BN / 32; ++j) tma_load_3d(sb + j * 4096, &tmB, full_bar(s), (int)(n0 + 32 * j), k, (int)bz);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer ----
-            const uint32_t mnbits = b_mn ? kIdescBMnMajor : 0u;
-            const uint32_t idesc32 = make_idesc(2u /*tf32*/, BM, BN) | mnbits, idesc16 = make_idesc(1u /*bf16*/, BM, BN) | mnbits;
+            uint32_t g = 0;      // k-blocks so far, across units: ring position and phase
             bool ok = true;
-            for (uint32_t c = 0; c < nchunks && ok; ++c) {
-                const uint32_t buf = c & 1u;
-                if (!mbar_wait_bounded(acc_empty_bar(buf), ((c >> 1) & 1u) ^ 1u, kWaitCycles)) {
-                    atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
-                    break;
+            for (uint32_t u = first; u < ca.units && ok; u += step) {
+                const Unit t = unit_at(u);
+                const CUtensorMap* const ta = TWO && t.p ? &tmA1 : &tmA0;
+                const CUtensorMap* const tb = TWO && t.p ? &tmB1 : &tmB0;
+                bool a_mn, b_mn;
+                is_mn(t.p, a_mn, b_mn);
+                for (uint32_t i = 0; i < t.nkb; ++i, ++g) {
+                    const int s = g % S;
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty_bar(s), ((g / S) & 1u) ^ 1u, kWaitCycles))) {
+                        if (lane == 0) atomicOr(ca.dev_status, FG_DEVERR_TMA_WAIT);
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + Cfg::kA32;
+                    const int k = (int)((t.kb0 + i) * BK);
+                    if (!elect_one()) continue;
+                    mbar_expect_tx(full_bar(s), Cfg::kA32 + Cfg::kB32);
+                    if (!a_mn) tma_load_3d(sa, ta, full_bar(s), k, (int)t.m0, (int)t.bz);
+                    else
+#pragma unroll
+                        for (int j = 0; j < BM / 32; ++j) tma_load_3d(sa + j * 4096, ta, full_bar(s), (int)(t.m0 + 32 * j), k, (int)t.bz);
+                    if (!b_mn) tma_load_3d(sb, tb, full_bar(s), k, (int)t.n0, (int)t.bz);
+                    else
+#pragma unroll
+                        for (int j = 0; j < BN / 32; ++j) tma_load_3d(sb + j * 4096, tb, full_bar(s), (int)(t.n0 + 32 * j), k, (int)t.bz);
                 }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                const uint32_t end = min(nkb, (c + 1) * kChunkKB);
-                for (uint32_t i = c * kChunkKB; i < end; ++i) {
-                    const int s = i % S;
-                    if (!mbar_wait_bounded(conv_bar(s), (i / S) & 1u, kWaitCycles)) {
-                        atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+            }
+        } else if (go && warp == 1) {
+            // ---- MMA issuer ----
+            bool ok = true;
+            uint32_t g = 0, gc = 0;      // k-blocks and chunks so far, across units
+            for (uint32_t u = first; u < ca.units && ok; u += step) {
+                const Unit t = unit_at(u);
+                bool a_mn, b_mn;
+                is_mn(t.p, a_mn, b_mn);
+                const uint32_t mnbits = b_mn ? kIdescBMnMajor : 0u;
+                const uint32_t idesc32 = make_idesc(2u /*tf32*/, BM, BN) | mnbits, idesc16 = make_idesc(1u /*bf16*/, BM, BN) | mnbits;
+                const uint32_t nchunks = (t.nkb + kChunkKB - 1) / kChunkKB;
+                for (uint32_t c = 0; c < nchunks && ok; ++c, ++gc) {
+                    const uint32_t buf = gc & 1u;
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(acc_empty_bar(buf), ((gc >> 1) & 1u) ^ 1u, kWaitCycles))) {
+                        if (lane == 0) atomicOr(ca.dev_status, FG_DEVERR_MMA_WAIT);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = base + s * Cfg::kStageBytes;
-                    const ConvOperand b = conv_operand<BN>(sa + Cfg::kA32, b_mn);
-                    const uint32_t a = tmem_base + 2 * BN + s * Cfg::kACols;
-                    const uint32_t first = (i == c * kChunkKB) ? 0u : 1u;      // a chunk starts from zero
+                    const uint32_t d_tmem = tmem_base + buf * BN;
+                    const uint32_t end = min(t.nkb, (c + 1) * kChunkKB);
+                    for (uint32_t i = c * kChunkKB; i < end; ++i, ++g) {
+                        const int s = g % S;
+                        if (!__all_sync(0xffffffffu, mbar_wait_bounded(conv_bar(s), (g / S) & 1u, kWaitCycles))) {
+                            if (lane == 0) atomicOr(ca.dev_status, FG_DEVERR_MMA_WAIT);
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t sa = base + s * Cfg::kStageBytes;
+                        const ConvOperand b = conv_operand<BN>(sa + Cfg::kA32, b_mn);
+                        const uint32_t a = tmem_base + 2 * BN + s * Cfg::kACols;
+                        const uint32_t acc = (i == c * kChunkKB) ? 0u : 1u;      // a chunk starts from zero
+                        if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < BK / 16; ++kk) {
-                        mma_f16_ta(d_tmem, a + 48 + kk * 8, b.h + (uint64_t)(kk * b.adv16), idesc16, first | (uint32_t)kk);
-                        mma_f16_ta(d_tmem, a + 32 + kk * 8, b.l + (uint64_t)(kk * b.adv16), idesc16, 1u);
+                            for (int kk = 0; kk < BK / 16; ++kk) {
+                                mma_f16_ta(d_tmem, a + 48 + kk * 8, b.h + (uint64_t)(kk * b.adv16), idesc16, acc | (uint32_t)kk);
+                                mma_f16_ta(d_tmem, a + 32 + kk * 8, b.l + (uint64_t)(kk * b.adv16), idesc16, 1u);
+                            }
+#pragma unroll
+                            for (int kk = 0; kk < BK / UK; ++kk)
+                                mma_tf32_ta(d_tmem, a + kk * 8, b.f + (uint64_t)(kk * b.adv32), idesc32, 1u);
+                            mma_commit(empty_bar(s));
+                        }
+                        __syncwarp();
                     }
-#pragma unroll
-                    for (int kk = 0; kk < BK / UK; ++kk)
-                        mma_tf32_ta(d_tmem, a + kk * 8, b.f + (uint64_t)(kk * b.adv32), idesc32, 1u);
-                    mma_commit(empty_bar(s));
+                    if (ok && elect_one()) mma_commit(acc_full_bar(buf));
+                    __syncwarp();
                 }
-                if (ok) mma_commit(acc_full_bar(buf));
             }
         }
-    } else if (warp >= 10) {
-        // ---- converters.  With two groups that take the k-blocks in turn one's waits (for the loads, shared memory and the
-        // proxy fence) pass under the other's work: best for 128 x 64 tiles; with 128 x 128 tiles all eight warps together are
-        // 4 % faster.  A group has the four warps that reach all 128 lanes of tensor memory, or eight.  Every stage belongs to
-        // one group: it is refilled only after its group has converted it, so that no wait, which names a phase by its parity
-        // alone, can meet the phase before or after the one it means. ----
+        if constexpr (SHARES) { __syncwarp(); cluster_sync_all(); cluster_sync_all(); }      // as the converters
+    } else if (warp >= Cfg::kConv0) {
+        reg_release<Cfg::kRegsConv>();
+        // ---- converters: two groups of eight warps take the k-blocks in turn, so that one's waits (for the loads, shared memory
+        // and the proxy fence) pass under the other's work.  Every stage belongs to one group: it is refilled only after its
+        // group has converted it, so that no wait, which names a phase by its parity alone, can meet the phase before or after
+        // the one it means. ----
         static_assert(S % Cfg::kGroups == 0 && Cfg::kGroup % 128 == 0, "see above");
-        const uint32_t ct = (threadIdx.x - 320) % Cfg::kGroup;
-        for (uint32_t i = (threadIdx.x - 320) / Cfg::kGroup; i < nkb; i += Cfg::kGroups) {
-            const int s = i % S;
-            unsigned char* const sa = base_ptr + s * Cfg::kStageBytes;
-            const bool got = mbar_wait_bounded(full_bar(s), (i / S) & 1u, kWaitCycles);
-            if (!__all_sync(0xffffffffu, got)) {
-                if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
-                break;
+        const uint32_t ct = (threadIdx.x - Cfg::kConv0 * 32) % Cfg::kGroup, mine = (threadIdx.x - Cfg::kConv0 * 32) / Cfg::kGroup;
+        uint32_t g = 0;
+        bool ok = go;
+        for (uint32_t u = first; u < ca.units && ok; u += step) {
+            const Unit t = unit_at(u);
+            bool a_mn, b_mn;
+            is_mn(t.p, a_mn, b_mn);
+            for (uint32_t i = 0; i < t.nkb; ++i, ++g) {
+                if (g % Cfg::kGroups != mine) continue;
+                const int s = g % S;
+                unsigned char* const sa = base_ptr + s * Cfg::kStageBytes;
+                const bool got = mbar_wait_bounded(full_bar(s), (g / S) & 1u, kWaitCycles);
+                if (!__all_sync(0xffffffffu, got)) {
+                    if (lane == 0) atomicOr(ca.dev_status, FG_DEVERR_TMA_WAIT);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();           // the stage's tensor memory has been read: its load was waited for after those MMAs
+                const uint32_t ta = tmem_base + ((uint32_t)(warp & 3) << 21) + 2 * BN + s * Cfg::kACols;
+                convert_a_row(sa, a_mn, warp & 3, lane, ct >> 7, ta);
+                convert_tile<BN, Cfg::kGroup>(sa + Cfg::kA32, b_mn, ct);
+                tmem_st_wait();
+                tc_fence_before();
+                fence_proxy_async();        // the planes are read by the tensor core
+                __syncwarp();
+                if (lane == 0) mbar_arrive(conv_bar(s));
             }
-            tc_fence_after();           // the stage's tensor memory has been read: its load was waited for after those MMAs
-            const uint32_t ta = tmem_base + ((uint32_t)(warp & 3) << 21) + 2 * BN + s * Cfg::kACols;
-            if constexpr (Cfg::kGroup == 256) convert_a_row(sa, a_mn, warp & 3, lane, ct >> 7, ta);
-            else { convert_a_row(sa, a_mn, warp & 3, lane, 0, ta); convert_a_row(sa, a_mn, warp & 3, lane, 1, ta); }
-            convert_tile<BN, Cfg::kGroup>(sa + Cfg::kA32, b_mn, ct);
-            tmem_st_wait();
-            tc_fence_before();
-            fence_proxy_async();        // the planes are read by the tensor core
+        }
+        if constexpr (SHARES) {
             __syncwarp();
-            if (lane == 0) mbar_arrive(conv_bar(s));
+            cluster_sync_all();      // every share's sums are in its CTA's shared memory
+            if (go) {
+                // This CTA's 32 x 32 blocks are every split-th of the tile, from its share's number on; a warp takes four rows of
+                // one, a lane four columns of a row.
+                const Unit t = unit_at(first);
+                const uint32_t rsub = lane >> 3, cc = lane & 7;
+                auto fold = [&](const Epilogue& ep) {
+                    float4* const csum = reinterpret_cast<float4*>(base_ptr + S * Cfg::kStageBytes);      // [block][eight times four rows][8 lanes]
+                    for (uint32_t v = warp - Cfg::kConv0, b; (b = share + split * (v >> 3)) < 4 * (BN / 32); v += 16) {
+                        const uint32_t lr = (b & 3u) * 32 + (v & 7u) * 4 + rsub, c0 = (b >> 2) * 32, row = t.m0 + lr;
+                        const ConvStore st(ep, t.n0 + c0 + cc * 4);
+                        const uint32_t at = base + ((lr * (BN / 4) + (((c0 >> 2) + cc) ^ (lr & 7))) << 4);
+                        float4 z[8];
+#pragma unroll
+                        for (uint32_t r = 0; r < 8; ++r)
+                            if (r < split) z[r] = ld_cluster_f4(map_to_cta(at, r));
+                        float bz[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) bz[j] = ep.bias && st.col + j < ep.N ? ep.bias[st.col + j] : 0.0f;
+#pragma unroll
+                        for (uint32_t r = 1; r < 8; ++r)        // in the order of the shares, whoever adds them
+                            if (r < split) z[0] = add4(z[0], z[r]);
+                        float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (st.live && row < ep.M) {
+                            const size_t off = (size_t)t.bz * ep.c_batch + (size_t)row * ep.N + st.col;
+                            const float4 w = add4(z[0], make_float4(bz[0], bz[1], bz[2], bz[3]));
+                            cs = st.plain ? st.put_plain(ep, off, w) : st.put(ep, off, w);
+                        }
+                        __syncwarp();
+                        if (ep.colsum_part) {
+                            cs = sum_column_lanes(cs);
+                            if (lane < 8) csum[v * 8 + lane] = cs;
+                        }
+                    }
+                    if (ep.colsum_part) {
+                        asm volatile("bar.sync 1, 512;" ::: "memory");      // the converters
+                        const uint32_t k = threadIdx.x - Cfg::kConv0 * 32, blk = k >> 3, b = share + split * blk;      // eight lanes per block
+                        if (b < 4 * (BN / 32) && t.m0 + (b & 3u) * 32 < ep.M) {
+                            float4 w = csum[blk * 64 + cc];
+#pragma unroll
+                            for (uint32_t j = 1; j < 8; ++j) w = add4(w, csum[blk * 64 + j * 8 + cc]);
+                            store_colsum(ep, t.m0 + (b & 3u) * 32, t.n0 + (b >> 2) * 32 + cc * 4, w);
+                        }
+                    }
+                };
+                if (!TWO || t.p == 0) fold(ca.ep[0]);
+                else fold(ca.ep[1]);
+            }
+            __syncwarp();
+            cluster_sync_all();      // no CTA leaves while another reads its sums
         }
     } else {
-        // ---- accumulate + epilogue: warps 2..9; warp w may touch TMEM lanes 32*(w%4) .. +31 ----
-        const int q = warp & 3, half = (warp - 2) >> 2;
-        float sum[CPT];
+        reg_acquire<Cfg::kRegsEpi>();
+        // ---- accumulate + epilogue: warps 4..11; warp w may touch TMEM lanes 32*(w%4) .. +31 ----
+        const int q = warp & 3, half = (warp - Cfg::kEpi0) >> 2;
+        bool ok = go;
+        uint32_t gc = 0;
+        float4* const tb4 = reinterpret_cast<float4*>(base_ptr + S * Cfg::kStageBytes) + (warp - Cfg::kEpi0) * (32 * 8);
+        const uint32_t rsub = lane >> 3, cc = lane & 7;
+        // A 32 x 32 block of whole sums, swizzled in tb4 (float4 c of row r at c ^ (r & 7)): four rows of 128 bytes per step.
+        auto store_block = [&](const Epilogue& ep, size_t cb, uint32_t row0, uint32_t col0, float bias) {
+            const ConvStore st(ep, col0 + cc * 4);
+            const float4 bz = make_float4(__shfl_sync(0xffffffffu, bias, cc * 4), __shfl_sync(0xffffffffu, bias, cc * 4 + 1),
+                                          __shfl_sync(0xffffffffu, bias, cc * 4 + 2), __shfl_sync(0xffffffffu, bias, cc * 4 + 3));
+            float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
+            size_t off = cb + (size_t)(row0 + rsub) * ep.N + st.col;
+            const uint32_t rows = st.live && row0 + rsub < ep.M ? (ep.M - row0 - rsub + 3) / 4 : 0u;      // this lane's, of eight
+            auto sum_at = [&](uint32_t i) {
+                const uint32_t lr = i * 4 + rsub;
+                return add4(tb4[lr * 8 + (cc ^ (lr & 7))], bz);
+            };
+            if (st.plain) {
 #pragma unroll
-        for (int j = 0; j < CPT; ++j) sum[j] = 0.0f;
-        bool ok = true;
-        for (uint32_t c = 0; c < nchunks; ++c) {
-            const uint32_t buf = c & 1u;
-            bool got = mbar_wait_bounded(acc_full_bar(buf), (c >> 1) & 1u, kWaitCycles + kWaitCycles / 2);
-            got = __all_sync(0xffffffffu, got);
-            if (!got) {
-                if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_EPI_WAIT);
-                ok = false;
-                break;
+                for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
+                    if (i < rows) cs = add4(cs, st.put_plain(ep, off, sum_at(i)));
+            } else {
+#pragma unroll 2
+                for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
+                    if (i < rows) cs = add4(cs, st.put(ep, off, sum_at(i)));
             }
-            tc_fence_after();
-            const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * CPT;
-#pragma unroll
-            for (int g = 0; g < CPT / 32; ++g) {
-                uint32_t r[32];
-                tmem_ld_32x32(t0 + g * 32, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) sum[g * 32 + j] += __uint_as_float(r[j]);
+            __syncwarp();
+            if (ep.colsum_part) {
+                cs = sum_column_lanes(cs);
+                if (lane < 8 && row0 < ep.M) store_colsum(ep, row0, st.col, cs);
             }
-            tc_fence_before();
-            if (lane == 0) mbar_arrive(acc_empty_bar(buf));
-        }
-        if (ok) {
-            // Every load and MMA of this CTA has finished (the last chunk is complete), so the first stage is free: each
-            // warp passes 32 x 32 blocks through its 4 KB of it and writes 4 rows x 128 bytes per instruction.
-            // A K-share goes out raw into its slot.
-            const bool part = ep.split > 1;
-            const uint32_t slot = (bz * gridDim.x + blockIdx.x) * ep.split + blockIdx.y;
-            float* const pout = part ? ep.partial + (size_t)slot * (BM * BN) : nullptr;
-            const size_t cb = (size_t)bz * ep.c_batch;
-            const bool vec = (ep.N % 4 == 0) && (ep.c_batch % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
-                             (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0) &&
-                             (!ep.mul_saved || (reinterpret_cast<uintptr_t>(ep.mul_saved) & 15u) == 0);
-            float4* const tb4 = reinterpret_cast<float4*>(base_ptr) + (warp - 2) * (32 * 8);
-            const uint32_t rsub = lane >> 3, cc = lane & 7;
-            const uint32_t row0 = m0 + q * 32;
+            __syncwarp();
+        };
+        for (uint32_t u = first; u < ca.units && ok; u += step) {
+            const Unit t = unit_at(u);
+            const uint32_t nchunks = (t.nkb + kChunkKB - 1) / kChunkKB;
+            // a lane holds the bias of one column per block: it is here long before the sums are
+            float bias[CPT / 32];
+            if constexpr (!SHARES) {
+                const float* const bp = ep_of(t.p, [](const Epilogue& e) { return e.bias; });
+                const uint32_t N = ep_of(t.p, [](const Epilogue& e) { return e.N; });
 #pragma unroll
-            for (int g = 0; g < CPT / 32; ++g) {
+                for (int gr = 0; gr < CPT / 32; ++gr) {
+                    const uint32_t c = t.n0 + half * CPT + gr * 32 + lane;
+                    bias[gr] = bp && c < N ? bp[c] : 0.0f;
+                }
+            }
+            float sum[CPT];
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    tb4[lane * 8 + (c ^ (lane & 7))] = make_float4(sum[g * 32 + 4 * c], sum[g * 32 + 4 * c + 1],
-                                                                   sum[g * 32 + 4 * c + 2], sum[g * 32 + 4 * c + 3]);
+            for (int j = 0; j < CPT; ++j) sum[j] = 0.0f;
+            for (uint32_t c = 0; c < nchunks; ++c, ++gc) {
+                const uint32_t buf = gc & 1u;
+                bool got = mbar_wait_bounded(acc_full_bar(buf), (gc >> 1) & 1u, kWaitCycles + kWaitCycles / 2);
+                got = __all_sync(0xffffffffu, got);
+                if (!got) {
+                    if (lane == 0) atomicOr(ca.dev_status, FG_DEVERR_EPI_WAIT);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * CPT;
+#pragma unroll
+                for (int gr = 0; gr < CPT / 32; ++gr) {
+                    uint32_t r[32];
+                    tmem_ld_32x32(t0 + gr * 32, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[gr * 32 + j] += __uint_as_float(r[j]);
+                }
+                tc_fence_before();
                 __syncwarp();
-                const uint32_t lcol = half * CPT + g * 32 + cc * 4, col = n0 + lcol;
-                if (part) {
+                if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+            }
+            if (!ok) break;
+            if constexpr (SHARES) {
+                // Every load and MMA of this CTA has finished (its last chunk is complete), so the stages are free: the share's
+                // sums as [row][BN], float4 c of a row at c ^ (row & 7).
+                float4* const part = reinterpret_cast<float4*>(base_ptr) + (q * 32 + lane) * (BN / 4);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const uint32_t lr = i * 4 + rsub;
-                        *reinterpret_cast<float4*>(pout + (size_t)(q * 32 + lr) * BN + lcol) = tb4[lr * 8 + (cc ^ (lr & 7))];
+                for (int c = 0; c < CPT / 4; ++c)
+                    part[(half * (CPT / 4) + c) ^ (lane & 7)] = make_float4(sum[4 * c], sum[4 * c + 1], sum[4 * c + 2], sum[4 * c + 3]);
+            } else {
+#pragma unroll 1
+                for (int gr = 0; gr < CPT / 32; ++gr) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        float4 v = make_float4(sum[4 * c], sum[4 * c + 1], sum[4 * c + 2], sum[4 * c + 3]);
+                        if (CPT > 32 && gr) v = make_float4(sum[CPT - 32 + 4 * c], sum[CPT - 32 + 4 * c + 1], sum[CPT - 32 + 4 * c + 2], sum[CPT - 32 + 4 * c + 3]);
+                        tb4[lane * 8 + (c ^ (lane & 7))] = v;
                     }
                     __syncwarp();
-                    continue;
+                    const uint32_t row0 = t.m0 + q * 32, col0 = t.n0 + half * CPT + gr * 32;
+                    const float bv = CPT > 32 && gr ? bias[CPT / 32 - 1] : bias[0];
+                    if (!TWO || t.p == 0) store_block(ca.ep[0], (size_t)t.bz * ca.ep[0].c_batch, row0, col0, bv);
+                    else store_block(ca.ep[1], (size_t)t.bz * ca.ep[1].c_batch, row0, col0, bv);
                 }
-                float4 bz4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (ep.bias) {
-                    if (col < ep.N) bz4.x = ep.bias[col];
-                    if (col + 1 < ep.N) bz4.y = ep.bias[col + 1];
-                    if (col + 2 < ep.N) bz4.z = ep.bias[col + 2];
-                    if (col + 3 < ep.N) bz4.w = ep.bias[col + 3];
-                }
-                float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
-                const bool fast = vec && col + 3 < ep.N;
-#pragma unroll 4
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t lr = i * 4 + rsub, row = row0 + lr;
-                    float4 z = tb4[lr * 8 + (cc ^ (lr & 7))];
-                    z.x += bz4.x; z.y += bz4.y; z.z += bz4.z; z.w += bz4.w;
-                    if (row < ep.M && col < ep.N) {
-                        const size_t off = cb + (size_t)row * ep.N + col;
-                        float4 o;
-                        if (fast) {
-                            if (ep.mul_saved) {
-                                const float4 sv = __ldg(reinterpret_cast<const float4*>(ep.mul_saved + off));
-                                o = make_float4(z.x * fg_act_grad_sel(ep.mul_act, sv.x), z.y * fg_act_grad_sel(ep.mul_act, sv.y),
-                                                z.z * fg_act_grad_sel(ep.mul_act, sv.z), z.w * fg_act_grad_sel(ep.mul_act, sv.w));
-                            } else if (ep.act != FG_ACT_NONE) {
-                                o = make_float4(fg_act_fwd_sel(ep.act, z.x), fg_act_fwd_sel(ep.act, z.y), fg_act_fwd_sel(ep.act, z.z),
-                                                fg_act_fwd_sel(ep.act, z.w));
-                            } else o = z;
-                            if (ep.preact) *reinterpret_cast<float4*>(ep.preact + off) = z;
-                            *reinterpret_cast<float4*>(ep.C + off) = o;
-                            if (ep.c_pairs) fg_store_pairs4(ep.c_pairs, ep.c_pairs_stride, off, o);
-                        } else {
-                            o = epi_store_edge(z, off, col, ep.N, (char*)ep.C, (char*)ep.preact, ep.c_pairs, ep.c_pairs_stride, ep.mul_saved,
-                                               ep.mul_act, ep.act, FG_DTYPE_F32);
-                        }
-                        cs.x += o.x; cs.y += o.y; cs.z += o.z; cs.w += o.w;
-                    }
-                }
-                if (ep.colsum_part) {
-                    cs.x += __shfl_xor_sync(0xffffffffu, cs.x, 8); cs.x += __shfl_xor_sync(0xffffffffu, cs.x, 16);
-                    cs.y += __shfl_xor_sync(0xffffffffu, cs.y, 8); cs.y += __shfl_xor_sync(0xffffffffu, cs.y, 16);
-                    cs.z += __shfl_xor_sync(0xffffffffu, cs.z, 8); cs.z += __shfl_xor_sync(0xffffffffu, cs.z, 16);
-                    cs.w += __shfl_xor_sync(0xffffffffu, cs.w, 8); cs.w += __shfl_xor_sync(0xffffffffu, cs.w, 16);
-                    if (lane < 8 && row0 < ep.M) {
-                        float* d = ep.colsum_part + (size_t)(row0 >> 5) * ep.N + col;
-                        if (col < ep.N) d[0] = cs.x;
-                        if (col + 1 < ep.N) d[1] = cs.y;
-                        if (col + 2 < ep.N) d[2] = cs.z;
-                        if (col + 3 < ep.N) d[3] = cs.w;
-                    }
-                }
-                __syncwarp();
             }
         }
+        if constexpr (SHARES) { __syncwarp(); cluster_sync_all(); cluster_sync_all(); }      // as the converters
     }
     tc_fence_before();
     __syncthreads();
@@ -1916,27 +2078,43 @@ struct ConvPlan {
     uint32_t bn, split;
     double cycles;       // estimate; 0: cannot run
 };
-// Estimated SM cycles of the kernels for [M,K] x [K,N] (times `batch`), from their per-k-block costs and fixed overheads.
-ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32_t batch) {
+struct ConvShape { uint32_t M, N, K, batch; };
+template <int BN> int conv_clusters(const fg_ctx* ctx, uint32_t split);
+// Estimated SM cycles of one launch for one or two products (the one with the longer k first), from measured costs: per k-block
+// 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
+// set-up and first loads, 2 - 3 us for the shares' sums to meet; 6 us more where a ragged N is stored element by element.
+ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n) {
     ConvPlan best{128, 1, 0.0};
-    const uint64_t sms = (uint64_t)ctx->sm_count, nkb = (K + 31) / 32;
+    const uint64_t sms = (uint64_t)ctx->sm_count;
     for (uint32_t bn = 128; bn >= 64; bn -= 64) {
-        const uint64_t tiles = (uint64_t)((M + BM - 1) / BM) * ((N + bn - 1) / bn) * batch;
-        for (uint64_t split = 1; split <= 16 && (split == 1 || (split * 4 <= nkb && tiles * split <= 2 * sms)); ++split) {
-            const uint64_t waves = (tiles * split + sms - 1) / sms, kb = (nkb + split - 1) / split;
-            // measured slopes and offsets: 0.9 and 0.6 us per k-block, 7.2 and 5.3 us around them; a ragged N stored straight
-            // from the tiles, element by element, 6 us more; the fold 2 us and 4.3 TB/s
-            double c = (double)waves * ((double)kb * (bn == 128 ? 1700.0 : 1150.0) + (bn == 128 ? 13000.0 : 9800.0) +
-                                        (split == 1 && N % 4 != 0 ? 11000.0 : 0.0));
-            if (split > 1) c += 3700.0 + (double)(tiles * split) * BM * bn * 4.0 / 2300.0;
-            if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, (uint32_t)split, c};
+        uint64_t units[2] = {0, 0}, nkb[2] = {0, 0}, min_kb = ~0ull;
+        for (int i = 0; i < n; ++i) {
+            units[i] = (uint64_t)((sh[i].M + BM - 1) / BM) * ((sh[i].N + bn - 1) / bn) * sh[i].batch;
+            nkb[i] = (sh[i].K + 31) / 32;
+            if (nkb[i] < min_kb) min_kb = nkb[i];
+        }
+        const uint64_t all = units[0] + units[1];
+        const double kb = bn == 128 ? 1050.0 : 600.0, store = bn == 128 ? 5000.0 : 2800.0, around = 6500.0;
+        const double edge = sh[0].N % 4 != 0 || (n > 1 && sh[1].N % 4 != 0) ? (bn == 128 ? 11000.0 : 5500.0) : 0.0;
+        // whole units: the first CTA's units are one of every sms
+        const uint64_t rounds = (all + sms - 1) / sms, rounds0 = units[0] / sms + (units[0] % sms != 0);
+        auto unit = [&](int i) { return (double)nkb[i] * kb > store + edge ? (double)nkb[i] * kb : store + edge; };
+        double c = around + store + edge + (double)rounds0 * unit(0) + (double)(rounds - rounds0) * unit(1);
+        if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, 1, c};
+        for (uint32_t split = 2; split <= 8 && split * 2 <= min_kb && all * split <= 2 * sms; ++split) {
+            const int fit = bn == 128 ? conv_clusters<128>(ctx, split) : conv_clusters<64>(ctx, split);
+            if (fit < 1) continue;
+            const uint64_t turns = (all + fit - 1) / fit;
+            const double share = (double)((nkb[0] + split - 1) / split) * kb;
+            c = (double)turns * (share + around + 5500.0 + edge / split);
+            if (c < best.cycles) best = ConvPlan{bn, split, c};
         }
     }
     return best;
 }
-uint64_t conv_partial_bytes(const ConvPlan& p, uint32_t M, uint32_t N, uint32_t batch) {
-    if (p.split <= 1) return 0;
-    return (uint64_t)((M + BM - 1) / BM) * ((N + p.bn - 1) / p.bn) * batch * p.split * BM * p.bn * 4 + 256;
+ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32_t batch) {
+    const ConvShape sh{M, N, K, batch};
+    return plan_conv(ctx, &sh, 1);
 }
 // The pair kernel for one matrix: 256 x 256 tiles on SM pairs, plus the passes that make the pairs of `prep` elements.
 double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double prep_elems, int prep_launches) {
@@ -1954,55 +2132,113 @@ double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double
 }
 inline bool conv_allowed(const fg_ctx* ctx) { return ctx->opt_pairs && ctx->opt_tile_pair < 0 && ctx->tmap_encode; }
 
-template <int BN>
-int32_t launch_conv_bn(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, Epilogue ep, uint32_t batch) {
-    using Cfg = ConvCfg<BN>;
-    CUtensorMap tm[2];
-    int32_t s;
-    const PlaneSet* ops[2] = {&a, &b};
-    const uint32_t rows[2] = {ep.M, ep.N}, tile[2] = {(uint32_t)BM, (uint32_t)BN};
-    for (int i = 0; i < 2; ++i) {
-        const PlaneSet& o = *ops[i];
-        const uint64_t apart = (o.batch32 ? o.batch32 : (uint64_t)(o.mn ? ep.K : rows[i]) * o.ld32) * 4;
-        if (!o.mn) s = make_tmap3(ctx, &tm[i], o.p32, 0, ep.K, rows[i], batch, (uint64_t)o.ld32 * 4, apart, 32, tile[i], 1);
-        else s = make_tmap3(ctx, &tm[i], o.p32, 0, rows[i], ep.K, batch, (uint64_t)o.ld32 * 4, apart, 32, 32, 1, true);
-        if (s != FG_OK) return s;
-    }
-    ep.a_mn = a.mn ? 1u : 0u;
-    ep.b_mn = b.mn ? 1u : 0u;
-    static std::atomic<uint64_t> attr_done{0};       // one bit per device
-    if (!(attr_done.load(std::memory_order_acquire) >> (ctx->device & 63) & 1ull)) {
-        FG_CUDA(ctx, FG_ERR_INTERNAL,
-                cudaFuncSetAttribute(gemm_tc_conv_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-        attr_done.fetch_or(1ull << (ctx->device & 63), std::memory_order_release);
-    }
-    const uint64_t tiles_m = (ep.M + BM - 1) / BM, tiles = tiles_m * ((ep.N + BN - 1) / BN);
-    if (tiles > (1ull << 30) || batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM: too many tiles");
-    ep.group = (uint32_t)tiles_m;         // down the columns of tiles: the CTAs at work share a few tile columns of B
-    ep.batch = batch;
-    ep.t_full = 0;
-    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, 2.0 * batch * ep.M * ep.N * ep.K);
-    fg_launch(ctx, gemm_tc_conv_kernel<BN>, dim3((unsigned)tiles, ep.split, batch), Cfg::kThreads, Cfg::kSmemBytes, tm[0], tm[1], ep);
-    FG_LAUNCHED(ctx);
-    if (ep.split > 1) {
-        fg_launch(ctx, gemm_tc_fold_kernel<BM, BN>, (unsigned)(tiles * batch * (BM / 32) * (BN / 32)), 256, 0, ep);
-        FG_LAUNCHED(ctx);
-    }
-    fg_time_end(ctx, tr);
-    return FG_OK;
+// The kernel may use its shared memory, on this device (one bit per device).
+template <int BN, bool TWO, bool SHARES>
+cudaError_t conv_attr(const fg_ctx* ctx) {
+    static std::atomic<uint64_t> done{0};
+    if (done.load(std::memory_order_acquire) >> (ctx->device & 63) & 1ull) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_tc_conv_kernel<BN, TWO, SHARES>, cudaFuncAttributeMaxDynamicSharedMemorySize, ConvCfg<BN>::kSmemBytes);
+    if (e == cudaSuccess) done.fetch_or(1ull << (ctx->device & 63), std::memory_order_release);
+    return e;
 }
-// The caller has reserved conv_partial_bytes().
-int32_t launch_conv(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilogue& ep_in, const ConvPlan& p, uint32_t batch) {
-    Epilogue ep = ep_in;
-    ep.split = p.split;
-    ep.partial = nullptr;
-    if (p.split > 1) {
-        void* part;
-        int32_t s = fg_ws_alloc(ctx, conv_partial_bytes(p, ep.M, ep.N, batch), &part);
-        if (s != FG_OK) return s;
-        ep.partial = (float*)part;
+// Clusters of `split` CTAs that are resident at once (asked of the runtime, once per device: how the SMs are grouped is not
+// documented); 0 if they cannot be launched.
+template <int BN>
+int conv_clusters(const fg_ctx* ctx, uint32_t split) {
+    static std::atomic<int> known[64][9];       // zero-initialised; the same value whoever computes it, stored plus one
+    std::atomic<int>& k = known[ctx->device & 63][split];
+    int n = k.load(std::memory_order_acquire) - 1;
+    if (n >= 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(split * 64);
+    cfg.blockDim = dim3(ConvCfg<BN>::kThreads);
+    cfg.dynamicSmemBytes = ConvCfg<BN>::kSmemBytes;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = split; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (conv_attr<BN, false, true>(ctx) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_tc_conv_kernel<BN, false, true>, &cfg) != cudaSuccess || n < 0) {
+        cudaGetLastError();
+        n = 0;
     }
-    return p.bn == 128 ? launch_conv_bn<128>(ctx, a, b, ep, batch) : launch_conv_bn<64>(ctx, a, b, ep, batch);
+    k.store(n + 1, std::memory_order_release);
+    return n;
+}
+
+// One product of a launch: its operands, their roles and the epilogue.
+struct ConvProduct {
+    PlaneSet a, b;
+    Epilogue ep;
+    uint32_t batch;
+};
+template <int BN>
+int32_t launch_conv_bn(fg_ctx* ctx, const ConvProduct* pr, int n, uint32_t split) {
+    using Cfg = ConvCfg<BN>;
+    CUtensorMap tm[4];
+    ConvArgs ca{};
+    uint64_t units = 0;
+    double flop = 0.0;
+    for (int j = 0; j < n; ++j) {
+        const ConvProduct& c = pr[j];
+        const PlaneSet* ops[2] = {&c.a, &c.b};
+        const uint32_t rows[2] = {c.ep.M, c.ep.N}, tile[2] = {(uint32_t)BM, (uint32_t)BN};
+        for (int i = 0; i < 2; ++i) {
+            const PlaneSet& o = *ops[i];
+            const uint64_t apart = (o.batch32 ? o.batch32 : (uint64_t)(o.mn ? c.ep.K : rows[i]) * o.ld32) * 4;
+            int32_t s;
+            if (!o.mn) s = make_tmap3(ctx, &tm[2 * j + i], o.p32, 0, c.ep.K, rows[i], c.batch, (uint64_t)o.ld32 * 4, apart, 32, tile[i], 1);
+            else s = make_tmap3(ctx, &tm[2 * j + i], o.p32, 0, rows[i], c.ep.K, c.batch, (uint64_t)o.ld32 * 4, apart, 32, 32, 1, true);
+            if (s != FG_OK) return s;
+        }
+        ca.ep[j] = c.ep;
+        ca.ep[j].a_mn = c.a.mn ? 1u : 0u;
+        ca.ep[j].b_mn = c.b.mn ? 1u : 0u;
+        const uint64_t tiles = (uint64_t)((c.ep.M + BM - 1) / BM) * ((c.ep.N + BN - 1) / BN);
+        if (tiles > (1ull << 30) || c.batch > 65535 || units + tiles * c.batch > (1ull << 31))
+            return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM: too many tiles");
+        units += tiles * c.batch;
+        if (j == 0) ca.units0 = (uint32_t)units;
+        flop += 2.0 * c.batch * c.ep.M * c.ep.N * c.ep.K;
+    }
+    if (n == 1) { tm[2] = tm[0]; tm[3] = tm[1]; }
+    ca.units = (uint32_t)units;
+    ca.split = split;
+    ca.dev_status = ctx->dev_status;
+    const uint64_t sms = (uint64_t)ctx->sm_count;
+    const uint32_t grid = (uint32_t)(split > 1 ? units * split : units < sms ? units : sms);
+    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, flop);
+    auto launch = [&](auto two, auto shares) -> int32_t {
+        constexpr bool T = decltype(two)::value, S = decltype(shares)::value;
+        FG_CUDA(ctx, FG_ERR_INTERNAL, (conv_attr<BN, T, S>(ctx)));
+        fg_launch_cluster(ctx, gemm_tc_conv_kernel<BN, T, S>, grid, Cfg::kThreads, Cfg::kSmemBytes, split, tm[0], tm[1], tm[2], tm[3], ca);
+        FG_LAUNCHED(ctx);
+        return FG_OK;
+    };
+    const std::true_type yes{};
+    const std::false_type no{};
+    const int32_t s = n == 2 ? (split > 1 ? launch(yes, yes) : launch(yes, no)) : split > 1 ? launch(no, yes) : launch(no, no);
+    fg_time_end(ctx, tr);
+    return s;
+}
+int32_t launch_conv(fg_ctx* ctx, const ConvProduct* pr, int n, const ConvPlan& p) {
+    return p.bn == 128 ? launch_conv_bn<128>(ctx, pr, n, p.split) : launch_conv_bn<64>(ctx, pr, n, p.split);
+}
+int32_t launch_conv(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilogue& ep, const ConvPlan& p, uint32_t batch) {
+    const ConvProduct pr{a, b, ep, batch};
+    return launch_conv(ctx, &pr, 1, p);
+}
+// The two gradients of a layer in one launch: more units to share out, and one wave's end instead of two.  The longer k goes
+// first, so that the short units fill the last round.  Two launches where each wants K-shares of its own (128 x 4096 x 1024: k of
+// 4096 on eight tiles and of 128 on 256 of them, 60 us together, 39 apart).
+int32_t launch_conv_both(fg_ctx* ctx, const ConvProduct& x, const ConvProduct& y) {
+    const ConvProduct pr[2] = {x.ep.K >= y.ep.K ? x : y, x.ep.K >= y.ep.K ? y : x};
+    const ConvShape sh[2] = {{pr[0].ep.M, pr[0].ep.N, pr[0].ep.K, pr[0].batch}, {pr[1].ep.M, pr[1].ep.N, pr[1].ep.K, pr[1].batch}};
+    const ConvPlan together = plan_conv(ctx, sh, 2), one = plan_conv(ctx, sh, 1), two = plan_conv(ctx, sh + 1, 1);
+    if (together.cycles <= one.cycles + two.cycles) return launch_conv(ctx, pr, 2, together);
+    const int32_t s = launch_conv(ctx, pr, 1, one);
+    return s != FG_OK ? s : launch_conv(ctx, pr + 1, 1, two);
 }
 
 // A dense [R, C] f32 tensor (`batch` of them, x_batch apart) can be loaded as it lies when rows and matrices start on
@@ -2240,7 +2476,7 @@ int32_t gemm_fwd_core(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
         const Route r = pick_route(ctx, M, N, K, pair_ok, (A.pairs ? 0.0 : (double)M * K) + (B.pairs ? 0.0 : (double)K * N), !A.pairs + !B.pairs,
                                    (ca ? (double)M * K : 0.0) + (cb ? (double)K * N : 0.0), (ca != 0) + (cb != 0));
         if (r.kind == kRouteConv) {
-            int32_t s = fg_ws_ensure(ctx, ca + cb + conv_partial_bytes(r.conv, M, N, 1) + 1024);
+            int32_t s = fg_ws_ensure(ctx, ca + cb + 1024);
             if (s != FG_OK) return s;
             PlaneSet pa, pb;
             if ((s = loadable32(ctx, A.x, rows_a, pitch_a, 1, 0, &pa)) != FG_OK) return s;
@@ -2468,7 +2704,7 @@ uint64_t bwd_planes_need(uint32_t M, uint32_t N, uint32_t K) {
 // Pairs that are not supplied are made in the scratch arena.  The caller has reserved bwd_paired_need().
 uint32_t colsum_room(uint32_t M, uint32_t N) { return N <= 16 ? fg_gemm_skinny_colsum_rows(M) : (M + 31) / 32; }
 uint64_t bwd_paired_need(uint32_t M, uint32_t N, uint32_t K) {
-    // (the conversion kernel's K-shares take less than kPairPartialBytes, its padded copies less than the planes)
+    // (the conversion kernel's padded copies take less than the planes)
     return 4ull * ((uint64_t)M * K + (uint64_t)K * N + (uint64_t)M * N) + (uint64_t)colsum_room(M, N) * K * 4 +
            2 * kPairPartialBytes + 4096 + fg_gemm_skinny_scratch_bytes(M, N, K) + bwd_planes_need(M, N, K);
 }
@@ -2528,6 +2764,8 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         if (ldz == N && (s = loadable32(ctx, dZ.x, M, N, 1, 0, &z32)) != FG_OK) return s;
         if (ldz != N) { z32 = PlaneSet{}; z32.p32 = const_cast<float*>(dZ.x); z32.ld32 = ldz; }
     }
+    const bool one = conv_b && conv_a && !exch_buf;      // both gradients in one launch
+    ConvProduct both[2];
     if (pair_b) {
         if ((s = make_pairs(A, mk)) != FG_OK) return s;
         // operands Aᵀ (rows = K) and dZᵀ (rows = N), both read from [M, .] storage: contraction over the rows
@@ -2539,7 +2777,8 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         PlaneSet a32;
         if ((s = loadable32(ctx, A.x, M, K, 1, 0, &a32)) != FG_OK) return s;
         const Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
-        if ((s = launch_conv(ctx, as_operand(a32, true), as_operand(z32, true), ep, rt.dB.conv, 1)) != FG_OK) return s;
+        both[0] = ConvProduct{as_operand(a32, true), as_operand(z32, true), ep, 1};
+        if (!one && (s = launch_conv(ctx, &both[0], 1, rt.dB.conv)) != FG_OK) return s;
     } else if (dB && (s = gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, A.x, nullptr, dZ.x, FG_ACT_NONE, nullptr, nullptr, dB, nullptr,
                                           nullptr, nullptr, 0)) != FG_OK) return s;
     if (exch_buf && (s = fg_allreduce_sum_f32(ctx, exch_buf, exch_count)) != FG_OK) return s;
@@ -2558,7 +2797,8 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         ep.mul_saved = o.mul_saved;
         ep.mul_act = o.mul_act;
         ep.colsum_part = o.colsum_part;
-        if ((s = launch_conv(ctx, as_operand(z32, false), as_operand(b32, false), ep, rt.dA.conv, 1)) != FG_OK) return s;
+        both[1] = ConvProduct{as_operand(z32, false), as_operand(b32, false), ep, 1};
+        if ((s = one ? launch_conv_both(ctx, both[0], both[1]) : launch_conv(ctx, &both[1], 1, rt.dA.conv)) != FG_OK) return s;
     } else if (dA) {        // (o is left to the caller)
         return gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, nullptr, B.x, dZ.x, FG_ACT_NONE, nullptr, dA, nullptr, nullptr, nullptr, nullptr, 0);
     }
@@ -2648,9 +2888,9 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
             else {       // dZ and what each product carves: never more than the operand planes of both would take
                 if (own_z) need += (uint64_t)M * round4(N) * 4 + 256;
                 if (dB) need += rt.dB.kind == kRoutePlanes ? planes_bytes(1, N, M) + planes_bytes(1, K, M) + kPairPartialBytes + 4096
-                                                           : copy32_bytes(A, M, K, 1, 0) + conv_partial_bytes(rt.dB.conv, K, N, 1);
+                                                           : copy32_bytes(A, M, K, 1, 0);
                 if (dA) need += rt.dA.kind == kRoutePlanes ? planes_bytes(1, M, N) + planes_bytes(1, K, N) + kPairPartialBytes + 4096
-                                                           : copy32_bytes(B, K, N, 1, 0) + conv_partial_bytes(rt.dA.conv, M, K, 1);
+                                                           : copy32_bytes(B, K, N, 1, 0);
             }
             { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
             int32_t s;
@@ -2787,8 +3027,7 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
     if (batch_route_open(ctx, mode, M, N, K)) {
         if (batch_converts(ctx, batch, M, N, K, paired_shape_ok(ctx, M, N, K, K, N))) {
             auto need = [&](uint32_t t) {
-                return copy32_bytes(A, M, K, t, strideA) + copy32_bytes(B, K, N, t, strideB) +
-                       conv_partial_bytes(plan_conv(ctx, M, N, K, t), M, N, t) + 1024;
+                return copy32_bytes(A, M, K, t, strideA) + copy32_bytes(B, K, N, t, strideB) + 1024;
             };
             const uint32_t part = batch_part(ctx, batch, planes_bytes(1, M, K) + planes_bytes(1, N, K) + kPairPartialBytes + 1024, need);
             for (uint32_t t0 = 0; t0 < batch; t0 += part) {
@@ -2879,17 +3118,18 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
         const bool own_z = act != FG_ACT_NONE;
         auto need = [&](uint32_t t) {
             return (own_z ? (uint64_t)t * M * round4(N) * 4 + 256 : copy32_bytes(dY, M, N, t, strideC)) +
-                   (dB ? copy32_bytes(A, M, K, t, strideA) + conv_partial_bytes(plan_conv(ctx, K, N, M, t), K, N, t) : 0) +
-                   (dA ? copy32_bytes(B, K, N, t, strideB) + conv_partial_bytes(plan_conv(ctx, M, K, N, t), M, K, t) : 0) + 2048;
+                   (dB ? copy32_bytes(A, M, K, t, strideA) : 0) +
+                   (dA ? copy32_bytes(B, K, N, t, strideB) : 0) + 2048;
         };
         const uint64_t loop = 2048 + (dA ? planes_bytes(1, M, N) + planes_bytes(1, K, N) + kPairPartialBytes : 0) +
                               (dB ? planes_bytes(1, N, M) + planes_bytes(1, K, M) + kPairPartialBytes : 0);
         const uint32_t part = all ? batch_part(ctx, batch, loop, need) : 0;
-        // dZ for a part of the batch in one pass, then one launch per product
+        // dZ for a part of the batch in one pass, then one launch for the product or both
         for (uint32_t t0 = 0; t0 < batch && all; t0 += part) {
             const uint32_t t = batch - t0 < part ? batch - t0 : part;
             const float* const dy = dY + t0 * strideC;
             PlaneSet z, x;
+            ConvProduct both[2];
             ctx->ws_used = 0;
             int32_t s = fg_ws_ensure(ctx, need(t));
             if (s != FG_OK) return s;
@@ -2908,13 +3148,15 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
                 if ((s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &x)) != FG_OK) return s;
                 Epilogue ep{dB + t0 * strideB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
                 ep.c_batch = t > 1 ? strideB : 0;
-                if ((s = launch_conv(ctx, as_operand(x, true), as_operand(z, true), ep, plan_conv(ctx, K, N, M, t), t)) != FG_OK) return s;
+                both[0] = ConvProduct{as_operand(x, true), as_operand(z, true), ep, t};
+                if (!dA && (s = launch_conv(ctx, &both[0], 1, plan_conv(ctx, K, N, M, t))) != FG_OK) return s;
             }
             if (dA) {
                 if ((s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &x)) != FG_OK) return s;
                 Epilogue ep{dA + t0 * strideA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
                 ep.c_batch = t > 1 ? strideA : 0;
-                if ((s = launch_conv(ctx, as_operand(z, false), as_operand(x, false), ep, plan_conv(ctx, M, K, N, t), t)) != FG_OK) return s;
+                both[1] = ConvProduct{as_operand(z, false), as_operand(x, false), ep, t};
+                if ((s = dB ? launch_conv_both(ctx, both[0], both[1]) : launch_conv(ctx, &both[1], 1, plan_conv(ctx, M, K, N, t))) != FG_OK) return s;
             }
         }
         if (all) return FG_OK;
