@@ -125,3 +125,45 @@ def test_gelu_of_extreme_values(ctx, dtype):
         dz = ctx.new_tensor((n,))
         ctx.act_bwd(ones, t, dz, n, "gelu")
         assert np.array_equal(ctx.to_numpy(dz), g, equal_nan=True)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("n", [7, 2048, 2049, 4097, 50003])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_packed_arithmetic_rounds_as_single_steps_do(ctx, dtype, n, shift):
+    # + - * / on 16-bit elements, two at a time or not, equals the f32 operation followed by one rounding: bit for bit, with
+    # subnormals, infinities and NaN among the values; tiles of 2048, an incomplete last one, tensors off the boundary of four
+    import torch
+    td = {"f16": torch.float16, "bf16": torch.bfloat16}[dtype]
+    gen = torch.Generator().manual_seed(n + shift)
+    special = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), 1e-7, -1e-7, 6e4, -6e4, 1e-39, -1e-39, 1.0])
+
+    def values():
+        v = torch.randn(n, generator=gen)
+        at = torch.randint(0, n, (max(1, n // 5),), generator=gen)
+        v[at] = special[torch.randint(0, len(special), (len(at),), generator=gen)]
+        return v.to(td)
+
+    x, y, g = values(), values(), values()
+    place = lambda v: torch.cat([torch.zeros(shift, dtype=td), v]).cuda()   # noqa: E731
+    r = lambda v: v.to(td).float()                                          # noqa: E731
+    xf, yf, gf = x.float(), y.float(), g.float()
+    prog = [("input", 0, 0, 0.0), ("input", 1, 0, 0.0), ("add", 0, 1, 0.0), ("mul", 2, 0, 0.0), ("sub", 1, 3, 0.0), ("div", 4, 1, 0.0),
+            ("neg", 5, 0, 0.0), ("abs", 4, 0, 0.0), ("add", 6, 7, 0.0), ("relu", 8, 0, 0.0)]
+    a = r(xf + yf)
+    m = r(a * xf)
+    d = r(yf - m)
+    t = r(-r(d / yf) + d.abs())
+    want = torch.where(t > 0, t, torch.zeros_like(t)).to(td)
+    xd, yd, gd, out, dx, dy = (place(v) for v in (x, y, g, torch.zeros_like(x), torch.zeros_like(x), torch.zeros_like(x)))
+    torch.cuda.synchronize()
+    p = lambda v: v.data_ptr() + 2 * shift                                  # noqa: E731
+    ctx.eltwise_chain_fwd(prog, [p(xd), p(yd)], p(out), n, dtype=dtype)
+    ctx.sync()
+    same = lambda u, v: torch.equal(torch.nan_to_num(u, nan=123.0), torch.nan_to_num(v, nan=123.0)) and torch.equal(u.isnan(), v.isnan())  # noqa: E731
+    assert same(out.cpu()[shift:], want)
+    ctx.eltwise_chain_bwd([("input", 0, 0, 0.0), ("input", 1, 0, 0.0), ("mul", 0, 1, 0.0), ("relu", 2, 0, 0.0)], [p(xd), p(yd)], p(gd),
+                          [p(dx), p(dy)], n, dtype=dtype)
+    ctx.sync()
+    adj = gf * (r(xf * yf) > 0).float()
+    assert same(dx.cpu()[shift:], (adj * yf).to(td)) and same(dy.cpu()[shift:], (adj * xf).to(td))
