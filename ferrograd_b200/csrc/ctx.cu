@@ -216,8 +216,8 @@ int32_t fg_ctx_create_on_stream(int32_t device, void* cuda_stream, fg_ctx** out)
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         !create_events(c->ev_ckpt, 8) ||
-        cudaMalloc((void**)&c->dev_status, 256) != cudaSuccess ||
-        cudaMemset(c->dev_status, 0, 256) != cudaSuccess) {
+        cudaMalloc((void**)&c->dev_status, kFgStatusBytes) != cudaSuccess ||
+        cudaMemset(c->dev_status, 0, kFgStatusBytes) != cudaSuccess) {
         // release whatever was created before the failure (the struct was zeroed: untouched members are NULL)
         if (c->comm_stream) cudaStreamDestroy(c->comm_stream);
         if (c->copy_stream) cudaStreamDestroy(c->copy_stream);

@@ -76,6 +76,23 @@ __global__ void __launch_bounds__(256) act_bwd_kernel(uint64_t n, int act, const
         dz[i] = act == FG_ACT_NONE ? dy[i] : dy[i] * fg_act_grad(act, saved[i]);
 }
 
+// The sum of the blocks' sums (`s` in thread 0 of 256) by the block that arrives last: partials in strides of 256, then across the
+// threads.
+__device__ __forceinline__ void fold_sums(float s, float* __restrict__ partials, unsigned* arrivals, float* __restrict__ out, float* red) {
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (!fg_last_block(arrivals, gridDim.x)) return;
+    s = 0.0f;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += 256) s += __ldcg(partials + i);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.0f;
+        for (int w = 0; w < 8; ++w) t += red[w];
+        *out = t;
+    }
+}
+
 struct MseTerm {   // loss = d*d, grad = 2*d*scale
     static __device__ __forceinline__ float loss(float p, float t) { const float d = p - t; return d * d; }
     static __device__ __forceinline__ float grad(float p, float t, float scale) { return (2.0f * (p - t)) * scale; }
@@ -85,11 +102,12 @@ struct BceTerm {   // on probabilities: loss = -(t*log(p) + (1-t)*log(1-p)), gra
     static __device__ __forceinline__ float grad(float p, float t, float scale) { return (p - t) * scale; }
 };
 
-// Per-element loss and gradient of MSE or BCE; per-CTA partial sums of the loss go to `partials`.
+// Per-element loss and gradient of MSE or BCE, and the sum of the losses through `partials`, one per block.
 template <class TERM, bool VEC>
 __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ pred, const float* __restrict__ target,
                                                    uint64_t n, float scale, float* __restrict__ loss_elem,
-                                                   float* __restrict__ grad, float* __restrict__ partials) {
+                                                   float* __restrict__ grad, float* __restrict__ partials,
+                                                   unsigned* arrivals, float* __restrict__ sum) {
     fg_grid_enter();
     __shared__ float red[8];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -114,33 +132,16 @@ __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ pre
         s = warp_sum(s);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            float t = 0.0f;
-            for (int w = 0; w < 8; ++w) t += red[w];
-            partials[blockIdx.x] = t;
-        }
-    }
-}
-
-// One CTA folds the partials in a fixed order.
-__global__ void __launch_bounds__(256) fold_partials_kernel(const float* __restrict__ partials, int n,
-                                                            float* __restrict__ out) {
-    fg_grid_enter();
-    __shared__ float red[8];
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < n; i += 256) s += partials[i];
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
         float t = 0.0f;
-        for (int w = 0; w < 8; ++w) t += red[w];
-        *out = t;
+        if (threadIdx.x == 0)
+            for (int w = 0; w < 8; ++w) t += red[w];
+        fold_sums(t, partials, arrivals, sum, red);
     }
 }
 
-// Sum of n values, stage 1: one partial per CTA (grid-stride over float4, fixed order inside a CTA).
-__global__ void __launch_bounds__(256) sum_partial_kernel(const float* __restrict__ x, uint64_t n, float* __restrict__ partials) {
+// Sum of n values: one partial per block (grid-stride over float4, fixed order inside a block), then the partials.
+__global__ void __launch_bounds__(256) sum_kernel(const float* __restrict__ x, uint64_t n, float* __restrict__ partials, unsigned* arrivals,
+                                                  float* __restrict__ out) {
     fg_grid_enter();
     __shared__ float red[8];
     float s = 0.0f;
@@ -153,16 +154,38 @@ __global__ void __launch_bounds__(256) sum_partial_kernel(const float* __restric
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
+    float t = 0.0f;
+    if (threadIdx.x == 0)
         for (int w = 0; w < 8; ++w) t += red[w];
-        partials[blockIdx.x] = t;
+    fold_sums(t, partials, arrivals, out, red);
+}
+
+// out[c] = sum over chunks of part[k][c], for 32 columns and 256 threads.  The eight warps each add every eighth chunk into eight
+// sums in turn, which are added in pairs, then the warps' sums in order: 64 short chains of additions (50000 rows in 1563
+// chunks: 3.0e-7 of the sums' 2-norm from 64 bits with eight long ones, 1.3e-7 so).
+__device__ __forceinline__ void fold_chunks_of_columns(uint32_t c, uint32_t gy, uint32_t cx, uint32_t cols, uint32_t nchunks, const float* part,
+                                                       float* __restrict__ out, float (*red)[33]) {
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (c < cols)
+        for (uint64_t k = gy; k < nchunks; k += 64) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (k + 8 * j < nchunks) s[j] += __ldcg(part + (size_t)(k + 8 * j) * cols + c);
+        }
+    red[gy][cx] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    __syncthreads();
+    if (gy == 0 && c < cols) {
+        float t = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[w][cx];
+        out[c] = t;
     }
 }
 
-// Column sums, stage 1: block (32 x 8) covers 32 columns and `chunk` rows.
-__global__ void __launch_bounds__(256) colsum_partial_kernel(uint32_t rows, uint32_t cols, uint32_t chunk,
-                                                             const float* __restrict__ x, float* __restrict__ part) {
+// Column sums: block (32 x 8) covers 32 columns and `chunk` rows and leaves their sums in part[blockIdx.y]; with `out`, the last
+// block of those columns adds the chunks.
+__global__ void __launch_bounds__(256) colsum_kernel(uint32_t rows, uint32_t cols, uint32_t chunk, const float* __restrict__ x, float* part,
+                                                     unsigned* arrivals, float* __restrict__ out) {
     fg_grid_enter();
     __shared__ float red[8][33];
     const uint32_t c = blockIdx.x * 32 + threadIdx.x;
@@ -179,31 +202,16 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(uint32_t rows, uint
         for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
         part[(size_t)blockIdx.y * cols + c] = t;
     }
+    if (!out || !fg_last_block(arrivals + blockIdx.x, gridDim.y)) return;
+    fold_chunks_of_columns(c, threadIdx.y, threadIdx.x, cols, gridDim.y, part, out, red);
 }
-// out[c] = sum over chunks of part[k][c].  A block covers 32 columns; its eight warps each add every eighth chunk into eight
-// sums in turn, which are added in pairs, then the warps' sums in order: 64 short chains of additions (50000 rows in 1563
-// chunks: 3.0e-7 of the sums' 2-norm from 64 bits with eight long ones, 1.3e-7 so).
+// The chunks of column sums that other kernels left; a block covers 32 columns.
 __global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_t nchunks,
                                                           const float* __restrict__ part, float* __restrict__ out) {
     fg_grid_enter();
     __shared__ float red[8][33];
-    const uint32_t cx = threadIdx.x & 31u, gy = threadIdx.x >> 5;
-    const uint32_t c = blockIdx.x * 32 + cx;
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (c < cols)
-        for (uint64_t k = gy; k < nchunks; k += 64) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (k + 8 * j < nchunks) s[j] += part[(size_t)(k + 8 * j) * cols + c];
-        }
-    red[gy][cx] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
-    __syncthreads();
-    if (gy == 0 && c < cols) {
-        float t = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) t += red[w][cx];
-        out[c] = t;
-    }
+    const uint32_t cx = threadIdx.x & 31u;
+    fold_chunks_of_columns(blockIdx.x * 32 + cx, threadIdx.x >> 5, cx, cols, nchunks, part, out, red);
 }
 
 // ---- chains ----
@@ -796,21 +804,24 @@ int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, cons
 }
 
 int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* out) {
-    const uint32_t chunk = 256;
+    const uint32_t chunk = 256, groups = (cols + 31) / 32;
     const uint32_t nchunks = (rows + chunk - 1) / chunk;
-    dim3 grid((cols + 31) / 32, nchunks), block(32, 8);
+    dim3 grid(groups, nchunks), block(32, 8);
     if (nchunks == 1) {      // the only partial is the sum
-        fg_launch(ctx, colsum_partial_kernel, grid, block, 0, rows, cols, chunk, x, out);
+        fg_launch(ctx, colsum_kernel, grid, block, 0, rows, cols, chunk, x, out, (unsigned*)nullptr, (float*)nullptr);
         FG_LAUNCHED(ctx);
         return FG_OK;
     }
     void* part;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)nchunks * cols * sizeof(float), &part);
     if (s != FG_OK) return s;
-    fg_launch(ctx, colsum_partial_kernel, grid, block, 0, rows, cols, chunk, x, (float*)part);
+    const bool one = groups <= kFgArrivals;      // a counter for each group of columns
+    fg_launch(ctx, colsum_kernel, grid, block, 0, rows, cols, chunk, x, (float*)part, fg_arrivals(ctx), one ? out : (float*)nullptr);
     FG_LAUNCHED(ctx);
-    fg_launch(ctx, colsum_fold_kernel, (cols + 31) / 32, 256, 0, cols, nchunks, (const float*)part, out);
-    FG_LAUNCHED(ctx);
+    if (!one) {
+        fg_launch(ctx, colsum_fold_kernel, groups, 256, 0, cols, nchunks, (const float*)part, out);
+        FG_LAUNCHED(ctx);
+    }
     return FG_OK;
 }
 
@@ -853,9 +864,7 @@ int32_t fg_sum_f32(fg_ctx* ctx, const float* x, uint64_t n, float* out) {
     void* p;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &p);
     if (s != FG_OK) return s;
-    fg_launch(ctx, sum_partial_kernel, grid, 256, 0, x, n, (float*)p);
-    FG_LAUNCHED(ctx);
-    fg_launch(ctx, fold_partials_kernel, 1, 256, 0, (const float*)p, grid, out);
+    fg_launch(ctx, sum_kernel, grid, 256, 0, x, n, (float*)p, fg_arrivals(ctx), out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
@@ -879,14 +888,10 @@ int32_t fg_mse_loss_grad(fg_ctx* ctx, const float* pred, const float* target, ui
         partials = (float*)p;
     }
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (8.0 + (loss_elem_out ? 4.0 : 0.0) + (grad_out ? 4.0 : 0.0)) * n);
-    if (vec) fg_launch(ctx, loss_kernel<MseTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
-    else fg_launch(ctx, loss_kernel<MseTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
+    if (vec) fg_launch(ctx, loss_kernel<MseTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
+    else fg_launch(ctx, loss_kernel<MseTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
-    if (loss_sum_out) {
-        fg_launch(ctx, fold_partials_kernel, 1, 256, 0, partials, grid, loss_sum_out);
-        FG_LAUNCHED(ctx);
-    }
     return FG_OK;
 }
 
@@ -909,14 +914,10 @@ int32_t fg_bce_loss_grad(fg_ctx* ctx, const float* pred, const float* target, ui
         partials = (float*)p;
     }
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (8.0 + (loss_elem_out ? 4.0 : 0.0) + (grad_out ? 4.0 : 0.0)) * n);
-    if (vec) fg_launch(ctx, loss_kernel<BceTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
-    else fg_launch(ctx, loss_kernel<BceTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials);
+    if (vec) fg_launch(ctx, loss_kernel<BceTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
+    else fg_launch(ctx, loss_kernel<BceTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
-    if (loss_sum_out) {
-        fg_launch(ctx, fold_partials_kernel, 1, 256, 0, partials, grid, loss_sum_out);
-        FG_LAUNCHED(ctx);
-    }
     return FG_OK;
 }
 

@@ -161,6 +161,24 @@ inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, 
 }
 __device__ __forceinline__ void fg_grid_enter() { cudaGridDependencySynchronize(); }
 
+// Reductions over blocks without a second launch: every block leaves its part in memory and counts itself; the one that arrives
+// last sees all parts and adds them, in an order that does not depend on who it is.  The counters (behind the device error word)
+// start at zero and wrap back to it; the kernels of a context run one after the other, so one set serves all of them.
+// A launch of its own for the fold cost 2 - 2.5 us of a training step each.
+constexpr uint32_t kFgArrivals = 1024;
+inline unsigned* fg_arrivals(const fg_ctx* ctx) { return reinterpret_cast<unsigned*>(ctx->dev_status) + 64; }
+constexpr size_t kFgStatusBytes = 256 + kFgArrivals * sizeof(unsigned);
+// Called by all threads of a block after they have written their part; true in the block that is the last of `blocks`.
+__device__ __forceinline__ bool fg_last_block(unsigned* arrivals, unsigned blocks) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) last = atomicInc(arrivals, blocks - 1) == blocks - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
 // Brackets one kernel launch with events when timing is enabled (never while capturing).
 inline fg_time_rec* fg_time_begin(fg_ctx* ctx, int kind, double work) {
     if (!ctx->timing_on || ctx->capturing || !ctx->time_recs || ctx->time_count >= FG_TIME_MAX_RECS) return nullptr;
@@ -355,5 +373,10 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
                                  float* dB);
 int32_t fg_convert_launch(fg_ctx* ctx, const void* src, int src_dtype, void* dst, int dst_dtype, uint64_t n);
 int32_t fg_act_bwd_launch(fg_ctx* ctx, uint64_t n, int act, const float* dy, const float* saved, float* dz);
+// Which tensors' bf16 pairs the forward and backward products of [M,K] x [K,N] read when they exist: 1 A, 2 B, 4 dZ.
+uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K);
+// fg_ce_loss_grad with the sum of the losses; its arguments have been checked.
+int32_t fg_ce_loss_grad_sum(fg_ctx* ctx, const float* probs, const uint32_t* labels, uint32_t rows, uint32_t cols, float* loss_out,
+                            float* grad_out, float* loss_sum_out);
 int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* out);
 int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, float* out);

@@ -2855,6 +2855,29 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
     return FG_OK;
 }
 
+}  // namespace
+
+uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K) {
+    if (N <= 16) return 0;
+    float* const any = reinterpret_cast<float*>(uintptr_t(256));      // only the alignment counts, and that pairs are there
+    const PairedArg t{any, any, 0};
+    uint32_t bits = 0;
+    if (pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 2) {
+        const int ca = !in_place32(any, K, 1, 0), cb = !in_place32(any, N, 1, 0);
+        const Route r = pick_route(ctx, M, N, K, paired_shape_ok(ctx, M, N, K, K, N) && N % 4 == 0, 0.0, 0, (ca ? (double)M * K : 0.0) + (cb ? (double)K * N : 0.0),
+                                   ca + cb);
+        if (r.kind == kRoutePair) bits |= 1 | 2;
+    }
+    for (int want = 1; want < 4; ++want) {      // dB, dA or both
+        const BwdRoutes r = pick_bwd_routes(ctx, M, N, K, t, t, t, want & 1 ? any : nullptr, want & 2 ? any : nullptr, nullptr);
+        if ((want & 1) && !r.planes && r.dB.kind == kRoutePair) bits |= 1 | 4;
+        if ((want & 2) && !r.planes && r.dA.kind == kRoutePair) bits |= 2 | 4;
+    }
+    return bits;
+}
+
+namespace {
+
 // Backward of Y = act(A·B + bias) from dY: forms dZ = dY * act'(saved) first.
 int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_t K, const float* A, const float* B,
                       const float* dY, int32_t act, const float* saved, float* dA, float* dB, float* dbias,

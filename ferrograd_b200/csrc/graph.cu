@@ -436,7 +436,9 @@ int32_t lower(fg_exec* e) {
     e->pairs_version.assign(nin, 0);
     e->pairs_fresh.assign(nin, 0);
 
-    // ---- bf16 pairs of everything a matmul reads, and of the dZ a fused backward epilogue hands down ----
+    // ---- bf16 pairs of what a matmul reads them of, and of the dZ a fused backward epilogue hands down.  Narrow and small layers
+    // run without pairs; making them all the same was a launch per tensor (two of the twelve of a 2-16-2 training step).  A
+    // product that takes another route after an option was changed makes the pairs it misses. ----
     if (e->paired) {
         auto want_pairs = [&](int node) -> int32_t {
             ENode& en = e->n[node];
@@ -444,12 +446,14 @@ int32_t lower(fg_exec* e) {
         };
         for (GemmStep& gs : e->gemms) {
             if (gs.batch != 1) continue;
-            if ((s = want_pairs(gs.a)) != FG_OK || (s = want_pairs(gs.b)) != FG_OK) return s;
+            const uint32_t reads = fg_gemm_reads_pairs(e->ctx, gs.M, gs.N, gs.K);
+            if ((reads & 1 && (s = want_pairs(gs.a)) != FG_OK) || (reads & 2 && (s = want_pairs(gs.b)) != FG_OK)) return s;
         }
         for (GemmStep& gs : e->gemms) {
             if (gs.batch != 1) continue;
             const int h = e->n[gs.a].produced_by_gemm;
             if (h >= 0 && e->n[gs.a].consumers == 1 && e->gemms[h].batch == 1 && !e->gemms[h].dz_pairs &&
+                (fg_gemm_reads_pairs(e->ctx, e->gemms[h].M, e->gemms[h].N, e->gemms[h].K) & 4) &&
                 (s = fg_alloc(e->ctx, pstride(e, gs.a) * 4, &e->gemms[h].dz_pairs)) != FG_OK)
                 return s;
         }
@@ -705,9 +709,8 @@ static int32_t loss_eager(fg_exec* e, const fg_buf* target) {
     const uint32_t cols = o.dims.back();
     const uint32_t rows = (uint32_t)(o.numel / cols);
     FG_REQUIRE(e->ctx, target->bytes >= (uint64_t)rows * 4, "dispatch_loss: one u32 label per row is required");
-    const int32_t s = fg_ce_loss_grad(e->ctx, vptr(e, e->last), (const uint32_t*)target->ptr, rows, cols, (float*)e->loss_t->ptr,
-                                      (float*)e->seed->ptr);
-    return s != FG_OK ? s : fg_sum_f32(e->ctx, (const float*)e->loss_t->ptr, o.numel, lsum);
+    return fg_ce_loss_grad_sum(e->ctx, vptr(e, e->last), (const uint32_t*)target->ptr, rows, cols, (float*)e->loss_t->ptr,
+                               (float*)e->seed->ptr, lsum);
 }
 
 // The backward of one matmul in the graph's storage type.

@@ -736,18 +736,31 @@ __global__ void softmax_bwd_kernel(uint32_t rows, uint32_t cols, const float* __
     }
 }
 
-// The reference's unfused per-element CE on probabilities.
+// The reference's unfused per-element CE on probabilities; with `sum`, also the sum of the losses, through one partial per block.
 __global__ void ce_elem_kernel(const float* __restrict__ p, const uint32_t* __restrict__ labels, uint32_t rows,
-                               uint32_t cols, float* __restrict__ loss, float* __restrict__ grad) {
+                               uint32_t cols, float* __restrict__ loss, float* __restrict__ grad, float* partials, unsigned* arrivals,
+                               float* __restrict__ sum) {
     fg_grid_enter();
+    __shared__ float red[32];
+    float s = 0.0f;
     const uint64_t n = (uint64_t)rows * cols;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t r = (uint32_t)(i / cols), c = (uint32_t)(i - (uint64_t)r * cols);
         float pv = p[i];
         bool hit = labels[r] == c;
-        loss[i] = hit ? -logf(pv) : 0.0f;
+        const float l = hit ? -logf(pv) : 0.0f;
+        loss[i] = l;
         grad[i] = hit ? pv - 1.0f : pv;
+        s += l;
     }
+    if (!sum) return;
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (!fg_last_block(arrivals, gridDim.x)) return;
+    s = 0.0f;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) s += __ldcg(partials + i);
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) *sum = s;
 }
 
 // Fixed-order mean of the per-row losses (one CTA).
@@ -857,6 +870,19 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
 
 }  // namespace
 
+static int32_t ce_elem_launch(fg_ctx* ctx, const float* probs, const uint32_t* labels, uint32_t rows, uint32_t cols, float* loss_out,
+                              float* grad_out, float* loss_sum_out) {
+    const int grid = fg_stream_grid(ctx, (uint64_t)rows * cols, 256, 8);
+    void* part = nullptr;
+    if (loss_sum_out) {
+        const int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &part);
+        if (s != FG_OK) return s;
+    }
+    fg_launch(ctx, ce_elem_kernel, grid, 256, 0, probs, labels, rows, cols, loss_out, grad_out, (float*)part, fg_arrivals(ctx), loss_sum_out);
+    FG_LAUNCHED(ctx);
+    return FG_OK;
+}
+
 extern "C" {
 
 int32_t fg_softmax_fwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* y) {
@@ -949,10 +975,14 @@ int32_t fg_ce_loss_grad(fg_ctx* ctx, const float* probs, const uint32_t* labels,
     FG_REQUIRE(ctx, probs && labels && loss_out && grad_out, "fg_ce_loss_grad: NULL pointer");
     FG_REQUIRE(ctx, cols >= 1, "fg_ce_loss_grad: cols must be >= 1");
     if (rows == 0) return FG_OK;
-    int grid = fg_stream_grid(ctx, (uint64_t)rows * cols, 256, 8);
-    fg_launch(ctx, ce_elem_kernel, grid, 256, 0, probs, labels, rows, cols, loss_out, grad_out);
-    FG_LAUNCHED(ctx);
-    return FG_OK;
+    return ce_elem_launch(ctx, probs, labels, rows, cols, loss_out, grad_out, nullptr);
 }
 
 }  // extern "C"
+
+int32_t fg_ce_loss_grad_sum(fg_ctx* ctx, const float* probs, const uint32_t* labels, uint32_t rows, uint32_t cols, float* loss_out,
+                            float* grad_out, float* loss_sum_out) {
+    FG_ENTER(ctx);
+    if (rows == 0) return fg_sum_f32(ctx, loss_out, 0, loss_sum_out);
+    return ce_elem_launch(ctx, probs, labels, rows, cols, loss_out, grad_out, loss_sum_out);
+}

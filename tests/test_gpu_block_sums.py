@@ -1,0 +1,44 @@
+"""Sums that the last block to arrive adds up (loss sums, column sums): one block, a few, all of them; the counters serve the next
+call, of another size, as they did the first."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    yield c
+    c.sync()
+    c.destroy()
+
+
+def test_loss_sums(ctx):
+    r = np.random.Generator(np.random.Philox(3))
+    for n in (1, 255, 1025, 4096, 300007, 5, 2000003, 1024):
+        p, t = r.random(n, np.float32) * 0.8 + 0.1, r.random(n, np.float32)
+        pd, td, out, loss = ctx.init_tensor_f32((n,), p), ctx.init_tensor_f32((n,), t), ctx.new_tensor((1,)), ctx.new_tensor((n,))
+        for again in range(2):
+            ctx.mse_loss_grad(pd, td, n, loss_elem=loss, loss_sum=out)
+            want = ((p.astype(np.float64) - t) ** 2).sum()
+            # chains of at most 30 additions: 1e-5 is above 30 * 2^-24 and the roundings of the squares
+            assert abs(ctx.to_numpy(out)[0] - want) <= 1e-5 * want
+            ctx._check(ctx.lib.fg_sum_f32(ctx.handle, pd.ptr, n, out.ptr))
+            want = p.astype(np.float64).sum()
+            assert abs(ctx.to_numpy(out)[0] - want) <= 1e-5 * want
+
+
+@pytest.mark.parametrize("M,N", [(1, 20), (255, 33), (257, 32), (512, 31), (513, 1000), (5000, 10), (4096, 64), (300, 40000)])
+def test_column_sums(ctx, M, N):
+    r = np.random.Generator(np.random.Philox(M + N))
+    K = 4      # the exact path, whose bias gradient is a pass of its own
+    dY, A = r.standard_normal((M, N), np.float32), r.standard_normal((M, K), np.float32)
+    db, dB = ctx.new_tensor((N,)), ctx.new_tensor((K, N))
+    dyd, ad = ctx.init_tensor_f32((M, N), dY), ctx.init_tensor_f32((M, K), A)
+    for again in range(2):
+        ctx.gemm_bwd(ad, None, dyd, M, N, K, dB=dB, dbias=db, mode="simt")
+        want = dY.astype(np.float64).sum(0)
+        # chains of at most 32 + 8 additions of partial sums below 4 sqrt(M): far below 1e-5 sqrt(M)
+        assert np.abs(ctx.to_numpy(db) - want).max() <= 1e-5 * np.sqrt(M)
