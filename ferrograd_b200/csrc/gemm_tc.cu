@@ -1511,7 +1511,9 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         a = ep_of(p, [](const Epilogue& e) { return e.a_mn != 0; });
         b = ep_of(p, [](const Epilogue& e) { return e.b_mn != 0; });
     };
-    constexpr uint32_t kChunkKB = kChunkK / BK;
+    // Chunks of 128 k, half of the other kernels': fewer additions in the tensor core's truncating accumulator, as K-shares of that
+    // length had, and the epilogue warps have the time (a tile's drain takes a tenth of its four k-blocks).
+    constexpr uint32_t kChunkKB = 128 / BK;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(conv_bar(s), Cfg::kGroup / 32); mbar_init(empty_bar(s), 1); }
