@@ -1272,7 +1272,7 @@ int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 
 //   warp 0 loads, warp 1 issues MMAs, warps 4..11 drain accumulators and store, warps 12..27 convert.
 // Measured (start: operand planes or pairs, then a 256 x 256 or 128-row tile each; then with A in shared memory, eight converter
 // warps, K-shares folded by a second launch and one launch per product; now): 100 x 4096 x 4096 129 -> 35 -> 30 us,
-// 16 x (384 x 512 x 320) forward and backward 1530 -> 86 -> 51 us, the 200-256-256-10 step 195 -> 91 -> 74 us.
+// 16 x (384 x 512 x 320) forward and backward 1530 -> 86 -> 48 us, the 200-256-256-10 step 195 -> 91 -> 70 us.
 // Bound by shared-memory bandwidth: per k-block of 32 a 128 x 128 tile moves 32 KB in by TMA, 32 KB into the converters, 32 KB
 // out of them (B) and 32 KB into the MMAs (B): 1024 cycles at 128 B per cycle, 1040 measured (128 x 64: 640, 590 - 630 measured).
 // ------------------------------------------------------------------------------------
@@ -2082,8 +2082,8 @@ struct ConvPlan {
 };
 struct ConvShape { uint32_t M, N, K, batch; };
 template <int BN> int conv_clusters(const fg_ctx* ctx, uint32_t split);
-// Estimated SM cycles of one launch for one or two products (the one with the longer k first), from measured costs: per k-block
-// 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
+// Estimated SM cycles of one launch for one or two products (the one with the longer k first), from costs fitted to
+// whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
 // set-up and first loads, 2 - 3 us for the shares' sums to meet; 6 us more where a ragged N is stored element by element.
 ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n) {
     ConvPlan best{128, 1, 0.0};
