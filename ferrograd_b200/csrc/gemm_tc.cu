@@ -1431,6 +1431,9 @@ struct ConvStore {
         if (!vec)
             return epi_store_edge(z, off, col, ep.N, (char*)ep.C, (char*)ep.preact, ep.c_pairs, ep.c_pairs_stride, ep.mul_saved, ep.mul_act,
                                   ep.act, FG_DTYPE_F32);
+        return put_vec(ep, off, z);
+    }
+    __device__ __forceinline__ float4 put_vec(const Epilogue& ep, size_t off, float4 z) const {
         float4 o = z;
         if (kind == 1) {
             o = make_float4(fg_act_fwd_sel(act, z.x), fg_act_fwd_sel(act, z.y), fg_act_fwd_sel(act, z.z), fg_act_fwd_sel(act, z.w));
@@ -1721,6 +1724,27 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         // A 32 x 32 block of whole sums, swizzled in tb4 (float4 c of row r at c ^ (r & 7)): four rows of 128 bytes per step.
         auto store_block = [&](const Epilogue& ep, size_t cb, uint32_t row0, uint32_t col0, float bias) {
             const ConvStore st(ep, col0 + cc * 4);
+            if (!st.vec) {
+                // Rows that do not start on 16 bytes: a lane per column, a row of 128 bytes per step (four single words per lane
+                // and step, 16 bytes apart between lanes, took 11000 cycles for a 128 x 128 tile: backward of 1000 x 777 x 1001 51.0 -> 40.9 us).
+                const uint32_t c = col0 + lane, rows = c < ep.N && row0 < ep.M ? min(32u, ep.M - row0) : 0u;
+                const float* const tb = reinterpret_cast<const float*>(tb4);
+                size_t off = cb + (size_t)row0 * ep.N + c;
+                float cs = 0.0f;
+#pragma unroll 4
+                for (uint32_t r = 0; r < 32; ++r, off += ep.N) {
+                    if (r >= rows) continue;
+                    const float z = tb[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)] + bias;
+                    const float o = st.kind == 2 ? z * fg_act_grad_fast(st.act, ep.mul_saved[off]) : st.kind == 1 ? fg_act_fwd_sel(st.act, z) : z;
+                    if (ep.preact) ep.preact[off] = z;
+                    ep.C[off] = o;
+                    if (ep.c_pairs) fg_store_pairs1(ep.c_pairs, ep.c_pairs_stride, off, o);
+                    cs += o;
+                }
+                if (ep.colsum_part && rows) ep.colsum_part[(size_t)(row0 >> 5) * ep.N + c] = cs;
+                __syncwarp();
+                return;
+            }
             const float4 bz = make_float4(__shfl_sync(0xffffffffu, bias, cc * 4), __shfl_sync(0xffffffffu, bias, cc * 4 + 1),
                                           __shfl_sync(0xffffffffu, bias, cc * 4 + 2), __shfl_sync(0xffffffffu, bias, cc * 4 + 3));
             float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1737,7 +1761,7 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
             } else {
 #pragma unroll 2
                 for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
-                    if (i < rows) cs = add4(cs, st.put(ep, off, sum_at(i)));
+                    if (i < rows) cs = add4(cs, st.put_vec(ep, off, sum_at(i)));
             }
             __syncwarp();
             if (ep.colsum_part) {
@@ -2084,7 +2108,8 @@ struct ConvShape { uint32_t M, N, K, batch; };
 template <int BN> int conv_clusters(const fg_ctx* ctx, uint32_t split);
 // Estimated SM cycles of one launch for one or two products (the one with the longer k first), from costs fitted to
 // whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
-// set-up and first loads, 2 - 3 us for the shares' sums to meet; 6 us more where a ragged N is stored element by element.
+// set-up and first loads, 2 - 3 us for the shares' sums to meet; where a ragged N is stored word by word 1.5 us more, and 6 us
+// divided among the shares.
 ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n) {
     ConvPlan best{128, 1, 0.0};
     const uint64_t sms = (uint64_t)ctx->sm_count;
@@ -2097,7 +2122,8 @@ ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n) {
         }
         const uint64_t all = units[0] + units[1];
         const double kb = bn == 128 ? 1050.0 : 600.0, store = bn == 128 ? 5000.0 : 2800.0, around = 6500.0;
-        const double edge = sh[0].N % 4 != 0 || (n > 1 && sh[1].N % 4 != 0) ? (bn == 128 ? 11000.0 : 5500.0) : 0.0;
+        const bool ragged = sh[0].N % 4 != 0 || (n > 1 && sh[1].N % 4 != 0);
+        const double edge = ragged ? (bn == 128 ? 3000.0 : 1500.0) : 0.0;
         // whole units: the first CTA's units are one of every sms
         const uint64_t rounds = (all + sms - 1) / sms, rounds0 = units[0] / sms + (units[0] % sms != 0);
         auto unit = [&](int i) { return (double)nkb[i] * kb > store + edge ? (double)nkb[i] * kb : store + edge; };
@@ -2108,7 +2134,7 @@ ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n) {
             if (fit < 1) continue;
             const uint64_t turns = (all + fit - 1) / fit;
             const double share = (double)((nkb[0] + split - 1) / split) * kb;
-            c = (double)turns * (share + around + 5500.0 + edge / split);
+            c = (double)turns * (share + around + 5500.0 + (ragged ? (bn == 128 ? 11000.0 : 5500.0) / split : 0.0));
             if (c < best.cycles) best = ConvPlan{bn, split, c};
         }
     }
