@@ -2257,16 +2257,34 @@ int32_t launch_conv(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epi
     const ConvProduct pr{a, b, ep, batch};
     return launch_conv(ctx, &pr, 1, p);
 }
+// Does what `w` stores (C, and its pairs) lie over an operand of `r`?
+bool stores_over(const ConvProduct& w, const ConvProduct& r) {
+    auto meets = [](const void* p, uint64_t np, const void* q, uint64_t nq) {      // bytes from the first to behind the last element
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+        return p && q && a < b + nq && b < a + np;
+    };
+    const uint64_t mn = (uint64_t)w.ep.M * w.ep.N, c_bytes = ((uint64_t)(w.batch - 1) * w.ep.c_batch + mn) * 4;
+    const PlaneSet* const ops[2] = {&r.a, &r.b};
+    const uint32_t rows[2] = {r.ep.M, r.ep.N};
+    for (int i = 0; i < 2; ++i) {
+        const PlaneSet& o = *ops[i];
+        const uint64_t one = (uint64_t)(o.mn ? r.ep.K : rows[i]) * o.ld32, bytes = ((uint64_t)(r.batch - 1) * (o.batch32 ? o.batch32 : one) + one) * 4;
+        if (meets(w.ep.C, c_bytes, o.p32, bytes) || meets(w.ep.c_pairs, (w.ep.c_pairs_stride + mn) * 2, o.p32, bytes)) return true;
+    }
+    return false;
+}
 // The two gradients of a layer in one launch: more units to share out, and one wave's end instead of two.  The longer k goes
 // first, so that the short units fill the last round.  Two launches where each wants K-shares of its own (128 x 4096 x 1024: k of
-// 4096 on eight tiles and of 128 on 256 of them, 60 us together, 39 apart).
-int32_t launch_conv_both(fg_ctx* ctx, const ConvProduct& x, const ConvProduct& y) {
-    const ConvProduct pr[2] = {x.ep.K >= y.ep.K ? x : y, x.ep.K >= y.ep.K ? y : x};
+// 4096 on eight tiles and of 128 on 256 of them, 60 us together, 39 apart), and where dA lies over what dB reads (the gradient of
+// an activation may overwrite the activation): dB is then complete before dA is written, as on every other route.
+int32_t launch_conv_both(fg_ctx* ctx, const ConvProduct& dB, const ConvProduct& dA) {
+    const ConvProduct pr[2] = {dB.ep.K >= dA.ep.K ? dB : dA, dB.ep.K >= dA.ep.K ? dA : dB};
     const ConvShape sh[2] = {{pr[0].ep.M, pr[0].ep.N, pr[0].ep.K, pr[0].batch}, {pr[1].ep.M, pr[1].ep.N, pr[1].ep.K, pr[1].batch}};
     const ConvPlan together = plan_conv(ctx, sh, 2), one = plan_conv(ctx, sh, 1), two = plan_conv(ctx, sh + 1, 1);
-    if (together.cycles <= one.cycles + two.cycles) return launch_conv(ctx, pr, 2, together);
-    const int32_t s = launch_conv(ctx, pr, 1, one);
-    return s != FG_OK ? s : launch_conv(ctx, pr + 1, 1, two);
+    if (together.cycles <= one.cycles + two.cycles && !stores_over(dA, dB)) return launch_conv(ctx, pr, 2, together);
+    const bool b_first = dB.ep.K >= dA.ep.K;
+    const int32_t s = launch_conv(ctx, &dB, 1, b_first ? one : two);
+    return s != FG_OK ? s : launch_conv(ctx, &dA, 1, b_first ? two : one);
 }
 
 // A dense [R, C] f32 tensor (`batch` of them, x_batch apart) can be loaded as it lies when rows and matrices start on

@@ -187,7 +187,7 @@ int32_t fg_gemm_f32(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
  *   dB = Aᵀ·dZ  [K,N]   (skipped when dB == NULL)
  *   dbias = column sums of dZ [N] (skipped when NULL)
  *   dZ_out (NULL or [M,N]) receives dZ.
- * The ReLU mask is saved > 0 (the standard mask). */
+ * dB is complete before dA is written: dA may be A itself.  The ReLU mask is saved > 0 (the standard mask). */
 int32_t fg_gemm_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_t K,
                         const float* A, const float* B, const float* dY,
                         int32_t act, const float* saved,

@@ -151,6 +151,30 @@ def test_backward_onto_the_layer_below(ctx, oracle, M, N, K, shift_saved, shift_
     check(ctx.to_numpy(below), want.sum(0), TOL, "bias gradient of the layer below")
 
 
+# more samples than outputs and fewer (the longer k is dB's or dA's), more tiles than SMs, both gradients in a launch or one each
+@pytest.mark.parametrize("M,N,K", [(1024, 256, 256), (384, 256, 256), (128, 4096, 1024), (2048, 512, 1024), (64, 1024, 1024)])
+@pytest.mark.parametrize("how", ["gemm_bwd", "paired", "batched"])
+def test_gradient_that_overwrites_the_activation(ctx, oracle, M, N, K, how):
+    # dB is complete before dA is written, so dA may be A itself
+    T = 4 if how == "batched" else 1
+    r = rng(M + N + 3 * K)
+    A, B = np.tanh(r.standard_normal((T, M, K))).astype(np.float32), r.standard_normal((T, K, N), np.float32) * 0.1
+    dZ = r.standard_normal((T, M, N), np.float32)
+    dA = np.stack([oracle.gemm(z, b, transB=True, f64=True) for z, b in zip(dZ, B)])
+    dB = np.stack([oracle.gemm(a, z, transA=True, f64=True) for a, z in zip(A, dZ)])
+    Bd, Zd = up(ctx, B), up(ctx, dZ)
+    for again in range(3):
+        x, g = up(ctx, A), ctx.new_tensor((T, K, N))
+        if how == "gemm_bwd":
+            ctx.gemm_bwd(x, Bd, Zd, M, N, K, dA=x, dB=g)
+        elif how == "paired":
+            ctx.gemm_bwd_paired(x, Bd, Zd, M, N, K, dB=g, dA=x, below_act="tanh", below_saved=x)
+        else:
+            ctx.gemm_batched_bwd(x, Bd, Zd, T, M, N, K, dA=x, dB=g)
+        check(ctx.to_numpy(g), dB, TOL, "dB")
+        check(ctx.to_numpy(x), dA * (1.0 - A.astype(np.float64) ** 2) if how == "paired" else dA, TOL, "dA over A")
+
+
 def test_batched_refuses_what_one_product_refuses(ctx):
     # an unknown mode and a contraction over nothing: an argument error as from the per-matrix calls, before any launch
     from ferrograd_b200.backend import GEMM_MODE
