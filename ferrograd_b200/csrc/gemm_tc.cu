@@ -2874,6 +2874,17 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         return FG_OK;
     }
     const BwdRoutes rt = pick_bwd_routes(ctx, M, N, K, A, B, dZ, dB, dA, o.mul_saved);
+    if (dA && o.mul_saved && (rt.planes || rt.dA.kind == kRoutePlanes)) {
+        // There the factor is applied after the whole of dA has been written: where dA lies over the saved tensor, from a copy (in
+        // the room of the pairs, which this route does not make).
+        const uint64_t bytes = (uint64_t)M * K * 4;
+        const uintptr_t d = reinterpret_cast<uintptr_t>(dA), v = reinterpret_cast<uintptr_t>(o.mul_saved);
+        if (d < v + bytes && v < d + bytes) {
+            if ((s = fg_ws_alloc(ctx, bytes, &p)) != FG_OK) return s;
+            FG_CUDA(ctx, FG_ERR_FAILED_BUFFER_COPY, cudaMemcpyAsync(p, o.mul_saved, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+            o.mul_saved = (const float*)p;
+        }
+    }
     if (!rt.planes && (dA || dB)) {
         PairedOut po = o;
         po.colsum_part = cs_part;

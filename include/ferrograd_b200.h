@@ -239,7 +239,7 @@ int32_t fg_gemm_paired_f32(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K,
  * where below_act / below_saved describe the layer BELOW (the one whose output A is; FG_ACT_NONE: no
  * factor), so dA is that layer's dZ, ready to be passed to its own backward call.  dA_pairs_out (may be
  * NULL) receives dA's pairs and below_dbias (may be NULL, [K]) its column sums, the bias gradient of the
- * layer below -- all from the dA epilogue.  Any of the input pairs may be NULL. */
+ * layer below -- all from the dA epilogue.  Any of the input pairs may be NULL.  dA may be A or below_saved itself. */
 int32_t fg_gemm_bwd_paired_f32(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K,
                                const float* A, const void* A_pairs, uint64_t A_stride,
                                const float* B, const void* B_pairs, uint64_t B_stride,

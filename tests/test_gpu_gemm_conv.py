@@ -175,6 +175,27 @@ def test_gradient_that_overwrites_the_activation(ctx, oracle, M, N, K, how):
         check(ctx.to_numpy(x), dA * (1.0 - A.astype(np.float64) ** 2) if how == "paired" else dA, TOL, "dA over A")
 
 
+# the exact path, a narrow layer, operand planes (one gradient or both), the pair kernel
+@pytest.mark.parametrize("M,N,K", [(33, 20, 40), (200, 10, 512), (300, 33, 75), (64, 700, 1021), (2048, 64, 4094), (1024, 1024, 2048)])
+@pytest.mark.parametrize("pairs", ["1", "0"])
+def test_gradient_that_overwrites_the_saved_tensor(oracle, M, N, K, pairs):
+    # dA = (dZ B^T) * act'(saved) may lie over the saved tensor, which is A, on every route
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    c.set_option("gemm_pairs", pairs)
+    r = rng(M + N + 5 * K)
+    A, B = np.tanh(r.standard_normal((M, K))).astype(np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    dZ = r.standard_normal((M, N), np.float32)
+    x, dB, below = up(c, A), c.new_tensor((K, N)), c.new_tensor((K,))
+    c.gemm_bwd_paired(x, up(c, B), up(c, dZ), M, N, K, dB=dB, dA=x, below_act="tanh", below_saved=x, below_dbias=below)
+    want = oracle.gemm(dZ, B, transB=True, f64=True) * (1.0 - A.astype(np.float64) ** 2)
+    check(c.to_numpy(x), want, TOL, "dA over A")
+    check(c.to_numpy(dB), oracle.gemm(A, dZ, transA=True, f64=True), TOL, "dB")
+    check(c.to_numpy(below), want.sum(0), TOL, "bias gradient of the layer below")
+    assert c.device_status() == 0
+    c.destroy()
+
+
 def test_batched_refuses_what_one_product_refuses(ctx):
     # an unknown mode and a contraction over nothing: an argument error as from the per-matrix calls, before any launch
     from ferrograd_b200.backend import GEMM_MODE
