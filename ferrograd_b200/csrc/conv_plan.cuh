@@ -1,0 +1,60 @@
+// How the conversion kernel's work is split over the SMs: host arithmetic on sizes and counts alone, free of CUDA, so that it can be
+// compiled and checked without a device.
+#pragma once
+#include <stdint.h>
+
+constexpr uint32_t kConvTileM = 128;
+struct ConvShape { uint32_t M, N, K, batch; };
+struct ConvPlan {
+    uint32_t bn, split;      // tile width; K-shares of a tile
+    double cycles;           // estimate; 0: cannot run
+};
+
+// SMs that a kernel whose CTAs stay to its end may count on: while a gradient exchange runs beside it, `reserved` are the
+// exchange's (see fg_comm_init).
+inline uint64_t fg_sms_beside(int sms, bool exchange, int reserved) { return (uint64_t)(exchange && reserved > 0 && reserved < sms ? sms - reserved : sms); }
+
+// CTAs of a launch: one for each K-share, or no more than SMs that walk the units.
+inline uint64_t conv_grid(uint64_t units, uint32_t split, uint64_t sms) { return split > 1 ? units * split : units < sms ? units : sms; }
+
+// Estimated SM cycles of one launch for one or two products (the one with the longer k first) on `sms` SMs, from costs fitted to
+// whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
+// set-up and first loads, 2 - 3 us for the shares' sums to meet; where a ragged N is stored word by word 1.5 us more, and 6 us
+// divided among the shares.  clusters(bn, split): clusters of `split` CTAs that run at once, below one if there are none.
+template <class Clusters>
+ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters) {
+    ConvPlan best{128, 1, 0.0};
+    for (uint32_t bn = 128; bn >= 64; bn -= 64) {
+        uint64_t units[2] = {0, 0}, nkb[2] = {0, 0}, min_kb = ~0ull;
+        for (int i = 0; i < n; ++i) {
+            units[i] = (uint64_t)((sh[i].M + kConvTileM - 1) / kConvTileM) * ((sh[i].N + bn - 1) / bn) * sh[i].batch;
+            nkb[i] = (sh[i].K + 31) / 32;
+            if (nkb[i] < min_kb) min_kb = nkb[i];
+        }
+        const uint64_t all = units[0] + units[1];
+        const double kb = bn == 128 ? 1050.0 : 600.0, store = bn == 128 ? 5000.0 : 2800.0, around = 6500.0;
+        const bool ragged = sh[0].N % 4 != 0 || (n > 1 && sh[1].N % 4 != 0);
+        const double edge = ragged ? (bn == 128 ? 3000.0 : 1500.0) : 0.0;
+        // whole units: the first CTA's units are one of every sms
+        const uint64_t rounds = (all + sms - 1) / sms, rounds0 = units[0] / sms + (units[0] % sms != 0);
+        auto unit = [&](int i) { return (double)nkb[i] * kb > store + edge ? (double)nkb[i] * kb : store + edge; };
+        double c = around + store + edge + (double)rounds0 * unit(0) + (double)(rounds - rounds0) * unit(1);
+        if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, 1, c};
+        for (uint32_t split = 2; split <= 8 && split * 2 <= min_kb && all * split <= 2 * sms; ++split) {
+            const int fit = clusters(bn, split);
+            if (fit < 1) continue;
+            const uint64_t turns = (all + fit - 1) / fit;
+            const double share = (double)((nkb[0] + split - 1) / split) * kb;
+            c = (double)turns * (share + around + 5500.0 + (ragged ? (bn == 128 ? 11000.0 : 5500.0) / split : 0.0));
+            if (c < best.cycles) best = ConvPlan{bn, split, c};
+        }
+    }
+    return best;
+}
+
+// Of `fit` clusters that run at once on `all` SMs, those that do on `sms` of them: the exchange's CTAs may sit anywhere.
+inline int conv_clusters_beside(int fit, uint64_t sms, uint64_t all) {
+    if (fit < 1 || sms >= all) return fit;
+    const int n = (int)((uint64_t)fit * sms / all);
+    return n < 1 ? 1 : n;
+}

@@ -607,10 +607,10 @@ int32_t fg_comm_init(fg_ctx* ctx, int32_t nranks, int32_t rank, const uint8_t id
     if (!ctx->nccl_lib) return fg_fail(ctx, FG_ERR_UNSUPPORTED_FEATURE, "fg_comm_init: libnccl.so.2 not found");
     auto init = (pfn_ncclCommInitRank)dlsym(ctx->nccl_lib, "ncclCommInitRank");
     if (!init) return fg_fail(ctx, FG_ERR_UNSUPPORTED_FEATURE, "fg_comm_init: ncclCommInitRank missing");
-    // An exchange CTA and a GEMM CTA cannot share an SM (registers, shared memory), and the pair GEMM is
-    // persistent: if it took every SM the exchange would start only when it ended, and if the exchange
+    // An exchange CTA and a GEMM CTA cannot share an SM (registers, shared memory), and the pair GEMM and the conversion
+    // kernel are persistent: if one took every SM the exchange would start only when it ended, and if the exchange
     // took some first the GEMM's last CTAs would start late with a full share of tiles.  So the exchange
-    // is held to 12 CTAs (unless the caller's environment says otherwise) and the GEMM leaves 16 SMs free
+    // is held to 12 CTAs (unless the caller's environment says otherwise) and they leave 16 SMs free
     // while one is in flight (options comm_max_ctas and comm_sms; comm_sms 0 turns the reservation off).  Measured on
     // two GPUs (config-4 step, ms): 12 CTAs / 16 SMs 2.04, 8 / 12 2.03-2.07, 16 / 20 2.12, 4 / 8 2.42
     // (exchange-bound), no reservation 2.15-2.18; one GPU alone 1.96-2.00.

@@ -10,6 +10,7 @@
 #include <utility>
 
 #include "../../include/ferrograd_b200.h"
+#include "conv_plan.cuh"
 
 // Device error word bits, set by kernels whose bounded waits ran out.
 #define FG_DEVERR_TMA_WAIT 1
@@ -48,7 +49,7 @@ struct fg_ctx {
     cudaEvent_t ev_fork, ev_join;
     bool comm_pending;
     cudaEvent_t ev_ckpt[8];             // exchange checkpoints (fg_comm_checkpoint / fg_comm_wait)
-    int comm_reserved_sms;              // SMs the persistent GEMM leaves free while an exchange is in flight
+    int comm_reserved_sms;              // SMs the persistent GEMMs leave free while an exchange is in flight
     cudaStream_t copy_stream;           // host->device prefetches that overlap compute
     cudaEvent_t ev_copy_done, ev_main_mark;
     bool mark_valid;
@@ -204,6 +205,9 @@ int32_t fg_ws_alloc(fg_ctx* ctx, uint64_t bytes, void** out);
 // Room for `bytes` more in the arena (grows it when nothing has been carved yet for this operation).
 int32_t fg_ws_ensure(fg_ctx* ctx, uint64_t bytes);
 bool fg_ws_try(fg_ctx* ctx, uint64_t bytes);      // the same, but a failure changes nothing and is no error
+
+// SMs for a kernel whose CTAs take one each and stay to its end.
+inline uint64_t fg_free_sms(const fg_ctx* ctx) { return fg_sms_beside(ctx->sm_count, ctx->comm_pending, ctx->comm_reserved_sms); }
 
 // Grid for a bandwidth-bound grid-stride kernel: a multiple of the SM count.
 inline int fg_stream_grid(const fg_ctx* ctx, uint64_t work_items, int threads, int per_sm) {

@@ -34,6 +34,7 @@ using namespace fgptx;
 namespace {
 
 constexpr int BM = 128;         // rows of the output tile = UMMA M
+static_assert(BM == (int)kConvTileM, "the plan's tiles");
 // BK (template parameter): f32 per k-block = one swizzled shared-memory row: 32 (128-byte swizzle) or 16 (64-byte).
 constexpr int UK = 8;           // K of one tcgen05.mma kind::tf32
 constexpr long long kWaitCycles = 2000000000LL;   // bound on every device-side wait (about 1 s)
@@ -2061,11 +2062,7 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
         max_clusters[ctx->device & 63].store(n, std::memory_order_release);
     }
     uint64_t slots = (uint64_t)max_clusters[ctx->device & 63].load(std::memory_order_acquire);
-    if (ctx->comm_pending && ctx->comm_reserved_sms > 0) {
-        // leave room for the gradient exchange that runs beside this GEMM (see fg_comm_init)
-        const uint64_t lim = (uint64_t)(ctx->sm_count - ctx->comm_reserved_sms) / 2;
-        if (lim >= 1 && lim < slots) slots = lim;
-    }
+    if (fg_free_sms(ctx) / 2 < slots) slots = fg_free_sms(ctx) / 2;      // room for the gradient exchange that runs beside this GEMM
     // The last wave: `rem` tiles for `slots` pairs.  When at least two pairs are free per tile, each tail
     // tile is cut into K-shares (whole accumulation chunks, at least two per share) so that the wave
     // lasts a fraction of a tile time; the shares are folded by a second, bandwidth-bound kernel.
@@ -2100,49 +2097,16 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
 }
 
 // ---- conversion kernel, host side ----
-struct ConvPlan {
-    uint32_t bn, split;
-    double cycles;       // estimate; 0: cannot run
-};
-struct ConvShape { uint32_t M, N, K, batch; };
 template <int BN> int conv_clusters(const fg_ctx* ctx, uint32_t split);
-// Estimated SM cycles of one launch for one or two products (the one with the longer k first), from costs fitted to
-// whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
-// set-up and first loads, 2 - 3 us for the shares' sums to meet; where a ragged N is stored word by word 1.5 us more, and 6 us
-// divided among the shares.
-ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n) {
-    ConvPlan best{128, 1, 0.0};
-    const uint64_t sms = (uint64_t)ctx->sm_count;
-    for (uint32_t bn = 128; bn >= 64; bn -= 64) {
-        uint64_t units[2] = {0, 0}, nkb[2] = {0, 0}, min_kb = ~0ull;
-        for (int i = 0; i < n; ++i) {
-            units[i] = (uint64_t)((sh[i].M + BM - 1) / BM) * ((sh[i].N + bn - 1) / bn) * sh[i].batch;
-            nkb[i] = (sh[i].K + 31) / 32;
-            if (nkb[i] < min_kb) min_kb = nkb[i];
-        }
-        const uint64_t all = units[0] + units[1];
-        const double kb = bn == 128 ? 1050.0 : 600.0, store = bn == 128 ? 5000.0 : 2800.0, around = 6500.0;
-        const bool ragged = sh[0].N % 4 != 0 || (n > 1 && sh[1].N % 4 != 0);
-        const double edge = ragged ? (bn == 128 ? 3000.0 : 1500.0) : 0.0;
-        // whole units: the first CTA's units are one of every sms
-        const uint64_t rounds = (all + sms - 1) / sms, rounds0 = units[0] / sms + (units[0] % sms != 0);
-        auto unit = [&](int i) { return (double)nkb[i] * kb > store + edge ? (double)nkb[i] * kb : store + edge; };
-        double c = around + store + edge + (double)rounds0 * unit(0) + (double)(rounds - rounds0) * unit(1);
-        if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, 1, c};
-        for (uint32_t split = 2; split <= 8 && split * 2 <= min_kb && all * split <= 2 * sms; ++split) {
-            const int fit = bn == 128 ? conv_clusters<128>(ctx, split) : conv_clusters<64>(ctx, split);
-            if (fit < 1) continue;
-            const uint64_t turns = (all + fit - 1) / fit;
-            const double share = (double)((nkb[0] + split - 1) / split) * kb;
-            c = (double)turns * (share + around + 5500.0 + (ragged ? (bn == 128 ? 11000.0 : 5500.0) / split : 0.0));
-            if (c < best.cycles) best = ConvPlan{bn, split, c};
-        }
-    }
-    return best;
+ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n, uint64_t sms) {
+    return conv_plan(sh, n, sms, [&](uint32_t bn, uint32_t split) {
+        return conv_clusters_beside(bn == 128 ? conv_clusters<128>(ctx, split) : conv_clusters<64>(ctx, split), sms, (uint64_t)ctx->sm_count);
+    });
 }
+// One product with the whole GPU: what the choice of a kernel goes by, which does not depend on a running exchange.
 ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32_t batch) {
     const ConvShape sh{M, N, K, batch};
-    return plan_conv(ctx, &sh, 1);
+    return plan_conv(ctx, &sh, 1, (uint64_t)ctx->sm_count);
 }
 // The pair kernel for one matrix: 256 x 256 tiles on SM pairs, plus the passes that make the pairs of `prep` elements.
 double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double prep_elems, int prep_launches) {
@@ -2234,8 +2198,7 @@ int32_t launch_conv_bn(fg_ctx* ctx, const ConvProduct* pr, int n, uint32_t split
     ca.units = (uint32_t)units;
     ca.split = split;
     ca.dev_status = ctx->dev_status;
-    const uint64_t sms = (uint64_t)ctx->sm_count;
-    const uint32_t grid = (uint32_t)(split > 1 ? units * split : units < sms ? units : sms);
+    const uint32_t grid = (uint32_t)conv_grid(units, split, fg_free_sms(ctx));
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, flop);
     auto launch = [&](auto two, auto shares) -> int32_t {
         constexpr bool T = decltype(two)::value, S = decltype(shares)::value;
@@ -2250,7 +2213,13 @@ int32_t launch_conv_bn(fg_ctx* ctx, const ConvProduct* pr, int n, uint32_t split
     fg_time_end(ctx, tr);
     return s;
 }
-int32_t launch_conv(fg_ctx* ctx, const ConvProduct* pr, int n, const ConvPlan& p) {
+inline ConvShape conv_shape(const ConvProduct& c) { return ConvShape{c.ep.M, c.ep.N, c.ep.K, c.batch}; }
+int32_t launch_conv(fg_ctx* ctx, const ConvProduct* pr, int n, ConvPlan p) {
+    // beside an exchange the units are split for the SMs that it leaves (n = 2 comes from launch_conv_both, which has done so)
+    if (n == 1 && fg_free_sms(ctx) != (uint64_t)ctx->sm_count) {
+        const ConvShape sh = conv_shape(pr[0]);
+        p = plan_conv(ctx, &sh, 1, fg_free_sms(ctx));
+    }
     return p.bn == 128 ? launch_conv_bn<128>(ctx, pr, n, p.split) : launch_conv_bn<64>(ctx, pr, n, p.split);
 }
 int32_t launch_conv(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilogue& ep, const ConvPlan& p, uint32_t batch) {
@@ -2279,8 +2248,9 @@ bool stores_over(const ConvProduct& w, const ConvProduct& r) {
 // an activation may overwrite the activation): dB is then complete before dA is written, as on every other route.
 int32_t launch_conv_both(fg_ctx* ctx, const ConvProduct& dB, const ConvProduct& dA) {
     const ConvProduct pr[2] = {dB.ep.K >= dA.ep.K ? dB : dA, dB.ep.K >= dA.ep.K ? dA : dB};
-    const ConvShape sh[2] = {{pr[0].ep.M, pr[0].ep.N, pr[0].ep.K, pr[0].batch}, {pr[1].ep.M, pr[1].ep.N, pr[1].ep.K, pr[1].batch}};
-    const ConvPlan together = plan_conv(ctx, sh, 2), one = plan_conv(ctx, sh, 1), two = plan_conv(ctx, sh + 1, 1);
+    const ConvShape sh[2] = {conv_shape(pr[0]), conv_shape(pr[1])};
+    const uint64_t sms = fg_free_sms(ctx);
+    const ConvPlan together = plan_conv(ctx, sh, 2, sms), one = plan_conv(ctx, sh, 1, sms), two = plan_conv(ctx, sh + 1, 1, sms);
     if (together.cycles <= one.cycles + two.cycles && !stores_over(dA, dB)) return launch_conv(ctx, pr, 2, together);
     const bool b_first = dB.ep.K >= dA.ep.K;
     const int32_t s = launch_conv(ctx, &dB, 1, b_first ? one : two);

@@ -102,7 +102,7 @@ uint64_t fg_ctx_workspace_bytes(fg_ctx* ctx);
  *                   layers plain launches keep the GPU fed, and four graph launches per step cost more than
  *                   they save (measured: 1.87 against 1.82 ms per step on 784-4096-4096-10 on one GPU)
  *   "comm_max_ctas" CTAs the communicator may use (default 12; read by fg_comm_init)
- *   "comm_sms"      SMs the persistent GEMM leaves free while an exchange is in flight (default 16; 0 = none)
+ *   "comm_sms"      SMs the persistent GEMMs leave free while an exchange is in flight (default 16; 0 = none)
  *   "comm_min_exchange"  the graph engine starts a gradient exchange during the backward pass once this many
  *                   elements are complete (default 1048576); smaller ranges wait for the next one
  * The environment variables FG_GEMM_TILE, FG_GEMM_NO_SPLITK, FG_GEMM_NO_PAIRS, FG_EXEC_NO_PLANS,

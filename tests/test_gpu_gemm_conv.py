@@ -196,6 +196,35 @@ def test_gradient_that_overwrites_the_saved_tensor(oracle, M, N, K, pairs):
     c.destroy()
 
 
+@pytest.mark.parametrize("T,M,N,K", [(1, 384, 256, 256), (1, 100, 1024, 2048), (9, 384, 512, 320), (1, 1000, 777, 1001)])
+def test_products_beside_an_exchange(oracle, T, M, N, K):
+    # a communicator of one rank: launches in plain order, units walked by the SMs that the exchange leaves
+    import torch  # noqa: F401  (its NCCL is the one that the process loads)
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    c.comm_init(1, 0, c.comm_unique_id())
+    r = rng(T + M + N + K)
+    A, B, dY = (r.standard_normal(s, np.float32) for s in ((T, M, K), (T, K, N), (T, M, N)))
+    B *= 0.1
+    out, dA, dB, sums = c.new_tensor((T, M, N)), c.new_tensor((T, M, K)), c.new_tensor((T, K, N)), up(c, np.arange(4096.0))
+    Ad, Bd, Yd = up(c, A), up(c, B), up(c, dY)
+    c.allreduce_sum(sums, 4096)             # in flight until it is joined
+    if T > 1:
+        c.gemm_batched(Ad, Bd, out, T, M, N, K)
+        c.gemm_batched_bwd(Ad, Bd, Yd, T, M, N, K, dA=dA, dB=dB)
+    else:
+        c.gemm(Ad, Bd, out, M, N, K)
+        c.gemm_bwd(Ad, Bd, Yd, M, N, K, dA=dA, dB=dB)
+    c.comm_sync(20000)
+    got, gA, gB = (c.to_numpy(t) for t in (out, dA, dB))
+    for t in range(T):
+        check(got[t], oracle.gemm(A[t], B[t], f64=True), TOL, f"output {t}")
+        check(gA[t], oracle.gemm(dY[t], B[t], transB=True, f64=True), TOL, f"dA {t}")
+        check(gB[t], oracle.gemm(A[t], dY[t], transA=True, f64=True), TOL, f"dB {t}")
+    assert (c.to_numpy(sums) == np.arange(4096.0)).all() and c.device_status() == 0
+    c.destroy()
+
+
 def test_batched_refuses_what_one_product_refuses(ctx):
     # an unknown mode and a contraction over nothing: an argument error as from the per-matrix calls, before any launch
     from ferrograd_b200.backend import GEMM_MODE
