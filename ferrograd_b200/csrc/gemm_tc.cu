@@ -1731,7 +1731,7 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                 const uint32_t c = col0 + lane, rows = c < ep.N && row0 < ep.M ? min(32u, ep.M - row0) : 0u;
                 const float* const tb = reinterpret_cast<const float*>(tb4);
                 size_t off = cb + (size_t)row0 * ep.N + c;
-                float cs = 0.0f;
+                float cs[4] = {0.f, 0.f, 0.f, 0.f};      // row r in chain r % 4, as the lanes below have it
 #pragma unroll 4
                 for (uint32_t r = 0; r < 32; ++r, off += ep.N) {
                     if (r >= rows) continue;
@@ -1740,9 +1740,9 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                     if (ep.preact) ep.preact[off] = z;
                     ep.C[off] = o;
                     if (ep.c_pairs) fg_store_pairs1(ep.c_pairs, ep.c_pairs_stride, off, o);
-                    cs += o;
+                    cs[r & 3] += o;
                 }
-                if (ep.colsum_part && rows) ep.colsum_part[(size_t)(row0 >> 5) * ep.N + c] = cs;
+                if (ep.colsum_part && rows) ep.colsum_part[(size_t)(row0 >> 5) * ep.N + c] = (cs[0] + cs[1]) + (cs[2] + cs[3]);
                 __syncwarp();
                 return;
             }

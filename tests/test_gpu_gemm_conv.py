@@ -256,6 +256,26 @@ def test_bias_gradient_of_many_samples(ctx, M, N, K):
     assert np.mean(errors) <= 2.3e-7, errors
 
 
+@pytest.mark.parametrize("M", [96, 90, 97])
+@pytest.mark.parametrize("K", [2044, 2045])
+def test_fused_column_sums_in_four_chains(ctx, M, K):
+    # Rows on the 16-byte boundary or off it: the same sums, bit for bit.  A block of 32 rows is added in four chains of eight (row
+    # r in chain r % 4), which are added in pairs; then the blocks in order.  (N below 64: one k-block or two, no K-shares.)
+    N = 24
+    r = rng(M + K)
+    B, dZ = r.standard_normal((K, N), np.float32), r.standard_normal((M, N), np.float32)
+    dA, below = ctx.new_tensor((M, K)), ctx.new_tensor((K,))
+    ctx.gemm_bwd_paired(None, up(ctx, B), up(ctx, dZ), M, N, K, dA=dA, below_dbias=below)
+    got = ctx.to_numpy(dA)
+    want = np.zeros(K, np.float32)
+    for m in range(0, M, 32):
+        chains = np.zeros((4, K), np.float32)
+        for i, row in enumerate(got[m:m + 32]):
+            chains[i % 4] += row
+        want += (chains[0] + chains[1]) + (chains[2] + chains[3])
+    assert np.array_equal(ctx.to_numpy(below), want)
+
+
 @pytest.mark.parametrize("M,N,K", [(96, 2048, 2048), (128, 1024, 4096), (128, 4096, 1024), (4096, 64, 4096), (16384, 32, 1024), (300, 100, 304)])
 @pytest.mark.parametrize("paired", [False, True])
 def test_backward_keeps_the_error_of_the_planes(ctx, oracle, M, N, K, paired):
