@@ -1,6 +1,7 @@
 // How the conversion kernel's work is split over the SMs: host arithmetic on sizes and counts alone, free of CUDA, so that it can be
 // compiled and checked without a device.
 #pragma once
+#include <atomic>
 #include <stdint.h>
 
 constexpr uint32_t kConvTileM = 128;
@@ -57,4 +58,16 @@ inline int conv_clusters_beside(int fit, uint64_t sms, uint64_t all) {
     if (fit < 1 || sms >= all) return fit;
     const int n = (int)((uint64_t)fit * sms / all);
     return n < 1 ? 1 : n;
+}
+
+// A property of the device: asked until an answer has been given (query(&value) is true then, whatever the value), kept from then on.
+// `known` starts at zero and holds the value plus one.  A query that fails says nothing about the device: `fallback` for this call.
+template <class Query>
+int fg_asked_once(std::atomic<int>& known, int fallback, Query query) {
+    const int k = known.load(std::memory_order_acquire);
+    if (k > 0) return k - 1;
+    int n = 0;
+    if (!query(&n) || n < 0) return fallback;
+    known.store(n + 1, std::memory_order_release);      // the same value whoever asks
+    return n;
 }

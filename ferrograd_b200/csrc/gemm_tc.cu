@@ -1991,6 +1991,23 @@ int32_t launch_tc(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilo
 // Scratch the pair kernel's split-K tail may need: at most one 256x256 f32 slot per resident pair.
 constexpr uint64_t kPairPartialBytes = 80ull * (2 * BM) * 256 * 4 + 256;
 
+// How many clusters of `size` CTAs run at once; false if the runtime does not say (its error is taken off the context's thread).
+template <typename Kernel>
+bool cluster_query(int* n, Kernel kernel, unsigned grid, unsigned threads, size_t smem, unsigned size) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(n, kernel, &cfg) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 template <int BK, int FMT>
 int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilogue& ep_in) {
     Epilogue ep = ep_in;
@@ -2043,25 +2060,10 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     ep.group = ctx->opt_tile_group > 0 ? (uint32_t)ctx->opt_tile_group : (ep.K <= 2048 ? 16u : 8u);
     // persistent: one CTA pair per SM pair, each walking tiles pair, pair + P, ...
     // How many pairs can be resident at once is asked of the runtime (not every SM need be pairable).
-    static std::atomic<int> max_clusters[64];       // zero-initialised; the same value whoever computes it
-    if (max_clusters[ctx->device & 63].load(std::memory_order_acquire) == 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)ctx->sm_count & ~1u);
-        cfg.blockDim = dim3(kPairThreads);
-        cfg.dynamicSmemBytes = Cfg::kSmemBytes;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<BK, FMT>, &cfg) != cudaSuccess || n < 1) {
-            cudaGetLastError();
-            n = ctx->sm_count / 2;
-        }
-        max_clusters[ctx->device & 63].store(n, std::memory_order_release);
-    }
-    uint64_t slots = (uint64_t)max_clusters[ctx->device & 63].load(std::memory_order_acquire);
+    static std::atomic<int> max_clusters[64];       // zero-initialised
+    uint64_t slots = (uint64_t)fg_asked_once(max_clusters[ctx->device & 63], ctx->sm_count / 2, [&](int* n) {
+        return cluster_query(n, gemm_tc_pair_kernel<BK, FMT>, (unsigned)ctx->sm_count & ~1u, kPairThreads, Cfg::kSmemBytes, 2) && *n >= 1;
+    });
     if (fg_free_sms(ctx) / 2 < slots) slots = fg_free_sms(ctx) / 2;      // room for the gradient exchange that runs beside this GEMM
     // The last wave: `rem` tiles for `slots` pairs.  When at least two pairs are free per tile, each tail
     // tile is cut into K-shares (whole accumulation chunks, at least two per share) so that the wave
@@ -2137,26 +2139,11 @@ cudaError_t conv_attr(const fg_ctx* ctx) {
 // documented); 0 if they cannot be launched.
 template <int BN>
 int conv_clusters(const fg_ctx* ctx, uint32_t split) {
-    static std::atomic<int> known[64][9];       // zero-initialised; the same value whoever computes it, stored plus one
-    std::atomic<int>& k = known[ctx->device & 63][split];
-    int n = k.load(std::memory_order_acquire) - 1;
-    if (n >= 0) return n;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(split * 64);
-    cfg.blockDim = dim3(ConvCfg<BN>::kThreads);
-    cfg.dynamicSmemBytes = ConvCfg<BN>::kSmemBytes;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = split; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (conv_attr<BN, false, true>(ctx) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, gemm_tc_conv_kernel<BN, false, true>, &cfg) != cudaSuccess || n < 0) {
-        cudaGetLastError();
-        n = 0;
-    }
-    k.store(n + 1, std::memory_order_release);
-    return n;
+    static std::atomic<int> known[64][9];       // zero-initialised
+    return fg_asked_once(known[ctx->device & 63][split], 0, [&](int* n) {
+        if (conv_attr<BN, false, true>(ctx) != cudaSuccess) { cudaGetLastError(); return false; }
+        return cluster_query(n, gemm_tc_conv_kernel<BN, false, true>, split * 64, ConvCfg<BN>::kThreads, ConvCfg<BN>::kSmemBytes, split);
+    });
 }
 
 // One product of a launch: its operands, their roles and the epilogue.

@@ -18,6 +18,10 @@ double plan(uint32_t M, uint32_t N, uint32_t K, uint32_t batch, uint32_t N2, uin
     *bn = p.bn; *split = p.split;
     return p.cycles;
 }
+std::atomic<int> known[2];
+int asked_once(int which, int answers, int value, int* asked) {
+    return fg_asked_once(known[which], -7, [&](int* n) { ++*asked; *n = value; return answers != 0; });
+}
 }
 """
 
@@ -75,3 +79,13 @@ def test_every_shape_has_a_plan(shim, sms):
                         shortest = min(K, second[1]) if second[0] else K
                         assert bn in (64, 128) and cycles > 0
                         assert split == 1 or 2 * split <= (shortest + 31) // 32        # two k-blocks for every share
+
+
+def test_a_query_that_failed_is_asked_again(shim):
+    # an answer is kept, zero too; a failure is not: the next call asks again
+    asked = C.c_int(0)
+    ask = lambda which, answers, value: shim.asked_once(which, answers, value, C.byref(asked))          # noqa: E731
+    assert ask(0, 0, 5) == -7 and ask(0, 0, 5) == -7 and asked.value == 2
+    assert ask(0, 1, 5) == 5 and asked.value == 3
+    assert ask(0, 1, 9) == 5 and ask(0, 0, 9) == 5 and asked.value == 3
+    assert ask(1, 1, 0) == 0 and ask(1, 1, 3) == 0 and asked.value == 4
