@@ -53,6 +53,16 @@ ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters) 
     return best;
 }
 
+// Tile width and K-shares as given (option gemm_conv), with fewer shares where the shorter k or the clusters do not allow them.  The
+// cost is the least there is: such a plan is taken.
+template <class Clusters>
+ConvPlan conv_plan_fixed(const ConvShape* sh, int n, uint32_t bn, uint32_t split, Clusters clusters) {
+    uint32_t k = sh[0].K;
+    if (n > 1 && sh[1].K < k) k = sh[1].K;
+    while (split > 1 && (split * 2 > (k + 31) / 32 || clusters(bn, split) < 1)) --split;
+    return ConvPlan{bn, split, 1.0};
+}
+
 // Of `fit` clusters that run at once on `all` SMs, those that do on `sms` of them: the exchange's CTAs may sit anywhere.
 inline int conv_clusters_beside(int fit, uint64_t sms, uint64_t all) {
     if (fit < 1 || sms >= all) return fit;

@@ -134,6 +134,15 @@ int32_t fg_ctx_set_option(fg_ctx* ctx, const char* name, const char* value) {
         }
         return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "fg_ctx_set_option: gemm_tile is auto, pair, 256x32, 256x16, 128x32 or 128x16");
     }
+    if (!strcmp(name, "gemm_conv")) {
+        int bn = 0, split = 0;
+        if (!strcmp(value, "auto")) { ctx->opt_conv_bn = 0; return FG_OK; }
+        if (sscanf(value, "%dx%d", &bn, &split) == 2 && (bn == 64 || bn == 128) && split >= 1 && split <= 8) {
+            ctx->opt_conv_bn = bn; ctx->opt_conv_split = split;
+            return FG_OK;
+        }
+        return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "fg_ctx_set_option: gemm_conv is auto, or a tile width of 64 or 128 and 1 to 8 K-shares, as in 64x3");
+    }
     if (!strcmp(name, "gemm_split_k")) return truth(&ctx->opt_split_k);
     if (!strcmp(name, "gemm_pairs")) return truth(&ctx->opt_pairs);
     if (!strcmp(name, "exec_plans")) {
@@ -184,6 +193,7 @@ int32_t fg_ctx_create_on_stream(int32_t device, void* cuda_stream, fg_ctx** out)
     c->sm_count = prop.multiProcessorCount;
     c->opt_tile_pair = -1;
     c->opt_tile_group = 0;
+    c->opt_conv_bn = 0;
     c->opt_split_k = true;
     c->opt_pairs = true;
     c->opt_exec_plans = -1;

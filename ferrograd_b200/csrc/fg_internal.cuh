@@ -77,6 +77,7 @@ struct fg_ctx {
     int opt_tile_group;         // pair kernel: tile rows per group of the tile order (0: the default, eight)
     int opt_tile_pair;          // -1: chosen per shape; 1: CTA pairs whenever the shape allows; 0: opt_tile_bn x opt_tile_bk
     int opt_tile_bn, opt_tile_bk;
+    int opt_conv_bn, opt_conv_split;      // conversion kernel: its tile width and K-shares wherever it can run (0: by estimate)
     bool opt_split_k;           // split-K tail of the pair kernel
     bool opt_pairs;             // multiply f32 tensors as they lie (bf16 pairs) where the shape allows
     int opt_exec_plans;         // the graph engine records each dispatch as a CUDA graph: 1 always, 0 never, -1 when launch-bound

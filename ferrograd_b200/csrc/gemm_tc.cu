@@ -2101,9 +2101,11 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
 // ---- conversion kernel, host side ----
 template <int BN> int conv_clusters(const fg_ctx* ctx, uint32_t split);
 ConvPlan plan_conv(const fg_ctx* ctx, const ConvShape* sh, int n, uint64_t sms) {
-    return conv_plan(sh, n, sms, [&](uint32_t bn, uint32_t split) {
+    auto clusters = [&](uint32_t bn, uint32_t split) {
         return conv_clusters_beside(bn == 128 ? conv_clusters<128>(ctx, split) : conv_clusters<64>(ctx, split), sms, (uint64_t)ctx->sm_count);
-    });
+    };
+    if (ctx->opt_conv_bn) return conv_plan_fixed(sh, n, (uint32_t)ctx->opt_conv_bn, (uint32_t)ctx->opt_conv_split, clusters);
+    return conv_plan(sh, n, sms, clusters);
 }
 // One product with the whole GPU: what the choice of a kernel goes by, which does not depend on a running exchange.
 ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32_t batch) {
@@ -2427,7 +2429,7 @@ Route pick_route(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool pai
     // planes: both operands read and written twice over, transposed on the way, then 256 x 256 or 128-row tiles
     const double other = pair_ok ? pair_cycles(ctx, M, N, K, missing, missing_n)
                        : M > (uint32_t)BM && N > 128 ? pair_cycles(ctx, M, N, K, 2.0 * ((double)M * K + (double)N * K), 2) : 1e30;
-    if (conv <= other) r.kind = kRouteConv;
+    if (conv <= other || ctx->opt_conv_bn) r.kind = kRouteConv;
     return r;
 }
 

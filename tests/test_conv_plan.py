@@ -18,6 +18,10 @@ double plan(uint32_t M, uint32_t N, uint32_t K, uint32_t batch, uint32_t N2, uin
     *bn = p.bn; *split = p.split;
     return p.cycles;
 }
+uint32_t fixed(uint32_t K, uint32_t K2, uint32_t split, uint32_t largest) {
+    const ConvShape sh[2] = {{128, 128, K, 1}, {128, 128, K2, 1}};
+    return conv_plan_fixed(sh, K2 ? 2 : 1, 64, split, [&](uint32_t, uint32_t s) { return s <= largest ? 9 : 0; }).split;
+}
 std::atomic<int> known[2];
 int asked_once(int which, int answers, int value, int* asked) {
     return fg_asked_once(known[which], -7, [&](int* n) { ++*asked; *n = value; return answers != 0; });
@@ -79,6 +83,12 @@ def test_every_shape_has_a_plan(shim, sms):
                         shortest = min(K, second[1]) if second[0] else K
                         assert bn in (64, 128) and cycles > 0
                         assert split == 1 or 2 * split <= (shortest + 31) // 32        # two k-blocks for every share
+
+
+def test_given_shares_shrink_to_what_can_run(shim):
+    # two k-blocks of 32 for each share, of the shorter k; clusters that can be launched
+    assert shim.fixed(512, 0, 8, 8) == 8 and shim.fixed(480, 0, 8, 8) == 7 and shim.fixed(512, 130, 8, 8) == 2
+    assert shim.fixed(32, 0, 5, 8) == 1 and shim.fixed(4096, 4096, 8, 4) == 4
 
 
 def test_a_query_that_failed_is_asked_again(shim):

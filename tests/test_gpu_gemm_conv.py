@@ -1,5 +1,5 @@
 """The conversion kernel (f32 tensors straight into tensor-core tiles), its K-shares, padded copies and batches: sizes around
-tiles of 128 x 64 / 128, k-blocks of 32 and accumulation chunks of 256."""
+tiles of 128 x 64 / 128, k-blocks of 32 and accumulation chunks of 128."""
 import numpy as np
 import pytest
 
@@ -135,7 +135,7 @@ def test_batched(ctx, oracle, T, M, N, K, gap):
 @pytest.mark.parametrize("shift_saved,shift_out", [(0, 0), (1, 0), (0, 1), (1, 1)])
 @pytest.mark.parametrize("M,N,K", [(128, 512, 512), (100, 256, 1024), (384, 256, 256), (512, 128, 384)])
 def test_backward_onto_the_layer_below(ctx, oracle, M, N, K, shift_saved, shift_out):
-    # dA * act'(saved) and its column sums in the epilogue, or in the fold when K is cut into shares; the layer below's tensor
+    # dA * act'(saved) and its column sums in the epilogue, or where a cluster adds its K-shares; the layer below's tensor
     # and dA may start one element off a 16-byte boundary
     r = rng(M + N + K)
     A, B = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * 0.1
@@ -223,6 +223,75 @@ def test_products_beside_an_exchange(oracle, T, M, N, K):
         check(gB[t], oracle.gemm(A[t], dY[t], transA=True, f64=True), TOL, f"dB {t}")
     assert (c.to_numpy(sums) == np.arange(4096.0)).all() and c.device_status() == 0
     c.destroy()
+
+
+@pytest.fixture(params=["64x1", "128x1", "64x2", "128x2", "64x3", "128x3", "64x5", "128x5", "64x8", "128x8"])
+def given(request):
+    """A context whose f32 products take the conversion kernel with this tile width and these K-shares."""
+    from ferrograd_b200 import GpuContext
+    c = GpuContext(0)
+    c.set_option("gemm_conv", request.param)
+    yield c
+    assert c.device_status() == 0
+    c.destroy()
+
+
+def n8(n):
+    return (n + 7) // 8 * 8
+
+
+def pairs_of(c, t, n):
+    p = c.new_tensor((2, n8(n)), np.uint16)
+    c.pairs_from_f32(t, n, p, n8(n))
+    return c.to_numpy(p)[:, :n]
+
+
+# edges of tiles with rows on the 16-byte boundary and off it; more tiles than SMs, with k of their own for either gradient
+@pytest.mark.parametrize("M,N,K", [(520, 516, 260), (517, 531, 261), (2100, 540, 1100), (2101, 541, 1101)])
+def test_every_tile_and_share(given, oracle, M, N, K):
+    c = given
+    r = rng(M + N + K)
+    A, B = np.tanh(r.standard_normal((M, K))).astype(np.float32), r.standard_normal((K, N), np.float32) * 0.1
+    dZ, bias = r.standard_normal((M, N), np.float32), r.standard_normal(N, np.float32)
+    Ad, Bd, Zd = up(c, A), up(c, B), up(c, dZ)
+    f64 = lambda x: x.astype(np.float64)                                                                # noqa: E731
+    # forward: bias, activation, pre-activation, pairs
+    C, P, Cp = c.new_tensor((M, N)), c.new_tensor((M, N)), c.new_tensor((2, n8(M * N)), np.uint16)
+    c.gemm_paired(Ad, Bd, C, M, N, K, bias=up(c, bias), act="gelu", C_pairs=Cp, C_stride=n8(M * N))
+    y, z = oracle.bias_act_fwd((f64(A) @ f64(B)).astype(np.float32), bias, "gelu")
+    check(c.to_numpy(C), y, TOL_ACT, "output")
+    assert np.array_equal(c.to_numpy(Cp)[:, :M * N], pairs_of(c, C, M * N))
+    c.gemm(Ad, Bd, C, M, N, K, bias=up(c, bias), act="gelu", preact_out=P)
+    check(c.to_numpy(P), z, TOL, "pre-activation")
+    # backward onto the layer below: act' factor, pairs, column sums; both gradients in a launch, then one at a time
+    wantA, wantB = (f64(dZ) @ f64(B).T) * (1.0 - f64(A) ** 2), f64(A).T @ f64(dZ)
+    dA, dB, below, Ap = c.new_tensor((M, K)), c.new_tensor((K, N)), c.new_tensor((K,)), c.new_tensor((2, n8(M * K)), np.uint16)
+    more = dict(below_act="tanh", below_saved=Ad, below_dbias=below, dA_pairs=Ap, dA_stride=n8(M * K))
+    before = c.launch_count()
+    c.gemm_bwd_paired(Ad, Bd, Zd, M, N, K, dB=dB, dA=dA, **more)
+    if N % 4 == 0 and K % 4 == 0:
+        assert c.launch_count() - before == 2           # the products, and the fold of the column sums
+    gotA, gotB = c.to_numpy(dA), c.to_numpy(dB)
+    check(gotA, wantA, TOL, "dA")
+    check(gotB, wantB, TOL, "dB")
+    check(c.to_numpy(below), wantA.sum(0), TOL, "bias gradient of the layer below")
+    assert np.array_equal(c.to_numpy(Ap)[:, :M * K], pairs_of(c, dA, M * K))
+    c.gemm_bwd_paired(None, Bd, Zd, M, N, K, dA=dA, **more)
+    c.gemm_bwd_paired(Ad, None, Zd, M, N, K, dB=dB)
+    assert np.array_equal(c.to_numpy(dA), gotA) and np.array_equal(c.to_numpy(dB), gotB)      # k is long enough for all shares
+
+
+@pytest.mark.parametrize("T,M,N,K", [(3, 130, 516, 520), (5, 129, 517, 515)])
+def test_every_tile_and_share_of_a_batch(given, T, M, N, K):
+    r = rng(T + M + N + K)
+    A, B, dY = (r.standard_normal(s, np.float32) for s in ((T, M, K), (T, K, N), (T, M, N)))
+    Ad, Bd, Yd = up(given, A), up(given, B), up(given, dY)
+    C, dA, dB = given.new_tensor((T, M, N)), given.new_tensor((T, M, K)), given.new_tensor((T, K, N))
+    given.gemm_batched(Ad, Bd, C, T, M, N, K)
+    given.gemm_batched_bwd(Ad, Bd, Yd, T, M, N, K, dA=dA, dB=dB)
+    for got, want in ((C, np.matmul(A, B, dtype=np.float64)), (dA, np.matmul(dY, B.transpose(0, 2, 1), dtype=np.float64)),
+                      (dB, np.matmul(A.transpose(0, 2, 1), dY, dtype=np.float64))):
+        check(given.to_numpy(got), want, TOL, "batch")
 
 
 def test_batched_refuses_what_one_product_refuses(ctx):
