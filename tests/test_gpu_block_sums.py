@@ -42,3 +42,22 @@ def test_column_sums(ctx, M, N):
         want = dY.astype(np.float64).sum(0)
         # chains of at most 32 + 8 additions of partial sums below 4 sqrt(M): far below 1e-5 sqrt(M)
         assert np.abs(ctx.to_numpy(db) - want).max() <= 1e-5 * np.sqrt(M)
+
+
+def test_cross_entropy_sums(ctx):
+    # the loss dispatch of a graph that ends in softmax: one row to more elements than all blocks hold at once
+    from ferrograd_b200.mlp import GraphMLP
+    r = np.random.Generator(np.random.Philox(4))
+    for rows, cols in ((1, 5), (64, 10), (33, 1000), (2500, 1001), (7, 3)):
+        net = GraphMLP(ctx, [4, cols], rows, "gelu", "ce", ("sgd", 1e-3))
+        net.set_params([r.standard_normal((4, cols), np.float32)], [r.standard_normal(cols, np.float32)])
+        t = r.integers(0, cols, rows).astype(np.uint32)
+        net.upload_batch(r.standard_normal((rows, 4), np.float32), t)
+        for again in range(2):
+            ctx.dispatch_forward(net.schedule)
+            ctx.dispatch_loss(net.schedule, net.target)
+            p = net.get_output().astype(np.float64)
+            want = -np.log(p[np.arange(rows), t]).sum()
+            # positive terms in at most 9 + 5 + 8 + 5 + 5 + 8 additions, and the logarithm's own roundings
+            assert abs(net.get_loss() - want) <= 45 * 2.0 ** -24 * want, (rows, cols)
+        net.destroy()
