@@ -2,14 +2,17 @@
 than the 126 MB L2 so DRAM counters mean something, but well under a few GB on the device
 and only a handful of launches.
 
-    python -m ferrograd_b200.cases gemm|gemm_bwd|gemm_bf16|layer|softmax|softmax_ce|adamw|sgd|eltwise|skinny|mlp|graph_mlp [--iters N]
+    python -m ferrograd_b200.cases gemm|gemm_bwd|gemm_bf16|gemm_conv|layer|softmax|softmax_ce|adamw|sgd|eltwise|chain_ops|skinny|mlp|graph_mlp [--iters N]
 
 mlp runs training steps of a benchmark workload (--workload c4|c5|c5s) through MLPTrainer, graph_mlp the same
 through the graph API (dispatch_forward / loss / backward / optim); c5s is the eight-layer workload at 4096-wide
 layers and 4096 samples, small enough for a multi-pass capture.  layer runs the three GEMMs of one hidden layer on
 f32 tensors with bf16 pairs as a training step launches them (forward with bias, tanh and the output's pairs; dW; dX
 with the activation factor of the layer below, its pairs and its bias gradient) at --m samples, --k inputs, --nn
-outputs (default 2048 x 8192 x 8192, one layer of the eight-layer workload).
+outputs (default 2048 x 8192 x 8192, one layer of the eight-layer workload).  gemm_conv runs a product on the conversion
+kernel with a given tile width and K-shares (--plan, option gemm_conv) at --k and at twice --k: the difference is the cost of
+k / 32 k-blocks.  chain_ops runs elementwise programs of 2 and of 12 equal operations in f32 and f16: the difference is the
+cost of ten of them.
 """
 import argparse
 import sys
@@ -22,8 +25,8 @@ from .mlp import MLPTrainer
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["gemm", "gemm_bwd", "gemm_bf16", "layer", "softmax", "softmax_ce", "adamw", "sgd", "eltwise", "skinny",
-                                     "mlp", "graph_mlp"])
+    ap.add_argument("case", choices=["gemm", "gemm_bwd", "gemm_bf16", "gemm_conv", "layer", "softmax", "softmax_ce", "adamw", "sgd",
+                                     "eltwise", "chain_ops", "skinny", "mlp", "graph_mlp"])
     ap.add_argument("--workload", default="c4", choices=["c4", "c5", "c5s"])
     ap.add_argument("--m", type=int, default=2048)
     ap.add_argument("--k", type=int, default=8192)
@@ -31,6 +34,7 @@ def main():
     ap.add_argument("--iters", type=int, default=3)
     ap.add_argument("--n", type=int, default=0, help="override the problem size")
     ap.add_argument("--mode", default="auto", choices=["auto", "simt", "3xtf32", "tf32_bf16x2"], help="GEMM mode")
+    ap.add_argument("--plan", default="128x1", help="gemm_conv: tile width and K-shares")
     a = ap.parse_args()
     ctx = GpuContext(0)
     r = np.random.Generator(np.random.Philox(1))
@@ -57,6 +61,14 @@ def main():
         Cm = ctx.new_tensor((n, n), np.uint16)
         for _ in range(a.iters):
             ctx.gemm_lowp(A, B, Cm, n, n, n, "bf16", bias=bias, act="relu")
+    elif a.case == "gemm_conv":
+        ctx.set_option("gemm_conv", a.plan)
+        for k in (a.k, 2 * a.k):
+            A = ctx.init_tensor_f32((a.m, k), r.standard_normal((a.m, k), np.float32))
+            B = ctx.init_tensor_f32((k, a.nn), r.standard_normal((k, a.nn), np.float32) * np.float32(k ** -0.5))
+            Cm = ctx.new_tensor((a.m, a.nn))
+            for _ in range(a.iters):
+                ctx.gemm(A, B, Cm, a.m, a.nn, k)
     elif a.case == "layer":
         M, K, N = a.m, a.k, a.nn
         f = lambda shape, scale: ctx.init_tensor_f32(shape, r.standard_normal(shape, np.float32) * np.float32(scale))
@@ -111,6 +123,15 @@ def main():
             ctx.bce_loss_grad(t[0], t[1], n, 0.5, loss_elem=t[2], loss_sum=one, grad=t[3])
             ctx.eltwise_chain_fwd(chain, [t[0], t[1]], t[2], n)
             ctx.eltwise_chain_bwd(chain, [t[0], t[1]], t[2], [t[3], None], n)
+    elif a.case == "chain_ops":
+        n = a.n or (1 << 20)
+        for dtype, init in (("f32", ctx.init_tensor_f32), ("f16", ctx.init_tensor_f16)):
+            x, y, out = (init((n,), r.random(n, np.float32) + np.float32(0.5)) for _ in range(3))
+            ctx.eltwise_chain_fwd([("input", 0, 0, 0.0)], [x], out, n, dtype=dtype)
+            for op in ("mul", "neg", "gelu", "exp"):
+                for k in (2, 12):
+                    prog = [("input", 0, 0, 0.0), ("input", 1, 0, 0.0)] + [(op, i + (i > 0), 1, 0.0) for i in range(k)]
+                    ctx.eltwise_chain_fwd(prog, [x, y], out, n, dtype=dtype)
     elif a.case == "skinny":
         # the three kernels of a 10-class output layer on 32768 x 4096 activations (512 MB)
         M, K, N = a.n or 32768, 4096, 10

@@ -214,18 +214,13 @@ __global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_
     fold_chunks_of_columns(blockIdx.x * 32 + cx, threadIdx.x >> 5, cx, cols, nchunks, part, out, red);
 }
 
-// ---- chains ----
-// Storage type of a chain's tensors.  Values are held as float in registers; with 16-bit storage every
-// operation's result is rounded to the storage type (round to nearest even), which for + - * / equals
-// native half arithmetic (float carries more than twice the bits, so the double rounding is harmless).
-// ld4w / st4w move four consecutive elements starting at element i (one 128-bit access for f32, one 64-bit access for the
-// 16-bit types; the caller has checked the alignment).
+// ---- storage types ----
+// Elements of a type as f32, for conversions (to the nearest, ties to even).  ld4w / st4w move four consecutive elements starting
+// at element i (one 128-bit access for f32, one 64-bit access for the 16-bit types; the caller has checked the alignment).
 template <int DT> struct Stored;
 template <> struct Stored<FG_DTYPE_F32> {
-    typedef float T;
     static __device__ __forceinline__ float ld(const void* p, uint64_t i) { return static_cast<const float*>(p)[i]; }
     static __device__ __forceinline__ void st(void* p, uint64_t i, float v) { static_cast<float*>(p)[i] = v; }
-    static __device__ __forceinline__ float r(float v) { return v; }
     static __device__ __forceinline__ void ld4w(const void* p, uint64_t i, float* o) {
         const float4 v = *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i);
         o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
@@ -235,10 +230,8 @@ template <> struct Stored<FG_DTYPE_F32> {
     }
 };
 template <> struct Stored<FG_DTYPE_F16> {
-    typedef __half T;
     static __device__ __forceinline__ float ld(const void* p, uint64_t i) { return __half2float(static_cast<const __half*>(p)[i]); }
     static __device__ __forceinline__ void st(void* p, uint64_t i, float v) { static_cast<__half*>(p)[i] = __float2half_rn(v); }
-    static __device__ __forceinline__ float r(float v) { return __half2float(__float2half_rn(v)); }
     static __device__ __forceinline__ void ld4w(const void* p, uint64_t i, float* o) {
         const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const __half*>(p) + i);
         const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
@@ -253,10 +246,8 @@ template <> struct Stored<FG_DTYPE_F16> {
     }
 };
 template <> struct Stored<FG_DTYPE_BF16> {
-    typedef __nv_bfloat16 T;
     static __device__ __forceinline__ float ld(const void* p, uint64_t i) { return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]); }
     static __device__ __forceinline__ void st(void* p, uint64_t i, float v) { static_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v); }
-    static __device__ __forceinline__ float r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
     static __device__ __forceinline__ void ld4w(const void* p, uint64_t i, float* o) {
         const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p) + i);
         o[0] = __uint_as_float(u.x << 16); o[1] = __uint_as_float(u.x & 0xffff0000u);
@@ -302,11 +293,12 @@ constexpr int kVmThreads = 128;
 constexpr int kVmWords = 8;         // 32-bit words of a value that a thread holds: eight f32 elements, or sixteen 16-bit ones in pairs
 constexpr int kVmSlotUnits = 2 * kVmThreads;
 
-// A value's words: Lanes<DT> does arithmetic on them.  16-bit types stay packed: + - * on two elements at once in the type's
-// own arithmetic, which rounds as an operation in f32 followed by a rounding to the type does (f32 has more than twice the
-// bits); functions and the quotient on f32 lanes.
+// A value's words: Lanes<DT> does arithmetic on them.  With 16-bit storage every operation's result is rounded to the type.  The
+// words stay packed: + - * on two elements at once in the type's own arithmetic, functions and the quotient on f32 lanes and
+// then rounded.  For + - * both ways give the same bits (f32 has at least two bits more than twice the type's, so its own
+// rounding does no harm), but for bf16 products below f32's normal range (2^-126), where f32 rounds coarser and the packed product, which
+// is rounded once, is the nearer one.
 template <int DT> struct Lanes {
-    typedef Stored<DT> S;
     typedef typename std::conditional<DT == FG_DTYPE_F16, __half2, __nv_bfloat162>::type P;
     static constexpr int kE = 2;
     static __device__ __forceinline__ P p(uint32_t u) { return *reinterpret_cast<P*>(&u); }

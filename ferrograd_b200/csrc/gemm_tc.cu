@@ -14,14 +14,14 @@
 // Four ways to get hi and lo to the tensor core, chosen by estimates of their times (pick_route and its callers):
 //   * pairs: the f32 tensor as it lies (the MMA truncates it) beside bf16 planes kept with it or made in one pass;
 //     256 x 256 tiles on SM pairs.  Large products.
-//   * conversion kernel: the f32 tensors alone; warps round and split each k-block in shared memory.  Small and
-//     middling products, batches.
+//   * conversion kernel: the f32 tensors alone; warps round and split each k-block, one operand into tensor memory and the
+//     other in shared memory.  Small and middling products, batches.
 //   * operand planes: a pre-pass writes hi and lo planes of each operand into the scratch arena, contraction index
 //     contiguous, transposing on the way; dY * act'(saved) is applied there.  Any shape; the strict mode.
 //   * 16-bit tensors go to kind::f16 as they lie, with a padded copy where rows are not 16-byte aligned.
-// Every kernel is a warp-specialised pipeline: one thread issues bulk-tensor loads (no multicast) into swizzled shared
-// memory, one thread issues tcgen05.mma, other warps read the accumulators back with tcgen05.ld and apply bias and
-// activation while storing.
+// Every kernel is a warp-specialised pipeline: one warp issues bulk-tensor loads (no multicast) into swizzled shared
+// memory, one warp issues tcgen05.mma (a lane of each, elected where the warp runs the role as a whole), other warps read the
+// accumulators back with tcgen05.ld and apply bias and activation while storing.
 #include <atomic>
 #include <cuda_bf16.h>
 #include <stdlib.h>
@@ -906,14 +906,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
 }
 
-// Folds the K-shares of tiles of TM x TN in a fixed order, then does what the kernels' own epilogues do for a whole
+// Folds the pair kernel's K-shares of a 256 x 256 tile in a fixed order, then does what its own epilogue does for a whole
 // tile: bias, activation (or the act' factor), store, bf16 pairs, column sums.
 // A block of 256 threads per 32 x 32 sub-block (so that a block owns whole 32-row column sums); thread t handles four
 // consecutive columns of row t / 8.
-template <int TM, int TN>
 __global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
     fg_grid_enter();
     __shared__ float cs_sm[8][32];
+    constexpr uint32_t TM = 2 * BM, TN = 256;
     constexpr uint32_t kSubN = TN / 32, kSubs = (TM / 32) * kSubN;
     const uint32_t pairs_m = (ep.M + TM - 1) / TM, pairs_n = (ep.N + TN - 1) / TN;
     const uint32_t tail = blockIdx.x / kSubs, sub = blockIdx.x % kSubs;
@@ -2091,7 +2091,7 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     gemm_tc_pair_kernel<BK, FMT><<<grid, kPairThreads, Cfg::kSmemBytes, ctx->stream>>>(tmA, tmB, tmA16, tmB16, ep);
     FG_LAUNCHED(ctx);
     if (ep.split > 1) {
-        fg_launch(ctx, gemm_tc_fold_kernel<2 * BM, 256>, (unsigned)((ntiles - ep.t_full) * 64), 256, 0, ep);
+        fg_launch(ctx, gemm_tc_fold_kernel, (unsigned)((ntiles - ep.t_full) * 64), 256, 0, ep);
         FG_LAUNCHED(ctx);
     }
     fg_time_end(ctx, tr);
@@ -3047,8 +3047,8 @@ int32_t fg_gemm_bwd_paired_f32(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, 
 
 // Batched forms: `batch` independent products, operand t at base + t*stride (strides in elements).
 // The reference steps A, B and C by one matrix per Z index of a rank-3 matmul (kernel/forward.rs:159-190).
-// Rank-3 products.  Small matrices (the SIMT path's range) and middling ones (the conversion kernel) run as ONE launch
-// with the matrix index in the grid's z, as the reference's generated kernel does (kernel/forward.rs:159-190).  Large
+// Rank-3 products.  Small matrices (the SIMT path's range: the matrix index is the grid's z, as in the reference's generated
+// kernel, kernel/forward.rs:159-190) and middling ones (the conversion kernel: it is part of the unit's number) run as ONE launch.  Large
 // ones: the bf16 pairs of the whole batch are made by one pass per operand, then one GEMM launch per matrix reads its
 // slice (batch + 2 launches, and a launch that fills the GPU gains nothing from being merged with its neighbours).
 int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, const float* A,
