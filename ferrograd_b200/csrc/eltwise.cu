@@ -76,23 +76,6 @@ __global__ void __launch_bounds__(256) act_bwd_kernel(uint64_t n, int act, const
         dz[i] = act == FG_ACT_NONE ? dy[i] : dy[i] * fg_act_grad(act, saved[i]);
 }
 
-// The sum of the blocks' sums (`s` in thread 0 of 256) by the block that arrives last: partials in strides of 256, then across the
-// threads.
-__device__ __forceinline__ void fold_sums(float s, float* __restrict__ partials, unsigned* arrivals, float* __restrict__ out, float* red) {
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
-    if (!fg_last_block(arrivals, gridDim.x)) return;
-    s = 0.0f;
-    for (uint32_t i = threadIdx.x; i < gridDim.x; i += 256) s += __ldcg(partials + i);
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < 8; ++w) t += red[w];
-        *out = t;
-    }
-}
-
 struct MseTerm {   // loss = d*d, grad = 2*d*scale
     static __device__ __forceinline__ float loss(float p, float t) { const float d = p - t; return d * d; }
     static __device__ __forceinline__ float grad(float p, float t, float scale) { return (2.0f * (p - t)) * scale; }
@@ -102,12 +85,11 @@ struct BceTerm {   // on probabilities: loss = -(t*log(p) + (1-t)*log(1-p)), gra
     static __device__ __forceinline__ float grad(float p, float t, float scale) { return (p - t) * scale; }
 };
 
-// Per-element loss and gradient of MSE or BCE, and the sum of the losses through `partials`, one per block.
+// Per-element loss and gradient of MSE or BCE; with `partials`, the sum of the losses, one part per block (see fg_leave_sum).
 template <class TERM, bool VEC>
 __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ pred, const float* __restrict__ target,
                                                    uint64_t n, float scale, float* __restrict__ loss_elem,
-                                                   float* __restrict__ grad, float* __restrict__ partials,
-                                                   unsigned* arrivals, float* __restrict__ sum) {
+                                                   float* __restrict__ grad, float* partials, unsigned* arrivals, float* sum) {
     fg_grid_enter();
     __shared__ float red[8];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -135,13 +117,12 @@ __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ pre
         float t = 0.0f;
         if (threadIdx.x == 0)
             for (int w = 0; w < 8; ++w) t += red[w];
-        fold_sums(t, partials, arrivals, sum, red);
+        fg_leave_sum(t, partials, arrivals, sum, red);
     }
 }
 
-// Sum of n values: one partial per block (grid-stride over float4, fixed order inside a block), then the partials.
-__global__ void __launch_bounds__(256) sum_kernel(const float* __restrict__ x, uint64_t n, float* __restrict__ partials, unsigned* arrivals,
-                                                  float* __restrict__ out) {
+// Sum of n values: one part per block (grid-stride over float4, fixed order inside a block), then the parts.
+__global__ void __launch_bounds__(256) sum_kernel(const float* __restrict__ x, uint64_t n, float* partials, unsigned* arrivals, float* out) {
     fg_grid_enter();
     __shared__ float red[8];
     float s = 0.0f;
@@ -157,7 +138,15 @@ __global__ void __launch_bounds__(256) sum_kernel(const float* __restrict__ x, u
     float t = 0.0f;
     if (threadIdx.x == 0)
         for (int w = 0; w < 8; ++w) t += red[w];
-    fold_sums(t, partials, arrivals, out, red);
+    fg_leave_sum(t, partials, arrivals, out, red);
+}
+
+// The partial sums that a launch left, in the order of its last block.
+__global__ void __launch_bounds__(256) fold_partials_kernel(const float* partials, uint32_t n, float* __restrict__ out) {
+    fg_grid_enter();
+    __shared__ float red[8];
+    const float s = fg_sum_partials(partials, n, red);
+    if (threadIdx.x == 0) *out = s;
 }
 
 // out[c] = sum over chunks of part[k][c], for 32 columns and 256 threads.  The eight warps each add every eighth chunk into eight
@@ -182,8 +171,9 @@ __device__ __forceinline__ void fold_chunks_of_columns(uint32_t c, uint32_t gy, 
     }
 }
 
-// Column sums: block (32 x 8) covers 32 columns and `chunk` rows and leaves their sums in part[blockIdx.y]; with `out`, the last
+// Column sums: block (32 x 8) covers 32 columns and `chunk` rows and leaves their sums in part[blockIdx.y]; with FOLD, the last
 // block of those columns adds the chunks.
+template <bool FOLD>
 __global__ void __launch_bounds__(256) colsum_kernel(uint32_t rows, uint32_t cols, uint32_t chunk, const float* __restrict__ x, float* part,
                                                      unsigned* arrivals, float* __restrict__ out) {
     fg_grid_enter();
@@ -202,8 +192,9 @@ __global__ void __launch_bounds__(256) colsum_kernel(uint32_t rows, uint32_t col
         for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
         part[(size_t)blockIdx.y * cols + c] = t;
     }
-    if (!out || !fg_last_block(arrivals + blockIdx.x, gridDim.y)) return;
-    fold_chunks_of_columns(c, threadIdx.y, threadIdx.x, cols, gridDim.y, part, out, red);
+    if constexpr (FOLD)
+        if (fg_last_block(arrivals + blockIdx.x, gridDim.y))
+            fold_chunks_of_columns(c, threadIdx.y, threadIdx.x, cols, gridDim.y, part, out, red);
 }
 // The chunks of column sums that other kernels left; a block covers 32 columns.
 __global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_t nchunks,
@@ -795,25 +786,44 @@ int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, cons
     return FG_OK;
 }
 
+int32_t fg_block_sums(fg_ctx* ctx, int grid, float* sum, FgBlockSums* b) {
+    *b = FgBlockSums{sum, nullptr, sum, grid};
+    if (!sum || grid == 1) return FG_OK;
+    void* p;
+    const int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &p);
+    if (s != FG_OK) return s;
+    b->partials = (float*)p;
+    if (fg_fold_in_launch(ctx, (uint64_t)grid)) b->out = sum;
+    return FG_OK;
+}
+int32_t fg_block_sums_end(fg_ctx* ctx, const FgBlockSums& b) {
+    if (b.out || b.partials == b.sum) return FG_OK;
+    fg_launch(ctx, fold_partials_kernel, 1, 256, 0, (const float*)b.partials, (uint32_t)b.grid, b.sum);
+    FG_LAUNCHED(ctx);
+    return FG_OK;
+}
+
 int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* out) {
     const uint32_t chunk = 256, groups = (cols + 31) / 32;
     const uint32_t nchunks = (rows + chunk - 1) / chunk;
     dim3 grid(groups, nchunks), block(32, 8);
     if (nchunks == 1) {      // the only partial is the sum
-        fg_launch(ctx, colsum_kernel, grid, block, 0, rows, cols, chunk, x, out, (unsigned*)nullptr, (float*)nullptr);
+        fg_launch(ctx, colsum_kernel<false>, grid, block, 0, rows, cols, chunk, x, out, (unsigned*)nullptr, (float*)nullptr);
         FG_LAUNCHED(ctx);
         return FG_OK;
     }
     void* part;
     int32_t s = fg_ws_alloc(ctx, (uint64_t)nchunks * cols * sizeof(float), &part);
     if (s != FG_OK) return s;
-    const bool one = groups <= kFgArrivals;      // a counter for each group of columns
-    fg_launch(ctx, colsum_kernel, grid, block, 0, rows, cols, chunk, x, (float*)part, fg_arrivals(ctx), one ? out : (float*)nullptr);
-    FG_LAUNCHED(ctx);
-    if (!one) {
-        fg_launch(ctx, colsum_fold_kernel, groups, 256, 0, cols, nchunks, (const float*)part, out);
+    if (groups <= kFgArrivals && fg_fold_in_launch(ctx, (uint64_t)groups * nchunks)) {      // a counter for each group of columns
+        fg_launch(ctx, colsum_kernel<true>, grid, block, 0, rows, cols, chunk, x, (float*)part, fg_arrivals(ctx), out);
         FG_LAUNCHED(ctx);
+        return FG_OK;
     }
+    fg_launch(ctx, colsum_kernel<false>, grid, block, 0, rows, cols, chunk, x, (float*)part, (unsigned*)nullptr, (float*)nullptr);
+    FG_LAUNCHED(ctx);
+    fg_launch(ctx, colsum_fold_kernel, groups, 256, 0, cols, nchunks, (const float*)part, out);
+    FG_LAUNCHED(ctx);
     return FG_OK;
 }
 
@@ -853,12 +863,12 @@ int32_t fg_sum_f32(fg_ctx* ctx, const float* x, uint64_t n, float* out) {
         return FG_OK;
     }
     const int grid = fg_stream_grid(ctx, (n + 3) / 4, 256, 4);
-    void* p;
-    int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &p);
+    FgBlockSums b;
+    const int32_t s = fg_block_sums(ctx, grid, out, &b);
     if (s != FG_OK) return s;
-    fg_launch(ctx, sum_kernel, grid, 256, 0, x, n, (float*)p, fg_arrivals(ctx), out);
+    fg_launch(ctx, sum_kernel, grid, 256, 0, x, n, b.partials, fg_arrivals(ctx), b.out);
     FG_LAUNCHED(ctx);
-    return FG_OK;
+    return fg_block_sums_end(ctx, b);
 }
 
 int32_t fg_mse_loss_grad(fg_ctx* ctx, const float* pred, const float* target, uint64_t n, float grad_scale,
@@ -872,19 +882,15 @@ int32_t fg_mse_loss_grad(fg_ctx* ctx, const float* pred, const float* target, ui
     }
     const bool vec = aligned16(pred) && aligned16(target) && aligned16(loss_elem_out) && aligned16(grad_out);
     const int grid = fg_stream_grid(ctx, vec ? (n + 3) / 4 : n, 256, 8);
-    float* partials = nullptr;
-    if (loss_sum_out) {
-        void* p;
-        int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &p);
-        if (s != FG_OK) return s;
-        partials = (float*)p;
-    }
+    FgBlockSums b;
+    const int32_t s = fg_block_sums(ctx, grid, loss_sum_out, &b);
+    if (s != FG_OK) return s;
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (8.0 + (loss_elem_out ? 4.0 : 0.0) + (grad_out ? 4.0 : 0.0)) * n);
-    if (vec) fg_launch(ctx, loss_kernel<MseTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
-    else fg_launch(ctx, loss_kernel<MseTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
+    if (vec) fg_launch(ctx, loss_kernel<MseTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, b.partials, fg_arrivals(ctx), b.out);
+    else fg_launch(ctx, loss_kernel<MseTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, b.partials, fg_arrivals(ctx), b.out);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
-    return FG_OK;
+    return fg_block_sums_end(ctx, b);
 }
 
 int32_t fg_bce_loss_grad(fg_ctx* ctx, const float* pred, const float* target, uint64_t n, float grad_scale,
@@ -898,19 +904,15 @@ int32_t fg_bce_loss_grad(fg_ctx* ctx, const float* pred, const float* target, ui
     }
     const bool vec = aligned16(pred) && aligned16(target) && aligned16(loss_elem_out) && aligned16(grad_out);
     const int grid = fg_stream_grid(ctx, vec ? (n + 3) / 4 : n, 256, 8);
-    float* partials = nullptr;
-    if (loss_sum_out) {
-        void* p;
-        int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &p);
-        if (s != FG_OK) return s;
-        partials = (float*)p;
-    }
+    FgBlockSums b;
+    const int32_t s = fg_block_sums(ctx, grid, loss_sum_out, &b);
+    if (s != FG_OK) return s;
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, (8.0 + (loss_elem_out ? 4.0 : 0.0) + (grad_out ? 4.0 : 0.0)) * n);
-    if (vec) fg_launch(ctx, loss_kernel<BceTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
-    else fg_launch(ctx, loss_kernel<BceTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, partials, fg_arrivals(ctx), loss_sum_out);
+    if (vec) fg_launch(ctx, loss_kernel<BceTerm, true>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, b.partials, fg_arrivals(ctx), b.out);
+    else fg_launch(ctx, loss_kernel<BceTerm, false>, grid, 256, 0, pred, target, n, grad_scale, loss_elem_out, grad_out, b.partials, fg_arrivals(ctx), b.out);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
-    return FG_OK;
+    return fg_block_sums_end(ctx, b);
 }
 
 int32_t fg_eltwise_chain_fwd_dt(fg_ctx* ctx, int32_t dtype, uint64_t n, const fg_ew_instr* prog, int32_t ninstr,

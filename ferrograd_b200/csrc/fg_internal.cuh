@@ -163,13 +163,18 @@ inline void fg_launch(fg_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, 
 }
 __device__ __forceinline__ void fg_grid_enter() { cudaGridDependencySynchronize(); }
 
-// Reductions over blocks without a second launch: every block leaves its part in memory and counts itself; the one that arrives
-// last sees all parts and adds them, in an order that does not depend on who it is.  The counters (behind the device error word)
+// Sums over the blocks of a launch: every block leaves its part in memory, and the parts are added in an order that does not depend
+// on who adds them, by the block that counts itself last or by a launch of its own.  The counters (behind the device error word)
 // start at zero and wrap back to it; the kernels of a context run one after the other, so one set serves all of them.
-// A launch of its own for the fold cost 2 - 2.5 us of a training step each.
 constexpr uint32_t kFgArrivals = 1024;
 inline unsigned* fg_arrivals(const fg_ctx* ctx) { return reinterpret_cast<unsigned*>(ctx->dev_status) + 64; }
 constexpr size_t kFgStatusBytes = 256 + kFgArrivals * sizeof(unsigned);
+// Does the last block add?  Recorded in a plan, a second launch costs the device 0.9 us, and the fence, the counter and the way to the
+// other parts 1.7 us or more, for every wave of blocks; called one by one, every launch costs the host 2 us, which is more than
+// either while the blocks are few.  MSE of 4096 and of 1 Mi elements, column sums of 384 x 256 and of 16384 x 1000, us:
+// in a plan 2.2 / 4.3 / 2.8 / 8.3 with a second launch and 3.2 / 6.7 / 3.4 / 13.3 in one; called one by one 6.2 / 6.2 / 6.1 /
+// 8.9 and 4.1 / 7.0 / 4.5 / 13.4.
+inline bool fg_fold_in_launch(const fg_ctx* ctx, uint64_t blocks) { return !ctx->capturing && blocks <= 2 * (uint64_t)ctx->sm_count; }
 // Called by all threads of a block after they have written their part; true in the block that is the last of `blocks`.
 __device__ __forceinline__ bool fg_last_block(unsigned* arrivals, unsigned blocks) {
     __shared__ int last;
@@ -179,6 +184,26 @@ __device__ __forceinline__ bool fg_last_block(unsigned* arrivals, unsigned block
     __syncthreads();
     if (last) __threadfence();
     return last != 0;
+}
+// The sum of n partial sums, in thread 0 of 256: in strides of 256, then across the threads.
+__device__ __forceinline__ float fg_sum_partials(const float* partials, uint32_t n, float* red) {
+    float s = 0.0f;
+    for (uint32_t i = threadIdx.x; i < n; i += 256) s += __ldcg(partials + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0.0f;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < 8; ++w) s += red[w];
+    return s;
+}
+// A block's sum (in thread 0 of 256) goes to the partials; with `out`, the last block adds them.
+__device__ __forceinline__ void fg_leave_sum(float s, float* partials, unsigned* arrivals, float* out, float* red) {
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (!out || !fg_last_block(arrivals, gridDim.x)) return;
+    s = fg_sum_partials(partials, gridDim.x, red);
+    if (threadIdx.x == 0) *out = s;
 }
 
 // Brackets one kernel launch with events when timing is enabled (never while capturing).
@@ -383,5 +408,10 @@ uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t
 // fg_ce_loss_grad with the sum of the losses; its arguments have been checked.
 int32_t fg_ce_loss_grad_sum(fg_ctx* ctx, const float* probs, const uint32_t* labels, uint32_t rows, uint32_t cols, float* loss_out,
                             float* grad_out, float* loss_sum_out);
+// Where `grid` blocks leave their partial sums (scratch, or *sum itself for one block), where the last of them leaves the sum, if it
+// adds them; fg_block_sums_end(), after the launch, has them added otherwise.  No sum wanted: both NULL.
+struct FgBlockSums { float *partials, *out, *sum; int grid; };
+int32_t fg_block_sums(fg_ctx* ctx, int grid, float* sum, FgBlockSums* b);
+int32_t fg_block_sums_end(fg_ctx* ctx, const FgBlockSums& b);
 int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* out);
 int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, float* out);

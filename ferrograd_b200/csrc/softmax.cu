@@ -736,10 +736,10 @@ __global__ void softmax_bwd_kernel(uint32_t rows, uint32_t cols, const float* __
     }
 }
 
-// The reference's unfused per-element CE on probabilities; with `sum`, also the sum of the losses, through one partial per block.
-__global__ void ce_elem_kernel(const float* __restrict__ p, const uint32_t* __restrict__ labels, uint32_t rows,
+// The reference's unfused per-element CE on probabilities; with `partials`, also the sum of the losses, one part per block.
+__global__ void __launch_bounds__(256) ce_elem_kernel(const float* __restrict__ p, const uint32_t* __restrict__ labels, uint32_t rows,
                                uint32_t cols, float* __restrict__ loss, float* __restrict__ grad, float* partials, unsigned* arrivals,
-                               float* __restrict__ sum) {
+                               float* sum) {
     fg_grid_enter();
     __shared__ float red[32];
     float s = 0.0f;
@@ -753,14 +753,7 @@ __global__ void ce_elem_kernel(const float* __restrict__ p, const uint32_t* __re
         grad[i] = hit ? pv - 1.0f : pv;
         s += l;
     }
-    if (!sum) return;
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
-    if (!fg_last_block(arrivals, gridDim.x)) return;
-    s = 0.0f;
-    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) s += __ldcg(partials + i);
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) *sum = s;
+    if (partials) fg_leave_sum(block_sum(s, red), partials, arrivals, sum, red);
 }
 
 // Fixed-order mean of the per-row losses (one CTA).
@@ -873,14 +866,12 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
 static int32_t ce_elem_launch(fg_ctx* ctx, const float* probs, const uint32_t* labels, uint32_t rows, uint32_t cols, float* loss_out,
                               float* grad_out, float* loss_sum_out) {
     const int grid = fg_stream_grid(ctx, (uint64_t)rows * cols, 256, 8);
-    void* part = nullptr;
-    if (loss_sum_out) {
-        const int32_t s = fg_ws_alloc(ctx, (uint64_t)grid * sizeof(float), &part);
-        if (s != FG_OK) return s;
-    }
-    fg_launch(ctx, ce_elem_kernel, grid, 256, 0, probs, labels, rows, cols, loss_out, grad_out, (float*)part, fg_arrivals(ctx), loss_sum_out);
+    FgBlockSums b;
+    const int32_t s = fg_block_sums(ctx, grid, loss_sum_out, &b);
+    if (s != FG_OK) return s;
+    fg_launch(ctx, ce_elem_kernel, grid, 256, 0, probs, labels, rows, cols, loss_out, grad_out, b.partials, fg_arrivals(ctx), b.out);
     FG_LAUNCHED(ctx);
-    return FG_OK;
+    return fg_block_sums_end(ctx, b);
 }
 
 extern "C" {

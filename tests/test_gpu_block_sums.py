@@ -1,5 +1,5 @@
-"""Sums that the last block to arrive adds up (loss sums, column sums): one block, a few, all of them; the counters serve the next
-call, of another size, as they did the first."""
+"""Sums over blocks (loss sums, column sums), which the last block to arrive adds up or a second launch: one block, a few, all of
+them; the counters serve the next call, of another size, as they did the first."""
 import numpy as np
 import pytest
 
@@ -61,3 +61,49 @@ def test_cross_entropy_sums(ctx):
             # positive terms in at most 9 + 5 + 8 + 5 + 5 + 8 additions, and the logarithm's own roundings
             assert abs(net.get_loss() - want) <= 45 * 2.0 ** -24 * want, (rows, cols)
         net.destroy()
+
+
+@pytest.mark.parametrize("n,called,recorded", [(1000, 1, 1), (100_001, 1, 2), (3_000_003, 2, 2)])
+def test_sums_in_one_launch_or_two(ctx, n, called, recorded):
+    # one block has the sum; a few are added by the last of them where the call's launches cost more, and by a second launch in a
+    # plan; many by a second launch.  The same additions every time.
+    r = np.random.Generator(np.random.Philox(n))
+    p, t = ctx.init_tensor_f32((n,), r.random(n, np.float32) * 0.8 + 0.1), ctx.init_tensor_f32((n,), r.random(n, np.float32))
+    outs = [ctx.new_tensor((1,)) for _ in range(3)]
+    calls = [lambda: ctx.mse_loss_grad(p, t, n, loss_sum=outs[0]), lambda: ctx.bce_loss_grad(p, t, n, loss_sum=outs[1]),
+             lambda: ctx._check(ctx.lib.fg_sum_f32(ctx.handle, p.ptr, n, outs[2].ptr))]
+    for call, out in zip(calls, outs):
+        before = ctx.launch_count()
+        call()
+        assert ctx.launch_count() - before == called
+        first = ctx.to_numpy(out)[0]
+        ctx.plan_begin()
+        call()
+        plan = ctx.plan_end()
+        for again in range(2):
+            ctx.memset_zero(out)
+            before = ctx.launch_count()
+            plan.launch()
+            assert ctx.launch_count() - before == recorded
+            assert ctx.to_numpy(out)[0] == first
+        plan.destroy()
+
+
+@pytest.mark.parametrize("M,N,called,recorded", [(200, 1000, 1, 1), (300, 1000, 1, 2), (3000, 40, 1, 2), (9000, 300, 2, 2)])
+def test_column_sums_in_one_launch_or_two(ctx, M, N, called, recorded):
+    r = np.random.Generator(np.random.Philox(M + N))
+    dY, db = ctx.init_tensor_f32((M, N), r.standard_normal((M, N), np.float32)), ctx.new_tensor((N,))
+    call = lambda: ctx.gemm_bwd(None, None, dY, M, N, 1, dbias=db, mode="simt")             # noqa: E731
+    before = ctx.launch_count()
+    call()
+    assert ctx.launch_count() - before == called
+    first = ctx.to_numpy(db)
+    ctx.plan_begin()
+    call()
+    plan = ctx.plan_end()
+    ctx.memset_zero(db)
+    before = ctx.launch_count()
+    plan.launch()
+    assert ctx.launch_count() - before == recorded
+    assert np.array_equal(ctx.to_numpy(db), first)
+    plan.destroy()
