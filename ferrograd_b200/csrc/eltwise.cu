@@ -281,7 +281,9 @@ struct VmArgs {
 static_assert(sizeof(VmArgs) <= 4096, "kernel parameters");
 
 constexpr int kVmThreads = 128;
-constexpr int kVmWords = 8;         // 32-bit words of a value that a thread holds: eight f32 elements, or sixteen 16-bit ones in pairs
+// 32-bit words of a value that a thread holds (template parameter W): eight, that is eight f32 elements or sixteen 16-bit ones in
+// pairs; four where the tensor is small (see launch_chain).
+constexpr int kVmWords = 8;
 constexpr int kVmSlotUnits = 2 * kVmThreads;
 
 // A value's words: Lanes<DT> does arithmetic on them.  With 16-bit storage every operation's result is rounded to the type.  The
@@ -292,6 +294,7 @@ constexpr int kVmSlotUnits = 2 * kVmThreads;
 template <int DT> struct Lanes {
     typedef typename std::conditional<DT == FG_DTYPE_F16, __half2, __nv_bfloat162>::type P;
     static constexpr int kE = 2;
+    static constexpr uint32_t kOne = DT == FG_DTYPE_F16 ? 0x3c00u : 0x3f80u;      // 1
     static __device__ __forceinline__ P p(uint32_t u) { return *reinterpret_cast<P*>(&u); }
     static __device__ __forceinline__ uint32_t u(P v) { return *reinterpret_cast<uint32_t*>(&v); }
     static __device__ __forceinline__ float2 f(uint32_t v) {
@@ -328,6 +331,7 @@ template <int DT> struct Lanes {
 };
 template <> struct Lanes<FG_DTYPE_F32> {
     static constexpr int kE = 1;
+    static constexpr uint32_t kOne = 0x3f800000u;
     static __device__ __forceinline__ float f(uint32_t v) { return __uint_as_float(v); }
     static __device__ __forceinline__ uint32_t u(float v) { return __float_as_uint(v); }
     static __device__ __forceinline__ uint32_t all(float v) { return u(v); }
@@ -344,56 +348,63 @@ template <> struct Lanes<FG_DTYPE_F32> {
 };
 
 // Slots are in shared memory (a program is only known at run time, so its values cannot be named registers): a slot holds
-// the words of each thread as two planes of one uint4 per thread, so that every access is a conflict-free 128-bit one.
-__device__ __forceinline__ void slot_ld(const uint4* sm, uint32_t off, uint32_t* o) {
-    const uint4 a = sm[off], b = sm[off + kVmThreads];
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+// the words of each thread as planes of one uint4 per thread, so that every access is a conflict-free 128-bit one.
+template <int W> __device__ __forceinline__ void slot_ld(const uint4* sm, uint32_t off, uint32_t* o) {
+#pragma unroll
+    for (int j = 0; j < W / 4; ++j) {
+        const uint4 a = sm[off + j * kVmThreads];
+        o[4 * j] = a.x; o[4 * j + 1] = a.y; o[4 * j + 2] = a.z; o[4 * j + 3] = a.w;
+    }
 }
-__device__ __forceinline__ void slot_st(uint4* sm, uint32_t off, const uint32_t* v) {
-    sm[off] = make_uint4(v[0], v[1], v[2], v[3]);
-    sm[off + kVmThreads] = make_uint4(v[4], v[5], v[6], v[7]);
+template <int W> __device__ __forceinline__ void slot_st(uint4* sm, uint32_t off, const uint32_t* v) {
+#pragma unroll
+    for (int j = 0; j < W / 4; ++j) sm[off + j * kVmThreads] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 }
 
 // A thread's words of a tensor.  VEC: groups of four elements, kVmThreads groups apart, in a tile that is whole; otherwise
-// single elements, kVmThreads apart, as far as the tensor goes.
-template <int DT, bool VEC>
+// single elements, kVmThreads apart, as far as the tensor goes, and ones beyond it (the quotient of zeros takes the long way
+// round: x / (1 + exp(-x)) * y backward on 100 000 halves 9.2 us, 8.4 with ones).
+template <int DT, bool VEC, int W>
 __device__ __forceinline__ void words_ld(const void* t, uint64_t i, uint64_t n, uint32_t* o) {
     if constexpr (VEC && DT == FG_DTYPE_F32) {
         const uint4* p = reinterpret_cast<const uint4*>(static_cast<const float*>(t) + i);
-        const uint4 a = p[0], b = p[kVmThreads];
-        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+        uint4 a[W / 4];
+#pragma unroll
+        for (int j = 0; j < W / 4; ++j) a[j] = p[j * kVmThreads];
+#pragma unroll
+        for (int j = 0; j < W / 4; ++j) { o[4 * j] = a[j].x; o[4 * j + 1] = a[j].y; o[4 * j + 2] = a[j].z; o[4 * j + 3] = a[j].w; }
     } else if constexpr (VEC) {
         const uint2* p = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(t) + i);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { const uint2 a = p[j * kVmThreads]; o[2 * j] = a.x; o[2 * j + 1] = a.y; }
+        for (int j = 0; j < W / 2; ++j) { const uint2 a = p[j * kVmThreads]; o[2 * j] = a.x; o[2 * j + 1] = a.y; }
     } else if constexpr (DT == FG_DTYPE_F32) {
 #pragma unroll
-        for (int w = 0; w < kVmWords; ++w) o[w] = i + w * kVmThreads < n ? static_cast<const uint32_t*>(t)[i + w * kVmThreads] : 0u;
+        for (int w = 0; w < W; ++w) o[w] = i + w * kVmThreads < n ? static_cast<const uint32_t*>(t)[i + w * kVmThreads] : Lanes<DT>::kOne;
     } else {
 #pragma unroll
-        for (int w = 0; w < kVmWords; ++w) {
+        for (int w = 0; w < W; ++w) {
             const uint64_t e = i + 2 * w * kVmThreads;
-            o[w] = (e < n ? Lanes<DT>::bits(t, e) : 0u) | (e + kVmThreads < n ? Lanes<DT>::bits(t, e + kVmThreads) : 0u) << 16;
+            o[w] = (e < n ? Lanes<DT>::bits(t, e) : Lanes<DT>::kOne) | (e + kVmThreads < n ? Lanes<DT>::bits(t, e + kVmThreads) : Lanes<DT>::kOne) << 16;
         }
     }
 }
-template <int DT, bool VEC>
+template <int DT, bool VEC, int W>
 __device__ __forceinline__ void words_st(void* t, uint64_t i, uint64_t n, const uint32_t* v) {
     if constexpr (VEC && DT == FG_DTYPE_F32) {
         uint4* p = reinterpret_cast<uint4*>(static_cast<float*>(t) + i);
-        p[0] = make_uint4(v[0], v[1], v[2], v[3]);
-        p[kVmThreads] = make_uint4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+        for (int j = 0; j < W / 4; ++j) p[j * kVmThreads] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     } else if constexpr (VEC) {
         uint2* p = reinterpret_cast<uint2*>(static_cast<uint16_t*>(t) + i);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) p[j * kVmThreads] = make_uint2(v[2 * j], v[2 * j + 1]);
+        for (int j = 0; j < W / 2; ++j) p[j * kVmThreads] = make_uint2(v[2 * j], v[2 * j + 1]);
     } else if constexpr (DT == FG_DTYPE_F32) {
 #pragma unroll
-        for (int w = 0; w < kVmWords; ++w)
+        for (int w = 0; w < W; ++w)
             if (i + w * kVmThreads < n) static_cast<uint32_t*>(t)[i + w * kVmThreads] = v[w];
     } else {
 #pragma unroll
-        for (int w = 0; w < kVmWords; ++w) {
+        for (int w = 0; w < W; ++w) {
             const uint64_t e = i + 2 * w * kVmThreads;
             if (e < n) Lanes<DT>::put(t, e, v[w]);
             if (e + kVmThreads < n) Lanes<DT>::put(t, e + kVmThreads, v[w] >> 16);
@@ -409,24 +420,24 @@ __device__ __forceinline__ void words_st(void* t, uint64_t i, uint64_t n, const 
 // Forward and backward: gelu(x * y) + x on 32 Mi f32 257 -> 211 us (3.8 TB/s), x / (1 + exp(-x)) * y on 3 000 001 halves
 // 42.3 -> 21.5 us, with both launches.  Requesting the next tile's words ahead through cp.async lost 6 % (the copies out of the
 // staging cost more issue slots than the waits); sixteen words per thread gain 3 % in f32 and lose 30 % on halves.
-template <int DT, bool VEC>
+template <int DT, bool VEC, int W>
 __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
     typedef Lanes<DT> L;
-    uint32_t v[kVmWords];
+    uint32_t v[W];
 #pragma unroll
-    for (int w = 0; w < kVmWords; ++w) v[w] = 0u;
-#define FG_VM_1(expr) _Pragma("unroll") for (int w = 0; w < kVmWords; ++w) { const uint32_t x = v[w]; v[w] = (expr); } break
+    for (int w = 0; w < W; ++w) v[w] = 0u;
+#define FG_VM_1(expr) _Pragma("unroll") for (int w = 0; w < W; ++w) { const uint32_t x = v[w]; v[w] = (expr); } break
 #define FG_VM_2(expr)                                                                                       \
     {                                                                                                       \
-        uint32_t yy[kVmWords];                                                                              \
-        slot_ld(sm, c.y, yy);                                                                         \
-        _Pragma("unroll") for (int w = 0; w < kVmWords; ++w) { const uint32_t x = v[w], y = yy[w]; v[w] = (expr); } \
+        uint32_t yy[W];                                                                              \
+        slot_ld<W>(sm, c.y, yy);                                                                            \
+        _Pragma("unroll") for (int w = 0; w < W; ++w) { const uint32_t x = v[w], y = yy[w]; v[w] = (expr); } \
     } break
 #pragma unroll 1
     for (int k = 0; k < a.nops; ++k) {
         const uint4 c = a.ops[k];
         const uint32_t flags = c.x;
-        if (flags & kVmFetch) slot_ld(sm, c.z & 0xffffu, v);
+        if (flags & kVmFetch) slot_ld<W>(sm, c.z & 0xffffu, v);
         switch (c.x & 255u) {
             case FG_EW_CONST: {
                 const uint32_t k0 = L::all(__uint_as_float(c.y));
@@ -452,20 +463,20 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
             case VM_G_GELU: FG_VM_2(L::mul(x, L::map(y, [](float p) { return fg_gelu_grad(p); })));
             case VM_G_ELU: FG_VM_2(L::where_ge0(y, x, L::mul(x, L::add(y, L::all(1.0f)))));
             case VM_G_ABS: FG_VM_2(L::where_ge0(y, x, L::neg(x)));
-            case VM_LD: words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
+            case VM_LD: words_ld<DT, VEC, W>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
             case VM_LD2: {                                  // both on their way at once
-                uint32_t yy[kVmWords];
-                words_ld<DT, VEC>(a.ptr[c.x >> 24], i, a.n, yy);
-                words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v);
-                slot_st(sm, c.y, yy);
+                uint32_t yy[W];
+                words_ld<DT, VEC, W>(a.ptr[c.x >> 24], i, a.n, yy);
+                words_ld<DT, VEC, W>(a.ptr[c.x >> 16 & 255u], i, a.n, v);
+                slot_st<W>(sm, c.y, yy);
                 break;
             }
-            case VM_ST: words_st<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
+            case VM_ST: words_st<DT, VEC, W>(a.ptr[c.x >> 16 & 255u], i, a.n, v); break;
             case VM_LDADD: {
-                uint32_t yy[kVmWords];
-                words_ld<DT, VEC>(a.ptr[c.x >> 16 & 255u], i, a.n, yy);
+                uint32_t yy[W];
+                words_ld<DT, VEC, W>(a.ptr[c.x >> 16 & 255u], i, a.n, yy);
 #pragma unroll
-                for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
+                for (int w = 0; w < W; ++w) v[w] = L::add(yy[w], v[w]);
                 break;
             }
             case VM_COPY: break;
@@ -473,36 +484,36 @@ __device__ __forceinline__ void vm_run(const VmArgs& a, uint64_t i, uint4* sm) {
         }
         if (flags & (kVmAdd | kVmKeep)) {
             if (flags & kVmAdd) {
-                uint32_t yy[kVmWords];
-                slot_ld(sm, c.z >> 16, yy);
+                uint32_t yy[W];
+                slot_ld<W>(sm, c.z >> 16, yy);
 #pragma unroll
-                for (int w = 0; w < kVmWords; ++w) v[w] = L::add(yy[w], v[w]);
+                for (int w = 0; w < W; ++w) v[w] = L::add(yy[w], v[w]);
             }
-            if (flags & kVmKeep) slot_st(sm, c.w, v);
+            if (flags & kVmKeep) slot_st<W>(sm, c.w, v);
         }
     }
 #undef FG_VM_1
 #undef FG_VM_2
 }
 
-// A block takes one tile of kVmWords words per thread at a time; block 0 of a vectorised launch has the incomplete last tile
+// A block takes one tile of W words per thread at a time; block 0 of a vectorised launch has the incomplete last tile
 // instead, element by element, so that no other tile needs bounds.
-template <int DT, bool VEC>
+template <int DT, bool VEC, int W>
 __global__ void __launch_bounds__(kVmThreads, 10) chain_kernel(const __grid_constant__ VmArgs a) {
     fg_grid_enter();
     extern __shared__ uint4 chain_smem[];
     uint4* const sm = chain_smem + threadIdx.x;
-    constexpr uint32_t kTile = kVmWords * Lanes<DT>::kE * kVmThreads;
+    constexpr uint32_t kTile = W * Lanes<DT>::kE * kVmThreads;
     if constexpr (VEC) {
         const uint64_t whole = a.n / kTile;
         const uint32_t rest = a.n % kTile != 0;
         if (rest && blockIdx.x == 0) {
-            vm_run<DT, false>(a, whole * kTile + threadIdx.x, sm);
+            vm_run<DT, false, W>(a, whole * kTile + threadIdx.x, sm);
             return;
         }
-        for (uint64_t t = blockIdx.x - rest; t < whole; t += gridDim.x - rest) vm_run<DT, true>(a, t * kTile + threadIdx.x * 4, sm);
+        for (uint64_t t = blockIdx.x - rest; t < whole; t += gridDim.x - rest) vm_run<DT, true, W>(a, t * kTile + threadIdx.x * 4, sm);
     } else {
-        for (uint64_t t = blockIdx.x; t * kTile < a.n; t += gridDim.x) vm_run<DT, false>(a, t * kTile + threadIdx.x, sm);
+        for (uint64_t t = blockIdx.x; t * kTile < a.n; t += gridDim.x) vm_run<DT, false, W>(a, t * kTile + threadIdx.x, sm);
     }
 }
 
@@ -719,27 +730,39 @@ __global__ void __launch_bounds__(256) convert_kernel(const void* __restrict__ s
 constexpr int kSlotBytes = kVmSlotUnits * (int)sizeof(uint4);
 constexpr int kChainSmemMax = 2 * FG_EW_MAX_INSTR * kSlotBytes;
 int32_t launch_chain(fg_ctx* ctx, int dtype, VmBuilder& b, VmArgs& a, double bytes) {
-    static std::atomic<uint64_t> done[3][2];
+    static std::atomic<uint64_t> done[3][2][2];
     const uint64_t bit = 1ull << (ctx->device & 63);
     const size_t smem = (size_t)b.finish(&a) * kSlotBytes;
     if (smem > (size_t)kChainSmemMax) return fg_fail(ctx, FG_ERR_INTERNAL, "eltwise chain: too many live values");
-    auto of_type = [&](auto vec) {
+    // As many blocks as an SM holds at once (ten by registers, fewer when the slots fill the shared memory), each with the same
+    // number of tiles: a grid of sixteen per SM ran as one full wave and a second of three quarters.
+    const size_t fit = (220u * 1024u) / (smem + 1024);
+    const uint64_t per_sm = fit < 1 ? 1 : fit > 10 ? 10 : fit, cap_sm = (uint64_t)ctx->sm_count * per_sm;
+    // Small tensors: a thread's elements come one after the other and the SMs are half empty, so four words each while that makes
+    // five blocks per SM or fewer, two for a program of one operation, which waits for its loads.  Us with four words and with
+    // eight: x / (1 + exp(-x)) * y backward 8.4 and 14.4 on 100 000 halves, 8.8 and 11.3 on 757 760 (five blocks per SM), 10.0 and 11.8
+    // on 1 Mi, 27 and 24 on 3 M; x + y 1.9 and 2.1 on 300 001, 2.1 and 2.0 on 500 000; in f32 gelu(x * y) + x forward 2.2 and 2.4 on
+    // 100 000, 2.6 and 2.6 on 300 001, 3.3 and 3.0 on 757 760.
+    const uint64_t blocks = a.nops <= 4 ? 2 : per_sm < 5 ? per_sm : 5;
+    const bool few = a.n <= (uint64_t)ctx->sm_count * blocks * (kVmWords / 2) * (dtype == FG_DTYPE_F32 ? 1 : 2) * kVmThreads;
+    const int words = few ? kVmWords / 2 : kVmWords;
+    auto of_type = [&](auto vec, auto small) {
         constexpr bool V = decltype(vec)::value;
-        return dtype == FG_DTYPE_F32 ? chain_kernel<FG_DTYPE_F32, V> : dtype == FG_DTYPE_F16 ? chain_kernel<FG_DTYPE_F16, V> : chain_kernel<FG_DTYPE_BF16, V>;
+        constexpr int W = decltype(small)::value ? kVmWords / 2 : kVmWords;
+        return dtype == FG_DTYPE_F32 ? chain_kernel<FG_DTYPE_F32, V, W> : dtype == FG_DTYPE_F16 ? chain_kernel<FG_DTYPE_F16, V, W> : chain_kernel<FG_DTYPE_BF16, V, W>;
     };
-    auto kernel = a.vec ? of_type(std::true_type{}) : of_type(std::false_type{});
-    std::atomic<uint64_t>& set = done[dtype][a.vec ? 1 : 0];
+    const std::true_type yes{};
+    const std::false_type no{};
+    auto kernel = a.vec ? (few ? of_type(yes, yes) : of_type(yes, no)) : few ? of_type(no, yes) : of_type(no, no);
+    std::atomic<uint64_t>& set = done[dtype][a.vec ? 1 : 0][few ? 1 : 0];
     if (!(set.load(std::memory_order_acquire) & bit)) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmemMax);
         if (e != cudaSuccess) return fg_fail_cuda(ctx, FG_ERR_INTERNAL, "cudaFuncSetAttribute(chain kernel)", e);
         set.fetch_or(bit, std::memory_order_release);
     }
-    // As many blocks as an SM holds at once (ten by registers, fewer when the slots fill the shared memory), each with the same
-    // number of tiles: a grid of sixteen per SM ran as one full wave and a second of three quarters.
-    const size_t fit = (220u * 1024u) / (smem + 1024);
-    const uint64_t tile = (uint64_t)kVmWords * (dtype == FG_DTYPE_F32 ? 1 : 2) * kVmThreads;
+    const uint64_t tile = (uint64_t)words * (dtype == FG_DTYPE_F32 ? 1 : 2) * kVmThreads;
     const uint64_t rest = a.vec && a.n % tile ? 1 : 0, tiles = a.vec ? a.n / tile : (a.n + tile - 1) / tile;
-    const uint64_t cap = (uint64_t)ctx->sm_count * (fit < 1 ? 1 : fit > 10 ? 10 : fit) - rest;
+    const uint64_t cap = cap_sm - rest;
     const uint64_t rounds = tiles ? (tiles + cap - 1) / cap : 1;
     const int grid = (int)((tiles + rounds - 1) / rounds + rest);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_ELTWISE, bytes);

@@ -167,3 +167,34 @@ def test_packed_arithmetic_rounds_as_single_steps_do(ctx, dtype, n, shift):
     ctx.sync()
     adj = gf * (r(xf * yf) > 0).float()
     assert same(dx.cpu()[shift:], (adj * yf).to(td)) and same(dy.cpu()[shift:], (adj * xf).to(td))
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("per_sm,per_block", [(2, 4), (5, 4)])
+def test_threads_with_four_words_and_with_eight_do_the_same(ctx, dtype, shift, per_sm, per_block):
+    # one element below, at and above the size up to which a thread has four words (two or five blocks per SM): the same elements
+    # have the same results, forward and backward, whatever the split
+    import torch
+    td = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[dtype]
+    edge = torch.cuda.get_device_properties(0).multi_processor_count * per_sm * 128 * per_block * (1 if dtype == "f32" else 2)
+    prog = [("input", 0, 0, 0.0), ("input", 1, 0, 0.0), ("add", 0, 1, 0.0)]
+    if per_sm == 5:
+        prog = prog[:2] + [("exp", 0, 0, 0.0), ("const", 0, 0, 1.5), ("add", 2, 3, 0.0), ("div", 1, 4, 0.0), ("gelu", 5, 0, 0.0), ("mul", 6, 0, 0.0)]
+    gen = torch.Generator().manual_seed(edge + shift)
+    place = lambda v: torch.cat([torch.zeros(shift, dtype=td), v.to(td)]).cuda()          # noqa: E731
+    x, y, g = (place(torch.randn(edge + 1, generator=gen)) for _ in range(3))
+    p = lambda v: v.data_ptr() + shift * v.element_size()                                 # noqa: E731
+    seen = []
+    for n in (edge - 1, edge, edge + 1):
+        out, dx, dy = (torch.full((edge + 1 + shift,), 7.0, dtype=td, device="cuda") for _ in range(3))
+        torch.cuda.synchronize()
+        ctx.eltwise_chain_fwd(prog, [p(x), p(y)], p(out), n, dtype=dtype)
+        ctx.eltwise_chain_bwd(prog, [p(x), p(y)], p(g), [p(dx), p(dy)], n, dtype=dtype)
+        ctx.sync()
+        for v in (out, dx, dy):
+            assert (v[shift + n:] == 7.0).all() and (v[:shift] == 7.0).all()
+        seen.append([v[shift:shift + edge - 1].clone() for v in (out, dx, dy)])
+    assert all(torch.equal(a, b) for a, b in zip(seen[0], seen[1])) and all(torch.equal(a, b) for a, b in zip(seen[0], seen[2]))
+    if per_sm == 2:
+        assert torch.equal(seen[0][0], (x + y)[shift:shift + edge - 1])
