@@ -19,7 +19,8 @@ inline uint64_t fg_sms_beside(int sms, bool exchange, int reserved) { return (ui
 inline uint64_t conv_grid(uint64_t units, uint32_t split, uint64_t sms) { return split > 1 ? units * split : units < sms ? units : sms; }
 
 // Estimated SM cycles of one launch for one or two products (the one with the longer k first) on `sms` SMs, from costs fitted to
-// whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones, storing a tile 2.7 and 1.5 us (hidden but for the last one), 3.5 us of
+// whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones (0.34 - 0.37 with a long k), storing a tile 2.7
+// and 1.5 us (hidden but for the last one), 3.5 us of
 // set-up and first loads, 2 - 3 us for the shares' sums to meet; where a ragged N is stored word by word 1.5 us more, and 6 us
 // divided among the shares.  clusters(bn, split): clusters of `split` CTAs that run at once, below one if there are none.
 template <class Clusters>
