@@ -383,6 +383,52 @@ int32_t fg_gemm_simt_launch(fg_ctx* ctx, int transA, int transB, uint32_t M, uin
 int32_t fg_gemm_simt_batched_launch(fg_ctx* ctx, int transA, int transB, uint32_t batch, uint32_t M, uint32_t N, uint32_t K,
                                     const float* A, uint64_t sA, const float* B, uint64_t sB, float* C, uint64_t sC,
                                     const float* bias, int act, float* preact_out);
+// Does the exact path take its 64 x 64 tiles for these products?
+bool fg_gemm_simt_large(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t batch);
+// dB = Aᵀ·dZ and dA = dZ·Bᵀ of a batch in one launch, where fg_gemm_simt_large says no for both.
+int32_t fg_gemm_simt_batched_bwd_launch(fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, const float* A, uint64_t sA, const float* B,
+                                        uint64_t sB, const float* dZ, uint64_t sC, float* dA, float* dB);
+// Do two ranges of bytes overlap (NULL: no)?
+bool fg_ranges_meet(const void* p, uint64_t np, const void* q, uint64_t nq);
+// One product of the FMA kernel: C[M,N] = op(A)[M,K] · op(B)[K,N], operands dense as they are stored (ta: A is [K,M], tb: B is
+// [N,K]), batch strides in elements.  All pointers but A, B and C may be NULL.
+struct FgFmaOp {
+    int ta, tb;
+    uint32_t M, N, K;
+    const float *A, *B;
+    float* C;
+    const float* factor;              // ta xor tb: the operand that is not transposed is x * act'(factor)
+    int factor_act;
+    const float* bias;                // C = act(sum + bias), or (sum + bias) * act'(mul_saved)
+    int act;
+    float* preact;
+    const float* mul_saved;
+    int mul_act;
+    __nv_bfloat16* pairs;             // of C
+    uint64_t pairs_stride;
+    float *colsum_b, *colsum_c;       // [N]: sums over k of the B operand (ta only), over the rows of C
+    uint64_t sA, sB, sC;
+};
+// One product, or two in one launch (the first with ta, the second with tb).  in_order: every sum is one chain of FMAs in the order of
+// k, the exact path's results.  Room in the arena for one row of C's column sums per 32 rows.
+int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch, bool in_order);
+// A layer's backward pass with it: dZ = dZ * act'(factor); dB, dbias; the exchange; dA (* act'(mul_saved), pairs, column sums).
+struct FgFmaBwd {
+    uint32_t M, N, K;
+    const float *A, *B, *dZ, *factor;
+    int factor_act;
+    float *dA, *dB, *dbias;
+    const float* mul_saved;
+    int mul_act;
+    __nv_bfloat16* pairs;
+    uint64_t pairs_stride;
+    float* below_dbias;
+    float* exch_buf;
+    uint64_t exch_count;
+};
+int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b);
+// Does the backward pass of this layer sum dZ's columns on its way (fg_gemm_bwd_paired_f32's dbias costs nothing)?
+bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K);
 uint64_t fg_gemm_skinny_scratch_bytes(uint32_t M, uint32_t N, uint32_t K);   // enough for any one skinny launch
 int32_t fg_gemm_skinny_n_launch(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, const float* A, const float* B, float* C,
                                 const float* bias, int act, float* preact_out);

@@ -5,8 +5,7 @@
 // out = fmaf(As[ly][i], Bs[i][lx], out) over 16-wide k tiles), so results are bit-identical
 // to a sequential-k f32 FMA chain.  Unlike the reference (no bounds checks, shapes must be
 // multiples of 16: crates/fused_gpu/src/dispatch/backend/mod.rs:617-619) any M, N, K is
-// accepted.  Used for small shapes (the 2->16->2 MLP), as the on-device exact reference
-// for the tensor-core path, and when FG_GEMM_SIMT is requested.
+// accepted.  The on-device exact reference for the other kernels: it runs when FG_GEMM_SIMT is requested.
 //
 // TM x TN output tile per CTA, a thread owns RPT rows x 4 columns, k tiles of 32 through two shared-memory buffers.
 #include <atomic>
@@ -20,24 +19,25 @@ constexpr int TK = 32;
 // The order of a sum is fixed, so K cannot be split and what counts is the time per k tile: the next tile's words are
 // requested before this one is multiplied, and a tile costs one barrier (384 x 256 x 10: 21.4 -> 6.9 us, 64 x 16 x 2:
 // 4.8 -> 2.5 us against unpipelined 64 x 64 x 16 tiles).  Which tile: see fg_gemm_simt_batched_launch.
+// `tile` is the block's number among the column and row tiles, `z` its matrix of a batch (the reference puts the batch index in the
+// grid's z: crates/fused_gpu/src/dispatch/backend/kernel/forward.rs:159-190); the strides are in elements.
+template <int TM, int TN>
+struct SimtBuffers {
+    float a[2][TK][TM + 4], b[2][TK][TN + 4];
+};
 template <bool TA, bool TB, int TM, int TN, int RPT>
-__global__ void __launch_bounds__(TM * TN / (4 * RPT)) gemm_simt_kernel(uint32_t M, uint32_t N, uint32_t K,
-                                                        const float* __restrict__ A, const float* __restrict__ B,
-                                                        float* __restrict__ C, const float* __restrict__ bias, int act,
-                                                        float* __restrict__ preact, uint64_t sA, uint64_t sB, uint64_t sC) {
-    fg_grid_enter();
+__device__ __forceinline__ void simt_tile(uint32_t M, uint32_t N, uint32_t K, const float* __restrict__ A, const float* __restrict__ B,
+                                          float* __restrict__ C, const float* __restrict__ bias, int act, float* __restrict__ preact,
+                                          uint64_t sA, uint64_t sB, uint64_t sC, uint32_t m0, uint32_t n0, uint32_t z, SimtBuffers<TM, TN>& sm) {
     constexpr int T = TM * TN / (4 * RPT), NA = TM * TK / T, NB = TN * TK / T;
     static_assert(RPT == 1 || RPT == 4, "a thread's rows are read as one word or one float4");
-    __shared__ __align__(16) float As[2][TK][TM + 4];
-    __shared__ __align__(16) float Bs[2][TK][TN + 4];
-    // blockIdx.z is the matrix of a batch (the reference puts the batch index in the grid's z too:
-    // crates/fused_gpu/src/dispatch/backend/kernel/forward.rs:159-190); the strides are in elements
-    A += blockIdx.z * sA;
-    B += blockIdx.z * sB;
-    C += blockIdx.z * sC;
-    if (preact) preact += blockIdx.z * sC;
+    auto& As = sm.a;
+    auto& Bs = sm.b;
+    A += z * sA;
+    B += z * sB;
+    C += z * sC;
+    if (preact) preact += z * sC;
     const int tx = threadIdx.x % (TN / 4), ty = threadIdx.x / (TN / 4);
-    const uint32_t m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     float ra[NA], rb[NB];
     // opA[m0+m, k0+k] and opB[k0+k, n0+n], lanes along the stored tensor's contiguous index
     auto fetch = [&](uint32_t k0) {
@@ -106,6 +106,40 @@ __global__ void __launch_bounds__(TM * TN / (4 * RPT)) gemm_simt_kernel(uint32_t
             if (preact) preact[o] = z;
             C[o] = fg_act_fwd(act, z);
         }
+    }
+}
+
+template <bool TA, bool TB, int TM, int TN, int RPT>
+__global__ void __launch_bounds__(TM * TN / (4 * RPT)) gemm_simt_kernel(uint32_t M, uint32_t N, uint32_t K,
+                                                        const float* __restrict__ A, const float* __restrict__ B,
+                                                        float* __restrict__ C, const float* __restrict__ bias, int act,
+                                                        float* __restrict__ preact, uint64_t sA, uint64_t sB, uint64_t sC) {
+    fg_grid_enter();
+    __shared__ __align__(16) SimtBuffers<TM, TN> sm;
+    simt_tile<TA, TB, TM, TN, RPT>(M, N, K, A, B, C, bias, act, preact, sA, sB, sC, blockIdx.y * TM, blockIdx.x * TN, blockIdx.z, sm);
+}
+
+// Both gradients of the matrices of a batch, dB = Aᵀ·dZ and dA = dZ·Bᵀ for A [M,K], B [K,N]: the blocks of dB first.  Either has too few
+// tiles to fill the SMs, so that one launch takes as long as the longer of the two (16 x (128 x 120 x 128): 17.5 -> 14.5 us, 2 x (512 x 512 x 15) 21.6 -> 11.8).
+struct SimtBwd {
+    uint32_t M, N, K;
+    const float *A, *B, *dZ;
+    float *dA, *dB;
+    uint64_t sA, sB, sC;
+    uint32_t cols_b, tiles_b, blocks_b, cols_a, tiles_a;      // column tiles, tiles of a matrix, blocks of the whole batch
+};
+template <int TM, int TN, int RPT>
+__global__ void __launch_bounds__(TM * TN / (4 * RPT)) gemm_simt_bwd_kernel(const SimtBwd p) {
+    fg_grid_enter();
+    __shared__ __align__(16) SimtBuffers<TM, TN> sm;
+    if (blockIdx.x < p.blocks_b) {
+        const uint32_t z = blockIdx.x / p.tiles_b, t = blockIdx.x % p.tiles_b;
+        simt_tile<true, false, TM, TN, RPT>(p.K, p.N, p.M, p.A, p.dZ, p.dB, nullptr, FG_ACT_NONE, nullptr, p.sA, p.sC, p.sB, t / p.cols_b * TM,
+                                            t % p.cols_b * TN, z, sm);
+    } else {
+        const uint32_t u = blockIdx.x - p.blocks_b, z = u / p.tiles_a, t = u % p.tiles_a;
+        simt_tile<false, true, TM, TN, RPT>(p.M, p.K, p.N, p.dZ, p.B, p.dA, nullptr, FG_ACT_NONE, nullptr, p.sC, p.sB, p.sA, t / p.cols_a * TM,
+                                            t % p.cols_a * TN, z, sm);
     }
 }
 
@@ -666,17 +700,32 @@ int32_t fg_gemm_skinny_tn_launch(fg_ctx* ctx, uint32_t M, uint32_t Kd, uint32_t 
     return FG_OK;
 }
 
+// Up to four 16 x 32 tiles an SM, as many threads as two 64 x 64 tiles, take no longer than one of those (per 4096 of k:
+// 98 us for one, 123, 168 and 223 for two to four, 220 for one of 64 x 64); beyond that the larger tiles' arithmetic per
+// word read counts (768 x 768 x 2048: 117 us against 221).  Both add in the same order.
+bool fg_gemm_simt_large(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t batch) {
+    const uint64_t tiles16 = (uint64_t)((M + 15) / 16) * ((N + 31) / 32) * batch;
+    return tiles16 > 4ull * (uint64_t)ctx->sm_count || M > 65535u * 16u;
+}
+
+int32_t fg_gemm_simt_batched_bwd_launch(fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, const float* A, uint64_t sA, const float* B,
+                                        uint64_t sB, const float* dZ, uint64_t sC, float* dA, float* dB) {
+    SimtBwd p{M, N, K, A, B, dZ, dA, dB, sA, sB, sC, (N + 31) / 32, 0, 0, (K + 31) / 32, 0};
+    p.tiles_b = p.cols_b * ((K + 15) / 16);
+    p.tiles_a = p.cols_a * ((M + 15) / 16);
+    p.blocks_b = p.tiles_b * batch;      // (small products: at most four tiles an SM each)
+    fg_launch(ctx, gemm_simt_bwd_kernel<16, 32, 1>, p.blocks_b + p.tiles_a * batch, 128, 0, p);
+    FG_LAUNCHED(ctx);
+    return FG_OK;
+}
+
 int32_t fg_gemm_simt_batched_launch(fg_ctx* ctx, int transA, int transB, uint32_t batch, uint32_t M, uint32_t N, uint32_t K,
                                     const float* A, uint64_t sA, const float* B, uint64_t sB, float* C, uint64_t sC,
                                     const float* bias, int act, float* preact_out) {
     if (M > 65535u * 64u) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: M too large");
     if (batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "SIMT GEMM: more than 65535 matrices in a batch");
     if (batch == 0) return FG_OK;
-    // Up to four 16 x 32 tiles an SM, as many threads as two 64 x 64 tiles, take no longer than one of those (per 4096 of k:
-    // 98 us for one, 123, 168 and 223 for two to four, 220 for one of 64 x 64); beyond that the larger tiles' arithmetic per
-    // word read counts (768 x 768 x 2048: 117 us against 221).  Both add in the same order.
-    const uint64_t tiles16 = (uint64_t)((M + 15) / 16) * ((N + 31) / 32) * batch;
-    const bool large = tiles16 > 4ull * (uint64_t)ctx->sm_count || M > 65535u * 16u;
+    const bool large = fg_gemm_simt_large(ctx, M, N, batch);
     if (large) launch_simt_tile<64, 64, 4>(ctx, transA, transB, batch, M, N, K, A, sA, B, sB, C, sC, bias, act, preact_out);
     else launch_simt_tile<16, 32, 1>(ctx, transA, transB, batch, M, N, K, A, sA, B, sB, C, sC, bias, act, preact_out);
     FG_LAUNCHED(ctx);

@@ -2461,6 +2461,12 @@ int32_t gemm_fwd_core(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
     const int path = pick_path(ctx, mode, M, N, K);
     // The result's pairs, when no GEMM epilogue wrote them.
     auto pairs_after = [&]() -> int32_t { return c_pairs ? launch_pairs(ctx, C, mn, c_pairs, c_stride) : FG_OK; };
+    if (path == 0 && mode == FG_GEMM_AUTO) {
+        FgFmaOp o{};
+        o.ta = transA; o.tb = transB; o.M = M; o.N = N; o.K = K; o.A = A.x; o.B = B.x; o.C = C;
+        o.bias = bias; o.act = act; o.preact = preact_out; o.pairs = c_pairs; o.pairs_stride = c_stride;
+        return fg_gemm_fma_launch(ctx, &o, 1, 1, false);
+    }
     if (path == 0) {
         int32_t s = fg_gemm_simt_launch(ctx, transA, transB, M, N, K, A.x, B.x, C, bias, act, preact_out);
         return s != FG_OK ? s : pairs_after();
@@ -2598,12 +2604,18 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
     const uint64_t mn = (uint64_t)M * N;
 
     if (path == 0) {
-        // Exact path: materialise dZ, then two SIMT GEMMs.
         const float* dz = dY;
         {
             uint64_t need = mn * 4 + (uint64_t)((M + 255) / 256) * N * 4 + 1024;
             { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
         }
+        if (mode == FG_GEMM_AUTO && !dZ_out) {
+            FgFmaBwd b{};
+            b.M = M; b.N = N; b.K = K; b.A = A; b.B = B; b.dZ = dY; b.factor = fuse ? saved : nullptr; b.factor_act = act;
+            b.dA = dA; b.dB = dB; b.dbias = dbias; b.exch_buf = exch_buf; b.exch_count = exch_count;
+            return fg_gemm_fma_bwd(ctx, b);
+        }
+        // Exact path: materialise dZ, then two SIMT GEMMs.
         if (fuse || dZ_out) {
             float* buf = dZ_out;
             if (!buf) {
@@ -2811,16 +2823,37 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
 }
 
 int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, float* dB,
-                             float* dA, PairedOut o, float* dbias_prev, float* exch_buf, uint64_t exch_count) {
+                             float* dA, PairedOut o, float* dbias, float* dbias_prev, float* exch_buf, uint64_t exch_count) {
     int32_t s;
     void* p;
+    // Where dA lies over the saved tensor its factor comes from a copy on the routes that apply it elsewhere than they read it (in
+    // the room of the pairs, which those routes do not make).
+    auto saved_apart = [&]() -> int32_t {
+        const uint64_t bytes = (uint64_t)M * K * 4;
+        if (!o.mul_saved || !fg_ranges_meet(dA, bytes, o.mul_saved, bytes)) return FG_OK;
+        if ((s = fg_ws_alloc(ctx, bytes, &p)) != FG_OK) return s;
+        FG_CUDA(ctx, FG_ERR_FAILED_BUFFER_COPY, cudaMemcpyAsync(p, o.mul_saved, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        o.mul_saved = (const float*)p;
+        return FG_OK;
+    };
+    const bool narrow = N <= 16, exact = pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 0;
+    const BwdRoutes rt = narrow ? BwdRoutes{} : pick_bwd_routes(ctx, M, N, K, A, B, dZ, dB, dA, o.mul_saved);
+    if (exact && (narrow || rt.planes)) {
+        if (dA && o.mul_saved != dA && (s = saved_apart()) != FG_OK) return s;      // (an element is read and written by one thread)
+        FgFmaBwd b{};
+        b.M = M; b.N = N; b.K = K; b.A = A.x; b.B = B.x; b.dZ = dZ.x; b.dA = dA; b.dB = dB; b.dbias = dbias;
+        b.mul_saved = o.mul_saved; b.mul_act = o.mul_act; b.pairs = o.pairs; b.pairs_stride = o.stride; b.below_dbias = dbias_prev;
+        b.exch_buf = exch_buf; b.exch_count = exch_count;
+        return fg_gemm_fma_bwd(ctx, b);
+    }
+    if (dbias && (s = fg_colsum_launch(ctx, M, N, dZ.x, dbias)) != FG_OK) return s;
     const uint32_t cs_chunks = (M + 31) / 32;
     float* cs_part = nullptr;
     if (dA && dbias_prev) {
         if ((s = fg_ws_alloc(ctx, (uint64_t)colsum_room(M, N) * K * 4, &p)) != FG_OK) return s;
         cs_part = (float*)p;
     }
-    if (N <= 16) {
+    if (narrow) {
         // narrow layer: plain-FMA streaming kernels on the tensors themselves
         if (dB && (s = fg_gemm_skinny_tn_launch(ctx, M, K, N, A.x, dZ.x, dB)) != FG_OK) return s;
         if (exch_buf && (s = fg_allreduce_sum_f32(ctx, exch_buf, exch_count)) != FG_OK) return s;
@@ -2832,18 +2865,8 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         }
         return FG_OK;
     }
-    const BwdRoutes rt = pick_bwd_routes(ctx, M, N, K, A, B, dZ, dB, dA, o.mul_saved);
-    if (dA && o.mul_saved && (rt.planes || rt.dA.kind == kRoutePlanes)) {
-        // There the factor is applied after the whole of dA has been written: where dA lies over the saved tensor, from a copy (in
-        // the room of the pairs, which this route does not make).
-        const uint64_t bytes = (uint64_t)M * K * 4;
-        const uintptr_t d = reinterpret_cast<uintptr_t>(dA), v = reinterpret_cast<uintptr_t>(o.mul_saved);
-        if (d < v + bytes && v < d + bytes) {
-            if ((s = fg_ws_alloc(ctx, bytes, &p)) != FG_OK) return s;
-            FG_CUDA(ctx, FG_ERR_FAILED_BUFFER_COPY, cudaMemcpyAsync(p, o.mul_saved, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-            o.mul_saved = (const float*)p;
-        }
-    }
+    // There the factor is applied after the whole of dA has been written.
+    if (dA && (rt.planes || rt.dA.kind == kRoutePlanes) && (s = saved_apart()) != FG_OK) return s;
     if (!rt.planes && (dA || dB)) {
         PairedOut po = o;
         po.colsum_part = cs_part;
@@ -2872,6 +2895,13 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
 }
 
 }  // namespace
+
+bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K) {
+    if (pick_path(ctx, FG_GEMM_AUTO, M, N, K) != 0) return false;
+    float* const any = reinterpret_cast<float*>(uintptr_t(256));      // only the alignment counts
+    const PairedArg t{any, any, 0};
+    return N <= 16 || (pick_bwd_routes(ctx, M, N, K, t, t, t, any, any, any).planes && pick_bwd_routes(ctx, M, N, K, t, t, t, any, nullptr, nullptr).planes);
+}
 
 uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K) {
     if (N <= 16) return 0;
@@ -2983,6 +3013,11 @@ bool batch_route_open(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, u
            (N > 16 || mode != FG_GEMM_AUTO);
 }
 
+// Small matrices: the sums of a batch come in the order of k from either kernel.  Where the exact path would take its large tiles the FMA
+// kernel's are the faster ones forward and for both gradients together (31 x (60 x 500 x 500) 45 -> 34 and 92 -> 76 us), not for a
+// gradient by itself (dB of 30 x (100 x 100 x 400) 17.7 us, 20.7 with it) nor for a short k (24 x (182 x 151 x 30) 6.2, 7.6 with it).
+bool batch_large(const fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t M, uint32_t N) { return mode == FG_GEMM_AUTO && fg_gemm_simt_large(ctx, M, N, batch); }
+
 // Matrices per launch: the whole batch if the scratch arena has room for it or can be grown (64 x (512 x 512 x 512) backward with
 // an activation: 323 us, 360 in parts).  Otherwise (out of memory, a recording whose arena was sized for less) as many as find
 // room in the arena or in what the loop over the matrices would make of it (`loop`).  need(t): bytes for t matrices.
@@ -3034,15 +3069,11 @@ int32_t fg_gemm_bwd_paired_f32(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, 
     if (exch_buf && !ctx->comm) return fg_fail(ctx, FG_ERR_NOT_INITIALIZED, "fg_gemm_bwd_paired_f32: call fg_comm_init first");
     FG_REQUIRE(ctx, !exch_buf || exch_count > 0, "fg_gemm_bwd_paired_f32: nothing to exchange");
     { int32_t s0 = fg_ws_ensure(ctx, bwd_paired_need(M, N, K)); if (s0 != FG_OK) return s0; }
-    if (dbias) {
-        const int32_t s0 = fg_colsum_launch(ctx, M, N, dZ, dbias);
-        if (s0 != FG_OK) return s0;
-    }
     const bool mul = below_act != FG_ACT_NONE;
     return gemm_bwd_paired_core(ctx, M, N, K, PairedArg{A, A_pairs, A_stride}, PairedArg{B, B_pairs, B_stride},
                                 PairedArg{dZ, dZ_pairs, dZ_stride}, dB, dA,
                                 PairedOut{(__nv_bfloat16*)dA_pairs_out, dA_stride, mul ? below_saved : nullptr, below_act, nullptr},
-                                below_dbias, exch_buf, exch_count);
+                                dbias, below_dbias, exch_buf, exch_count);
 }
 
 // Batched forms: `batch` independent products, operand t at base + t*stride (strides in elements).
@@ -3061,6 +3092,12 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
                "fg_gemm_batched_f32: a stride is smaller than its matrix (for one B shared by all products, "
                "call fg_gemm_f32 with batch*M rows)");
     if (batch == 0 || (uint64_t)M * N == 0) return FG_OK;
+    if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && K >= 64 && batch_large(ctx, mode, batch, M, N)) {
+        FgFmaOp o{};
+        o.M = M; o.N = N; o.K = K; o.A = A; o.B = B; o.C = C; o.bias = bias; o.act = act; o.preact = preact_out;
+        o.sA = strideA; o.sB = strideB; o.sC = strideC;
+        return fg_gemm_fma_launch(ctx, &o, 1, batch, true);
+    }
     if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && K > 0)
         return fg_gemm_simt_batched_launch(ctx, 0, 0, batch, M, N, K, A, strideA, B, strideB, C, strideC, bias, act, preact_out);
     if (batch_route_open(ctx, mode, M, N, K)) {
@@ -3131,8 +3168,8 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
     FG_REQUIRE(ctx, strideA >= (uint64_t)M * K && strideB >= (uint64_t)K * N && strideC >= (uint64_t)M * N,
                "fg_gemm_batched_bwd_f32: a stride is smaller than its matrix");
     if (batch == 0 || (uint64_t)M * N == 0 || (!dA && !dB)) return FG_OK;
-    if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && strideC == (uint64_t)M * N) {
-        // three launches for the whole batch: dZ = dY * act'(saved), dB[t] = A[t]^T dZ[t], dA[t] = dZ[t] B[t]^T
+    if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && (strideC == (uint64_t)M * N || (act == FG_ACT_NONE && K > 0))) {
+        // dZ = dY * act'(saved) for the whole batch, then dB[t] = A[t]^T dZ[t] and dA[t] = dZ[t] B[t]^T: sums in the order of k
         const float* dz = dY;
         if (act != FG_ACT_NONE) {
             const uint64_t n = (uint64_t)batch * M * N;
@@ -3144,11 +3181,21 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
             dz = (const float*)p;
         }
         int32_t s;
-        if (dB && (s = fg_gemm_simt_batched_launch(ctx, 1, 0, batch, K, N, M, A, strideA, dz, strideC, dB, strideB, nullptr,
-                                                   FG_ACT_NONE, nullptr)) != FG_OK) return s;
-        if (dA && (s = fg_gemm_simt_batched_launch(ctx, 0, 1, batch, M, K, N, dz, strideC, B, strideB, dA, strideA, nullptr,
-                                                   FG_ACT_NONE, nullptr)) != FG_OK) return s;
-        return FG_OK;
+        const bool large_b = batch_large(ctx, mode, batch, K, N), large_a = batch_large(ctx, mode, batch, M, K);
+        FgFmaOp ops[2] = {};
+        FgFmaOp &w = ops[0], &x = ops[1];
+        w.ta = 1; w.M = K; w.N = N; w.K = M; w.A = A; w.B = dz; w.C = dB; w.sA = strideA; w.sB = strideC; w.sC = strideB;
+        x.tb = 1; x.M = M; x.N = K; x.K = N; x.A = dz; x.B = B; x.C = dA; x.sA = strideC; x.sB = strideB; x.sC = strideA;
+        // one launch for both where nothing was formed before, unless a gradient lies over what the other product reads
+        const uint64_t na = ((batch - 1) * strideA + (uint64_t)M * K) * 4, nb = ((batch - 1) * strideB + (uint64_t)K * N) * 4,
+                       nc = ((batch - 1) * strideC + (uint64_t)M * N) * 4;
+        auto over = [&](const void* p, uint64_t n) { return fg_ranges_meet(p, n, A, na) || fg_ranges_meet(p, n, B, nb) || fg_ranges_meet(p, n, dz, nc); };
+        if (dA && dB && act == FG_ACT_NONE && mode == FG_GEMM_AUTO && large_a == large_b && !over(dA, na) && !over(dB, nb)) {
+            return large_a ? fg_gemm_fma_launch(ctx, ops, 2, batch, true)
+                           : fg_gemm_simt_batched_bwd_launch(ctx, batch, M, N, K, A, strideA, B, strideB, dz, strideC, dA, dB);
+        }
+        if (dB && (s = fg_gemm_simt_batched_launch(ctx, 1, 0, batch, K, N, M, A, strideA, dz, strideC, dB, strideB, nullptr, FG_ACT_NONE, nullptr)) != FG_OK) return s;
+        return dA ? fg_gemm_simt_batched_launch(ctx, 0, 1, batch, M, K, N, dz, strideC, B, strideB, dA, strideA, nullptr, FG_ACT_NONE, nullptr) : FG_OK;
     }
     if (batch_route_open(ctx, mode, M, N, K)) {
         const bool n8 = N % 8 == 0 && K % 8 == 0;
