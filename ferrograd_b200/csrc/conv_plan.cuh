@@ -18,25 +18,35 @@ inline uint64_t fg_sms_beside(int sms, bool exchange, int reserved) { return (ui
 // CTAs of a launch: one for each K-share, or no more than SMs that walk the units.
 inline uint64_t conv_grid(uint64_t units, uint32_t split, uint64_t sms) { return split > 1 ? units * split : units < sms ? units : sms; }
 
-// Estimated SM cycles of one launch for one or two products (the one with the longer k first) on `sms` SMs, from costs fitted to
-// whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones (0.34 - 0.37 with a long k), storing a tile 2.7
-// and 1.5 us (hidden but for the last one), 3.5 us of
-// set-up and first loads, 2 - 3 us for the shares' sums to meet; where a ragged N is stored word by word 1.5 us more, and 6 us
-// divided among the shares.  clusters(bn, split): clusters of `split` CTAs that run at once, below one if there are none.
+// What a launch is estimated by, in SM cycles: with tiles 128 and 64 wide, a k-block of `kblock`, storing a tile (hidden but for the
+// last one), what storing a ragged N adds, and what it adds to a meeting of shares, divided among them; set-up and first loads, and
+// the meeting itself.
+struct ConvCosts {
+    uint32_t kblock;
+    double kb[2], store[2], ragged[2], ragged_shares[2], around, meet;
+};
+// The conversion kernel, fitted to whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones (0.34 - 0.37
+// with a long k), storing a tile 2.7 and 1.5 us, 3.5 us of set-up and first loads, 2 - 3 us for the shares' sums to meet; where a
+// ragged N is stored word by word 1.5 us more, and 6 us divided among the shares.
+constexpr ConvCosts kConvCosts = {32, {1050.0, 600.0}, {5000.0, 2800.0}, {3000.0, 1500.0}, {11000.0, 5500.0}, 6500.0, 5500.0};
+
+// Estimated SM cycles of one launch for one or two products (the one with the longer k first) on `sms` SMs.  clusters(bn, split):
+// clusters of `split` CTAs that run at once, below one if there are none.
 template <class Clusters>
-ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters) {
+ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters, const ConvCosts& cost = kConvCosts) {
     ConvPlan best{128, 1, 0.0};
     for (uint32_t bn = 128; bn >= 64; bn -= 64) {
         uint64_t units[2] = {0, 0}, nkb[2] = {0, 0}, min_kb = ~0ull;
         for (int i = 0; i < n; ++i) {
             units[i] = (uint64_t)((sh[i].M + kConvTileM - 1) / kConvTileM) * ((sh[i].N + bn - 1) / bn) * sh[i].batch;
-            nkb[i] = (sh[i].K + 31) / 32;
+            nkb[i] = (sh[i].K + cost.kblock - 1) / cost.kblock;
             if (nkb[i] < min_kb) min_kb = nkb[i];
         }
         const uint64_t all = units[0] + units[1];
-        const double kb = bn == 128 ? 1050.0 : 600.0, store = bn == 128 ? 5000.0 : 2800.0, around = 6500.0;
+        const int w = bn == 128 ? 0 : 1;
+        const double kb = cost.kb[w], store = cost.store[w], around = cost.around;
         const bool ragged = sh[0].N % 4 != 0 || (n > 1 && sh[1].N % 4 != 0);
-        const double edge = ragged ? (bn == 128 ? 3000.0 : 1500.0) : 0.0;
+        const double edge = ragged ? cost.ragged[w] : 0.0;
         // whole units: the first CTA's units are one of every sms
         const uint64_t rounds = (all + sms - 1) / sms, rounds0 = units[0] / sms + (units[0] % sms != 0);
         auto unit = [&](int i) { return (double)nkb[i] * kb > store + edge ? (double)nkb[i] * kb : store + edge; };
@@ -47,7 +57,7 @@ ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters) 
             if (fit < 1) continue;
             const uint64_t turns = (all + fit - 1) / fit;
             const double share = (double)((nkb[0] + split - 1) / split) * kb;
-            c = (double)turns * (share + around + 5500.0 + (ragged ? (bn == 128 ? 11000.0 : 5500.0) / split : 0.0));
+            c = (double)turns * (share + around + cost.meet + (ragged ? cost.ragged_shares[w] / split : 0.0));
             if (c < best.cycles) best = ConvPlan{bn, split, c};
         }
     }
@@ -57,10 +67,10 @@ ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters) 
 // Tile width and K-shares as given (option gemm_conv), with fewer shares where the shorter k or the clusters do not allow them.  The
 // cost is the least there is: such a plan is taken.
 template <class Clusters>
-ConvPlan conv_plan_fixed(const ConvShape* sh, int n, uint32_t bn, uint32_t split, Clusters clusters) {
+ConvPlan conv_plan_fixed(const ConvShape* sh, int n, uint32_t bn, uint32_t split, Clusters clusters, uint32_t kblock = kConvCosts.kblock) {
     uint32_t k = sh[0].K;
     if (n > 1 && sh[1].K < k) k = sh[1].K;
-    while (split > 1 && (split * 2 > (k + 31) / 32 || clusters(bn, split) < 1)) --split;
+    while (split > 1 && (split * 2 > (k + kblock - 1) / kblock || clusters(bn, split) < 1)) --split;
     return ConvPlan{bn, split, 1.0};
 }
 

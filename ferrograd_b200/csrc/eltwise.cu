@@ -149,62 +149,6 @@ __global__ void __launch_bounds__(256) fold_partials_kernel(const float* partial
     if (threadIdx.x == 0) *out = s;
 }
 
-// out[c] = sum over chunks of part[k][c], for 32 columns and 256 threads.  The eight warps each add every eighth chunk into eight
-// sums in turn, which are added in pairs, then the warps' sums in order: 64 short chains of additions (50000 rows in 1563
-// chunks: 3.0e-7 of the sums' 2-norm from 64 bits with eight long ones, 1.3e-7 so).
-__device__ __forceinline__ void fold_chunks_of_columns(uint32_t c, uint32_t gy, uint32_t cx, uint32_t cols, uint32_t nchunks, const float* part,
-                                                       float* __restrict__ out, float (*red)[33]) {
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (c < cols)
-        for (uint64_t k = gy; k < nchunks; k += 64) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (k + 8 * j < nchunks) s[j] += __ldcg(part + (size_t)(k + 8 * j) * cols + c);
-        }
-    red[gy][cx] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
-    __syncthreads();
-    if (gy == 0 && c < cols) {
-        float t = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) t += red[w][cx];
-        out[c] = t;
-    }
-}
-
-// Column sums: block (32 x 8) covers 32 columns and `chunk` rows and leaves their sums in part[blockIdx.y]; with FOLD, the last
-// block of those columns adds the chunks.
-template <bool FOLD>
-__global__ void __launch_bounds__(256) colsum_kernel(uint32_t rows, uint32_t cols, uint32_t chunk, const float* __restrict__ x, float* part,
-                                                     unsigned* arrivals, float* __restrict__ out) {
-    fg_grid_enter();
-    __shared__ float red[8][33];
-    const uint32_t c = blockIdx.x * 32 + threadIdx.x;
-    const uint32_t r0 = blockIdx.y * chunk;
-    const uint32_t r1 = min(rows, r0 + chunk);
-    float s = 0.0f;
-    if (c < cols)
-        for (uint32_t r = r0 + threadIdx.y; r < r1; r += 8) s += x[(size_t)r * cols + c];
-    red[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0 && c < cols) {
-        float t = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
-        part[(size_t)blockIdx.y * cols + c] = t;
-    }
-    if constexpr (FOLD)
-        if (fg_last_block(arrivals + blockIdx.x, gridDim.y))
-            fold_chunks_of_columns(c, threadIdx.y, threadIdx.x, cols, gridDim.y, part, out, red);
-}
-// The chunks of column sums that other kernels left; a block covers 32 columns.
-__global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_t nchunks,
-                                                          const float* __restrict__ part, float* __restrict__ out) {
-    fg_grid_enter();
-    __shared__ float red[8][33];
-    const uint32_t cx = threadIdx.x & 31u;
-    fold_chunks_of_columns(blockIdx.x * 32 + cx, threadIdx.x >> 5, cx, cols, nchunks, part, out, red);
-}
-
 // ---- storage types ----
 // Elements of a type as f32, for conversions (to the nearest, ties to even).  ld4w / st4w move four consecutive elements starting
 // at element i (one 128-bit access for f32, one 64-bit access for the 16-bit types; the caller has checked the alignment).
@@ -251,6 +195,65 @@ template <> struct Stored<FG_DTYPE_BF16> {
         *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p) + i) = u;
     }
 };
+
+// out[c] = sum over chunks of part[k][c], for 32 columns and 256 threads.  The eight warps each add every eighth chunk into eight
+// sums in turn, which are added in pairs, then the warps' sums in order: 64 short chains of additions (50000 rows in 1563
+// chunks: 3.0e-7 of the sums' 2-norm from 64 bits with eight long ones, 1.3e-7 so).  `out` is of storage type DT.
+template <int DT>
+__device__ __forceinline__ void fold_chunks_of_columns(uint32_t c, uint32_t gy, uint32_t cx, uint32_t cols, uint32_t nchunks, const float* part,
+                                                       void* __restrict__ out, float (*red)[33]) {
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (c < cols)
+        for (uint64_t k = gy; k < nchunks; k += 64) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (k + 8 * j < nchunks) s[j] += __ldcg(part + (size_t)(k + 8 * j) * cols + c);
+        }
+    red[gy][cx] = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    __syncthreads();
+    if (gy == 0 && c < cols) {
+        float t = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[w][cx];
+        Stored<DT>::st(out, c, t);
+    }
+}
+
+// Column sums: block (32 x 8) covers 32 columns and `chunk` rows and leaves their sums in part[blockIdx.y]; with FOLD, the last
+// block of those columns adds the chunks.
+template <bool FOLD>
+__global__ void __launch_bounds__(256) colsum_kernel(uint32_t rows, uint32_t cols, uint32_t chunk, const float* __restrict__ x, float* part,
+                                                     unsigned* arrivals, float* __restrict__ out) {
+    fg_grid_enter();
+    __shared__ float red[8][33];
+    const uint32_t c = blockIdx.x * 32 + threadIdx.x;
+    const uint32_t r0 = blockIdx.y * chunk;
+    const uint32_t r1 = min(rows, r0 + chunk);
+    float s = 0.0f;
+    if (c < cols)
+        for (uint32_t r = r0 + threadIdx.y; r < r1; r += 8) s += x[(size_t)r * cols + c];
+    red[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && c < cols) {
+        float t = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
+        part[(size_t)blockIdx.y * cols + c] = t;
+    }
+    if constexpr (FOLD)
+        if (fg_last_block(arrivals + blockIdx.x, gridDim.y))
+            fold_chunks_of_columns<FG_DTYPE_F32>(c, threadIdx.y, threadIdx.x, cols, gridDim.y, part, out, red);
+}
+// The chunks of column sums that other kernels left; a block covers 32 columns.
+template <int DT>
+__global__ void __launch_bounds__(256) colsum_fold_kernel(uint32_t cols, uint32_t nchunks,
+                                                          const float* __restrict__ part, void* __restrict__ out) {
+    fg_grid_enter();
+    __shared__ float red[8][33];
+    const uint32_t cx = threadIdx.x & 31u;
+    fold_chunks_of_columns<DT>(blockIdx.x * 32 + cx, threadIdx.x >> 5, cx, cols, nchunks, part, out, red);
+}
+
 
 // ---- chain programs as run by the kernel ----
 // The host turns a chain (forward, or backward = the values it needs followed by the adjoints) into a list of
@@ -803,8 +806,11 @@ int32_t fg_act_bwd_launch(fg_ctx* ctx, uint64_t n, int act, const float* dy, con
     return FG_OK;
 }
 
-int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, float* out) {
-    fg_launch(ctx, colsum_fold_kernel, (cols + 31) / 32, 256, 0, cols, nchunks, part, out);
+int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, void* out, int out_dtype) {
+    const uint32_t grid = (cols + 31) / 32;
+    if (out_dtype == FG_DTYPE_F32) fg_launch(ctx, colsum_fold_kernel<FG_DTYPE_F32>, grid, 256, 0, cols, nchunks, part, out);
+    else if (out_dtype == FG_DTYPE_F16) fg_launch(ctx, colsum_fold_kernel<FG_DTYPE_F16>, grid, 256, 0, cols, nchunks, part, out);
+    else fg_launch(ctx, colsum_fold_kernel<FG_DTYPE_BF16>, grid, 256, 0, cols, nchunks, part, out);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }
@@ -845,9 +851,7 @@ int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float*
     }
     fg_launch(ctx, colsum_kernel<false>, grid, block, 0, rows, cols, chunk, x, (float*)part, (unsigned*)nullptr, (float*)nullptr);
     FG_LAUNCHED(ctx);
-    fg_launch(ctx, colsum_fold_kernel, groups, 256, 0, cols, nchunks, (const float*)part, out);
-    FG_LAUNCHED(ctx);
-    return FG_OK;
+    return fg_colsum_fold_launch(ctx, cols, nchunks, (const float*)part, out);
 }
 
 extern "C" {

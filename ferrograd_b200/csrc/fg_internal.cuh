@@ -460,4 +460,4 @@ struct FgBlockSums { float *partials, *out, *sum; int grid; };
 int32_t fg_block_sums(fg_ctx* ctx, int grid, float* sum, FgBlockSums* b);
 int32_t fg_block_sums_end(fg_ctx* ctx, const FgBlockSums& b);
 int32_t fg_colsum_launch(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* x, float* out);
-int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, float* out);
+int32_t fg_colsum_fold_launch(fg_ctx* ctx, uint32_t cols, uint32_t nchunks, const float* part, void* out, int out_dtype = FG_DTYPE_F32);

@@ -41,7 +41,7 @@ constexpr long long kWaitCycles = 2000000000LL;   // bound on every device-side 
 
 struct Epilogue {
     float* C;
-    const float* bias;
+    const float* bias;   // in the storage type, see epi_bias
     float* preact;
     uint32_t M, N, K;
     int act;
@@ -50,7 +50,7 @@ struct Epilogue {
     // partial sums over equal shares of the K chunks, written raw to `partial` and folded by a second kernel.
     float* partial;
     uint32_t t_full, split;
-    int out_dtype;       // storage type of C and preact (fg_dtype); bias and partial are always f32
+    int out_dtype;       // storage type of C, preact and bias (fg_dtype); partial is always f32
     // ---- pair kernel on f32 tensors with bf16 pairs (FMT 1) ----
     uint32_t a_mn, b_mn;              // the operand's storage has the non-contraction index contiguous
     __nv_bfloat16* c_pairs;           // optional: bf16 pairs of the stored C (see pairs_kernel)
@@ -82,6 +82,11 @@ __device__ __forceinline__ void store_out4(void* base, size_t idx, float4 v, int
         u.y = *reinterpret_cast<const uint32_t*>(&hi);
         *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(base) + idx) = u;
     }
+}
+// The bias of column c, which lies in the output's storage type.
+__device__ __forceinline__ float epi_bias(const float* bias, uint32_t c, int dt) {
+    if (dt == FG_DTYPE_F32) return bias[c];
+    return dt == FG_DTYPE_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[c]) : __half2float(reinterpret_cast<const __half*>(bias)[c]);
 }
 __device__ __forceinline__ void store_out1(void* base, size_t idx, float v, int dt) {
     if (dt == FG_DTYPE_F32) static_cast<float*>(base)[idx] = v;
@@ -817,7 +822,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const bool fast = vec && col + 3 < col_lim;                    // the whole float4 is inside the matrix
                 float4 bz = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (ep.bias && !part) {
-                    if (col + 3 < col_lim) bz = __ldg(reinterpret_cast<const float4*>(ep.bias + col));
+                    if (kDirect16) {
+                        if (col < col_lim) bz.x = epi_bias(ep.bias, col, ep.out_dtype);
+                        if (col + 1 < col_lim) bz.y = epi_bias(ep.bias, col + 1, ep.out_dtype);
+                        if (col + 2 < col_lim) bz.z = epi_bias(ep.bias, col + 2, ep.out_dtype);
+                        if (col + 3 < col_lim) bz.w = epi_bias(ep.bias, col + 3, ep.out_dtype);
+                    } else if (col + 3 < col_lim) bz = __ldg(reinterpret_cast<const float4*>(ep.bias + col));
                     else {
                         if (col < col_lim) bz.x = ep.bias[col];
                         if (col + 1 < col_lim) bz.y = ep.bias[col + 1];
@@ -933,7 +943,7 @@ __global__ void __launch_bounds__(256) gemm_tc_fold_kernel(Epilogue ep) {
         float zz[4] = {z.x, z.y, z.z, z.w};
         if (ep.bias) {
 #pragma unroll
-            for (int t = 0; t < 4; ++t) if (col + t < ep.N) zz[t] += ep.bias[col + t];
+            for (int t = 0; t < 4; ++t) if (col + t < ep.N) zz[t] += epi_bias(ep.bias, col + t, ep.out_dtype);
         }
         const size_t off = (size_t)row * ep.N + col;
         const bool vec_ok = (ep.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
@@ -1846,6 +1856,326 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
     }
 }
 
+// ------------------------------------------------------------------------------------
+// Sixteen-bit tensors, small and middling products: the conversion kernel's scheme without its converters.  The pair kernel's 256 x 256
+// tiles leave most SMs idle on a product of a few tiles and cost 15 - 20 us whatever the product's size (layers of 100 - 500 samples:
+// three of them, 65 us forward and backward).  Here a CTA owns a 128 x BN tile (BN 128 or 64), k-blocks of 64 go from the tensors as
+// they lie through shared memory into kind::f16 MMAs, K-shares are the CTAs of a cluster, whose sums meet in distributed shared
+// memory, and both gradients of a layer are one launch.
+//   warp 0 loads, warp 1 issues MMAs, warps 4..11 drain accumulators, add up the shares and store.
+// Bound by shared memory on long k (128 x 128: 32 KB in and 32 KB out of it per k-block, 512 cycles; the tensor core needs 256), by the
+// ends of the launch on short ones.
+// ------------------------------------------------------------------------------------
+template <int BN>
+struct HalfCfg {
+    static constexpr int kA = BM * 128, kB = BN * 128, kStageBytes = kA + kB;      // 64 values of k: rows of 128 bytes
+    static constexpr int kStages = BN == 128 ? 6 : 8;
+    static constexpr int kThreads = 384, kEpi0 = 4;
+    static constexpr int kStoreBytes = 8 * 32 * 32 * 4;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256;
+    static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
+    static_assert(kStages * kStageBytes >= BM * BN * 4, "a K-share's sums lie in the stages");
+    static constexpr int kTmemCols = 2 * BN;
+};
+struct HalfArgs {
+    Epilogue ep[2];
+    uint32_t units0, units, split;
+    int* dev_status;
+};
+
+template <int BN, bool TWO, bool SHARES>
+__global__ void __launch_bounds__(HalfCfg<BN>::kThreads, 1)
+gemm_tc_half_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
+                    const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmB1,
+                    const __grid_constant__ HalfArgs ha) {
+    using Cfg = HalfCfg<BN>;
+    constexpr int S = Cfg::kStages, BK = 64, CPT = BN / 2;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    unsigned char* const base_ptr = smem_raw + (base - raw);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(base_ptr + S * Cfg::kStageBytes + Cfg::kStoreBytes);
+    const uint32_t bar0 = base + S * Cfg::kStageBytes + Cfg::kStoreBytes;
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (S + s); };
+    auto acc_full_bar = [&](int b) { return bar0 + 8u * (2 * S + b); };
+    auto acc_empty_bar = [&](int b) { return bar0 + 8u * (2 * S + 2 + b); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * S + 4);
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t split = SHARES ? ha.split : 1u, share = SHARES ? cluster_ctarank() : 0u;
+    const uint32_t first = SHARES ? blockIdx.x / split : blockIdx.x, step = SHARES ? ha.units : gridDim.x;
+    struct Unit { uint32_t p, m0, n0, kb0, nkb; };
+    auto ep_of = [&](uint32_t p, auto field) { return !TWO || p == 0 ? field(ha.ep[0]) : field(ha.ep[1]); };
+    auto unit_at = [&](uint32_t u) -> Unit {
+        Unit t;
+        t.p = TWO && u >= ha.units0 ? 1u : 0u;
+        const uint32_t tile = u - (t.p ? ha.units0 : 0u), K = ep_of(t.p, [](const Epilogue& e) { return e.K; });
+        const uint32_t tiles_m = ep_of(t.p, [](const Epilogue& e) { return (e.M + BM - 1) / BM; });
+        t.m0 = tile % tiles_m * BM;
+        t.n0 = tile / tiles_m * BN;
+        const uint32_t all = (K + BK - 1) / BK;      // the host keeps split <= all
+        t.kb0 = (uint32_t)((uint64_t)share * all / split);
+        t.nkb = (uint32_t)((uint64_t)(share + 1) * all / split) - t.kb0;
+        return t;
+    };
+    auto is_mn = [&](uint32_t p, bool& a, bool& b) {
+        a = ep_of(p, [](const Epilogue& e) { return e.a_mn != 0; });
+        b = ep_of(p, [](const Epilogue& e) { return e.b_mn != 0; });
+    };
+    constexpr uint32_t kChunkKB = 1024 / BK;      // k per accumulation chunk, as in the pair kernel
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full_bar(b), 1); mbar_init(acc_empty_bar(b), 8); }
+        fence_mbar_init();
+        prefetch_tmap(&tmA0);
+        prefetch_tmap(&tmB0);
+        if (TWO) { prefetch_tmap(&tmA1); prefetch_tmap(&tmB1); }
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), Cfg::kTmemCols);
+        tmem_relinquish();
+    }
+    // Everything up to here needs nothing of the kernels before this one: it passes while the last of them drains.
+    fg_grid_enter();
+    __shared__ int s_abort;      // see gemm_tc_kernel; the CTAs of a cluster stay together to the end, whatever they have read
+    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(ha.dev_status);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const bool go = __all_sync(0xffffffffu, s_abort == 0);
+
+    if (go && warp == 0) {
+        // ---- producer ----
+        uint32_t g = 0;      // k-blocks so far, across units: ring position and phase
+        bool ok = true;
+        for (uint32_t u = first; u < ha.units && ok; u += step) {
+            const Unit t = unit_at(u);
+            const CUtensorMap* const ta = TWO && t.p ? &tmA1 : &tmA0;
+            const CUtensorMap* const tb = TWO && t.p ? &tmB1 : &tmB0;
+            bool a_mn, b_mn;
+            is_mn(t.p, a_mn, b_mn);
+            for (uint32_t i = 0; i < t.nkb; ++i, ++g) {
+                const int s = g % S;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty_bar(s), ((g / S) & 1u) ^ 1u, kWaitCycles))) {
+                    if (lane == 0) atomicOr(ha.dev_status, FG_DEVERR_TMA_WAIT);
+                    ok = false;
+                    break;
+                }
+                const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + Cfg::kA;
+                const int k = (int)((t.kb0 + i) * BK);
+                if (!elect_one()) continue;
+                mbar_expect_tx(full_bar(s), Cfg::kStageBytes);
+                // K-major storage: one box; MN-major ([k][rows]): boxes of 64 rows x 64 k, each [k][64 rows]
+                if (!a_mn) tma_load_3d(sa, ta, full_bar(s), k, (int)t.m0, 0);
+                else
+#pragma unroll
+                    for (int j = 0; j < BM / 64; ++j) tma_load_3d(sa + j * 8192, ta, full_bar(s), (int)(t.m0 + 64 * j), k, 0);
+                if (!b_mn) tma_load_3d(sb, tb, full_bar(s), k, (int)t.n0, 0);
+                else
+#pragma unroll
+                    for (int j = 0; j < BN / 64; ++j) tma_load_3d(sb + j * 8192, tb, full_bar(s), (int)(t.n0 + 64 * j), k, 0);
+            }
+        }
+    } else if (go && warp == 1) {
+        // ---- MMA issuer ----
+        bool ok = true;
+        uint32_t g = 0, gc = 0;      // k-blocks and chunks so far, across units
+        for (uint32_t u = first; u < ha.units && ok; u += step) {
+            const Unit t = unit_at(u);
+            bool a_mn, b_mn;
+            is_mn(t.p, a_mn, b_mn);
+            const uint32_t idesc = make_idesc(ha.ep[0].out_dtype == FG_DTYPE_BF16 ? 1u : 0u, BM, BN) | (a_mn ? kIdescAMnMajor : 0u) | (b_mn ? kIdescBMnMajor : 0u);
+            const uint32_t a_adv = a_mn ? 128u : 2u, b_adv = b_mn ? 128u : 2u;
+            const uint32_t nchunks = (t.nkb + kChunkKB - 1) / kChunkKB;
+            for (uint32_t c = 0; c < nchunks && ok; ++c, ++gc) {
+                const uint32_t buf = gc & 1u;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(acc_empty_bar(buf), ((gc >> 1) & 1u) ^ 1u, kWaitCycles))) {
+                    if (lane == 0) atomicOr(ha.dev_status, FG_DEVERR_MMA_WAIT);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + buf * BN;
+                const uint32_t end = min(t.nkb, (c + 1) * kChunkKB);
+                for (uint32_t i = c * kChunkKB; i < end; ++i, ++g) {
+                    const int s = g % S;
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(full_bar(s), (g / S) & 1u, kWaitCycles))) {
+                        if (lane == 0) atomicOr(ha.dev_status, FG_DEVERR_MMA_WAIT);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sa = base + s * Cfg::kStageBytes, sb = sa + Cfg::kA;
+                    const uint64_t a_d = a_mn ? make_desc_mnmajor(sa, 8192, 1024, 2) : make_desc_kmajor<128>(sa);
+                    const uint64_t b_d = b_mn ? make_desc_mnmajor(sb, 8192, 1024, 2) : make_desc_kmajor<128>(sb);
+                    const uint32_t acc = (i == c * kChunkKB) ? 0u : 1u;      // a chunk starts from zero
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < BK / 16; ++kk)
+                            mma_f16(d_tmem, a_d + (uint64_t)(kk * a_adv), b_d + (uint64_t)(kk * b_adv), idesc, acc | (uint32_t)kk);
+                        mma_commit(empty_bar(s));
+                    }
+                    __syncwarp();
+                }
+                if (ok && elect_one()) mma_commit(acc_full_bar(buf));
+                __syncwarp();
+            }
+        }
+    } else if (warp >= Cfg::kEpi0) {
+        // ---- accumulate + epilogue: warps 4..11; warp w may touch TMEM lanes 32*(w%4) .. +31 ----
+        const int q = warp & 3, half = (warp - Cfg::kEpi0) >> 2;
+        bool ok = go;
+        uint32_t gc = 0;
+        float4* const tb4 = reinterpret_cast<float4*>(base_ptr + S * Cfg::kStageBytes) + (warp - Cfg::kEpi0) * (32 * 8);
+        const uint32_t rsub = lane >> 3, cc = lane & 7;
+        // (a launch of two products, the gradients, has none)
+        auto bias_at = [&](uint32_t c) { return !TWO && ha.ep[0].bias && c < ha.ep[0].N ? epi_bias(ha.ep[0].bias, c, ha.ep[0].out_dtype) : 0.0f; };
+        // Four columns of a row from their sums with the bias.
+        auto put4 = [&](const Epilogue& ep, size_t off, uint32_t col, bool vec, float4 z) {
+            if (vec) {      // (N is a multiple of four: a live group is whole)
+                const float4 o = ep.act == FG_ACT_NONE ? z : make_float4(fg_act_fwd_sel(ep.act, z.x), fg_act_fwd_sel(ep.act, z.y),
+                                                                         fg_act_fwd_sel(ep.act, z.z), fg_act_fwd_sel(ep.act, z.w));
+                if (ep.preact) store_out4(ep.preact, off, z, ep.out_dtype);
+                store_out4(ep.C, off, o, ep.out_dtype);
+            } else {
+                epi_store_edge(z, off, col, ep.N, (char*)ep.C, (char*)ep.preact, nullptr, 0, nullptr, 0, ep.act, ep.out_dtype);
+            }
+        };
+        auto vec_ok = [&](const Epilogue& ep) {      // (C and preact start on 16 bytes)
+            return ep.N % 4 == 0;
+        };
+        // A 32 x 32 block of whole sums, swizzled in tb4 (float4 c of row r at c ^ (r & 7)): four rows of 64 bytes per step, or, where
+        // rows do not start on eight bytes, a lane per column and a row per step.
+        auto store_block = [&](const Epilogue& ep, uint32_t row0, uint32_t col0, float bias) {
+            if (!vec_ok(ep)) {
+                const uint32_t c = col0 + lane, rows = c < ep.N && row0 < ep.M ? min(32u, ep.M - row0) : 0u;
+                const float* const tb = reinterpret_cast<const float*>(tb4);
+                size_t off = (size_t)row0 * ep.N + c;
+#pragma unroll 4
+                for (uint32_t r = 0; r < 32; ++r, off += ep.N) {
+                    if (r >= rows) continue;
+                    const float z = tb[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)] + bias;
+                    if (ep.preact) store_out1(ep.preact, off, z, ep.out_dtype);
+                    store_out1(ep.C, off, fg_act_fwd_sel(ep.act, z), ep.out_dtype);
+                }
+                __syncwarp();
+                return;
+            }
+            const float4 bz = make_float4(__shfl_sync(0xffffffffu, bias, cc * 4), __shfl_sync(0xffffffffu, bias, cc * 4 + 1),
+                                          __shfl_sync(0xffffffffu, bias, cc * 4 + 2), __shfl_sync(0xffffffffu, bias, cc * 4 + 3));
+            const uint32_t col = col0 + cc * 4;
+            size_t off = (size_t)(row0 + rsub) * ep.N + col;
+            const uint32_t rows = col < ep.N && row0 + rsub < ep.M ? (ep.M - row0 - rsub + 3) / 4 : 0u;      // this lane's, of eight
+#pragma unroll 4
+            for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N) {
+                const uint32_t lr = i * 4 + rsub;
+                if (i < rows) put4(ep, off, col, true, add4(tb4[lr * 8 + (cc ^ (lr & 7))], bz));
+            }
+            __syncwarp();
+        };
+        for (uint32_t u = first; u < ha.units && ok; u += step) {
+            const Unit t = unit_at(u);
+            const uint32_t nchunks = (t.nkb + kChunkKB - 1) / kChunkKB;
+            // a lane holds the bias of one column per block: it is here long before the sums are
+            float bias[CPT / 32];
+            if constexpr (!SHARES) {
+#pragma unroll
+                for (int gr = 0; gr < CPT / 32; ++gr) bias[gr] = bias_at(t.n0 + half * CPT + gr * 32 + lane);
+            }
+            float sum[CPT];
+#pragma unroll
+            for (int j = 0; j < CPT; ++j) sum[j] = 0.0f;
+            for (uint32_t c = 0; c < nchunks; ++c, ++gc) {
+                const uint32_t buf = gc & 1u;
+                bool got = mbar_wait_bounded(acc_full_bar(buf), (gc >> 1) & 1u, kWaitCycles + kWaitCycles / 2);
+                got = __all_sync(0xffffffffu, got);
+                if (!got) {
+                    if (lane == 0) atomicOr(ha.dev_status, FG_DEVERR_EPI_WAIT);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * CPT;
+#pragma unroll
+                for (int gr = 0; gr < CPT / 32; ++gr) {
+                    uint32_t r[32];
+                    tmem_ld_32x32(t0 + gr * 32, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[gr * 32 + j] += __uint_as_float(r[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+            }
+            if (!ok) break;
+            if constexpr (SHARES) {
+                // Every load and MMA of this CTA has finished (its last chunk is complete), so the stages are free: the share's
+                // sums as [row][BN], float4 c of a row at c ^ (row & 7).
+                float4* const part = reinterpret_cast<float4*>(base_ptr) + (q * 32 + lane) * (BN / 4);
+#pragma unroll
+                for (int c = 0; c < CPT / 4; ++c)
+                    part[(half * (CPT / 4) + c) ^ (lane & 7)] = make_float4(sum[4 * c], sum[4 * c + 1], sum[4 * c + 2], sum[4 * c + 3]);
+            } else {
+#pragma unroll
+                for (int gr = 0; gr < CPT / 32; ++gr) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        tb4[lane * 8 + (c ^ (lane & 7))] = make_float4(sum[gr * 32 + 4 * c], sum[gr * 32 + 4 * c + 1], sum[gr * 32 + 4 * c + 2], sum[gr * 32 + 4 * c + 3]);
+                    __syncwarp();
+                    const uint32_t row0 = t.m0 + q * 32, col0 = t.n0 + half * CPT + gr * 32;
+                    if (!TWO || t.p == 0) store_block(ha.ep[0], row0, col0, bias[gr]);
+                    else store_block(ha.ep[1], row0, col0, bias[gr]);
+                }
+            }
+        }
+        if constexpr (SHARES) {
+            __syncwarp();
+            cluster_sync_all();      // every share's sums are in its CTA's shared memory
+            if (go) {
+                // This CTA's 32 x 32 blocks are every split-th of the tile, from its share's number on; a warp takes four rows of
+                // one, a lane four columns of a row.
+                const Unit t = unit_at(first);
+                auto fold = [&](const Epilogue& ep) {
+                    for (uint32_t v = warp - Cfg::kEpi0, b; (b = share + split * (v >> 3)) < 4 * (BN / 32); v += 8) {
+                        const uint32_t lr = (b & 3u) * 32 + (v & 7u) * 4 + rsub, c0 = (b >> 2) * 32, row = t.m0 + lr, col = t.n0 + c0 + cc * 4;
+                        const uint32_t at = base + ((lr * (BN / 4) + (((c0 >> 2) + cc) ^ (lr & 7))) << 4);
+                        float4 z[8];
+#pragma unroll
+                        for (uint32_t r = 0; r < 8; ++r)
+                            if (r < split) z[r] = ld_cluster_f4(map_to_cta(at, r));
+                        float bz[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) bz[j] = bias_at(col + j);
+#pragma unroll
+                        for (uint32_t r = 1; r < 8; ++r)        // in the order of the shares, whoever adds them
+                            if (r < split) z[0] = add4(z[0], z[r]);
+                        if (col < ep.N && row < ep.M)
+                            put4(ep, (size_t)row * ep.N + col, col, vec_ok(ep), add4(z[0], make_float4(bz[0], bz[1], bz[2], bz[3])));
+                        __syncwarp();
+                    }
+                };
+                if (!TWO || t.p == 0) fold(ha.ep[0]);
+                else fold(ha.ep[1]);
+            }
+            __syncwarp();
+            cluster_sync_all();      // no CTA leaves while another reads its sums
+        }
+    }
+    if constexpr (SHARES) {
+        if (warp < Cfg::kEpi0) { __syncwarp(); cluster_sync_all(); cluster_sync_all(); }      // as the epilogue warps
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    }
+}
+
 inline uint32_t round4(uint32_t v) { return (v + 3u) & ~3u; }
 inline uint32_t round8(uint32_t v) { return (v + 7u) & ~7u; }
 inline uint64_t align256(uint64_t v) { return (v + 255u) & ~uint64_t(255); }
@@ -2244,6 +2574,94 @@ int32_t launch_conv_both(fg_ctx* ctx, const ConvProduct& dB, const ConvProduct& 
     const bool b_first = dB.ep.K >= dA.ep.K;
     const int32_t s = launch_conv(ctx, &dB, 1, b_first ? one : two);
     return s != FG_OK ? s : launch_conv(ctx, &dA, 1, b_first ? two : one);
+}
+
+// ---- the same for sixteen-bit tensors ----
+// Costs fitted to 87 products under the pair kernel and every plan (2 % slower than the best of each in the geometric mean).
+constexpr ConvCosts kHalfCosts = {64, {520.0, 305.0}, {600.0, 300.0}, {950.0, 1250.0}, {800.0, 650.0}, 2400.0, 1600.0};
+template <int BN, bool TWO, bool SHARES>
+cudaError_t half_attr(const fg_ctx* ctx) {
+    static std::atomic<uint64_t> done{0};
+    if (done.load(std::memory_order_acquire) >> (ctx->device & 63) & 1ull) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_tc_half_kernel<BN, TWO, SHARES>, cudaFuncAttributeMaxDynamicSharedMemorySize, HalfCfg<BN>::kSmemBytes);
+    if (e == cudaSuccess) done.fetch_or(1ull << (ctx->device & 63), std::memory_order_release);
+    return e;
+}
+template <int BN>
+int half_clusters(const fg_ctx* ctx, uint32_t split) {
+    static std::atomic<int> known[64][9];       // zero-initialised
+    return fg_asked_once(known[ctx->device & 63][split], 0, [&](int* n) {
+        if (half_attr<BN, false, true>(ctx) != cudaSuccess) { cudaGetLastError(); return false; }
+        return cluster_query(n, gemm_tc_half_kernel<BN, false, true>, split * 64, HalfCfg<BN>::kThreads, HalfCfg<BN>::kSmemBytes, split);
+    });
+}
+ConvPlan plan_half(const fg_ctx* ctx, const ConvShape* sh, int n) {
+    const uint64_t sms = fg_free_sms(ctx);
+    auto clusters = [&](uint32_t bn, uint32_t split) {
+        return conv_clusters_beside(bn == 128 ? half_clusters<128>(ctx, split) : half_clusters<64>(ctx, split), sms, (uint64_t)ctx->sm_count);
+    };
+    if (ctx->opt_conv_bn) return conv_plan_fixed(sh, n, (uint32_t)ctx->opt_conv_bn, (uint32_t)ctx->opt_conv_split, clusters, kHalfCosts.kblock);
+    return conv_plan(sh, n, sms, clusters, kHalfCosts);
+}
+template <int BN>
+int32_t launch_half_bn(fg_ctx* ctx, const ConvProduct* pr, int n, uint32_t split) {
+    using Cfg = HalfCfg<BN>;
+    CUtensorMap tm[4];
+    HalfArgs ha{};
+    uint64_t units = 0;
+    double flop = 0.0;
+    for (int j = 0; j < n; ++j) {
+        const ConvProduct& c = pr[j];
+        const PlaneSet* ops[2] = {&c.a, &c.b};
+        const uint32_t rows[2] = {c.ep.M, c.ep.N}, tile[2] = {(uint32_t)BM, (uint32_t)BN};
+        const int elem = c.ep.out_dtype == FG_DTYPE_BF16 ? 1 : 2;
+        for (int i = 0; i < 2; ++i) {
+            const PlaneSet& o = *ops[i];
+            const int32_t s = !o.mn ? make_tmap(ctx, &tm[2 * j + i], o.p16, elem, 1, rows[i], c.ep.K, o.ld16, tile[i], 64)
+                                    : make_tmap3(ctx, &tm[2 * j + i], o.p16, elem, rows[i], c.ep.K, 1, (uint64_t)o.ld16 * 2, (uint64_t)c.ep.K * o.ld16 * 2, 64, 64, 1);
+            if (s != FG_OK) return s;
+        }
+        ha.ep[j] = c.ep;
+        ha.ep[j].a_mn = c.a.mn ? 1u : 0u;
+        ha.ep[j].b_mn = c.b.mn ? 1u : 0u;
+        units += (uint64_t)((c.ep.M + BM - 1) / BM) * ((c.ep.N + BN - 1) / BN);
+        if (units > (1ull << 28)) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM: too many tiles");
+        if (j == 0) ha.units0 = (uint32_t)units;
+        flop += 2.0 * c.ep.M * c.ep.N * c.ep.K;
+    }
+    if (n == 1) { tm[2] = tm[0]; tm[3] = tm[1]; }
+    ha.units = (uint32_t)units;
+    ha.split = split;
+    ha.dev_status = ctx->dev_status;
+    const uint32_t grid = (uint32_t)conv_grid(units, split, fg_free_sms(ctx));
+    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, flop);
+    auto launch = [&](auto two, auto shares) -> int32_t {
+        constexpr bool T = decltype(two)::value, S = decltype(shares)::value;
+        FG_CUDA(ctx, FG_ERR_INTERNAL, (half_attr<BN, T, S>(ctx)));
+        fg_launch_cluster(ctx, gemm_tc_half_kernel<BN, T, S>, grid, Cfg::kThreads, Cfg::kSmemBytes, split, tm[0], tm[1], tm[2], tm[3], ha);
+        FG_LAUNCHED(ctx);
+        return FG_OK;
+    };
+    const std::true_type yes{};
+    const std::false_type no{};
+    const int32_t s = n == 2 ? (split > 1 ? launch(yes, yes) : launch(yes, no)) : split > 1 ? launch(no, yes) : launch(no, no);
+    fg_time_end(ctx, tr);
+    return s;
+}
+int32_t launch_half(fg_ctx* ctx, const ConvProduct* pr, int n, const ConvPlan& p) {
+    return p.bn == 128 ? launch_half_bn<128>(ctx, pr, n, p.split) : launch_half_bn<64>(ctx, pr, n, p.split);
+}
+// The pair kernel on 16-bit tensors by the same fit: tiles of 256 x 256, K-shares of 2048 or more in the last wave.
+double pair16_cycles(const fg_ctx* ctx, const ConvShape& sh) {
+    const uint64_t pairs = fg_free_sms(ctx) / 2, tiles = (uint64_t)((sh.M + 255) / 256) * ((sh.N + 255) / 256);
+    const double kb = (double)((sh.K + 63) / 64) * 395.0, tile = kb > 2500.0 ? kb : 2500.0, whole = (double)(tiles / pairs) * tile;
+    const uint64_t rem = tiles % pairs, nchunks = (sh.K + 1023) / 1024;
+    double tail = rem ? tile : 0.0;
+    uint64_t split = rem ? pairs / rem : 1;
+    if (split > nchunks / 2) split = nchunks / 2;
+    if (split > 4) split = 4;
+    if (split >= 2 && ctx->opt_split_k) tail = tail / (double)split + 3300.0;
+    return whole + tail + 26600.0;
 }
 
 // A dense [R, C] f32 tensor (`batch` of them, x_batch apart) can be loaded as it lies when rows and matrices start on
@@ -3296,10 +3714,41 @@ PlaneSet operand16(const void* p, uint32_t ld, bool mn) {
     return o;
 }
 
-int32_t lowp_gemm(fg_ctx* ctx, int dtype, const PlaneSet& pa, const PlaneSet& pb, uint32_t M, uint32_t N, uint32_t K, void* C,
-                  const float* bias32, int act, void* preact) {
-    Epilogue ep{(float*)C, bias32, (float*)preact, M, N, K, act, ctx->dev_status, nullptr, 0, 1, dtype};
-    return dtype == FG_DTYPE_BF16 ? launch_tc_pair<32, 2>(ctx, pa, pb, ep) : launch_tc_pair<32, 3>(ctx, pa, pb, ep);
+Epilogue epilogue16(const fg_ctx* ctx, int dtype, uint32_t M, uint32_t N, uint32_t K, void* C, const void* bias, int act, void* preact) {
+    return Epilogue{(float*)C, (const float*)bias, (float*)preact, M, N, K, act, ctx->dev_status, nullptr, 0, 1, dtype};
+}
+// The pair kernel or the half kernel, whichever is estimated to end first (option gemm_tile: the pair kernel; gemm_conv: the other).
+bool half_suits(const fg_ctx* ctx, const ConvShape& sh, ConvPlan* plan) {
+    if (ctx->opt_tile_pair == 1) return false;
+    *plan = plan_half(ctx, &sh, 1);
+    return ctx->opt_conv_bn || plan->cycles <= pair16_cycles(ctx, sh);
+}
+int32_t launch_pair16(fg_ctx* ctx, const ConvProduct& p) {
+    return p.ep.out_dtype == FG_DTYPE_BF16 ? launch_tc_pair<32, 2>(ctx, p.a, p.b, p.ep) : launch_tc_pair<32, 3>(ctx, p.a, p.b, p.ep);
+}
+int32_t lowp_gemm(fg_ctx* ctx, const ConvProduct& p) {
+    ConvPlan plan;
+    return half_suits(ctx, conv_shape(p), &plan) ? launch_half(ctx, &p, 1, plan) : launch_pair16(ctx, p);
+}
+// Both gradients of a layer, dB first: one launch where both are for the half kernel, they are estimated to end sooner together, and
+// neither lies over what the other reads.
+int32_t lowp_gemm_both(fg_ctx* ctx, const ConvProduct& dB, const ConvProduct& dA) {
+    ConvPlan b, a;
+    const bool hb = half_suits(ctx, conv_shape(dB), &b), ha = half_suits(ctx, conv_shape(dA), &a);
+    if (hb && ha) {
+        const ConvProduct pr[2] = {dB.ep.K >= dA.ep.K ? dB : dA, dB.ep.K >= dA.ep.K ? dA : dB};      // the longer k first
+        const ConvShape sh[2] = {conv_shape(pr[0]), conv_shape(pr[1])};
+        const ConvPlan both = plan_half(ctx, sh, 2);
+        auto over = [](const ConvProduct& w, const ConvProduct& r) {
+            const uint64_t n = (uint64_t)w.ep.M * w.ep.N * 2;
+            return fg_ranges_meet(w.ep.C, n, r.a.p16, (uint64_t)(r.a.mn ? r.ep.K : r.ep.M) * r.a.ld16 * 2) ||
+                   fg_ranges_meet(w.ep.C, n, r.b.p16, (uint64_t)(r.b.mn ? r.ep.K : r.ep.N) * r.b.ld16 * 2);
+        };
+        // (a second launch costs 2500 more than the estimates know)
+        if (both.cycles <= b.cycles + a.cycles + 2500.0 && !over(dB, dA) && !over(dA, dB)) return launch_half(ctx, pr, 2, both);
+    }
+    const int32_t s = hb ? launch_half(ctx, &dB, 1, b) : launch_pair16(ctx, dB);
+    return s != FG_OK ? s : ha ? launch_half(ctx, &dA, 1, a) : launch_pair16(ctx, dA);
 }
 
 }  // namespace
@@ -3315,20 +3764,15 @@ int32_t fg_gemm_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, act >= FG_ACT_NONE && act <= FG_ACT_GELU, "fg_gemm_lowp: unknown activation");
     FG_REQUIRE(ctx, fg_aligned16(C) && (!preact_out || fg_aligned16(preact_out)), "fg_gemm_lowp: outputs must be 16-byte aligned");
     if (!ctx->tmap_encode) return fg_fail(ctx, FG_ERR_UNSUPPORTED_FEATURE, "fg_gemm_lowp: tensor maps unavailable");
-    const uint64_t need = copy16_bytes(A, M, K) + copy16_bytes(B, K, N) + (uint64_t)N * 4 + kPairPartialBytes + 2048;
+    const uint64_t need = copy16_bytes(A, M, K) + copy16_bytes(B, K, N) + kPairPartialBytes + 2048;
     { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
     int32_t s;
     const void *a, *b;
     uint32_t lda, ldb;
     if ((s = loadable16(ctx, dtype, A, M, K, &a, &lda)) != FG_OK) return s;
     if ((s = loadable16(ctx, dtype, B, K, N, &b, &ldb)) != FG_OK) return s;
-    void* bias32 = nullptr;
-    if (bias) {
-        if ((s = fg_ws_alloc(ctx, (uint64_t)N * 4, &bias32)) != FG_OK) return s;
-        if ((s = fg_convert_launch(ctx, bias, dtype, bias32, FG_DTYPE_F32, N)) != FG_OK) return s;
-    }
     // A [M][K] has the contraction index contiguous, B [K][N] its rows (the output's columns)
-    return lowp_gemm(ctx, dtype, operand16(a, lda, false), operand16(b, ldb, true), M, N, K, C, (const float*)bias32, act, preact_out);
+    return lowp_gemm(ctx, ConvProduct{operand16(a, lda, false), operand16(b, ldb, true), epilogue16(ctx, dtype, M, N, K, C, bias, act, preact_out), 1});
 }
 
 int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uint32_t K, const void* A, const void* B,
@@ -3350,7 +3794,7 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
     if ((dA || dB) && !dz_direct) need += (uint64_t)M * pad8(N) * 2 + 256;
     if (dA) need += copy16_bytes(B, K, N);
     if (dB) need += copy16_bytes(A, M, K);
-    if (dbias) need += (uint64_t)nchunk_rows * N * 4 + (uint64_t)N * 4 + 512;
+    if (dbias) need += (uint64_t)nchunk_rows * N * 4 + 256;
     { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
     int32_t s;
     void *dz = const_cast<void*>(dY), *cs_part = nullptr;
@@ -3366,27 +3810,21 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
         pz.colsum_part = (float*)cs_part;
     }
     if ((pz.out || pz.colsum_part) && (s = launch_prep(ctx, dtype, pz)) != FG_OK) return s;
+    if (dbias && (s = fg_colsum_fold_launch(ctx, N, nchunk_rows, (const float*)cs_part, dbias, dtype)) != FG_OK) return s;
     const void* x;
     uint32_t ldx;
+    ConvProduct w{}, v{};
     if (dB) {
         // dB[K,N] = A^T · dZ: contraction over M, the row index of both tensors
         if ((s = loadable16(ctx, dtype, A, M, K, &x, &ldx)) != FG_OK) return s;
-        if ((s = lowp_gemm(ctx, dtype, operand16(x, ldx, true), operand16(dz, ldz, true), K, N, M, dB, nullptr, FG_ACT_NONE, nullptr)) != FG_OK)
-            return s;
+        w = ConvProduct{operand16(x, ldx, true), operand16(dz, ldz, true), epilogue16(ctx, dtype, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr), 1};
+        if (!dA) return lowp_gemm(ctx, w);
     }
-    if (dbias) {
-        void* db32;
-        if ((s = fg_ws_alloc(ctx, (uint64_t)N * 4, &db32)) != FG_OK) return s;
-        if ((s = fg_colsum_fold_launch(ctx, N, nchunk_rows, (const float*)cs_part, (float*)db32)) != FG_OK) return s;
-        if ((s = fg_convert_launch(ctx, db32, FG_DTYPE_F32, dbias, dtype, N)) != FG_OK) return s;
-    }
-    if (dA) {
-        // dA[M,K] = dZ · B^T: contraction over N, contiguous in both
-        if ((s = loadable16(ctx, dtype, B, K, N, &x, &ldx)) != FG_OK) return s;
-        if ((s = lowp_gemm(ctx, dtype, operand16(dz, ldz, false), operand16(x, ldx, false), M, K, N, dA, nullptr, FG_ACT_NONE, nullptr)) != FG_OK)
-            return s;
-    }
-    return FG_OK;
+    if (!dA) return FG_OK;
+    // dA[M,K] = dZ · B^T: contraction over N, contiguous in both
+    if ((s = loadable16(ctx, dtype, B, K, N, &x, &ldx)) != FG_OK) return s;
+    v = ConvProduct{operand16(dz, ldz, false), operand16(x, ldx, false), epilogue16(ctx, dtype, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr), 1};
+    return dB ? lowp_gemm_both(ctx, w, v) : lowp_gemm(ctx, v);
 }
 
 }  // extern "C"

@@ -92,8 +92,8 @@ uint64_t fg_ctx_workspace_bytes(fg_ctx* ctx);
 /* Tuning and debugging switches of one context (no counterpart in the reference, whose only switch is
  * CompilationOptions: dispatch/mod.rs:369-455).  Values are strings.
  *   "gemm_tile"     "auto" (default) | "pair" | "256x32" | "256x16" | "128x32" | "128x16": the tensor-core tile
- *   "gemm_conv"     "auto" (default) | "<width>x<shares>" with a tile width of 64 or 128 and 1..8 K-shares, as "64x3": f32
- *                   products that the conversion kernel can run go to it, with this tile and (where k is long enough)
+ *   "gemm_conv"     "auto" (default) | "<width>x<shares>" with a tile width of 64 or 128 and 1..8 K-shares, as "64x3": f32 and 16-bit
+ *                   products that the conversion or the half kernel can run go to it, with this tile and (where k is long enough)
  *                   these shares, and both gradients of a layer in one launch
  *   "gemm_split_k"  "1" (default) | "0": cut the tiles of an under-filled last wave into K-shares
  *   "gemm_group"    "0" (default: by shape) | 1..64: tile rows per group of the pair kernel's tile order
