@@ -26,6 +26,8 @@
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "fg_internal.cuh"
 #include "ptx_sm100.cuh"
 
@@ -1194,82 +1196,139 @@ template <> __device__ __forceinline__ float lp_from_float<float>(float v) { ret
 template <> __device__ __forceinline__ __half lp_from_float<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 lp_from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-// W columns per thread (16 bytes, or 1: any shape and alignment), 32 rows x 32 * W columns per block.
-template <typename T, int W>
-__global__ void __launch_bounds__(256) prep_kernel(const PrepArgs a) {
-    fg_grid_enter();
-    __shared__ float cs[8][32 * W + 1];
-    const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * W;
-    const uint32_t r0 = blockIdx.y * 32;
-    struct __align__(W * sizeof(T)) Vec { T e[W]; };
-    const T* const x = static_cast<const T*>(a.x) + blockIdx.z * a.x_batch;
-    const T* const saved = a.saved ? static_cast<const T*>(a.saved) + blockIdx.z * a.x_batch : nullptr;
-    T* const out = a.out ? static_cast<T*>(a.out) + (size_t)blockIdx.z * a.R * a.ld : nullptr;
-    T* const copy = a.copy ? static_cast<T*>(a.copy) + (size_t)blockIdx.z * a.R * a.C : nullptr;
+// 32 rows x 32 * W columns per block, W columns per thread: 16 bytes of them, or, for any shape and alignment, one in 32.  All loads
+// first, three blocks an SM by registers and column sums that lie 36 words apart: with eight apart and two blocks an SM, dZ of
+// 2048 x 4096 bf16 through GELU took 20 - 30 us for 50 MB.
+constexpr int kPrepPitch = 36;
+template <typename T, int W, bool VEC>
+__device__ __forceinline__ void prep_block(const PrepArgs& a, uint32_t bx, uint32_t by, uint32_t bz, float* cs) {
+    const uint32_t x0 = bx * 32 * W, c = VEC ? x0 + threadIdx.x * W : x0 + threadIdx.x, r0 = by * 32 + threadIdx.y;
+    struct __align__(VEC ? W * sizeof(T) : sizeof(T)) Vec { T e[W]; };
+    const T* const x = static_cast<const T*>(a.x) + bz * a.x_batch;
+    const T* const saved = a.saved ? static_cast<const T*>(a.saved) + bz * a.x_batch : nullptr;
+    T* const out = a.out ? static_cast<T*>(a.out) + (size_t)bz * a.R * a.ld : nullptr;
+    T* const copy = a.copy ? static_cast<T*>(a.copy) + (size_t)bz * a.R * a.C : nullptr;
+    auto load = [&](const T* p, uint32_t r, Vec& v) {
+        p += (size_t)r * a.C + c;
+        if constexpr (VEC) v = *reinterpret_cast<const Vec*>(p);
+        else
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+                if (c + 32 * w < a.C) v.e[w] = p[32 * w];
+    };
+    auto store = [&](T* p, uint32_t r, uint32_t ld, const Vec& v) {
+        p += (size_t)r * ld + c;
+        if constexpr (VEC) *reinterpret_cast<Vec*>(p) = v;
+        else
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+                if (c + 32 * w < a.C) p[32 * w] = v.e[w];
+    };
     float sum[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) sum[w] = 0.0f;
     if (c < a.C) {
         Vec v[4], sv[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {       // all loads first
-            const uint32_t r = r0 + threadIdx.y + 8 * k;
-            if (r >= a.R) continue;
-            v[k] = *reinterpret_cast<const Vec*>(x + (size_t)r * a.C + c);
-            if (saved) sv[k] = *reinterpret_cast<const Vec*>(saved + (size_t)r * a.C + c);
-        }
+        for (int k = 0; k < 4; ++k)
+            if (r0 + 8 * k < a.R) {
+                load(x, r0 + 8 * k, v[k]);
+                if (saved) load(saved, r0 + 8 * k, sv[k]);
+            }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint32_t r = r0 + threadIdx.y + 8 * k;
+            const uint32_t r = r0 + 8 * k;
             if (r >= a.R) continue;
             if (saved) {
+                // (the activation is chosen for a row: between choices the W elements' chains run side by side)
+                auto factor = [&](auto act) {
 #pragma unroll
-                for (int w = 0; w < W; ++w) v[k].e[w] = lp_from_float<T>(lp_to_float(v[k].e[w]) * fg_act_grad(a.act, lp_to_float(sv[k].e[w])));
+                    for (int w = 0; w < W; ++w) v[k].e[w] = lp_from_float<T>(lp_to_float(v[k].e[w]) * fg_act_grad(decltype(act)::value, lp_to_float(sv[k].e[w])));
+                };
+                if (a.act == FG_ACT_GELU) factor(std::integral_constant<int, FG_ACT_GELU>{});
+                else if (a.act == FG_ACT_TANH) factor(std::integral_constant<int, FG_ACT_TANH>{});
+                else if (a.act == FG_ACT_RELU) factor(std::integral_constant<int, FG_ACT_RELU>{});
             }
-            if (out) *reinterpret_cast<Vec*>(out + (size_t)r * a.ld + c) = v[k];
-            if (copy) *reinterpret_cast<Vec*>(copy + (size_t)r * a.C + c) = v[k];
+            if (out) store(out, r, a.ld, v[k]);
+            if (copy) store(copy, r, a.C, v[k]);
 #pragma unroll
             for (int w = 0; w < W; ++w) sum[w] += lp_to_float(v[k].e[w]);
         }
     }
     if (!a.colsum_part) return;
 #pragma unroll
-    for (int w = 0; w < W; ++w) cs[threadIdx.y][threadIdx.x * W + w] = sum[w];
+    for (int w = 0; w < W; ++w) cs[(threadIdx.y * W + w) * kPrepPitch + threadIdx.x] = sum[w];
     __syncthreads();
-    const uint32_t t = threadIdx.y * 32 + threadIdx.x, col = blockIdx.x * (32 * W) + t;
+    const uint32_t t = threadIdx.y * 32 + threadIdx.x, col = x0 + t;
     if (t < 32 * W && col < a.C) {
         float z = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) z += cs[k][t];
-        a.colsum_part[(size_t)blockIdx.y * a.C + col] = z;
+        for (int k = 0; k < 8; ++k) z += cs[(k * W + (VEC ? t % W : t / 32)) * kPrepPitch + (VEC ? t / W : t % 32)];
+        a.colsum_part[(size_t)by * a.C + col] = z;
     }
 }
 
-// a.out, when given, is scratch: 16-byte aligned with a 16-byte pitch.
-int32_t launch_prep(fg_ctx* ctx, int dtype, const PrepArgs& a, uint32_t batch = 1) {
-    const uint32_t per16 = dtype == FG_DTYPE_F32 ? 4 : 8;
-    const bool vec = a.C % per16 == 0 && (batch == 1 || a.x_batch % per16 == 0) && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved)) &&
-                     (!a.copy || fg_aligned16(a.copy));
-    const uint32_t w = 32 * (vec ? per16 : 1);
-    dim3 grid((a.C + w - 1) / w, (a.R + 31) / 32, batch), block(32, 8);
-    if (grid.y > 65535 || batch > 65535) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM operand has too many rows");
-    const double es = dtype == FG_DTYPE_F32 ? 4.0 : 2.0;
-    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT,
-                                    es * batch * a.R * a.C * (1.0 + (a.saved ? 1.0 : 0.0) + (a.out ? 1.0 : 0.0) + (a.copy ? 1.0 : 0.0)));
-    if (dtype == FG_DTYPE_F32) {
-        if (vec) fg_launch(ctx, prep_kernel<float, 4>, grid, block, 0, a);
-        else fg_launch(ctx, prep_kernel<float, 1>, grid, block, 0, a);
-    } else if (dtype == FG_DTYPE_F16) {
-        if (vec) fg_launch(ctx, prep_kernel<__half, 8>, grid, block, 0, a);
-        else fg_launch(ctx, prep_kernel<__half, 1>, grid, block, 0, a);
-    } else {
-        if (vec) fg_launch(ctx, prep_kernel<__nv_bfloat16, 8>, grid, block, 0, a);
-        else fg_launch(ctx, prep_kernel<__nv_bfloat16, 1>, grid, block, 0, a);
-    }
-    fg_time_end(ctx, tr);
-    FG_LAUNCHED(ctx);
-    return FG_OK;
+// Up to three passes in a launch, one after the other in the grid: what a product or a backward pass needs beforehand are short,
+// independent passes (a ragged layer's dZ and copies of its input and weights, 3.5 - 5 us each: backward of 1000 x 777 x 1001
+// 40.9 -> 38 - 39 us).
+struct PrepJobs {
+    PrepArgs job[3];
+    uint32_t width[3], gx[3], gy[3], first[4];      // columns per thread (0: 16 bytes of them); blocks across and down a matrix; the first block of each
+};
+template <typename T>
+__global__ void __launch_bounds__(256, 3) prep_kernel(const __grid_constant__ PrepJobs p) {
+    fg_grid_enter();
+    constexpr int W = 16 / sizeof(T);
+    __shared__ float room[8 * W * kPrepPitch];
+    const uint32_t j = blockIdx.x >= p.first[2] ? 2u : blockIdx.x >= p.first[1] ? 1u : 0u, b = blockIdx.x - p.first[j];
+    const uint32_t bx = b % p.gx[j], r = b / p.gx[j], by = r % p.gy[j], bz = r / p.gy[j];
+    if (p.width[j] == 0) prep_block<T, W, true>(p.job[j], bx, by, bz, room);
+    else if (p.width[j] == 4) prep_block<T, 4, false>(p.job[j], bx, by, bz, room);
+    else prep_block<T, 2, false>(p.job[j], bx, by, bz, room);
 }
+
+// Passes that have been asked for and not been launched.
+struct PrepBatch {
+    PrepJobs jobs{};
+    int n = 0, dtype = FG_DTYPE_F32;
+    double bytes = 0.0;
+
+    // a.out, when given, is scratch: 16-byte aligned with a 16-byte pitch.
+    int32_t add(fg_ctx* ctx, int type, const PrepArgs& a, uint32_t batch = 1) {
+        if (n == 3 || (n && type != dtype)) {
+            const int32_t s = launch(ctx);
+            if (s != FG_OK) return s;
+        }
+        dtype = type;
+        const uint32_t per16 = dtype == FG_DTYPE_F32 ? 4 : 8;
+        const bool vec = a.C % per16 == 0 && (batch == 1 || a.x_batch % per16 == 0) && fg_aligned16(a.x) && (!a.saved || fg_aligned16(a.saved)) &&
+                         (!a.copy || fg_aligned16(a.copy));
+        // four columns a thread where that still makes two blocks an SM (backward of 1000 x 777 x 1001 37.8 us, 39.5 with two)
+        const uint32_t wide = (uint64_t)((a.C + 127) / 128) * ((a.R + 31) / 32) * batch >= 2ull * (uint64_t)ctx->sm_count ? 4 : 2;
+        const uint32_t w = 32 * (vec ? per16 : wide), gx = (a.C + w - 1) / w, gy = (a.R + 31) / 32;
+        const uint64_t end = jobs.first[n] + (uint64_t)gx * gy * batch;
+        if (gy > 65535 || batch > 65535 || end > 0x7fffffffull) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM operand has too many rows");
+        jobs.job[n] = a;
+        jobs.width[n] = vec ? 0 : wide; jobs.gx[n] = gx; jobs.gy[n] = gy;
+        for (int k = ++n; k < 4; ++k) jobs.first[k] = (uint32_t)end;
+        bytes += (dtype == FG_DTYPE_F32 ? 4.0 : 2.0) * batch * a.R * a.C * (1.0 + (a.saved ? 1.0 : 0.0) + (a.out ? 1.0 : 0.0) + (a.copy ? 1.0 : 0.0));
+        return FG_OK;
+    }
+    int32_t launch(fg_ctx* ctx) {
+        if (!n) return FG_OK;
+        const dim3 block(32, 8);
+        fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT, bytes);
+        if (dtype == FG_DTYPE_F32) fg_launch(ctx, prep_kernel<float>, jobs.first[n], block, 0, jobs);
+        else if (dtype == FG_DTYPE_F16) fg_launch(ctx, prep_kernel<__half>, jobs.first[n], block, 0, jobs);
+        else fg_launch(ctx, prep_kernel<__nv_bfloat16>, jobs.first[n], block, 0, jobs);
+        fg_time_end(ctx, tr);
+        n = 0;
+        bytes = 0.0;
+        jobs.first[0] = 0;
+        FG_LAUNCHED(ctx);
+        return FG_OK;
+    }
+};
 
 // ------------------------------------------------------------------------------------
 // Conversion kernel: small and middling products of f32 tensors, straight from the tensors.
@@ -2665,14 +2724,14 @@ double pair16_cycles(const fg_ctx* ctx, const ConvShape& sh) {
 }
 
 // A dense [R, C] f32 tensor (`batch` of them, x_batch apart) can be loaded as it lies when rows and matrices start on
-// 16-byte boundaries; otherwise from a padded copy.
+// 16-byte boundaries; otherwise from a padded copy (loadable32 leaves it to `prep`).
 inline bool in_place32(const float* x, uint32_t C, uint32_t batch, uint64_t x_batch) {
     return fg_aligned16(x) && C % 4 == 0 && (batch == 1 || x_batch % 4 == 0);
 }
 inline uint64_t copy32_bytes(const float* x, uint32_t R, uint32_t C, uint32_t batch, uint64_t x_batch) {
     return in_place32(x, C, batch, x_batch) ? 0 : (uint64_t)batch * R * round4(C) * 4 + 256;
 }
-int32_t loadable32(fg_ctx* ctx, const float* x, uint32_t R, uint32_t C, uint32_t batch, uint64_t x_batch, PlaneSet* o) {
+int32_t loadable32(fg_ctx* ctx, const float* x, uint32_t R, uint32_t C, uint32_t batch, uint64_t x_batch, PlaneSet* o, PrepBatch* prep) {
     *o = PlaneSet{};
     o->p32 = const_cast<float*>(x);
     o->ld32 = C;
@@ -2686,7 +2745,7 @@ int32_t loadable32(fg_ctx* ctx, const float* x, uint32_t R, uint32_t C, uint32_t
     o->p32 = (float*)p;
     o->ld32 = a.ld;
     o->batch32 = (uint64_t)R * a.ld;
-    return launch_prep(ctx, FG_DTYPE_F32, a, batch);
+    return prep->add(ctx, FG_DTYPE_F32, a, batch);
 }
 inline PlaneSet as_operand(PlaneSet o, bool mn) { o.mn = mn; return o; }
 
@@ -2908,8 +2967,10 @@ int32_t gemm_fwd_core(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
             int32_t s = fg_ws_ensure(ctx, ca + cb + 1024);
             if (s != FG_OK) return s;
             PlaneSet pa, pb;
-            if ((s = loadable32(ctx, A.x, rows_a, pitch_a, 1, 0, &pa)) != FG_OK) return s;
-            if ((s = loadable32(ctx, B.x, rows_b, pitch_b, 1, 0, &pb)) != FG_OK) return s;
+            PrepBatch prep;
+            if ((s = loadable32(ctx, A.x, rows_a, pitch_a, 1, 0, &pa, &prep)) != FG_OK) return s;
+            if ((s = loadable32(ctx, B.x, rows_b, pitch_b, 1, 0, &pb, &prep)) != FG_OK) return s;
+            if ((s = prep.launch(ctx)) != FG_OK) return s;
             Epilogue ep{C, bias, preact_out, M, N, K, act, ctx->dev_status};
             ep.c_pairs = c_pairs;
             ep.c_pairs_stride = c_stride;
@@ -3180,7 +3241,8 @@ BwdRoutes pick_bwd_routes(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K,
 // The two products of a backward step by their routes; dZ has row pitch ldz (N, or padded for the conversion kernel).  The
 // caller has reserved what they carve.
 int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, PairedArg A, PairedArg B, PairedArg dZ, uint32_t ldz,
-                          const BwdRoutes& rt, float* dB, float* dA, const PairedOut& o, float* exch_buf, uint64_t exch_count) {
+                          const BwdRoutes& rt, float* dB, float* dA, const PairedOut& o, float* exch_buf, uint64_t exch_count, PrepBatch& prep,
+                          uint32_t bias_rows, const float* bias_part, float* dbias) {
     int32_t s;
     const uint64_t mk = (uint64_t)M * K, kn = (uint64_t)K * N, mn = (uint64_t)M * N;
     const bool pair_b = dB && rt.dB.kind == kRoutePair, pair_a = dA && rt.dA.kind == kRoutePair;
@@ -3193,12 +3255,17 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         t.pairs = q; t.stride = n;
         return FG_OK;
     };
-    PlaneSet z32;
-    if ((pair_a || pair_b) && (s = make_pairs(dZ, mn)) != FG_OK) return s;
+    // What the conversion kernel cannot read in place joins the passes that the caller has left; then the layer's bias gradient.
+    PlaneSet z32, a32, b32;
     if (conv_b || conv_a) {
-        if (ldz == N && (s = loadable32(ctx, dZ.x, M, N, 1, 0, &z32)) != FG_OK) return s;
+        if (ldz == N && (s = loadable32(ctx, dZ.x, M, N, 1, 0, &z32, &prep)) != FG_OK) return s;
         if (ldz != N) { z32 = PlaneSet{}; z32.p32 = const_cast<float*>(dZ.x); z32.ld32 = ldz; }
     }
+    if (conv_b && (s = loadable32(ctx, A.x, M, K, 1, 0, &a32, &prep)) != FG_OK) return s;
+    if (conv_a && (s = loadable32(ctx, B.x, K, N, 1, 0, &b32, &prep)) != FG_OK) return s;
+    if ((s = prep.launch(ctx)) != FG_OK) return s;
+    if (dbias && (s = fg_colsum_fold_launch(ctx, N, bias_rows, bias_part, dbias)) != FG_OK) return s;
+    if ((pair_a || pair_b) && (s = make_pairs(dZ, mn)) != FG_OK) return s;
     const bool one = conv_b && conv_a && !exch_buf;      // both gradients in one launch
     ConvProduct both[2];
     if (pair_b) {
@@ -3209,8 +3276,6 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         if ((s = paired_gemm(ctx, pa, pz, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr, PairedOut{nullptr, 0, nullptr, 0, nullptr})) != FG_OK)
             return s;
     } else if (conv_b) {
-        PlaneSet a32;
-        if ((s = loadable32(ctx, A.x, M, K, 1, 0, &a32)) != FG_OK) return s;
         const Epilogue ep{dB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
         both[0] = ConvProduct{as_operand(a32, true), as_operand(z32, true), ep, 1};
         if (!one && (s = launch_conv(ctx, &both[0], 1, rt.dB.conv)) != FG_OK) return s;
@@ -3224,8 +3289,6 @@ int32_t gemm_bwd_products(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Paire
         const PlaneSet pb = paired_operand(B.x, B.pairs, B.stride, N, true);
         if ((s = paired_gemm(ctx, pz, pb, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr, o)) != FG_OK) return s;
     } else if (conv_a) {
-        PlaneSet b32;
-        if ((s = loadable32(ctx, B.x, K, N, 1, 0, &b32)) != FG_OK) return s;
         Epilogue ep{dA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
         ep.c_pairs = o.pairs;
         ep.c_pairs_stride = o.stride;
@@ -3288,7 +3351,8 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
     if (!rt.planes && (dA || dB)) {
         PairedOut po = o;
         po.colsum_part = cs_part;
-        if ((s = gemm_bwd_products(ctx, M, N, K, A, B, dZ, N, rt, dB, dA, po, exch_buf, exch_count)) != FG_OK) return s;
+        PrepBatch prep;
+        if ((s = gemm_bwd_products(ctx, M, N, K, A, B, dZ, N, rt, dB, dA, po, exch_buf, exch_count, prep, 0, nullptr, nullptr)) != FG_OK) return s;
         if (!dA || rt.dA.kind != kRoutePlanes)
             return cs_part ? fg_colsum_fold_launch(ctx, K, cs_chunks, cs_part, dbias_prev) : FG_OK;
     } else if ((s = gemm_bwd_planes(ctx, FG_GEMM_AUTO, M, N, K, A.x, B.x, dZ.x, FG_ACT_NONE, nullptr, dA, dB, nullptr, nullptr, exch_buf,
@@ -3381,6 +3445,7 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
             }
             { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
             int32_t s;
+            PrepBatch prep;
             void *pz = nullptr, *dzb = nullptr, *csp = nullptr;
             if (dbias && (s = fg_ws_alloc(ctx, (uint64_t)cs_chunks * N * 4, &csp)) != FG_OK) return s;
             PairedArg z{dY, nullptr, 0};
@@ -3401,12 +3466,11 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
                     a.out = dzb; a.ld = round4(N);
                     a.copy = dZ_out;
                 } else a.copy = dZ_out;
-                if ((s = launch_prep(ctx, FG_DTYPE_F32, a)) != FG_OK) return s;
+                if ((s = prep.add(ctx, FG_DTYPE_F32, a)) != FG_OK) return s;
                 if (own_z) z.x = dzb ? (const float*)dzb : dZ_out;
             }
-            if (dbias && (s = fg_colsum_fold_launch(ctx, N, cs_chunks, (const float*)csp, dbias)) != FG_OK) return s;
             return gemm_bwd_products(ctx, M, N, K, PairedArg{A, nullptr, 0}, PairedArg{B, nullptr, 0}, z, own_z && !z_dense && !want_pairs ? round4(N) : N, rt,
-                                     dB, dA, PairedOut{nullptr, 0, nullptr, 0, nullptr}, exch_buf, exch_count);
+                                     dB, dA, PairedOut{nullptr, 0, nullptr, 0, nullptr}, exch_buf, exch_count, prep, cs_chunks, (const float*)csp, dbias);
         }
     }
     return gemm_bwd_planes(ctx, mode, M, N, K, A, B, dY, act, saved, dA, dB, dbias, dZ_out, exch_buf, exch_count);
@@ -3530,8 +3594,10 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
                 ctx->ws_used = 0;
                 int32_t s = fg_ws_ensure(ctx, need(t));
                 if (s != FG_OK) return s;
-                if ((s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &pa)) != FG_OK) return s;
-                if ((s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &pb)) != FG_OK) return s;
+                PrepBatch prep;
+                if ((s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &pa, &prep)) != FG_OK) return s;
+                if ((s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &pb, &prep)) != FG_OK) return s;
+                if ((s = prep.launch(ctx)) != FG_OK) return s;
                 Epilogue ep{C + t0 * strideC, bias, preact_out ? preact_out + t0 * strideC : nullptr, M, N, K, act, ctx->dev_status};
                 ep.c_batch = t > 1 ? strideC : 0;
                 if ((s = launch_conv(ctx, as_operand(pa, false), as_operand(pb, true), ep, plan_conv(ctx, M, N, K, t), t)) != FG_OK) return s;
@@ -3632,7 +3698,8 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
         for (uint32_t t0 = 0; t0 < batch && all; t0 += part) {
             const uint32_t t = batch - t0 < part ? batch - t0 : part;
             const float* const dy = dY + t0 * strideC;
-            PlaneSet z, x;
+            PlaneSet z, xa, xb;
+            PrepBatch prep;
             ConvProduct both[2];
             ctx->ws_used = 0;
             int32_t s = fg_ws_ensure(ctx, need(t));
@@ -3642,24 +3709,25 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
                 if ((s = fg_ws_alloc(ctx, (uint64_t)t * M * round4(N) * 4, &p)) != FG_OK) return s;
                 PrepArgs a{};
                 a.x = dy; a.saved = saved + t0 * strideC; a.act = act; a.R = M; a.C = N; a.x_batch = strideC; a.out = p; a.ld = round4(N);
-                if ((s = launch_prep(ctx, FG_DTYPE_F32, a, t)) != FG_OK) return s;
+                if ((s = prep.add(ctx, FG_DTYPE_F32, a, t)) != FG_OK) return s;
                 z = PlaneSet{};
                 z.p32 = (float*)p;
                 z.ld32 = round4(N);
                 z.batch32 = (uint64_t)M * round4(N);
-            } else if ((s = loadable32(ctx, dy, M, N, t, strideC, &z)) != FG_OK) return s;
+            } else if ((s = loadable32(ctx, dy, M, N, t, strideC, &z, &prep)) != FG_OK) return s;
+            if (dB && (s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &xa, &prep)) != FG_OK) return s;
+            if (dA && (s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &xb, &prep)) != FG_OK) return s;
+            if ((s = prep.launch(ctx)) != FG_OK) return s;
             if (dB) {
-                if ((s = loadable32(ctx, A + t0 * strideA, M, K, t, strideA, &x)) != FG_OK) return s;
                 Epilogue ep{dB + t0 * strideB, nullptr, nullptr, K, N, M, FG_ACT_NONE, ctx->dev_status};
                 ep.c_batch = t > 1 ? strideB : 0;
-                both[0] = ConvProduct{as_operand(x, true), as_operand(z, true), ep, t};
+                both[0] = ConvProduct{as_operand(xa, true), as_operand(z, true), ep, t};
                 if (!dA && (s = launch_conv(ctx, &both[0], 1, plan_conv(ctx, K, N, M, t))) != FG_OK) return s;
             }
             if (dA) {
-                if ((s = loadable32(ctx, B + t0 * strideB, K, N, t, strideB, &x)) != FG_OK) return s;
                 Epilogue ep{dA + t0 * strideA, nullptr, nullptr, M, K, N, FG_ACT_NONE, ctx->dev_status};
                 ep.c_batch = t > 1 ? strideA : 0;
-                both[1] = ConvProduct{as_operand(z, false), as_operand(x, false), ep, t};
+                both[1] = ConvProduct{as_operand(z, false), as_operand(xb, false), ep, t};
                 if ((s = dB ? launch_conv_both(ctx, both[0], both[1]) : launch_conv(ctx, &both[1], 1, plan_conv(ctx, M, K, N, t))) != FG_OK) return s;
             }
         }
@@ -3691,7 +3759,7 @@ inline bool in_place16(const void* p, uint32_t cols) { return fg_aligned16(p) &&
 inline uint64_t copy16_bytes(const void* p, uint32_t rows, uint32_t cols) { return in_place16(p, cols) ? 0 : (uint64_t)rows * pad8(cols) * 2 + 256; }
 
 // x itself, or its copy with a padded pitch; *ld receives the pitch.
-int32_t loadable16(fg_ctx* ctx, int dtype, const void* x, uint32_t rows, uint32_t cols, const void** out, uint32_t* ld) {
+int32_t loadable16(fg_ctx* ctx, int dtype, const void* x, uint32_t rows, uint32_t cols, const void** out, uint32_t* ld, PrepBatch* prep) {
     *out = x;
     *ld = cols;
     if (in_place16(x, cols)) return FG_OK;
@@ -3702,7 +3770,7 @@ int32_t loadable16(fg_ctx* ctx, int dtype, const void* x, uint32_t rows, uint32_
     a.x = x; a.R = rows; a.C = cols; a.out = p; a.ld = pad8(cols);
     *out = p;
     *ld = a.ld;
-    return launch_prep(ctx, dtype, a);
+    return prep->add(ctx, dtype, a);
 }
 
 // An operand whose rows are the output's rows or columns; mn: the storage is [contraction][rows].
@@ -3769,8 +3837,10 @@ int32_t fg_gemm_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uint32_
     int32_t s;
     const void *a, *b;
     uint32_t lda, ldb;
-    if ((s = loadable16(ctx, dtype, A, M, K, &a, &lda)) != FG_OK) return s;
-    if ((s = loadable16(ctx, dtype, B, K, N, &b, &ldb)) != FG_OK) return s;
+    PrepBatch prep;
+    if ((s = loadable16(ctx, dtype, A, M, K, &a, &lda, &prep)) != FG_OK) return s;
+    if ((s = loadable16(ctx, dtype, B, K, N, &b, &ldb, &prep)) != FG_OK) return s;
+    if ((s = prep.launch(ctx)) != FG_OK) return s;
     // A [M][K] has the contraction index contiguous, B [K][N] its rows (the output's columns)
     return lowp_gemm(ctx, ConvProduct{operand16(a, lda, false), operand16(b, ldb, true), epilogue16(ctx, dtype, M, N, K, C, bias, act, preact_out), 1});
 }
@@ -3809,22 +3879,20 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
         if ((s = fg_ws_alloc(ctx, (uint64_t)nchunk_rows * N * 4, &cs_part)) != FG_OK) return s;
         pz.colsum_part = (float*)cs_part;
     }
-    if ((pz.out || pz.colsum_part) && (s = launch_prep(ctx, dtype, pz)) != FG_OK) return s;
+    // dZ and the copies of what cannot be read in place: one launch
+    PrepBatch prep;
+    const void *xa = nullptr, *xb = nullptr;
+    uint32_t lda = 0, ldb = 0;
+    if ((pz.out || pz.colsum_part) && (s = prep.add(ctx, dtype, pz)) != FG_OK) return s;
+    if (dB && (s = loadable16(ctx, dtype, A, M, K, &xa, &lda, &prep)) != FG_OK) return s;
+    if (dA && (s = loadable16(ctx, dtype, B, K, N, &xb, &ldb, &prep)) != FG_OK) return s;
+    if ((s = prep.launch(ctx)) != FG_OK) return s;
     if (dbias && (s = fg_colsum_fold_launch(ctx, N, nchunk_rows, (const float*)cs_part, dbias, dtype)) != FG_OK) return s;
-    const void* x;
-    uint32_t ldx;
-    ConvProduct w{}, v{};
-    if (dB) {
-        // dB[K,N] = A^T · dZ: contraction over M, the row index of both tensors
-        if ((s = loadable16(ctx, dtype, A, M, K, &x, &ldx)) != FG_OK) return s;
-        w = ConvProduct{operand16(x, ldx, true), operand16(dz, ldz, true), epilogue16(ctx, dtype, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr), 1};
-        if (!dA) return lowp_gemm(ctx, w);
-    }
-    if (!dA) return FG_OK;
-    // dA[M,K] = dZ · B^T: contraction over N, contiguous in both
-    if ((s = loadable16(ctx, dtype, B, K, N, &x, &ldx)) != FG_OK) return s;
-    v = ConvProduct{operand16(dz, ldz, false), operand16(x, ldx, false), epilogue16(ctx, dtype, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr), 1};
-    return dB ? lowp_gemm_both(ctx, w, v) : lowp_gemm(ctx, v);
+    // dB[K,N] = A^T · dZ: contraction over M, the row index of both tensors; dA[M,K] = dZ · B^T: contraction over N, contiguous in both
+    const ConvProduct w{operand16(xa, lda, true), operand16(dz, ldz, true), epilogue16(ctx, dtype, K, N, M, dB, nullptr, FG_ACT_NONE, nullptr), 1};
+    const ConvProduct v{operand16(dz, ldz, false), operand16(xb, ldb, false), epilogue16(ctx, dtype, M, K, N, dA, nullptr, FG_ACT_NONE, nullptr), 1};
+    if (dB && dA) return lowp_gemm_both(ctx, w, v);
+    return dB ? lowp_gemm(ctx, w) : dA ? lowp_gemm(ctx, v) : FG_OK;
 }
 
 }  // extern "C"
