@@ -74,6 +74,28 @@ ConvPlan conv_plan_fixed(const ConvShape* sh, int n, uint32_t bn, uint32_t split
     return ConvPlan{bn, split, 1.0};
 }
 
+// Two products walked by `pairs` workers in one launch: worker p takes tiles p, p + pairs, ... of the n0 of the first, which cost w0
+// each, then a run of the n1 tiles of the second (w1 <= w0 each), longer for those with fewer of the first.  Workers below `extra`
+// have one more of the first and take run[0] of the second, the others run[1]; the largest sum is `cost`, the least there is.
+struct PairRuns { uint64_t pairs; uint32_t extra, run[2]; double cost; };
+inline PairRuns pair_runs(uint64_t pairs, uint64_t n0, double w0, uint64_t n1, double w1) {
+    const uint64_t c0 = n0 / pairs, extra = n0 % pairs;
+    PairRuns best{pairs, (uint32_t)extra, {0, 0}, 0.0};
+    const double more = (double)(extra ? c0 + 1 : c0) * w0, less = (double)c0 * w0;
+    // the cost is a worker's own: `more` or `less` and a whole number of w1
+    const uint64_t most = (n1 + pairs - 1) / pairs + (uint64_t)(w0 / w1) + 2;
+    for (uint64_t i = 0; i <= most; ++i)
+        for (int from = 0; from < 2; ++from) {
+            const double cost = (from ? more : less) + (double)i * w1;
+            if (cost < more || (best.cost > 0.0 && cost >= best.cost)) continue;
+            const uint64_t s0 = (uint64_t)((cost - more) / w1 + 1e-6), s1 = (uint64_t)((cost - less) / w1 + 1e-6);
+            if (extra * s0 + (pairs - extra) * s1 < n1) continue;
+            best.run[0] = (uint32_t)s0; best.run[1] = (uint32_t)s1;
+            best.cost = cost;
+        }
+    return best;
+}
+
 // Of `fit` clusters that run at once on `all` SMs, those that do on `sms` of them: the exchange's CTAs may sit anywhere.
 inline int conv_clusters_beside(int fit, uint64_t sms, uint64_t all) {
     if (fit < 1 || sms >= all) return fit;

@@ -436,10 +436,21 @@ struct PairCfg {
 // while the epilogue warps apply bias/activation and store tile t from their registers, the loads and
 // MMAs of tile t+1 are already under way (per-tile set-up, fill and store cost 20-55 us per wave when
 // every tile was its own CTA pair: 17 % of a 4096^3 GEMM, more than half of a K = 784 one).
-template <int BK, int FMT>
+// Two products in a launch (both gradients of a 16-bit layer): a pair takes tiles pair, pair + P, ... of the first, then a run of the
+// second's, as long as evens the pairs out (the host's counts, see pair_runs): 384 tiles of which 128 have twice the k are seven
+// times of the short ones on 74 pairs instead of the eight of two launches.
+template <bool TWO>
+struct PairArgs {
+    Epilogue ep[TWO ? 2 : 1];
+    uint32_t extra;          // pairs with one tile of the first product more than the others: pairs 0 ... extra - 1
+    uint32_t run[2];         // tiles of the second product for one of those, and for one of the others
+};
+template <int BK, int FMT, bool TWO>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ CUtensorMap tmA16, const __grid_constant__ CUtensorMap tmB16, Epilogue ep) {
+                    const __grid_constant__ CUtensorMap tmA16, const __grid_constant__ CUtensorMap tmB16,
+                    const __grid_constant__ PairArgs<TWO> pa) {
+    static_assert(!TWO || FMT >= 2, "the second product's maps take the place of the f32 ones");
     static_assert(FMT == 0 || BK == 32, "the bf16 planes use 64-byte rows: 32 values of k per block");
     // FMT 2 (bf16) and 3 (f16): the operands ARE 16-bit tensors, loaded as they lie (64 values of k per k-block)
     // and multiplied by one kind::f16 MMA per 16 values of k.
@@ -467,28 +478,43 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank(), 0);
     const bool leader = rank == 0;
-    const uint32_t pairs_m = (ep.M + 2 * BM - 1) / (2 * BM), pairs_n = (ep.N + BN - 1) / BN;
-    const uint32_t ntiles = pairs_m * pairs_n;
     const uint32_t npairs = gridDim.x >> 1, pair = blockIdx.x >> 1;
-    auto tile_origin = [&](uint32_t tile, uint32_t& m0, uint32_t& n0) {
-        pair_tile_origin(tile, pairs_m, pairs_n, 2 * BM, BN, ep.group, m0, n0);
+    constexpr uint32_t kChunkKB = kChunk / KBE;
+    int* const dev_status = pa.ep[0].dev_status;
+    // One product's tiles and units.  Work units: whole tiles first, then the tail tiles in `split` K-shares each (the host sizes the
+    // tail so that it fills one last wave instead of leaving most pairs idle for a whole tile time).
+    struct Units {
+        uint32_t pairs_m, pairs_n, nkb, nchunks, n;
+    };
+    auto units_of = [&](const Epilogue& ep) -> Units {
+        Units w;
+        w.pairs_m = (ep.M + 2 * BM - 1) / (2 * BM);
+        w.pairs_n = (ep.N + BN - 1) / BN;
+        w.nkb = (ep.K + KBE - 1) / KBE;
+        w.nchunks = (w.nkb + kChunkKB - 1) / kChunkKB;
+        w.n = ep.t_full + (w.pairs_m * w.pairs_n - ep.t_full) * ep.split;
+        return w;
+    };
+    auto tile_origin = [&](const Epilogue& ep, const Units& w, uint32_t tile, uint32_t& m0, uint32_t& n0) {
+        pair_tile_origin(tile, w.pairs_m, w.pairs_n, 2 * BM, BN, ep.group, m0, n0);
         m0 += rank * BM;                                               // this CTA's rows of A and C
     };
-    const uint32_t nkb = (ep.K + KBE - 1) / KBE;
-    constexpr uint32_t kChunkKB = kChunk / KBE;
-    const uint32_t nchunks = (nkb + kChunkKB - 1) / kChunkKB;
-    // Work units: whole tiles first, then the tail tiles in `split` K-shares each (the host sizes the
-    // tail so that it fills one last wave instead of leaving most pairs idle for a whole tile time).
-    const uint32_t nunits = ep.t_full + (ntiles - ep.t_full) * ep.split;
-    auto unit_at = [&](uint32_t u, uint32_t& tile, uint32_t& c0, uint32_t& c1, uint32_t& slot) -> bool {
-        if (u < ep.t_full) { tile = u; c0 = 0; c1 = nchunks; slot = 0; return false; }
+    auto unit_at = [&](const Epilogue& ep, const Units& w, uint32_t u, uint32_t& tile, uint32_t& c0, uint32_t& c1, uint32_t& slot) -> bool {
+        if (u < ep.t_full) { tile = u; c0 = 0; c1 = w.nchunks; slot = 0; return false; }
         const uint32_t v = u - ep.t_full, p = v % ep.split;
         tile = ep.t_full + v / ep.split;
-        c0 = p * nchunks / ep.split;
-        c1 = (p + 1) * nchunks / ep.split;
+        c0 = p * w.nchunks / ep.split;
+        c1 = (p + 1) * w.nchunks / ep.split;
         slot = v;
         return true;
     };
+    // This pair's run of the second product.
+    uint32_t run0 = 0, run1 = 0;
+    if constexpr (TWO) {
+        const bool more = pair < pa.extra;
+        run0 = more ? pair * pa.run[0] : pa.extra * pa.run[0] + (pair - pa.extra) * pa.run[1];
+        run1 = min(run0 + pa.run[more ? 0 : 1], units_of(pa.ep[1]).n);
+    }
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
@@ -517,12 +543,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             bool ok = true;
             long long prof_a = 0;
             (void)prof_a;
-            for (uint32_t u = pair; u < nunits && ok; u += npairs) {
+            auto produce = [&](const Epilogue& ep, const CUtensorMap& map_a, const CUtensorMap& map_b, uint32_t first, uint32_t end, uint32_t step) {
+            const Units w = units_of(ep);
+            for (uint32_t u = first; u < end && ok; u += step) {
                 uint32_t tile, c0, c1, slot, m0, n0;
-                unit_at(u, tile, c0, c1, slot);
-                tile_origin(tile, m0, n0);
+                unit_at(ep, w, u, tile, c0, c1, slot);
+                tile_origin(ep, w, tile, m0, n0);
                 const uint32_t nb0 = n0 + rank * HB;                    // the rows of B this CTA loads
-                const uint32_t kb_last = min(nkb, c1 * kChunkKB);
+                const uint32_t kb_last = min(w.nkb, c1 * kChunkKB);
                 for (uint32_t kb = c0 * kChunkKB; kb < kb_last; ++kb, ++g) {
                     const int s = g % S;
                     const uint32_t ph = (g / S) & 1u;
@@ -531,7 +559,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(empty_bar(s), ph ^ 1u, kPairWaitCycles));
                         PROF_ADD(prof_a);
                         if (!got) {
-                            if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_TMA_WAIT);
+                            if (lane == 0) atomicOr(dev_status, FG_DEVERR_TMA_WAIT);
                             ok = false;
                             break;
                         }
@@ -551,8 +579,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                 tma_load_3d_pair(dst + 8192, t16, lf, (int)(r0 + 64), (int)(kb * KBE), 0);
                             }
                         };
-                        load16(sa, &tmA16, ep.a_mn != 0, m0);
-                        load16(sa + Cfg::kABytes, &tmB16, ep.b_mn != 0, nb0);
+                        load16(sa, &map_a, ep.a_mn != 0, m0);
+                        load16(sa + Cfg::kABytes, &map_b, ep.b_mn != 0, nb0);
                         continue;
                     }
                     if (leader) mbar_expect_tx(full_bar(s), 2 * Cfg::kStageBytes);   // both CTAs' bytes
@@ -574,14 +602,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                     tma_load_3d_pair(dst + BM * BK * 4 + i * 8192, t16, lf, (int)(r0 + 64 * i), (int)(kb * BK), 0);
                             }
                         };
-                        load_tile(sa, &tmA, &tmA16, ep.a_mn != 0, m0);
-                        load_tile(sa + Cfg::kABytes, &tmB, &tmB16, ep.b_mn != 0, nb0);
+                        load_tile(sa, &tmA, &map_a, ep.a_mn != 0, m0);
+                        load_tile(sa + Cfg::kABytes, &tmB, &map_b, ep.b_mn != 0, nb0);
                     } else {
                         tma_load_3d_pair(sa, &tmA, lf, (int)(kb * BK), (int)m0, 0);
                         tma_load_3d_pair(sa + Cfg::kABytes, &tmB, lf, (int)(kb * BK), (int)nb0, 0);
                     }
                 }
             }
+            };
+            produce(pa.ep[0], tmA16, tmB16, pair, units_of(pa.ep[0]).n, npairs);
+            if constexpr (TWO) produce(pa.ep[1], tmA, tmB, run0, run1, 1);
 #ifdef FG_GEMM_PROFILE
             if (lane == 0) atomicAdd(&g_prof[6], (unsigned long long)prof_a);
 #endif
@@ -597,9 +628,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #ifdef FG_GEMM_PROFILE
             const long long prof_start = clock64();
 #endif
-            for (uint32_t u = pair; u < nunits && ok; u += npairs) {
+            auto issue = [&](const Epilogue& ep, uint32_t first_unit, uint32_t end, uint32_t step) {
+            const Units w = units_of(ep);
+            for (uint32_t u = first_unit; u < end && ok; u += step) {
                 uint32_t tile, c0, c1, slot;
-                unit_at(u, tile, c0, c1, slot);
+                unit_at(ep, w, u, tile, c0, c1, slot);
                 for (uint32_t c = c0; c < c1 && ok; ++c, ++gc) {
                     const uint32_t buf = gc & 1u;
                     // the accumulator must have been drained by both CTAs' epilogue warps (two chunks ago)
@@ -608,14 +641,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(acc_empty_bar(buf), ((gc >> 1) & 1u) ^ 1u, kPairWaitCycles));
                         PROF_ADD(prof_e);
                         if (!got) {
-                            if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+                            if (lane == 0) atomicOr(dev_status, FG_DEVERR_MMA_WAIT);
                             ok = false;
                             break;
                         }
                     }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + buf * BN;
-                    const uint32_t kb_end = min(nkb, (c + 1) * kChunkKB);
+                    const uint32_t kb_end = min(w.nkb, (c + 1) * kChunkKB);
                     for (uint32_t kb = c * kChunkKB; kb < kb_end; ++kb, ++g) {
                         const int s = g % S;
                         const uint32_t ph = (g / S) & 1u;
@@ -624,7 +657,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                             const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(full_bar(s), ph, kPairWaitCycles));
                             PROF_ADD(prof_f);
                             if (!got) {
-                                if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_MMA_WAIT);
+                                if (lane == 0) atomicOr(dev_status, FG_DEVERR_MMA_WAIT);
                                 ok = false;
                                 break;
                             }
@@ -711,6 +744,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     __syncwarp();
                 }
             }
+            };
+            issue(pa.ep[0], pair, units_of(pa.ep[0]).n, npairs);
+            if constexpr (TWO) issue(pa.ep[1], run0, run1, 1);
 #ifdef FG_GEMM_PROFILE
             if (lane == 0) {
             atomicAdd(&g_prof[0], (unsigned long long)prof_e);
@@ -726,8 +762,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         // ---- accumulate + epilogue (both CTAs, own 128 rows); see gemm_tc_kernel ----
         const int q = warp & 3;
         const int half = (warp - kPairEpiWarp0) >> 2;
-        const bool vec_ok = (ep.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
-                            (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0);
         const uint32_t leader_acc_empty0 = map_to_cta(acc_empty_bar(0), 0);
         float4* tbuf = reinterpret_cast<float4*>(base_ptr + S * Cfg::kStageBytes + 256);   // 8 warps x 32 rows x 8 chunks
         float sum[CPT];
@@ -735,10 +769,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         uint32_t gc = 0;
         long long prof_w = 0, prof_s = 0, prof_n = 0;
         (void)prof_w; (void)prof_s; (void)prof_n;
-        for (uint32_t u = pair; u < nunits && ok; u += npairs) {
+        auto drain = [&](const Epilogue& ep, uint32_t first, uint32_t end, uint32_t step) {
+        const Units w = units_of(ep);
+        const bool vec_ok = (ep.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(ep.C) & 15u) == 0) &&
+                            (!ep.preact || (reinterpret_cast<uintptr_t>(ep.preact) & 15u) == 0);
+        for (uint32_t u = first; u < end && ok; u += step) {
             uint32_t tile, c0, c1, slot, m0, n0;
-            const bool part = unit_at(u, tile, c0, c1, slot);
-            tile_origin(tile, m0, n0);
+            const bool part = unit_at(ep, w, u, tile, c0, c1, slot);
+            tile_origin(ep, w, tile, m0, n0);
 #pragma unroll
             for (int j = 0; j < CPT; ++j) sum[j] = 0.0f;
             // Where this warp's part of the tile goes (a K-share of a tail tile goes out raw into its 256 x 256 slot).
@@ -770,7 +808,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 PROF_ADD(prof_w);
                 got = __all_sync(0xffffffffu, got);
                 if (!got) {
-                    if (lane == 0) atomicOr(ep.dev_status, FG_DEVERR_EPI_WAIT);
+                    if (lane == 0) atomicOr(dev_status, FG_DEVERR_EPI_WAIT);
                     ok = false;
                     break;
                 }
@@ -901,6 +939,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             prof_n += 1;
 #endif
         }
+        };
+        drain(pa.ep[0], pair, units_of(pa.ep[0]).n, npairs);
+        if constexpr (TWO) drain(pa.ep[1], run0, run1, 1);
 #ifdef FG_GEMM_PROFILE
         if (warp == kPairEpiWarp0 && lane == 0 && leader) {
             atomicAdd(&g_prof[3], (unsigned long long)prof_w);
@@ -2397,6 +2438,42 @@ bool cluster_query(int* n, Kernel kernel, unsigned grid, unsigned threads, size_
     return false;
 }
 
+// The kernel may use its shared memory, on this device (one bit per device; several host threads, one context each, may arrive here
+// together, and setting the attribute twice is harmless).
+template <int BK, int FMT, bool TWO>
+cudaError_t pair_attr(const fg_ctx* ctx) {
+    static std::atomic<uint64_t> done{0};
+    if (done.load(std::memory_order_acquire) >> (ctx->device & 63) & 1ull) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<BK, FMT, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<BK, FMT>::kSmemBytes);
+    if (e == cudaSuccess) done.fetch_or(1ull << (ctx->device & 63), std::memory_order_release);
+    return e;
+}
+// CTA pairs that are resident at once (asked of the runtime: not every SM need be pairable), with room for the gradient exchange that
+// runs beside.
+template <int BK, int FMT>
+uint64_t pair_slots(const fg_ctx* ctx) {
+    static std::atomic<int> max_clusters[64];       // zero-initialised
+    const uint64_t slots = (uint64_t)fg_asked_once(max_clusters[ctx->device & 63], ctx->sm_count / 2, [&](int* n) {
+        return pair_attr<BK, FMT, false>(ctx) == cudaSuccess &&
+               cluster_query(n, gemm_tc_pair_kernel<BK, FMT, false>, (unsigned)ctx->sm_count & ~1u, kPairThreads, PairCfg<BK, FMT>::kSmemBytes, 2) && *n >= 1;
+    });
+    return fg_free_sms(ctx) / 2 < slots ? fg_free_sms(ctx) / 2 : slots;
+}
+// The map of a 16-bit operand of the pair kernel, 64 values of k per k-block: boxes of `tile_rows` rows x 64 k, or 64 k x 64 rows when
+// the rows are contiguous.
+template <int FMT>
+int32_t pair16_map(fg_ctx* ctx, CUtensorMap* t, const PlaneSet& o, uint32_t rows, uint32_t K, uint32_t tile_rows) {
+    const int elem = FMT == 2 ? 1 : 2;
+    if (!o.mn) return make_tmap(ctx, t, o.p16, elem, 1, rows, K, o.ld16, tile_rows, 64);
+    return make_tmap3(ctx, t, o.p16, elem, rows, K, 1, (uint64_t)o.ld16 * 2, (uint64_t)K * o.ld16 * 2, 64, 64, 1);
+}
+// Tile rows per group of the tile order: the pairs at work at one time cover `group` tile rows, whose slabs of A
+// (256 x K elements each) should stay in the L2 while the B slabs stream past.  Eight rows for long K; sixteen
+// when the slabs are small (K <= 2048: the dW products of the eight-layer workload ran 5 % faster, its step
+// 23.83 against 23.91 ms; on 784-4096-4096-10, all K = 4096, eight is best: 0.300 ms per launch against
+// 0.302 / 0.305 / 0.307 for 12 / 16 / 4).
+inline uint32_t pair_group(const fg_ctx* ctx, uint32_t K) { return ctx->opt_tile_group > 0 ? (uint32_t)ctx->opt_tile_group : (K <= 2048 ? 16u : 8u); }
+
 template <int BK, int FMT>
 int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const Epilogue& ep_in) {
     Epilogue ep = ep_in;
@@ -2405,15 +2482,8 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     int32_t s;
     constexpr bool kDirect16 = FMT >= 2;
     if (kDirect16) {
-        // the operands themselves, 64 values of k per k-block: boxes of 128 rows x 64 k, or 64 k x 64 rows when the
-        // rows are contiguous
-        auto map16 = [&](CUtensorMap* t, const PlaneSet& o, uint32_t rows, uint32_t tile_rows) -> int32_t {
-            const int elem = FMT == 2 ? 1 : 2;
-            if (!o.mn) return make_tmap(ctx, t, o.p16, elem, 1, rows, ep.K, o.ld16, tile_rows, 2 * BK);
-            return make_tmap3(ctx, t, o.p16, elem, rows, ep.K, 1, (uint64_t)o.ld16 * 2, (uint64_t)ep.K * o.ld16 * 2, 64, 2 * BK, 1);
-        };
-        if ((s = map16(&tmA16, a, ep.M, BM)) != FG_OK) return s;
-        if ((s = map16(&tmB16, b, ep.N, Cfg::kBN / 2)) != FG_OK) return s;
+        if ((s = pair16_map<FMT>(ctx, &tmA16, a, ep.M, ep.K, BM)) != FG_OK) return s;
+        if ((s = pair16_map<FMT>(ctx, &tmB16, b, ep.N, ep.K, Cfg::kBN / 2)) != FG_OK) return s;
         ep.a_mn = a.mn ? 1u : 0u;
         ep.b_mn = b.mn ? 1u : 0u;
         tmA = tmA16;
@@ -2431,29 +2501,12 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
             tmB16 = tmB;
         }
     }
-    // one bit per device; several host threads (one context each) may arrive here together, and setting the
-    // attribute twice is harmless
-    static std::atomic<uint64_t> attr_done{0};
-    if (!(attr_done.load(std::memory_order_acquire) >> (ctx->device & 63) & 1ull)) {
-        FG_CUDA(ctx, FG_ERR_INTERNAL,
-                cudaFuncSetAttribute(gemm_tc_pair_kernel<BK, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-        attr_done.fetch_or(1ull << (ctx->device & 63), std::memory_order_release);
-    }
+    FG_CUDA(ctx, FG_ERR_INTERNAL, (pair_attr<BK, FMT, false>(ctx)));
     const uint64_t ntiles = (uint64_t)((ep.M + 2 * BM - 1) / (2 * BM)) * ((ep.N + Cfg::kBN - 1) / Cfg::kBN);
     if (ntiles > (1ull << 30)) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM: too many tiles");
-    // Tile rows per group of the tile order: the pairs at work at one time cover `group` tile rows, whose slabs of A
-    // (256 x K elements each) should stay in the L2 while the B slabs stream past.  Eight rows for long K; sixteen
-    // when the slabs are small (K <= 2048: the dW products of the eight-layer workload ran 5 % faster, its step
-    // 23.83 against 23.91 ms; on 784-4096-4096-10, all K = 4096, eight is best: 0.300 ms per launch against
-    // 0.302 / 0.305 / 0.307 for 12 / 16 / 4).
-    ep.group = ctx->opt_tile_group > 0 ? (uint32_t)ctx->opt_tile_group : (ep.K <= 2048 ? 16u : 8u);
+    ep.group = pair_group(ctx, ep.K);
     // persistent: one CTA pair per SM pair, each walking tiles pair, pair + P, ...
-    // How many pairs can be resident at once is asked of the runtime (not every SM need be pairable).
-    static std::atomic<int> max_clusters[64];       // zero-initialised
-    uint64_t slots = (uint64_t)fg_asked_once(max_clusters[ctx->device & 63], ctx->sm_count / 2, [&](int* n) {
-        return cluster_query(n, gemm_tc_pair_kernel<BK, FMT>, (unsigned)ctx->sm_count & ~1u, kPairThreads, Cfg::kSmemBytes, 2) && *n >= 1;
-    });
-    if (fg_free_sms(ctx) / 2 < slots) slots = fg_free_sms(ctx) / 2;      // room for the gradient exchange that runs beside this GEMM
+    const uint64_t slots = pair_slots<BK, FMT>(ctx);
     // The last wave: `rem` tiles for `slots` pairs.  When at least two pairs are free per tile, each tail
     // tile is cut into K-shares (whole accumulation chunks, at least two per share) so that the wave
     // lasts a fraction of a tile time; the shares are folded by a second, bandwidth-bound kernel.
@@ -2477,7 +2530,9 @@ int32_t launch_tc_pair(fg_ctx* ctx, const PlaneSet& a, const PlaneSet& b, const 
     const uint64_t nunits = ep.t_full + (ntiles - ep.t_full) * ep.split;
     dim3 grid((unsigned)(2 * (nunits < slots ? nunits : slots)));
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, 2.0 * ep.M * ep.N * ep.K);
-    gemm_tc_pair_kernel<BK, FMT><<<grid, kPairThreads, Cfg::kSmemBytes, ctx->stream>>>(tmA, tmB, tmA16, tmB16, ep);
+    PairArgs<false> pa{};
+    pa.ep[0] = ep;
+    gemm_tc_pair_kernel<BK, FMT, false><<<grid, kPairThreads, Cfg::kSmemBytes, ctx->stream>>>(tmA, tmB, tmA16, tmB16, pa);
     FG_LAUNCHED(ctx);
     if (ep.split > 1) {
         fg_launch(ctx, gemm_tc_fold_kernel, (unsigned)((ntiles - ep.t_full) * 64), 256, 0, ep);
@@ -2711,16 +2766,22 @@ int32_t launch_half(fg_ctx* ctx, const ConvProduct* pr, int n, const ConvPlan& p
     return p.bn == 128 ? launch_half_bn<128>(ctx, pr, n, p.split) : launch_half_bn<64>(ctx, pr, n, p.split);
 }
 // The pair kernel on 16-bit tensors by the same fit: tiles of 256 x 256, K-shares of 2048 or more in the last wave.
+constexpr double kPair16Around = 26600.0;
+uint64_t pair_tiles(const ConvShape& sh) { return (uint64_t)((sh.M + 255) / 256) * ((sh.N + 255) / 256); }
+double pair16_tile(const ConvShape& sh) {
+    const double kb = (double)((sh.K + 63) / 64) * 395.0;
+    return kb > 2500.0 ? kb : 2500.0;
+}
 double pair16_cycles(const fg_ctx* ctx, const ConvShape& sh) {
-    const uint64_t pairs = fg_free_sms(ctx) / 2, tiles = (uint64_t)((sh.M + 255) / 256) * ((sh.N + 255) / 256);
-    const double kb = (double)((sh.K + 63) / 64) * 395.0, tile = kb > 2500.0 ? kb : 2500.0, whole = (double)(tiles / pairs) * tile;
+    const uint64_t pairs = fg_free_sms(ctx) / 2, tiles = pair_tiles(sh);
+    const double tile = pair16_tile(sh), whole = (double)(tiles / pairs) * tile;
     const uint64_t rem = tiles % pairs, nchunks = (sh.K + 1023) / 1024;
     double tail = rem ? tile : 0.0;
     uint64_t split = rem ? pairs / rem : 1;
     if (split > nchunks / 2) split = nchunks / 2;
     if (split > 4) split = 4;
     if (split >= 2 && ctx->opt_split_k) tail = tail / (double)split + 3300.0;
-    return whole + tail + 26600.0;
+    return whole + tail + kPair16Around;
 }
 
 // A dense [R, C] f32 tensor (`batch` of them, x_batch apart) can be loaded as it lies when rows and matrices start on
@@ -3794,26 +3855,61 @@ bool half_suits(const fg_ctx* ctx, const ConvShape& sh, ConvPlan* plan) {
 int32_t launch_pair16(fg_ctx* ctx, const ConvProduct& p) {
     return p.ep.out_dtype == FG_DTYPE_BF16 ? launch_tc_pair<32, 2>(ctx, p.a, p.b, p.ep) : launch_tc_pair<32, 3>(ctx, p.a, p.b, p.ep);
 }
+// Two products in a launch of the pair kernel, the one with the longer k first.
+template <int FMT>
+int32_t launch_pair16_two(fg_ctx* ctx, const ConvProduct* pr, const PairRuns& r) {
+    using Cfg = PairCfg<32, FMT>;
+    CUtensorMap tm[4];
+    PairArgs<true> pa{};
+    double flop = 0.0;
+    for (int j = 0; j < 2; ++j) {
+        const ConvProduct& c = pr[j];
+        int32_t s;
+        if ((s = pair16_map<FMT>(ctx, &tm[2 * j], c.a, c.ep.M, c.ep.K, BM)) != FG_OK) return s;
+        if ((s = pair16_map<FMT>(ctx, &tm[2 * j + 1], c.b, c.ep.N, c.ep.K, Cfg::kBN / 2)) != FG_OK) return s;
+        pa.ep[j] = c.ep;
+        pa.ep[j].a_mn = c.a.mn ? 1u : 0u;
+        pa.ep[j].b_mn = c.b.mn ? 1u : 0u;
+        pa.ep[j].group = pair_group(ctx, c.ep.K);
+        pa.ep[j].t_full = (uint32_t)pair_tiles(conv_shape(c));
+        flop += 2.0 * c.ep.M * c.ep.N * c.ep.K;
+    }
+    pa.extra = r.extra;
+    pa.run[0] = r.run[0]; pa.run[1] = r.run[1];
+    FG_CUDA(ctx, FG_ERR_INTERNAL, (pair_attr<32, FMT, true>(ctx)));
+    fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_GEMM_TC, flop);
+    gemm_tc_pair_kernel<32, FMT, true><<<(unsigned)(2 * r.pairs), kPairThreads, Cfg::kSmemBytes, ctx->stream>>>(tm[2], tm[3], tm[0], tm[1], pa);
+    fg_time_end(ctx, tr);
+    FG_LAUNCHED(ctx);
+    return FG_OK;
+}
 int32_t lowp_gemm(fg_ctx* ctx, const ConvProduct& p) {
     ConvPlan plan;
     return half_suits(ctx, conv_shape(p), &plan) ? launch_half(ctx, &p, 1, plan) : launch_pair16(ctx, p);
 }
-// Both gradients of a layer, dB first: one launch where both are for the half kernel, they are estimated to end sooner together, and
-// neither lies over what the other reads.
+// Both gradients of a layer, dB first: one launch where they are estimated to end sooner together and neither lies over what the
+// other reads (layer of 2048 x 4096 x 4096: 122 -> 113 us for the two).
 int32_t lowp_gemm_both(fg_ctx* ctx, const ConvProduct& dB, const ConvProduct& dA) {
     ConvPlan b, a;
     const bool hb = half_suits(ctx, conv_shape(dB), &b), ha = half_suits(ctx, conv_shape(dA), &a);
-    if (hb && ha) {
+    auto over = [](const ConvProduct& w, const ConvProduct& r) {
+        const uint64_t n = (uint64_t)w.ep.M * w.ep.N * 2;
+        return fg_ranges_meet(w.ep.C, n, r.a.p16, (uint64_t)(r.a.mn ? r.ep.K : r.ep.M) * r.a.ld16 * 2) ||
+               fg_ranges_meet(w.ep.C, n, r.b.p16, (uint64_t)(r.b.mn ? r.ep.K : r.ep.N) * r.b.ld16 * 2);
+    };
+    if (!over(dB, dA) && !over(dA, dB)) {
         const ConvProduct pr[2] = {dB.ep.K >= dA.ep.K ? dB : dA, dB.ep.K >= dA.ep.K ? dA : dB};      // the longer k first
         const ConvShape sh[2] = {conv_shape(pr[0]), conv_shape(pr[1])};
-        const ConvPlan both = plan_half(ctx, sh, 2);
-        auto over = [](const ConvProduct& w, const ConvProduct& r) {
-            const uint64_t n = (uint64_t)w.ep.M * w.ep.N * 2;
-            return fg_ranges_meet(w.ep.C, n, r.a.p16, (uint64_t)(r.a.mn ? r.ep.K : r.ep.M) * r.a.ld16 * 2) ||
-                   fg_ranges_meet(w.ep.C, n, r.b.p16, (uint64_t)(r.b.mn ? r.ep.K : r.ep.N) * r.b.ld16 * 2);
-        };
         // (a second launch costs 2500 more than the estimates know)
-        if (both.cycles <= b.cycles + a.cycles + 2500.0 && !over(dB, dA) && !over(dA, dB)) return launch_half(ctx, pr, 2, both);
+        const double apart = (hb ? b.cycles : pair16_cycles(ctx, conv_shape(dB))) + (ha ? a.cycles : pair16_cycles(ctx, conv_shape(dA))) + 2500.0;
+        const uint64_t slots = ctx->opt_conv_bn ? 0 : dB.ep.out_dtype == FG_DTYPE_BF16 ? pair_slots<32, 2>(ctx) : pair_slots<32, 3>(ctx);
+        const uint64_t n0 = pair_tiles(sh[0]), n1 = pair_tiles(sh[1]);
+        PairRuns runs{};
+        if (slots && n0 + n1 < (1ull << 24)) runs = pair_runs(slots, n0, pair16_tile(sh[0]), n1, pair16_tile(sh[1]));
+        const double pairs = runs.pairs ? runs.cost + kPair16Around : 1e30;
+        const ConvPlan half = ctx->opt_tile_pair == 1 ? ConvPlan{128, 1, 1e30} : plan_half(ctx, sh, 2);
+        if (hb && ha && half.cycles <= apart && half.cycles <= pairs) return launch_half(ctx, pr, 2, half);
+        if (pairs < apart) return dB.ep.out_dtype == FG_DTYPE_BF16 ? launch_pair16_two<2>(ctx, pr, runs) : launch_pair16_two<3>(ctx, pr, runs);
     }
     const int32_t s = hb ? launch_half(ctx, &dB, 1, b) : launch_pair16(ctx, dB);
     return s != FG_OK ? s : ha ? launch_half(ctx, &dA, 1, a) : launch_pair16(ctx, dA);
