@@ -183,3 +183,13 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def calls():
+    """The CPython module of the frequent entry points (csrc/calls.cpp).  Raises if it is missing."""
+    load()
+    try:
+        from . import _calls
+    except ImportError as e:
+        raise ImportError(f"{e}: build it with `python -m ferrograd_b200.build` (there is no other path to the library)") from e
+    return _calls

@@ -85,7 +85,7 @@ class Plan:
         self.handle = handle
 
     def launch(self):
-        self.ctx._check(self.ctx.lib.fg_plan_launch(self.ctx.handle, self.handle))
+        self.ctx._check(self.ctx._c.fg_plan_launch(self.ctx._h, self.handle))
 
     def destroy(self):
         if self.handle:
@@ -116,6 +116,7 @@ class GpuContext:
             raise FgError(code, "could not create a context on device %d" % device)
         self.handle = h
         self.device = device
+        self._c, self._h = _lib.calls(), h.value      # the frequent entry points, and the handle as they take it
 
     # the reference spells the constructor GpuContext::new()
     @classmethod
@@ -123,13 +124,13 @@ class GpuContext:
         return cls(device)
 
     def _check(self, code):
-        if code != 0:
+        if code:
             raise FgError(code, (self.lib.fg_last_error(self.handle) or b"").decode())
 
     def destroy(self):
         if self.handle:
             self.lib.fg_ctx_destroy(self.handle)
-            self.handle = None
+            self.handle, self._h = None, 0
 
     # ---- GpuBackend: memory ----
     def alloc(self, nbytes):
@@ -272,13 +273,13 @@ class GpuContext:
     # ---- compute ----
     def gemm(self, A, B, Cout, M, N, K, transA=False, transB=False, bias=None, act="none", preact_out=None,
              mode="auto"):
-        self._check(self.lib.fg_gemm_f32(self.handle, GEMM_MODE[mode], int(transA), int(transB), M, N, K,
-                                         _ptr(A), _ptr(B), _ptr(Cout), _ptr(bias), ACT[act], _ptr(preact_out)))
+        self._check(self._c.fg_gemm_f32(self._h, GEMM_MODE[mode], int(transA), int(transB), M, N, K,
+                                         A, B, Cout, bias, ACT[act], preact_out))
 
     def gemm_bwd(self, A, B, dY, M, N, K, act="none", saved=None, dA=None, dB=None, dbias=None, dZ_out=None,
                  mode="auto"):
-        self._check(self.lib.fg_gemm_bwd_f32(self.handle, GEMM_MODE[mode], M, N, K, _ptr(A), _ptr(B), _ptr(dY),
-                                             ACT[act], _ptr(saved), _ptr(dA), _ptr(dB), _ptr(dbias), _ptr(dZ_out)))
+        self._check(self._c.fg_gemm_bwd_f32(self._h, GEMM_MODE[mode], M, N, K, A, B, dY,
+                                             ACT[act], saved, dA, dB, dbias, dZ_out))
 
     def gemm_bwd_exchange(self, A, B, dY, M, N, K, exch_buf, exch_count, act="none", saved=None, dA=None, dB=None,
                           dbias=None, mode="auto"):
@@ -293,60 +294,60 @@ class GpuContext:
 
     def gemm_paired(self, A, B, Cout, M, N, K, A_pairs=None, B_pairs=None, bias=None, act="none", preact_out=None,
                     C_pairs=None, A_stride=None, B_stride=None, C_stride=None):
-        self._check(self.lib.fg_gemm_paired_f32(self.handle, M, N, K, _ptr(A), _ptr(A_pairs), A_stride or M * K, _ptr(B),
-                                                _ptr(B_pairs), B_stride or K * N, _ptr(Cout), _ptr(bias), ACT[act],
-                                                _ptr(preact_out), _ptr(C_pairs), C_stride or M * N))
+        self._check(self._c.fg_gemm_paired_f32(self._h, M, N, K, A, A_pairs, A_stride or M * K, B,
+                                                B_pairs, B_stride or K * N, Cout, bias, ACT[act],
+                                                preact_out, C_pairs, C_stride or M * N))
 
     def gemm_bwd_paired(self, A, B, dZ, M, N, K, A_pairs=None, B_pairs=None, dZ_pairs=None, dB=None, dbias=None, dA=None,
                         below_act="none", below_saved=None, dA_pairs=None, below_dbias=None, exch_buf=None,
                         exch_count=0, A_stride=None, B_stride=None, dZ_stride=None, dA_stride=None):
-        self._check(self.lib.fg_gemm_bwd_paired_f32(
-            self.handle, M, N, K, _ptr(A), _ptr(A_pairs), A_stride or M * K, _ptr(B), _ptr(B_pairs), B_stride or K * N,
-            _ptr(dZ), _ptr(dZ_pairs), dZ_stride or M * N, _ptr(dB), _ptr(dbias), _ptr(dA), ACT[below_act], _ptr(below_saved),
-            _ptr(dA_pairs), dA_stride or M * K, _ptr(below_dbias), _ptr(exch_buf), exch_count))
+        self._check(self._c.fg_gemm_bwd_paired_f32(
+            self._h, M, N, K, A, A_pairs, A_stride or M * K, B, B_pairs, B_stride or K * N,
+            dZ, dZ_pairs, dZ_stride or M * N, dB, dbias, dA, ACT[below_act], below_saved,
+            dA_pairs, dA_stride or M * K, below_dbias, exch_buf, exch_count))
 
     def gemm_batched(self, A, B, Cout, batch, M, N, K, bias=None, act="none", preact_out=None, mode="auto",
                      strides=None):
         sa, sb, sc = strides or (M * K, K * N, M * N)
-        self._check(self.lib.fg_gemm_batched_f32(self.handle, GEMM_MODE[mode], batch, M, N, K, _ptr(A), sa, _ptr(B), sb,
-                                                 _ptr(Cout), sc, _ptr(bias), ACT[act], _ptr(preact_out)))
+        self._check(self._c.fg_gemm_batched_f32(self._h, GEMM_MODE[mode], batch, M, N, K, A, sa, B, sb,
+                                                 Cout, sc, bias, ACT[act], preact_out))
 
     def gemm_batched_bwd(self, A, B, dY, batch, M, N, K, act="none", saved=None, dA=None, dB=None, mode="auto",
                          strides=None):
         sa, sb, sc = strides or (M * K, K * N, M * N)
-        self._check(self.lib.fg_gemm_batched_bwd_f32(self.handle, GEMM_MODE[mode], batch, M, N, K, _ptr(A), sa,
-                                                     _ptr(B), sb, _ptr(dY), sc, ACT[act], _ptr(saved), _ptr(dA),
-                                                     _ptr(dB)))
+        self._check(self._c.fg_gemm_batched_bwd_f32(self._h, GEMM_MODE[mode], batch, M, N, K, A, sa,
+                                                     B, sb, dY, sc, ACT[act], saved, dA,
+                                                     dB))
 
     def bias_act_fwd(self, z, bias, act, y, rows, cols):
-        self._check(self.lib.fg_bias_act_fwd(self.handle, rows, cols, _ptr(z), _ptr(bias), ACT[act], _ptr(y)))
+        self._check(self._c.fg_bias_act_fwd(self._h, rows, cols, z, bias, ACT[act], y))
 
     def act_bwd(self, dy, saved, dz, n, act):
-        self._check(self.lib.fg_act_bwd(self.handle, n, ACT[act], _ptr(dy), _ptr(saved), _ptr(dz)))
+        self._check(self._c.fg_act_bwd(self._h, n, ACT[act], dy, saved, dz))
 
     def softmax_fwd(self, x, y, rows, cols):
-        self._check(self.lib.fg_softmax_fwd(self.handle, rows, cols, _ptr(x), _ptr(y)))
+        self._check(self._c.fg_softmax_fwd(self._h, rows, cols, x, y))
 
     def softmax_bwd(self, y, dy, dx, rows, cols, accumulate=False):
-        self._check(self.lib.fg_softmax_bwd(self.handle, rows, cols, _ptr(y), _ptr(dy), _ptr(dx), int(accumulate)))
+        self._check(self._c.fg_softmax_bwd(self._h, rows, cols, y, dy, dx, int(accumulate)))
 
     def softmax_ce(self, logits, labels, rows, cols, grad_scale=1.0, loss_row=None, loss_mean=None, dlogits=None,
                    probs=None, argmax=None):
-        self._check(self.lib.fg_softmax_ce_fwd_bwd(self.handle, _ptr(logits), _ptr(labels), rows, cols,
-                                                   grad_scale, _ptr(loss_row), _ptr(loss_mean), _ptr(dlogits),
-                                                   _ptr(probs), _ptr(argmax)))
+        self._check(self._c.fg_softmax_ce_fwd_bwd(self._h, logits, labels, rows, cols,
+                                                   grad_scale, loss_row, loss_mean, dlogits,
+                                                   probs, argmax))
 
     def ce_loss_grad(self, probs, labels, rows, cols, loss, grad):
-        self._check(self.lib.fg_ce_loss_grad(self.handle, _ptr(probs), _ptr(labels), rows, cols, _ptr(loss),
-                                             _ptr(grad)))
+        self._check(self._c.fg_ce_loss_grad(self._h, probs, labels, rows, cols, loss,
+                                             grad))
 
     def mse_loss_grad(self, pred, target, n, grad_scale=1.0, loss_elem=None, loss_sum=None, grad=None):
-        self._check(self.lib.fg_mse_loss_grad(self.handle, _ptr(pred), _ptr(target), n, grad_scale,
-                                              _ptr(loss_elem), _ptr(loss_sum), _ptr(grad)))
+        self._check(self._c.fg_mse_loss_grad(self._h, pred, target, n, grad_scale,
+                                              loss_elem, loss_sum, grad))
 
     def bce_loss_grad(self, pred, target, n, grad_scale=1.0, loss_elem=None, loss_sum=None, grad=None):
-        self._check(self.lib.fg_bce_loss_grad(self.handle, _ptr(pred), _ptr(target), n, grad_scale,
-                                              _ptr(loss_elem), _ptr(loss_sum), _ptr(grad)))
+        self._check(self._c.fg_bce_loss_grad(self._h, pred, target, n, grad_scale,
+                                              loss_elem, loss_sum, grad))
 
     def mse_loss_grad_noalloc(self, pred, target, n, grad_scale=1.0, loss_elem=None, loss_sum=None, grad=None):
         """fg_mse_loss_grad for hosts that must not allocate device memory: the reduction scratch is a
@@ -355,7 +356,7 @@ class GpuContext:
                                                       _ptr(loss_elem), _ptr(loss_sum), _ptr(grad)))
 
     def sgd_step(self, w, g, n, lr, grad_scale=1.0, zero_grad=True):
-        self._check(self.lib.fg_sgd_step(self.handle, _ptr(w), _ptr(g), n, lr, grad_scale, int(zero_grad)))
+        self._check(self._c.fg_sgd_step(self._h, w, g, n, lr, grad_scale, int(zero_grad)))
 
     def adamw_step(self, w, g, m, v, n, lr, beta1, beta2, eps, weight_decay, step=1, step_dev=None,
                    grad_scale=1.0, zero_grad=True):
@@ -395,40 +396,24 @@ class GpuContext:
     def counter_increment(self, counter):
         self._check(self.lib.fg_counter_increment(self.handle, _ptr(counter)))
 
-    @staticmethod
-    def _prog(instrs):
-        arr = (_lib.EwInstr * len(instrs))()
-        for i, (op, a, b, imm) in enumerate(instrs):
-            arr[i] = _lib.EwInstr(EW[op] if isinstance(op, str) else op, a, b, imm)
-        return arr
-
     def eltwise_chain_fwd(self, instrs, inputs, out, n, saved=None, dtype="f32"):
-        prog = self._prog(instrs)
-        inp = (C.c_void_p * len(inputs))(*[_ptr(x) for x in inputs])
-        sv = None
-        if saved:
-            sv = (C.c_void_p * len(instrs))(*[_ptr(saved.get(k)) for k in range(len(instrs))])
-        self._check(self.lib.fg_eltwise_chain_fwd_dt(self.handle, DTYPE[dtype], n, prog, len(instrs), inp, len(inputs),
-                                                     _ptr(out), sv))
+        sv = [saved.get(k) for k in range(len(instrs))] if saved else None
+        self._check(self._c.chain_fwd(self._h, DTYPE[dtype], n, instrs, inputs, out, sv))
 
     def eltwise_chain_bwd(self, instrs, inputs, seed, grads, n, accumulate=False, dtype="f32"):
-        prog = self._prog(instrs)
-        inp = (C.c_void_p * len(inputs))(*[_ptr(x) for x in inputs])
-        gp = (C.c_void_p * len(inputs))(*[_ptr(g) for g in grads])
-        self._check(self.lib.fg_eltwise_chain_bwd_dt(self.handle, DTYPE[dtype], n, prog, len(instrs), inp, len(inputs),
-                                                     _ptr(seed), gp, int(accumulate)))
+        self._check(self._c.chain_bwd(self._h, DTYPE[dtype], n, instrs, inputs, seed, grads, accumulate))
 
     def gemm_lowp(self, A, B, Cout, M, N, K, dtype, bias=None, act="none", preact_out=None):
         """GEMM on f16 / bf16 tensors: 16-bit operands straight into the tensor cores, f32 accumulate."""
-        self._check(self.lib.fg_gemm_lowp(self.handle, DTYPE[dtype], M, N, K, _ptr(A), _ptr(B), _ptr(Cout), _ptr(bias),
-                                          ACT[act], _ptr(preact_out)))
+        self._check(self._c.fg_gemm_lowp(self._h, DTYPE[dtype], M, N, K, A, B, Cout, bias,
+                                          ACT[act], preact_out))
 
     def gemm_bwd_lowp(self, A, B, dY, M, N, K, dtype, act="none", saved=None, dA=None, dB=None, dbias=None):
-        self._check(self.lib.fg_gemm_bwd_lowp(self.handle, DTYPE[dtype], M, N, K, _ptr(A), _ptr(B), _ptr(dY), ACT[act],
-                                              _ptr(saved), _ptr(dA), _ptr(dB), _ptr(dbias)))
+        self._check(self._c.fg_gemm_bwd_lowp(self._h, DTYPE[dtype], M, N, K, A, B, dY, ACT[act],
+                                              saved, dA, dB, dbias))
 
     def convert(self, src, src_dtype, dst, dst_dtype, n):
-        self._check(self.lib.fg_convert(self.handle, _ptr(src), DTYPE[src_dtype], _ptr(dst), DTYPE[dst_dtype], n))
+        self._check(self._c.fg_convert(self._h, src, DTYPE[src_dtype], dst, DTYPE[dst_dtype], n))
 
     # ---- plans ----
     def plan_begin(self):

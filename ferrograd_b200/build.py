@@ -1,10 +1,11 @@
-"""Builds libferrograd_b200.so in-tree with nvcc for sm_100a.
+"""Builds libferrograd_b200.so in-tree with nvcc for sm_100a, and the CPython module of its frequent entry points.
 
 Usage: python -m ferrograd_b200.build [--force] [--verbose]
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -18,7 +19,28 @@ def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
 
 
+CALLS_SRC = os.path.join(CSRC, "calls.cpp")
+CALLS = os.path.join(HERE, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_calls(force: bool = False) -> None:
+    """The module of frequent entry points (csrc/calls.cpp), beside the library that it calls."""
+    header = os.path.join(os.path.dirname(HERE), "include", "ferrograd_b200.h")
+    if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) >= _newest([CALLS_SRC, header]):
+        return
+    tmp = CALLS + ".tmp"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], CALLS_SRC, "-o", tmp,
+                    "-L", HERE, "-lferrograd_b200", "-Wl,-rpath,$ORIGIN"], check=True)
+    os.replace(tmp, CALLS)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    out = build_library(force, verbose)
+    build_calls(force)
+    return out
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
     deps = srcs + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
     deps.append(os.path.join(os.path.dirname(HERE), "include", "ferrograd_b200.h"))

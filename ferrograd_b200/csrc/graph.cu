@@ -1021,25 +1021,24 @@ static int32_t optim_eager(fg_exec* e) {
     return optim_many(e, all);
 }
 
-// Are this graph's dispatches recorded and replayed?  With option exec_plans = auto: when the graph is launch-bound,
-// i.e. its estimated device time per launch is under ten microseconds, or under 300 with a communicator (one
-// forward + backward pass estimated at
-// 300 TFLOP/s for the matmuls and 5 TB/s for every tensor touched three times, over about three launches per step of
-// the forward pass).
+// Are this graph's dispatches recorded and replayed?  With option exec_plans = auto: with a communicator, when a forward + backward pass
+// is estimated at under 300 us per launch (300 TFLOP/s for the matmuls and 5 TB/s for every tensor touched three times, over about
+// three launches per step of the forward pass).  Every step also enqueues collectives then, whose host-side cost a replayed graph
+// avoids (two GPUs, 784-4096-4096-10, about 125 us per launch: 1.97 ms per step replayed against 2.03 with plain launches; eight
+// 8192-wide layers, about 800 us per launch: 27.0 against 26.5 ms, so those stay with plain launches).
+// On one GPU a dispatch is a few launches, which the stream overlaps with each other and with those of the dispatch before; the start
+// and the end of a graph do not overlap with anything (us per step, replayed and plain: 2-16-2 22.5 / 18.8, 200-256-256-10 59.6 / 56.7,
+// 427-32-26-95 39.1 / 32.6, 64-1644-42-41 73.8 / 65.0; graphs for some of the dispatches are slower than either).
 static bool plans_wanted(const fg_exec* e) {
     if (!e->use_plans || e->ctx->opt_exec_plans == 0) return false;
     if (e->ctx->opt_exec_plans == 1) return true;
+    if (e->ctx->comm == nullptr || e->ctx->nranks <= 1) return false;
     double flop = 0.0, bytes = 0.0;
     for (const GemmStep& gs : e->gemms) flop += 3.0 * 2.0 * gs.batch * (double)gs.M * gs.N * gs.K;
     for (const ENode& en : e->n) bytes += 3.0 * (double)en.numel * (double)e->esize;
     const double est_us = flop / 300e6 + bytes / 5e6;
     const double launches = 3.0 * (double)std::max<size_t>(e->fwd.size(), 1);
-    // With a communicator every step also enqueues collectives, whose host-side cost a replayed graph avoids:
-    // worth it up to a few hundred microseconds per launch (two GPUs, 784-4096-4096-10, about 125 us per launch:
-    // 1.97 ms per step replayed against 2.03 with plain launches; eight 8192-wide layers, about 800 us per
-    // launch: 27.0 against 26.5 ms, so those stay with plain launches).
-    if (e->ctx->comm != nullptr && e->ctx->nranks > 1) return est_us / launches < 300.0;
-    return est_us / launches < 10.0;
+    return est_us / launches < 300.0;
 }
 
 // Runs one dispatch: eagerly the first time (which also sizes the scratch arena), recorded as a plan the

@@ -233,17 +233,17 @@ class GraphContextMixin:
         return Schedule(saved_tensors)
 
     def dispatch_forward(self, schedule):
-        self._check(self.lib.fg_exec_dispatch_forward(schedule.tensors.handle))
+        self._check(self._c.fg_exec_dispatch_forward(schedule.tensors.handle))
 
     def dispatch_backward(self, schedule):
-        self._check(self.lib.fg_exec_dispatch_backward(schedule.tensors.handle))
+        self._check(self._c.fg_exec_dispatch_backward(schedule.tensors.handle))
 
     def dispatch_loss(self, schedule, target):
         buf = target.as_buffer() if isinstance(target, Tensor) else target
-        self._check(self.lib.fg_exec_dispatch_loss(schedule.tensors.handle, buf.handle))
+        self._check(self._c.fg_exec_dispatch_loss(schedule.tensors.handle, buf.handle))
 
     def dispatch_optim(self, schedule):
-        self._check(self.lib.fg_exec_dispatch_optim(schedule.tensors.handle))
+        self._check(self._c.fg_exec_dispatch_optim(schedule.tensors.handle))
 
     def dispatch_single_optim(self, schedule, weight, grad, tensors=None):
         buf = weight.as_buffer() if isinstance(weight, Tensor) else weight
