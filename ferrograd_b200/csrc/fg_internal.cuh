@@ -454,6 +454,8 @@ uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t
 // fg_ce_loss_grad with the sum of the losses; its arguments have been checked.
 int32_t fg_ce_loss_grad_sum(fg_ctx* ctx, const float* probs, const uint32_t* labels, uint32_t rows, uint32_t cols, float* loss_out,
                             float* grad_out, float* loss_sum_out);
+// fg_adamw_step_multi (gradients zeroed) of step *counter + 1; `count`: the counter is that step afterwards.
+int32_t fg_adamw_next_step(fg_ctx* ctx, const fg_update_tensor* tensors, uint32_t n, const fg_adamw_hyper* h, uint32_t* counter, bool count);
 // Where `grid` blocks leave their partial sums (scratch, or *sum itself for one block), where the last of them leaves the sum, if it
 // adds them; fg_block_sums_end(), after the launch, has them added otherwise.  No sum wanted: both NULL.
 struct FgBlockSums { float *partials, *out, *sum; int grid; };

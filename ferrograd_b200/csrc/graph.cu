@@ -959,8 +959,10 @@ static int32_t optim_one(fg_exec* e, uint32_t slot, fg_buf* weight) {
 // Updates every bound tensor that is marked trainable (the reference updates all of them:
 // dispatch/mod.rs:735-748) and zeroes its gradient.
 // Updates the given input slots in one launch (f32 graphs), or one by one (16-bit storage).
-static int32_t optim_many(fg_exec* e, const std::vector<int>& slots) {
-    if (slots.empty()) return FG_OK;
+// AdamW's step counter has moved (`counted`), or moves with the last call of a dispatch.
+static int32_t optim_many(fg_exec* e, const std::vector<int>& slots, bool counted, bool last) {
+    const bool count = e->g.optim == FG_OPTIM_ADAMW && !counted && last;
+    if (slots.empty() && !count) return FG_OK;
     if (e->dtype != FG_DTYPE_F32) {
         for (int slot : slots) {
             const int32_t s = optim_one(e, (uint32_t)slot, e->n[e->inputs[slot]].value);
@@ -988,7 +990,9 @@ static int32_t optim_many(fg_exec* e, const std::vector<int>& slots) {
     else {
         fg_adamw_hyper h = e->hyper;
         h.lr = lr;
-        s = fg_adamw_step_multi(e->ctx, t.data(), (uint32_t)t.size(), &h, 0, (const uint32_t*)e->step_counter->ptr, 1.0f, 1);
+        uint32_t* const counter = (uint32_t*)e->step_counter->ptr;
+        s = counted ? fg_adamw_step_multi(e->ctx, t.data(), (uint32_t)t.size(), &h, 0, counter, 1.0f, 1)
+                    : fg_adamw_next_step(e->ctx, t.data(), (uint32_t)t.size(), &h, counter, count);
     }
     if (s != FG_OK) return s;
     for (int slot : slots)
@@ -1001,7 +1005,9 @@ static int32_t optim_many(fg_exec* e, const std::vector<int>& slots) {
 
 static int32_t optim_eager(fg_exec* e) {
     int32_t s;
-    if (e->g.optim == FG_OPTIM_ADAMW && (s = fg_counter_increment(e->ctx, (uint32_t*)e->step_counter->ptr)) != FG_OK) return s;
+    // The update moves AdamW's step counter itself, but not in a recorded plan (see fg_fold_in_launch), nor in 16-bit storage.
+    const bool counted = e->g.optim == FG_OPTIM_ADAMW && (e->ctx->capturing || e->dtype != FG_DTYPE_F32);
+    if (counted && (s = fg_counter_increment(e->ctx, (uint32_t*)e->step_counter->ptr)) != FG_OK) return s;
     if (dp_active(e)) {
         // Gradients in [0, final_lo) were summed over the ranks during dispatch_backward.  The sum of the rest
         // (the gradients the backward pass finished last) starts now; the tensors of the first range are updated
@@ -1011,14 +1017,14 @@ static int32_t optim_eager(fg_exec* e) {
         std::vector<int> early, late;
         for (int slot : e->arena_order)
             if (e->trainable[slot]) (e->arena_off[slot] + e->n[e->inputs[slot]].numel <= lo ? early : late).push_back(slot);
-        if ((s = optim_many(e, early)) != FG_OK) return s;
+        if ((s = optim_many(e, early, counted, false)) != FG_OK) return s;
         if ((s = fg_comm_join(e->ctx)) != FG_OK) return s;
-        return optim_many(e, late);
+        return optim_many(e, late, counted, true);
     }
     std::vector<int> all;
     for (int slot : e->arena_order)
         if (e->trainable[slot]) all.push_back(slot);
-    return optim_many(e, all);
+    return optim_many(e, all, counted, true);
 }
 
 // Are this graph's dispatches recorded and replayed?  With option exec_plans = auto: with a communicator, when a forward + backward pass

@@ -121,13 +121,29 @@ struct MultiArgs {
     int count;
 };
 
+// Where the step is read from, and who counts it: with `bump` the update is step *step_dev + 1, and the block that reads it last writes
+// that there (a launch of its own for the increment takes 2 us of a small model's step).
+struct StepSource {
+    uint32_t step;
+    const uint32_t* step_dev;
+    uint32_t ahead;
+    uint32_t* bump;
+    unsigned* arrivals;
+};
+
 template <bool ADAM, bool ZERO>
-__global__ void __launch_bounds__(256) update_multi_kernel(const __grid_constant__ MultiArgs a, AdamConsts c, uint32_t step,
-                                                           const uint32_t* __restrict__ step_dev) {
+__global__ void __launch_bounds__(256) update_multi_kernel(const __grid_constant__ MultiArgs a, AdamConsts c, const StepSource from) {
     fg_grid_enter();
     float inv_bc1 = 1.0f, inv_bc2 = 1.0f;
     if (ADAM) {
-        const uint32_t t = step_dev ? *step_dev : step;
+        const uint32_t t = from.step_dev ? *from.step_dev + from.ahead : from.step;
+        if (from.bump) {
+            __syncthreads();      // all threads of this block have read it
+            if (threadIdx.x == 0) {
+                __threadfence();
+                if (atomicInc(from.arrivals, gridDim.x - 1) == gridDim.x - 1) *from.bump = t;
+            }
+        }
         inv_bc1 = 1.0f / (1.0f - powf(c.b1, (float)t));
         inv_bc2 = 1.0f / (1.0f - powf(c.b2, (float)t));
     }
@@ -178,8 +194,8 @@ __global__ void __launch_bounds__(256) update_multi_kernel(const __grid_constant
     }
 }
 
-int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t count, AdamConsts c, uint32_t step,
-                     const uint32_t* step_dev, int32_t zero_grad, const char* who) {
+int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t count, AdamConsts c, const StepSource& source,
+                     int32_t zero_grad, const char* who) {
     for (uint32_t k = 0; k < count; ++k) {
         if (!t[k].w || !t[k].g || (adam && (!t[k].m || !t[k].v))) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, who);
         if (!fg_aligned16(t[k].w) || !fg_aligned16(t[k].g) || (adam && (!fg_aligned16(t[k].m) || !fg_aligned16(t[k].v))) ||
@@ -209,13 +225,16 @@ int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t
         a.first_chunk[cnt] = (uint32_t)chunks;
         a.count = cnt;
         const int grid = (int)std::min<uint64_t>(chunks, (uint64_t)ctx->sm_count * 8);
+        StepSource from = source;
+        for (uint32_t k = k0 + kMultiMax; k < count; ++k)
+            if (t[k].n) from.bump = nullptr;      // the last launch counts
         fg_time_rec* tr = fg_time_begin(ctx, adam ? FG_KERNEL_ADAMW : FG_KERNEL_SGD, bytes);
         if (adam) {
-            if (zero_grad) fg_launch(ctx, update_multi_kernel<true, true>, grid, 256, 0, a, c, step, step_dev);
-            else fg_launch(ctx, update_multi_kernel<true, false>, grid, 256, 0, a, c, step, step_dev);
+            if (zero_grad) fg_launch(ctx, update_multi_kernel<true, true>, grid, 256, 0, a, c, from);
+            else fg_launch(ctx, update_multi_kernel<true, false>, grid, 256, 0, a, c, from);
         } else {
-            if (zero_grad) fg_launch(ctx, update_multi_kernel<false, true>, grid, 256, 0, a, c, step, step_dev);
-            else fg_launch(ctx, update_multi_kernel<false, false>, grid, 256, 0, a, c, step, step_dev);
+            if (zero_grad) fg_launch(ctx, update_multi_kernel<false, true>, grid, 256, 0, a, c, from);
+            else fg_launch(ctx, update_multi_kernel<false, false>, grid, 256, 0, a, c, from);
         }
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
@@ -224,6 +243,17 @@ int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t
 }
 
 }  // namespace
+
+// The update of step *counter + 1; `count`: counter is that step afterwards.
+int32_t fg_adamw_next_step(fg_ctx* ctx, const fg_update_tensor* tensors, uint32_t n, const fg_adamw_hyper* h, uint32_t* counter, bool count) {
+    FG_ENTER(ctx);
+    uint64_t total = 0;
+    for (uint32_t k = 0; k < n; ++k) total += tensors[k].n;
+    if (total == 0) return count ? fg_counter_increment(ctx, counter) : FG_OK;
+    return update_multi(ctx, true, tensors, n, AdamConsts{h->lr, h->beta1, h->beta2, h->eps, h->weight_decay, 1.0f},
+                        StepSource{0, counter, 1, count ? counter : nullptr, fg_arrivals(ctx)}, 1,
+                        "AdamW update: a tensor is NULL, misaligned, or its pairs do not cover it");
+}
 
 extern "C" {
 
@@ -234,15 +264,15 @@ int32_t fg_adamw_step_multi(fg_ctx* ctx, const fg_update_tensor* tensors, uint32
     FG_REQUIRE(ctx, step_dev != nullptr || step >= 1, "fg_adamw_step_multi: step is 1-based");
     FG_REQUIRE(ctx, h->beta1 >= 0.f && h->beta1 < 1.f && h->beta2 >= 0.f && h->beta2 < 1.f,
                "fg_adamw_step_multi: betas must lie in [0,1)");
-    return update_multi(ctx, true, tensors, count, AdamConsts{h->lr, h->beta1, h->beta2, h->eps, h->weight_decay, grad_scale}, step,
-                        step_dev, zero_grad, "fg_adamw_step_multi: a tensor is NULL, misaligned, or its pairs do not cover it");
+    return update_multi(ctx, true, tensors, count, AdamConsts{h->lr, h->beta1, h->beta2, h->eps, h->weight_decay, grad_scale},
+                        StepSource{step, step_dev, 0, nullptr, nullptr}, zero_grad, "fg_adamw_step_multi: a tensor is NULL, misaligned, or its pairs do not cover it");
 }
 
 int32_t fg_sgd_step_multi(fg_ctx* ctx, const fg_update_tensor* tensors, uint32_t count, float lr, float grad_scale,
                           int32_t zero_grad) {
     FG_ENTER(ctx);
     FG_REQUIRE(ctx, tensors || count == 0, "fg_sgd_step_multi: NULL pointer");
-    return update_multi(ctx, false, tensors, count, AdamConsts{lr, 0.f, 0.f, 0.f, 0.f, grad_scale}, 1, nullptr, zero_grad,
+    return update_multi(ctx, false, tensors, count, AdamConsts{lr, 0.f, 0.f, 0.f, 0.f, grad_scale}, StepSource{1, nullptr, 0, nullptr, nullptr}, zero_grad,
                         "fg_sgd_step_multi: a tensor is NULL, misaligned, or its pairs do not cover it");
 }
 
