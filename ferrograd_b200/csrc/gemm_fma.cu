@@ -29,7 +29,7 @@ struct FmaArgs {
     const float *bias, *mul_saved;
     float *C, *preact;
     float* colsum_b;          // [N]: column sums of the B operand over k (the layer's bias gradient)
-    float* colsum_c;          // [tiles_m][N]: column sums of C over the rows of a tile
+    float* colsum_c;          // [N] column sums of C, or, of several tiles down, [ceil(M / 32)][N] of 32 rows each
     __nv_bfloat16* pairs;
     uint64_t pairs_stride, sA, sB, sC;
     uint32_t M, N, K, tiles_m, tiles;      // tiles of one matrix
@@ -104,22 +104,38 @@ __device__ __forceinline__ void copy_block(float* dst, uint32_t pitch, const flo
     if (v16) copy_chunks<ROWS, COLS, 4>(dst, pitch, src, ld, rows, cols);
     else copy_chunks<ROWS, COLS, 1>(dst, pitch, src, ld, rows, cols);
 }
-// dst *= act'(fac), the elements that this thread copied itself: no barrier between the copy and this.
+// dst *= act'(fac), the elements that this thread copied itself: no barrier between the copy and this.  The activation is chosen once
+// and the chunks are unrolled, so that their chains run side by side (chosen for each element, backward of 1936 x 19 x 958 took
+// twice as long).
+template <int ROWS, int COLS, int V, int ACT>
+__device__ __forceinline__ void factor_chunks(float* dst, const float* fac, uint32_t pitch) {
+    using C = Chunks<ROWS, COLS, V>;
+    const uint32_t r0 = C::row(), c = C::col();
+#pragma unroll 4
+    for (int i = 0; i < C::N; ++i) {
+        const uint32_t r = r0 + i * C::STEP, o = r * pitch + c;
+        if (!C::inside(r)) break;
+        if constexpr (V == 4) {
+            float4 v = *reinterpret_cast<float4*>(dst + o);
+            const float4 s = *reinterpret_cast<const float4*>(fac + o);
+            v.x *= fg_act_grad(ACT, s.x); v.y *= fg_act_grad(ACT, s.y); v.z *= fg_act_grad(ACT, s.z); v.w *= fg_act_grad(ACT, s.w);
+            *reinterpret_cast<float4*>(dst + o) = v;
+        } else {
+            dst[o] *= fg_act_grad(ACT, fac[o]);
+        }
+    }
+}
 template <int ROWS, int COLS>
 __device__ __forceinline__ void factor_block(float* dst, const float* fac, uint32_t pitch, bool v16, int act) {
-    if (v16) {
-        using C = Chunks<ROWS, COLS, 4>;
-#pragma unroll 2
-        for (uint32_t r = C::row(); r < ROWS; r += C::STEP) {
-            float4* const d = reinterpret_cast<float4*>(dst + r * pitch + C::col());
-            float4 v = *d;
-            const float4 s = *reinterpret_cast<const float4*>(fac + r * pitch + C::col());
-            v.x *= fg_act_grad(act, s.x); v.y *= fg_act_grad(act, s.y); v.z *= fg_act_grad(act, s.z); v.w *= fg_act_grad(act, s.w);
-            *d = v;
-        }
+    if (act == FG_ACT_GELU) {
+        if (v16) factor_chunks<ROWS, COLS, 4, FG_ACT_GELU>(dst, fac, pitch);
+        else factor_chunks<ROWS, COLS, 1, FG_ACT_GELU>(dst, fac, pitch);
+    } else if (act == FG_ACT_TANH) {
+        if (v16) factor_chunks<ROWS, COLS, 4, FG_ACT_TANH>(dst, fac, pitch);
+        else factor_chunks<ROWS, COLS, 1, FG_ACT_TANH>(dst, fac, pitch);
     } else {
-        using C = Chunks<ROWS, COLS, 1>;
-        for (uint32_t r = C::row(); r < ROWS; r += C::STEP) dst[r * pitch + C::col()] *= fg_act_grad(act, fac[r * pitch + C::col()]);
+        if (v16) factor_chunks<ROWS, COLS, 4, FG_ACT_RELU>(dst, fac, pitch);
+        else factor_chunks<ROWS, COLS, 1, FG_ACT_RELU>(dst, fac, pitch);
     }
 }
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
@@ -194,7 +210,7 @@ __device__ __forceinline__ void fma_unit(const FmaArgs& p, uint32_t unit, uint32
 #pragma unroll
         for (int j = 0; j < RN; ++j) acc[i][j] = 0.0f;
     const bool sum_b = TA && !TB && p.colsum_b && tm == 0;
-    float csb = 0.0f;
+    float csb = 0.0f, stages = 0.0f;      // a thread's share of a column's sum, and of that the last few stages'
     uint32_t slot = 0;
 #pragma unroll 1
     for (uint32_t t = t0; t < t1; ++t) {
@@ -211,8 +227,20 @@ __device__ __forceinline__ void fma_unit(const FmaArgs& p, uint32_t unit, uint32
         __syncthreads();      // everybody's copies of this stage are here, and nobody reads the one that is filled next
         load();
         if (TA && !TB && sum_b) {
-#pragma unroll 4
-            for (int k = 0; k < TK / (kT / kTN); ++k) csb += Bs[(k * (kT / kTN) + tid / kTN) * kTN + tid % kTN];
+            // A stage's terms in pairs, eight stages and all of them in a chain each.  Error against 64 bits over 36 layers of 34 to 5700
+            // rows: 0.6 to 1.2e-7 (column sums in a pass of their own: 0.8 to 1.5e-7; 4214 rows in one chain: 4.2e-7).
+            float part[2] = {0.0f, 0.0f};
+#pragma unroll 2
+            for (int k = 0; k < TK / (kT / kTN); k += 4) {
+                const float* const r = Bs + (k * (kT / kTN) + tid / kTN) * kTN + tid % kTN;
+                part[0] += r[0] + r[kT];
+                part[1] += r[2 * kT] + r[3 * kT];
+            }
+            stages += part[0] + part[1];
+            if ((t & 7u) == 7u) {
+                csb += stages;
+                stages = 0.0f;
+            }
         }
 #pragma unroll
         for (int q = 0; q < TK / KS / G; ++q) {
@@ -278,7 +306,6 @@ __device__ __forceinline__ void fma_unit(const FmaArgs& p, uint32_t unit, uint32
     cp_wait<0>();
     __syncthreads();
     __shared__ float colb[kT / kTN][kTN];
-    __shared__ float4 colc[kT];
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
         float* const r = sm + (g * TM + (TA ? ty * RM + i : ty + TY * i)) * kTN;
@@ -290,7 +317,7 @@ __device__ __forceinline__ void fma_unit(const FmaArgs& p, uint32_t unit, uint32
                 for (int j = h; j < h + 4; ++j) r[tx + TX * j] = acc[i][j];
         }
     }
-    if (TA && !TB && sum_b) colb[tid / kTN][tid % kTN] = csb;
+    if (TA && !TB && sum_b) colb[tid / kTN][tid % kTN] = csb + stages;
     __syncthreads();
     float4* const red = reinterpret_cast<float4*>(sm);
     auto group_sum = [&](uint32_t i) {
@@ -304,7 +331,7 @@ __device__ __forceinline__ void fma_unit(const FmaArgs& p, uint32_t unit, uint32
         __syncwarp();
         fgptx::cluster_sync_all();
     }
-    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4* const outs = red + TM * 16;      // (where the second group's sums were) what this CTA stores, for the column sums
     for (uint32_t e = tid; e < TM << lgq; e += kT) {
         const uint32_t m = e >> lgq, row = m0 + m, i = m * 16 + q0 + (e & (nq - 1));
         float4 z;
@@ -337,28 +364,46 @@ __device__ __forceinline__ void fma_unit(const FmaArgs& p, uint32_t unit, uint32
                 if (p.pairs) fg_store_pairs1(p.pairs, p.pairs_stride, off + j, o[j]);
             }
         }
-        cs = add4(cs, make_float4(o[0], o[1], o[2], o[3]));
+        if (G > 1 && p.colsum_c) outs[i] = make_float4(o[0], o[1], o[2], o[3]);
     }
-    if (p.colsum_c) {      // threads nq apart hold the same columns
-        colc[tid] = cs;
+    if (G > 1 && p.colsum_c) {
+        // In the order of the tensor-core kernels' epilogues: a block of 32 rows in four chains (row r in chain r % 4), which are added
+        // in pairs; then the blocks in order.
         __syncthreads();
-        if (tid < nq * 4) {
-            const uint32_t q = tid >> 2, j = tid & 3u, c = n0 + (q0 + q) * 4 + j;
-            float s = 0.0f;
-#pragma unroll 8
-            for (uint32_t k = q; k < (uint32_t)kT; k += nq) s += reinterpret_cast<const float*>(colc + k)[j];
-            if (c < p.N) p.colsum_c[(size_t)tm * p.N + c] = s;
+        const uint32_t q = q0 + (tid >> 2), j = tid & 3u, c = n0 + q * 4 + j;
+        if (tid < nq * 4 && c < p.N) {
+            float total = 0.0f;
+#pragma unroll 1
+            for (uint32_t b = 0; b < TM && m0 + b < p.M; b += 32) {
+                const uint32_t rows = min(min(32u, (uint32_t)TM), p.M - m0 - b);
+                float ch[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+                for (uint32_t r = 0; r < rows; r += 4)
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+                        if (r + t < rows) ch[t] += reinterpret_cast<const float*>(outs + (b + r + t) * 16 + q)[j];
+                const float sum = (ch[0] + ch[1]) + (ch[2] + ch[3]);
+                if (p.tiles_m > 1) p.colsum_c[(size_t)((m0 + b) >> 5) * p.N + c] = sum;
+                total += sum;
+            }
+            if (p.tiles_m == 1) p.colsum_c[c] = total;
         }
     }
     if (TA && !TB && sum_b && share == 0 && tid < kTN) {
         float s = 0.0f;
         for (uint32_t r = 0; r < split; ++r) {
             const uint32_t at = fgptx::smem_u32(&colb[0][tid]);
+            float v[kT / kTN];
 #pragma unroll
             for (int k = 0; k < kT / kTN; ++k) {
                 const uint32_t w = at + k * kTN * 4;
-                s += split > 1 ? fgptx::ld_cluster_f(fgptx::map_to_cta(w, r)) : colb[k][tid];
+                v[k] = split > 1 ? fgptx::ld_cluster_f(fgptx::map_to_cta(w, r)) : colb[k][tid];
             }
+#pragma unroll
+            for (int d = 1; d < kT / kTN; d *= 2)
+#pragma unroll
+                for (int k = 0; k < kT / kTN; k += 2 * d) v[k] += v[k + d];
+            s += v[0];
         }
         if (n0 + tid < p.N) p.colsum_b[n0 + tid] = s;
     }
@@ -387,10 +432,20 @@ __global__ void __launch_bounds__(kT, 2) gemm_fma_bwd_kernel(const __grid_consta
 struct FmaTile { uint32_t lg_tm, lg_tk; float cycles; };
 constexpr FmaTile kTiles[4] = {{2, 6, 45.0f}, {4, 6, 430.0f}, {5, 5, 790.0f}, {6, 5, 1530.0f}};
 
+// Are the rows of A, and those of B, copied in 16-byte chunks (with the factor that goes with them)?
+struct FmaRows { bool a16, b16; };
+bool rows16(const float* x, uint32_t cols, uint64_t stride, uint32_t batch) { return fg_aligned16(x) && cols % 4 == 0 && (batch == 1 || stride % 4 == 0); }
+FmaRows fma_rows(const FgFmaOp& o, uint32_t batch) {
+    return {rows16(o.A, o.ta ? o.M : o.K, o.sA, batch) && (!o.factor || o.ta || fg_aligned16(o.factor)),
+            rows16(o.B, o.tb ? o.K : o.N, o.sB, batch) && (!o.factor || o.tb || fg_aligned16(o.factor))};
+}
+
 struct FmaPlan { int tile[2]; uint32_t lg_split; float cycles; };
 // Tile heights and K-shares by estimated cycles, fitted to 49 calls under every tile and split (2.2 % slower than the best of each in
 // the geometric mean, 22 % at most): a stage takes a CTA no less than its copies' latency (270), the ends of a unit 1430, a meeting of
-// shares 180 + 150 each, and three CTAs share an SM.  (The host spends this on every call: shifts, no division.)
+// shares 180 + 150 each, and three CTAs share an SM.  A word that is copied alone and one that is added to a column's sum take 0.05 more:
+// with that, the gradients of 28 layers, 13 of them with odd rows, take 7 % more than under the best plan of each in the geometric mean
+// and 12 % without (2000 x 100 x 30: 17.7 and 23.1 us).  (The host spends this on every call: shifts, no division.)
 FmaPlan fma_plan(const fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch) {
     FmaPlan best{{0, 0}, 0, 0.0f};
     const float sms = (float)fg_free_sms(ctx), per_round = 1.0f / (3.0f * sms), per_sm = 0.4f / sms;
@@ -401,13 +456,17 @@ FmaPlan fma_plan(const fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch) {
         float ctas[2][4], work[2][4], alone[2][4];
         for (int j = 0; j < n; ++j) {
             const float cols = (float)((ops[j].N + kTN - 1) / kTN) * batch * (float)(1u << lg);
+            const FmaRows rows = fma_rows(ops[j], batch);
+            const float by_a = rows.a16 ? 0.0f : ops[j].factor && !ops[j].ta ? 0.1f : 0.05f;
+            const float by_b = (rows.b16 ? 0.0f : ops[j].factor && ops[j].ta ? 0.1f : 0.05f) + (ops[j].colsum_b ? 0.05f : 0.0f);
             for (int i = 0; i < 4; ++i) {
                 const FmaTile& t = kTiles[i];
+                const float more = (by_a * (float)(1u << t.lg_tm) + by_b * kTN) * (float)(1u << t.lg_tk);
                 const uint32_t nk = (ops[j].K + (1u << t.lg_tk) - 1) >> t.lg_tk;
                 const float steps = (float)((nk + (1u << lg) - 1) >> lg), tail = 1430.0f + (1u << t.lg_tm);
                 ctas[j][i] = (float)((ops[j].M + (1u << t.lg_tm) - 1) >> t.lg_tm) * cols;
-                work[j][i] = ctas[j][i] * (steps * t.cycles + 5.3f * tail);
-                alone[j][i] = steps * (t.cycles > 270.0f ? t.cycles : 270.0f) + tail;
+                work[j][i] = ctas[j][i] * (steps * (t.cycles + more) + 5.3f * tail);
+                alone[j][i] = steps * ((kTiles[i].cycles > 270.0f ? kTiles[i].cycles : 270.0f) + more) + tail;
             }
         }
         for (int i = 0; i < 4; ++i) {
@@ -483,17 +542,18 @@ int32_t launch_products(fg_ctx* ctx, const FgFmaOp* ops, uint32_t batch, bool in
         if ((tiles * batch + units) << plan.lg_split > 0x7fffffffull) return fg_fail(ctx, FG_ERR_INVALID_ARGUMENT, "GEMM: too many tiles");
         a.tiles = (uint32_t)tiles;
         a.act = o.act; a.factor_act = o.factor_act; a.mul_act = o.mul_act;
-        auto rows16 = [&](const float* x, uint32_t cols, uint64_t stride) { return fg_aligned16(x) && cols % 4 == 0 && (batch == 1 || stride % 4 == 0); };
-        a.a16 = rows16(o.A, o.ta ? o.M : o.K, o.sA) && (!o.factor || o.ta || fg_aligned16(o.factor));
-        a.b16 = rows16(o.B, o.tb ? o.K : o.N, o.sB) && (!o.factor || o.tb || fg_aligned16(o.factor));
-        a.c16 = rows16(o.C, o.N, o.sC) && (!o.preact || fg_aligned16(o.preact)) && (!o.mul_saved || fg_aligned16(o.mul_saved)) &&
+        const FmaRows rows = fma_rows(o, batch);
+        a.a16 = rows.a16;
+        a.b16 = rows.b16;
+        a.c16 = rows16(o.C, o.N, o.sC, batch) && (!o.preact || fg_aligned16(o.preact)) && (!o.mul_saved || fg_aligned16(o.mul_saved)) &&
                 (!o.pairs || (fg_aligned16(o.pairs) && o.pairs_stride % 4 == 0));
         if (o.colsum_c && tiles_m > 1) {
             void* p;
-            const int32_t s = fg_ws_alloc(ctx, (uint64_t)tiles_m * o.N * 4, &p);
+            part_rows = (o.M + 31) / 32;
+            const int32_t s = fg_ws_alloc(ctx, (uint64_t)part_rows * o.N * 4, &p);
             if (s != FG_OK) return s;
             a.colsum_c = part = (float*)p;
-            below = o.colsum_c; part_rows = tiles_m; part_cols = o.N;
+            below = o.colsum_c; part_cols = o.N;
         }
         auto room = [&](auto t) { return fma_smem<decltype(t)>(o, plan.lg_split); };
         const size_t bytes = in_order ? room(TileOrdered{}) : with_tile(plan.tile[j], room);
