@@ -412,6 +412,9 @@ struct FgFmaOp {
 // One product, or two in one launch (the first with ta, the second with tb).  in_order: every sum is one chain of FMAs in the order of
 // k, the exact path's results.  Room in the arena for one row of C's column sums per 32 rows.
 int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch, bool in_order);
+// Is it the kernel for the forward product of [M,K] x [K,N], or for one or both of its gradients?
+enum { kFgForward = 0, kFgGradB = 1, kFgGradA = 2 };
+bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products);
 // A layer's backward pass with it: dZ = dZ * act'(factor); dB, dbias; the exchange; dA (* act'(mul_saved), pairs, column sums).
 struct FgFmaBwd {
     uint32_t M, N, K;
@@ -428,7 +431,7 @@ struct FgFmaBwd {
 };
 int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b);
 // Does the backward pass of this layer sum dZ's columns on its way (fg_gemm_bwd_paired_f32's dbias costs nothing)?
-bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K);
+bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool dA);
 uint64_t fg_gemm_skinny_scratch_bytes(uint32_t M, uint32_t N, uint32_t K);   // enough for any one skinny launch
 int32_t fg_gemm_skinny_n_launch(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, const float* A, const float* B, float* C,
                                 const float* bias, int act, float* preact_out);

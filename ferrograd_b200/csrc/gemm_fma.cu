@@ -1,5 +1,6 @@
 // f32 products with plain FMAs in shares of k: what FG_GEMM_AUTO runs where the tensor-core kernels' fixed costs, or their tiles of
-// 128 rows, are the most of a product -- fewer than 64 samples, or fewer than 2^22 multiply-adds -- forward and both gradients.
+// 128 rows, are the most of a product -- fewer than 64 samples, or up to some 40 million multiply-adds (fg_gemm_fma_suits) --
+// forward and both gradients.
 //
 // What it replaces: the reference's tiled matmul and its backward edges (crates/ferrograd-nn/src/op/matmul/mod.rs:17-188,
 // generic.rs:13-325) with the elementwise work around them: bias and activation (kernel/forward.rs:373-457), the activation's
@@ -587,6 +588,19 @@ int32_t launch_products(fg_ctx* ctx, const FgFmaOp* ops, uint32_t batch, bool in
 int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch, bool in_order) {
     if (batch == 0) return FG_OK;
     return n > 1 ? launch_products<2>(ctx, ops, batch, in_order) : launch_products<1>(ctx, ops, batch, in_order);
+}
+
+// Multiply-adds of a launch with its tiles' padding, and up to how many of them this kernel is the faster one.  66 products of 1 to 130
+// million multiply-adds, this kernel and the tensor-core routes (us): forward 384 x 256 x 200 4.6 / 8.3, 256 x 448 x 320 5.2 / 7.4,
+// 512 x 800 x 128 7.2 / 7.0, 448 x 1024 x 200 10.2 / 8.4; dB with its bias gradient 384 x 256 x 200 6.0 / 9.4, 128 x 656 x 536 7.6 / 7.3; both
+// gradients 128 x 256 x 256 6.8 / 11.5, 128 x 640 x 208 10.3 / 12.0, 384 x 256 x 200 9.9 / 8.9; of dZ rows that are copied word by word
+// 1000 x 63 x 150 12.2 / 18.7, 2000 x 100 x 30 17.7 / 18.9, 2800 x 101 x 30 22.8 / 20.8.
+bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products) {
+    if (products != kFgForward && N <= 16) return false;                // the narrow layer's own kernels
+    auto padded = [](uint64_t m, uint64_t n, uint64_t k) { return (m + 15) / 16 * 16 * ((n + kTN - 1) / kTN * kTN) * ((k + 31) / 32 * 32); };
+    if (products == kFgForward) return N > 16 && padded(M, N, K) <= 45000000ull;
+    const uint64_t work = (products & kFgGradB ? padded(K, N, M) : 0) + (products & kFgGradA ? padded(M, K, N) : 0);
+    return work <= (products != (kFgGradA | kFgGradB) ? 40000000ull : N % 4 ? 24000000ull : 32000000ull);
 }
 
 // The backward pass of one layer, see FgFmaBwd.  The caller has reserved room for dZ (M * N floats) and for column sums of dA.

@@ -2981,6 +2981,13 @@ int pick_path(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K) {
     return 2;   // AUTO: tf32 main term + bf16 cross terms (same accuracy class, two thirds of the tensor work)
 }
 
+// Does FG_GEMM_AUTO take the FMA kernel for the forward product, or for one or both gradients?  (An option that names a tensor-core
+// kernel keeps what those can run.)
+bool takes_fma(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, int products) {
+    if (mode != FG_GEMM_AUTO) return false;
+    return pick_path(ctx, mode, M, N, K) == 0 || (conv_allowed(ctx) && !ctx->opt_conv_bn && fg_gemm_fma_suits(M, N, K, products));
+}
+
 }  // namespace
 
 namespace {
@@ -2999,7 +3006,7 @@ int32_t gemm_fwd_core(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
     const int path = pick_path(ctx, mode, M, N, K);
     // The result's pairs, when no GEMM epilogue wrote them.
     auto pairs_after = [&]() -> int32_t { return c_pairs ? launch_pairs(ctx, C, mn, c_pairs, c_stride) : FG_OK; };
-    if (path == 0 && mode == FG_GEMM_AUTO) {
+    if (takes_fma(ctx, mode, M, N, K, kFgForward)) {
         FgFmaOp o{};
         o.ta = transA; o.tb = transB; o.M = M; o.N = N; o.K = K; o.A = A.x; o.B = B.x; o.C = C;
         o.bias = bias; o.act = act; o.preact = preact_out; o.pairs = c_pairs; o.pairs_stride = c_stride;
@@ -3148,12 +3155,6 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
         {
             uint64_t need = mn * 4 + (uint64_t)((M + 255) / 256) * N * 4 + 1024;
             { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
-        }
-        if (mode == FG_GEMM_AUTO && !dZ_out) {
-            FgFmaBwd b{};
-            b.M = M; b.N = N; b.K = K; b.A = A; b.B = B; b.dZ = dY; b.factor = fuse ? saved : nullptr; b.factor_act = act;
-            b.dA = dA; b.dB = dB; b.dbias = dbias; b.exch_buf = exch_buf; b.exch_count = exch_count;
-            return fg_gemm_fma_bwd(ctx, b);
         }
         // Exact path: materialise dZ, then two SIMT GEMMs.
         if (fuse || dZ_out) {
@@ -3378,9 +3379,8 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         o.mul_saved = (const float*)p;
         return FG_OK;
     };
-    const bool narrow = N <= 16, exact = pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 0;
-    const BwdRoutes rt = narrow ? BwdRoutes{} : pick_bwd_routes(ctx, M, N, K, A, B, dZ, dB, dA, o.mul_saved);
-    if (exact && (narrow || rt.planes)) {
+    const bool narrow = N <= 16;
+    if ((dA || dB) && takes_fma(ctx, FG_GEMM_AUTO, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0))) {
         if (dA && o.mul_saved != dA && (s = saved_apart()) != FG_OK) return s;      // (an element is read and written by one thread)
         FgFmaBwd b{};
         b.M = M; b.N = N; b.K = K; b.A = A.x; b.B = B.x; b.dZ = dZ.x; b.dA = dA; b.dB = dB; b.dbias = dbias;
@@ -3388,6 +3388,7 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         b.exch_buf = exch_buf; b.exch_count = exch_count;
         return fg_gemm_fma_bwd(ctx, b);
     }
+    const BwdRoutes rt = narrow ? BwdRoutes{} : pick_bwd_routes(ctx, M, N, K, A, B, dZ, dB, dA, o.mul_saved);
     if (dbias && (s = fg_colsum_launch(ctx, M, N, dZ.x, dbias)) != FG_OK) return s;
     const uint32_t cs_chunks = (M + 31) / 32;
     float* cs_part = nullptr;
@@ -3439,11 +3440,8 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
 
 }  // namespace
 
-bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K) {
-    if (pick_path(ctx, FG_GEMM_AUTO, M, N, K) != 0) return false;
-    float* const any = reinterpret_cast<float*>(uintptr_t(256));      // only the alignment counts
-    const PairedArg t{any, any, 0};
-    return N <= 16 || (pick_bwd_routes(ctx, M, N, K, t, t, t, any, any, any).planes && pick_bwd_routes(ctx, M, N, K, t, t, t, any, nullptr, nullptr).planes);
+bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool dA) {
+    return takes_fma(ctx, FG_GEMM_AUTO, M, N, K, kFgGradB | (dA ? kFgGradA : 0));
 }
 
 uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K) {
@@ -3451,13 +3449,14 @@ uint32_t fg_gemm_reads_pairs(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t
     float* const any = reinterpret_cast<float*>(uintptr_t(256));      // only the alignment counts, and that pairs are there
     const PairedArg t{any, any, 0};
     uint32_t bits = 0;
-    if (pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 2) {
+    if (pick_path(ctx, FG_GEMM_AUTO, M, N, K) == 2 && !takes_fma(ctx, FG_GEMM_AUTO, M, N, K, kFgForward)) {
         const int ca = !in_place32(any, K, 1, 0), cb = !in_place32(any, N, 1, 0);
         const Route r = pick_route(ctx, M, N, K, paired_shape_ok(ctx, M, N, K, K, N) && N % 4 == 0, 0.0, 0, (ca ? (double)M * K : 0.0) + (cb ? (double)K * N : 0.0),
                                    ca + cb);
         if (r.kind == kRoutePair) bits |= 1 | 2;
     }
     for (int want = 1; want < 4; ++want) {      // dB, dA or both
+        if (takes_fma(ctx, FG_GEMM_AUTO, M, N, K, want)) continue;
         const BwdRoutes r = pick_bwd_routes(ctx, M, N, K, t, t, t, want & 1 ? any : nullptr, want & 2 ? any : nullptr, nullptr);
         if ((want & 1) && !r.planes && r.dB.kind == kRoutePair) bits |= 1 | 4;
         if ((want & 2) && !r.planes && r.dA.kind == kRoutePair) bits |= 2 | 4;
@@ -3481,6 +3480,14 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, !dB || A, "fg_gemm_bwd_f32: dB needs A");
     const bool fuse = act != FG_ACT_NONE;
     const int path = pick_path(ctx, mode, M, N, K);
+    if (!dZ_out && (path == 0 || dA || dB) && takes_fma(ctx, mode, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0))) {
+        int32_t s = fg_ws_ensure(ctx, (uint64_t)M * N * 4 + (uint64_t)((M + 255) / 256) * N * 4 + 1024);
+        if (s != FG_OK) return s;
+        FgFmaBwd b{};
+        b.M = M; b.N = N; b.K = K; b.A = A; b.B = B; b.dZ = dY; b.factor = fuse ? saved : nullptr; b.factor_act = act;
+        b.dA = dA; b.dB = dB; b.dbias = dbias; b.exch_buf = exch_buf; b.exch_count = exch_count;
+        return fg_gemm_fma_bwd(ctx, b);
+    }
     // (prep_kernel takes up to 65535 * 32 rows, the planes twice as many)
     if (path == 2 && N > 16 && (dA || dB) && M <= 65535u * 32u) {
         // dZ (with its pairs, if a product needs them) and the bias gradient's partials in one pass, then both products

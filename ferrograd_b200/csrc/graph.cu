@@ -786,7 +786,7 @@ static int32_t backward_eager(fg_exec* e) {
                     if (below_act != FG_ACT_NONE) below_saved = below_act == FG_ACT_GELU ? (const float*)below->preact->ptr : vptr(e, below->out);
                     da_pairs = below->dz_pairs ? below->dz_pairs->ptr : nullptr;
                     // (a small layer's own products sum its dZ on their way; beside an exchange the order of completion stays)
-                    const bool own_sums = !e->ctx->comm && wanted(below->b) && fg_gemm_bwd_sums_bias(e->ctx, below->M, below->N, below->K);
+                    const bool own_sums = !e->ctx->comm && wanted(below->b) && fg_gemm_bwd_sums_bias(e->ctx, below->M, below->N, below->K, wanted(below->a));
                     if (below->bias >= 0 && !written[below->bias] && wanted(below->bias) && !own_sums) below_dbias = gptr(e, below->bias);
                 }
                 float* dbias = (gs.bias >= 0 && !gs.dbias_done && wanted(gs.bias)) ? gptr(e, gs.bias) : nullptr;

@@ -122,6 +122,30 @@ def test_paired_backward(ctx, oracle, M, N, K, over):
     assert np.array_equal(p[0], to_bf16_bits(got).ravel()) and np.array_equal(p[1], to_bf16_bits(got - hi).ravel())
 
 
+# Around the most multiply-adds that this kernel takes: M * N * K, padded to its tiles, of 45 million forward and 32 or 40 million backward.
+@pytest.mark.parametrize("M,N,K", [(384, 256, 416), (352, 250, 481), (352, 250, 512), (128, 17, 1600), (128, 25, 1900), (1000, 100, 161), (96, 3000, 36)])
+@pytest.mark.parametrize("act", ["relu", "gelu"])
+def test_both_sides_of_the_range(ctx, oracle, M, N, K, act):
+    r = rng(M + N + K)
+    f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
+    A, B, dY, S, bias = f(M, K), f(K, N), f(M, N), f(M, N), f(N)
+    a, b, y, sv, v = (up(ctx, x) for x in (A, B, dY, S, bias))
+    C, P, dA, dB, db = (up(ctx, np.zeros(s)) for s in ((M, N), (M, N), (M, K), (K, N), (N,)))
+    # (the tensor-core kernels of the far side split an f32 into a tf32 and a bf16 rest: 2^-19 of a term)
+    close = lambda x, ref, k, what: rel_err_ok(x, ref, 2.0 ** -24 * (16 + 5 * math.sqrt(k)) + 2.0 ** -19)[0] or pytest.fail(what)   # noqa: E731
+    ctx.gemm(a[1], b[1], C[1], M, N, K, bias=v[1], act=act, preact_out=P[1])
+    close(ctx.to_numpy(P[0]).reshape(M, N), oracle.gemm(A, B, f64=True) + bias, K, "pre-activation")
+    dz = oracle.act_bwd(dY, S, act)
+    for grads in (("dA", "dB"), ("dB",), ("dA",)):
+        ctx.gemm_bwd(a[1], b[1], y[1], M, N, K, act=act, saved=sv[1], dA=dA[1] if "dA" in grads else None, dB=dB[1] if "dB" in grads else None,
+                     dbias=db[1])
+        if "dA" in grads:
+            close(ctx.to_numpy(dA[0]).reshape(M, K), oracle.gemm(dz, B, transB=True, f64=True), N, f"dA of {grads}")
+        if "dB" in grads:
+            close(ctx.to_numpy(dB[0]).reshape(K, N), oracle.gemm(A, dz, transA=True, f64=True), M, f"dB of {grads}")
+        close(ctx.to_numpy(db[0]), dz.astype(np.float64).sum(0), M, f"dbias of {grads}")
+
+
 @pytest.mark.parametrize("T,M,N,K", [(1, 4, 4, 4), (7, 33, 66, 97), (24, 128, 26, 44), (3, 2, 300, 256), (9, 19, 335, 256), (31, 60, 500, 70)])
 @pytest.mark.parametrize("act", ["none", "gelu"])
 @pytest.mark.parametrize("gap", [0, 5])
