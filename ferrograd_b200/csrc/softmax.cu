@@ -99,10 +99,31 @@ struct CeArgs {
     float* probs;
     uint32_t* argmax;
     float* y;   // MODE 0 output
+    float* mean;               // the mean of loss_row, by the block that arrives last (NULL: a launch of its own adds)
+    unsigned* arrivals;
 };
+
+// The mean of the rows' losses, in a fixed order, in thread 0 of a block.
+__device__ __forceinline__ void mean_of_rows(const float* x, uint32_t n, float* out, float* red) {
+    float s = 0.0f, v[8];
+    for (uint64_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {      // eight loads in flight, added in order
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = i0 + j * blockDim.x < n ? __ldcg(x + i0 + j * blockDim.x) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += v[j];
+    }
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) *out = s / (float)n;
+}
+// At the end of a kernel whose blocks have left their rows' losses.
+template <int MODE>
+__device__ __forceinline__ void leave_mean(const CeArgs& a, float* red) {
+    if (MODE == 1 && a.mean && fg_last_block(a.arrivals, gridDim.x)) mean_of_rows(a.loss_row, a.rows, a.mean, red);
+}
 
 template <int MODE, bool VEC>
 __global__ void softmax_stream_kernel(CeArgs a) {
+    fg_grid_enter();
     __shared__ float red[32];
     __shared__ uint32_t redi[32];
     const uint32_t cols = a.cols;
@@ -269,6 +290,7 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    fg_grid_enter();
     uint32_t row = blockIdx.x;
     if (tid == 0 && row < a.rows) prefetch_row(smem_u32(stage), a.x + (size_t)row * cols, row_bytes, bar);
     uint32_t parity = 0;
@@ -348,6 +370,7 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
         for (int j = 0; j < kRowNV; ++j)
             if (tid + j * kRowT < ncol4) softmax_put4<MODE>(a, o0, o1, tid + j * kRowT, lab, v[j], inv, true);
     }
+    leave_mean<MODE>(a, red_max);
 }
 
 // ------------------------------------------------------------------------------------
@@ -359,6 +382,7 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
 // ------------------------------------------------------------------------------------
 template <int MODE, int NV>
 __global__ void __launch_bounds__(256) softmax_held_kernel(CeArgs a) {
+    fg_grid_enter();
     __shared__ float red[32];
     __shared__ uint32_t redi[32];
     const uint32_t cols = a.cols, n4 = cols >> 2;
@@ -427,6 +451,7 @@ __global__ void __launch_bounds__(256) softmax_held_kernel(CeArgs a) {
             }
         }
     }
+    leave_mean<MODE>(a, red);
 }
 
 // The same for the backward pass: y and dy of a row are read once.
@@ -434,6 +459,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) softmax_bwd_held_kernel(uint32_t rows, uint32_t cols, const float* __restrict__ y,
                                                                const float* __restrict__ dy, float* __restrict__ dx,
                                                                int accumulate) {
+    fg_grid_enter();
     __shared__ float red[32];
     const uint32_t n4 = cols >> 2;
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -542,6 +568,8 @@ __global__ void __launch_bounds__(256) softmax_warp_kernel(CeArgs a) {
         for (int j = 0; j < NV; ++j)
             if (lane + 32u * j < cols) softmax_put<MODE>(a, base + lane + 32u * j, lane + 32u * j, lab, v[j], inv);
     }
+    __shared__ float red[32];
+    leave_mean<MODE>(a, red);
 }
 
 // Where the 16-byte accesses of a row start: `head` words before them, n4 groups of four, and `extra`, the index of the one
@@ -560,6 +588,7 @@ __device__ __forceinline__ RowEdges row_edges(const float* row, uint32_t cols) {
 
 template <int MODE, int NV>
 __global__ void __launch_bounds__(1024) softmax_edge_kernel(CeArgs a) {
+    fg_grid_enter();
     // one array per reduction, so that each costs one barrier: an array is written again only after another barrier
     __shared__ float red_max[32], red_sum[32];
     __shared__ uint32_t s_arg;
@@ -621,6 +650,7 @@ __global__ void __launch_bounds__(1024) softmax_edge_kernel(CeArgs a) {
             if (t + nt * j < ed.n4) softmax_put4<MODE>(a, o0, o1, t + nt * j, lab4, v[j], inv, true);
         if (ed.extra < cols) softmax_put<MODE>(a, base + ed.extra, ed.extra, lab, ve, inv);
     }
+    leave_mean<MODE>(a, red_sum);
 }
 
 template <int NV>
@@ -658,6 +688,7 @@ __global__ void __launch_bounds__(256) softmax_bwd_warp_kernel(uint32_t rows, ui
 template <int NV, bool ACC, bool ONCE>
 __global__ void __launch_bounds__(4096 / NV) softmax_bwd_edge_kernel(uint32_t rows, uint32_t cols, const float* __restrict__ y,
                                                                  const float* __restrict__ dy, float* __restrict__ dx) {
+    fg_grid_enter();
     __shared__ float red[2][32];        // rows take turns, so that the reduction costs one barrier
     auto fetch = [](const float4* p) { return ONCE ? __ldcs(p) : *p; };
     const uint32_t t = threadIdx.x, nt = blockDim.x, lane = t & 31u, nw = nt >> 5;
@@ -702,6 +733,7 @@ __global__ void __launch_bounds__(4096 / NV) softmax_bwd_edge_kernel(uint32_t ro
 template <bool VEC>
 __global__ void softmax_bwd_kernel(uint32_t rows, uint32_t cols, const float* __restrict__ y,
                                    const float* __restrict__ dy, float* __restrict__ dx, int accumulate) {
+    fg_grid_enter();
     __shared__ float red[32];
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const float* yr = y + (size_t)row * cols;
@@ -760,15 +792,7 @@ __global__ void __launch_bounds__(256) ce_elem_kernel(const float* __restrict__ 
 __global__ void mean_kernel(const float* __restrict__ x, uint32_t n, float* __restrict__ out) {
     fg_grid_enter();
     __shared__ float red[32];
-    float s = 0.0f, v[8];
-    for (uint64_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {      // eight loads in flight, added in order
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = i0 + j * blockDim.x < n ? x[i0 + j * blockDim.x] : 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s += v[j];
-    }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) *out = s / (float)n;
+    mean_of_rows(x, n, out, red);
 }
 
 // Algorithmic HBM bytes of the fused CE kernel: logits in, dlogits (and probs) out.
@@ -798,8 +822,22 @@ int rows_grid(const fg_ctx* ctx, uint64_t blocks, int threads) {
     return (int)(blocks < cap ? blocks : cap);
 }
 
+// Called by the kernels that can add the mean themselves: do they (see fg_fold_in_launch)?  Otherwise a.mean stays for the caller.
+// With that, and launches that start while the kernel before them ends, the loss of 712 x 768 takes 8.0 us instead of 9.2 and 11.2
+// before the calls had their own module, 2384 x 64 8.0 / 8.0 / 10.4, 600 x 32000 39.3 / 41.2, 8192 x 32000 361 / 365; softmax and its
+// gradient on 1728 x 1285 9.6 / 12.5, 4096 x 10001 132.6 / 137.1.
 template <int MODE>
-int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
+CeArgs with_mean(fg_ctx* ctx, CeArgs& a, int grid) {
+    CeArgs k = a;
+    if (MODE == 1 && a.mean && fg_fold_in_launch(ctx, (uint64_t)grid)) {
+        k.arrivals = fg_arrivals(ctx);
+        a.mean = nullptr;
+    } else k.mean = nullptr;
+    return k;
+}
+
+template <int MODE>
+int32_t launch_rows(fg_ctx* ctx, CeArgs& a) {
     const bool vec = (a.cols % 4 == 0) && fg_aligned16(a.x) &&
                      (MODE == 0 ? fg_aligned16(a.y)
                                 : ((!a.dlogits || fg_aligned16(a.dlogits)) && (!a.probs || fg_aligned16(a.probs))));
@@ -813,7 +851,8 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
         }
         int grid = (int)(a.rows < (uint32_t)ctx->sm_count ? a.rows : (uint32_t)ctx->sm_count);
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
-        softmax_rowreg_kernel<MODE><<<grid, kRowT, smem, ctx->stream>>>(a, ctx->dev_status);
+        const CeArgs k = with_mean<MODE>(ctx, a, grid);
+        fg_launch(ctx, softmax_rowreg_kernel<MODE>, grid, kRowT, smem, k, ctx->dev_status);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -823,10 +862,11 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
         const int grid = (int)(a.rows < cap ? a.rows : cap);
         const uint32_t nv = (a.cols / 4 + 255) / 256;      // float4s per thread: 1 .. 8
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
-        if (nv <= 1) softmax_held_kernel<MODE, 1><<<grid, 256, 0, ctx->stream>>>(a);
-        else if (nv <= 2) softmax_held_kernel<MODE, 2><<<grid, 256, 0, ctx->stream>>>(a);
-        else if (nv <= 4) softmax_held_kernel<MODE, 4><<<grid, 256, 0, ctx->stream>>>(a);
-        else softmax_held_kernel<MODE, 8><<<grid, 256, 0, ctx->stream>>>(a);
+        const CeArgs k = with_mean<MODE>(ctx, a, grid);
+        if (nv <= 1) fg_launch(ctx, softmax_held_kernel<MODE, 1>, grid, 256, 0, k);
+        else if (nv <= 2) fg_launch(ctx, softmax_held_kernel<MODE, 2>, grid, 256, 0, k);
+        else if (nv <= 4) fg_launch(ctx, softmax_held_kernel<MODE, 4>, grid, 256, 0, k);
+        else fg_launch(ctx, softmax_held_kernel<MODE, 8>, grid, 256, 0, k);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -834,9 +874,10 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
     if (a.cols <= kWarpRowCols) {
         const int grid = rows_grid(ctx, ((uint64_t)a.rows + 7) / 8, 256);
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
-        if (a.cols <= 32) fg_launch(ctx, softmax_warp_kernel<MODE, 1>, grid, 256, 0, a);
-        else if (a.cols <= 128) fg_launch(ctx, softmax_warp_kernel<MODE, 4>, grid, 256, 0, a);
-        else fg_launch(ctx, softmax_warp_kernel<MODE, 16>, grid, 256, 0, a);
+        const CeArgs k = with_mean<MODE>(ctx, a, grid);
+        if (a.cols <= 32) fg_launch(ctx, softmax_warp_kernel<MODE, 1>, grid, 256, 0, k);
+        else if (a.cols <= 128) fg_launch(ctx, softmax_warp_kernel<MODE, 4>, grid, 256, 0, k);
+        else fg_launch(ctx, softmax_warp_kernel<MODE, 16>, grid, 256, 0, k);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -846,7 +887,8 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
         const int threads = held_threads(a.cols, 32);
         const int grid = rows_grid(ctx, a.rows, threads);
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
-        softmax_edge_kernel<MODE, 8><<<grid, threads, 0, ctx->stream>>>(a);
+        const CeArgs k = with_mean<MODE>(ctx, a, grid);
+        fg_launch(ctx, softmax_edge_kernel<MODE, 8>, grid, threads, 0, k);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -854,8 +896,10 @@ int32_t launch_rows(fg_ctx* ctx, const CeArgs& a) {
     const int threads = stream_threads(ctx, a.rows, a.cols);
     const int grid = rows_grid(ctx, a.rows, threads);
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
-    if (vec) softmax_stream_kernel<MODE, true><<<grid, threads, 0, ctx->stream>>>(a);
-    else softmax_stream_kernel<MODE, false><<<grid, threads, 0, ctx->stream>>>(a);
+    CeArgs k = a;
+    k.mean = nullptr;
+    if (vec) fg_launch(ctx, softmax_stream_kernel<MODE, true>, grid, threads, 0, k);
+    else fg_launch(ctx, softmax_stream_kernel<MODE, false>, grid, threads, 0, k);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;
@@ -899,10 +943,10 @@ int32_t fg_softmax_bwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* y
         const int grid8 = (int)(rows < cap8 ? rows : cap8);
         const uint32_t nv = (cols / 4 + 255) / 256;
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, (accumulate ? 16.0 : 12.0) * rows * cols);
-        if (nv <= 1) softmax_bwd_held_kernel<1><<<grid8, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
-        else if (nv <= 2) softmax_bwd_held_kernel<2><<<grid8, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
-        else if (nv <= 4) softmax_bwd_held_kernel<4><<<grid8, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
-        else softmax_bwd_held_kernel<8><<<grid8, 256, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
+        if (nv <= 1) fg_launch(ctx, softmax_bwd_held_kernel<1>, grid8, 256, 0, rows, cols, y, dy, dx, accumulate);
+        else if (nv <= 2) fg_launch(ctx, softmax_bwd_held_kernel<2>, grid8, 256, 0, rows, cols, y, dy, dx, accumulate);
+        else if (nv <= 4) fg_launch(ctx, softmax_bwd_held_kernel<4>, grid8, 256, 0, rows, cols, y, dy, dx, accumulate);
+        else fg_launch(ctx, softmax_bwd_held_kernel<8>, grid8, 256, 0, rows, cols, y, dy, dx, accumulate);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -920,11 +964,11 @@ int32_t fg_softmax_bwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* y
     if (cols <= kEdgeRowColsBwd && lie_alike(y, dy) && lie_alike(y, dx)) {
         const int threads = held_threads(cols, accumulate ? 16 : 32), grid = rows_grid(ctx, rows, threads);
         if (accumulate) {
-            if (cols > 8192) softmax_bwd_edge_kernel<4, true, false><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
-            else softmax_bwd_edge_kernel<4, true, true><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
+            if (cols > 8192) fg_launch(ctx, softmax_bwd_edge_kernel<4, true, false>, grid, threads, 0, rows, cols, y, dy, dx);
+            else fg_launch(ctx, softmax_bwd_edge_kernel<4, true, true>, grid, threads, 0, rows, cols, y, dy, dx);
         } else {
-            if (cols > 8192) softmax_bwd_edge_kernel<8, false, false><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
-            else softmax_bwd_edge_kernel<8, false, true><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx);
+            if (cols > 8192) fg_launch(ctx, softmax_bwd_edge_kernel<8, false, false>, grid, threads, 0, rows, cols, y, dy, dx);
+            else fg_launch(ctx, softmax_bwd_edge_kernel<8, false, true>, grid, threads, 0, rows, cols, y, dy, dx);
         }
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
@@ -932,8 +976,8 @@ int32_t fg_softmax_bwd(fg_ctx* ctx, uint32_t rows, uint32_t cols, const float* y
     }
     const int threads = stream_threads(ctx, rows, cols);
     const int grid = rows_grid(ctx, rows, threads);
-    if (vec) softmax_bwd_kernel<true><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
-    else softmax_bwd_kernel<false><<<grid, threads, 0, ctx->stream>>>(rows, cols, y, dy, dx, accumulate);
+    if (vec) fg_launch(ctx, softmax_bwd_kernel<true>, grid, threads, 0, rows, cols, y, dy, dx, accumulate);
+    else fg_launch(ctx, softmax_bwd_kernel<false>, grid, threads, 0, rows, cols, y, dy, dx, accumulate);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;
@@ -951,9 +995,10 @@ int32_t fg_softmax_ce_fwd_bwd(fg_ctx* ctx, const float* logits, const uint32_t* 
     CeArgs a{};
     a.x = logits; a.labels = labels; a.rows = rows; a.cols = cols; a.scale = grad_scale;
     a.loss_row = loss_row_out; a.dlogits = dlogits_out; a.probs = probs_out; a.argmax = argmax_out;
+    a.mean = loss_mean_out;
     int32_t s = launch_rows<1>(ctx, a);
     if (s != FG_OK) return s;
-    if (loss_mean_out) {
+    if (a.mean) {
         fg_launch(ctx, mean_kernel, 1, 1024, 0, loss_row_out, rows, loss_mean_out);
         FG_LAUNCHED(ctx);
     }

@@ -106,3 +106,17 @@ def test_masked_columns_and_in_place(ctx, cols):
     x64 = x.astype(np.float64)
     e = np.exp(x64 - x64.max(1, keepdims=True))
     check(ctx.to_numpy(t), e / e.sum(1, keepdims=True), "masked softmax")
+
+
+# The mean of the losses is added by the last of up to two blocks per SM (of eight rows, or of one), or by a launch of its own.
+@pytest.mark.parametrize("rows,cols", [(1, 10), (295, 30), (2368, 129), (2369, 511), (295, 512), (297, 4096), (296, 1001), (300, 5001), (2, 8192), (700, 32768),
+                                       (40, 32769)])
+def test_mean_of_the_losses(ctx, rows, cols):
+    r = np.random.Generator(np.random.Philox(rows * cols))
+    x, lab = ctx.init_tensor_f32((rows, cols), r.standard_normal((rows, cols)).astype(np.float32)), r.integers(0, cols, rows).astype(np.uint32)
+    loss, mean, labels = ctx.new_tensor((rows,)), ctx.new_tensor((1,)), ctx.init_tensor_u32((rows,), lab)
+    for _ in range(2):
+        ctx.softmax_ce(x, labels, rows, cols, loss_row=loss, loss_mean=mean)
+        # positive terms, added in chains of rows / 32 at most and trees: (rows / 32 + 16) roundings at most
+        want = ctx.to_numpy(loss).astype(np.float64).mean()
+        assert abs(float(ctx.to_numpy(mean)[0]) - want) <= 2.0 ** -24 * (rows / 32 + 16) * want
