@@ -18,17 +18,17 @@ inline uint64_t fg_sms_beside(int sms, bool exchange, int reserved) { return (ui
 // CTAs of a launch: one for each K-share, or no more than SMs that walk the units.
 inline uint64_t conv_grid(uint64_t units, uint32_t split, uint64_t sms) { return split > 1 ? units * split : units < sms ? units : sms; }
 
-// What a launch is estimated by, in SM cycles: with tiles 128 and 64 wide, a k-block of `kblock`, storing a tile (hidden but for the
-// last one), what storing a ragged N adds, and what it adds to a meeting of shares, divided among them; set-up and first loads, and
-// the meeting itself.
+// What a launch is estimated by, in SM cycles: with tiles 128 and 64 wide, a k-block of `kblock`, storing a tile beside the next one's
+// k-blocks and what a ragged N adds to that, the same for the last tile of a CTA, and what a ragged N adds to a meeting of shares,
+// divided among them; set-up and first loads, and the meeting itself.
 struct ConvCosts {
     uint32_t kblock;
-    double kb[2], store[2], ragged[2], ragged_shares[2], around, meet;
+    double kb[2], store[2], ragged[2], last[2], ragged_last[2], ragged_shares[2], around, meet;
 };
-// The conversion kernel, fitted to whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.31 us with 128 x 64 ones (0.34 - 0.37
-// with a long k), storing a tile 2.7 and 1.5 us, 3.5 us of set-up and first loads, 2 - 3 us for the shares' sums to meet; where a
-// ragged N is stored word by word 1.5 us more, and 6 us divided among the shares.
-constexpr ConvCosts kConvCosts = {32, {1050.0, 600.0}, {5000.0, 2800.0}, {3000.0, 1500.0}, {11000.0, 5500.0}, 6500.0, 5500.0};
+// The conversion kernel, fitted to whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.33 us with 128 x 64 ones (0.34 - 0.37
+// with a long k), storing a tile 2.7 and 1.5 us (the last wide one 1.2, by twice the warps), 3.5 us of set-up and first loads, 2 - 3 us
+// for the shares' sums to meet; where a ragged N is stored word by word 1.5 us more, and 6 us divided among the shares.
+constexpr ConvCosts kConvCosts = {32, {1050.0, 630.0}, {5000.0, 2800.0}, {3000.0, 1500.0}, {2000.0, 2800.0}, {2000.0, 1500.0}, {11000.0, 5500.0}, 6500.0, 5500.0};
 
 // Estimated SM cycles of one launch for one or two products (the one with the longer k first) on `sms` SMs.  clusters(bn, split):
 // clusters of `split` CTAs that run at once, below one if there are none.
@@ -50,7 +50,7 @@ ConvPlan conv_plan(const ConvShape* sh, int n, uint64_t sms, Clusters clusters, 
         // whole units: the first CTA's units are one of every sms
         const uint64_t rounds = (all + sms - 1) / sms, rounds0 = units[0] / sms + (units[0] % sms != 0);
         auto unit = [&](int i) { return (double)nkb[i] * kb > store + edge ? (double)nkb[i] * kb : store + edge; };
-        double c = around + store + edge + (double)rounds0 * unit(0) + (double)(rounds - rounds0) * unit(1);
+        double c = around + cost.last[w] + (ragged ? cost.ragged_last[w] : 0.0) + (double)rounds0 * unit(0) + (double)(rounds - rounds0) * unit(1);
         if (best.cycles == 0.0 || c < best.cycles) best = ConvPlan{bn, 1, c};
         for (uint32_t split = 2; split <= 8 && split * 2 <= min_kb && all * split <= 2 * sms; ++split) {
             const int fit = clusters(bn, split);

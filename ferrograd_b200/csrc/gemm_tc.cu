@@ -1578,8 +1578,10 @@ __device__ __forceinline__ void store_colsum(const Epilogue& ep, uint32_t row0, 
 }
 
 // Units are walked persistently (unit, unit + CTAs, ...): the ring of loads, the conversion and the MMAs run across units, so
-// that a tile is stored while the next one is computed.  With K-shares a cluster of `split` CTAs takes one unit, a share each,
-// and the shares' sums meet through distributed shared memory: every CTA stores every split-th 32 x 32 block of the tile.
+// that a tile is stored while the next one is computed; a CTA's last wide tile is stored by the converters, who have nothing else left
+// to do and are twice as many (1024 x 256 x 2048 with bias 10.4 -> 10.0 us, with GELU 13.0 -> 11.0, 1000 x 256 x 2001 with GELU 23.8 ->
+// 16.8; gradients of 1000 x 777 x 1001 39.8 -> 34.7).  With K-shares a cluster of `split` CTAs takes one unit, a share each, and the shares'
+// sums meet through distributed shared memory: every CTA stores every split-th 32 x 32 block of the tile.
 template <int BN, bool TWO, bool SHARES>
 __global__ void __launch_bounds__(ConvCfg<BN>::kThreads, 1)
 gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
@@ -1625,6 +1627,9 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         a = ep_of(p, [](const Epilogue& e) { return e.a_mn != 0; });
         b = ep_of(p, [](const Epilogue& e) { return e.b_mn != 0; });
     };
+    // Do the converters store a CTA's last tile?  (Of narrow tiles, half as long to store, it slowed the others down: gradients of
+    // 16 x 384 x 512 x 320 29.7 -> 31.0 us.)
+    constexpr bool kHandOn = !SHARES && BN == 128;
     // Chunks of 128 k, half of the other kernels': fewer additions in the tensor core's truncating accumulator, as K-shares of that
     // length had, and the epilogue warps have the time (a tile's drain takes a tenth of its four k-blocks).
     constexpr uint32_t kChunkKB = 128 / BK;
@@ -1644,12 +1649,64 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
     // Everything up to here needs nothing of the kernels before this one: it passes while the last of them drains.
     fg_grid_enter();
     __shared__ int s_abort;      // see gemm_tc_kernel; the CTAs of a cluster stay together to the end, whatever they have read
-    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(ca.dev_status);
+    __shared__ int s_tail;       // the last tile's sums are in the stages
+    if (threadIdx.x == 0) {
+        s_abort = *reinterpret_cast<volatile int*>(ca.dev_status);
+        s_tail = 0;
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const bool go = __all_sync(0xffffffffu, s_abort == 0);
+
+    // A warp stores 32 columns of up to 32 rows of whole sums, which lie in shared memory in float4s: at(row, float4 of the row).
+    auto store_rows = [&](const Epilogue& ep, size_t cb, uint32_t row0, uint32_t col0, float bias, uint32_t rows, auto at) {
+        const uint32_t rsub = lane >> 3, cc = lane & 7;
+        const ConvStore st(ep, col0 + cc * 4);
+        if (!st.vec) {
+            // Rows that do not start on 16 bytes: a lane per column, a row of 128 bytes per step (four single words per lane
+            // and step, 16 bytes apart between lanes, took 11000 cycles for a 128 x 128 tile: backward of 1000 x 777 x 1001 51.0 -> 40.9 us).
+            const uint32_t c = col0 + lane;
+            if (c >= ep.N) rows = 0;
+            size_t off = cb + (size_t)row0 * ep.N + c;
+            float cs[4] = {0.f, 0.f, 0.f, 0.f};      // row r in chain r % 4, as the lanes below have it
+#pragma unroll 4
+            for (uint32_t r = 0; r < 32; ++r, off += ep.N) {
+                if (r >= rows) continue;
+                const float z = reinterpret_cast<const float*>(at(r, (uint32_t)lane >> 2))[lane & 3] + bias;
+                const float o = st.kind == 2 ? z * fg_act_grad_fast(st.act, ep.mul_saved[off]) : st.kind == 1 ? fg_act_fwd_sel(st.act, z) : z;
+                if (ep.preact) ep.preact[off] = z;
+                ep.C[off] = o;
+                if (ep.c_pairs) fg_store_pairs1(ep.c_pairs, ep.c_pairs_stride, off, o);
+                cs[r & 3] += o;
+            }
+            if (ep.colsum_part && rows) ep.colsum_part[(size_t)(row0 >> 5) * ep.N + c] = (cs[0] + cs[1]) + (cs[2] + cs[3]);
+            __syncwarp();
+            return;
+        }
+        const float4 bz = make_float4(__shfl_sync(0xffffffffu, bias, cc * 4), __shfl_sync(0xffffffffu, bias, cc * 4 + 1),
+                                      __shfl_sync(0xffffffffu, bias, cc * 4 + 2), __shfl_sync(0xffffffffu, bias, cc * 4 + 3));
+        float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
+        size_t off = cb + (size_t)(row0 + rsub) * ep.N + st.col;
+        const uint32_t mine = st.live && rsub < rows ? (rows - rsub + 3) / 4 : 0u;      // this lane's, of eight
+        auto sum_at = [&](uint32_t i) { return add4(*reinterpret_cast<const float4*>(at(i * 4 + rsub, cc)), bz); };
+        if (st.plain) {
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
+                if (i < mine) cs = add4(cs, st.put_plain(ep, off, sum_at(i)));
+        } else {
+#pragma unroll 2
+            for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
+                if (i < mine) cs = add4(cs, st.put_vec(ep, off, sum_at(i)));
+        }
+        __syncwarp();
+        if (ep.colsum_part) {
+            cs = sum_column_lanes(cs);
+            if (lane < 8 && rows) store_colsum(ep, row0, st.col, cs);
+        }
+        __syncwarp();
+    };
 
     if (warp < Cfg::kEpi0) {
         reg_release<Cfg::kRegsLow>();
@@ -1771,6 +1828,22 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                 if (lane == 0) mbar_arrive(conv_bar(s));
             }
         }
+        if constexpr (kHandOn) {
+            // The CTA's last tile, from the stages' room: a warp takes a block of 32 x 32.
+            const Unit t = unit_at(first + (ca.units - 1 - first) / step * step);
+            const uint32_t lr0 = (uint32_t)(warp - Cfg::kConv0) / (BN / 32) * 32, cb = (uint32_t)(warp - Cfg::kConv0) % (BN / 32);
+            auto store = [&](const Epilogue& ep) {
+                const uint32_t row0 = t.m0 + lr0, col0 = t.n0 + cb * 32;
+                const float bias = ep.bias && col0 + lane < ep.N ? ep.bias[col0 + lane] : 0.0f;
+                __syncwarp();
+                asm volatile("bar.sync 2, 768;" ::: "memory");      // the sums are there
+                if (s_tail && row0 < ep.M)
+                    store_rows(ep, (size_t)t.bz * ep.c_batch, row0, col0, bias, min(32u, ep.M - row0),
+                               [&](uint32_t r, uint32_t c) { return base_ptr + (((lr0 + r) * (BN / 4) + ((cb * 8 + c) ^ (r & 7))) << 4); });
+            };
+            if (!TWO || t.p == 0) store(ca.ep[0]);
+            else store(ca.ep[1]);
+        }
         if constexpr (SHARES) {
             __syncwarp();
             cluster_sync_all();      // every share's sums are in its CTA's shared memory
@@ -1831,62 +1904,13 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         bool ok = go;
         uint32_t gc = 0;
         float4* const tb4 = reinterpret_cast<float4*>(base_ptr + S * Cfg::kStageBytes) + (warp - Cfg::kEpi0) * (32 * 8);
-        const uint32_t rsub = lane >> 3, cc = lane & 7;
-        // A 32 x 32 block of whole sums, swizzled in tb4 (float4 c of row r at c ^ (r & 7)): four rows of 128 bytes per step.
-        auto store_block = [&](const Epilogue& ep, size_t cb, uint32_t row0, uint32_t col0, float bias) {
-            const ConvStore st(ep, col0 + cc * 4);
-            if (!st.vec) {
-                // Rows that do not start on 16 bytes: a lane per column, a row of 128 bytes per step (four single words per lane
-                // and step, 16 bytes apart between lanes, took 11000 cycles for a 128 x 128 tile: backward of 1000 x 777 x 1001 51.0 -> 40.9 us).
-                const uint32_t c = col0 + lane, rows = c < ep.N && row0 < ep.M ? min(32u, ep.M - row0) : 0u;
-                const float* const tb = reinterpret_cast<const float*>(tb4);
-                size_t off = cb + (size_t)row0 * ep.N + c;
-                float cs[4] = {0.f, 0.f, 0.f, 0.f};      // row r in chain r % 4, as the lanes below have it
-#pragma unroll 4
-                for (uint32_t r = 0; r < 32; ++r, off += ep.N) {
-                    if (r >= rows) continue;
-                    const float z = tb[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)] + bias;
-                    const float o = st.kind == 2 ? z * fg_act_grad_fast(st.act, ep.mul_saved[off]) : st.kind == 1 ? fg_act_fwd_sel(st.act, z) : z;
-                    if (ep.preact) ep.preact[off] = z;
-                    ep.C[off] = o;
-                    if (ep.c_pairs) fg_store_pairs1(ep.c_pairs, ep.c_pairs_stride, off, o);
-                    cs[r & 3] += o;
-                }
-                if (ep.colsum_part && rows) ep.colsum_part[(size_t)(row0 >> 5) * ep.N + c] = (cs[0] + cs[1]) + (cs[2] + cs[3]);
-                __syncwarp();
-                return;
-            }
-            const float4 bz = make_float4(__shfl_sync(0xffffffffu, bias, cc * 4), __shfl_sync(0xffffffffu, bias, cc * 4 + 1),
-                                          __shfl_sync(0xffffffffu, bias, cc * 4 + 2), __shfl_sync(0xffffffffu, bias, cc * 4 + 3));
-            float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
-            size_t off = cb + (size_t)(row0 + rsub) * ep.N + st.col;
-            const uint32_t rows = st.live && row0 + rsub < ep.M ? (ep.M - row0 - rsub + 3) / 4 : 0u;      // this lane's, of eight
-            auto sum_at = [&](uint32_t i) {
-                const uint32_t lr = i * 4 + rsub;
-                return add4(tb4[lr * 8 + (cc ^ (lr & 7))], bz);
-            };
-            if (st.plain) {
-#pragma unroll
-                for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
-                    if (i < rows) cs = add4(cs, st.put_plain(ep, off, sum_at(i)));
-            } else {
-#pragma unroll 2
-                for (uint32_t i = 0; i < 8; ++i, off += (size_t)4 * ep.N)
-                    if (i < rows) cs = add4(cs, st.put_vec(ep, off, sum_at(i)));
-            }
-            __syncwarp();
-            if (ep.colsum_part) {
-                cs = sum_column_lanes(cs);
-                if (lane < 8 && row0 < ep.M) store_colsum(ep, row0, st.col, cs);
-            }
-            __syncwarp();
-        };
         for (uint32_t u = first; u < ca.units && ok; u += step) {
             const Unit t = unit_at(u);
             const uint32_t nchunks = (t.nkb + kChunkKB - 1) / kChunkKB;
             // a lane holds the bias of one column per block: it is here long before the sums are
             float bias[CPT / 32];
-            if constexpr (!SHARES) {
+            const bool last = SHARES || (kHandOn && u + step >= ca.units);
+            if (!last) {
                 const float* const bp = ep_of(t.p, [](const Epilogue& e) { return e.bias; });
                 const uint32_t N = ep_of(t.p, [](const Epilogue& e) { return e.N; });
 #pragma unroll
@@ -1922,13 +1946,14 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                 if (lane == 0) mbar_arrive(acc_empty_bar(buf));
             }
             if (!ok) break;
-            if constexpr (SHARES) {
-                // Every load and MMA of this CTA has finished (its last chunk is complete), so the stages are free: the share's
-                // sums as [row][BN], float4 c of a row at c ^ (row & 7).
+            if (last) {
+                // Every load and MMA of this CTA has finished (its last chunk is complete), so the stages are free: the tile's or
+                // the share's sums as [row][BN], float4 c of a row at c ^ (row & 7).
                 float4* const part = reinterpret_cast<float4*>(base_ptr) + (q * 32 + lane) * (BN / 4);
 #pragma unroll
                 for (int c = 0; c < CPT / 4; ++c)
                     part[(half * (CPT / 4) + c) ^ (lane & 7)] = make_float4(sum[4 * c], sum[4 * c + 1], sum[4 * c + 2], sum[4 * c + 3]);
+                if (kHandOn && threadIdx.x == Cfg::kEpi0 * 32) s_tail = 1;
             } else {
 #pragma unroll 1
                 for (int gr = 0; gr < CPT / 32; ++gr) {
@@ -1941,12 +1966,17 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                     __syncwarp();
                     const uint32_t row0 = t.m0 + q * 32, col0 = t.n0 + half * CPT + gr * 32;
                     const float bv = CPT > 32 && gr ? bias[CPT / 32 - 1] : bias[0];
-                    if (!TWO || t.p == 0) store_block(ca.ep[0], (size_t)t.bz * ca.ep[0].c_batch, row0, col0, bv);
-                    else store_block(ca.ep[1], (size_t)t.bz * ca.ep[1].c_batch, row0, col0, bv);
+                    auto store = [&](const Epilogue& ep) {
+                        store_rows(ep, (size_t)t.bz * ep.c_batch, row0, col0, bv, row0 < ep.M ? min(32u, ep.M - row0) : 0u,
+                                   [&](uint32_t r, uint32_t c) { return reinterpret_cast<const unsigned char*>(tb4 + r * 8 + (c ^ (r & 7))); });
+                    };
+                    if (!TWO || t.p == 0) store(ca.ep[0]);
+                    else store(ca.ep[1]);
                 }
             }
         }
         if constexpr (SHARES) { __syncwarp(); cluster_sync_all(); cluster_sync_all(); }      // as the converters
+        if constexpr (kHandOn) { __syncwarp(); asm volatile("bar.sync 2, 768;" ::: "memory"); }      // the converters store the last tile
     }
     tc_fence_before();
     __syncthreads();
@@ -2692,7 +2722,7 @@ int32_t launch_conv_both(fg_ctx* ctx, const ConvProduct& dB, const ConvProduct& 
 
 // ---- the same for sixteen-bit tensors ----
 // Costs fitted to 87 products under the pair kernel and every plan (2 % slower than the best of each in the geometric mean).
-constexpr ConvCosts kHalfCosts = {64, {520.0, 305.0}, {600.0, 300.0}, {950.0, 1250.0}, {800.0, 650.0}, 2400.0, 1600.0};
+constexpr ConvCosts kHalfCosts = {64, {520.0, 305.0}, {600.0, 300.0}, {950.0, 1250.0}, {600.0, 300.0}, {950.0, 1250.0}, {800.0, 650.0}, 2400.0, 1600.0};
 template <int BN, bool TWO, bool SHARES>
 cudaError_t half_attr(const fg_ctx* ctx) {
     static std::atomic<uint64_t> done{0};
