@@ -1538,12 +1538,6 @@ struct ConvStore {
         *reinterpret_cast<float4*>(ep.C + off) = z;
         return z;
     }
-    __device__ __forceinline__ float4 put(const Epilogue& ep, size_t off, float4 z) const {
-        if (!vec)
-            return epi_store_edge(z, off, col, ep.N, (char*)ep.C, (char*)ep.preact, ep.c_pairs, ep.c_pairs_stride, ep.mul_saved, ep.mul_act,
-                                  ep.act, FG_DTYPE_F32);
-        return put_vec(ep, off, z);
-    }
     __device__ __forceinline__ float4 put_vec(const Epilogue& ep, size_t off, float4 z) const {
         float4 o = z;
         if (kind == 1) {
@@ -1852,7 +1846,7 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                 // one, a lane four columns of a row.
                 const Unit t = unit_at(first);
                 const uint32_t rsub = lane >> 3, cc = lane & 7;
-                auto fold = [&](const Epilogue& ep) {
+                auto fold = [&](const Epilogue& ep, auto ragged) {
                     float4* const csum = reinterpret_cast<float4*>(base_ptr + S * Cfg::kStageBytes);      // [block][eight times four rows][8 lanes]
                     for (uint32_t v = warp - Cfg::kConv0, b; (b = share + split * (v >> 3)) < 4 * (BN / 32); v += 16) {
                         const uint32_t lr = (b & 3u) * 32 + (v & 7u) * 4 + rsub, c0 = (b >> 2) * 32, row = t.m0 + lr;
@@ -1868,11 +1862,34 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
 #pragma unroll
                         for (uint32_t r = 1; r < 8; ++r)        // in the order of the shares, whoever adds them
                             if (r < split) z[0] = add4(z[0], z[r]);
+                        if constexpr (decltype(ragged)::value) {
+                            const float4 w = add4(z[0], make_float4(bz[0], bz[1], bz[2], bz[3]));
+                            // Rows that do not start on 16 bytes: a lane per column, one of the four rows per step, as in store_rows.
+                            const uint32_t c = t.n0 + c0 + lane, r0 = t.m0 + (b & 3u) * 32 + (v & 7u) * 4;
+                            size_t off = (size_t)t.bz * ep.c_batch + (size_t)r0 * ep.N + c;
+                            float o[4];
+#pragma unroll
+                            for (uint32_t i = 0; i < 4; ++i, off += ep.N) {
+                                const int from = (int)(i * 8 + (lane >> 2));
+                                const float x0 = __shfl_sync(0xffffffffu, w.x, from), x1 = __shfl_sync(0xffffffffu, w.y, from);
+                                const float x2 = __shfl_sync(0xffffffffu, w.z, from), x3 = __shfl_sync(0xffffffffu, w.w, from);
+                                const float x = lane & 2 ? (lane & 1 ? x3 : x2) : (lane & 1 ? x1 : x0);
+                                o[i] = 0.0f;
+                                if (c >= ep.N || r0 + i >= ep.M) continue;
+                                o[i] = st.kind == 2 ? x * fg_act_grad_fast(st.act, ep.mul_saved[off]) : st.kind == 1 ? fg_act_fwd_sel(st.act, x) : x;
+                                if (ep.preact) ep.preact[off] = x;
+                                ep.C[off] = o[i];
+                                if (ep.c_pairs) fg_store_pairs1(ep.c_pairs, ep.c_pairs_stride, off, o[i]);
+                            }
+                            if (ep.colsum_part) reinterpret_cast<float*>(csum)[v * 32 + lane] = (o[0] + o[1]) + (o[2] + o[3]);
+                            __syncwarp();
+                            continue;
+                        }
                         float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (st.live && row < ep.M) {
                             const size_t off = (size_t)t.bz * ep.c_batch + (size_t)row * ep.N + st.col;
                             const float4 w = add4(z[0], make_float4(bz[0], bz[1], bz[2], bz[3]));
-                            cs = st.plain ? st.put_plain(ep, off, w) : st.put(ep, off, w);
+                            cs = st.plain ? st.put_plain(ep, off, w) : st.put_vec(ep, off, w);
                         }
                         __syncwarp();
                         if (ep.colsum_part) {
@@ -1891,8 +1908,12 @@ gemm_tc_conv_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                         }
                     }
                 };
-                if (!TWO || t.p == 0) fold(ca.ep[0]);
-                else fold(ca.ep[1]);
+                auto fold_of = [&](const Epilogue& ep) {
+                    if (ConvStore(ep, 0).vec) fold(ep, std::false_type{});
+                    else fold(ep, std::true_type{});
+                };
+                if (!TWO || t.p == 0) fold_of(ca.ep[0]);
+                else fold_of(ca.ep[1]);
             }
             __syncwarp();
             cluster_sync_all();      // no CTA leaves while another reads its sums
