@@ -446,7 +446,8 @@ struct FmaPlan { int tile[2]; uint32_t lg_split; float cycles; };
 // the geometric mean, 22 % at most): a stage takes a CTA no less than its copies' latency (270), the ends of a unit 1430, a meeting of
 // shares 180 + 150 each, and three CTAs share an SM.  A word that is copied alone and one that is added to a column's sum take 0.05 more:
 // with that, the gradients of 28 layers, 13 of them with odd rows, take 7 % more than under the best plan of each in the geometric mean
-// and 12 % without (2000 x 100 x 30: 17.7 and 23.1 us).  (The host spends this on every call: shifts, no division.)
+// and 12 % without (2000 x 100 x 30: 17.7 and 23.1 us); not with 16 columns or fewer, where most of a row's words are only zeroed
+// (gradients of 1000 x 100 x 4 9.1 us with it, 7.6 without, 300 x 200 x 13 7.0 and 6.1, 500 x 300 x 10 8.1 and 8.9).  (The host spends this on every call: shifts, no division.)
 FmaPlan fma_plan(const fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch) {
     FmaPlan best{{0, 0}, 0, 0.0f};
     const float sms = (float)fg_free_sms(ctx), per_round = 1.0f / (3.0f * sms), per_sm = 0.4f / sms;
@@ -458,8 +459,9 @@ FmaPlan fma_plan(const fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch) {
         for (int j = 0; j < n; ++j) {
             const float cols = (float)((ops[j].N + kTN - 1) / kTN) * batch * (float)(1u << lg);
             const FmaRows rows = fma_rows(ops[j], batch);
-            const float by_a = rows.a16 ? 0.0f : ops[j].factor && !ops[j].ta ? 0.1f : 0.05f;
-            const float by_b = (rows.b16 ? 0.0f : ops[j].factor && ops[j].ta ? 0.1f : 0.05f) + (ops[j].colsum_b ? 0.05f : 0.0f);
+            const bool narrow = ops[j].N <= 16 || ops[j].K <= 16;
+            const float by_a = rows.a16 || narrow ? 0.0f : ops[j].factor && !ops[j].ta ? 0.1f : 0.05f;
+            const float by_b = (rows.b16 || narrow ? 0.0f : ops[j].factor && ops[j].ta ? 0.1f : 0.05f) + (ops[j].colsum_b && !narrow ? 0.05f : 0.0f);
             for (int i = 0; i < 4; ++i) {
                 const FmaTile& t = kTiles[i];
                 const float more = (by_a * (float)(1u << t.lg_tm) + by_b * kTN) * (float)(1u << t.lg_tk);
