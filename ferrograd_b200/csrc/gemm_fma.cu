@@ -447,7 +447,8 @@ struct FmaPlan { int tile[2]; uint32_t lg_split; float cycles; };
 // shares 180 + 150 each, and three CTAs share an SM.  A word that is copied alone and one that is added to a column's sum take 0.05 more:
 // with that, the gradients of 28 layers, 13 of them with odd rows, take 7 % more than under the best plan of each in the geometric mean
 // and 12 % without (2000 x 100 x 30: 17.7 and 23.1 us); not with 16 columns or fewer, where most of a row's words are only zeroed
-// (gradients of 1000 x 100 x 4 9.1 us with it, 7.6 without, 300 x 200 x 13 7.0 and 6.1, 500 x 300 x 10 8.1 and 8.9).  (The host spends this on every call: shifts, no division.)
+// (gradients of 1000 x 100 x 4 9.1 us with it, 7.6 without, 300 x 200 x 13 7.0 and 6.1, 500 x 300 x 10 8.1 and 8.9; by the narrow
+// layer's own kernels 25, 12.3 and 17.4).  (The host spends this on every call: shifts, no division.)
 FmaPlan fma_plan(const fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch) {
     FmaPlan best{{0, 0}, 0, 0.0f};
     const float sms = (float)fg_free_sms(ctx), per_round = 1.0f / (3.0f * sms), per_sm = 0.4f / sms;
