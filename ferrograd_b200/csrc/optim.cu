@@ -242,11 +242,15 @@ int32_t update_multi(fg_ctx* ctx, bool adam, const fg_update_tensor* t, uint32_t
     return FG_OK;
 }
 
+// A beta of one divides by zero in the bias correction: 1 / (1 - beta^t).
+bool betas_ok(const fg_adamw_hyper& h) { return h.beta1 >= 0.f && h.beta1 < 1.f && h.beta2 >= 0.f && h.beta2 < 1.f; }
+
 }  // namespace
 
 // The update of step *counter + 1; `count`: counter is that step afterwards.
 int32_t fg_adamw_next_step(fg_ctx* ctx, const fg_update_tensor* tensors, uint32_t n, const fg_adamw_hyper* h, uint32_t* counter, bool count) {
     FG_ENTER(ctx);
+    FG_REQUIRE(ctx, n == 0 || betas_ok(*h), "AdamW update: betas must lie in [0,1)");
     uint64_t total = 0;
     for (uint32_t k = 0; k < n; ++k) total += tensors[k].n;
     if (total == 0) return count ? fg_counter_increment(ctx, counter) : FG_OK;
@@ -262,8 +266,7 @@ int32_t fg_adamw_step_multi(fg_ctx* ctx, const fg_update_tensor* tensors, uint32
     FG_ENTER(ctx);
     FG_REQUIRE(ctx, (tensors || count == 0) && h, "fg_adamw_step_multi: NULL pointer");
     FG_REQUIRE(ctx, step_dev != nullptr || step >= 1, "fg_adamw_step_multi: step is 1-based");
-    FG_REQUIRE(ctx, h->beta1 >= 0.f && h->beta1 < 1.f && h->beta2 >= 0.f && h->beta2 < 1.f,
-               "fg_adamw_step_multi: betas must lie in [0,1)");
+    FG_REQUIRE(ctx, betas_ok(*h), "fg_adamw_step_multi: betas must lie in [0,1)");
     return update_multi(ctx, true, tensors, count, AdamConsts{h->lr, h->beta1, h->beta2, h->eps, h->weight_decay, grad_scale},
                         StepSource{step, step_dev, 0, nullptr, nullptr}, zero_grad, "fg_adamw_step_multi: a tensor is NULL, misaligned, or its pairs do not cover it");
 }
@@ -305,8 +308,7 @@ int32_t fg_adamw_step_paired(fg_ctx* ctx, float* w, float* g, float* m, float* v
     FG_REQUIRE(ctx, fg_aligned16(w) && fg_aligned16(g) && fg_aligned16(m) && fg_aligned16(v),
                "fg_adamw_step: pointers must be 16-byte aligned");
     FG_REQUIRE(ctx, step_dev != nullptr || step >= 1, "fg_adamw_step: step is 1-based");
-    FG_REQUIRE(ctx, h->beta1 >= 0.f && h->beta1 < 1.f && h->beta2 >= 0.f && h->beta2 < 1.f,
-               "fg_adamw_step: betas must lie in [0,1)");
+    FG_REQUIRE(ctx, betas_ok(*h), "fg_adamw_step: betas must lie in [0,1)");
     FG_REQUIRE(ctx, !w_pairs || (fg_aligned16(w_pairs) && pairs_stride % 8 == 0 && pairs_stride >= n),
                "fg_adamw_step_paired: pairs must be 16-byte aligned with a plane stride that is a multiple of 8 and at least n");
     if (n == 0) return FG_OK;

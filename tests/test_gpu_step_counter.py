@@ -49,3 +49,42 @@ def test_every_dispatch_is_one_step(oracle, tensors, plans):
             assert ok, f"tensor {k} after step {step}: {worst:.3g}"
     t.destroy()
     ctx.destroy()
+
+
+# A beta outside [0, 1) has no bias correction: the update is refused, before a weight, a moment or the counter changes, by plain launches
+# and by recorded ones (whose first dispatch is eager).  With the betas mended the same gradients make step one.
+@pytest.mark.parametrize("beta1,beta2", [(1.0, 0.999), (0.9, 1.0), (-0.1, 0.999), (0.9, float("nan"))])
+@pytest.mark.parametrize("plans", ["0", "1"])
+def test_betas_out_of_range_are_refused(oracle, beta1, beta2, plans):
+    import ctypes as C
+
+    from ferrograd_b200 import FgError, GpuContext, _lib
+    from ferrograd_b200.mlp import GraphMLP
+    ctx = GpuContext(0)
+    ctx.set_option("exec_plans", plans)
+    dims, batch, lr = [4, 8, 2], 16, 1e-2
+    r = np.random.Generator(np.random.Philox(3))
+    net = GraphMLP(ctx, dims, batch, "tanh", "mse", ("adamw", lr, beta1, beta2, 1e-8, 0.01))
+    W = [r.standard_normal((a, b), np.float32) for a, b in zip(dims, dims[1:])]
+    net.set_params(W, [np.zeros(d, np.float32) for d in dims[1:]])
+    net.upload_batch(r.standard_normal((batch, dims[0]), np.float32), r.standard_normal((batch, dims[-1]), np.float32))
+    ctx.dispatch_forward(net.schedule)
+    ctx.dispatch_loss(net.schedule, net.target)
+    ctx.dispatch_backward(net.schedule)
+    for call in (lambda: ctx.dispatch_optim(net.schedule), lambda: ctx.dispatch_optim(net.schedule),
+                 lambda: ctx.dispatch_single_optim(net.schedule, net.W[0], 0)):
+        with pytest.raises(FgError) as e:
+            call()
+        assert e.value.kind == "FG_ERR_INVALID_ARGUMENT"
+        assert all(np.array_equal(a, b) for a, b in zip(net.get_params()[0], W))
+    grads = {node: ctx.download(net.tensors.grad_tensors[i], np.empty(W[0].shape, np.float32))
+             for i, node in enumerate(net.tensors.grad_nodes) if node == 1}      # (node 0 is the batch, 1 the first weights)
+    good = _lib.AdamWHyper(lr, 0.9, 0.999, 1e-8, 0.01)
+    ctx._check(ctx.lib.fg_exec_set_adamw(net.tensors.handle, C.byref(good)))
+    ctx.dispatch_optim(net.schedule)
+    ref, m, v = W[0].copy(), np.zeros_like(W[0]), np.zeros_like(W[0])
+    oracle.adamw(ref, np.ascontiguousarray(grads[1]), m, v, lr, 0.9, 0.999, 1e-8, 0.01, 1)
+    ok, worst = rel_err_ok(net.get_params()[0][0], ref, 1e-6)      # (as above)
+    assert ok, f"{worst:.3g}"
+    net.tensors.destroy()
+    ctx.destroy()
