@@ -274,6 +274,15 @@ int32_t fg_ctx_destroy(fg_ctx* ctx) {
     return FG_OK;
 }
 
+// Reads the device error word of a context whose stream is idle.  When a wait has run out, the word is cleared together with the arrival
+// counters behind it: the blocks that gave up may not have counted themselves (see fg_last_block), and a counter that starts off zero
+// lets every later launch that uses it add before all parts are there.  On the context's stream, before whatever it launches next.
+static int32_t take_status(fg_ctx* ctx, int* status) {
+    FG_CUDA(ctx, FG_ERR_SYNC, cudaMemcpy(status, ctx->dev_status, sizeof(int), cudaMemcpyDeviceToHost));
+    if (*status) FG_CUDA(ctx, FG_ERR_SYNC, cudaMemsetAsync(ctx->dev_status, 0, kFgStatusBytes, ctx->stream));
+    return FG_OK;
+}
+
 int32_t fg_sync(fg_ctx* ctx) {
     if (!ctx) return FG_ERR_NOT_INITIALIZED;
     FG_CUDA(ctx, FG_ERR_INVALID_DEVICE, cudaSetDevice(ctx->device));
@@ -281,9 +290,9 @@ int32_t fg_sync(fg_ctx* ctx) {
     FG_CUDA(ctx, FG_ERR_SYNC, cudaStreamSynchronize(ctx->copy_stream));
     FG_CUDA(ctx, FG_ERR_SYNC, cudaStreamSynchronize(ctx->stream));
     int status = 0;
-    FG_CUDA(ctx, FG_ERR_SYNC, cudaMemcpy(&status, ctx->dev_status, sizeof(int), cudaMemcpyDeviceToHost));
+    const int32_t s = take_status(ctx, &status);
+    if (s != FG_OK) return s;
     if (status != 0) {
-        cudaMemset(ctx->dev_status, 0, sizeof(int));
         snprintf(ctx->err, sizeof(ctx->err), "a bounded device-side wait expired (status word 0x%x)", status);
         return FG_ERR_TIMEOUT;
     }
@@ -295,8 +304,8 @@ int32_t fg_ctx_device_status(fg_ctx* ctx, int32_t* status_word) {
     FG_CUDA(ctx, FG_ERR_INVALID_DEVICE, cudaSetDevice(ctx->device));
     FG_CUDA(ctx, FG_ERR_SYNC, cudaStreamSynchronize(ctx->stream));
     int status = 0;
-    FG_CUDA(ctx, FG_ERR_SYNC, cudaMemcpy(&status, ctx->dev_status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (status) cudaMemset(ctx->dev_status, 0, sizeof(int));
+    const int32_t s = take_status(ctx, &status);
+    if (s != FG_OK) return s;
     *status_word = status;
     return FG_OK;
 }

@@ -4053,9 +4053,10 @@ int32_t fg_gemm_bwd_lowp(fg_ctx* ctx, int32_t dtype, uint32_t M, uint32_t N, uin
 
 // ---- self-test of the bounded waits ----
 namespace {
-__global__ void bounded_wait_selftest_kernel(int* dev_status, long long max_cycles) {
+__global__ void bounded_wait_selftest_kernel(int* dev_status, unsigned* arrivals, long long max_cycles) {
     __shared__ unsigned long long bar;
     if (threadIdx.x == 0) {
+        atomicInc(arrivals, 1u);      // the first of two blocks of which the other gives up uncounted
         mbar_init(smem_u32(&bar), 1);
         fence_mbar_init();
         // nobody arrives on this barrier: the wait must give up after max_cycles and report it
@@ -4067,7 +4068,7 @@ __global__ void bounded_wait_selftest_kernel(int* dev_status, long long max_cycl
 extern "C" int32_t fg_selftest_bounded_wait(fg_ctx* ctx, uint32_t max_cycles) {
     FG_ENTER(ctx);
     const long long limit = max_cycles > 1000000u ? 1000000ll : (long long)max_cycles;
-    bounded_wait_selftest_kernel<<<1, 32, 0, ctx->stream>>>(ctx->dev_status, limit);
+    bounded_wait_selftest_kernel<<<1, 32, 0, ctx->stream>>>(ctx->dev_status, fg_arrivals(ctx), limit);
     FG_LAUNCHED(ctx);
     return FG_OK;
 }

@@ -309,6 +309,8 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
             if (tid == 0) atomicOr(dev_status, FG_DEVERR_TMA_WAIT);
             // give the copies in flight a bounded chance to land before the CTA retires
             if (!ok) mbar_wait_bounded(bar, parity ^ 1u);
+            // counted like the others, so that the counter wraps to zero; no mean is left here
+            if (MODE == 1 && a.mean && tid == 0) atomicInc(a.arrivals, gridDim.x - 1);
             return;
         }
         float4 v[kRowNV];

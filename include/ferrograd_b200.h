@@ -114,9 +114,10 @@ int32_t fg_ctx_set_option(fg_ctx* ctx, const char* name, const char* value);
 /* Self-test of the bounded device-side waits (no counterpart in the reference).  Launches one tiny kernel that
  * waits, for at most max_cycles SM clock cycles (clamped to 1,000,000), on an mbarrier nobody ever arrives on,
  * with the same wait routine the GEMM kernels use.  The wait runs out, the kernel records it in the device error
- * word and returns: fg_sync then reports FG_ERR_TIMEOUT once and the context stays usable.  Nothing faults or hangs. */
+ * word and returns: fg_sync then reports FG_ERR_TIMEOUT once and the context stays usable.  The kernel also leaves the counter of
+ * arrived blocks at one of two, as a launch does of which a block gave up; it is cleared with the word.  Nothing faults or hangs. */
 int32_t fg_selftest_bounded_wait(fg_ctx* ctx, uint32_t max_cycles);
-/* Reads and clears the device-side error word (bounded waits that expired). */
+/* Reads and clears the device-side error word (bounded waits that expired), and with it the counters of arrived blocks. */
 int32_t fg_ctx_device_status(fg_ctx* ctx, int32_t* status_word);
 
 /* Per-kernel timing for benchmarks (no counterpart in the reference; its examples time

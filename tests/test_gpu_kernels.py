@@ -838,6 +838,24 @@ def test_a_bounded_wait_that_runs_out_is_reported_and_the_context_survives(ctx, 
     assert ctx.device_status() == 0
 
 
+@pytest.mark.parametrize("clear", ["sync", "device_status"])
+def test_block_counters_start_at_zero_after_an_expired_wait(ctx, clear):
+    # the self-test counts one block of two, as a launch whose other block gave up: what is reported and cleared takes the counters along.
+    # The mean of one block's rows is left only by a block that counts itself first and last.
+    from ferrograd_b200 import FgError
+    x, labels = up(ctx, np.zeros((4, 10), np.float32)), ctx.init_tensor_u32((4,), np.zeros(4, np.uint32))
+    loss, mean = ctx.new_tensor((4,)), up(ctx, np.full(1, -1.0, np.float32))
+    ctx._check(ctx.lib.fg_selftest_bounded_wait(ctx.handle, 20000))
+    if clear == "sync":
+        with pytest.raises(FgError):
+            ctx.sync()
+    else:
+        assert ctx.device_status() != 0
+    ctx.softmax_ce(x, labels, 4, 10, loss_row=loss, loss_mean=mean)
+    assert abs(float(ctx.to_numpy(mean)[0]) - np.log(10.0)) < 1e-6
+    assert ctx.device_status() == 0
+
+
 def test_a_plan_recorded_before_the_scratch_arena_moved_is_refused(oracle):
     # A recorded plan carries addresses inside the scratch arena.  A later, larger eager call reallocates the arena;
     # replaying the old plan would touch freed memory, so fg_plan_launch refuses it.
