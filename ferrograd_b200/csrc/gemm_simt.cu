@@ -62,7 +62,8 @@ __device__ __forceinline__ void simt_tile(uint32_t M, uint32_t N, uint32_t K, co
 
     // Two tiles are on their way while one is multiplied (9 x (19 x 335 x 256), forward 9.5 -> 8.9 us, dA 8.7 -> 7.7); one where A is
     // transposed, whose words come in whole lines (dB of 10 x (192 x 48 x 23) 5.0 us, 5.4 with two), and in the large tiles, which
-    // have the work to wait behind.
+    // have the work to wait behind.  Two tiles a turn of the loop, so that the buffers are constants (forward 700 x 500 x 300 in large
+    // tiles 20.4 -> 16.7), but one where A is transposed: dB of 384 x 256 x 200 8.2 us, 11.2 with two, of 1000 x 64 x 1000 19.4 and 27.6.
     constexpr int AHEAD = RPT == 1 && !TA ? 2 : 1;
 #pragma unroll
     for (int d = 0; d < AHEAD; ++d) fetch(d * TK, d);
@@ -96,9 +97,14 @@ __device__ __forceinline__ void simt_tile(uint32_t M, uint32_t N, uint32_t K, co
                 for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
     };
-    for (uint32_t k0 = 0; k0 < K; k0 += 2 * TK) {
-        tile(k0, 0, 0);
-        if (k0 + TK < K) tile(k0 + TK, 1, AHEAD - 1);
+    if constexpr (!TA) {
+        for (uint32_t k0 = 0; k0 < K; k0 += 2 * TK) {
+            tile(k0, 0, 0);
+            if (k0 + TK < K) tile(k0 + TK, 1, AHEAD - 1);
+        }
+    } else {
+        int buf = 0;
+        for (uint32_t k0 = 0; k0 < K; k0 += TK, buf ^= 1) tile(k0, buf, 0);
     }
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
