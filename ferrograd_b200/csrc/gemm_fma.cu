@@ -606,6 +606,19 @@ bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products) {
     return work <= (products != (kFgGradA | kFgGradB) ? 40000000ull : N % 4 ? 24000000ull : 32000000ull);
 }
 
+// A narrow layer's dB is one tile across and a tile per 64 rows of B: its clusters go through all samples, where the narrow layer's own
+// kernels (gemm_skinny_tn_partial_kernel) spread them over the GPU.  Device times of 300 layers, this kernel and those (us): all gradients with the factor of
+// the layer below 1024 x 1 x 1 6.7 / 10.2, 1500 x 10 x 100 13.4 / 16.3, 3072 x 10 x 40 15.1 / 17.8, 4096 x 1 x 1 16.9 / 13.7, 1024 x 4 x 300
+// 13.9 / 13.3, 64 x 4 x 4000 7.5 / 10.1, 128 x 4 x 4000 11.4 / 10.9, 65536 x 4 x 4 285 / 64; the gradients alone 1500 x 1 x 64 8.8 / 9.1,
+// 3072 x 1 x 40 12.6 / 10.4; with an activation's factor on dZ 256 x 4 x 500 7.6 / 11.1, 512 x 4 x 200 10.4 / 10.7, 1024 x 10 x 64
+// 10.0 / 12.2, 1500 x 1 x 40 12.9 / 10.2.
+bool fg_gemm_fma_suits_small(uint32_t M, uint32_t N, uint32_t K, int products) {
+    if (N > 16 || products == kFgForward) return true;
+    const uint64_t mk = (uint64_t)M * K;
+    if (products & kFgFactor) return M <= 1024 && mk <= (M <= 256 ? 250000u : 100000u);
+    return M <= (products & kFgBelow ? 3072u : 2048u) && mk + 55ull * M <= 260000u;
+}
+
 // The backward pass of one layer, see FgFmaBwd.  The caller has reserved room for dZ (M * N floats) and for column sums of dA.
 int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b) {
     const uint64_t mn = (uint64_t)b.M * b.N * 4, mk = (uint64_t)b.M * b.K * 4, kn = (uint64_t)b.K * b.N * 4;

@@ -3036,7 +3036,15 @@ int pick_path(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K) {
 // kernel keeps what those can run.)
 bool takes_fma(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, int products) {
     if (mode != FG_GEMM_AUTO) return false;
-    return pick_path(ctx, mode, M, N, K) == 0 || (conv_allowed(ctx) && !ctx->opt_conv_bn && fg_gemm_fma_suits(M, N, K, products));
+    if (pick_path(ctx, mode, M, N, K) == 0) return fg_gemm_fma_suits_small(M, N, K, products);
+    return (conv_allowed(ctx) && !ctx->opt_conv_bn && fg_gemm_fma_suits(M, N, K, products & (kFgGradB | kFgGradA)));
+}
+// Are a layer's gradients the narrow layer's kernels'?  (Of small products with more rows than the pass over dZ always takes, 65535 tiles
+// of 32, the FMA kernel's after all.)
+bool takes_narrow(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, bool fuse) {
+    if (mode != FG_GEMM_AUTO || N > 16) return false;
+    return pick_path(ctx, mode, M, N, K) != 0 ||
+           (M <= 65535u * 32u && !fg_gemm_fma_suits_small(M, N, K, kFgGradB | kFgGradA | (fuse ? kFgFactor : 0)));
 }
 
 }  // namespace
@@ -3198,7 +3206,8 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
                         const float* dY, int32_t act, const float* saved, float* dA, float* dB, float* dbias,
                         float* dZ_out, float* exch_buf, uint64_t exch_count) {
     const bool fuse = act != FG_ACT_NONE;
-    const int path = pick_path(ctx, mode, M, N, K);
+    const bool skinny = takes_narrow(ctx, mode, M, N, K, fuse);
+    const int path = skinny ? 2 : pick_path(ctx, mode, M, N, K);
     const uint64_t mn = (uint64_t)M * N;
 
     if (path == 0) {
@@ -3238,7 +3247,6 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
     // A skinny layer (N <= 16, say 10 classes): dA is bound by writing it once and dB by reading A once, so
     // both run as plain-FMA kernels on dZ itself; the operand pre-passes and a tensor-core GEMM that could
     // only fill M/128 CTAs would cost several times more.
-    const bool skinny = mode == FG_GEMM_AUTO && N <= 16;
     const bool tc_da = dA && !skinny, tc_db = dB && !skinny;
     uint64_t need = 2048;
     if (tc_da) need += planes_bytes(fmt, M, N) + planes_bytes(fmt, K, N) + kPairPartialBytes;
@@ -3431,7 +3439,8 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
         return FG_OK;
     };
     const bool narrow = N <= 16;
-    if ((dA || dB) && takes_fma(ctx, FG_GEMM_AUTO, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0))) {
+    const int below = dA && (o.mul_saved || dbias_prev) ? kFgBelow : 0;
+    if ((dA || dB) && takes_fma(ctx, FG_GEMM_AUTO, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0) | below)) {
         if (dA && o.mul_saved != dA && (s = saved_apart()) != FG_OK) return s;      // (an element is read and written by one thread)
         FgFmaBwd b{};
         b.M = M; b.N = N; b.K = K; b.A = A.x; b.B = B.x; b.dZ = dZ.x; b.dA = dA; b.dB = dB; b.dbias = dbias;
@@ -3531,7 +3540,9 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, !dB || A, "fg_gemm_bwd_f32: dB needs A");
     const bool fuse = act != FG_ACT_NONE;
     const int path = pick_path(ctx, mode, M, N, K);
-    if (!dZ_out && (path == 0 || dA || dB) && takes_fma(ctx, mode, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0))) {
+    const bool fma = path == 0 ? mode == FG_GEMM_AUTO && !takes_narrow(ctx, mode, M, N, K, fuse)
+                               : (dA || dB) && takes_fma(ctx, mode, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0));
+    if (!dZ_out && fma) {
         int32_t s = fg_ws_ensure(ctx, (uint64_t)M * N * 4 + (uint64_t)((M + 255) / 256) * N * 4 + 1024);
         if (s != FG_OK) return s;
         FgFmaBwd b{};

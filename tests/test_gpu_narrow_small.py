@@ -51,3 +51,44 @@ def test_update_of_several_tensors(ctx, oracle, sizes):
         if n:
             oracle.sgd(a, b, 0.1)
             assert np.array_equal(ctx.to_numpy(dw), a) and (ctx.to_numpy(dg) == 0).all()
+
+
+# Small products of a narrow layer: the FMA kernel for few rows, the kernels above for many; either side of the lines between them (rows, and
+# rows x inputs; with the layer below, without, with an activation of its own), which kernels ran by the timing records.
+@pytest.mark.parametrize("M,N,K,narrow", [(3072, 4, 2, (False, True, True)), (3073, 4, 2, (True, True, True)), (2048, 3, 5, (False, False, True)),
+                                          (2049, 3, 5, (False, True, True)), (1024, 1, 97, (False, False, False)), (1024, 1, 98, (False, False, True)),
+                                          (1025, 16, 16, (False, False, True)), (1000, 4, 205, (False, False, True)), (1000, 4, 206, (True, True, True)),
+                                          (64, 1, 4007, (False, False, True)), (64, 1, 4008, (True, True, True)), (60_001, 10, 6, (True, True, True)),
+                                          (20, 16, 13_000, (True, True, True))])
+def test_few_rows_and_many(ctx, oracle, M, N, K, narrow):
+    r = np.random.Generator(np.random.Philox(M + N + K))
+    f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
+    up = lambda a: ctx.init_tensor_f32(a.shape, a)                            # noqa: E731
+    A, B, dY, S, S1 = f(M, K), f(K, N), f(M, N), np.tanh(f(M, N)), np.tanh(f(M, K))
+    a, b, y, s, s1 = (up(x) for x in (A, B, dY, S, S1))
+    dz = oracle.act_bwd(dY, S, "tanh")
+    out = lambda: [up(np.full(sh, np.nan, np.float32)) for sh in ((M, K), (K, N), (N,), (K,))]      # noqa: E731
+    # sums of k products in chains of at most k: 2^-24 * sqrt(k), five deviations of it, and 16 roundings of 2^-24 for the factor 1 - s * s and
+    # its product (three) and the oracle's own in f32
+    close = lambda x, ref, k, what: rel_err_ok(ctx.to_numpy(x), ref, 2.0 ** -24 * (16 + 5 * k ** 0.5))[0] or pytest.fail(what)      # noqa: E731
+
+    def ran(call):
+        ctx.timing_enable(True)
+        call()
+        n = ctx.timing_read("skinny")[0]
+        ctx.timing_enable(False)
+        return n > 0
+
+    dA, dB, db, below = out()
+    assert ran(lambda: ctx.gemm_bwd_paired(a, b, y, M, N, K, dB=dB, dbias=db, dA=dA, below_act="tanh", below_saved=s1, below_dbias=below)) == narrow[0]
+    ref = oracle.act_bwd(oracle.gemm(dY, B, transB=True, f64=True), S1, "tanh")
+    close(dA, ref, N, "dA below")
+    close(dB, oracle.gemm(A, dY, transA=True, f64=True), M, "dB below")
+    close(db, dY.astype(np.float64).sum(0), M, "dbias below")
+    close(below, ref.astype(np.float64).sum(0), M, "bias gradient of the layer below")
+    for k, (z, kw) in enumerate(((dY, dict(act="none")), (dz, dict(act="tanh", saved=s)))):
+        dA, dB, db, _ = out()
+        assert ran(lambda: ctx.gemm_bwd(a, b, y, M, N, K, dA=dA, dB=dB, dbias=db, **kw)) == narrow[1 + k]
+        close(dA, oracle.gemm(z, B, transB=True, f64=True), N, "dA")
+        close(dB, oracle.gemm(A, z, transA=True, f64=True), M, "dB")
+        close(db, z.astype(np.float64).sum(0), M, "dbias")
