@@ -383,6 +383,8 @@ int32_t fg_gemm_simt_launch(fg_ctx* ctx, int transA, int transB, uint32_t M, uin
 int32_t fg_gemm_simt_batched_launch(fg_ctx* ctx, int transA, int transB, uint32_t batch, uint32_t M, uint32_t N, uint32_t K,
                                     const float* A, uint64_t sA, const float* B, uint64_t sB, float* C, uint64_t sC,
                                     const float* bias, int act, float* preact_out);
+// Is the exact path the faster one for a small forward product whose order of sums is free?
+bool fg_gemm_simt_suits(uint32_t M, uint32_t N, uint32_t K);
 // Does the exact path take its 64 x 64 tiles for these products?
 bool fg_gemm_simt_large(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t batch);
 // dB = Aᵀ·dZ and dA = dZ·Bᵀ of a batch in one launch, where fg_gemm_simt_large says no for both.

@@ -722,6 +722,16 @@ bool fg_gemm_simt_large(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t batc
     return tiles16 > 4ull * (uint64_t)ctx->sm_count || M > 65535u * 16u;
 }
 
+// With one tile of k the FMA kernel's shares have nothing to share, its 64 columns are mostly padding in a narrow layer, and rows off the
+// 16-byte boundary are copied and stored word by word.  Device times of 500 products, this kernel and that (us): 64 x 2 x 1 1.9 / 2.5,
+// 8000 x 2 x 16 3.3 / 5.4, 20000 x 32 x 4 7.8 / 9.0, 16384 x 17 x 8 6.6 / 8.5, 3000 x 17 x 33 3.7 / 5.0, 300 x 65 x 64 2.9 / 3.4, 1 x 1001 x 30
+// 2.3 / 2.9, 300 x 5001 x 1 10.3 / 15.2; the other side 300 x 16 x 33 2.8 / 2.3, 1000 x 256 x 4 3.6 / 3.0, 64 x 17 x 100 4.0 / 3.5,
+// 8 x 30001 x 8 10.6 / 7.2, 16 x 5001 x 60 3.7 / 3.4, 65536 x 4 x 4 22.2 / 18.8, 120000 x 32 x 1 39 / 34.
+bool fg_gemm_simt_suits(uint32_t M, uint32_t N, uint32_t K) {
+    if (N % 4 == 0) return K <= TK && N <= 32 && M <= 32768;
+    return M <= 65535u * 64u && (K <= TK ? N <= 8192 : K <= 2 * TK && N <= 4096);
+}
+
 int32_t fg_gemm_simt_batched_bwd_launch(fg_ctx* ctx, uint32_t batch, uint32_t M, uint32_t N, uint32_t K, const float* A, uint64_t sA, const float* B,
                                         uint64_t sB, const float* dZ, uint64_t sC, float* dA, float* dB) {
     SimtBwd p{M, N, K, A, B, dZ, dA, dB, sA, sB, sC, (N + 31) / 32, 0, 0, (K + 31) / 32, 0};

@@ -185,3 +185,21 @@ def test_infinities_and_nan(ctx):
     ctx.gemm(up(ctx, A)[1], up(ctx, B)[1], C, M, N, K)
     got = ctx.to_numpy(C)
     assert np.isposinf(got[1]).all() and np.isnan(got[2]).all() and (got[[0, 3, 4]] == K).all()
+
+
+# Forward products of a short k: where the exact path is the faster one (one k tile of 32 and up to 32 columns, or rows off the 16-byte boundary
+# and up to two k tiles) AUTO's sums are in its order, bit for bit; beyond it they are in shares, which an output of thousands of sums shows.
+@pytest.mark.parametrize("M,N,K,exact", [(64, 16, 2, True), (1, 1, 1, True), (700, 32, 32, True), (700, 36, 32, False), (700, 33, 64, True), (700, 33, 65, False),
+                                         (16384, 17, 8, True), (300, 28, 33, False), (3, 8189, 32, True), (3, 8193, 32, False), (20, 4095, 64, True),
+                                         (20, 4097, 64, False), (5000, 17, 40, True), (32768, 32, 3, True)])
+def test_forward_of_a_short_k(ctx, oracle, M, N, K, exact):
+    r = rng(M + N + K)
+    A, B, bias = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32), r.standard_normal(N, np.float32)
+    a, b, v = up(ctx, A), up(ctx, B), up(ctx, bias)
+    C, P, E = (up(ctx, np.zeros((M, N))) for _ in range(3))
+    ctx.gemm(a[1], b[1], C[1], M, N, K, bias=v[1], act="tanh", preact_out=P[1])
+    ctx.gemm(a[1], b[1], E[1], M, N, K, bias=v[1], act="none", mode="simt")
+    got = ctx.to_numpy(P[0])
+    assert np.array_equal(got, ctx.to_numpy(E[0])) == exact
+    check(got.reshape(M, N), oracle.gemm(A, B, f64=True).astype(np.float64) + bias, K, "pre-activation")
+    check(ctx.to_numpy(C[0]), np.tanh(got.astype(np.float64)), 0, "output")
