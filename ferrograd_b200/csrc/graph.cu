@@ -136,6 +136,7 @@ struct fg_exec {
     // reference's Schedule is a captured hipGraph: rocm/mod.rs:324-389).  0 forward, 1 loss, 2 backward, 3 optim.
     fg_plan* plan[4] = {nullptr, nullptr, nullptr, nullptr};
     int calls[4] = {0, 0, 0, 0};
+    uint64_t first_launches[4] = {0, 0, 0, 0};      // kernels that each dispatch launched when it ran first
     const void* plan_key[4] = {nullptr, nullptr, nullptr, nullptr};   // loss: the target buffer
     const void* plan_ws[4] = {nullptr, nullptr, nullptr, nullptr};    // scratch arena the plan was recorded against
     bool use_plans = true;
@@ -1032,19 +1033,25 @@ static int32_t optim_eager(fg_exec* e) {
 // three launches per step of the forward pass).  Every step also enqueues collectives then, whose host-side cost a replayed graph
 // avoids (two GPUs, 784-4096-4096-10, about 125 us per launch: 1.97 ms per step replayed against 2.03 with plain launches; eight
 // 8192-wide layers, about 800 us per launch: 27.0 against 26.5 ms, so those stay with plain launches).
-// On one GPU a dispatch is a few launches, which the stream overlaps with each other and with those of the dispatch before; the start
-// and the end of a graph do not overlap with anything (us per step, replayed and plain: 2-16-2 22.5 / 18.8, 200-256-256-10 59.6 / 56.7,
-// 427-32-26-95 39.1 / 32.6, 64-1644-42-41 73.8 / 65.0; graphs for some of the dispatches are slower than either).
+// On one GPU a plain launch costs the host 2.1 to 2.6 us, beside the device's work, and the start and the end of a graph, four a step, overlap
+// with nothing: plain launches while they are few or long, by the same estimate over the launches that the dispatches made when they
+// ran first.  us per step, replayed and plain, on a host of 2.6 us: 2-16-2 22.5 / 18.8, 427-32-26-95 39.1 / 32.6, 200-256-256-10 59.6 / 56.7; layers of
+// n x n with a residual after each (nine launches a layer) on batches of b, n / b: two of 16 / 32 39 / 48, of 64 / 256 50 / 48, eight of 16 / 32
+// 113 / 173, of 64 / 256 148 / 175, of 256 / 256 199 / 203, of 512 / 512 309 / 306, forty of 16 / 32 516 / 819, of 512 / 512 1583 / 1555; without the
+// residual eight of 32 / 128 60 / 54, forty of 16 / 32 211 / 232.  Of 60 such networks the rule has none more than 4 % slower than the better
+// way there; where the host takes 2.1 us the smallest that are recorded lose (two of 16 / 32 43 / 40, of 32 / 128 47 / 40), the deep ones gain
+// less (forty of 16 / 32 588 / 679).
 static bool plans_wanted(const fg_exec* e) {
     if (!e->use_plans || e->ctx->opt_exec_plans == 0) return false;
     if (e->ctx->opt_exec_plans == 1) return true;
-    if (e->ctx->comm == nullptr || e->ctx->nranks <= 1) return false;
     double flop = 0.0, bytes = 0.0;
     for (const GemmStep& gs : e->gemms) flop += 3.0 * 2.0 * gs.batch * (double)gs.M * gs.N * gs.K;
     for (const ENode& en : e->n) bytes += 3.0 * (double)en.numel * (double)e->esize;
     const double est_us = flop / 300e6 + bytes / 5e6;
-    const double launches = 3.0 * (double)std::max<size_t>(e->fwd.size(), 1);
-    return est_us / launches < 300.0;
+    if (e->ctx->comm != nullptr && e->ctx->nranks > 1) return est_us / (3.0 * (double)std::max<size_t>(e->fwd.size(), 1)) < 300.0;
+    double launches = 0.0;
+    for (uint64_t n : e->first_launches) launches += (double)n;
+    return launches >= 16.0 && est_us < 0.5 * launches && launches >= 15.0 + 400.0 * est_us / launches;
 }
 
 // Runs one dispatch: eagerly the first time (which also sizes the scratch arena), recorded as a plan the
@@ -1053,10 +1060,17 @@ static bool plans_wanted(const fg_exec* e) {
 // simply enqueued, so that it becomes part of the caller's plan.
 static int32_t run_planned(fg_exec* e, int which, const void* key, const std::function<int32_t()>& eager) {
     fg_ctx* ctx = e->ctx;
-    if (!plans_wanted(e) || ctx->capturing) return eager();
+    if (ctx->capturing) return eager();
+    if (e->calls[which] == 0) {
+        e->calls[which] = 1;
+        const uint64_t before = ctx->launches;
+        const int32_t s = eager();
+        e->first_launches[which] = ctx->launches - before;
+        return s;
+    }
+    if (!plans_wanted(e)) return eager();
     if (e->plan[which] && e->plan_key[which] == key && e->plan_ws[which] == (const void*)ctx->ws)
         return fg_plan_launch(ctx, e->plan[which]);
-    if (e->calls[which]++ == 0) return eager();
     if (e->plan[which]) { fg_plan_destroy(e->plan[which]); e->plan[which] = nullptr; }
     int32_t s = fg_plan_begin(ctx);
     if (s != FG_OK) return eager();

@@ -101,8 +101,10 @@ uint64_t fg_ctx_workspace_bytes(fg_ctx* ctx);
  *                   allows; "0" sends every shape through operand planes written by a pre-pass
  *   "exec_plans"    "auto" (default) | "1" | "0": the graph engine records each dispatch as a CUDA graph and
  *                   replays it.  "auto" does so when the context has a communicator and the kernels are short to
- *                   medium-sized (the host-side cost of enqueueing collectives every step is avoided); on one GPU
- *                   plain launches overlap across the dispatches, which graphs do not
+ *                   medium-sized (the host-side cost of enqueueing collectives every step is avoided), and on one
+ *                   GPU when the dispatches make many short launches (from 16 on), which a host enqueues more
+ *                   slowly than the device runs them; others overlap across the dispatches as plain launches,
+ *                   which graphs do not
  *   "comm_max_ctas" CTAs the communicator may use (default 12; read by fg_comm_init)
  *   "comm_sms"      SMs the persistent GEMMs leave free while an exchange is in flight (default 16; 0 = none)
  *   "comm_min_exchange"  the graph engine starts a gradient exchange during the backward pass once this many

@@ -592,3 +592,40 @@ def test_graph_errors_are_values(ctx):
     empty = Graph.new(MEAN_SQUARED_ERROR, Optim.sgd().lower)
     with pytest.raises(FgError):
         ctx.alloc_tensors(empty, None, [f32_bits(0.1)])
+
+
+# Which graphs are recorded and replayed by default: those of many short launches, whose launching would cost the host more than the device
+# takes for them; not a few of them, nor long ones.  The same weights as with plain launches, bit for bit.
+@pytest.mark.parametrize("layers,width,batch,recorded", [(1, 16, 32, False), (2, 16, 32, True), (8, 16, 32, True), (20, 64, 256, True), (2, 512, 512, False)])
+def test_graphs_of_many_short_launches_are_recorded(layers, width, batch, recorded):
+    from ferrograd_b200 import GpuContext, Optim
+    ctx = GpuContext(0)
+
+    def define(g, fb, fw):
+        h = g.input([fb, fw])
+        for _ in range(layers):
+            h = g.add(g.tanh(g.add(g.matmul(h, g.input([fw, fw])), g.input([fw]))), h)
+
+    def train(plans):
+        ctx.set_option("exec_plans", plans)
+        r = np.random.Generator(np.random.Philox(layers))
+        graph, t, kernels, binding = build(ctx, define, [batch, width], optim=Optim.adamw(), lr=1e-2)
+        values = [r.standard_normal((batch, width), np.float32)]
+        for _ in range(layers):
+            values += [r.standard_normal((width, width), np.float32) * np.float32(width ** -0.5), np.zeros(width, np.float32)]
+        ins = [ctx.init_tensor_f32(a.shape, a) for a in values]
+        sch = ctx.schedule(kernels, binding, ins, t, [], Optim.adamw().state, trainable=[0] + [1] * (2 * layers))
+        target = ctx.init_tensor_f32((batch, width), r.standard_normal((batch, width), np.float32))
+        for step in range(4):
+            if plans == "auto":
+                assert t.plans_active() == (recorded and step > 0)      # (the first pass counts the launches)
+            ctx.dispatch_forward(sch)
+            ctx.dispatch_loss(sch, target)
+            ctx.dispatch_backward(sch)
+            ctx.dispatch_optim(sch)
+        out = [ctx.to_numpy(x).copy() for x in ins]
+        t.destroy()
+        return out
+    for a, b in zip(train("auto"), train("0")):
+        assert np.array_equal(a, b)
+    ctx.destroy()
