@@ -570,6 +570,8 @@ int32_t fg_exec_destroy(fg_exec* e) {
 int32_t fg_exec_set_adamw(fg_exec* e, const fg_adamw_hyper* h) {
     if (!e || !h) return FG_ERR_INVALID_ARGUMENT;
     e->hyper = *h;
+    if (e->plan[3]) fg_plan_destroy(e->plan[3]);      // recorded with the previous ones
+    e->plan[3] = nullptr;
     return FG_OK;
 }
 

@@ -88,3 +88,30 @@ def test_betas_out_of_range_are_refused(oracle, beta1, beta2, plans):
     assert ok, f"{worst:.3g}"
     net.tensors.destroy()
     ctx.destroy()
+
+
+def test_a_recorded_update_follows_the_hyperparameters():
+    import ctypes as C
+
+    from ferrograd_b200 import GpuContext, _lib
+    from ferrograd_b200.mlp import GraphMLP
+    dims, batch = [4, 8, 2], 16
+
+    def train(plans):
+        ctx = GpuContext(0)
+        ctx.set_option("exec_plans", plans)
+        r = np.random.Generator(np.random.Philox(5))
+        net = GraphMLP(ctx, dims, batch, "tanh", "mse", ("adamw", 1e-2, 0.9, 0.999, 1e-8, 0.01))
+        net.set_params([r.standard_normal((a, b), np.float32) for a, b in zip(dims, dims[1:])], [np.zeros(d, np.float32) for d in dims[1:]])
+        net.upload_batch(r.standard_normal((batch, dims[0]), np.float32), r.standard_normal((batch, dims[-1]), np.float32))
+        for step in range(6):
+            if step == 3:      # (recorded in the second step, replayed from then on)
+                hp = _lib.AdamWHyper(0.0, 0.5, 0.9, 1e-8, 0.3)
+                ctx._check(ctx.lib.fg_exec_set_adamw(net.tensors.handle, C.byref(hp)))
+            net.step()
+        out = net.get_params()
+        net.tensors.destroy()
+        ctx.destroy()
+        return out[0] + out[1]
+    for a, b in zip(train("1"), train("0")):
+        assert np.array_equal(a, b)
