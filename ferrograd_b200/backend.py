@@ -401,7 +401,7 @@ class GpuContext:
         self._check(self._c.chain_fwd(self._h, DTYPE[dtype], n, instrs, inputs, out, sv))
 
     def eltwise_chain_bwd(self, instrs, inputs, seed, grads, n, accumulate=False, dtype="f32"):
-        self._check(self._c.chain_bwd(self._h, DTYPE[dtype], n, instrs, inputs, seed, grads, accumulate))
+        self._check(self._c.chain_bwd(self._h, DTYPE[dtype], n, instrs, inputs, seed, grads, int(accumulate)))
 
     def gemm_lowp(self, A, B, Cout, M, N, K, dtype, bias=None, act="none", preact_out=None):
         """GEMM on f16 / bf16 tensors: 16-bit operands straight into the tensor cores, f32 accumulate."""

@@ -64,3 +64,21 @@ def test_programs(calls):
         calls.chain_fwd(None, 0, 4, prog, [1, 2], 2, [None])
     with pytest.raises(IndexError):
         calls.chain_bwd(None, 0, 4, prog, [1, 2], 3, [1, 2, 3], False)
+
+
+@pytest.mark.parametrize("accumulate", [True, 1, 1.0, "1"])
+@pytest.mark.parametrize("numpy_type", [None, "bool_", "int64", "float32"])
+def test_the_mirror_takes_what_int_takes(calls, accumulate, numpy_type):
+    # flags go through int(), as they did with the foreign-function calls; no device: the answer to a NULL context
+    import numpy as np
+
+    from ferrograd_b200 import FgError, GpuContext, _lib
+    ctx = GpuContext.__new__(GpuContext)
+    ctx.lib, ctx.handle, ctx._c, ctx._h = _lib.load(), None, calls, 0
+    flag = accumulate if numpy_type is None else getattr(np, numpy_type)(int(accumulate))
+    prog = [("input", 0, 0, 0.0), ("neg", 0, 0, 0.0)]
+    for call in (lambda: ctx.eltwise_chain_bwd(prog, [16], 16, [16], 4, accumulate=flag), lambda: ctx.softmax_bwd(16, 16, 16, 1, 1, accumulate=flag),
+                 lambda: ctx.sgd_step(16, 16, 1, 0.1, zero_grad=flag), lambda: ctx.gemm(16, 16, 16, 1, 1, 1, transA=flag, transB=flag)):
+        with pytest.raises(FgError) as e:
+            call()
+        assert e.value.code == NOT_INITIALIZED
