@@ -3626,7 +3626,12 @@ bool batch_route_open(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, u
            (N > 16 || mode != FG_GEMM_AUTO);
 }
 
-// Small matrices: the sums of a batch come in the order of k from either kernel.  Where the exact path would take its large tiles the FMA
+// Small matrices: the sums of a batch come in the order of k, whichever kernel adds them and also one matrix at a time (padding between the
+// matrices of a layer with an activation, more than 65535 of them): the loops ask for the exact path.
+int32_t batch_loop_mode(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_t K) {
+    return mode == FG_GEMM_AUTO && pick_path(ctx, mode, M, N, K) == 0 ? (int32_t)FG_GEMM_SIMT : mode;
+}
+// Where the exact path would take its large tiles the FMA
 // kernel's are the faster ones forward and for both gradients together (31 x (60 x 500 x 500) 45 -> 34 and 92 -> 76 us), not for a
 // gradient by itself (dB of 30 x (100 x 100 x 400) 17.7 us, 20.7 with it) nor for a short k (24 x (182 x 151 x 30) 6.2, 7.6 with it).
 bool batch_large(const fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t M, uint32_t N) { return mode == FG_GEMM_AUTO && fg_gemm_simt_large(ctx, M, N, batch); }
@@ -3764,7 +3769,7 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
                               preact_out ? preact_out + t * strideC : nullptr, nullptr, 0);
             ctx->ws_used = keep;
         } else {
-            s = fg_gemm_f32(ctx, mode, 0, 0, M, N, K, A + t * strideA, B + t * strideB, C + t * strideC, bias, act,
+            s = fg_gemm_f32(ctx, batch_loop_mode(ctx, mode, M, N, K), 0, 0, M, N, K, A + t * strideA, B + t * strideB, C + t * strideC, bias, act,
                             preact_out ? preact_out + t * strideC : nullptr);
         }
         if (s != FG_OK) return s;
@@ -3865,7 +3870,7 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
         if (all) return FG_OK;
     }
     for (uint32_t t = 0; t < batch; ++t) {
-        int32_t s = fg_gemm_bwd_f32(ctx, mode, M, N, K, A ? A + t * strideA : nullptr, B ? B + t * strideB : nullptr,
+        int32_t s = fg_gemm_bwd_f32(ctx, batch_loop_mode(ctx, mode, M, N, K), M, N, K, A ? A + t * strideA : nullptr, B ? B + t * strideB : nullptr,
                                     dY + t * strideC, act, saved ? saved + t * strideC : nullptr,
                                     dA ? dA + t * strideA : nullptr, dB ? dB + t * strideB : nullptr, nullptr, nullptr);
         if (s != FG_OK) return s;
