@@ -435,6 +435,7 @@ struct FgFmaBwd {
     uint64_t exch_count;
 };
 int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b);
+uint64_t fg_gemm_fma_bwd_scratch(const FgFmaBwd& b);      // what it carves from the arena, beside column sums of dA
 // Does the backward pass of this layer sum dZ's columns on its way (fg_gemm_bwd_paired_f32's dbias costs nothing)?
 bool fg_gemm_bwd_sums_bias(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool dA);
 uint64_t fg_gemm_skinny_scratch_bytes(uint32_t M, uint32_t N, uint32_t K);   // enough for any one skinny launch

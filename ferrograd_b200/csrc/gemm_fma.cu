@@ -619,21 +619,37 @@ bool fg_gemm_fma_suits_small(uint32_t M, uint32_t N, uint32_t K, int products) {
     return M <= (products & kFgBelow ? 3072u : 2048u) && mk + 55ull * M <= 260000u;
 }
 
-// The backward pass of one layer, see FgFmaBwd.  The caller has reserved room for dZ (M * N floats) and for column sums of dA.
-int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b) {
+namespace {
+// What a backward pass cannot do in one launch: an output lies over dZ or its factor, or over any operand; dZ is formed first, as it is
+// read after the first output is written, or for a bias gradient without dB.
+struct FmaBwdOverlap { bool over_z, over_in, forms_z; };
+FmaBwdOverlap bwd_overlap(const FgFmaBwd& b) {
     const uint64_t mn = (uint64_t)b.M * b.N * 4, mk = (uint64_t)b.M * b.K * 4, kn = (uint64_t)b.K * b.N * 4;
     const struct { const void* p; uint64_t n; } outs[5] = {{b.dA, mk}, {b.dB, kn}, {b.dbias, b.N * 4ull}, {b.below_dbias, b.K * 4ull},
                                                            {b.pairs, (b.pairs_stride + (uint64_t)b.M * b.K) * 2}};
-    bool over_z = false, over_in = false;      // an output lies over dZ or its factor; over any operand
+    FmaBwdOverlap r{};
     for (const auto& o : outs) {
-        over_z |= fg_ranges_meet(o.p, o.n, b.dZ, mn) || fg_ranges_meet(o.p, o.n, b.factor, mn);
-        over_in |= fg_ranges_meet(o.p, o.n, b.A, mk) || fg_ranges_meet(o.p, o.n, b.B, kn);
+        r.over_z |= fg_ranges_meet(o.p, o.n, b.dZ, mn) || fg_ranges_meet(o.p, o.n, b.factor, mn);
+        r.over_in |= fg_ranges_meet(o.p, o.n, b.A, mk) || fg_ranges_meet(o.p, o.n, b.B, kn);
     }
+    r.forms_z = b.factor && (r.over_z || (b.dbias && !b.dB));
+    return r;
+}
+}  // namespace
+
+uint64_t fg_gemm_fma_bwd_scratch(const FgFmaBwd& b) {
+    return (bwd_overlap(b).forms_z ? (uint64_t)b.M * b.N * 4 + 256 : 0) + (b.dbias && !b.dB ? (uint64_t)((b.M + 255) / 256) * b.N * 4 + 256 : 0);
+}
+
+// The backward pass of one layer, see FgFmaBwd.  The caller has reserved fg_gemm_fma_bwd_scratch() and room for column sums of dA.
+int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b) {
+    const FmaBwdOverlap lies = bwd_overlap(b);
     const float *dz = b.dZ, *factor = b.factor;
     int32_t s;
-    if (factor && (over_z || (b.dbias && !b.dB))) {      // dZ is formed first, as it is read after the first output is written
+    if (lies.forms_z) {
         void* p;
-        if ((s = fg_ws_alloc(ctx, mn, &p)) != FG_OK || (s = fg_act_bwd_launch(ctx, (uint64_t)b.M * b.N, b.factor_act, dz, factor, (float*)p)) != FG_OK) return s;
+        if ((s = fg_ws_alloc(ctx, (uint64_t)b.M * b.N * 4, &p)) != FG_OK ||
+            (s = fg_act_bwd_launch(ctx, (uint64_t)b.M * b.N, b.factor_act, dz, factor, (float*)p)) != FG_OK) return s;
         dz = (const float*)p;
         factor = nullptr;
     }
@@ -644,7 +660,7 @@ int32_t fg_gemm_fma_bwd(fg_ctx* ctx, const FgFmaBwd& b) {
     w.colsum_b = b.dbias;
     x.tb = 1; x.M = b.M; x.N = b.K; x.K = b.N; x.A = dz; x.B = b.B; x.C = b.dA; x.factor = factor; x.factor_act = b.factor_act;
     x.mul_saved = b.mul_saved; x.mul_act = b.mul_act; x.pairs = b.pairs; x.pairs_stride = b.pairs_stride; x.colsum_c = b.below_dbias;
-    if (b.dB && b.dA && !b.exch_buf && !over_z && !over_in) return fg_gemm_fma_launch(ctx, ops, 2, 1, false);
+    if (b.dB && b.dA && !b.exch_buf && !lies.over_z && !lies.over_in) return fg_gemm_fma_launch(ctx, ops, 2, 1, false);
     if (b.dB && (s = fg_gemm_fma_launch(ctx, &w, 1, 1, false)) != FG_OK) return s;
     if (b.exch_buf && (s = fg_allreduce_sum_f32(ctx, b.exch_buf, b.exch_count)) != FG_OK) return s;
     return b.dA ? fg_gemm_fma_launch(ctx, &x, 1, 1, false) : FG_OK;

@@ -3544,12 +3544,11 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     const bool fma = path == 0 ? mode == FG_GEMM_AUTO && !takes_narrow(ctx, mode, M, N, K, fuse)
                                : (dA || dB) && takes_fma(ctx, mode, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0));
     if (!dZ_out && fma) {
-        int32_t s = fg_ws_ensure(ctx, (uint64_t)M * N * 4 + (uint64_t)((M + 255) / 256) * N * 4 + 1024);
-        if (s != FG_OK) return s;
         FgFmaBwd b{};
         b.M = M; b.N = N; b.K = K; b.A = A; b.B = B; b.dZ = dY; b.factor = fuse ? saved : nullptr; b.factor_act = act;
         b.dA = dA; b.dB = dB; b.dbias = dbias; b.exch_buf = exch_buf; b.exch_count = exch_count;
-        return fg_gemm_fma_bwd(ctx, b);
+        const int32_t s = fg_ws_ensure(ctx, fg_gemm_fma_bwd_scratch(b));
+        return s != FG_OK ? s : fg_gemm_fma_bwd(ctx, b);
     }
     // (prep_kernel takes up to 65535 * 32 rows, the planes twice as many)
     if (path == 2 && N > 16 && (dA || dB) && M <= 65535u * 32u) {

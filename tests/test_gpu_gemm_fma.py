@@ -220,3 +220,32 @@ def test_batched_sums_are_in_order_with_an_activation(ctx, T, M, N, K, gap):
         out.append((ctx.to_numpy(dA[0]), ctx.to_numpy(dB[0])))
     for x, e in zip(*out):
         assert np.array_equal(x, e)
+
+
+@pytest.mark.parametrize("M,N,K,act", [(200, 256, 256, "none"), (200, 256, 256, "gelu"), (100, 20, 30, "tanh")])
+def test_backward_is_recorded_without_room_for_dz(oracle, M, N, K, act):
+    # the gradients take dZ through the activation as they read it: a recording needs no scratch arena of its size
+    from ferrograd_b200 import FgError, GpuContext
+    c = GpuContext(0)
+    c._check(c.lib.fg_ctx_reserve_workspace(c.handle, 1024))
+    r = rng(M)
+    f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
+    A, B, dY, S = f(M, K), f(K, N), f(M, N), np.tanh(f(M, N))
+    a, b, y, sv = (up(c, x) for x in (A, B, dY, S))
+    dA, dB, db = (up(c, np.zeros(s)) for s in ((M, K), (K, N), (N,)))
+    kw = dict(act=act, saved=sv[1] if act != "none" else None)
+    c.plan_begin()
+    c.gemm_bwd(a[1], b[1], y[1], M, N, K, dA=dA[1], dB=dB[1], dbias=db[1], **kw)
+    plan = c.plan_end()
+    plan.launch()
+    dz = oracle.act_bwd(dY, S, act) if act != "none" else dY
+    check(c.to_numpy(dA[0]).reshape(M, K), oracle.gemm(dz, B, transB=True, f64=True), N, "dA")
+    check(c.to_numpy(dB[0]).reshape(K, N), oracle.gemm(A, dz, transA=True, f64=True), M, "dB")
+    check(c.to_numpy(db[0]), dz.astype(np.float64).sum(0), M, "dbias")
+    plan.destroy()
+    if N == K and act != "none":      # dA over the saved tensor: dZ is formed first and does need its room
+        c.plan_begin()
+        with pytest.raises(FgError):
+            c.gemm_bwd(a[1], b[1], y[1], M, N, K, dA=sv[1], dB=dB[1], **kw)
+        c.plan_end().destroy()
+    c.destroy()
