@@ -3046,6 +3046,14 @@ bool takes_narrow(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t 
     return pick_path(ctx, mode, M, N, K) != 0 ||
            (M <= 65535u * 32u && !fg_gemm_fma_suits_small(M, N, K, kFgGradB | kFgGradA | (fuse ? kFgFactor : 0)));
 }
+// Scratch of the narrow layer's backward pass.  A small product that finds no room for it (a recording whose arena was sized for less) keeps
+// to the kernels that need less.
+uint64_t narrow_bwd_need(uint32_t M, uint32_t N, uint32_t K, bool dbias) {
+    return 2048 + (uint64_t)M * N * 4 + 256 + fg_gemm_skinny_scratch_bytes(M, N, K) + (dbias ? (uint64_t)((M + 31) / 32) * N * 4 + 256 : 0);
+}
+bool runs_narrow(fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, bool fuse, bool dbias) {
+    return takes_narrow(ctx, mode, M, N, K, fuse) && (pick_path(ctx, mode, M, N, K) != 0 || fg_ws_try(ctx, narrow_bwd_need(M, N, K, dbias)));
+}
 
 }  // namespace
 
@@ -3207,7 +3215,7 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
                         const float* dY, int32_t act, const float* saved, float* dA, float* dB, float* dbias,
                         float* dZ_out, float* exch_buf, uint64_t exch_count) {
     const bool fuse = act != FG_ACT_NONE;
-    const bool skinny = takes_narrow(ctx, mode, M, N, K, fuse);
+    const bool skinny = runs_narrow(ctx, mode, M, N, K, fuse, dbias != nullptr);
     const int path = skinny ? 2 : pick_path(ctx, mode, M, N, K);
     const uint64_t mn = (uint64_t)M * N;
 
@@ -3249,11 +3257,10 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
     // both run as plain-FMA kernels on dZ itself; the operand pre-passes and a tensor-core GEMM that could
     // only fill M/128 CTAs would cost several times more.
     const bool tc_da = dA && !skinny, tc_db = dB && !skinny;
-    uint64_t need = 2048;
+    uint64_t need = skinny ? narrow_bwd_need(M, N, K, dbias != nullptr) : 2048;
     if (tc_da) need += planes_bytes(fmt, M, N) + planes_bytes(fmt, K, N) + kPairPartialBytes;
     if (tc_db) need += planes_bytes(fmt, N, M) + planes_bytes(fmt, K, M) + kPairPartialBytes;
-    if (skinny) need += mn * 4 + 256 + fg_gemm_skinny_scratch_bytes(M, N, K);
-    if (dbias) need += (uint64_t)((M + 31) / 32) * N * 4 + 256;   // per-tile column sums from the pre-pass
+    if (dbias && !skinny) need += (uint64_t)((M + 31) / 32) * N * 4 + 256;   // per-tile column sums from the pre-pass
     { int32_t s0 = fg_ws_ensure(ctx, need); if (s0 != FG_OK) return s0; }
     PlaneSet dz_n{}, dz_t{}, b_n{}, a_t{};
     void* dz_val = dZ_out;
@@ -3541,7 +3548,7 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, !dB || A, "fg_gemm_bwd_f32: dB needs A");
     const bool fuse = act != FG_ACT_NONE;
     const int path = pick_path(ctx, mode, M, N, K);
-    const bool fma = path == 0 ? mode == FG_GEMM_AUTO && !takes_narrow(ctx, mode, M, N, K, fuse)
+    const bool fma = path == 0 ? mode == FG_GEMM_AUTO && !runs_narrow(ctx, mode, M, N, K, fuse, dbias != nullptr)
                                : (dA || dB) && takes_fma(ctx, mode, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0));
     if (!dZ_out && fma) {
         FgFmaBwd b{};

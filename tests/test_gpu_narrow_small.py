@@ -92,3 +92,27 @@ def test_few_rows_and_many(ctx, oracle, M, N, K, narrow):
         close(dA, oracle.gemm(z, B, transB=True, f64=True), N, "dA")
         close(dB, oracle.gemm(A, z, transA=True, f64=True), M, "dB")
         close(db, z.astype(np.float64).sum(0), M, "dbias")
+
+
+def test_many_rows_are_recorded_in_the_room_for_dz(oracle):
+    # 5000 rows are the narrow layer's kernels', but not where a recording's arena has room for dZ alone
+    from ferrograd_b200 import GpuContext
+    M, N, K = 5000, 2, 4
+    c = GpuContext(0)
+    c.reserve_workspace(M * N * 4 + (M + 255) // 256 * N * 4 + 1024)
+    r = np.random.Generator(np.random.Philox(8))
+    f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
+    A, B, dY, S = f(M, K), f(K, N), f(M, N), np.tanh(f(M, N))
+    t = [c.init_tensor_f32(x.shape, x) for x in (A, B, dY, S)]
+    dA, dB, db = (c.new_tensor(s) for s in ((M, K), (K, N), (N,)))
+    c.plan_begin()
+    c.gemm_bwd(t[0], t[1], t[2], M, N, K, act="tanh", saved=t[3], dA=dA, dB=dB, dbias=db)
+    plan = c.plan_end()
+    plan.launch()
+    dz = oracle.act_bwd(dY, S, "tanh")
+    close = lambda x, ref, what: rel_err_ok(c.to_numpy(x), ref, 2.0 ** -24 * (16 + 5 * M ** 0.5))[0] or pytest.fail(what)      # noqa: E731
+    close(dA, oracle.gemm(dz, B, transB=True, f64=True), "dA")
+    close(dB, oracle.gemm(A, dz, transA=True, f64=True), "dB")
+    close(db, dz.astype(np.float64).sum(0), "dbias")
+    plan.destroy()
+    c.destroy()
