@@ -412,7 +412,7 @@ struct FgFmaOp {
     uint64_t sA, sB, sC;
 };
 // One product, or two in one launch (the first with ta, the second with tb).  in_order: every sum is one chain of FMAs in the order of
-// k, the exact path's results.  Room in the arena for one row of C's column sums per 32 rows.
+// k, the exact path's results (forward, or both gradients).  Room in the arena for one row of C's column sums per 32 rows.
 int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch, bool in_order);
 // Is it the kernel for the forward product of [M,K] x [K,N], or for one or both of its gradients?  kFgFactor: dZ is formed on the way;
 // kFgBelow: dA becomes the dZ of the layer below.

@@ -577,7 +577,7 @@ int32_t launch_products(fg_ctx* ctx, const FgFmaOp* ops, uint32_t batch, bool in
             if (ops[0].ta) return ops[0].tb ? launch([] { return gemm_fma_kernel<T, true, true>; }) : launch([] { return gemm_fma_kernel<T, true, false>; });
             return ops[0].tb ? launch([] { return gemm_fma_kernel<T, false, true>; }) : launch([] { return gemm_fma_kernel<T, false, false>; });
         };
-        s = in_order ? one(TileOrdered{}) : with_tile(plan.tile[0], one);
+        s = in_order ? launch([] { return gemm_fma_kernel<TileOrdered, false, false>; }) : with_tile(plan.tile[0], one);      // (in order: forward alone)
     } else {
         auto both = [&](auto tb, auto ta) { return launch([] { return gemm_fma_bwd_kernel<decltype(tb), decltype(ta)>; }); };
         s = in_order ? both(TileOrdered{}, TileOrdered{})
@@ -590,6 +590,7 @@ int32_t launch_products(fg_ctx* ctx, const FgFmaOp* ops, uint32_t batch, bool in
 
 int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch, bool in_order) {
     if (batch == 0) return FG_OK;
+    if (in_order && n == 1 && (ops[0].ta || ops[0].tb)) return fg_fail(ctx, FG_ERR_INTERNAL, "FMA kernel: one gradient in order is the exact path's");
     return n > 1 ? launch_products<2>(ctx, ops, batch, in_order) : launch_products<1>(ctx, ops, batch, in_order);
 }
 
