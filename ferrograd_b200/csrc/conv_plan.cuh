@@ -26,9 +26,11 @@ struct ConvCosts {
     double kb[2], store[2], ragged[2], last[2], ragged_last[2], ragged_shares[2], around, meet;
 };
 // The conversion kernel, fitted to whole launches: per k-block 0.55 us with 128 x 128 tiles and 0.33 us with 128 x 64 ones (0.34 - 0.37
-// with a long k), storing a tile 2.1 and 1.5 us (the last wide one 1.2, by twice the warps), 3.5 us of set-up and first loads, 2 - 3 us
-// for the shares' sums to meet; where a ragged N is stored word by word 0.5 to 2 us more, and 3.6 us divided among the shares.
-constexpr ConvCosts kConvCosts = {32, {1050.0, 630.0}, {4000.0, 2800.0}, {1500.0, 2000.0}, {2000.0, 2800.0}, {1000.0, 3900.0}, {6800.0, 3500.0}, 6500.0, 5500.0};
+// with a long k), storing a tile 2.6 and 1.5 us (the last wide one 1.2, by twice the warps), 3.5 us of set-up and first loads, 2 - 3 us
+// for the shares' sums to meet; where a ragged N is stored word by word 0.5 to 2 us more, and 3.6 us divided among the shares.  (With a wide
+// tile's store at 2.1 us, products of a few k-blocks and several units per CTA took wide tiles: 15064 x 400 x 1 17.3 us, 15.7 with narrow ones,
+// 4390 x 632 x 2 11.1 and 9.8, dA of 1920 x 96 x 1384 10.6 and 9.0.)
+constexpr ConvCosts kConvCosts = {32, {1050.0, 630.0}, {5000.0, 2800.0}, {1500.0, 2000.0}, {2000.0, 2800.0}, {1000.0, 3900.0}, {6800.0, 3500.0}, 6500.0, 5500.0};
 
 // Estimated SM cycles of one launch for one or two products (the one with the longer k first) on `sms` SMs.  clusters(bn, split):
 // clusters of `split` CTAs that run at once, below one if there are none.

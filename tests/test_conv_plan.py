@@ -99,3 +99,11 @@ def test_a_query_that_failed_is_asked_again(shim):
     assert ask(0, 1, 5) == 5 and asked.value == 3
     assert ask(0, 1, 9) == 5 and ask(0, 0, 9) == 5 and asked.value == 3
     assert ask(1, 1, 0) == 0 and ask(1, 1, 3) == 0 and asked.value == 4
+
+
+# Of a few k-blocks and more than one unit per CTA, what a unit waits for is the store of its tile: narrow tiles where they take fewer of those
+# in all, wide ones where a wide tile per CTA is all there is, or the k is long.
+@pytest.mark.parametrize("M,N,K,width", [(15064, 400, 1, 64), (4390, 632, 2, 64), (3520, 744, 3, 64), (1920, 1384, 96, 64), (4096, 512, 32, 128),
+                                         (6000, 256, 32, 128), (2048, 1024, 1024, 128)])
+def test_the_width_of_a_short_k(shim, M, N, K, width):
+    assert plan(shim, M, N, K, 148)[:2] == (width, 1)
