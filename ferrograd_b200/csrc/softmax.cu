@@ -103,12 +103,13 @@ struct CeArgs {
     unsigned* arrivals;
 };
 
-// The mean of the rows' losses, in a fixed order, in thread 0 of a block.
+// The mean of the rows' losses, in a fixed order, in thread 0 of a block (L2: they come from other blocks of the same launch).
+template <bool L2>
 __device__ __forceinline__ void mean_of_rows(const float* x, uint32_t n, float* out, float* red) {
     float s = 0.0f, v[8];
     for (uint64_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {      // eight loads in flight, added in order
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = i0 + j * blockDim.x < n ? __ldcg(x + i0 + j * blockDim.x) : 0.0f;
+        for (int j = 0; j < 8; ++j) v[j] = i0 + j * blockDim.x < n ? (L2 ? __ldcg(x + i0 + j * blockDim.x) : x[i0 + j * blockDim.x]) : 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += v[j];
     }
@@ -116,9 +117,8 @@ __device__ __forceinline__ void mean_of_rows(const float* x, uint32_t n, float* 
     if (threadIdx.x == 0) *out = s / (float)n;
 }
 // At the end of a kernel whose blocks have left their rows' losses.
-template <int MODE>
 __device__ __forceinline__ void leave_mean(const CeArgs& a, float* red) {
-    if (MODE == 1 && a.mean && fg_last_block(a.arrivals, gridDim.x)) mean_of_rows(a.loss_row, a.rows, a.mean, red);
+    if (a.mean && fg_last_block(a.arrivals, gridDim.x)) mean_of_rows<true>(a.loss_row, a.rows, a.mean, red);
 }
 
 template <int MODE, bool VEC>
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
         for (int j = 0; j < kRowNV; ++j)
             if (tid + j * kRowT < ncol4) softmax_put4<MODE>(a, o0, o1, tid + j * kRowT, lab, v[j], inv, true);
     }
-    leave_mean<MODE>(a, red_max);
+    if constexpr (MODE == 1) leave_mean(a, red_max);
 }
 
 // ------------------------------------------------------------------------------------
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kRowT, 1) softmax_rowreg_kernel(CeArgs a, int*
 // L1/L2) and evaluates every exponential twice; with its few loads in flight per thread it reached 49 % of the
 // DRAM rate on 16384 x 4096.  MODE as above.
 // ------------------------------------------------------------------------------------
-template <int MODE, int NV>
+template <int MODE, int NV, bool MEAN = false>
 __global__ void __launch_bounds__(256) softmax_held_kernel(CeArgs a) {
     fg_grid_enter();
     __shared__ float red[32];
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256) softmax_held_kernel(CeArgs a) {
             }
         }
     }
-    leave_mean<MODE>(a, red);
+    if constexpr (MEAN) leave_mean(a, red);
 }
 
 // The same for the backward pass: y and dy of a row are read once.
@@ -527,7 +527,7 @@ __device__ __forceinline__ void softmax_put(const CeArgs& a, size_t off, uint32_
     }
 }
 
-template <int MODE, int NV>
+template <int MODE, int NV, bool MEAN = false>
 __global__ void __launch_bounds__(256) softmax_warp_kernel(CeArgs a) {
     fg_grid_enter();
     const uint32_t cols = a.cols, lane = threadIdx.x & 31u, step = gridDim.x * 8;
@@ -570,8 +570,10 @@ __global__ void __launch_bounds__(256) softmax_warp_kernel(CeArgs a) {
         for (int j = 0; j < NV; ++j)
             if (lane + 32u * j < cols) softmax_put<MODE>(a, base + lane + 32u * j, lane + 32u * j, lab, v[j], inv);
     }
-    __shared__ float red[32];
-    leave_mean<MODE>(a, red);
+    if constexpr (MEAN) {
+        __shared__ float red[32];
+        leave_mean(a, red);
+    }
 }
 
 // Where the 16-byte accesses of a row start: `head` words before them, n4 groups of four, and `extra`, the index of the one
@@ -588,7 +590,7 @@ __device__ __forceinline__ RowEdges row_edges(const float* row, uint32_t cols) {
     return e;
 }
 
-template <int MODE, int NV>
+template <int MODE, int NV, bool MEAN = false>
 __global__ void __launch_bounds__(1024) softmax_edge_kernel(CeArgs a) {
     fg_grid_enter();
     // one array per reduction, so that each costs one barrier: an array is written again only after another barrier
@@ -652,7 +654,7 @@ __global__ void __launch_bounds__(1024) softmax_edge_kernel(CeArgs a) {
             if (t + nt * j < ed.n4) softmax_put4<MODE>(a, o0, o1, t + nt * j, lab4, v[j], inv, true);
         if (ed.extra < cols) softmax_put<MODE>(a, base + ed.extra, ed.extra, lab, ve, inv);
     }
-    leave_mean<MODE>(a, red_sum);
+    if constexpr (MEAN) leave_mean(a, red_sum);
 }
 
 template <int NV>
@@ -794,7 +796,7 @@ __global__ void __launch_bounds__(256) ce_elem_kernel(const float* __restrict__ 
 __global__ void mean_kernel(const float* __restrict__ x, uint32_t n, float* __restrict__ out) {
     fg_grid_enter();
     __shared__ float red[32];
-    mean_of_rows(x, n, out, red);
+    mean_of_rows<false>(x, n, out, red);
 }
 
 // Algorithmic HBM bytes of the fused CE kernel: logits in, dlogits (and probs) out.
@@ -865,10 +867,10 @@ int32_t launch_rows(fg_ctx* ctx, CeArgs& a) {
         const uint32_t nv = (a.cols / 4 + 255) / 256;      // float4s per thread: 1 .. 8
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
         const CeArgs k = with_mean<MODE>(ctx, a, grid);
-        if (nv <= 1) fg_launch(ctx, softmax_held_kernel<MODE, 1>, grid, 256, 0, k);
-        else if (nv <= 2) fg_launch(ctx, softmax_held_kernel<MODE, 2>, grid, 256, 0, k);
-        else if (nv <= 4) fg_launch(ctx, softmax_held_kernel<MODE, 4>, grid, 256, 0, k);
-        else fg_launch(ctx, softmax_held_kernel<MODE, 8>, grid, 256, 0, k);
+        if (nv <= 1) fg_launch(ctx, k.mean ? softmax_held_kernel<MODE, 1, MODE == 1> : softmax_held_kernel<MODE, 1>, grid, 256, 0, k);
+        else if (nv <= 2) fg_launch(ctx, k.mean ? softmax_held_kernel<MODE, 2, MODE == 1> : softmax_held_kernel<MODE, 2>, grid, 256, 0, k);
+        else if (nv <= 4) fg_launch(ctx, k.mean ? softmax_held_kernel<MODE, 4, MODE == 1> : softmax_held_kernel<MODE, 4>, grid, 256, 0, k);
+        else fg_launch(ctx, k.mean ? softmax_held_kernel<MODE, 8, MODE == 1> : softmax_held_kernel<MODE, 8>, grid, 256, 0, k);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -877,9 +879,9 @@ int32_t launch_rows(fg_ctx* ctx, CeArgs& a) {
         const int grid = rows_grid(ctx, ((uint64_t)a.rows + 7) / 8, 256);
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
         const CeArgs k = with_mean<MODE>(ctx, a, grid);
-        if (a.cols <= 32) fg_launch(ctx, softmax_warp_kernel<MODE, 1>, grid, 256, 0, k);
-        else if (a.cols <= 128) fg_launch(ctx, softmax_warp_kernel<MODE, 4>, grid, 256, 0, k);
-        else fg_launch(ctx, softmax_warp_kernel<MODE, 16>, grid, 256, 0, k);
+        if (a.cols <= 32) fg_launch(ctx, k.mean ? softmax_warp_kernel<MODE, 1, MODE == 1> : softmax_warp_kernel<MODE, 1>, grid, 256, 0, k);
+        else if (a.cols <= 128) fg_launch(ctx, k.mean ? softmax_warp_kernel<MODE, 4, MODE == 1> : softmax_warp_kernel<MODE, 4>, grid, 256, 0, k);
+        else fg_launch(ctx, k.mean ? softmax_warp_kernel<MODE, 16, MODE == 1> : softmax_warp_kernel<MODE, 16>, grid, 256, 0, k);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
@@ -890,7 +892,7 @@ int32_t launch_rows(fg_ctx* ctx, CeArgs& a) {
         const int grid = rows_grid(ctx, a.rows, threads);
         fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SOFTMAX_CE, MODE == 1 ? ce_bytes(a) : 8.0 * a.rows * a.cols);
         const CeArgs k = with_mean<MODE>(ctx, a, grid);
-        fg_launch(ctx, softmax_edge_kernel<MODE, 8>, grid, threads, 0, k);
+        fg_launch(ctx, k.mean ? softmax_edge_kernel<MODE, 8, MODE == 1> : softmax_edge_kernel<MODE, 8>, grid, threads, 0, k);
         fg_time_end(ctx, tr);
         FG_LAUNCHED(ctx);
         return FG_OK;
