@@ -415,8 +415,8 @@ struct FgFmaOp {
 // k, the exact path's results (forward, or both gradients).  Room in the arena for one row of C's column sums per 32 rows.
 int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batch, bool in_order);
 // Is it the kernel for the forward product of [M,K] x [K,N], or for one or both of its gradients?  kFgFactor: dZ is formed on the way;
-// kFgBelow: dA becomes the dZ of the layer below.
-enum { kFgForward = 0, kFgGradB = 1, kFgGradA = 2, kFgFactor = 4, kFgBelow = 8 };
+// kFgBelow: dA becomes the dZ of the layer below; kFgBias: with the bias gradient.
+enum { kFgForward = 0, kFgGradB = 1, kFgGradA = 2, kFgFactor = 4, kFgBelow = 8, kFgBias = 16 };
 bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products);
 // The same for products too small for the tensor cores: the narrow layer's own kernels take the gradients of up to 16 columns and many rows.
 bool fg_gemm_fma_suits_small(uint32_t M, uint32_t N, uint32_t K, int products);

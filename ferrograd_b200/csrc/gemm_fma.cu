@@ -608,16 +608,19 @@ bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products) {
 }
 
 // A narrow layer's dB is one tile across and a tile per 64 rows of B: its clusters go through all samples, where the narrow layer's own
-// kernels (gemm_skinny_tn_partial_kernel) spread them over the GPU.  Device times of 300 layers, this kernel and those (us): all gradients with the factor of
-// the layer below 1024 x 1 x 1 6.7 / 10.2, 1500 x 10 x 100 13.4 / 16.3, 3072 x 10 x 40 15.1 / 17.8, 4096 x 1 x 1 16.9 / 13.7, 1024 x 4 x 300
-// 13.9 / 13.3, 64 x 4 x 4000 7.5 / 10.1, 128 x 4 x 4000 11.4 / 10.9, 65536 x 4 x 4 285 / 64; the gradients alone 1500 x 1 x 64 8.8 / 9.1,
-// 3072 x 1 x 40 12.6 / 10.4; with an activation's factor on dZ 256 x 4 x 500 7.6 / 11.1, 512 x 4 x 200 10.4 / 10.7, 1024 x 10 x 64
-// 10.0 / 12.2, 1500 x 1 x 40 12.9 / 10.2.
+// kernels (gemm_skinny_tn_partial_kernel) spread them over the GPU, taking longer with more columns; rows off 16 bytes are copied word
+// by word here.  Device times of 300 layers, this kernel and those (us): all gradients with the factor of the layer below 1024 x 1 x 1 6.7 /
+// 10.2, 1500 x 10 x 100 13.4 / 16.3, 3072 x 10 x 40 15.1 / 17.8, 4096 x 16 x 16 14.5 / 22.4, 4096 x 1 x 1 16.9 / 13.7, 1024 x 4 x 300 13.9 / 13.3,
+// 64 x 4 x 4000 7.5 / 10.1, 128 x 4 x 4000 11.4 / 10.9, 65536 x 4 x 4 285 / 64; the gradients alone 1500 x 1 x 64 8.8 / 9.1, 3072 x 4 x 40
+// 10.5 / 11.2, 496 x 16 x 496 (dB) 5.2 / 9.1, 3072 x 1 x 40 12.6 / 10.4; with an activation's factor on dZ 256 x 4 x 500 7.6 / 11.1,
+// 512 x 4 x 200 10.4 / 10.7, 1024 x 10 x 64 10.0 / 12.2, 2048 x 16 x 64 13.3 / 14.5, 1500 x 1 x 40 12.9 / 10.2; dA alone 1024 x 4 x 2 2.9 / 2.3.
 bool fg_gemm_fma_suits_small(uint32_t M, uint32_t N, uint32_t K, int products) {
     if (N > 16 || products == kFgForward) return true;
+    const bool quads = N % 4 == 0, wide = quads && N >= 12;
     const uint64_t mk = (uint64_t)M * K;
-    if (products & kFgFactor) return M <= 1024 && mk <= (M <= 256 ? 250000u : 100000u);
-    return M <= (products & kFgBelow ? 3072u : 2048u) && mk + 55ull * M <= 260000u;
+    if (!(products & kFgGradB)) return products & (kFgFactor | kFgBelow | kFgBias) ? M <= 4096 : M < 64;
+    if (products & kFgFactor) return M <= (wide ? 2048u : 1024u) && mk <= (M <= 256 ? 250000u : wide ? 140000u : 100000u);
+    return M <= (wide ? 4096u : quads || (products & kFgBelow) ? 3072u : 2048u) && mk + 55ull * M <= (wide ? 380000u : 260000u);
 }
 
 namespace {

@@ -3041,18 +3041,21 @@ bool takes_fma(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, 
 }
 // Are a layer's gradients the narrow layer's kernels'?  (Of small products with more rows than the pass over dZ always takes, 65535 tiles
 // of 32, the FMA kernel's after all.)
-bool takes_narrow(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, bool fuse) {
+bool takes_narrow(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, int products) {
     if (mode != FG_GEMM_AUTO || N > 16) return false;
-    return pick_path(ctx, mode, M, N, K) != 0 ||
-           (M <= 65535u * 32u && !fg_gemm_fma_suits_small(M, N, K, kFgGradB | kFgGradA | (fuse ? kFgFactor : 0)));
+    return pick_path(ctx, mode, M, N, K) != 0 || (M <= 65535u * 32u && products && !fg_gemm_fma_suits_small(M, N, K, products));
+}
+int grad_products(const float* dA, const float* dB, const float* dbias, bool fuse) {
+    return (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0) | (dbias ? kFgBias : 0) | (fuse ? kFgFactor : 0);
 }
 // Scratch of the narrow layer's backward pass.  A small product that finds no room for it (a recording whose arena was sized for less) keeps
 // to the kernels that need less.
 uint64_t narrow_bwd_need(uint32_t M, uint32_t N, uint32_t K, bool dbias) {
     return 2048 + (uint64_t)M * N * 4 + 256 + fg_gemm_skinny_scratch_bytes(M, N, K) + (dbias ? (uint64_t)((M + 31) / 32) * N * 4 + 256 : 0);
 }
-bool runs_narrow(fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, bool fuse, bool dbias) {
-    return takes_narrow(ctx, mode, M, N, K, fuse) && (pick_path(ctx, mode, M, N, K) != 0 || fg_ws_try(ctx, narrow_bwd_need(M, N, K, dbias)));
+bool runs_narrow(fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, int products) {
+    return takes_narrow(ctx, mode, M, N, K, products) &&
+           (pick_path(ctx, mode, M, N, K) != 0 || fg_ws_try(ctx, narrow_bwd_need(M, N, K, (products & kFgBias) != 0)));
 }
 
 }  // namespace
@@ -3215,7 +3218,7 @@ int32_t gemm_bwd_planes(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint3
                         const float* dY, int32_t act, const float* saved, float* dA, float* dB, float* dbias,
                         float* dZ_out, float* exch_buf, uint64_t exch_count) {
     const bool fuse = act != FG_ACT_NONE;
-    const bool skinny = runs_narrow(ctx, mode, M, N, K, fuse, dbias != nullptr);
+    const bool skinny = runs_narrow(ctx, mode, M, N, K, grad_products(dA, dB, dbias, fuse));
     const int path = skinny ? 2 : pick_path(ctx, mode, M, N, K);
     const uint64_t mn = (uint64_t)M * N;
 
@@ -3448,7 +3451,7 @@ int32_t gemm_bwd_paired_core(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, Pa
     };
     const bool narrow = N <= 16;
     const int below = dA && (o.mul_saved || dbias_prev) ? kFgBelow : 0;
-    if ((dA || dB) && takes_fma(ctx, FG_GEMM_AUTO, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0) | below)) {
+    if ((dA || dB) && takes_fma(ctx, FG_GEMM_AUTO, M, N, K, grad_products(dA, dB, dbias, false) | below)) {
         if (dA && o.mul_saved != dA && (s = saved_apart()) != FG_OK) return s;      // (an element is read and written by one thread)
         FgFmaBwd b{};
         b.M = M; b.N = N; b.K = K; b.A = A.x; b.B = B.x; b.dZ = dZ.x; b.dA = dA; b.dB = dB; b.dbias = dbias;
@@ -3548,7 +3551,7 @@ int32_t gemm_bwd_impl(fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_
     FG_REQUIRE(ctx, !dB || A, "fg_gemm_bwd_f32: dB needs A");
     const bool fuse = act != FG_ACT_NONE;
     const int path = pick_path(ctx, mode, M, N, K);
-    const bool fma = path == 0 ? mode == FG_GEMM_AUTO && !runs_narrow(ctx, mode, M, N, K, fuse, dbias != nullptr)
+    const bool fma = path == 0 ? mode == FG_GEMM_AUTO && !runs_narrow(ctx, mode, M, N, K, grad_products(dA, dB, dbias, fuse))
                                : (dA || dB) && takes_fma(ctx, mode, M, N, K, (dB ? kFgGradB : 0) | (dA ? kFgGradA : 0));
     if (!dZ_out && fma) {
         FgFmaBwd b{};

@@ -55,11 +55,12 @@ def test_update_of_several_tensors(ctx, oracle, sizes):
 
 # Small products of a narrow layer: the FMA kernel for few rows, the kernels above for many; either side of the lines between them (rows, and
 # rows x inputs; with the layer below, without, with an activation of its own), which kernels ran by the timing records.
-@pytest.mark.parametrize("M,N,K,narrow", [(3072, 4, 2, (False, True, True)), (3073, 4, 2, (True, True, True)), (2048, 3, 5, (False, False, True)),
-                                          (2049, 3, 5, (False, True, True)), (1024, 1, 97, (False, False, False)), (1024, 1, 98, (False, False, True)),
-                                          (1025, 16, 16, (False, False, True)), (1000, 4, 205, (False, False, True)), (1000, 4, 206, (True, True, True)),
-                                          (64, 1, 4007, (False, False, True)), (64, 1, 4008, (True, True, True)), (60_001, 10, 6, (True, True, True)),
-                                          (20, 16, 13_000, (True, True, True))])
+@pytest.mark.parametrize("M,N,K,narrow", [(3072, 3, 2, (False, True, True)), (3073, 3, 2, (True, True, True)), (3072, 4, 2, (False, False, True)),
+                                          (3073, 4, 2, (True, True, True)), (2048, 3, 5, (False, False, True)), (2049, 3, 5, (False, True, True)),
+                                          (1024, 1, 97, (False, False, False)), (1024, 1, 98, (False, False, True)), (4096, 16, 3, (False, False, True)),
+                                          (4097, 16, 3, (True, True, True)), (2048, 16, 60, (False, False, False)), (2049, 16, 60, (False, False, True)),
+                                          (1000, 4, 205, (False, False, True)), (1000, 4, 206, (True, True, True)), (64, 1, 4007, (False, False, True)),
+                                          (64, 1, 4008, (True, True, True)), (60_001, 10, 6, (True, True, True)), (20, 16, 19_000, (True, True, True))])
 def test_few_rows_and_many(ctx, oracle, M, N, K, narrow):
     r = np.random.Generator(np.random.Philox(M + N + K))
     f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
@@ -91,6 +92,9 @@ def test_few_rows_and_many(ctx, oracle, M, N, K, narrow):
         assert ran(lambda: ctx.gemm_bwd(a, b, y, M, N, K, dA=dA, dB=dB, dbias=db, **kw)) == narrow[1 + k]
         close(dA, oracle.gemm(z, B, transB=True, f64=True), N, "dA")
         close(dB, oracle.gemm(A, z, transA=True, f64=True), M, "dB")
+        alone = out()[0]
+        ctx.gemm_bwd(None, b, y, M, N, K, dA=alone, **kw)
+        close(alone, oracle.gemm(z, B, transB=True, f64=True), N, "dA alone")
         close(db, z.astype(np.float64).sum(0), M, "dbias")
 
 
