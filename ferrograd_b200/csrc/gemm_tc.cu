@@ -2610,7 +2610,12 @@ ConvPlan plan_conv(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, uint32
 // The pair kernel for one matrix: 256 x 256 tiles on SM pairs, plus the passes that make the pairs of `prep` elements.
 double pair_cycles(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, double prep_elems, int prep_launches) {
     const uint64_t pairs = (uint64_t)ctx->sm_count / 2, tiles = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
-    const double tile = (double)((K + 31) / 32) * 1250.0, whole = (double)(tiles / pairs) * tile;
+    // A tile's k-blocks, or, of a few of them, the store that they hide only partly (8192 x 2048 with k of 32 / 128 / 512: 45 / 51 / 70 us); where
+    // rows of the result start off 16 bytes, four words to a lane, both (9128 x 1497 with k of 3 / 256 / 1000 113 / 119 / 195 us, 3000 x 3001 x 1000
+    // 135; by the conversion kernel 61 / 79 / 164 and 110).
+    const double nkb = (double)((K + 31) / 32), store = 12500.0 + nkb * 750.0;
+    const double tile = N % 4 ? 45000.0 + nkb * 1300.0 : nkb * 1250.0 > store ? nkb * 1250.0 : store;
+    const double whole = (double)(tiles / pairs) * tile;
     const uint64_t rem = tiles % pairs;
     double tail = rem ? tile : 0.0;
     const uint64_t nchunks = (K + kChunkK - 1) / kChunkK;
@@ -3014,7 +3019,10 @@ Route pick_route(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool pai
     Route r{pair_ok ? (int)kRoutePair : (int)kRoutePlanes, ConvPlan{}};
     if (!conv_allowed(ctx)) return r;
     r.conv = plan_conv(ctx, M, N, K, 1);
-    const double conv = r.conv.cycles + copied * 8.0 / 2500.0 + 4000.0 * copied_n;
+    // (beside the pair kernel's, the time of several units on every SM is 8 % short: 8192 x 2048 x 512 76 us, by the pair kernel 70, dB of 1500 x 2048 x
+    // 2048 60 and 49)
+    const bool several = r.conv.split == 1 && (uint64_t)((M + BM - 1) / BM) * ((N + r.conv.bn - 1) / r.conv.bn) > (uint64_t)ctx->sm_count;
+    const double conv = r.conv.cycles * (pair_ok && several ? 1.08 : 1.0) + copied * 8.0 / 2500.0 + 4000.0 * copied_n;
     // planes: both operands read and written twice over, transposed on the way, then 256 x 256 or 128-row tiles
     const double other = pair_ok ? pair_cycles(ctx, M, N, K, missing, missing_n)
                        : M > (uint32_t)BM && N > 128 ? pair_cycles(ctx, M, N, K, 2.0 * ((double)M * K + (double)N * K), 2) : 1e30;
