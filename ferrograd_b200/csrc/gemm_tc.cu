@@ -1238,8 +1238,9 @@ template <> __device__ __forceinline__ __half lp_from_float<__half>(float v) { r
 template <> __device__ __forceinline__ __nv_bfloat16 lp_from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
 // 32 rows x 32 * W columns per block, W columns per thread: 16 bytes of them, or, for any shape and alignment, one in 32.  All loads
-// first, three blocks an SM by registers and column sums that lie 36 words apart: with eight apart and two blocks an SM, dZ of
-// 2048 x 4096 bf16 through GELU took 20 - 30 us for 50 MB.
+// first, and column sums that lie 36 words apart: with eight apart and two blocks an SM, dZ of 2048 x 4096 bf16 through GELU took 20 -
+// 30 us for 50 MB.  Blocks an SM by registers: three of bf16, four of f16, five of f32 (asked for three, the compiler took 40 registers
+// for f32 and spilled: dB and bias gradient of 9216 x 4096 x 8 93 us, 85 with five; f16 4096 x 4096 x 64 23.8 with three, 21.0 with four).
 constexpr int kPrepPitch = 36;
 template <typename T, int W, bool VEC>
 __device__ __forceinline__ void prep_block(const PrepArgs& a, uint32_t bx, uint32_t by, uint32_t bz, float* cs) {
@@ -1317,7 +1318,7 @@ struct PrepJobs {
     uint32_t width[3], gx[3], gy[3], first[4];      // columns per thread (0: 16 bytes of them); blocks across and down a matrix; the first block of each
 };
 template <typename T>
-__global__ void __launch_bounds__(256, 3) prep_kernel(const __grid_constant__ PrepJobs p) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : std::is_same_v<T, __half> ? 4 : 3) prep_kernel(const __grid_constant__ PrepJobs p) {
     fg_grid_enter();
     constexpr int W = 16 / sizeof(T);
     __shared__ float room[8 * W * kPrepPitch];
