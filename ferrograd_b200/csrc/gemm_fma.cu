@@ -602,7 +602,10 @@ int32_t fg_gemm_fma_launch(fg_ctx* ctx, const FgFmaOp* ops, int n, uint32_t batc
 bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products) {
     if (products != kFgForward && N <= 16) return false;                // the narrow layer's own kernels
     auto padded = [](uint64_t m, uint64_t n, uint64_t k) { return (m + 15) / 16 * 16 * ((n + kTN - 1) / kTN * kTN) * ((k + 31) / 32 * 32); };
-    if (products == kFgForward) return N > 16 && padded(M, N, K) <= 45000000ull;
+    // (where the conversion kernel needs no copies and its tiles wait for their stores alone it is ahead sooner: 6000 x 128 x 32 5.9 us, 5.1 by that
+    // kernel, 2500 x 256 x 48 7.5 / 5.5, 1000 x 400 x 96 6.3 / 5.9; 2500 x 128 x 32 4.4 / 5.1, 256 x 2000 x 64 5.4 / 5.5)
+    const uint64_t most = K % 4 || N % 4 || K > 128 ? 45000000ull : K <= 32 ? 18000000ull : K <= 64 ? 36000000ull : 40000000ull;
+    if (products == kFgForward) return N > 16 && padded(M, N, K) <= most;
     const uint64_t work = (products & kFgGradB ? padded(K, N, M) : 0) + (products & kFgGradA ? padded(M, K, N) : 0);
     return work <= (products != (kFgGradA | kFgGradB) ? 40000000ull : N % 4 ? 24000000ull : 32000000ull);
 }
