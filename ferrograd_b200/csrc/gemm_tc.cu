@@ -3085,7 +3085,7 @@ int32_t gemm_fwd_core(fg_ctx* ctx, int32_t mode, int32_t transA, int32_t transB,
     const int path = pick_path(ctx, mode, M, N, K);
     // The result's pairs, when no GEMM epilogue wrote them.
     auto pairs_after = [&]() -> int32_t { return c_pairs ? launch_pairs(ctx, C, mn, c_pairs, c_stride) : FG_OK; };
-    const bool short_k = path == 0 && !transA && !transB && !c_pairs && fg_gemm_simt_suits(M, N, K);
+    const bool short_k = path == 0 && mode == FG_GEMM_AUTO && !c_pairs && fg_gemm_simt_suits(M, N, K);
     if (!short_k && takes_fma(ctx, mode, M, N, K, kFgForward)) {
         FgFmaOp o{};
         o.ta = transA; o.tb = transB; o.M = M; o.N = N; o.K = K; o.A = A.x; o.B = B.x; o.C = C;

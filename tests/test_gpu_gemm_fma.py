@@ -192,13 +192,14 @@ def test_infinities_and_nan(ctx):
 @pytest.mark.parametrize("M,N,K,exact", [(64, 16, 2, True), (1, 1, 1, True), (700, 32, 32, True), (700, 36, 32, False), (700, 33, 64, True), (700, 33, 65, False),
                                          (16384, 17, 8, True), (300, 28, 33, False), (3, 8189, 32, True), (3, 8193, 32, False), (20, 4095, 64, True),
                                          (20, 4097, 64, False), (5000, 17, 40, True), (32768, 32, 3, True)])
-def test_forward_of_a_short_k(ctx, oracle, M, N, K, exact):
+@pytest.mark.parametrize("tA,tB", [(False, False), (True, False), (False, True), (True, True)])
+def test_forward_of_a_short_k(ctx, oracle, M, N, K, exact, tA, tB):
     r = rng(M + N + K)
     A, B, bias = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32), r.standard_normal(N, np.float32)
-    a, b, v = up(ctx, A), up(ctx, B), up(ctx, bias)
+    a, b, v = up(ctx, A.T if tA else A), up(ctx, B.T if tB else B), up(ctx, bias)
     C, P, E = (up(ctx, np.zeros((M, N))) for _ in range(3))
-    ctx.gemm(a[1], b[1], C[1], M, N, K, bias=v[1], act="tanh", preact_out=P[1])
-    ctx.gemm(a[1], b[1], E[1], M, N, K, bias=v[1], act="none", mode="simt")
+    ctx.gemm(a[1], b[1], C[1], M, N, K, transA=tA, transB=tB, bias=v[1], act="tanh", preact_out=P[1])
+    ctx.gemm(a[1], b[1], E[1], M, N, K, transA=tA, transB=tB, bias=v[1], act="none", mode="simt")
     got = ctx.to_numpy(P[0])
     assert np.array_equal(got, ctx.to_numpy(E[0])) == exact
     check(got.reshape(M, N), oracle.gemm(A, B, f64=True).astype(np.float64) + bias, K, "pre-activation")
