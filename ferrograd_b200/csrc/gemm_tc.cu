@@ -3644,8 +3644,8 @@ bool batch_route_open(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, u
            (N > 16 || mode != FG_GEMM_AUTO);
 }
 
-// Small matrices: the sums of a batch come in the order of k, whichever kernel adds them and also one matrix at a time (padding between the
-// matrices of a layer with an activation, more than 65535 of them): the loops ask for the exact path.
+// Small matrices: the sums of a batch come in the order of k, whichever kernel adds them and also one matrix at a time (more than 65535 of
+// them, or no room for the dZ of matrices with room between them): the loops ask for the exact path.
 int32_t batch_loop_mode(const fg_ctx* ctx, int32_t mode, uint32_t M, uint32_t N, uint32_t K) {
     return mode == FG_GEMM_AUTO && pick_path(ctx, mode, M, N, K) == 0 ? (int32_t)FG_GEMM_SIMT : mode;
 }
@@ -3806,34 +3806,46 @@ int32_t fg_gemm_batched_bwd_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint3
     FG_REQUIRE(ctx, strideA >= (uint64_t)M * K && strideB >= (uint64_t)K * N && strideC >= (uint64_t)M * N,
                "fg_gemm_batched_bwd_f32: a stride is smaller than its matrix");
     if (batch == 0 || (uint64_t)M * N == 0 || (!dA && !dB)) return FG_OK;
-    if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && (strideC == (uint64_t)M * N || (act == FG_ACT_NONE && K > 0))) {
+    // (of matrices with room between them dZ is formed without it, if the arena has the room for that; the pass takes 65535 tiles of 32 rows)
+    const bool dense_z = strideC == (uint64_t)M * N;
+    auto apart_z = [&] { return K > 0 && M <= 65535u * 32u && fg_ws_try(ctx, (uint64_t)batch * M * N * 4 + 512); };
+    if (pick_path(ctx, mode, M, N, K) == 0 && batch <= 65535 && (dense_z || (act == FG_ACT_NONE ? K > 0 : apart_z()))) {
         // dZ = dY * act'(saved) for the whole batch, then dB[t] = A[t]^T dZ[t] and dA[t] = dZ[t] B[t]^T: sums in the order of k
         const float* dz = dY;
+        uint64_t sz = strideC;
         if (act != FG_ACT_NONE) {
             const uint64_t n = (uint64_t)batch * M * N;
             void* p;
             int32_t s = fg_ws_ensure(ctx, n * 4 + 512);
             if (s != FG_OK) return s;
             if ((s = fg_ws_alloc(ctx, n * 4, &p)) != FG_OK) return s;
-            if ((s = fg_act_bwd_launch(ctx, n, act, dY, saved, (float*)p)) != FG_OK) return s;
+            if (dense_z) s = fg_act_bwd_launch(ctx, n, act, dY, saved, (float*)p);
+            else {
+                PrepArgs a{};
+                a.x = dY; a.saved = saved; a.act = act; a.R = M; a.C = N; a.x_batch = strideC; a.out = p; a.ld = N;
+                PrepBatch prep;
+                if ((s = prep.add(ctx, FG_DTYPE_F32, a, batch)) == FG_OK) s = prep.launch(ctx);
+                sz = (uint64_t)M * N;
+            }
+            if (s != FG_OK) return s;
             dz = (const float*)p;
         }
         int32_t s;
         const bool large_b = batch_large(ctx, mode, batch, K, N), large_a = batch_large(ctx, mode, batch, M, K);
         FgFmaOp ops[2] = {};
         FgFmaOp &w = ops[0], &x = ops[1];
-        w.ta = 1; w.M = K; w.N = N; w.K = M; w.A = A; w.B = dz; w.C = dB; w.sA = strideA; w.sB = strideC; w.sC = strideB;
-        x.tb = 1; x.M = M; x.N = K; x.K = N; x.A = dz; x.B = B; x.C = dA; x.sA = strideC; x.sB = strideB; x.sC = strideA;
+        w.ta = 1; w.M = K; w.N = N; w.K = M; w.A = A; w.B = dz; w.C = dB; w.sA = strideA; w.sB = sz; w.sC = strideB;
+        x.tb = 1; x.M = M; x.N = K; x.K = N; x.A = dz; x.B = B; x.C = dA; x.sA = sz; x.sB = strideB; x.sC = strideA;
         // one launch for both where nothing was formed before, unless a gradient lies over what the other product reads
         const uint64_t na = ((batch - 1) * strideA + (uint64_t)M * K) * 4, nb = ((batch - 1) * strideB + (uint64_t)K * N) * 4,
-                       nc = ((batch - 1) * strideC + (uint64_t)M * N) * 4;
+                       nc = ((batch - 1) * sz + (uint64_t)M * N) * 4;
         auto over = [&](const void* p, uint64_t n) { return fg_ranges_meet(p, n, A, na) || fg_ranges_meet(p, n, B, nb) || fg_ranges_meet(p, n, dz, nc); };
         if (dA && dB && act == FG_ACT_NONE && mode == FG_GEMM_AUTO && large_a == large_b && !over(dA, na) && !over(dB, nb)) {
             return large_a ? fg_gemm_fma_launch(ctx, ops, 2, batch, true)
-                           : fg_gemm_simt_batched_bwd_launch(ctx, batch, M, N, K, A, strideA, B, strideB, dz, strideC, dA, dB);
+                           : fg_gemm_simt_batched_bwd_launch(ctx, batch, M, N, K, A, strideA, B, strideB, dz, sz, dA, dB);
         }
-        if (dB && (s = fg_gemm_simt_batched_launch(ctx, 1, 0, batch, K, N, M, A, strideA, dz, strideC, dB, strideB, nullptr, FG_ACT_NONE, nullptr)) != FG_OK) return s;
-        return dA ? fg_gemm_simt_batched_launch(ctx, 0, 1, batch, M, K, N, dz, strideC, B, strideB, dA, strideA, nullptr, FG_ACT_NONE, nullptr) : FG_OK;
+        if (dB && (s = fg_gemm_simt_batched_launch(ctx, 1, 0, batch, K, N, M, A, strideA, dz, sz, dB, strideB, nullptr, FG_ACT_NONE, nullptr)) != FG_OK) return s;
+        return dA ? fg_gemm_simt_batched_launch(ctx, 0, 1, batch, M, K, N, dz, sz, B, strideB, dA, strideA, nullptr, FG_ACT_NONE, nullptr) : FG_OK;
     }
     if (batch_route_open(ctx, mode, M, N, K)) {
         const bool n8 = N % 8 == 0 && K % 8 == 0;

@@ -209,7 +209,7 @@ def test_forward_of_a_short_k(ctx, oracle, M, N, K, exact, tA, tB):
 @pytest.mark.parametrize("T,M,N,K", [(7, 33, 66, 97), (3, 2, 300, 256), (5, 200, 10, 70)])
 @pytest.mark.parametrize("gap", [0, 5])
 def test_batched_sums_are_in_order_with_an_activation(ctx, T, M, N, K, gap):
-    # room between the matrices changes no bit: with an activation they are then taken one at a time
+    # room between the matrices changes no bit, nor the number of launches: dZ of the whole batch, then the products
     r = rng(T + M)
     f = lambda *s: up(ctx, r.standard_normal(s).astype(np.float32))           # noqa: E731
     st = (M * K + gap, K * N + gap, M * N + gap)
@@ -218,6 +218,9 @@ def test_batched_sums_are_in_order_with_an_activation(ctx, T, M, N, K, gap):
     for mode in ("auto", "simt"):
         dA, dB = up(ctx, np.zeros((T, st[0]))), up(ctx, np.zeros((T, st[1])))
         ctx.gemm_batched_bwd(a[1], b[1], y[1], T, M, N, K, act="gelu", saved=sv[1], dA=dA[1], dB=dB[1], strides=st, mode=mode)
+        before = ctx.launch_count()
+        ctx.gemm_batched_bwd(a[1], b[1], y[1], T, M, N, K, act="gelu", saved=sv[1], dA=dA[1], dB=dB[1], strides=st, mode=mode)
+        assert ctx.launch_count() - before == 3
         out.append((ctx.to_numpy(dA[0]), ctx.to_numpy(dB[0])))
     for x, e in zip(*out):
         assert np.array_equal(x, e)
