@@ -867,11 +867,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         if (col + 1 < col_lim) bz.y = epi_bias(ep.bias, col + 1, ep.out_dtype);
                         if (col + 2 < col_lim) bz.z = epi_bias(ep.bias, col + 2, ep.out_dtype);
                         if (col + 3 < col_lim) bz.w = epi_bias(ep.bias, col + 3, ep.out_dtype);
-                    } else if (col + 3 < col_lim) bz = __ldg(reinterpret_cast<const float4*>(ep.bias + col));
-                    else {
+                    } else if (col + 3 < col_lim && (reinterpret_cast<uintptr_t>(ep.bias) & 15u) == 0) {
+                        bz = __ldg(reinterpret_cast<const float4*>(ep.bias + col));
+                    } else {      // the last columns, or a bias that starts off 16 bytes
                         if (col < col_lim) bz.x = ep.bias[col];
                         if (col + 1 < col_lim) bz.y = ep.bias[col + 1];
                         if (col + 2 < col_lim) bz.z = ep.bias[col + 2];
+                        if (col + 3 < col_lim) bz.w = ep.bias[col + 3];
                     }
                 }
                 float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);     // column sums of what this lane stores (rows i*4 + rsub)
