@@ -2915,10 +2915,12 @@ int32_t tc_gemm(fg_ctx* ctx, int fmt, const PlaneSet& a, const PlaneSet& b, uint
 // descriptors, so nothing is ever transposed, and whoever produces a tensor (a GEMM
 // epilogue, the optimizer, the kernels below) writes its pairs in the same pass.
 // ------------------------------------------------------------------------------------
+// (VEC: x starts on 16 bytes)
+template <bool VEC>
 __global__ void __launch_bounds__(256) pairs_kernel(const float* __restrict__ x, uint64_t n, __nv_bfloat16* __restrict__ pairs,
                                                     uint64_t plane_stride) {
     fg_grid_enter();
-    const uint64_t nv = n >> 2, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t nv = VEC ? n >> 2 : 0, stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride)
         fg_store_pairs4(pairs, plane_stride, i * 4, __ldcs(reinterpret_cast<const float4*>(x) + i));
     for (uint64_t i = (nv << 2) + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
@@ -2950,7 +2952,8 @@ __global__ void __launch_bounds__(128) dz_pairs_kernel(uint32_t R, uint32_t C, c
 
 int32_t launch_pairs(fg_ctx* ctx, const float* x, uint64_t n, __nv_bfloat16* pairs, uint64_t plane_stride) {
     fg_time_rec* tr = fg_time_begin(ctx, FG_KERNEL_SPLIT, 8.0 * (double)n);
-    fg_launch(ctx, pairs_kernel, fg_stream_grid(ctx, (n + 3) / 4, 256, 8), 256, 0, x, n, pairs, plane_stride);
+    if (fg_aligned16(x)) fg_launch(ctx, pairs_kernel<true>, fg_stream_grid(ctx, (n + 3) / 4, 256, 8), 256, 0, x, n, pairs, plane_stride);
+    else fg_launch(ctx, pairs_kernel<false>, fg_stream_grid(ctx, n, 256, 8), 256, 0, x, n, pairs, plane_stride);
     fg_time_end(ctx, tr);
     FG_LAUNCHED(ctx);
     return FG_OK;

@@ -46,3 +46,25 @@ def test_a_bias_off_the_boundary(ctx, oracle, shift, tile, M, N, K, mode):
     z = oracle.gemm(A, B, f64=True).astype(np.float64) + bias
     ok, worst = rel_err_ok(ctx.to_numpy(C[0]).reshape(M, N), np.maximum(z, 0), TOL)
     assert ok, f"{worst:.3g}"
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", [(4096, 10, 512), (300, 101, 1000), (40, 24, 16)])
+def test_pairs_of_results_off_the_boundary(ctx, oracle, shift, M, N, K):
+    # forward (a narrow layer, a ragged one, a small one) and dA of the layer above, whose pairs are those of what was stored
+    from ferrograd_b200.backend import to_bf16_bits
+    r = rng(M + N + K)
+    A, B, dZ = r.standard_normal((M, K), np.float32), r.standard_normal((K, N), np.float32) * np.float32(K ** -0.5), r.standard_normal((M, N), np.float32)
+    a, b, z = up(ctx, A), up(ctx, B), up(ctx, dZ)
+    C, dA, dB = up(ctx, np.zeros((M, N)), shift), up(ctx, np.zeros((M, K)), shift), up(ctx, np.zeros((K, N)))
+    sc, sa = (M * N + 7) // 8 * 8, (M * K + 7) // 8 * 8
+    pc, pa = ctx.new_tensor((2, sc), np.uint16), ctx.new_tensor((2, sa), np.uint16)
+    ctx.gemm_paired(a[1], b[1], C[1], M, N, K, C_pairs=pc, C_stride=sc)
+    ctx.gemm_bwd_paired(a[1], b[1], z[1], M, N, K, dB=dB[1], dA=dA[1], dA_pairs=pa, dA_stride=sa)
+    for x, p, ref, what in ((C, pc, oracle.gemm(A, B, f64=True), "C"), (dA, pa, oracle.gemm(dZ, B, transB=True, f64=True), "dA")):
+        got = ctx.to_numpy(x[0])[shift:].reshape(ref.shape)
+        ok, worst = rel_err_ok(got, ref, TOL)
+        assert ok, f"{what}: {worst:.3g}"
+        hi = (got.view(np.uint32) & np.uint32(0xffffe000)).view(np.float32)
+        q = ctx.to_numpy(p)[:, :got.size]
+        assert np.array_equal(q[0], to_bf16_bits(got).ravel()) and np.array_equal(q[1], to_bf16_bits(got - hi).ravel()), what
