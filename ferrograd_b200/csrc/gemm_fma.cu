@@ -603,8 +603,8 @@ bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products) {
     if (products != kFgForward && N <= 16) return false;                // the narrow layer's own kernels
     auto padded = [](uint64_t m, uint64_t n, uint64_t k) { return (m + 15) / 16 * 16 * ((n + kTN - 1) / kTN * kTN) * ((k + 31) / 32 * 32); };
     // (where the conversion kernel needs no copies and its tiles wait for their stores alone it is ahead sooner: 6000 x 128 x 32 5.9 us, 5.1 by that
-    // kernel, 2500 x 256 x 48 7.5 / 5.5, 1000 x 400 x 96 6.3 / 5.9; 2500 x 128 x 32 4.4 / 5.1, 256 x 2000 x 64 5.4 / 5.5)
-    const uint64_t most = K % 4 || N % 4 || K > 128 ? 45000000ull : K <= 32 ? 18000000ull : K <= 64 ? 36000000ull : 40000000ull;
+    // kernel, 2500 x 256 x 48 7.5 / 5.5, 1000 x 400 x 96 6.3 / 5.9; 2500 x 128 x 32 4.4 / 5.1, 240 x 2368 x 24 4.9 / 5.9, 256 x 2000 x 64 5.4 / 5.5)
+    const uint64_t most = K % 4 || N % 4 || K > 128 ? 45000000ull : K <= 32 ? 19000000ull : K <= 64 ? 36000000ull : 40000000ull;
     if (products == kFgForward) return N > 16 && padded(M, N, K) <= most;
     const uint64_t work = (products & kFgGradB ? padded(K, N, M) : 0) + (products & kFgGradA ? padded(M, K, N) : 0);
     return work <= (products != (kFgGradA | kFgGradB) ? 40000000ull : N % 4 ? 24000000ull : 32000000ull);
@@ -616,13 +616,13 @@ bool fg_gemm_fma_suits(uint32_t M, uint32_t N, uint32_t K, int products) {
 // 10.2, 1500 x 10 x 100 13.4 / 16.3, 3072 x 10 x 40 15.1 / 17.8, 4096 x 16 x 16 14.5 / 22.4, 4096 x 1 x 1 16.9 / 13.7, 1024 x 4 x 300 13.9 / 13.3,
 // 64 x 4 x 4000 7.5 / 10.1, 128 x 4 x 4000 11.4 / 10.9, 65536 x 4 x 4 285 / 64; the gradients alone 1500 x 1 x 64 8.8 / 9.1, 3072 x 4 x 40
 // 10.5 / 11.2, 496 x 16 x 496 (dB) 5.2 / 9.1, 3072 x 1 x 40 12.6 / 10.4; with an activation's factor on dZ 256 x 4 x 500 7.6 / 11.1,
-// 512 x 4 x 200 10.4 / 10.7, 1024 x 10 x 64 10.0 / 12.2, 2048 x 16 x 64 13.3 / 14.5, 1500 x 1 x 40 12.9 / 10.2; dA alone 1024 x 4 x 2 2.9 / 2.3.
+// 512 x 4 x 200 10.4 / 10.7, 536 x 12 x 336 9.6 / 12.9, 1024 x 10 x 64 10.0 / 12.2, 2048 x 16 x 64 13.3 / 14.5, 1500 x 1 x 40 12.9 / 10.2; dA alone 1024 x 4 x 2 2.9 / 2.3.
 bool fg_gemm_fma_suits_small(uint32_t M, uint32_t N, uint32_t K, int products) {
     if (N > 16 || products == kFgForward) return true;
     const bool quads = N % 4 == 0, wide = quads && N >= 12;
     const uint64_t mk = (uint64_t)M * K;
     if (!(products & kFgGradB)) return products & (kFgFactor | kFgBelow | kFgBias) ? M <= 4096 : M < 64;
-    if (products & kFgFactor) return M <= (wide ? 2048u : 1024u) && mk <= (M <= 256 ? 250000u : wide ? 140000u : 100000u);
+    if (products & kFgFactor) return M <= (wide ? 2048u : 1024u) && mk <= (M <= (wide ? 600u : 256u) ? 250000u : wide ? 140000u : 100000u);
     return M <= (wide ? 4096u : quads || (products & kFgBelow) ? 3072u : 2048u) && mk + 55ull * M <= (wide ? 380000u : 260000u);
 }
 
