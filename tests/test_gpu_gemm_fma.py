@@ -1,5 +1,6 @@
 """Products with plain FMAs in shares of k (few samples, or few multiply-adds): sizes around the four tile heights (4, 16, 32, 64),
-the tile's 64 columns, the stages' 32 and 64 k and the clusters' shares, in every orientation, on 16-byte boundaries and off them."""
+the tile's 64 columns, the stages' 32 and 64 k and the clusters' shares, in every orientation, on 16-byte boundaries and off them.  Among
+them forward products of a short k, which are the exact path's."""
 import math
 
 import numpy as np
@@ -36,7 +37,7 @@ def check(x, ref, k, what):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 64, 4096), (3, 65, 33), (4, 129, 200), (5, 63, 64), (16, 64, 2050), (17, 100, 31), (32, 16, 515),
-                                   (33, 200, 96), (63, 1, 1000), (40, 288, 2016), (64, 64, 64), (100, 130, 65), (1, 4100, 36)])
+                                   (33, 200, 96), (63, 1, 1000), (40, 288, 2016), (64, 64, 64), (100, 130, 65), (1, 4100, 36), (5, 63, 66), (3, 65, 97)])
 @pytest.mark.parametrize("tA,tB", [(False, False), (True, False), (False, True), (True, True)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_forward(ctx, oracle, M, N, K, tA, tB, shift):
@@ -62,24 +63,31 @@ def test_backward(ctx, oracle, M, N, K, act, shift):
     f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
     A, B, dY, S = f(M, K), f(K, N), f(M, N), np.tanh(f(M, N))
     t = [up(ctx, x, shift) for x in (A, B, dY, S)]
-    dA, dB, db = (up(ctx, np.zeros(s), shift) for s in ((M, K), (K, N), (N,)))
+    empty = lambda: [up(ctx, np.full(s, np.nan), shift) for s in ((M, K), (K, N), (N,))]      # noqa: E731
     dz = oracle.act_bwd(dY, S, act) if act != "none" else dY
+    refs = ((oracle.gemm(dz, B, transB=True, f64=True), N, "dA"), (oracle.gemm(A, dz, transA=True, f64=True), M, "dB"), (dz.astype(np.float64).sum(0), M, "dbias"))
 
-    def same(what):
-        check(ctx.to_numpy(dA[0])[shift:].reshape(M, K), oracle.gemm(dz, B, transB=True, f64=True), N, what + "dA")
-        check(ctx.to_numpy(dB[0])[shift:].reshape(K, N), oracle.gemm(A, dz, transA=True, f64=True), M, what + "dB")
-        check(ctx.to_numpy(db[0])[shift:], dz.astype(np.float64).sum(0), M, what + "dbias")
+    def same(outs, what, wanted=(True, True, True)):
+        for o, (ref, k, name), wants in zip(outs, refs, wanted):
+            x = ctx.to_numpy(o[0])[shift:].reshape(ref.shape)
+            if wants:
+                check(x, ref, k, what + name)
+            else:
+                assert np.isnan(x).all(), what + name + " was not asked for"
 
     sv = t[3][1] if act != "none" else None
+    dA, dB, db = empty()
     ctx.gemm_bwd(t[0][1], t[1][1], t[2][1], M, N, K, act=act, saved=sv, dA=dA[1], dB=dB[1], dbias=db[1])
-    same("")
+    same((dA, dB, db), "")
     # the gradients one by one, and the gradient of A over A itself
+    dA, dB, db = empty()
     ctx.gemm_bwd(t[0][1], None, t[2][1], M, N, K, act=act, saved=sv, dB=dB[1])
+    same((dA, dB, db), "one by one, ", (False, True, False))
     ctx.gemm_bwd(None, t[1][1], t[2][1], M, N, K, act=act, saved=sv, dA=dA[1], dbias=db[1])
-    same("one by one, ")
-    dA = t[0]
+    same((dA, dB, db), "one by one, ")
+    _, dB, db = empty()
     ctx.gemm_bwd(t[0][1], t[1][1], t[2][1], M, N, K, act=act, saved=sv, dA=t[0][1], dB=dB[1], dbias=db[1])
-    same("over A, ")
+    same((t[0], dB, db), "over A, ")
 
 
 @pytest.mark.parametrize("M,N", [(40, 40), (8, 200)])
@@ -130,19 +138,23 @@ def test_both_sides_of_the_range(ctx, oracle, M, N, K, act):
     f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
     A, B, dY, S, bias = f(M, K), f(K, N), f(M, N), f(M, N), f(N)
     a, b, y, sv, v = (up(ctx, x) for x in (A, B, dY, S, bias))
-    C, P, dA, dB, db = (up(ctx, np.zeros(s)) for s in ((M, N), (M, N), (M, K), (K, N), (N,)))
+    C, P = (up(ctx, np.full((M, N), np.nan)) for _ in range(2))
     # (the tensor-core kernels of the far side split an f32 into a tf32 and a bf16 rest: 2^-19 of a term)
     close = lambda x, ref, k, what: rel_err_ok(x, ref, 2.0 ** -24 * (16 + 5 * math.sqrt(k)) + 2.0 ** -19)[0] or pytest.fail(what)   # noqa: E731
     ctx.gemm(a[1], b[1], C[1], M, N, K, bias=v[1], act=act, preact_out=P[1])
     close(ctx.to_numpy(P[0]).reshape(M, N), oracle.gemm(A, B, f64=True) + bias, K, "pre-activation")
     dz = oracle.act_bwd(dY, S, act)
+    refs = {"dA": (oracle.gemm(dz, B, transB=True, f64=True), N), "dB": (oracle.gemm(A, dz, transA=True, f64=True), M)}
     for grads in (("dA", "dB"), ("dB",), ("dA",)):
-        ctx.gemm_bwd(a[1], b[1], y[1], M, N, K, act=act, saved=sv[1], dA=dA[1] if "dA" in grads else None, dB=dB[1] if "dB" in grads else None,
-                     dbias=db[1])
-        if "dA" in grads:
-            close(ctx.to_numpy(dA[0]).reshape(M, K), oracle.gemm(dz, B, transB=True, f64=True), N, f"dA of {grads}")
-        if "dB" in grads:
-            close(ctx.to_numpy(dB[0]).reshape(K, N), oracle.gemm(A, dz, transA=True, f64=True), M, f"dB of {grads}")
+        out = {"dA": up(ctx, np.full((M, K), np.nan)), "dB": up(ctx, np.full((K, N), np.nan))}
+        db = up(ctx, np.full(N, np.nan))
+        ctx.gemm_bwd(a[1], b[1], y[1], M, N, K, act=act, saved=sv[1], dbias=db[1], **{g: out[g][1] for g in grads})
+        for g, (ref, k) in refs.items():
+            x = ctx.to_numpy(out[g][0]).reshape(ref.shape)
+            if g in grads:
+                close(x, ref, k, f"{g} of {grads}")
+            else:
+                assert np.isnan(x).all(), f"{g} of {grads}"
         close(ctx.to_numpy(db[0]), dz.astype(np.float64).sum(0), M, f"dbias of {grads}")
 
 
@@ -175,9 +187,9 @@ def test_batched(ctx, oracle, T, M, N, K, act, gap):
         check(got(dB, K * N).reshape(K, N), oracle.gemm(At, dz, transA=True, f64=True), M, "dB")
 
 
-def test_infinities_and_nan(ctx):
+@pytest.mark.parametrize("M,N,K", [(5, 70, 40), (5, 72, 40), (5, 70, 100)])
+def test_infinities_and_nan(ctx, M, N, K):
     # what is outside the tensors does not meet them: an infinity reaches its own row and column, a NaN too, and zeros times them
-    M, N, K = 5, 70, 40
     A, B = np.ones((M, K), np.float32), np.ones((K, N), np.float32)
     A[1, 3] = np.inf
     A[2, K - 1] = np.nan

@@ -1,5 +1,5 @@
-"""The narrow layer's backward kernels at few samples, where chunks shrink and a single chunk takes the exact path, and the
-multi-tensor update at the sizes where its chunks shrink."""
+"""The narrow layer's backward kernels at few samples, where chunks shrink and a single chunk takes the exact path (of a long k: the FMA
+kernel takes the smaller layers), the line between the two, and the multi-tensor update at the sizes where its chunks shrink."""
 import numpy as np
 import pytest
 
@@ -23,7 +23,8 @@ def check(x, ref, what):
     assert ok, f"{what}: {worst:.3g}"
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 2, 16), (8, 16, 5), (64, 16, 2), (65, 10, 33), (100, 4, 520), (384, 12, 256), (1100, 3, 64), (64, 1, 8193), (50, 2, 20001)])
+@pytest.mark.parametrize("M,N,K", [(1, 2, 16), (8, 16, 5), (64, 16, 2), (65, 10, 33), (100, 4, 520), (384, 12, 256), (1100, 3, 64), (64, 1, 8193), (50, 2, 20001),
+                                   (8, 16, 50_000), (64, 16, 4100), (65, 13, 5100), (100, 4, 10_600), (384, 12, 920), (1100, 3, 1300)])
 def test_backward(ctx, oracle, M, N, K):
     r = np.random.Generator(np.random.Philox(M + N + K))
     f = lambda *s: r.standard_normal(s).astype(np.float32)                    # noqa: E731
