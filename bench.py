@@ -509,7 +509,7 @@ def run_ours(args, rank, world, local_rank):
 
     # ---- warm-up: plain launches first (they size the scratch arena), then the engine's own choice between
     #      plain launches and recorded CUDA graphs per dispatch (the reference's Schedule is a captured graph:
-    #      rocm/mod.rs:324-389; here only launch-bound graphs, and medium ones with a communicator, are recorded);
+    #      rocm/mod.rs:324-389; here graphs of many short launches, and medium ones with a communicator, are recorded);
     #      a dispatch is recorded on its second call, so four more steps settle that ----
     ctx.set_option("exec_plans", "0")
     net.upload_batch_async(xs[0], ts[0])
@@ -521,7 +521,7 @@ def run_ours(args, rank, world, local_rank):
     barrier()
     mode = ("dispatch_forward + dispatch_loss + dispatch_backward + dispatch_optim through the graph API, "
             + ("each replayed as a recorded CUDA graph" if net.tensors.plans_active() else
-               "plain asynchronous launches (the engine records CUDA graphs only for launch-bound graphs)")
+               "plain asynchronous launches (the engine records CUDA graphs only where the launches are many and short)")
             + ("; gradients summed over the ranks inside dispatch_backward / dispatch_optim (NCCL)" if world > 1 else ""))
     sampler = ClockSampler(local_rank) if rank == 0 else None
     if sampler:

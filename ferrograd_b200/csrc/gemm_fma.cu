@@ -1,6 +1,7 @@
 // f32 products with plain FMAs in shares of k: what FG_GEMM_AUTO runs where the tensor-core kernels' fixed costs, or their tiles of
-// 128 rows, are the most of a product -- fewer than 64 samples, or up to some 40 million multiply-adds (fg_gemm_fma_suits) --
-// forward and both gradients.
+// 128 rows, are the most of a product -- fewer than 64 samples, or up to some 20 to 45 million multiply-adds (fg_gemm_fma_suits) --
+// forward and both gradients, but for forward products of a short k (fg_gemm_simt_suits) and narrow layers of many rows
+// (fg_gemm_fma_suits_small).
 //
 // What it replaces: the reference's tiled matmul and its backward edges (crates/ferrograd-nn/src/op/matmul/mod.rs:17-188,
 // generic.rs:13-325) with the elementwise work around them: bias and activation (kernel/forward.rs:373-457), the activation's
@@ -444,7 +445,10 @@ FmaRows fma_rows(const FgFmaOp& o, uint32_t batch) {
 struct FmaPlan { int tile[2]; uint32_t lg_split; float cycles; };
 // Tile heights and K-shares by estimated cycles, fitted to 49 calls under every tile and split (2.2 % slower than the best of each in
 // the geometric mean, 22 % at most): a stage takes a CTA no less than its copies' latency (270), the ends of a unit 1430, a meeting of
-// shares 180 + 150 each, and three CTAs share an SM.  A word that is copied alone and one that is added to a column's sum take 0.05 more:
+// shares 180 + 150 each.  The fit counts rounds at three CTAs an SM; two are resident (102 to 128 registers a thread).  For two products the
+// rounds of all units times the longest unit of either only puts the plans in order: it is no time, least of all where one of them has many
+// units and the other a long k.
+// A word that is copied alone and one that is added to a column's sum take 0.05 more:
 // with that, the gradients of 28 layers, 13 of them with odd rows, take 7 % more than under the best plan of each in the geometric mean
 // and 12 % without (2000 x 100 x 30: 17.7 and 23.1 us); not with 16 columns or fewer, where most of a row's words are only zeroed
 // (gradients of 1000 x 100 x 4 9.1 us with it, 7.6 without, 300 x 200 x 13 7.0 and 6.1, 500 x 300 x 10 8.1 and 8.9; by the narrow

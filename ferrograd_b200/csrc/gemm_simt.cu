@@ -5,7 +5,8 @@
 // out = fmaf(As[ly][i], Bs[i][lx], out) over 16-wide k tiles), so results are bit-identical
 // to a sequential-k f32 FMA chain.  Unlike the reference (no bounds checks, shapes must be
 // multiples of 16: crates/fused_gpu/src/dispatch/backend/mod.rs:617-619) any M, N, K is
-// accepted.  The on-device exact reference for the other kernels: it runs when FG_GEMM_SIMT is requested.
+// accepted.  The on-device exact reference for the other kernels: it runs when FG_GEMM_SIMT is requested, and for FG_GEMM_AUTO's forward
+// products of a short k (fg_gemm_simt_suits), its small batches and its small gradients with dZ_out.
 //
 // TM x TN output tile per CTA, a thread owns RPT rows x 4 columns, k tiles of 32 through two shared-memory buffers.
 #include <atomic>

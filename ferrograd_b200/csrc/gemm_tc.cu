@@ -3036,7 +3036,8 @@ Route pick_route(const fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, bool pai
     return r;
 }
 
-// Which path a request takes: 0 = SIMT, otherwise the plane format + 1.
+// Which path a request takes: 0 = plain f32 FMAs (the exact path, or with FG_GEMM_AUTO the FMA kernel or the narrow layer's), otherwise the
+// plane format + 1.
 int pick_path(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K) {
     if (mode == FG_GEMM_SIMT) return 0;
     if (mode == FG_GEMM_3XTF32) return 1;
@@ -3047,7 +3048,7 @@ int pick_path(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K) {
 }
 
 // Does FG_GEMM_AUTO take the FMA kernel for the forward product, or for one or both gradients?  (An option that names a tensor-core
-// kernel keeps what those can run.)
+// kernel keeps what those can run; gemm_fwd_core keeps the forward products of a short k for the exact path's kernel.)
 bool takes_fma(const fg_ctx* ctx, int mode, uint32_t M, uint32_t N, uint32_t K, int products) {
     if (mode != FG_GEMM_AUTO) return false;
     if (pick_path(ctx, mode, M, N, K) == 0) return fg_gemm_fma_suits_small(M, N, K, products);
@@ -3719,7 +3720,7 @@ int32_t fg_gemm_bwd_paired_f32(fg_ctx* ctx, uint32_t M, uint32_t N, uint32_t K, 
 
 // Batched forms: `batch` independent products, operand t at base + t*stride (strides in elements).
 // The reference steps A, B and C by one matrix per Z index of a rank-3 matmul (kernel/forward.rs:159-190).
-// Rank-3 products.  Small matrices (the SIMT path's range: the matrix index is the grid's z, as in the reference's generated
+// Rank-3 products.  Small matrices (below the tensor cores' sizes: the matrix index is the grid's z, as in the reference's generated
 // kernel, kernel/forward.rs:159-190) and middling ones (the conversion kernel: it is part of the unit's number) run as ONE launch.  Large
 // ones: the bf16 pairs of the whole batch are made by one pass per operand, then one GEMM launch per matrix reads its
 // slice (batch + 2 launches, and a launch that fills the GPU gains nothing from being merged with its neighbours).
@@ -3765,7 +3766,7 @@ int32_t fg_gemm_batched_f32(fg_ctx* ctx, int32_t mode, uint32_t batch, uint32_t 
         }
     }
     const bool dense = strideA == (uint64_t)M * K && strideB == (uint64_t)K * N;
-    // the condition under which every per-matrix call below takes the path that reads pairs
+    // the condition under which a per-matrix call below takes the path that reads pairs, if it takes the pair kernel
     const bool shared_pairs = dense && mode == FG_GEMM_AUTO && N > 16 && N % 4 == 0 && strideC % 4 == 0 && fg_aligned16(A) &&
                               fg_aligned16(B) && fg_aligned16(C) && (!preact_out || fg_aligned16(preact_out)) &&
                               paired_shape_ok(ctx, M, N, K, K, N);

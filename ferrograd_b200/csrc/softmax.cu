@@ -827,9 +827,9 @@ int rows_grid(const fg_ctx* ctx, uint64_t blocks, int threads) {
 }
 
 // Called by the kernels that can add the mean themselves: do they (see fg_fold_in_launch)?  Otherwise a.mean stays for the caller.
-// With that, and launches that start while the kernel before them ends, the loss of 712 x 768 takes 8.0 us instead of 9.2 and 11.2
-// before the calls had their own module, 2384 x 64 8.0 / 8.0 / 10.4, 600 x 32000 39.3 / 41.2, 8192 x 32000 361 / 365; softmax and its
-// gradient on 1728 x 1285 9.6 / 12.5, 4096 x 10001 132.6 / 137.1.
+// With that, and launches that start while the kernel before them ends, back to back (before that, plain launches): the loss of 712 x 768 takes
+// 4.5 us (6.8), 2384 x 64 4.5 (6.1), 300 x 1001 4.6 (6.8), 600 x 32000 36.1 (37.4), 8192 x 32000 391 (391); softmax
+// and its gradient on 1728 x 1285 9.6 (12.5), 4096 x 10001 132.6 (137.1).
 template <int MODE>
 CeArgs with_mean(fg_ctx* ctx, CeArgs& a, int grid) {
     CeArgs k = a;

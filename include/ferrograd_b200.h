@@ -54,9 +54,12 @@ enum fg_act { FG_ACT_NONE = 0, FG_ACT_RELU = 1, FG_ACT_TANH = 2, FG_ACT_GELU = 3
 
 /* How the f32 GEMM is computed. */
 enum fg_gemm_mode {
-    FG_GEMM_AUTO = 0,   /* FG_GEMM_TF32_BF16X2 when the shape is large enough; plain-FMA streaming
-                           kernels when N <= 16 (a narrow output layer); else plain FMAs with
-                           the sums over k in shares (fewer than 64 rows or 2^22 multiply-adds) */
+    FG_GEMM_AUTO = 0,   /* by size.  From 64 rows and 2^22 multiply-adds on FG_GEMM_TF32_BF16X2, with two
+                           exceptions in plain f32 FMAs: N <= 16 (a narrow output layer: streaming kernels),
+                           and up to some 20 - 45 million multiply-adds (the sums over k in shares).  Smaller
+                           products: plain FMAs, the sums in shares; in sequence, as FG_GEMM_SIMT, for
+                           forward products of a short k, for batches and for gradients with dZ_out; the
+                           streaming kernels for the gradients of N <= 16 with many rows */
     FG_GEMM_SIMT = 1,   /* sequential-k fmaf, bit-identical to the reference kernel body
                            (crates/ferrograd-nn/src/op/matmul/generic.rs:98-319) */
     FG_GEMM_3XTF32 = 2, /* tcgen05 kind::tf32, hi/lo split, three MMAs per k-step */
